@@ -962,3 +962,16 @@ def test_score_softcap_in_every_attention_kernel(ops, dtype, plan, seqs, spike):
     uncapped, exp_uncapped, _, _ = attention_case(ops, dtype, Hq, Hkv, D, page, seqs, plan=plan, spike=spike, window=190)
     assert rel(uncapped, exp_uncapped) < TOL[dtype]
     assert (exp - exp_uncapped).abs().max() > 0.05                          # the cap is what the comparison above rests on
+
+
+@pytest.mark.parametrize("B,M,N,K,off", [(1, 64, 128, 16, 0), (1, 65, 129, 20, 0), (1, 63, 127, 4100, 0), (1, 300, 2304, 2048, 0), (1, 40, 3, 8192, 0),
+                                         (1, 34, 260, 1021, 0), (1, 129, 130, 516, 3), (3, 70, 40, 260, 0), (5, 33, 257, 1283, 1)])
+def test_gemm_f32_tile_ranges(ops, B, M, N, K, off):
+    """The tile form at the edges of its tiles, with one K range and with several that a cluster adds up, in 16-byte and in
+    single copies, alone and in a batch.  A sum of K products of unit-variance values in 32 bits, in any order, is off by less than
+    K roundings of its running magnitude: sqrt(K) * 2^-24 * sqrt(K) against a result of sqrt(K)."""
+    g = torch.Generator().manual_seed(17)
+    x, w = torch.randn(B, M, K + 4, generator=g).to(DEV)[:, :, off:off + K], torch.randn(B, N, K, generator=g).to(DEV)
+    exp = torch.einsum("bmk,bnk->bmn", x.double(), w.double())
+    got = ops.batched_linear(x, w) if B > 1 else ops.linear(x[0], w[0], torch.ones(N, device=DEV))[None] - 1.0
+    assert (got.double() - exp).abs().max().item() < 4 * K ** 0.5 * K ** 0.5 * 2.0 ** -24 + 2e-6

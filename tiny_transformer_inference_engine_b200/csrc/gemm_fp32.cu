@@ -1,67 +1,164 @@
 // True 32-bit matrix product for the float32 path: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]).
 // Plain FFMA with float32 accumulation - no tensor cores, no TF32 - so that the float32
 // path shows faults that reduced precision would hide.  Any M, N, K.
-// Two kernels: a 64 x 64 tile for prompt portions, and for up to 16 rows (decode steps) a form that streams the weight
+// Two kernels: a 64 x 128 tile for prompt portions, and for up to 16 rows (decode steps) a form that streams the weight
 // matrix once: a warp owns four weight rows at a time, its lanes walk K in 16-byte steps, and the activations - a few
 // rows that every warp reads - come through the cache.
 #include "common.cuh"
 using namespace ttie;
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;      // 256 threads, 4x4 outputs each
+// ---- the tile form.  What bounds it is the FMA pipe (74 TFLOP/s nominal), so everything else has to hide behind it: a thread
+// owns 8 x 8 outputs (one shared-memory load of 16 bytes feeds 16 multiply-adds), both operands lie in shared memory as they
+// do in memory, K along the row, so that they travel as asynchronous 16-byte copies through three stages without a register or
+// a transposition in between, and a load's four values along K are two pairs for the packed multiply-add.  Accumulators are
+// pairs too (even and odd K), added at the end.  Rows are 20 floats apart: the eight rows that a warp reads at once fall into
+// different banks.  Too few tiles for the GPU: a cluster of CTAs shares a tile, each walks a range of K, and the partial tiles
+// are added through distributed shared memory in the order of the ranges.
+// 300 rows times [2304, 2048], [2048, 2048], [16384, 2048] and [2048, 8192] (36 GFLOP): 1,121 us, 32 TFLOP/s; 2,393 us as a 64 x 64
+// tile of 4 x 4 outputs staged through registers.
+constexpr int BM = 64, BN = 128, BK = 16, PITCH = BK + 4, STAGES = 3, MAX_RANGES = 8;
+constexpr int STAGE_FLOATS = (BM + BN) * PITCH;
+constexpr int TILE_SMEM = STAGES * STAGE_FLOATS * 4;                  // 46,080 bytes; holds a partial tile (32,768) at the end
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
-                long long batch_a, long long batch_w, long long batch_c) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    A += blockIdx.z * batch_a; W += blockIdx.z * batch_w; C += blockIdx.z * batch_c;      // (a batch of products: grid z)
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int tx = tid % 16, ty = tid / 16;
-    float acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+__device__ __forceinline__ void fma_pair(float2& d, float2 a, float2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+}
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64 rows x 16 k per operand = 1024 elements, 4 per thread; k is the fast index in memory
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int e = tid + i * 256;
-            const int r = e / BK, kk = e % BK;
-            const int gm = m0 + r, gn = n0 + r, gk = k0 + kk;
-            As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
-            Ws[kk][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], w[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * TM + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tx * TN + j;
-            if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j] + (bias ? bias[gn] : 0.f);
-        }
+// VEC: rows start on 16 bytes and K is a multiple of 4, so a row travels in 16-byte copies; else value by value.
+template <bool VEC>
+__device__ __forceinline__ void stage_operand(float* dst, const float* src, int ld, int rows, int row0, int row_end, int k0, int k_end) {
+    constexpr int W = VEC ? 4 : 1, PER_ROW = BK / W;
+    for (int e = threadIdx.x; e < rows * PER_ROW; e += 128) {
+        const int r = e / PER_ROW, k = (e % PER_ROW) * W;
+        const bool in = row0 + r < row_end && k0 + k < k_end;
+        const float* p = in ? src + (size_t)(row0 + r) * ld + k0 + k : src;        // (nothing is read where the size is 0)
+        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + r * PITCH + k);
+        if (VEC) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(p), "r"(in ? 16 : 0) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(d), "l"(p), "r"(in ? 4 : 0) : "memory");
     }
 }
+
+template <bool VEC>
+__global__ void __launch_bounds__(128, 2)
+gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
+                long long batch_a, long long batch_w, long long batch_c, int ranges, int range_len) {
+    __shared__ __align__(16) float smem[STAGES * STAGE_FLOATS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = blockIdx.x % ranges;                                                 // clusters are consecutive CTAs along x
+    A += blockIdx.z * batch_a; W += blockIdx.z * batch_w; C += blockIdx.z * batch_c;      // (a batch of products: grid z)
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x / ranges * BN;
+    const int k_lo = rank * range_len, k_hi = min(K, k_lo + range_len);
+    const int tm = (warp >> 1) * 32 + (lane >> 3), tn = (warp & 1) * 64 + (lane & 7);     // the thread's rows tm + 4 i, columns tn + 8 j
+    float2 acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    const int steps = (k_hi - k_lo + BK - 1) / BK;
+    auto stage = [&](int it) {
+        if (it < steps) {
+            float* s = smem + it % STAGES * STAGE_FLOATS;
+            stage_operand<VEC>(s, A, lda, BM, m0, M, k_lo + it * BK, k_hi);
+            stage_operand<VEC>(s + BM * PITCH, W, ldw, BN, n0, N, k_lo + it * BK, k_hi);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int it = 0; it < STAGES - 1; ++it) stage(it);
+    for (int it = 0; it < steps; ++it) {
+        asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2) : "memory");
+        __syncthreads();                                              // this step's rows are there, and everyone is done with the stage refilled next
+        stage(it + STAGES - 1);
+        const float* as = smem + it % STAGES * STAGE_FLOATS + tm * PITCH;
+        const float* ws = smem + it % STAGES * STAGE_FLOATS + (BM + tn) * PITCH;
+#pragma unroll
+        for (int k = 0; k < BK; k += 4) {
+            float4 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(as + 4 * i * PITCH + k);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 w = *reinterpret_cast<const float4*>(ws + 8 * j * PITCH + k);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    fma_pair(acc[i][j], make_float2(a[i].x, a[i].y), make_float2(w.x, w.y));
+                    fma_pair(acc[i][j], make_float2(a[i].z, a[i].w), make_float2(w.z, w.w));
+                }
+            }
+        }
+    }
+    if (ranges == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int gm = m0 + tm + 4 * i;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int gn = n0 + tn + 8 * j;
+                if (gm < M && gn < N) C[(size_t)gm * ldc + gn] = acc[i][j].x + acc[i][j].y + (bias ? bias[gn] : 0.f);
+            }
+        }
+        return;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                                  // the stages are free: they take the partial tile
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) smem[(tm + 4 * i) * BN + tn + 8 * j] = acc[i][j].x + acc[i][j].y;
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(smem);
+    for (int e = rank * 128 + tid; e < BM * BN / 4; e += ranges * 128) {
+        const int gm = m0 + e / (BN / 4), gn = n0 + e % (BN / 4) * 4;
+        if (gm >= M || gn >= N) continue;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int r = 0; r < ranges; ++r) {
+            uint32_t remote;
+            float p[4];
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(mine + e * 16), "r"(r));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3]) : "r"(remote) : "memory");
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[c] += p[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (gn + c < N) C[(size_t)gm * ldc + gn + c] = v[c] + (bias ? bias[gn + c] : 0.f);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // (no CTA leaves while its tile is read)
+}
+
+int launch_tiles(const float* A, const float* W, const float* bias, float* C, int B, int M, int N, int K, int lda, int ldw, int ldc,
+                 long long batch_a, long long batch_w, long long batch_c, cudaStream_t s) {
+    const long long tiles = (long long)B * ceil_div(M, BM) * ceil_div(N, BN), slots = 2LL * num_sms();
+    // K ranges per tile: the fewest waves of two CTAs per SM times a wave's length, a range's fixed cost taken as 64 values of K
+    // (filling the stages) and 48 more for adding the partial tiles.  [300, 2048] x [2304, 2048]: 90 tiles alone leave half
+    // of the SMs' places empty.
+    int ranges = 1;
+    long long best = -1;
+    for (int r = 1; r <= MAX_RANGES; ++r) {
+        const int len = ceil_div(ceil_div(K, r), BK) * BK;
+        if (r > 1 && (len < 128 || ceil_div(K, len) != r)) continue;
+        const long long cost = (tiles * r + slots - 1) / slots * (len + 64 + (r > 1 ? 48 : 0));
+        if (best < 0 || cost < best) { best = cost; ranges = r; }
+    }
+    const int range_len = ceil_div(ceil_div(K, ranges), BK) * BK;
+    const dim3 grid(ceil_div(N, BN) * ranges, ceil_div(M, BM), B);
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && batch_a % 4 == 0 && batch_w % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    // (an ordinary launch, as the tile kernel always was: it reads its operands from the first instruction on)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(128); cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranges; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = ranges > 1 ? 1 : 0;
+    const cudaError_t e = vec ? cudaLaunchKernelEx(&cfg, gemm_f32_kernel<true>, A, W, bias, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, ranges, range_len)
+                              : cudaLaunchKernelEx(&cfg, gemm_f32_kernel<false>, A, W, bias, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, ranges, range_len);
+    if (e != cudaSuccess) TTIE_FAIL("gemm_f32: launch failed: %s", cudaGetErrorString(e));
+    return 0;
+}
+
 // ---- up to 16 activation rows.  acc[m][r]: lane-partial dot product of activation row m with weight row r of the warp's
 // four; the lanes' partial sums are added by shuffles in a fixed order.  Rows of 4-element-aligned length and stride only.
 constexpr int GV_WARPS = 8, GV_ROWS = 4;
@@ -140,11 +237,8 @@ extern "C" int ttie_gemm_f32(const float* A, const float* W, const float* bias, 
         }
         return 0;
     }
-    dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
-    if (grid.y > 65535) TTIE_FAIL("gemm_f32: M=%d too large for one launch", M);
-    gemm_f32_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, 0, 0, 0);
-    TTIE_CHECK_LAUNCH("gemm_f32");
-    return 0;
+    if (ceil_div(M, BM) > 65535) TTIE_FAIL("gemm_f32: M=%d too large for one launch", M);
+    return launch_tiles(A, W, bias, C, 1, M, N, K, lda, ldw, ldc, 0, 0, 0, (cudaStream_t)stream);
 }
 
 // A batch of products of one shape: C[b] = A[b] * W[b]^T, the operands of batch b at b * batch_a / batch_w / batch_c elements
@@ -154,9 +248,6 @@ extern "C" int ttie_gemm_f32_batched(const float* A, const float* W, float* C, i
                                      void* stream) {
     if (B <= 0 || M <= 0 || N <= 0) return 0;
     if (K <= 0) TTIE_FAIL("gemm_f32_batched: K must be positive, got %d", K);
-    dim3 grid(ceil_div(N, BN), ceil_div(M, BM), B);
-    if (grid.y > 65535 || B > 65535) TTIE_FAIL("gemm_f32_batched: M=%d, B=%d too large for one launch", M, B);
-    gemm_f32_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(A, W, nullptr, C, M, N, K, (int)lda, (int)ldw, (int)ldc, batch_a, batch_w, batch_c);
-    TTIE_CHECK_LAUNCH("gemm_f32_batched");
-    return 0;
+    if (ceil_div(M, BM) > 65535 || B > 65535) TTIE_FAIL("gemm_f32_batched: M=%d, B=%d too large for one launch", M, B);
+    return launch_tiles(A, W, nullptr, C, B, M, N, K, (int)lda, (int)ldw, (int)ldc, batch_a, batch_w, batch_c, (cudaStream_t)stream);
 }
