@@ -1,0 +1,184 @@
+"""The matrix-state recurrences over prompts in chunks of 64 tokens on tensor cores, against the token-by-token recurrence in 64 bits, and
+against the walk that decoded tokens run."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture()
+def ops():
+    from tiny_transformer_inference_engine_b200.ops import get_ops
+    o = get_ops(DEV)
+    keep = o.scan_chunk_tokens, o.scan_chunk_bytes
+    yield o
+    o.scan_chunk_tokens, o.scan_chunk_bytes = keep
+
+
+def step_tensors(lens):
+    qsl = [0]
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    slots = [(2 * i + 1) % (len(lens) + 1) for i in range(len(lens))] if len(lens) % 2 == 0 else list(range(len(lens)))[::-1]
+    return torch.tensor(qsl, dtype=torch.int32, device=DEV), torch.tensor(slots, dtype=torch.int32, device=DEV), qsl, slots
+
+
+class Scan:
+    """One kind of recurrence on random inputs: run(ops) -> (out, state tensors), exact() the same in 64 bits."""
+
+    def __init__(self, kind, lens, H, D, Dv, seed=0, strong=False, values=torch.bfloat16):
+        self.kind, self.lens, self.H, self.D, self.Dv = kind, lens, H, D, Dv
+        g = torch.Generator(device=DEV)
+        g.manual_seed(seed)
+        T, R = sum(lens), len(lens) + 2
+        rn = lambda *s: torch.randn(s, generator=g, device=DEV)
+        self.qsl, self.slots, self.q_at, self.s_at = step_tensors(lens)
+        P = 4
+        while P < D:
+            P *= 2
+        self.S0 = torch.zeros(R, H, Dv, P, device=DEV)
+        self.S0[..., :D] = rn(R, H, Dv, D) * 0.5
+        if kind == "retention":
+            self.qk = rn(T, 2 * H * D) * torch.cat([torch.ones(H * D), torch.full((H * D,), D ** -0.5)]).to(DEV)
+            self.q, self.k = self.qk[:, :H * D], self.qk[:, H * D:]
+            self.v = rn(T, H * Dv).to(values)
+            base = [1.0, 0.0, 0.5, -0.7] if strong else [1 - 2.0 ** (-5 - i % 4) for i in range(H)]
+            self.decay = torch.tensor([base[i % len(base)] for i in range(H)], device=DEV)
+        elif kind == "mlstm":
+            proj = rn(T, 2 * H * D + H * Dv).bfloat16()
+            self.q, self.k, self.v = proj[:, :H * D], proj[:, H * D:2 * H * D], proj[:, 2 * H * D:]
+            self.pre = rn(T, 2 * H) * (15.0 if strong else 1.5) + torch.cat([torch.zeros(H), torch.linspace(1, 6, H)]).to(DEV)
+            self.n0, self.m0 = torch.zeros(R, H, P, device=DEV), rn(R, H)
+            self.n0[..., :D] = rn(R, H, D)
+        else:
+            proj = rn(3, T, H * D).bfloat16()
+            self.q, self.k, self.v = proj
+            self.w = torch.exp(-torch.exp(torch.rand(T, H * D, generator=g, device=DEV) * (13.0 if strong else 6.5) - (8.0 if strong else 6.0)))
+            self.u, self.x, self.prev0 = rn(H * D) * 0.5, rn(T, 40).bfloat16(), rn(R, 40)
+
+    def run(self, ops):
+        H, D, Dv, N = self.H, self.D, self.Dv, len(self.lens)
+        S = self.S0.clone()
+        if self.kind == "retention":
+            return ops.retention_scan(self.q, self.k, self.v, self.decay, S, self.qsl, self.slots, N, H, D, Dv), [S]
+        if self.kind == "mlstm":
+            n, m = self.n0.clone(), self.m0.clone()
+            if ops.mlstm_in_chunks(self.q, self.k, self.v, N, D, Dv):
+                return ops.mlstm_chunks(self.q, self.k, self.v, self.pre, S, n, m, self.qsl, self.slots, N, H, D, Dv, 15.0, D ** -0.5), [S, n, m]
+            w, before = ops.mlstm_gates(self.pre, m, n, self.qsl, self.slots, N, H, 15.0)
+            return ops.mlstm_scan(self.q, self.k, self.v, w, S, n, before, self.qsl, self.slots, N, H, D, Dv, D ** -0.5), [S, n, m]
+        prev = self.prev0.clone()
+        return ops.wkv_scan(self.q, self.k, self.v, self.w, self.u, S, self.x, prev, self.qsl, self.slots, N, H, D), [S, prev]
+
+    def exact(self):
+        H, D, Dv = self.H, self.D, self.Dv
+        heads = lambda x, d: x.double().reshape(x.shape[0], H, d)
+        q, k, v = heads(self.q, D), heads(self.k, D), heads(self.v, Dv)
+        out, S_all = torch.empty(q.shape[0], H, Dv, dtype=torch.float64, device=DEV), self.S0.double()
+        n_all = m_all = None
+        self.near = torch.zeros(q.shape[0], H, dtype=torch.bool, device=DEV)   # rows that divide by a sum that nearly cancels
+        if self.kind == "mlstm":
+            n_all, m_all = self.n0.double(), self.m0.double()
+            ig = 15.0 * torch.tanh(self.pre[:, :H].double() / 15.0)
+            fg = torch.nn.functional.logsigmoid(15.0 * torch.tanh(self.pre[:, H:].double() / 15.0))
+        for r, slot in enumerate(self.s_at):
+            S = S_all[slot, :, :, :D]
+            for t in range(self.q_at[r], self.q_at[r + 1]):
+                kv = v[t][:, :, None] * k[t][:, None, :]
+                if self.kind == "retention":
+                    S = S * self.decay.double()[:, None, None] + kv
+                    out[t] = (S @ q[t][:, :, None])[..., 0]
+                elif self.kind == "wkv":
+                    out[t] = ((S + heads(self.u[None], D)[0][:, None, :] * kv) @ q[t][:, :, None])[..., 0]
+                    S = S * heads(self.w[t:t + 1], D)[0][:, None, :] + kv
+                else:
+                    n, m = n_all[slot, :, :D], m_all[slot]
+                    m1 = torch.maximum(fg[t] + m, ig[t])
+                    a, b = torch.exp(fg[t] + m - m1)[:, None], torch.exp(ig[t] - m1)[:, None]
+                    S, n = a[..., None] * S + b[..., None] * kv, a * n + b * k[t]
+                    qs = q[t] * D ** -0.5
+                    den = torch.maximum((n * qs).sum(-1).abs(), torch.exp(-m1)) + 1e-6
+                    self.near[t] = den < 0.02 * n.norm(dim=-1) * qs.norm(dim=-1)
+                    out[t] = (S @ qs[:, :, None])[..., 0] / den[:, None]
+                    n_all[slot, :, :D], m_all[slot] = n, m1
+            S_all[slot, :, :, :D] = S
+        return out.flatten(1), [S_all] + ([n_all, m_all] if self.kind == "mlstm" else [])
+
+
+def rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+KINDS = ["retention", "mlstm", "wkv"]
+SIZES = [([64], 2, 64, 64), ([65, 1], 3, 128, 128), ([63, 1, 130], 2, 48, 72), ([300], 4, 8, 8), ([1, 200, 2, 17], 1, 128, 136), ([129, 127], 2, 24, 16),
+         ([1000], 4, 64, 128)]
+
+
+@pytest.mark.parametrize("strong", [False, True])
+@pytest.mark.parametrize("lens,H,D,Dv", SIZES)
+@pytest.mark.parametrize("kind", KINDS)
+def test_chunks_against_64_bits(ops, kind, lens, H, D, Dv, strong):
+    """Whole and partial chunks, one and several requests, heads that do not fill a tile, decays from none to ones that leave nothing
+    (negative and zero ones too).  The bound: a read-out adds up some hundreds of products whose factors carry a few
+    roundings each, 2^-24 apart.  The matrix memory divides by a sum that can nearly cancel, which multiplies the error of that row:
+    rows whose divisor is below 2 % of what it could be are left out, the others' error may be fifty times as large."""
+    if kind == "wkv":
+        Dv = D
+    sc = Scan(kind, lens, H, D, Dv, seed=len(lens) + D, strong=strong)
+    ops.scan_chunk_tokens = 1
+    out, states = sc.run(ops)
+    exp, exp_states = sc.exact()
+    bound = 2e-5 if kind == "mlstm" else 1e-6
+    rows = lambda x: x.double().view(-1, H, Dv)[~sc.near]
+    assert sc.near.float().mean() < 0.25
+    assert rel(rows(out), rows(exp)) < bound
+    for s, e in zip(states, exp_states):
+        assert rel(s, e) < 1e-6
+    ops.scan_chunk_tokens = 1 << 30
+    walk, walk_states = sc.run(ops)
+    assert rel(rows(walk), rows(exp)) < bound
+    if kind == "wkv":
+        assert torch.equal(states[1], walk_states[1])                 # the request's last input
+    print(kind, lens, D, Dv, strong, "out %.3g %.3g" % (rel(rows(out), rows(exp)), rel(rows(walk), rows(exp))),
+          "states", ["%.3g" % rel(s, e) for s, e in zip(states, exp_states)], ["%.3g" % rel(s, e) for s, e in zip(walk_states, exp_states)])
+
+
+def test_retention_chunks_with_32_bit_values(ops):
+    sc = Scan("retention", [200, 70], 2, 128, 128, seed=9, values=torch.float32)
+    ops.scan_chunk_tokens = 1
+    out, (S,) = sc.run(ops)
+    exp, (e,) = sc.exact()
+    assert rel(out, exp) < 1e-6 and rel(S, e) < 1e-6
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_chunks_in_passes(ops, kind):
+    """A step whose states between chunks do not fit the workspace runs in passes that carry the state rows on: the same bits."""
+    sc = Scan(kind, [500, 3, 260], 2, 64, 64, seed=4)
+    ops.scan_chunk_tokens = 1
+    out, states = sc.run(ops)
+    ops.scan_chunk_bytes = 3 * 2 * 64 * 64 * 4
+    out2, states2 = sc.run(ops)
+    assert torch.equal(out, out2) and all(torch.equal(a, b) for a, b in zip(states, states2))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("what", ["v", "k"])
+def test_what_is_not_finite_stays_behind(ops, kind, what):
+    """A value or key that is not finite reaches its own and later tokens of its request; earlier tokens and other requests are as if
+    it were not there."""
+    lens, at = [150, 40], 75
+    for bad in (float("inf"), float("nan")):
+        sc, clean = Scan(kind, lens, 2, 64, 64, seed=5), Scan(kind, lens, 2, 64, 64, seed=5)
+        getattr(sc, what)[at, 70] = bad
+        ops.scan_chunk_tokens = 1
+        out, states = sc.run(ops)
+        ref, _ = clean.run(ops)
+        # (the 16 rows around a value that is not finite are summed token by token: other roundings)
+        assert torch.allclose(out[:at], ref[:at], rtol=1e-5, atol=1e-5) and torch.equal(out[150:], ref[150:])
+        assert not torch.isfinite(out[at + 1:150, 64:]).all()
+        ops.scan_chunk_tokens = 1 << 30
+        walk, walk_states = sc.run(ops)
+        assert torch.equal(torch.isfinite(out), torch.isfinite(walk))
+        assert torch.equal(torch.isfinite(states[0]), torch.isfinite(walk_states[0]))

@@ -1,0 +1,818 @@
+// The matrix-state recurrences of matrix_memory.cu (retention, the xLSTM matrix memory, the RWKV-style time mix) over prompts, in
+// chunks of 64 tokens instead of token by token.
+//
+// A token-by-token walk has no parallelism but the state's elements and waits for its own chain: one prompt of 2,048 tokens and 16
+// heads of 128 x 128 took 514 us at 3 TFLOP/s.  Over a chunk the same sums are four small matrix products, and only the state
+// between chunks is a chain.  Three launches:
+//
+//   chunk_sum     per (chunk, head): the chunk's own contribution to the state at its end, sum_j (decay from j to the end) v_j k_j^T
+//   chunk_carry   per state element: walks the request's chunks; leaves the state BEFORE each chunk where the chunk's own sum lay
+//                 and the request's new state in its state row
+//   chunk_out     per (chunk, head): o_i = (decay to i) S q_i + sum_(j <= i) (decay from j to i) (q_i . k_j) v_j
+//
+// Everything stays 32-bit as in the walk.  The products run on the tensor cores as bfloat16 instructions on operands split into
+// planes: a 32-bit value is the exact sum of three bfloat16 (8 + 8 + 8 bits), so a product of two of them is the six plane products
+// that matter at 32 bits, in 32-bit sums; a bfloat16 operand is one plane.  Decays are never divided by: every factor is a product of
+// decays over a span of tokens, or the exponential of a difference that cannot be positive, so nothing overflows however strong a
+// decay is.
+//
+//   retention   the decay is a constant: powers from a table evaluated in 64 bits.
+//   mlstm       with F_i the sum of the log forget gates up to i within the chunk, x_j = i_j - F_j and M_i = max(m before the
+//               chunk, max_(j<=i) x_j), the running maximum is m_i = F_i + M_i and the weight of token j in row i is
+//               exp(x_j - M_i) <= 1.  F, x and M are 64-bit: they grow with the chunk while their differences stay small.
+//   wkv         the decay is per key channel, so it sits inside the product over channels.  A chunk is four blocks of 16 tokens: between
+//               blocks a row is multiplied by the decays from its block's start to itself and a key by those from itself to
+//               its block's end, whole blocks between them as a vector on the rows; inside a block the 136 scores are summed on the
+//               ordinary cores with running products.
+//
+// A row of keys or values that is not finite reaches only its own and later tokens, as in the walk (masked weights are selected, not
+// multiplied, and the one place where a zero weight would meet a later value - a row's own block of 16 - is summed token
+// by token when a value there is not finite).
+//
+// Chunks are numbered over the whole step: request s owns the numbers from qsl[s] / 64 + s on, which leaves room for its last
+// partial chunk and needs nothing of the host but the number of tokens and requests.
+//
+// One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 28 + 9 + 62 against the walk's 514; 16 of 64 x 128
+// (mlstm) 13 + 9 + 44 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 39 + 16 + 87 against 473.  What bounds the out kernel is
+// latency: 8 to 12 warps per SM (registers and the planes in shared memory), issue slots 27 % used, the tensor pipe 37 / 15 / 12 %.
+// Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
+// 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 4.6e-8 (4.4e-8).
+#include "common.cuh"
+#include "run_reduce.cuh"
+#include <math.h>
+#include <type_traits>
+using namespace ttie;
+
+namespace {
+constexpr int CT = 64;                       // tokens per chunk
+constexpr int VT_COLS = 64, VLD = VT_COLS + 8;  // value columns per pass; row pitch of the staged values
+constexpr int CARRY = 128;                   // threads of a carry block
+enum Mode { RET = 0, MLSTM = 1, WKV = 2 };
+
+struct ChunkArgs {
+    const void* q; const void* k; long long ld_qk;                    // [T, H*D]; float32 (retention) or bfloat16
+    const void* v; long long ld_v;                                    // [T, H*Dv], bfloat16 or (retention) float32
+    const float* pre; long long ld_pre; float cap;                    // mlstm: gate pre-activations [T, 2H]
+    const float* decay;                                               // retention [H]; wkv [T, H*D]
+    const float* u;                                                   // wkv [H*D]
+    float* S; float* nrm; float* mx; int state_rows;                  // state rows (mlstm: normaliser and running maximum too)
+    const void* x; long long ld_x; int d; float* prev; int prev_rows; // wkv: the mixer's input and the rows that keep its last token
+    const int* qsl; const int* slot_ids; int num_seqs;
+    float* out;                                                       // [T, H*Dv]
+    int H, D, Dv, Dpad; float qscale;
+    int slot_lo, slots;                                               // the chunk numbers of this pass
+    float* part;                                                      // [slots, H, Dv, Dpad]
+    float* aux;                                                       // mlstm: [slots, H, Dpad] normaliser sums; wkv: [slots, H, 2, Dpad] chunk decays and what rounding them left
+    double2* span;                                                    // mlstm: [slots, H] (F at the end, max of x)
+    float2* mm;                                                       // mlstm: [slots, H] the running maximum before and behind the chunk
+};
+
+__device__ __forceinline__ int state_row(int slot, int num_rows) { return slot < 0 ? num_rows - 1 : slot; }
+
+// chunk number -> request, chunk of the request, first token (of the step's rows) and number of tokens; false: the number is not in use
+__device__ __forceinline__ bool find_chunk(const int* qsl, int num_seqs, int number, int& s, int& c, int& t0, int& n) {
+    int lo = 0, hi = num_seqs - 1;
+    while (lo < hi) {                                                 // the last request whose first number is <= number
+        const int mid = (lo + hi + 1) >> 1;
+        if ((qsl[mid] >> 6) + mid <= number) lo = mid; else hi = mid - 1;
+    }
+    s = lo;
+    c = number - (qsl[s] >> 6) - s;
+    const int len = qsl[s + 1] - qsl[s];
+    t0 = qsl[s] + c * CT;
+    n = min(CT, len - c * CT);
+    return c >= 0 && n > 0;
+}
+
+// ---- planes
+// a pair of values as three pairs of bfloat16 whose sum it is
+__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    auto pack = [](float a, float b) { const __nv_bfloat162 t = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&t); };
+    p0 = pack(x, y);
+    const float rx = x - __uint_as_float(p0 << 16), ry = y - __uint_as_float(p0 & 0xffff0000u);
+    p1 = pack(rx, ry);
+    p2 = pack(rx - __uint_as_float(p1 << 16), ry - __uint_as_float(p1 & 0xffff0000u));
+}
+// one value known in 64 bits (its third plane keeps what rounding it to 32 would cut)
+__device__ __forceinline__ void split3(double x, uint16_t& p0, uint16_t& p1, uint16_t& p2) {
+    const float hi = (float)x, lo = (float)(x - (double)hi);
+    const __nv_bfloat16 a = __float2bfloat16_rn(hi);
+    const float r = hi - __bfloat162float(a);
+    const __nv_bfloat16 b = __float2bfloat16_rn(r);
+    p0 = __bfloat16_as_ushort(a); p1 = __bfloat16_as_ushort(b); p2 = __bfloat16_as_ushort(__float2bfloat16_rn((r - __bfloat162float(b)) + lo));
+}
+__device__ __forceinline__ float2 unpack(uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); }
+
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two neighbouring 8-column tiles: the plane products of weight 2^-16 and up of 16 terms.  The tensor cores cut the bits below a sum's
+// last instead of rounding them (accumulating everything in one place left seven times the walk's error), so the 16 products of the
+// leading planes - 16 bits each, their sum all but exact - and the smaller ones are summed apart, each from zero, and
+// added to the running sum by ordinary additions.
+template <int NA, int NB>
+__device__ __forceinline__ void mma_planes(float (&c0)[4], float (&c1)[4], const uint32_t (&a)[NA][4], const uint32_t (&b)[NB][4]) {
+    float h0[4] = {0.f, 0.f, 0.f, 0.f}, h1[4] = {0.f, 0.f, 0.f, 0.f};
+    mma(h0, a[0], b[0][0], b[0][1]);
+    mma(h1, a[0], b[0][2], b[0][3]);
+    if constexpr (NA + NB > 2) {
+        float l0[4] = {0.f, 0.f, 0.f, 0.f}, l1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int sum = 2; sum >= 1; --sum)
+#pragma unroll
+            for (int i = 0; i < NA; ++i) {
+                const int j = sum - i;
+                if (j >= 0 && j < NB) {
+                    mma(l0, a[i], b[j][0], b[j][1]);
+                    mma(l1, a[i], b[j][2], b[j][3]);
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { h0[i] += l0[i]; h1[i] += l1[i]; }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { c0[i] += h0[i]; c1[i] += h1[i]; }
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], const uint16_t* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    if (TRANS) asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+    else asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+// B operand of 16 columns (two tiles) by 16 k: stored with a row per column (k along the row) ...
+__device__ __forceinline__ const uint16_t* at_cols(const uint16_t* base, int ld, int n0, int k0, int lane) {
+    return base + (n0 + (lane & 7) + (lane >> 4) * 8) * ld + k0 + ((lane >> 3) & 1) * 8;
+}
+// ... or with a row per k (columns along the row; loaded transposed)
+__device__ __forceinline__ const uint16_t* at_rows(const uint16_t* base, int ld, int n0, int k0, int lane) {
+    return base + (k0 + (lane & 7) + ((lane >> 3) & 1) * 8) * ld + n0 + (lane >> 4) * 8;
+}
+// A operand of 16 rows by 16 k, stored with a row per k (loaded transposed)
+__device__ __forceinline__ const uint16_t* at_rows_a(const uint16_t* base, int ld, int m0, int k0, int lane) {
+    return base + (k0 + (lane & 7) + (lane >> 4) * 8) * ld + m0 + ((lane >> 3) & 1) * 8;
+}
+
+// eight consecutive values of a row as floats (zeros where `in` is false)
+__device__ __forceinline__ void load8(const float* p, bool in, float (&o)[8]) {
+    const float4 a = in ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 b = in ? *reinterpret_cast<const float4*>(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, bool in, float (&o)[8]) {
+    const uint4 a = in ? *reinterpret_cast<const uint4*>(p) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 f = unpack(w[i]); o[2 * i] = f.x; o[2 * i + 1] = f.y; }
+}
+// eight values into PL planes at element offset `at`, planes `step` elements apart (PL 1: the values are bfloat16 already)
+template <int PL>
+__device__ __forceinline__ void store_planes(uint16_t* base, int step, int at, const float (&x)[8]) {
+    uint32_t p[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split3(x[2 * i], x[2 * i + 1], p[0][i], p[1][i], p[2][i]);
+#pragma unroll
+    for (int l = 0; l < PL; ++l) *reinterpret_cast<uint4*>(base + l * step + at) = make_uint4(p[l][0], p[l][1], p[l][2], p[l][3]);
+}
+
+// 64 rows of COLS values into PL planes: row j's columns from src + j * ld, zero where in(j, column) is false, behind scale(j, values).  The
+// loads of four pieces are on their way before the first is split.
+template <int PL, int COLS, int LDS, typename E, typename In, typename Scale>
+__device__ __forceinline__ void stage_rows(uint16_t* dst, const E* src, long long ld, In in, Scale scale) {
+    constexpr int PIECES = COLS / 8, ITERS = CT * PIECES / 128, BATCH = 4;
+    static_assert(ITERS % BATCH == 0, "64 rows of a multiple of 64 values over 128 threads");
+#pragma unroll
+    for (int i0 = 0; i0 < ITERS; i0 += BATCH) {
+        float x[BATCH][8];
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int e = (i0 + i) * 128 + threadIdx.x, j = e / PIECES, c = (e % PIECES) * 8;
+            load8(src + (size_t)j * ld + c, in(j, c), x[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int e = (i0 + i) * 128 + threadIdx.x, j = e / PIECES, c = (e % PIECES) * 8;
+            scale(j, x[i]);
+            store_planes<PL>(dst, CT * LDS, j * LDS + c, x[i]);
+        }
+    }
+}
+
+// rows t0 .. t0 + n - 1, columns col0 .. col0 + 63 of a head's values; `bad`: per 16 tokens, whether a value is not finite
+template <typename VT, int VPL>
+__device__ __forceinline__ void stage_values(uint16_t* v_s, const VT* vp, long long ld, int n, int col0, int Dv, int* bad) {
+    stage_rows<VPL, VT_COLS, VLD>(v_s, vp + col0, ld, [&](int j, int c) { return j < n && col0 + c < Dv; }, [&](int j, const float (&x)[8]) {
+        if (bad == nullptr) return;
+        bool fine = true;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fine = fine && isfinite(x[i]);
+        if (!fine) bad[j >> 4] = 1;
+    });
+}
+
+// ---- the matrix memory's gates over a chunk: threads 0 .. 63 (two warps), thread = token.  F: inclusive sum of the log forget gates,
+// x = i - F, X: inclusive maximum of x.  Tokens behind the chunk's n-th: F stays, x = -inf.  `half` holds four doubles in shared memory.
+__device__ __forceinline__ void chunk_gates(const ChunkArgs& a, int t0, int n, int h, double* half, double& F, double& x, double& X) {
+    const int j = threadIdx.x, lane = j & 31;
+    double f = 0.0, ig = -INFINITY;
+    x = X = 0.0;
+    if (j < n) {
+        const float* g = a.pre + (size_t)(t0 + j) * a.ld_pre;
+        ig = (double)(a.cap * tanhf(g[h] / a.cap));
+        const float z = a.cap * tanhf(g[a.H + h] / a.cap);
+        f = (double)(fminf(z, 0.f) - log1pf(expf(-fabsf(z))));
+    }
+    F = f;
+    if (j < CT) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const double y = __shfl_up_sync(0xffffffffu, F, o); if (lane >= o) F += y; }
+        if (j == 31) half[0] = F;
+    }
+    __syncthreads();
+    if (j < CT) {
+        if (j >= 32) F += half[0];
+        x = ig - F;
+        X = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const double y = __shfl_up_sync(0xffffffffu, X, o); if (lane >= o) X = fmax(X, y); }
+        if (j == 31) half[1] = X;
+    }
+    __syncthreads();
+    if (j >= 32 && j < CT) X = fmax(X, half[1]);
+    if (j == CT - 1) { half[2] = F; half[3] = X; }
+    __syncthreads();
+}
+
+// ------------------------------------------------------------------------------------------- chunk_sum
+template <int MODE, int KP> struct SumSmem {
+    static constexpr int LD = KP + 8;
+    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + (MODE == WKV ? KP * 8 : CT * 4); }
+};
+
+template <int MODE, int KP, typename VT>
+__global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
+    constexpr int LD = KP + 8, VPL = sizeof(VT) == 4 ? 3 : 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint16_t* kd = reinterpret_cast<uint16_t*>(smem_raw);                             // [3][CT][LD]: decayed keys
+    uint16_t* v_s = kd + 3 * CT * LD;                                                 // [VPL][CT][VLD]
+    double* half = reinterpret_cast<double*>(v_s + VPL * CT * VLD);                   // [8]
+    float* wt = reinterpret_cast<float*>(half + 8);                                   // [CT]: a token's weight at the chunk's end
+    TTIE_PDL_ENTRY();
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int s, c, t0, n;
+    if (!find_chunk(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
+    const size_t unit = (size_t)blockIdx.x * a.H + h;
+    const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
+
+    if constexpr (MODE == WKV) {
+        // a thread per channel and run of LEN tokens: the decays of the run, its product, then keys times the decays behind them (products
+        // of up to 64 decays in 64 bits: in 32 they leave more than the walk's one rounding per token)
+        constexpr int LEN = CT * KP / 128, RUNS = CT / LEN;
+        double* tot = half;                                                           // [KP]: product over the last run (RUNS == 2; over wt, which is not used here)
+        const int ch = tid % KP, run = tid / KP;
+        const bool in = ch < a.D;
+        const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D + ch;
+        const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D + ch;
+        float w[LEN];
+        __nv_bfloat16 kv[LEN];
+#pragma unroll
+        for (int i = 0; i < LEN; ++i) {
+            const int j = run * LEN + i;
+            w[i] = in && j < n ? wp[(size_t)j * a.H * a.D] : 1.f;
+            kv[i] = in && j < n ? kp[(size_t)j * a.ld_qk] : __float2bfloat16(0.f);
+        }
+        stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
+        double all = 1.0;
+#pragma unroll
+        for (int i = LEN - 1; i >= 0; --i) all *= (double)w[i];
+        if (RUNS == 2 && run == 1) tot[ch] = all;
+        __syncthreads();
+        double suf = RUNS == 2 && run == 0 ? tot[ch] : 1.0;
+        if (run == 0 && ch < a.Dpad) {
+            const double f = in ? all * suf : 1.0;
+            a.aux[2 * unit * a.Dpad + ch] = (float)f;
+            a.aux[(2 * unit + 1) * a.Dpad + ch] = (float)(f - (double)(float)f);
+        }
+#pragma unroll
+        for (int i = LEN - 1; i >= 0; --i) {
+            const int j = run * LEN + i;
+            split3((double)to_f32(kv[i]) * suf, kd[j * LD + ch], kd[CT * LD + j * LD + ch], kd[2 * CT * LD + j * LD + ch]);
+            suf *= (double)w[i];
+        }
+    } else {
+        stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
+        if constexpr (MODE == RET) {
+            if (tid < CT) wt[tid] = tid < n ? (float)pow((double)a.decay[h], (double)(n - 1 - tid)) : 0.f;
+        } else {
+            double F, x, X;
+            chunk_gates(a, t0, n, h, half, F, x, X);
+            if (tid < CT) wt[tid] = expf((float)(x - half[3]));
+            if (tid == 0) a.span[unit] = make_double2(half[2], half[3]);
+        }
+        __syncthreads();
+        using KT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
+        const KT* kp = reinterpret_cast<const KT*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
+        stage_rows<3, KP, LD>(kd, kp, a.ld_qk, [&](int j, int ch) { return j < n && ch < a.D; }, [&](int j, float (&x)[8]) {
+            const float w = wt[j];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = j < n ? x[i] * w : 0.f;
+        });
+    }
+    __syncthreads();
+    if (MODE == MLSTM && tid < a.Dpad) {                                              // the normaliser's sum: the same without the values
+        float sum = 0.f;
+        for (int j = 0; j < CT; ++j)
+            sum += __uint_as_float((uint32_t)kd[j * LD + tid] << 16) + (__uint_as_float((uint32_t)kd[CT * LD + j * LD + tid] << 16) + __uint_as_float((uint32_t)kd[2 * CT * LD + j * LD + tid] << 16));
+        a.aux[unit * a.Dpad + tid] = sum;
+    }
+    const int g = lane >> 2, t = lane & 3;
+    for (int col0 = 0; col0 < a.Dv; col0 += VT_COLS) {
+        if (col0 > 0) {
+            __syncthreads();
+            stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv, nullptr);
+            __syncthreads();
+        }
+        float acc[KP / 8][4];
+#pragma unroll
+        for (int i = 0; i < KP / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll
+        for (int k0 = 0; k0 < CT; k0 += 16) {
+            uint32_t av[VPL][4];
+#pragma unroll
+            for (int l = 0; l < VPL; ++l) ldsm<true>(av[l], at_rows_a(v_s + l * CT * VLD, VLD, warp * 16, k0, lane));
+#pragma unroll
+            for (int np = 0; np < KP / 16; ++np) {
+                uint32_t b[3][4];
+#pragma unroll
+                for (int l = 0; l < 3; ++l) ldsm<true>(b[l], at_rows(kd + l * CT * LD, LD, np * 16, k0, lane));
+                mma_planes<VPL, 3>(acc[2 * np], acc[2 * np + 1], av, b);
+            }
+        }
+        float* dst = a.part + (unit * a.Dv + col0 + warp * 16) * a.Dpad;
+#pragma unroll
+        for (int i = 0; i < KP / 8; ++i) {
+            const int ch = i * 8 + 2 * t;
+            if (ch < a.Dpad) {
+                if (col0 + warp * 16 + g < a.Dv) *reinterpret_cast<float2*>(dst + (size_t)g * a.Dpad + ch) = make_float2(acc[i][0], acc[i][1]);
+                if (col0 + warp * 16 + g + 8 < a.Dv) *reinterpret_cast<float2*>(dst + (size_t)(g + 8) * a.Dpad + ch) = make_float2(acc[i][2], acc[i][3]);
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------- chunk_carry
+// A thread per four elements of a (request, head)'s state; the request's chunks of this pass one after the other, the next chunks'
+// sums on their way meanwhile.  mlstm: the elements behind the state are the normaliser's.
+template <int MODE>
+__global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
+    __shared__ float powers[2];
+    TTIE_PDL_ENTRY();
+    const int h = blockIdx.y, s = blockIdx.z;
+    const int q0 = a.qsl[s], len = a.qsl[s + 1] - q0;
+    const int base = (q0 >> 6) + s;
+    const int c_lo = max(0, a.slot_lo - base), c_hi = min((len + CT - 1) / CT, a.slot_lo + a.slots - base);
+    if (c_lo >= c_hi) return;
+    if (MODE == RET) {
+        const int last = len - (c_hi - 1) * CT;
+        if (threadIdx.x < 2) powers[threadIdx.x] = (float)pow((double)a.decay[h], (double)(threadIdx.x == 0 ? CT : min(CT, last)));
+        __syncthreads();
+    }
+    const size_t row = state_row(a.slot_ids[s], a.state_rows);
+    if (MODE == WKV && h == 0 && blockIdx.x == 0 && c_hi == (len + CT - 1) / CT) {     // the request's last input is the next step's previous token
+        const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(a.x) + (size_t)(q0 + len - 1) * a.ld_x;
+        float* p = a.prev + (size_t)state_row(a.slot_ids[s], a.prev_rows) * a.d;
+        for (int i = threadIdx.x; i < a.d; i += blockDim.x) p[i] = to_f32(x[i]);
+    }
+    const int state = a.Dv * a.Dpad;
+    const int e = (blockIdx.x * CARRY + threadIdx.x) * 4;
+    if (e >= state + (MODE == MLSTM ? a.Dpad : 0)) return;
+    const bool in_state = e < state;                                                  // (only mlstm has elements behind it)
+    float* sp = in_state ? a.S + (row * a.H + h) * state + e : a.nrm + (row * a.H + h) * a.Dpad + (e - state);
+    float* pp = in_state ? a.part + e : a.aux + (e - state);
+    const size_t step = (size_t)a.H * (in_state ? state : a.Dpad);
+    const size_t unit = (size_t)(base + c_lo - a.slot_lo) * a.H + h;                  // of chunk c_lo
+    pp += (in_state ? state : a.Dpad) * unit;
+    float4 S = *reinterpret_cast<const float4*>(sp);
+    // the running maximum as the request's state row has it; every CTA reads the row here, so the new one is written by chunk_out
+    double m = MODE == MLSTM ? (double)a.mx[row * a.H + h] : 0.0;
+    // two batches of chunks in registers: the next one's sums are on their way while this one is worked off
+    constexpr int AHEAD = MODE == RET ? 8 : 4;
+    float4 p[2][AHEAD], w[2][MODE == WKV ? AHEAD : 1], wl[2][MODE == WKV ? AHEAD : 1];
+    double2 sc[2][MODE == MLSTM ? AHEAD : 1];
+    auto fetch = [&](int b, int c0) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            if (c0 + i >= c_hi) continue;
+            const size_t off = (size_t)(c0 + i - c_lo);
+            p[b][i] = *reinterpret_cast<const float4*>(pp + off * step);
+            if constexpr (MODE == WKV) {
+                const float* f = a.aux + 2 * (unit + off * a.H) * a.Dpad + e % a.Dpad;
+                w[b][i] = *reinterpret_cast<const float4*>(f);
+                wl[b][i] = *reinterpret_cast<const float4*>(f + a.Dpad);
+            }
+            if constexpr (MODE == MLSTM) sc[b][i] = a.span[unit + off * a.H];
+        }
+    };
+    auto work = [&](int b, int c0) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            if (c0 + i >= c_hi) continue;
+            const size_t off = (size_t)(c0 + i - c_lo);
+            *reinterpret_cast<float4*>(pp + off * step) = S;
+            float4 f, x = p[b][i];
+            if constexpr (MODE == RET) {
+                const float d = powers[c0 + i == c_hi - 1 ? 1 : 0];
+                f = make_float4(d, d, d, d);
+            } else if constexpr (MODE == WKV) {
+                f = w[b][i];
+                const float4 l = wl[b][i];
+                x = make_float4(fmaf(l.x, S.x, x.x), fmaf(l.y, S.y, x.y), fmaf(l.z, S.z, x.z), fmaf(l.w, S.w, x.w));
+            } else {
+                const double next = (double)(float)(sc[b][i].x + fmax(m, sc[b][i].y));      // as the state row will hold it
+                const float d = expf((float)(sc[b][i].x + m - next)), own = expf((float)(sc[b][i].x + sc[b][i].y - next));
+                f = make_float4(d, d, d, d);
+                x = make_float4(x.x * own, x.y * own, x.z * own, x.w * own);
+                if (e == 0) a.mm[unit + off * a.H] = make_float2((float)m, (float)next);
+                m = next;
+            }
+            S.x = fmaf(f.x, S.x, x.x); S.y = fmaf(f.y, S.y, x.y); S.z = fmaf(f.z, S.z, x.z); S.w = fmaf(f.w, S.w, x.w);
+        }
+    };
+    fetch(0, c_lo);
+    for (int c0 = c_lo; c0 < c_hi; c0 += 2 * AHEAD) {
+        fetch(1, c0 + AHEAD);
+        work(0, c0);
+        fetch(0, c0 + 2 * AHEAD);
+        work(1, c0 + AHEAD);
+    }
+    *reinterpret_cast<float4*>(sp) = S;
+}
+
+// ------------------------------------------------------------------------------------------- chunk_out
+template <int MODE, int KP> struct OutSmem {
+    static constexpr int LD = KP + 8, FLD = KP + 4;
+    static constexpr int EXTRA = MODE == WKV ? (2 * CT * FLD + 4 * KP + 4 * 16 * 17) * 4 : MODE == MLSTM ? CT * 24 + KP * 4 : (CT + 1 + 3) * 4;
+    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 16 + 64 + EXTRA; }
+};
+
+template <int MODE, int KP, typename VT>
+__global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
+    constexpr int LD = KP + 8, FLD = KP + 4, VPL = sizeof(VT) == 4 ? 3 : 1;
+    constexpr int QPL = MODE == MLSTM ? 1 : 3, KPL = MODE == MLSTM ? 1 : 3, KS = KP / 16;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint16_t* pl = reinterpret_cast<uint16_t*>(smem_raw);                             // [3][CT][LD]: keys, then 64 columns of the state
+    uint16_t* v_s = pl + 3 * CT * LD;                                                 // [VPL][CT][VLD]
+    int* bad = reinterpret_cast<int*>(v_s + VPL * CT * VLD);                          // [4]
+    double* half = reinterpret_cast<double*>(bad + 4);                                // [8]
+    unsigned char* extra = reinterpret_cast<unsigned char*>(half + 8);
+    TTIE_PDL_ENTRY();
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    int s, c, t0, n;
+    if (!find_chunk(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
+    const size_t unit = (size_t)blockIdx.x * a.H + h;
+    using QT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
+    const QT* qp = reinterpret_cast<const QT*>(a.q) + (size_t)t0 * a.ld_qk + h * a.D;
+    const QT* kp = reinterpret_cast<const QT*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
+    const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
+    const int r0 = warp * 16 + g, r1 = r0 + 8;                                        // this lane's rows (tokens of the chunk)
+    if (tid < 4) bad[tid] = 0;
+    __syncthreads();
+    stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv, bad);
+
+    // a lane's part of a 16 x 16 piece of the query rows: rows r0 / r1, channels c0 + 2t, + 1 and those + 8
+    auto load_q = [&](int c0, float (&f)[8]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = i & 1 ? r1 : r0, ch = c0 + 2 * t + (i & 2 ? 8 : 0);
+            const bool in = r < n && ch < a.D;
+            if constexpr (MODE == RET) {
+                const float2 x = in ? *reinterpret_cast<const float2*>(qp + (size_t)r * a.ld_qk + ch) : make_float2(0.f, 0.f);
+                f[2 * i] = x.x; f[2 * i + 1] = x.y;
+            } else {
+                const float2 x = unpack(in ? *reinterpret_cast<const uint32_t*>(qp + (size_t)r * a.ld_qk + ch) : 0u);
+                f[2 * i] = x.x; f[2 * i + 1] = x.y;
+            }
+        }
+    };
+    auto planes_of = [&](const float (&f)[8], uint32_t (&q)[QPL][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t p0, p1, p2;
+            split3(f[2 * i], f[2 * i + 1], p0, p1, p2);
+            q[0][i] = p0;
+            if constexpr (QPL == 3) { q[1][i] = p1; q[2][i] = p2; }
+        }
+    };
+
+    float P[8][4];                                                                    // scores, then weights: rows r0, r0, r1, r1; columns 8 i + 2t, + 1
+#pragma unroll
+    for (int i = 0; i < 8; ++i) P[i][0] = P[i][1] = P[i][2] = P[i][3] = 0.f;
+    float rq[MODE == WKV ? KS : 1][8];                                                // wkv: the rows with their decays from the chunk's start
+    float row_in[2], den[2] = {0.f, 0.f}, floor_[2] = {0.f, 0.f};                     // factor of the state before the chunk; mlstm: denominator, e^-m
+
+    if constexpr (MODE == WKV) {
+        float* ws = reinterpret_cast<float*>(extra);                                  // [CT][FLD] decays
+        float* pre = ws + CT * FLD;                                                   // [CT][FLD] product of the block's decays before the token
+        float* blk = pre + CT * FLD;                                                  // [4][KP] product over a block
+        float* diag = blk + 4 * KP;                                                   // [4][16][17] scores inside a block
+        for (int e = tid; e < 4 * KP; e += 128) {
+            const int J = e / KP, ch = e % KP;
+            const bool in = ch < a.D;
+            const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D + ch;
+            float w[16], k[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int j = J * 16 + i;
+                w[i] = in && j < n ? wp[(size_t)j * a.H * a.D] : 1.f;
+                k[i] = in && j < n ? to_f32(kp[(size_t)j * a.ld_qk + ch]) : 0.f;
+            }
+            double f = 1.0;                                                           // (in 64 bits, as in chunk_sum)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) { ws[(J * 16 + i) * FLD + ch] = w[i]; pre[(J * 16 + i) * FLD + ch] = (float)f; f *= (double)w[i]; }
+            blk[J * KP + ch] = (float)f;
+            f = 1.0;
+#pragma unroll
+            for (int i = 15; i >= 0; --i) {
+                const int at = (J * 16 + i) * LD + ch;
+                split3((double)k[i] * f, pl[at], pl[CT * LD + at], pl[2 * CT * LD + at]);
+                f *= (double)w[i];
+            }
+        }
+        __syncthreads();
+        // inside the block: lanes own channels, running products from every key on; 16 sums over the lanes at a time
+        float* dg = diag + warp * 16 * 17;
+        for (int ch0 = 0; ch0 < KP; ch0 += 64) {
+            float r[16][2], ub[2];
+            bool in[2];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                in[m] = ch0 + lane + 32 * m < a.D;
+                ub[m] = in[m] ? a.u[h * a.D + ch0 + lane + 32 * m] : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+                    r[i][m] = in[m] && warp * 16 + i < n ? to_f32(qp[(size_t)(warp * 16 + i) * a.ld_qk + ch0 + lane + 32 * m]) : 0.f;
+            const float* w = ws + warp * 16 * FLD + ch0 + lane;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                float p[2], sum[16];
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+                    p[m] = in[m] && warp * 16 + j < n ? to_f32(kp[(size_t)(warp * 16 + j) * a.ld_qk + ch0 + lane + 32 * m]) : 0.f;
+#pragma unroll
+                for (int i = 0; i < j; ++i) sum[i] = 0.f;
+                sum[j] = fmaf(r[j][1], ub[1] * p[1], r[j][0] * (ub[0] * p[0]));
+#pragma unroll
+                for (int i = j + 1; i < 16; ++i) {
+                    sum[i] = fmaf(r[i][1], p[1], r[i][0] * p[0]);
+                    p[0] *= w[i * FLD]; p[1] *= w[i * FLD + 32];
+                }
+                int first = 0;
+                RunReduce<16, 16>::run(sum, lane, first);
+                if ((lane & 1) == 0) {
+                    float* o = dg + first * 17 + j;
+                    *o = ch0 == 0 ? sum[0] : *o + sum[0];
+                }
+            }
+        }
+        __syncwarp();
+        // between blocks: rows times the decays from their block's start, then times whole blocks going back
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+            load_q(ks * 16, rq[ks]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = (i >> 1) & 1 ? r1 : r0, ch = ks * 16 + 2 * t + (i & 4 ? 8 : 0) + (i & 1);
+                rq[ks][i] *= pre[r * FLD + ch];
+            }
+        }
+#pragma unroll
+        for (int J = 2; J >= 0; --J) {
+            if (J >= warp) continue;
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks) {
+                uint32_t q[QPL][4], b[3][4];
+                planes_of(rq[ks], q);
+#pragma unroll
+                for (int l = 0; l < 3; ++l) ldsm<false>(b[l], at_cols(pl + l * CT * LD, LD, J * 16, ks * 16, lane));
+                mma_planes<3, 3>(P[2 * J], P[2 * J + 1], q, b);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) rq[ks][i] *= blk[J * KP + ks * 16 + 2 * t + (i & 4 ? 8 : 0) + (i & 1)];
+            }
+        }
+#pragma unroll
+        for (int J = 0; J < 4; ++J)
+            if (J == warp)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const int r = g + (b & 2 ? 8 : 0), col = i * 8 + 2 * t + (b & 1);
+                        P[2 * J + i][b] = col <= r ? dg[r * 17 + col] : 0.f;
+                    }
+        row_in[0] = row_in[1] = 1.f;
+    } else {
+        stage_rows<KPL, KP, LD>(pl, kp, a.ld_qk, [&](int j, int ch) { return j < n && ch < a.D; }, [](int, float (&)[8]) {});
+        float* pw = reinterpret_cast<float*>(extra);                                  // retention: powers 0 .. CT of the decay
+        double* xs = reinterpret_cast<double*>(extra);                                // mlstm: x, M and F of every token; the normaliser before the chunk
+        double* Ms = xs + CT;
+        double* Fs = Ms + CT;
+        float* nb = reinterpret_cast<float*>(Fs + CT);
+        if constexpr (MODE == RET) {
+            if (tid <= CT) pw[tid] = (float)pow((double)a.decay[h], (double)tid);
+            __syncthreads();
+        } else {
+            double F, x, X;
+            chunk_gates(a, t0, n, h, half, F, x, X);
+            const float2 mm = a.mm[unit];
+            const double m = (double)mm.x;
+            if (tid < CT) { xs[tid] = x; Ms[tid] = fmax(m, X); Fs[tid] = F; }
+            if (tid < KP) nb[tid] = tid < a.Dpad ? a.aux[unit * a.Dpad + tid] : 0.f;
+            // (a chunk is the request's last of this pass if the next chunk is not there or not in the pass)
+            if (tid == 0 && ((c + 1) * CT >= a.qsl[s + 1] - a.qsl[s] || (int)blockIdx.x + 1 == a.slots))
+                a.mx[(size_t)state_row(a.slot_ids[s], a.state_rows) * a.H + h] = mm.y;
+            __syncthreads();
+            row_in[0] = expf((float)(m - Ms[r0])); row_in[1] = expf((float)(m - Ms[r1]));
+            floor_[0] = expf((float)-(Fs[r0] + Ms[r0])); floor_[1] = expf((float)-(Fs[r1] + Ms[r1]));
+        }
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+            float f[8];
+            uint32_t q[QPL][4];
+            load_q(ks * 16, f);
+            planes_of(f, q);
+            if constexpr (MODE == MLSTM) {                                            // q . n before the chunk
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float x = f[i] * nb[ks * 16 + 2 * t + (i & 4 ? 8 : 0) + (i & 1)];
+                    if ((i >> 1) & 1) den[1] += x; else den[0] += x;
+                }
+            }
+#pragma unroll
+            for (int J = 0; J < 4; ++J) {
+                if (J > warp) continue;                                               // keys behind all of the warp's rows
+                uint32_t b[KPL][4];
+#pragma unroll
+                for (int l = 0; l < KPL; ++l) ldsm<false>(b[l], at_cols(pl + l * CT * LD, LD, J * 16, ks * 16, lane));
+                mma_planes<QPL, KPL>(P[2 * J], P[2 * J + 1], q, b);
+            }
+        }
+        if constexpr (MODE == RET) {
+            row_in[0] = pw[r0 + 1]; row_in[1] = pw[r1 + 1];
+        } else {
+            den[0] *= row_in[0]; den[1] *= row_in[1];
+        }
+        const double M0 = MODE == MLSTM ? Ms[r0] : 0.0, M1 = MODE == MLSTM ? Ms[r1] : 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int r = b & 2 ? r1 : r0, j = i * 8 + 2 * t + (b & 1);
+                float w = 0.f;
+                if (j <= r) {
+                    if constexpr (MODE == RET) w = P[i][b] * pw[r - j];
+                    else { w = P[i][b] * expf((float)(xs[j] - (b & 2 ? M1 : M0))); den[b >> 1] += w; }
+                }
+                P[i][b] = w;
+            }
+        if constexpr (MODE == MLSTM) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                den[b] += __shfl_xor_sync(0xffffffffu, den[b], 1);
+                den[b] += __shfl_xor_sync(0xffffffffu, den[b], 2);
+                den[b] = fmaxf(fabsf(den[b] * a.qscale), floor_[b]) + 1e-6f;
+            }
+        }
+    }
+
+    for (int col0 = 0; col0 < a.Dv; col0 += VT_COLS) {
+        __syncthreads();                                                              // the keys (or the last columns) have been read by everyone
+        if (col0 > 0) {
+            if (tid < 4) bad[tid] = 0;
+            __syncthreads();
+            stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv, bad);
+        }
+        const float* sp = a.part + (unit * a.Dv + col0) * a.Dpad;
+        stage_rows<3, KP, LD>(pl, sp, a.Dpad, [&](int j, int ch) { return col0 + j < a.Dv && ch < a.Dpad; }, [](int, float (&)[8]) {});
+        __syncthreads();
+        float acc[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+            uint32_t q[QPL][4];
+            if constexpr (MODE == WKV) planes_of(rq[ks], q);
+            else { float f[8]; load_q(ks * 16, f); planes_of(f, q); }
+#pragma unroll
+            for (int np = 0; np < 4; ++np) {
+                uint32_t b[3][4];
+#pragma unroll
+                for (int l = 0; l < 3; ++l) ldsm<false>(b[l], at_cols(pl + l * CT * LD, LD, np * 16, ks * 16, lane));
+                mma_planes<QPL, 3>(acc[2 * np], acc[2 * np + 1], q, b);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            acc[i][0] *= row_in[0]; acc[i][1] *= row_in[0]; acc[i][2] *= row_in[1]; acc[i][3] *= row_in[1];
+        }
+#pragma unroll
+        for (int J = 0; J < 4; ++J) {
+            if (J > warp) continue;
+            if (J == warp && bad[J]) {                                                // a value of the rows' own block is not finite: token by token
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float p0 = __shfl_sync(0xffffffffu, P[2 * J + (j >> 3)][j & 1], (lane & 28) + ((j & 7) >> 1));
+                    const float p1 = __shfl_sync(0xffffffffu, P[2 * J + (j >> 3)][2 + (j & 1)], (lane & 28) + ((j & 7) >> 1));
+                    if (J * 16 + j >= n) continue;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            const int col = col0 + i * 8 + 2 * t + b;
+                            if (col >= a.Dv) continue;
+                            const float x = to_f32(vp[(size_t)(J * 16 + j) * a.ld_v + col]);
+                            if (j <= g) acc[i][b] = fmaf(p0, x, acc[i][b]);
+                            if (j <= g + 8) acc[i][2 + b] = fmaf(p1, x, acc[i][2 + b]);
+                        }
+                }
+                continue;
+            }
+            uint32_t p[3][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) split3(P[2 * J + (i >> 1)][(i & 1) * 2], P[2 * J + (i >> 1)][(i & 1) * 2 + 1], p[0][i], p[1][i], p[2][i]);
+#pragma unroll
+            for (int np = 0; np < 4; ++np) {
+                uint32_t b[VPL][4];
+#pragma unroll
+                for (int l = 0; l < VPL; ++l) ldsm<true>(b[l], at_rows(v_s + l * CT * VLD, VLD, np * 16, J * 16, lane));
+                mma_planes<3, VPL>(acc[2 * np], acc[2 * np + 1], p, b);
+            }
+        }
+        const size_t ld_o = (size_t)a.H * a.Dv;
+        float* op = a.out + (size_t)t0 * ld_o + h * a.Dv + col0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int col = i * 8 + 2 * t;
+            if (col0 + col >= a.Dv) continue;
+            float y[4] = {acc[i][0], acc[i][1], acc[i][2], acc[i][3]};
+            if constexpr (MODE == MLSTM) {
+                y[0] = y[0] * a.qscale / den[0]; y[1] = y[1] * a.qscale / den[0]; y[2] = y[2] * a.qscale / den[1]; y[3] = y[3] * a.qscale / den[1];
+            }
+            if (r0 < n) *reinterpret_cast<float2*>(op + (size_t)r0 * ld_o + col) = make_float2(y[0], y[1]);
+            if (r1 < n) *reinterpret_cast<float2*>(op + (size_t)r1 * ld_o + col) = make_float2(y[2], y[3]);
+        }
+    }
+}
+
+template <int MODE, int KP, typename VT>
+int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
+    constexpr int VPL = sizeof(VT) == 4 ? 3 : 1;
+    const size_t sum_smem = SumSmem<MODE, KP>::bytes(VPL), out_smem = OutSmem<MODE, KP>::bytes(VPL);
+    cudaFuncSetAttribute(chunk_sum_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
+    cudaFuncSetAttribute(chunk_out_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+    a.slot_lo = first; a.slots = slots;
+    const dim3 grid(slots, a.H);
+    const dim3 carry(ceil_div(a.Dv * a.Dpad + (MODE == MLSTM ? a.Dpad : 0), 4 * CARRY), a.H, a.num_seqs);
+    TTIE_LAUNCH((chunk_sum_kernel<MODE, KP, VT>), grid, 128, sum_smem, st, a);
+    TTIE_LAUNCH((chunk_carry_kernel<MODE>), carry, CARRY, 0, st, a);
+    TTIE_LAUNCH((chunk_out_kernel<MODE, KP, VT>), grid, 128, out_smem, st, a);
+    TTIE_CHECK_LAUNCH("matrix_chunks");
+    return 0;
+}
+}  // namespace
+
+// mode: 0 retention (q, k float32; v either type), 1 mlstm, 2 wkv (q, k, v bfloat16).  T: rows of the step.  D and Dv multiples of
+// 8, D at most 128, rows that start on 16 bytes.  part / aux / span / mm hold `slots` chunk numbers' worth; a step of more chunk
+// numbers (T / 64 + requests) is done in passes.
+extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, int v_dtype,
+                                  const float* pre, long long ld_pre, float cap, const float* decay, const float* u, float* S, float* nrm,
+                                  float* mx, int state_rows, const void* x, long long ld_x, int d, float* prev, int prev_rows, const int* qsl,
+                                  const int* slot_ids, int num_seqs, int T, float* out, int H, int D, int Dv, int Dpad, float qscale,
+                                  float* part, float* aux, void* span, void* mm, int slots, void* stream) {
+    if (num_seqs <= 0 || T <= 0) return 0;
+    if (mode < 0 || mode > 2 || (v_dtype != kBF16 && !(v_dtype == kF32 && mode == RET))) TTIE_FAIL("matrix_chunks: mode %d with values of type %d", mode, v_dtype);
+    const int ce = mode == RET ? 4 : 8, ve = v_dtype == kF32 ? 4 : 8;                 // values per 16 bytes
+    if (D < 8 || D > 128 || D % 8 || Dv < 8 || Dv % 8 || Dpad < D || Dpad > 128 || Dpad % 8 || ld_qk % ce || ld_v % ve || (mode == WKV && D != Dv)
+        || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)S | (uintptr_t)nrm | (uintptr_t)part | (uintptr_t)aux) & 15))
+        TTIE_FAIL("matrix_chunks: heads of %d key channels (padded %d) and %d value channels, strides %lld and %lld: multiples of 8, at most 128 key channels, rows on 16 bytes", D, Dpad, Dv, ld_qk, ld_v);
+    if (slots < 1 || H > 65535 || num_seqs > 65535) TTIE_FAIL("matrix_chunks: %d chunks a pass, %d heads, %d requests", slots, H, num_seqs);
+    ChunkArgs a = {};
+    a.q = q; a.k = k; a.ld_qk = ld_qk; a.v = v; a.ld_v = ld_v; a.pre = pre; a.ld_pre = ld_pre; a.cap = cap; a.decay = decay; a.u = u;
+    a.S = S; a.nrm = nrm; a.mx = mx; a.state_rows = state_rows; a.x = x; a.ld_x = ld_x; a.d = d; a.prev = prev; a.prev_rows = prev_rows;
+    a.qsl = qsl; a.slot_ids = slot_ids; a.num_seqs = num_seqs; a.out = out; a.H = H; a.D = D; a.Dv = Dv; a.Dpad = Dpad; a.qscale = qscale;
+    a.part = part; a.aux = aux; a.span = (double2*)span; a.mm = (float2*)mm;
+    const int total = T / CT + num_seqs;
+    cudaStream_t st = (cudaStream_t)stream;
+    for (int first = 0; first < total; first += slots) {
+        const int cnt = total - first < slots ? total - first : slots;
+        int rc;
+        if (mode == RET && v_dtype == kF32) rc = Dpad <= 64 ? launch_chunks<RET, 64, float>(a, first, cnt, st) : launch_chunks<RET, 128, float>(a, first, cnt, st);
+        else if (mode == RET) rc = Dpad <= 64 ? launch_chunks<RET, 64, __nv_bfloat16>(a, first, cnt, st) : launch_chunks<RET, 128, __nv_bfloat16>(a, first, cnt, st);
+        else if (mode == MLSTM) rc = Dpad <= 64 ? launch_chunks<MLSTM, 64, __nv_bfloat16>(a, first, cnt, st) : launch_chunks<MLSTM, 128, __nv_bfloat16>(a, first, cnt, st);
+        else rc = Dpad <= 64 ? launch_chunks<WKV, 64, __nv_bfloat16>(a, first, cnt, st) : launch_chunks<WKV, 128, __nv_bfloat16>(a, first, cnt, st);
+        if (rc) return rc;
+    }
+    return 0;
+}

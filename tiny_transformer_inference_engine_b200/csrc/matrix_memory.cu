@@ -26,6 +26,7 @@
 //   retention_scan    S <- decay_h S + k v^T, o = S^T q, with q and k 32-bit (already rotated and scaled)
 //   head_norm_gate    out = o / rms(o over the head) * weight * act(gate)   (act: silu or sigmoid; the weight is optional)
 #include "common.cuh"
+#include "run_reduce.cuh"
 #include <math.h>
 using namespace ttie;
 
@@ -156,32 +157,6 @@ __device__ __forceinline__ void lds_keys(const __nv_bfloat16* p, float* o) {
     }
 }
 
-// Sums over the SL adjacent lanes of a column of CNT values per lane at once (the partial read-outs of a run of tokens): at
-// every step a lane hands half of its values to the partner and adds the partner's other half to the half it keeps, so the
-// run costs CNT - 1 shuffles instead of CNT * log2(SL); once a lane is down to one value the remaining steps are plain
-// butterfly additions.  Afterwards a lane holds, in v[0 ..], the totals of the tokens base, base + 1, ... (max(1, CNT / SL) of them).
-template <int O, int CNT>
-struct RunReduce {
-    static __device__ __forceinline__ void run(float* v, int slice, int& base) {
-        if constexpr (O >= 1) {
-            if constexpr (CNT > 1) {
-                constexpr int HALF = CNT / 2;
-                const bool up = (slice & O) != 0;
-#pragma unroll
-                for (int i = 0; i < HALF; ++i) {
-                    const float send = up ? v[i] : v[i + HALF];
-                    const float keep = up ? v[i + HALF] : v[i];
-                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-                }
-                if (up) base += HALF;
-                RunReduce<O / 2, HALF>::run(v, slice, base);
-            } else {
-                v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
-                RunReduce<O / 2, 1>::run(v, slice, base);
-            }
-        }
-    }
-};
 // tokens a lane holds after RunReduce, and whether it is the one of several equal lanes that writes them
 template <int SL, int N> struct RunOwner {
     static constexpr int COUNT = N >= SL ? N / SL : 1;

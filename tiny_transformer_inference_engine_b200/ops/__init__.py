@@ -134,6 +134,9 @@ _SIGNATURES = {
     "ttie_rotate_heads": [_c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_int, _c_float, _c_void, _c_int, _c_void],
     "ttie_retention_scan": [_c_void, _c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int,
                             _c_int, _c_int, _c_int, _c_void, _c_int, _c_void],
+    "ttie_matrix_chunks": [_c_int, _c_void, _c_void, _c_ll, _c_void, _c_ll, _c_int, _c_void, _c_ll, _c_float, _c_void, _c_void, _c_void, _c_void,
+                           _c_void, _c_int, _c_void, _c_ll, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_int, _c_void, _c_int, _c_int,
+                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_void],
     "ttie_head_norm_gate": [_c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void, _c_int, _c_void],
     "ttie_activation": [_c_void, _c_void, _c_ll, _c_int, _c_float, _c_float, _c_int, _c_int, _c_void],
     "ttie_matrix_state_pad": [_c_int],
@@ -1321,6 +1324,9 @@ class CudaOps:
         out = torch.empty((T, num_heads * dim), dtype=torch.float32, device=r.device)
         if not (r.stride(0) == k.stride(0) == v.stride(0)):
             raise KernelError("wkv_scan: r, k and v must share a row stride")
+        if r.dtype == torch.bfloat16 and self._in_chunks(T, num_seqs, dim, dim, r, k, v):
+            self._matrix_chunks(2, r, k, v, None, 0.0, decay, u, state, None, None, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, dim, 1.0)
+            return out
         self._check(self.lib.ttie_wkv_scan(_ptr(r), _ptr(k), _ptr(v), r.stride(0), _ptr(decay), _ptr(u),
                                            _ptr(state), state.shape[0], _ptr(x), x.stride(0), x.shape[1], _ptr(prev), prev.shape[0],
                                            _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), _ptr(out), num_heads, dim,
@@ -1357,6 +1363,43 @@ class CudaOps:
         self.launches += 1
         return out
 
+    def mlstm_in_chunks(self, q, k, v, num_seqs, dim, v_dim):
+        """Whether ``mlstm_chunks`` takes this step (in place of ``mlstm_gates`` and ``mlstm_scan``)."""
+        return q.dtype == torch.bfloat16 and q.stride(0) == k.stride(0) == v.stride(0) and self._in_chunks(q.shape[0], num_seqs, dim, v_dim, q, k, v)
+
+    def mlstm_chunks(self, q, k, v, pre, S, n, m, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, cap, q_scale):
+        """The matrix memory over a step with a prompt portion, in chunks of 64 tokens: ``mlstm_gates`` and ``mlstm_scan`` in one.  ``pre``:
+        the gates' pre-activations float32 [T, 2H]; the state rows S, n and m are advanced in place.  Returns o float32 [T, H*v_dim]."""
+        out = torch.empty((q.shape[0], num_heads * v_dim), dtype=torch.float32, device=q.device)
+        self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale)
+        return out
+
+    scan_chunk_tokens = 48                  # tokens that one request of a step may bring from which the matrix-state scans run in chunks;
+    scan_chunk_bytes = 128 << 20            # bytes of the states between chunks that are held at a time (about the L2: a longer step runs in passes)
+
+    def _in_chunks(self, num_tokens, num_seqs, dim, v_dim, q, k, v) -> bool:
+        """Whether a step's matrix-state recurrence runs in chunks of 64 tokens on tensor cores (``csrc/matrix_chunks.cu``) rather than
+        token by token: a request may bring ``scan_chunk_tokens`` or more (the step's tokens less one for every other request: the
+        host knows no more, and the number holds for a captured graph), and the head sizes and rows are what 16-byte loads and
+        16-channel products take."""
+        return (num_tokens - (int(num_seqs) - 1) >= self.scan_chunk_tokens and 8 <= dim <= 128 and dim % 8 == 0 and v_dim % 8 == 0
+                and all(t.stride(1) == 1 and t.stride(0) * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
+
+    def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale):
+        T, pad, dev = q.shape[0], S.shape[-1], q.device
+        total = T // 64 + int(num_seqs)                                # chunk numbers of the step
+        slots = max(1, min(total, self.scan_chunk_bytes // (num_heads * v_dim * pad * 4)))
+        part = torch.empty((slots, num_heads, v_dim, pad), dtype=torch.float32, device=dev)
+        aux = torch.empty((slots, num_heads, mode, pad), dtype=torch.float32, device=dev) if mode else None
+        span = torch.empty((slots, num_heads, 2), dtype=torch.float64, device=dev) if mode == 1 else None
+        mm = torch.empty((slots, num_heads, 2), dtype=torch.float32, device=dev) if mode == 1 else None
+        self._check(self.lib.ttie_matrix_chunks(
+            mode, _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), self._dt(v), _ptr(pre), 0 if pre is None else pre.stride(0), float(cap),
+            _ptr(decay), _ptr(u), _ptr(S), _ptr(n), _ptr(m), S.shape[0], _ptr(x), 0 if x is None else x.stride(0), 0 if x is None else x.shape[1],
+            _ptr(prev), 0 if prev is None else prev.shape[0], _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), T, _ptr(out), num_heads, dim,
+            v_dim, pad, float(q_scale), _ptr(part), _ptr(aux), _ptr(span), _ptr(mm), slots, self._stream(q)), "matrix_chunks")
+        self.launches += 3 * math.ceil(total / slots)
+
     def rotate_heads(self, src, heads, dim, cs_table, rot, style, scale_from=None, scale=1.0):
         """float32 [T, heads * dim]: the ``heads`` head rows of ``dim`` values at the start of every row of ``src`` (a view with a
         row stride), the first ``rot`` values of each rotated at the token's position (``cs_table`` from ``rope_table``;
@@ -1374,13 +1417,17 @@ class CudaOps:
         place): S <- decay_h S + k v^T, o = S^T q.  q, k float32 [T, H*dim] views with one row stride; v [T, H*v_dim] in the
         compute dtype, a view with a row stride; ``decay`` float32 [H].  Returns o float32 [T, H*v_dim].
 
-        A step that may hold a long prompt (the step's tokens less one for every other request: the host knows no more, and
-        the number holds for a captured graph) is walked in ``parts`` (``retention_parts``) by two launches: the decay is a
+        A step that may hold a prompt portion runs in chunks of 64 tokens (``_in_chunks``).  Head sizes that those do not take are walked
+        token by token, and a long prompt (the step's tokens less one for every other request: the host knows no more, and
+        the number holds for a captured graph) in ``parts`` (``retention_parts``) by two launches: the decay is a
         constant, so every part's own sum needs no other part and the parts' first states follow from those sums."""
         T = q.shape[0]
         out = torch.empty((T, num_heads * v_dim), dtype=torch.float32, device=q.device)
         if q.stride(0) != k.stride(0) or q.dtype != torch.float32 or k.dtype != torch.float32:
             raise KernelError("retention_scan: q and k must be float32 and share a row stride")
+        if self._in_chunks(T, num_seqs, dim, v_dim, q, k, v):
+            self._matrix_chunks(0, q, k, v, None, 0.0, decay, None, S, None, None, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, 1.0)
+            return out
         parts = self.retention_parts(T, int(num_seqs), S[0].numel())
         scratch = torch.empty((int(num_seqs) * parts,) + tuple(S.shape[1:]), dtype=torch.float32, device=q.device) if parts > 1 else None
         self._check(self.lib.ttie_retention_scan(_ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(decay), _ptr(S), S.shape[0],

@@ -74,8 +74,12 @@ class MLSTM(Mixer):
         proj = ops.linear(x, self.w_in, None)                                                  # [T, q | k | v | g]
         gates = ops.linear(x, self.w_gates, self.b_gates, out_dtype=torch.float32)             # [T, 2H] float32
         q, k, v, g = proj[:, :H * D], proj[:, H * D:2 * H * D], proj[:, 2 * H * D:2 * H * D + H * Dv], proj[:, 2 * H * D + H * Dv:]
-        weights, n_before = ops.mlstm_gates(gates, mx.state, nrm.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, self.gate_cap)
-        o = ops.mlstm_scan(q, k, v, weights, S.state, nrm.state, n_before, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs,
-                           H, D, Dv, D ** -0.5)
+        if hasattr(ops, "mlstm_chunks") and ops.mlstm_in_chunks(q, k, v, ctx.num_seqs, D, Dv):
+            o = ops.mlstm_chunks(q, k, v, gates, S.state, nrm.state, mx.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, Dv,
+                                 self.gate_cap, D ** -0.5)
+        else:
+            weights, n_before = ops.mlstm_gates(gates, mx.state, nrm.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, self.gate_cap)
+            o = ops.mlstm_scan(q, k, v, weights, S.state, nrm.state, n_before, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs,
+                               H, D, Dv, D ** -0.5)
         y = ops.head_norm_gate(o, g, self.norm_w, H, Dv, self.eps, "sigmoid")
         return ops.linear(y, self.w_out, None, partial_ok=True)
