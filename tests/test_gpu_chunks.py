@@ -11,9 +11,10 @@ DEV = "cuda:0"
 def ops():
     from tiny_transformer_inference_engine_b200.ops import get_ops
     o = get_ops(DEV)
-    keep = o.scan_chunk_tokens, o.scan_chunk_bytes
+    keep = o.scan_chunk_tokens, o.scan_chunk_more, o.scan_chunk_bytes
+    o.scan_chunk_more = 0
     yield o
-    o.scan_chunk_tokens, o.scan_chunk_bytes = keep
+    o.scan_chunk_tokens, o.scan_chunk_more, o.scan_chunk_bytes = keep
 
 
 def step_tensors(lens):

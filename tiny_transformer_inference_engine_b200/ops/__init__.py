@@ -1374,15 +1374,20 @@ class CudaOps:
         self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale)
         return out
 
-    scan_chunk_tokens = 48                  # tokens that one request of a step may bring from which the matrix-state scans run in chunks;
+    scan_chunk_tokens = 160                 # tokens that one request of a step may bring from which the matrix-state scans run in chunks,
+    scan_chunk_more = 12                    # and how many more for every other request;
     scan_chunk_bytes = 128 << 20            # bytes of the states between chunks that are held at a time (about the L2: a longer step runs in passes)
 
     def _in_chunks(self, num_tokens, num_seqs, dim, v_dim, q, k, v) -> bool:
         """Whether a step's matrix-state recurrence runs in chunks of 64 tokens on tensor cores (``csrc/matrix_chunks.cu``) rather than
-        token by token: a request may bring ``scan_chunk_tokens`` or more (the step's tokens less one for every other request: the
+        token by token: a request may bring enough tokens (the step's tokens less one for every other request: the
         host knows no more, and the number holds for a captured graph), and the head sizes and rows are what 16-byte loads and
-        16-channel products take."""
-        return (num_tokens - (int(num_seqs) - 1) >= self.scan_chunk_tokens and 8 <= dim <= 128 and dim % 8 == 0 and v_dim % 8 == 0
+        16-channel products take.  Measured at width 2,048: the walk takes 0.17 to 0.23 us a token of the longest request and 0.3 to 0.9 us a
+        request, chunks 32 to 36 us (mlstm 25) and 1.4 to 2.9 us for every further request, so they meet at 160 tokens (mlstm 120) of a
+        lone request and some 10 tokens later for each further one (one request of 128 tokens: retention 41.8 us in chunks, 30.5
+        walked; beside 7 decoding requests 58.6 and 40.5; of 2,048 tokens 100 and 514)."""
+        others = int(num_seqs) - 1
+        return (num_tokens - others >= self.scan_chunk_tokens + self.scan_chunk_more * others and 8 <= dim <= 128 and dim % 8 == 0 and v_dim % 8 == 0
                 and all(t.stride(1) == 1 and t.stride(0) * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
 
     def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale):
