@@ -1,0 +1,64 @@
+"""The row kernels of prompt portions (wide loads, several values per thread) against 64 bits, at sizes they take and sizes they leave to
+the general forms."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tiny_transformer_inference_engine_b200.ops import get_ops
+    return get_ops(DEV)
+
+
+def randn(seed, *shape):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    return torch.randn(shape, generator=g, device=DEV)
+
+
+# one rounding to bfloat16 (2^-9 of the value) over a few 32-bit roundings
+BF16 = dict(rtol=2.0 ** -8, atol=1e-6)
+
+
+@pytest.mark.parametrize("T,H,Dv,weight,act", [(1, 1, 16, True, "silu"), (3, 3, 32, False, "sigmoid"), (67, 5, 64, True, "sigmoid"), (130, 2, 128, False, "silu"),
+                                               (9, 3, 20, True, "silu"), (5, 2, 256, True, "silu")])
+def test_head_norm_gate(ops, T, H, Dv, weight, act):
+    o, wide = randn(1, T, H * Dv) * 3, randn(2, T, H * Dv + 8).bfloat16()
+    gate = wide[:, 4:4 + H * Dv]
+    w = randn(3, H * Dv) if weight else None
+    got = ops.head_norm_gate(o, gate, w, H, Dv, 1e-6, act)
+    x = o.double().view(T, H, Dv)
+    x = (x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6)).flatten(1)
+    g = torch.sigmoid(gate.double()) * (gate.double() if act == "silu" else 1.0)
+    assert torch.allclose(got.double(), x * (w.double() if weight else 1.0) * g, **BF16)
+
+
+@pytest.mark.parametrize("style", [0, 1])
+@pytest.mark.parametrize("T,heads,D,rot", [(65, 1, 8, 8), (70, 3, 128, 128), (67, 4, 64, 32), (66, 2, 48, 8), (90, 3, 24, 0), (9, 2, 20, 12), (6, 2, 40, 20), (64, 2, 64, 64)])
+def test_rotate_heads(ops, T, heads, D, rot, style):
+    src = randn(4, T, heads * D + 8).bfloat16()
+    pos = torch.arange(T, dtype=torch.int32, device=DEV) * 37
+    inv = (1.0 / 10000.0 ** (torch.arange(0, max(rot, 2), 2, device=DEV).float() / max(rot, 2)))
+    cs = ops.rope_table(pos, inv) if rot else None
+    got = ops.rotate_heads(src, heads, D, cs, rot, style, scale_from=1, scale=0.125)
+    x = src[:, :heads * D].double().view(T, heads, D).clone()
+    if rot:
+        c, s = cs[..., 0].double()[:, None], cs[..., 1].double()[:, None]
+        a, b = (x[..., 0:rot:2], x[..., 1:rot:2]) if style == 0 else (x[..., :rot // 2], x[..., rot // 2:rot])
+        ra, rb = a * c - b * s, b * c + a * s
+        if style == 0:
+            x[..., 0:rot:2], x[..., 1:rot:2] = ra, rb
+        else:
+            x[..., :rot // 2], x[..., rot // 2:rot] = ra, rb
+    x[:, 1:] *= 0.125
+    assert torch.allclose(got.double().view(T, heads, D), x, rtol=1e-6, atol=1e-6)     # two products and a sum in 32 bits
+
+
+@pytest.mark.parametrize("T,HD", [(1, 4), (67, 64), (5, 130), (3, 7)])
+def test_wkv_decay(ops, T, HD):
+    wide, w0 = randn(5, T, HD + 4) * 2, randn(6, HD)
+    got = ops.wkv_decay(wide[:, :HD], w0)
+    assert torch.allclose(got.double(), torch.exp(-torch.exp(wide[:, :HD].double() + w0.double())), rtol=1e-5, atol=1e-7)
