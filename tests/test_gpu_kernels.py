@@ -466,6 +466,36 @@ def test_sampling_after_a_top_k_cut(ops, V, ctas):
     assert int((probs[4] > 0).sum()) > V // 5 and int((probs[5] > 0).sum()) > V // 3 - 1     # the equal values stayed together
 
 
+@pytest.mark.parametrize("V,ctas", [(515, 1), (32000, 1), (32000, 4), (32000, 8)])
+def test_sampling_at_the_edges_of_the_short_list(ops, V, ctas):
+    """Top-k up to a quarter of the row's warps takes its bound from the warps' maxima, the next larger one from a CTA's threads; a list of
+    320 tokens is cut by comparing all pairs, one of 321 by digits.  Plateaus of equal values put lists of both lengths there,
+    with the cut inside and above them."""
+    quarter = 32 * ctas // 4
+    g = torch.Generator().manual_seed(V + ctas)
+    rows, logits = [], []
+    for i, (top_k, plateau) in enumerate([(quarter, 0), (quarter + 1, 0), (1, 0), (quarter, 320), (quarter, 321), (2, 319), (quarter, 40), (quarter + 1, 320)]):
+        x = torch.randn(V, generator=g)
+        if plateau:
+            x = x.clamp(max=3.0)
+            x[torch.randperm(V, generator=g)[:plateau]] = 4.0
+            if i % 2:
+                x[torch.randperm(V, generator=g)[:max(1, top_k // 2)]] = 5.0
+        logits.append(x)
+        rows.append((31 + i, i, top_k, 0.9, 1.0 if i % 3 == 2 else 0.8, 0))
+    logits = torch.stack(logits)
+    out, probs = torch.empty(len(rows), dtype=torch.int32, device=DEV), torch.zeros(len(rows), V, device=DEV)
+    ops.sample(logits.to(DEV), torch.arange(len(rows), dtype=torch.int32).to(DEV), sampler_state(rows).to(DEV), out, probs_out=probs, ctas_per_row=ctas)
+    out, probs = out.cpu(), probs.cpu()
+    for r, (seed, draws, top_k, temp, top_p, _) in enumerate(rows):
+        exp = PLAIN.filtered_probs(logits[r], temp, top_k, top_p).float()
+        assert torch.equal(probs[r] > 0, exp > 0), f"row {r}: kept sets differ"
+        assert torch.allclose(probs[r], exp, atol=2e-6, rtol=1e-4)
+        u = uniform_from_state(seed & 0x7fffffff, seed >> 31, draws)
+        cdf, tok = torch.cumsum(probs[r].double(), 0), int(out[r])
+        assert (cdf[tok - 1].item() if tok else 0.0) - 1e-5 <= u <= cdf[tok].item() + 1e-5
+
+
 @pytest.mark.parametrize("V,ctas", [(515, 1), (32000, 0), (32000, 1), (65024, 2), (256000, 0)])
 def test_sampling_with_top_p_alone(ops, V, ctas):
     """Top-p without a top-k: peaked rows, where the tokens of 1/1,024 of the mass or more reach past the cut and the

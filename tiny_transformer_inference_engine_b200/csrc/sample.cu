@@ -22,6 +22,7 @@ namespace {
 constexpr int THREADS = 1024;
 constexpr int LIST_TOP_K = 256;                                      // largest top-k for which the short list is tried
 constexpr int KEEP_CAP = 1024;                                       // tokens one CTA may hand in to the short list
+constexpr int SMALL_LIST = 320;                                      // tokens of a list whose cuts are found by comparing all pairs
 constexpr float LIST_TOP_P = 1024.f;                                 // top-p alone: the list takes tokens of 1 / 1024 of the row's mass or more
 typedef unsigned long long u64;
 
@@ -151,11 +152,14 @@ __device__ __forceinline__ void all_gather(T* buf, int n, T v, unsigned rank) {
 // for that (staged == 0) is read from global memory every time.  Maxima, histograms and sums of the slices are
 // exchanged through distributed shared memory; every CTA then takes the same decisions from the same integers.
 //
-// With a top-k of a few hundred at most the row is left after two walks.  Every thread knows the largest value among its
-// own tokens from the first walk; the k-th largest of a CTA's 1,024 such values is a bound that at least k tokens of the
-// slice reach, so nothing below it can be among the row's k largest.  The tokens at or above the bound (a few more than k
-// per CTA) are gathered in token order, handed to the first CTA of the cluster, and that CTA alone does the exact top-k
-// cut, top-p and the draw on the list (`list_cap` entries fit the shared memory that held its slice).  If the list would
+// With a top-k of a few hundred at most the row is left after two walks.  Every warp knows the largest value among its
+// own tokens from the first walk, and the exchange that finds the row's maximum brings all of them to every CTA: the k-th largest
+// of the row's 32 C such values is a bound that at least k tokens of the row reach, so nothing below it can be among the
+// k largest (8 CTAs, k 32: some 40 tokens are left; 8 rows of 32,000 tokens take 15.3 us, 29.1 when every CTA took the k-th largest of
+// its own threads' maxima by a radix select, which left 300).  Where k is more than a quarter of the warps, a CTA's bound is that radix select.
+// The tokens at or above the bound are gathered in token order, handed to the first CTA of the cluster, and that CTA alone does the exact top-k
+// cut, top-p and the draw on the list (`list_cap` entries fit the shared memory that held its slice).  A list of up to SMALL_LIST
+// tokens needs no radix select for that: every token counts the tokens and the mass above it, which decides both cuts at once.  If the list would
 // overflow (thousands of equal values at the bound), every CTA goes on with its whole slice instead.
 // Top-p without a top-k leaves the row the same way when the distribution is peaked: the (at most 1,024) tokens that hold
 // 1 / 1,024 of the row's mass or more each are listed, and if together they hold more than top_p of the mass the cut lies
@@ -171,12 +175,15 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     __shared__ u64 s_hist[256];
     __shared__ u64 x_hist[2][C * 256];                               // exchange buffers, by exchange parity
     __shared__ u64 x_u64[2][C];
-    __shared__ float x_val[C];
-    __shared__ int x_idx[C];
+    __shared__ u64 x_best[C * (THREADS / 32)];                        // every warp's maximum: place (high word) and value
     __shared__ int x_cnt[C];
     __shared__ float c_y[KEEP_CAP];                                   // this slice's tokens for the short list: value ...
     __shared__ int c_i[KEEP_CAP];                                     // ... and place in the slice
     __shared__ int s_scan[THREADS / 32];
+    // a short list's masses and keys: they lie where the slices' histograms are exchanged while there is no list
+    static_assert(SMALL_LIST * 12 <= 2 * 256 * 8 && 8 * (THREADS / 32) <= SMALL_LIST, "one CTA's exchange buffers hold a short list");
+    u64* l_mass = &x_hist[0][0];
+    unsigned* l_key = reinterpret_cast<unsigned*>(l_mass + SMALL_LIST);
     __shared__ unsigned s_prefix;
     __shared__ u64 s_acc;
     __shared__ int s_found;
@@ -227,29 +234,25 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
         const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
         if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
     }
-    if (lane == 0) { s_val[warp] = best; s_idx[warp] = best_i; }
+    if (lane == 0) { s_val[warp] = best; s_idx[warp] = best_i == 0x7fffffff ? 0x7fffffff : best_i + v0; }
     __syncthreads();
-    if (warp == 0) {
-        best = s_val[lane]; best_i = s_idx[lane];
+    // every warp's maximum to every CTA in one exchange; the row's is the largest of them (lower tokens win ties)
+    if (C > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    all_gather<C, u64>(x_best, THREADS / 32,
+                       tid < THREADS / 32 ? ((u64)(unsigned)s_idx[tid] << 32) | __float_as_uint(s_val[tid]) : 0, rank);
+    best = -INFINITY; best_i = 0x7fffffff;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-            if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
-        }
-        if (lane == 0) { s_val[0] = best; s_idx[0] = best_i == 0x7fffffff ? 0x7fffffff : best_i + v0; }
+    for (int k = 0; k < C; ++k) {
+        const u64 x = x_best[k * (THREADS / 32) + lane];
+        const float ov = __uint_as_float((unsigned)x);
+        const int oi = (int)(x >> 32);
+        if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
     }
-    __syncthreads();
-    if (C > 1) {                                                      // the slices' maxima, in rank order: lower tokens win ties
-        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-        all_gather<C, float>(x_val, 1, s_val[0], rank);
-        all_gather<C, int>(x_idx, 1, s_idx[0], rank);
-        best = -INFINITY; best_i = 0x7fffffff;
 #pragma unroll
-        for (int k = 0; k < C; ++k)
-            if (x_val[k] > best || (x_val[k] == best && x_idx[k] < best_i)) { best = x_val[k]; best_i = x_idx[k]; }
-    } else {
-        best = s_val[0]; best_i = s_idx[0];
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
+        if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
     }
     if (best_i == 0x7fffffff) best_i = 0;                            // a row of NaNs: report token 0
     if (greedy) {
@@ -299,7 +302,27 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     unsigned low_key = 0;                                             // the list takes every token at or above this key
     u64 z_row = 0, limit_row = 0;                                     // top-p alone: the row's whole mass and top_p of it
     bool have_z = false;
-    if (staged && list_cap > 0 && top_k > 0 && top_k < V && top_k <= LIST_TOP_K) {
+    constexpr int GROUPS = C * (THREADS / 32), PER_GROUP = THREADS / GROUPS;
+    if (staged && list_cap > 0 && top_k > 0 && top_k < V && 4 * top_k <= GROUPS) {
+        // (a) the bound: the top_k-th largest of the row's warps' maxima, PER_GROUP neighbouring lanes counting for each
+        const int g = tid / PER_GROUP;
+        if (tid < GROUPS) l_key[tid] = ordered_key(__uint_as_float((unsigned)x_best[tid]) / temperature);
+        __syncthreads();
+        const unsigned key = l_key[g];
+        int above = 0, same = 0;
+        for (int j = tid % PER_GROUP; j < GROUPS; j += PER_GROUP) {
+            const unsigned other = l_key[j];
+            above += other > key; same += other == key;
+        }
+#pragma unroll
+        for (int o = 1; o < PER_GROUP; o <<= 1) {
+            above += __shfl_xor_sync(0xffffffffu, above, o);
+            same += __shfl_xor_sync(0xffffffffu, same, o);
+        }
+        if (above < top_k && above + same >= top_k) s_prefix = key;   // (several write the same value)
+        __syncthreads();
+        low_key = s_prefix; try_list = true;
+    } else if (staged && list_cap > 0 && top_k > 0 && top_k < V && top_k <= LIST_TOP_K) {
         // (a) the bound: the top_k-th largest of the threads' own maxima (a radix select over one key per thread)
         const unsigned tkey = ordered_key(my_best / temperature);
         unsigned prefix = 0; u64 remaining = (u64)top_k;
@@ -402,12 +425,44 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
         }
     }
 
+    // A short list: the tokens and the mass above every token by comparing all pairs (neighbouring lanes share a token), which
+    // decides both cuts - a token is among the k largest iff fewer than k are larger, and stays under top-p iff the mass of the
+    // larger ones (which stay if it does) is at most top_p of the mass of the k largest.  Sums of integers: the order is nothing.
+    unsigned cut_key = 0;
+    const bool pairs = listed && n_cur <= SMALL_LIST;
+    if (pairs) {
+        int sh = 0;
+        while (sh < 5 && (n_cur << (sh + 1)) <= THREADS) ++sh;
+        for (int i = tid; i < n_cur; i += THREADS) { const float y = u_y[i]; l_key[i] = ordered_key(y); l_mass[i] = mass_of(y, ymax); }
+        if (tid == 0) s_prefix = 0xffffffffu;
+        __syncthreads();
+        const int i = tid >> sh, part = tid & ((1 << sh) - 1);
+        const unsigned key = i < n_cur ? l_key[i] : 0xffffffffu;
+        int above = 0;
+        u64 mass_above = 0;
+        if (i < n_cur)
+            for (int j = part; j < n_cur; j += 1 << sh)
+                if (l_key[j] > key) { ++above; mass_above += l_mass[j]; }
+        for (int o = 1; o < (1 << sh); o <<= 1) {
+            above += __shfl_xor_sync(0xffffffffu, above, o);
+            mass_above += __shfl_xor_sync(0xffffffffu, mass_above, o);
+        }
+        bool stays = i < n_cur && !(top_k > 0 && top_k < V && above >= top_k);
+        if (top_p < 1.0f) {
+            const u64 z = have_z ? z_row : block_sum_u64(stays && part == 0 ? l_mass[i] : 0, s_u64);
+            stays = stays && mass_above <= (u64)((double)top_p * (double)z);
+        }
+        if (stays && part == 0) atomicMin(&s_prefix, key);
+        __syncthreads();
+        cut_key = s_prefix;
+    }
+
     // The passes below visit every token of the slice several times.  A slice of up to 8 tokens per thread is kept in
     // registers as (key, probability mass) - the mass is computed once, not once per pass - ; a longer one is read from
     // shared (or global) memory and its masses recomputed on each visit.
     constexpr int EPT = 8;
     const int iters = (n_cur + THREADS - 1) / THREADS;             // visits per thread (the same for all: whole warps go round together)
-    const bool cached = iters <= EPT && (top_k > 0 || top_p < 1.0f);
+    const bool cached = !pairs && iters <= EPT && (top_k > 0 || top_p < 1.0f);
     unsigned ck[EPT];
     u64 cm[EPT];
 #pragma unroll
@@ -432,8 +487,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     };
 
     // 2. top-k threshold: the k-th largest key, by radix select over 4 digits of 8 bits
-    unsigned cut_key = 0;
-    if (top_k > 0 && top_k < V) {
+    if (!pairs && top_k > 0 && top_k < V) {
         unsigned prefix = 0; u64 remaining = (u64)top_k;
         for (int shift = 24; shift >= 0; shift -= 8) {
             for (int b = tid; b < 256; b += THREADS) s_hist[b] = 0;
@@ -457,7 +511,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     }
 
     // 3. top-p threshold: the smallest key whose strictly-larger keys hold mass <= top_p * total
-    if (top_p < 1.0f) {
+    if (!pairs && top_p < 1.0f) {
         u64 z = z_row;                                                // (known already if the short list was tried for top-p alone)
         if (!have_z) {
             for_all(true, [&](bool there, unsigned key, u64 mass) { if (there && key >= cut_key) z += mass; });
