@@ -62,3 +62,43 @@ def test_wkv_decay(ops, T, HD):
     wide, w0 = randn(5, T, HD + 4) * 2, randn(6, HD)
     got = ops.wkv_decay(wide[:, :HD], w0)
     assert torch.allclose(got.double(), torch.exp(-torch.exp(wide[:, :HD].double() + w0.double())), rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("lens,I,N", [([1], 8, 16), ([7, 1, 9], 130, 16), ([64], 128, 4), ([65, 200], 129, 5), ([300], 40, 8), ([8, 16, 2], 7, 1), ([700, 3], 264, 13),
+                                      ([2100], 16, 16)])
+def test_selective_scan_forms(ops, lens, I, N, wide):
+    """A thread per channel and a thread per four states, in one piece and in parts, against the recurrence in 64 bits.  Operands are
+    bfloat16; decays come from the hardware's exponential (2^-22 each, whose errors add up over a state's memory)."""
+    T, R, pad = sum(lens), len(lens), ops.selective_state_pad(N)
+    u, z, low = randn(11, T, I).bfloat16(), randn(12, T, I + 8).bfloat16()[:, 8:], randn(13, T, 2 * N + 8).bfloat16()
+    dt, bias, D, xin = randn(14, T, I), randn(15, I) - 4, randn(16, I), randn(17, T, I).bfloat16()
+    A = torch.zeros(I, pad, device=DEV)
+    A[:, :N] = -torch.exp(randn(18, I, N))
+    S0 = torch.zeros(R + 1, I, pad, device=DEV)
+    S0[..., :N] = randn(19, R + 1, I, N)
+    tail0 = randn(20, R + 1, 3, I)
+    qsl = [0]
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    keep = ops.selective_wide_work
+    ops.selective_wide_work = 0 if wide else 1 << 60
+    S, tail = S0.clone(), tail0.clone()
+    try:
+        got = ops.selective_scan(u, dt, bias, A, D, low, 8, 8 + N, z, S, xin, tail, 4, t(qsl), t(list(range(R))[::-1]), R, N)
+    finally:
+        ops.selective_wide_work = keep
+    d = torch.nn.functional.softplus(dt.double() + bias.double())
+    for r in range(R):
+        slot = R - 1 - r
+        s = S0[slot, :, :N].double()
+        for k in range(qsl[r], qsl[r + 1]):
+            s = torch.exp(d[k][:, None] * A[:, :N].double()) * s + (d[k] * u[k].double())[:, None] * low[k, 8:8 + N].double()
+            y = s @ low[k, 8 + N:8 + 2 * N].double() + D.double() * u[k].double()
+            e = y * z[k].double() * torch.sigmoid(z[k].double())
+            assert torch.allclose(got[k].double(), e, rtol=2.0 ** -7, atol=2e-2 * float(e.abs().max()) / 10), (r, k)
+        assert ((S[slot, :, :N].double() - s).norm() / s.norm()).item() < 2e-5
+        want = torch.cat([tail0[slot].double(), xin[qsl[r]:qsl[r + 1]].double()])[-3:]
+        assert torch.equal(tail[slot].double(), want)
+    assert torch.equal(S[R], S0[R])

@@ -217,6 +217,17 @@ __device__ __forceinline__ float walk(const SelArgs& a, int t0, int n, int c, bo
     return sum_dt;
 }
 
+// the convolution's last taps - 1 inputs of a channel, oldest first: those of this step, and before them what the row held
+template <typename T>
+__device__ __forceinline__ void move_tail(const SelArgs& a, int s, int q0, int n, int ch) {
+    const T* x = reinterpret_cast<const T*>(a.xin) + ch;
+    float* mine = a.tail + (size_t)slot_row_(a.slot_ids[s], a.tail_rows) * (a.taps - 1) * a.I + ch;
+    for (int i = 0; i < a.taps - 1; ++i) {                           // ascending: row i takes from an old row behind it, or from the step
+        const int idx = n - (a.taps - 1) + i;
+        mine[(size_t)i * a.I] = idx >= 0 ? to_f32(x[(size_t)(q0 + idx) * a.ld_x]) : mine[(size_t)(a.taps - 1 + idx) * a.I];
+    }
+}
+
 template <typename T, int SL>
 __global__ void __launch_bounds__(NT) selective_scan_kernel(const SelArgs a) {
     pdl_wait();                                                      // (the successor is let in at the end: its waiting CTAs would sit on the SMs of a long, latency-bound walk)
@@ -263,16 +274,176 @@ __global__ void __launch_bounds__(NT) selective_scan_kernel(const SelArgs a) {
         *reinterpret_cast<float4*>(local ? scratch_at(p) : sp) = make_float4(S[0], S[1], S[2], S[3]);
         if (local && slice == 0) a.scratch_dt[((size_t)s * a.parts + p) * a.I + c] = sum_dt;
     }
-    if (!local && p == p_last && a.taps > 1 && threadIdx.x < CH && c0 + (int)threadIdx.x < a.I) {
-        // the convolution's last taps - 1 inputs, oldest first: those of this step, and before them what the row held
-        const int ch = c0 + threadIdx.x;
-        const T* x = reinterpret_cast<const T*>(a.xin) + ch;
-        float* mine = a.tail + (size_t)slot_row_(a.slot_ids[s], a.tail_rows) * (a.taps - 1) * a.I + ch;
-        for (int i = 0; i < a.taps - 1; ++i) {                       // ascending: row i takes from an old row behind it, or from the step
-            const int idx = n - (a.taps - 1) + i;
-            mine[(size_t)i * a.I] = idx >= 0 ? to_f32(x[(size_t)(q0 + idx) * a.ld_x]) : mine[(size_t)(a.taps - 1 + idx) * a.I];
+    if (!local && p == p_last && threadIdx.x < CH && c0 + (int)threadIdx.x < a.I) move_tail<T>(a, s, q0, n, c0 + threadIdx.x);
+}
+
+// ---- bfloat16 prompt portions of up to 16 states: a thread owns a channel with all its states (NS of them, padded to 4, 8 or 16).
+// What a token costs besides its states - loads, softplus, silu, the store - is then paid once per channel instead of being
+// dealt out to the lanes of a channel with shuffles and predicates (that was seven of twelve instructions per state), rows
+// of a warp's 32 channels are 64 and 128 contiguous bytes, and the states' multiplications go in pairs (one instruction for two;
+// the exponentials have no such form).  B and C of a run of tokens lie in shared memory, which every thread reads at
+// the same address.  The next run's values are in registers while this one is computed.  What bounds
+// it is the exponential unit: 16 a token for the states and five for softplus and silu, 73 us for the two walks of 2,048 tokens of
+// 4,096 channels, which take 117 (141 with a thread per four states).
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)), "l"(reinterpret_cast<const unsigned long long&>(c)));
+    return d;
+}
+
+template <int NS, bool READ>
+__device__ __forceinline__ float wide_walk(const SelArgs& a, int t0, int n, int c, bool cv, const float2 (&A)[NS / 2], float2 (&S)[NS / 2], float (*smem)[2][TB][NS]) {
+    using T = __nv_bfloat16;
+    using Raw = unsigned short;
+    const int cc = cv ? c : 0;
+    const float* dp = a.dt + (size_t)t0 * a.ld_dt + cc;
+    const Raw* up = reinterpret_cast<const Raw*>(a.u) + (size_t)t0 * a.ld_u + cc;
+    const Raw* zp = reinterpret_cast<const Raw*>(a.z) + (size_t)t0 * a.ld_z + cc;
+    const Raw* bc = reinterpret_cast<const Raw*>(a.bc) + (size_t)t0 * a.ld_bc;
+    T* op = reinterpret_cast<T*>(a.out) + (size_t)t0 * a.I + cc;
+    const float bias = a.dt_bias[cc], Dc = a.D[cc];
+    auto wide = [](Raw r) { return __uint_as_float((unsigned)r << 16); };
+    float sum_dt = 0.f, d_next[TB];
+    Raw u_next[TB], z_next[TB];
+    constexpr int PB = (TB * NS + NT - 1) / NT;                      // values of B (and of C) of a run per thread
+    Raw b_next[PB], c_next[PB];
+    auto fetch = [&](int r0, int nb) {
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {
+            const int e = i * NT + threadIdx.x, tt = e / NS, k = e % NS;
+            const bool ok = tt < nb && k < a.N;
+            b_next[i] = ok ? bc[(size_t)(r0 + tt) * a.ld_bc + a.col_b + k] : (Raw)0;
+            if (READ) c_next[i] = ok ? bc[(size_t)(r0 + tt) * a.ld_bc + a.col_c + k] : (Raw)0;
         }
+        const float* d = dp + (size_t)r0 * a.ld_dt;
+        const Raw* u = up + (size_t)r0 * a.ld_u;
+        const Raw* z = zp + (size_t)r0 * a.ld_z;
+#pragma unroll
+        for (int tt = 0; tt < TB; ++tt) {
+            if (tt < nb) {                                            // (the same for every thread)
+                d_next[tt] = *d; u_next[tt] = *u;
+                if (READ) z_next[tt] = *z;
+            }
+            d += a.ld_dt; u += a.ld_u; z += a.ld_z;
+        }
+    };
+    auto settle = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {
+            const int e = i * NT + threadIdx.x;
+            if (e < TB * NS) { (&smem[buf][0][0][0])[e] = wide(b_next[i]); if (READ) (&smem[buf][1][0][0])[e] = wide(c_next[i]); }
+        }
+    };
+    fetch(0, min(TB, n));
+    settle(0);
+    __syncthreads();
+    for (int r0 = 0, it = 0; r0 < n; r0 += TB, ++it) {
+        const int nb = min(TB, n - r0), buf = it & 1;
+        float d[TB];
+        Raw u[TB], z[TB];
+#pragma unroll
+        for (int tt = 0; tt < TB; ++tt) { d[tt] = d_next[tt]; u[tt] = u_next[tt]; if (READ) z[tt] = z_next[tt]; }
+        const bool more = r0 + TB < n;
+        if (more) fetch(r0 + TB, min(TB, n - r0 - TB));
+        T* o = op + (size_t)r0 * a.I;
+#pragma unroll
+        for (int tt = 0; tt < TB; ++tt) {
+            if (tt < nb) {
+                const float dt = Act<T>::softplus(d[tt] + bias), uv = wide(u[tt]);
+                const float2 dt2 = make_float2(dt, dt), du2 = make_float2(dt * uv, dt * uv);
+                float2 y2 = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < NS / 2; i += 2) {
+                    const float4 b = *reinterpret_cast<const float4*>(&smem[buf][0][tt][2 * i]);
+                    const float2 e0 = mul2(dt2, A[i]), e1 = mul2(dt2, A[i + 1]);
+                    S[i] = fma2(make_float2(ex2(e0.x), ex2(e0.y)), S[i], mul2(du2, make_float2(b.x, b.y)));
+                    S[i + 1] = fma2(make_float2(ex2(e1.x), ex2(e1.y)), S[i + 1], mul2(du2, make_float2(b.z, b.w)));
+                    if (READ) {
+                        const float4 q = *reinterpret_cast<const float4*>(&smem[buf][1][tt][2 * i]);
+                        y2 = fma2(S[i], make_float2(q.x, q.y), y2);
+                        y2 = fma2(S[i + 1], make_float2(q.z, q.w), y2);
+                    }
+                }
+                if (READ) {
+                    if (cv) *o = from_f32<T>(fmaf(Dc, uv, y2.x + y2.y) * Act<T>::silu(wide(z[tt])));
+                    o += a.I;
+                } else sum_dt += dt;
+            }
+        }
+        if (more) settle(buf ^ 1);                                    // (read two runs ago, with a barrier since)
+        __syncthreads();
     }
+    return sum_dt;
+}
+
+template <int NS>
+__global__ void __launch_bounds__(NT) selective_wide_kernel(const SelArgs a) {
+    pdl_wait();                                                      // (the successor is let in at the end, as in the other form)
+    __shared__ __align__(16) float smem[2][2][TB][NS];               // two buffers of B and C
+    const int s = blockIdx.y / a.parts, p = blockIdx.y - s * a.parts;
+    const int q0 = a.qsl[s], n = a.qsl[s + 1] - q0;
+    int L = n, p_last = 0;                                           // tokens of a part, the part of the request's last token
+    if (a.parts > 1 && n > 0) {
+        L = max(PART_MIN_TOKENS, ((n + a.parts - 1) / a.parts + TB - 1) / TB * TB);
+        p_last = (n - 1) / L;
+    }
+    const bool local = a.mode == 1;
+    const bool copies = local && p_last > 0 && p == a.parts - 1;     // (never a part that mode 1 walks: those lie before p_last)
+    if (n <= 0 || (local ? (p >= p_last && !copies) : p > p_last)) return;
+    const int c = blockIdx.x * NT + threadIdx.x;
+    const bool cv = c < a.I;
+    const int cc = cv ? c : 0;
+    float* sp = a.state + ((size_t)slot_row_(a.slot_ids[s], a.state_rows) * a.I + cc) * NS;
+    auto scratch_at = [&](int part) { return a.scratch + (((size_t)s * a.parts + part) * a.I + cc) * NS; };
+    float2 A[NS / 2], S[NS / 2];
+    auto load = [&](const float* src, float2 (&v)[NS / 2]) {
+#pragma unroll
+        for (int i = 0; i < NS / 2; i += 2) {
+            const float4 x = *reinterpret_cast<const float4*>(src + 2 * i);
+            v[i] = make_float2(x.x, x.y); v[i + 1] = make_float2(x.z, x.w);
+        }
+    };
+    auto store = [&](float* dst) {
+#pragma unroll
+        for (int i = 0; i < NS / 2; i += 2) *reinterpret_cast<float4*>(dst + 2 * i) = make_float4(S[i].x, S[i].y, S[i + 1].x, S[i + 1].y);
+    };
+    if (copies) {
+        load(sp, S);
+        if (cv) store(scratch_at(p));
+        return;
+    }
+    load(a.A + (size_t)cc * NS, A);
+#pragma unroll
+    for (int i = 0; i < NS / 2; ++i) {
+        A[i] = make_float2(Decay<__nv_bfloat16>::hold(A[i].x), Decay<__nv_bfloat16>::hold(A[i].y));
+        S[i] = make_float2(0.f, 0.f);
+    }
+    float sum_dt = 0.f;
+    if (local) {
+        sum_dt = wide_walk<NS, false>(a, q0 + p * L, min(L, n - p * L), c, cv, A, S, smem);
+    } else {
+        load(p_last == 0 ? sp : scratch_at(a.parts - 1), S);         // the state row as it was before the step
+        for (int j = 0; j < p; ++j) {                                // then the parts before this one
+            float2 add[NS / 2];
+            load(scratch_at(j), add);
+            const float sdt = a.scratch_dt[((size_t)s * a.parts + j) * a.I + cc];
+#pragma unroll
+            for (int i = 0; i < NS / 2; ++i) S[i] = fma2(make_float2(ex2(sdt * A[i].x), ex2(sdt * A[i].y)), S[i], add[i]);
+        }
+        wide_walk<NS, true>(a, q0 + p * L, min(L, n - p * L), c, cv, A, S, smem);
+    }
+    pdl_launch_dependents();
+    if (cv && (local || p == p_last)) {
+        store(local ? scratch_at(p) : sp);
+        if (local) a.scratch_dt[((size_t)s * a.parts + p) * a.I + c] = sum_dt;
+    }
+    if (!local && p == p_last && cv) move_tail<__nv_bfloat16>(a, s, q0, n, c);
 }
 
 int state_slices(int N) {
@@ -285,13 +456,15 @@ int state_slices(int N) {
 // padded states of a state row (0: more states than the kernel takes)
 extern "C" int ttie_selective_state_pad(int N) { return N < 1 || N > 128 ? 0 : state_slices(N) * KPT; }
 
+// wide: a thread per channel (16-bit operands, up to 16 states), else a thread per four states.
 // parts > 1: scratch holds requests * parts * channels * (padded states + 1) floats
 extern "C" int ttie_selective_scan(const void* u, long long ld_u, const float* dt, long long ld_dt, const float* dt_bias, const float* A,
                                    const float* D, const void* bc, long long ld_bc, int col_b, int col_c, const void* z, long long ld_z,
                                    float* state, int state_rows, const void* xin, long long ld_x, float* tail, int tail_rows, int taps,
                                    const int* qsl, const int* slot_ids, int num_seqs, void* out, int I, int N, int parts, float* scratch,
-                                   int dtype, void* stream) {
+                                   int wide, int dtype, void* stream) {
     if (num_seqs <= 0) return 0;
+    if (wide && (dtype != kBF16 || N > 16)) TTIE_FAIL("selective_scan: a thread per channel takes 16-bit operands and up to 16 states (%d)", N);
     if (N < 1 || N > 128) TTIE_FAIL("selective_scan: %d states per channel (1 to 128)", N);
     if (parts < 1 || (parts > 1 && !scratch) || (long long)num_seqs * parts > 65535)
         TTIE_FAIL("selective_scan: %d parts for %d requests", parts, num_seqs);
@@ -304,10 +477,17 @@ extern "C" int ttie_selective_scan(const void* u, long long ld_u, const float* d
     const int sl = state_slices(N);
     a.Np = KPT * sl; a.parts = parts; a.scratch = scratch;
     a.scratch_dt = scratch ? scratch + (size_t)num_seqs * parts * I * a.Np : nullptr;
-    const dim3 grid(ceil_div(I, NT / sl), num_seqs * parts);
+    const dim3 grid(wide ? ceil_div(I, NT) : ceil_div(I, NT / sl), num_seqs * parts);
     cudaStream_t s = (cudaStream_t)stream;
     for (int mode = parts > 1 ? 1 : 0; mode >= 0; --mode) {          // (mode 1: every part's own sum, from a zero state)
         a.mode = mode;
+        if (wide) {
+            if (sl == 1) TTIE_LAUNCH(selective_wide_kernel<4>, grid, NT, 0, s, a);
+            else if (sl == 2) TTIE_LAUNCH(selective_wide_kernel<8>, grid, NT, 0, s, a);
+            else TTIE_LAUNCH(selective_wide_kernel<16>, grid, NT, 0, s, a);
+            TTIE_CHECK_LAUNCH("selective_scan");
+            continue;
+        }
 #define SEL_CASE(L_)                                                                                                      \
         if (sl == L_) {                                                                                                   \
             if (dtype == kF32) TTIE_LAUNCH((selective_scan_kernel<float, L_>), grid, NT, 0, s, a);                        \

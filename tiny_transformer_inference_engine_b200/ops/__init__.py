@@ -79,7 +79,7 @@ _SIGNATURES = {
                          _c_void, _c_void, _c_void, _c_void, _c_void, _c_int, _c_void],
     "ttie_selective_scan": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_void, _c_ll,
                             _c_void, _c_int, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_void, _c_void, _c_int, _c_void, _c_int, _c_int, _c_int,
-                            _c_void, _c_int, _c_void],
+                            _c_void, _c_int, _c_int, _c_void],
     "ttie_selective_state_pad": [_c_int],
     "ttie_sandwich_norm": [_c_void, _c_void, _c_void, _c_int, _c_ll, _c_void, _c_void, _c_float, _c_void, _c_float, _c_void, _c_int, _c_int,
                            _c_int, _c_void],
@@ -1188,13 +1188,25 @@ class CudaOps:
     selective_max_parts = 16                # at most this many a request,
     selective_part_tokens = 64              # of at least this many tokens
 
-    def selective_parts(self, num_tokens: int, num_seqs: int, channels: int, states: int) -> int:
+    selective_wide_work = 4 << 20           # tokens x channels of a step from which a thread owns a channel with all its states;
+    selective_wide_warps = 28               # the warps per SM that parts are made for then,
+    selective_wide_parts = 32               # and the most parts
+
+    def selective_wide(self, dtype, num_tokens: int, num_seqs: int, channels: int, states: int) -> bool:
+        """Whether a thread owns a channel (16-bit operands, up to 16 states) rather than four states of one: fewer instructions and a
+        quarter of the threads, so it needs a step large enough to fill the GPU all the same.  16 states, us of a thread per
+        channel | per four states: 4,096 channels 512 tokens 42 | 40, 1,024 tokens 68 | 73, 2,048 tokens 117 | 141, four requests of
+        512 107 | 134; 2,048 channels 2,048 tokens 73 | 74; 8,192 channels 256 tokens 41 | 39, 512 65 | 70, 2,048 204 | 273."""
+        return dtype == torch.bfloat16 and states <= 16 and (num_tokens - (num_seqs - 1)) * channels >= self.selective_wide_work
+
+    def selective_parts(self, num_tokens: int, num_seqs: int, channels: int, states: int, wide: bool = False) -> int:
         """Into how many parts a request's tokens are walked: every part but the last is walked twice, which pays while the
         channels alone give the SMs too few warps to hide a token's latency."""
         longest = num_tokens - (num_seqs - 1)                          # the most tokens one request of the step can bring
-        lanes = self.selective_state_pad(states) // 4
+        lanes = 1 if wide else self.selective_state_pad(states) // 4
         warps = num_seqs * -(-channels * lanes // 32)
-        return max(1, min(self.selective_max_parts, longest // self.selective_part_tokens, self.selective_warps * self.num_sms // warps))
+        target, most = (self.selective_wide_warps, self.selective_wide_parts) if wide else (self.selective_warps, self.selective_max_parts)
+        return max(1, min(most, longest // self.selective_part_tokens, target * self.num_sms // warps))
 
     @staticmethod
     def selective_state_pad(states: int) -> int:
@@ -1212,12 +1224,13 @@ class CudaOps:
         convolution's inputs) into the state rows ``tail`` (None with one tap)."""
         T, I = u.shape
         out = torch.empty((T, I), dtype=u.dtype, device=u.device)
-        parts = self.selective_parts(T, int(num_seqs), I, int(states))
+        wide = self.selective_wide(u.dtype, T, int(num_seqs), I, int(states))
+        parts = self.selective_parts(T, int(num_seqs), I, int(states), wide)
         scratch = torch.empty(int(num_seqs) * parts * I * (A.shape[1] + 1), dtype=torch.float32, device=u.device) if parts > 1 else None
         self._check(self.lib.ttie_selective_scan(
             _ptr(u), u.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(A), _ptr(D), _ptr(bc), bc.stride(0), int(col_b), int(col_c), _ptr(z),
             z.stride(0), _ptr(state), state.shape[0], _ptr(xin), xin.stride(0), _ptr(tail), 0 if tail is None else tail.shape[0], int(taps),
-            _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), _ptr(out), I, int(states), parts, _ptr(scratch), self._dt(u), self._stream(u)),
+            _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), _ptr(out), I, int(states), parts, _ptr(scratch), 1 if wide else 0, self._dt(u), self._stream(u)),
             "selective_scan")
         self.launches += 2 if parts > 1 else 1
         return out
