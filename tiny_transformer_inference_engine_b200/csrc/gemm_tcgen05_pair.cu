@@ -20,6 +20,11 @@
 // peer the matching 128 up rows, so accumulator column j is gate column j and column 128 + j its up column, and the
 // epilogue writes silu(g) * u (models/mlp.py:24-32; silu in 32-bit as kernels/fused_swiglu/kernel.py:20-25) without
 // the [T, 2F] round trip through memory.
+// Grouped form (mixtures of experts): the rows of A are sorted by expert, W holds one matrix per expert, and a tile belongs to one
+// expert's rows - its W rows start at the expert's matrix, and rows behind the expert's last (the next expert's, or zeros) are computed
+// and not stored.  Where the experts' rows start is read on the device (`offsets`), every CTA turns it into its own list of tiles;
+// an expert's tiles of one column range are neighbours, so its matrix comes from HBM once.  16 experts [2048, 2048] and the unit behind
+// them, 8,192 rows: 74 us with the rows' gathering, 84 as the library's grouped product and the activation kernel.
 // Every mbarrier wait is bounded by a clock deadline; a wait that runs out records a code in the error word of the
 // tensor-core product kernels and the CTA leaves its loops; both CTAs meet at the end before tensor memory is freed.
 #include "common.cuh"
@@ -113,11 +118,35 @@ struct PairParams {
     int up_offset;            // SwiGLU: row of W (and entry of bias) where the up projection starts
     int gelu;                 // SwiGLU's epilogue with the tanh form of gelu on the gate
     ErrorWords err;           // where a wait that runs out leaves its code
+    // grouped form: rows offsets[e] .. offsets[e + 1] - 1 of A belong to expert e, whose matrix starts at row e * w_rows of W; the unit's
+    // constants (limit <= 0: no clamps)
+    const int* offsets; int experts, w_rows;
+    float alpha, limit, shift;
 };
+constexpr int MAX_GROUPS = 512;
+
+// a 256-row tile: first row, row behind the last one that is stored, column tile, first row of its matrix in W
+struct Tile { int m0, row_end, tn, w0; };
+template <bool GROUPED>
+__device__ __forceinline__ Tile tile_of(const PairParams& p, const int* group_tiles, int tile, int tiles_m, int tiles_n) {
+    Tile t;
+    if (!GROUPED) {
+        t.m0 = tile % tiles_m * (2 * HM); t.tn = tile / tiles_m; t.row_end = p.M; t.w0 = 0;
+        return t;
+    }
+    int lo = 0, hi = p.experts - 1;
+    while (lo < hi) {                                            // the last expert whose first tile is <= tile (experts without rows have none)
+        const int mid = (lo + hi + 1) >> 1;
+        if (group_tiles[mid] * tiles_n <= tile) lo = mid; else hi = mid - 1;
+    }
+    const int i = tile - group_tiles[lo] * tiles_n, mt = group_tiles[lo + 1] - group_tiles[lo];
+    t.m0 = p.offsets[lo] + i % mt * (2 * HM); t.tn = i / mt; t.row_end = p.offsets[lo + 1]; t.w0 = lo * p.w_rows;
+    return t;
+}
 
 // EPI 0: C = A W^T (+ bias) as OutT; EPI 1: C = silu(A Wg^T + bg) * (A Wu^T + bu) as bfloat16 (OutT)
 // KPS: 64-wide K blocks per stage of the ring (one barrier round trip of the issuing thread per stage)
-template <int STAGES, int KPS, int EPI, typename OutT>
+template <int STAGES, int KPS, int EPI, typename OutT, bool GROUPED>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PairParams p) {
     constexpr uint32_t A_BYTES = HM * BK * 2, B_BYTES = HN * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = KPS * BLOCK_BYTES;
@@ -127,12 +156,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) unsigned long long bars[2 * STAGES + 4];
     __shared__ uint32_t tmem_slot;
+    __shared__ int group_tiles[GROUPED ? MAX_GROUPS + 1 : 1];    // row tiles of the experts before each
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned rank;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    const int tiles_m = (p.M + 2 * HM - 1) / (2 * HM), tiles_n = (p.N + TILE_N - 1) / TILE_N, num_tiles = tiles_m * tiles_n;
+    const int tiles_m = (p.M + 2 * HM - 1) / (2 * HM), tiles_n = (p.N + TILE_N - 1) / TILE_N;
     const int num_kb = (p.K + KPS * BK - 1) / (KPS * BK);        // stages per tile
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]);
     const uint32_t accfull0 = smem_u32(&bars[2 * STAGES]), accempty0 = smem_u32(&bars[2 * STAGES + 2]);
@@ -149,11 +179,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    if (GROUPED && warp == 2) {
+        int before = 0;
+        for (int e0 = 0; e0 < p.experts; e0 += 32) {
+            const int e = e0 + lane;
+            int incl = e < p.experts ? (p.offsets[e + 1] - p.offsets[e] + 2 * HM - 1) / (2 * HM) : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int up = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += up; }
+            if (e < p.experts) group_tiles[e + 1] = before + incl;
+            before += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) group_tiles[0] = 0;
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync_all();                                          // the peer's barriers exist before anything arrives on them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_slot;
+    const int num_tiles = (GROUPED ? group_tiles[p.experts] : tiles_m) * tiles_n;
 
     // Tiles are dealt round-robin to the resident pairs; M tiles are the fast index, so pairs that run together share a
     // W tile (read from HBM once) and the activations stay in L2.
@@ -161,9 +204,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (lane == 0) {
             int kc = 0;
             for (int tile = pair; tile < num_tiles; tile += num_pairs) {
-                const int m0 = (tile % tiles_m) * (2 * HM) + (int)rank * HM;
-                const int tn = tile / tiles_m;
-                const int w0 = EPI == 1 ? (int)rank * p.up_offset + tn * HN : tn * (2 * HN) + (int)rank * HN;
+                const Tile t = tile_of<GROUPED>(p, group_tiles, tile, tiles_m, tiles_n);
+                const int m0 = t.m0 + (int)rank * HM;
+                const int w0 = t.w0 + (EPI == 1 ? (int)rank * p.up_offset + t.tn * HN : t.tn * (2 * HN) + (int)rank * HN);
                 bool ok = true;
                 for (int kb = 0; kb < num_kb; ++kb, ++kc) {
                     const int s = kc % STAGES;
@@ -210,11 +253,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     } else {
         // epilogue warps 2..5: warp w may touch TMEM lanes 32*(w%4) .. +31 = rows of this CTA's half of the tile
         const int quarter = warp & 3;
+        const float limit = p.limit > 0.f ? p.limit : INFINITY;
         int lt = 0;
         for (int tile = pair; tile < num_tiles; tile += num_pairs, ++lt) {
-            const int m0 = (tile % tiles_m) * (2 * HM) + (int)rank * HM, n0 = (tile / tiles_m) * TILE_N;
+            const Tile t = tile_of<GROUPED>(p, group_tiles, tile, tiles_m, tiles_n);
+            const int n0 = t.tn * TILE_N;
             const int ab = lt & 1;
-            const int row = m0 + quarter * 32 + lane;
+            const int row = t.m0 + (int)rank * HM + quarter * 32 + lane;
             bool ok = mbar_wait(accfull0 + 8 * ab, (lt >> 1) & 1, 23, p.err);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -228,15 +273,26 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     uint32_t u[32];
                     tmem_ld32(tmem_acc + (uint32_t)(HN + c * 32), u);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (!GROUPED && p.bias) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const int col = min(n0 + c * 32 + j, p.N - 1);
+                            v[j] = __float_as_uint(__uint_as_float(v[j]) + __bfloat162float(p.bias[col]));
+                            u[j] = __float_as_uint(__uint_as_float(u[j]) + __bfloat162float(p.bias[p.up_offset + col]));
+                        }
+                    }
+                    // (the result is rounded to bfloat16: the fast exponential and division, about 2^-21, do not show; a full division
+                    // here is a call per value that made a tile's epilogue longer than its products)
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        float g = __uint_as_float(v[j]), up = __uint_as_float(u[j]);
-                        if (p.bias) {
-                            const int col = min(n0 + c * 32 + j, p.N - 1);
-                            g += __bfloat162float(p.bias[col]); up += __bfloat162float(p.bias[p.up_offset + col]);
+                        float g = __uint_as_float(v[j]), up = __uint_as_float(u[j]), z;
+                        if (GROUPED) {
+                            g = fminf(g, limit); up = fminf(fmaxf(up, -limit), limit) + p.shift;
+                            z = p.alpha * g;
+                        } else {
+                            z = p.gelu ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
                         }
-                        const float z = p.gelu ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
-                        v[j] = __float_as_uint(g / (1.f + __expf(-z)) * up);
+                        v[j] = __float_as_uint(__fdividef(g, 1.f + __expf(-z)) * up);
                     }
                 } else {
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -247,7 +303,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     }
                 }
                 const int col0 = n0 + c * 32;
-                if (row < p.M && col0 < p.N) {
+                if (row < t.row_end && col0 < p.N) {
                     OutT* dst = reinterpret_cast<OutT*>(p.C) + (long long)row * p.ldc + col0;
                     const bool full = col0 + 32 <= p.N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
                     if (full) {
@@ -268,7 +324,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                                                                 __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
                         }
                     } else {
-                        for (int j = 0; j < 32 && col0 + j < p.N; ++j) dst[j] = from_f32<OutT>(__uint_as_float(v[j]));
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)                 // (unrolled: an index known at run time would put the values into memory)
+                            if (col0 + j < p.N) dst[j] = from_f32<OutT>(__uint_as_float(v[j]));
                     }
                 }
             }
@@ -287,10 +345,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
 }
 
-template <int STAGES, int KPS, int EPI, typename OutT>
+// (the grouped form is given a bound on its tiles: how many there are is known on the device)
+template <int STAGES, int KPS, int EPI, typename OutT, bool GROUPED = false>
 int launch(const CUtensorMap& a, const CUtensorMap& b, const PairParams& p, cudaStream_t s) {
     const size_t smem = (size_t)STAGES * KPS * (HM * BK * 2 + HN * BK * 2) + 1024;
-    auto k = gemm_tc_pair_kernel<STAGES, KPS, EPI, OutT>;
+    auto k = gemm_tc_pair_kernel<STAGES, KPS, EPI, OutT, GROUPED>;
     static bool allowed[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
@@ -300,8 +359,8 @@ int launch(const CUtensorMap& a, const CUtensorMap& b, const PairParams& p, cuda
         allowed[dev] = true;
     }
     const int tile_n = EPI == 1 ? HN : 2 * HN;
-    const int tiles = ceil_div(p.M, 2 * HM) * ceil_div(p.N, tile_n);
-    const int pairs = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
+    const long long tiles = (long long)(GROUPED ? p.M / (2 * HM) + p.experts : ceil_div(p.M, 2 * HM)) * ceil_div(p.N, tile_n);
+    const int pairs = tiles < num_sms() / 2 ? (int)tiles : num_sms() / 2;
     cudaError_t e = launch_kernel(k, dim3(2 * pairs), dim3(192), smem, s, dim3(2, 1, 1), a, b, p);
     if (e != cudaSuccess) TTIE_FAIL("gemm_tc_pair: launch failed: %s", cudaGetErrorString(e));
     return 0;
@@ -320,7 +379,7 @@ extern "C" int ttie_gemm_tc_pair(const void* A, long long lda, const void* W, lo
     CUtensorMap ma, mb;
     if (gemm_tc_make_map(&ma, A, M, K, lda, HM)) return -1;
     if (gemm_tc_make_map(&mb, W, swiglu ? 2LL * N : N, K, ldw, HN)) return -1;
-    PairParams p;
+    PairParams p = {};
     p.C = C; p.ldc = ldc; p.bias = (const __nv_bfloat16*)bias; p.M = M; p.N = N; p.K = K; p.up_offset = swiglu ? N : 0; p.gelu = swiglu == 2;
     if (gemm_tc_error_words(&p.err.word, &p.err.mirror)) TTIE_FAIL("gemm_tc_pair: the error word's address is not to be had");
     cudaStream_t s = (cudaStream_t)stream;
@@ -328,4 +387,26 @@ extern "C" int ttie_gemm_tc_pair(const void* A, long long lda, const void* W, lo
     // thread's barrier round trips are not what bounds this kernel)
     if (swiglu) return launch<6, 1, 1, __nv_bfloat16>(ma, mb, p, s);
     return out_f32 ? launch<6, 1, 0, float>(ma, mb, p, s) : launch<6, 1, 0, __nv_bfloat16>(ma, mb, p, s);
+}
+
+// Rows sorted by expert times their expert's matrix: A bfloat16 [P, K] (row stride lda), W bfloat16 [E, w_rows, K] contiguous, rows
+// offsets[e] .. offsets[e + 1] - 1 (int32 [E + 1] on the device) are expert e's.  glu == 0: C[P, N] = A W_e^T, N = w_rows.  glu == 1: W_e is
+// [2N, K], gate rows then up rows, C[P, N] = g' sigmoid(alpha g') (u' + shift) with g' = min(g, limit), u' = clamp(u, +-limit)
+// (limit <= 0: no clamps).  C bfloat16; rows behind offsets[E] are not written.
+extern "C" int ttie_grouped_gemm_tc(const void* A, long long lda, const void* W, void* C, long long ldc, const int* offsets, int E, int P, int N,
+                                    int K, int glu, float alpha, float limit, float shift, void* stream) {
+    if (P <= 0 || N <= 0 || E <= 0) return 0;
+    if (K <= 0 || K % 8 || lda % 8) TTIE_FAIL("grouped_gemm_tc: K and the row stride must be positive multiples of 8");
+    if (((uintptr_t)A | (uintptr_t)W) & 15) TTIE_FAIL("grouped_gemm_tc: operand pointers must be 16-byte aligned");
+    if (E > MAX_GROUPS) TTIE_FAIL("grouped_gemm_tc: %d experts (at most %d)", E, MAX_GROUPS);
+    PairParams p = {};
+    p.C = C; p.ldc = ldc; p.M = P; p.N = N; p.K = K; p.up_offset = glu ? N : 0;
+    p.offsets = offsets; p.experts = E; p.w_rows = glu ? 2 * N : N; p.alpha = alpha; p.limit = limit; p.shift = shift;
+    if ((long long)E * p.w_rows > 0x7fffffffLL) TTIE_FAIL("grouped_gemm_tc: %d matrices of %d rows", E, p.w_rows);
+    CUtensorMap ma, mb;
+    if (gemm_tc_make_map(&ma, A, P, K, lda, HM)) return -1;
+    if (gemm_tc_make_map(&mb, W, (long long)E * p.w_rows, K, K, HN)) return -1;
+    if (gemm_tc_error_words(&p.err.word, &p.err.mirror)) TTIE_FAIL("grouped_gemm_tc: the error word's address is not to be had");
+    cudaStream_t s = (cudaStream_t)stream;
+    return glu ? launch<6, 1, 1, __nv_bfloat16, true>(ma, mb, p, s) : launch<6, 1, 0, __nv_bfloat16, true>(ma, mb, p, s);
 }

@@ -66,6 +66,8 @@ _SIGNATURES = {
                                         _c_int, _c_void, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_tc": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_tc_pair": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
+    "ttie_grouped_gemm_tc": [_c_void, _c_ll, _c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_float,
+                             _c_void],
     "ttie_scale_add_layernorm": [_c_void, _c_void, _c_int, _c_void, _c_int, _c_ll, _c_void, _c_void, _c_void, _c_int, _c_void, _c_int,
                                  _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_void],
     "ttie_cast_rows": [_c_void, _c_void, _c_ll, _c_int, _c_void],
@@ -1646,6 +1648,38 @@ class CudaOps:
             return 0
         return 2 if pairs > 6 * experts else 1
 
+    def _rows_by_expert(self, x, plan, gather_div):
+        """The rows of x in the order of the plan's pairs (``gather_div`` 0: they are already)."""
+        if not gather_div:
+            return x
+        rows = torch.empty((plan["pairs"], x.shape[1]), dtype=x.dtype, device=x.device)
+        self._check(self.lib.ttie_gather_rows(_ptr(x), x.stride(0), _ptr(plan["pair_of_pos"]), int(gather_div), plan["pairs"],
+                                              x.shape[1], _ptr(rows), self._dt(x), self._stream(x)), "gather_rows")
+        self.launches += 1
+        return rows
+
+    grouped_tc_plain_rows = 512             # rows per expert up to which a grouped product without a gated unit runs on this package's kernel
+
+    def _grouped_tc(self, x, w, plan, gather_div, hidden=0, alpha=1.0, limit=0.0, shift=0.0):
+        """The grouped product on pairs of CTAs (``hidden``: with the gated unit in its epilogue), or None where it does not apply.  With the
+        unit it is ahead of the library's product and the activation kernel at every size measured (16 experts, us, own | library:
+        width 1,024, 24 rows per expert 13.9 | 19.1, 1,024 rows 39 | 59; width 2,048 34 | 43 and 125 | 140; width 4,096 113 | 127 and
+        449 | 476); without it up to some 512 rows per expert (width 2,048: 24 rows 18.4 | 24.8, 256 rows 25.9 | 28.2, 512 rows
+        38.9 | 38.3, 1,024 rows 63 | 58), where the library's smaller tiles fill the last wave better."""
+        E, N, K = w.shape
+        if (x.dtype != torch.bfloat16 or K % 8 or not w.is_contiguous() or not 0 < E <= 512 or w.data_ptr() % 16
+                or (not hidden and plan["pairs"] >= self.grouped_tc_plain_rows * max(1, plan["real_experts"]))):
+            return None
+        rows = self._rows_by_expert(x, plan, gather_div)
+        if rows.stride(0) % 8 or rows.stride(1) != 1 or rows.data_ptr() % 16:
+            return None
+        out = torch.empty((plan["pairs"], hidden or N), dtype=x.dtype, device=x.device)
+        self._check(self.lib.ttie_grouped_gemm_tc(_ptr(rows), rows.stride(0), _ptr(w), _ptr(out), out.stride(0), _ptr(plan["offsets"]), E,
+                                                  plan["pairs"], hidden or N, K, 1 if hidden else 0, float(alpha), float(limit or 0.0), float(shift),
+                                                  self._stream(x)), "grouped_gemm_tc")
+        self.launches += 1
+        return out
+
     def _library_grouped(self, x, w, plan, gather_div):
         """The library's grouped product (bfloat16, many rows): rows gathered into expert order, then one call whose group
         boundaries are read on the device.  None where it does not apply (sizes, or a build of the library without it)."""
@@ -1655,12 +1689,7 @@ class CudaOps:
             self._grouped_mm = getattr(torch.nn.functional, "grouped_mm", None) or getattr(torch, "_grouped_mm", None) or False
             if self._grouped_mm is False:
                 return None
-        rows = x
-        if gather_div:
-            rows = torch.empty((plan["pairs"], x.shape[1]), dtype=x.dtype, device=x.device)
-            self._check(self.lib.ttie_gather_rows(_ptr(x), x.stride(0), _ptr(plan["pair_of_pos"]), int(gather_div), plan["pairs"],
-                                                  x.shape[1], _ptr(rows), self._dt(x), self._stream(x)), "gather_rows")
-            self.launches += 1
+        rows = self._rows_by_expert(x, plan, gather_div)
         try:
             return self._grouped_mm(rows, w.transpose(1, 2), offs=plan["offsets"][1:w.shape[0] + 1])
         except (RuntimeError, TypeError, NotImplementedError):
@@ -1692,7 +1721,8 @@ class CudaOps:
 
     def grouped_glu(self, x, w_gu, plan, gather_div, hidden, alpha=1.0, limit=0.0, shift=0.0):
         """The experts' gate/up products over rows sorted by expert, then the gated unit: [pairs, hidden].  Few rows: one
-        kernel (the unit in the weight-streaming product's epilogue); many: the grouped product and the activation kernel."""
+        kernel (the unit in the weight-streaming product's epilogue); many: the rows gathered and one tcgen05 product with the unit in
+        its epilogue (``_grouped_tc``), or, for what that does not take, a grouped product and the activation kernel."""
         few = self._grouped_few(x, plan)
         E, N, K = w_gu.shape
         vn = 4 if x.dtype == torch.float32 else 8
@@ -1704,6 +1734,9 @@ class CudaOps:
                                                    float(alpha), float(limit or 0.0), float(shift), self._stream(x)), "grouped_gemm (gated)")
             self.launches += 1
             return out
+        out = None if few else self._grouped_tc(x, w_gu, plan, gather_div, hidden, alpha, limit, shift)
+        if out is not None:
+            return out
         return self.glu(self.grouped_linear(x, w_gu, plan, gather_div), hidden, alpha, limit, shift)
 
     _ROW_ACTS = {None: 0, "relu2": 1}
@@ -1713,13 +1746,15 @@ class CudaOps:
         ``act(s * (x[pair_of_pos[pos] // gather_div] @ w_up[e].T))`` -> [pairs, F] in the compute dtype.  ``row_scale`` float32
         [T, top]: s is the pair's routing weight - the weight goes in AHEAD of the expert (it multiplies the expert's input; the
         product being linear, it is applied to the 32-bit sums) -, None: 1.  ``act``: "relu2" or None.  Few rows, or 32-bit: the
-        activation is the product's epilogue; many rows in bfloat16: the library's grouped product, then one pass in place."""
+        activation is the product's epilogue; many rows in bfloat16: the tcgen05 or the library's grouped product, then one pass in place."""
         E, N, K = w_up.shape
         code = self._ROW_ACTS[act]
         few = self._grouped_few(x, plan)
         scale_of = plan["pair_of_pos"] if row_scale is not None else None
         if not few and x.dtype == torch.bfloat16:
-            out = self._library_grouped(x, w_up, plan, gather_div)
+            out = self._grouped_tc(x, w_up, plan, gather_div)
+            if out is None:
+                out = self._library_grouped(x, w_up, plan, gather_div)
             if out is not None:
                 if code or row_scale is not None:
                     self._check(self.lib.ttie_row_scale_act(_ptr(out), out.stride(0), plan["pairs"], N, code, _ptr(row_scale), _ptr(scale_of),
@@ -1738,12 +1773,14 @@ class CudaOps:
     def grouped_linear(self, x, w, plan, gather_div=0, out_dtype=None):
         """Rows sorted by expert times their expert's matrix: w [E, N, K]; row ``pos`` of the result is
         x[pair_of_pos[pos] // gather_div] @ w[e].T (``gather_div`` 0: x[pos]).  Few rows: a kernel that streams each tile's
-        weights once; many rows in bfloat16: the library's grouped product (its result is bfloat16 whatever ``out_dtype``
-        asks: it has no wider output); else (float32) FFMA tiles."""
+        weights once; many rows in bfloat16: the tcgen05 grouped product, or from ``grouped_tc_plain_rows`` rows per expert the library's (the
+        result is bfloat16 whatever ``out_dtype`` asks); else (float32) FFMA tiles."""
         E, N, K = w.shape
         few = self._grouped_few(x, plan)
         if not few and x.dtype == torch.bfloat16:
-            out = self._library_grouped(x, w, plan, gather_div)
+            out = self._grouped_tc(x, w, plan, gather_div)
+            if out is None:
+                out = self._library_grouped(x, w, plan, gather_div)
             if out is not None:
                 return out
         out = torch.empty((plan["pairs"], N), dtype=out_dtype or x.dtype, device=x.device)
