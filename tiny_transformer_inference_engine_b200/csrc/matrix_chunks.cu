@@ -32,9 +32,11 @@
 // Chunks are numbered over the whole step: request s owns the numbers from qsl[s] / 64 + s on, which leaves room for its last
 // partial chunk and needs nothing of the host but the number of tokens and requests.
 //
-// One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 28 + 9 + 62 against the walk's 514; 16 of 64 x 128
-// (mlstm) 13 + 9 + 44 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 39 + 16 + 87 against 473.  What bounds the out kernel is
-// latency: 8 to 12 warps per SM (registers and the planes in shared memory), issue slots 27 % used, the tensor pipe 37 / 15 / 12 %.
+// One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 28 + 9 + 65 against the walk's 514; 16 of 64 x 128
+// (mlstm) 13 + 9 + 46 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 30 + 18 + 79 against 473.  What bounds the out kernel is
+// latency: 12 warps per SM (168 registers, the planes in shared memory), issue slots 27 % used, the tensor pipe 37 / 15 / 12 %.  The wkv
+// kernels were 39 and 87 with half the threads in the sum (a run of 32 tokens' decays per thread is one serial chain of loads and
+// multiplications in 64 bits) and two blocks of out per SM instead of three.
 // Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
 // 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 4.6e-8 (4.4e-8).
 #include "common.cuh"
@@ -82,6 +84,18 @@ __device__ __forceinline__ bool find_chunk(const int* qsl, int num_seqs, int num
     t0 = qsl[s] + c * CT;
     n = min(CT, len - c * CT);
     return c >= 0 && n > 0;
+}
+
+// x^n for 0 <= n <= 64 in 64 bits by squaring (0^0 = 1: a head that keeps nothing still sees the token itself): seven roundings at most, a
+// tenth of the time of the general function
+__device__ __forceinline__ double power(double x, int n) {
+    double r = 1.0;
+#pragma unroll
+    for (int b = 0; b < 7; ++b) {
+        if (n >> b & 1) r *= x;
+        x *= x;
+    }
+    return r;
 }
 
 // ---- planes
@@ -177,21 +191,21 @@ __device__ __forceinline__ void store_planes(uint16_t* base, int step, int at, c
 
 // 64 rows of COLS values into PL planes: row j's columns from src + j * ld, zero where in(j, column) is false, behind scale(j, values).  The
 // loads of four pieces are on their way before the first is split.
-template <int PL, int COLS, int LDS, typename E, typename In, typename Scale>
+template <int PL, int COLS, int LDS, int NT = 128, typename E, typename In, typename Scale>
 __device__ __forceinline__ void stage_rows(uint16_t* dst, const E* src, long long ld, In in, Scale scale) {
-    constexpr int PIECES = COLS / 8, ITERS = CT * PIECES / 128, BATCH = 4;
-    static_assert(ITERS % BATCH == 0, "64 rows of a multiple of 64 values over 128 threads");
+    constexpr int PIECES = COLS / 8, ITERS = CT * PIECES / NT, BATCH = ITERS < 4 ? ITERS : 4;
+    static_assert(ITERS > 0 && ITERS % BATCH == 0, "64 rows of a multiple of 64 values");
 #pragma unroll
     for (int i0 = 0; i0 < ITERS; i0 += BATCH) {
         float x[BATCH][8];
 #pragma unroll
         for (int i = 0; i < BATCH; ++i) {
-            const int e = (i0 + i) * 128 + threadIdx.x, j = e / PIECES, c = (e % PIECES) * 8;
+            const int e = (i0 + i) * NT + threadIdx.x, j = e / PIECES, c = (e % PIECES) * 8;
             load8(src + (size_t)j * ld + c, in(j, c), x[i]);
         }
 #pragma unroll
         for (int i = 0; i < BATCH; ++i) {
-            const int e = (i0 + i) * 128 + threadIdx.x, j = e / PIECES, c = (e % PIECES) * 8;
+            const int e = (i0 + i) * NT + threadIdx.x, j = e / PIECES, c = (e % PIECES) * 8;
             scale(j, x[i]);
             store_planes<PL>(dst, CT * LDS, j * LDS + c, x[i]);
         }
@@ -199,9 +213,9 @@ __device__ __forceinline__ void stage_rows(uint16_t* dst, const E* src, long lon
 }
 
 // rows t0 .. t0 + n - 1, columns col0 .. col0 + 63 of a head's values; `bad`: per 16 tokens, whether a value is not finite
-template <typename VT, int VPL>
+template <typename VT, int VPL, int NT = 128>
 __device__ __forceinline__ void stage_values(uint16_t* v_s, const VT* vp, long long ld, int n, int col0, int Dv, int* bad) {
-    stage_rows<VPL, VT_COLS, VLD>(v_s, vp + col0, ld, [&](int j, int c) { return j < n && col0 + c < Dv; }, [&](int j, const float (&x)[8]) {
+    stage_rows<VPL, VT_COLS, VLD, NT>(v_s, vp + col0, ld, [&](int j, int c) { return j < n && col0 + c < Dv; }, [&](int j, const float (&x)[8]) {
         if (bad == nullptr) return;
         bool fine = true;
 #pragma unroll
@@ -246,19 +260,20 @@ __device__ __forceinline__ void chunk_gates(const ChunkArgs& a, int t0, int n, i
 // ------------------------------------------------------------------------------------------- chunk_sum
 template <int MODE, int KP> struct SumSmem {
     static constexpr int LD = KP + 8;
-    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + (MODE == WKV ? KP * 8 : CT * 4); }
+    static constexpr int NT = MODE == WKV ? 256 : 128;               // wkv: a thread per channel and run of tokens, so more of them
+    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + (MODE == WKV ? NT * 8 : CT * 4); }
 };
 
 template <int MODE, int KP, typename VT>
-__global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
-    constexpr int LD = KP + 8, VPL = sizeof(VT) == 4 ? 3 : 1;
+__global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const ChunkArgs a) {
+    constexpr int NT = SumSmem<MODE, KP>::NT, PARTS = NT / 128, LD = KP + 8, VPL = sizeof(VT) == 4 ? 3 : 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* kd = reinterpret_cast<uint16_t*>(smem_raw);                             // [3][CT][LD]: decayed keys
     uint16_t* v_s = kd + 3 * CT * LD;                                                 // [VPL][CT][VLD]
     double* half = reinterpret_cast<double*>(v_s + VPL * CT * VLD);                   // [8]
     float* wt = reinterpret_cast<float*>(half + 8);                                   // [CT]: a token's weight at the chunk's end
     TTIE_PDL_ENTRY();
-    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 3, part = tid >> 7;      // (part: which share of the key channels)
     int s, c, t0, n;
     if (!find_chunk(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
     const size_t unit = (size_t)blockIdx.x * a.H + h;
@@ -267,8 +282,8 @@ __global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
     if constexpr (MODE == WKV) {
         // a thread per channel and run of LEN tokens: the decays of the run, its product, then keys times the decays behind them (products
         // of up to 64 decays in 64 bits: in 32 they leave more than the walk's one rounding per token)
-        constexpr int LEN = CT * KP / 128, RUNS = CT / LEN;
-        double* tot = half;                                                           // [KP]: product over the last run (RUNS == 2; over wt, which is not used here)
+        constexpr int LEN = CT * KP / NT, RUNS = CT / LEN;
+        double* tot = half;                                                           // [RUNS][KP]: product over a run (over wt, which is not used here)
         const int ch = tid % KP, run = tid / KP;
         const bool in = ch < a.D;
         const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D + ch;
@@ -281,13 +296,16 @@ __global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
             w[i] = in && j < n ? wp[(size_t)j * a.H * a.D] : 1.f;
             kv[i] = in && j < n ? kp[(size_t)j * a.ld_qk] : __float2bfloat16(0.f);
         }
-        stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
+        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
         double all = 1.0;
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) all *= (double)w[i];
-        if (RUNS == 2 && run == 1) tot[ch] = all;
+        tot[run * KP + ch] = all;
         __syncthreads();
-        double suf = RUNS == 2 && run == 0 ? tot[ch] : 1.0;
+        double suf = 1.0;
+#pragma unroll
+        for (int i = RUNS - 1; i > 0; --i)
+            if (i > run) suf *= tot[i * KP + ch];
         if (run == 0 && ch < a.Dpad) {
             const double f = in ? all * suf : 1.0;
             a.aux[2 * unit * a.Dpad + ch] = (float)f;
@@ -300,9 +318,9 @@ __global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
             suf *= (double)w[i];
         }
     } else {
-        stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
+        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
         if constexpr (MODE == RET) {
-            if (tid < CT) wt[tid] = tid < n ? (float)pow((double)a.decay[h], (double)(n - 1 - tid)) : 0.f;
+            if (tid < CT) wt[tid] = tid < n ? (float)power((double)a.decay[h], n - 1 - tid) : 0.f;
         } else {
             double F, x, X;
             chunk_gates(a, t0, n, h, half, F, x, X);
@@ -312,7 +330,7 @@ __global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
         __syncthreads();
         using KT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
         const KT* kp = reinterpret_cast<const KT*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
-        stage_rows<3, KP, LD>(kd, kp, a.ld_qk, [&](int j, int ch) { return j < n && ch < a.D; }, [&](int j, float (&x)[8]) {
+        stage_rows<3, KP, LD, NT>(kd, kp, a.ld_qk, [&](int j, int ch) { return j < n && ch < a.D; }, [&](int j, float (&x)[8]) {
             const float w = wt[j];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = j < n ? x[i] * w : 0.f;
@@ -329,29 +347,30 @@ __global__ void __launch_bounds__(128) chunk_sum_kernel(const ChunkArgs a) {
     for (int col0 = 0; col0 < a.Dv; col0 += VT_COLS) {
         if (col0 > 0) {
             __syncthreads();
-            stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv, nullptr);
+            stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, col0, a.Dv, nullptr);
             __syncthreads();
         }
-        float acc[KP / 8][4];
+        constexpr int NP = KP / 16 / PARTS;                                           // 16-channel tiles of this warp
+        float acc[2 * NP][4];
 #pragma unroll
-        for (int i = 0; i < KP / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+        for (int i = 0; i < 2 * NP; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 #pragma unroll
         for (int k0 = 0; k0 < CT; k0 += 16) {
             uint32_t av[VPL][4];
 #pragma unroll
             for (int l = 0; l < VPL; ++l) ldsm<true>(av[l], at_rows_a(v_s + l * CT * VLD, VLD, warp * 16, k0, lane));
 #pragma unroll
-            for (int np = 0; np < KP / 16; ++np) {
+            for (int np = 0; np < NP; ++np) {
                 uint32_t b[3][4];
 #pragma unroll
-                for (int l = 0; l < 3; ++l) ldsm<true>(b[l], at_rows(kd + l * CT * LD, LD, np * 16, k0, lane));
+                for (int l = 0; l < 3; ++l) ldsm<true>(b[l], at_rows(kd + l * CT * LD, LD, (part * NP + np) * 16, k0, lane));
                 mma_planes<VPL, 3>(acc[2 * np], acc[2 * np + 1], av, b);
             }
         }
         float* dst = a.part + (unit * a.Dv + col0 + warp * 16) * a.Dpad;
 #pragma unroll
-        for (int i = 0; i < KP / 8; ++i) {
-            const int ch = i * 8 + 2 * t;
+        for (int i = 0; i < 2 * NP; ++i) {
+            const int ch = part * NP * 16 + i * 8 + 2 * t;
             if (ch < a.Dpad) {
                 if (col0 + warp * 16 + g < a.Dv) *reinterpret_cast<float2*>(dst + (size_t)g * a.Dpad + ch) = make_float2(acc[i][0], acc[i][1]);
                 if (col0 + warp * 16 + g + 8 < a.Dv) *reinterpret_cast<float2*>(dst + (size_t)(g + 8) * a.Dpad + ch) = make_float2(acc[i][2], acc[i][3]);
@@ -374,7 +393,7 @@ __global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
     if (c_lo >= c_hi) return;
     if (MODE == RET) {
         const int last = len - (c_hi - 1) * CT;
-        if (threadIdx.x < 2) powers[threadIdx.x] = (float)pow((double)a.decay[h], (double)(threadIdx.x == 0 ? CT : min(CT, last)));
+        if (threadIdx.x < 2) powers[threadIdx.x] = (float)power((double)a.decay[h], threadIdx.x == 0 ? CT : min(CT, last));
         __syncthreads();
     }
     const size_t row = state_row(a.slot_ids[s], a.state_rows);
@@ -451,12 +470,12 @@ __global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
 // ------------------------------------------------------------------------------------------- chunk_out
 template <int MODE, int KP> struct OutSmem {
     static constexpr int LD = KP + 8, FLD = KP + 4;
-    static constexpr int EXTRA = MODE == WKV ? (2 * CT * FLD + 4 * KP + 4 * 16 * 17) * 4 : MODE == MLSTM ? CT * 24 + KP * 4 : (CT + 1 + 3) * 4;
+    static constexpr int EXTRA = MODE == WKV ? (2 * CT * FLD + 4 * KP) * 4 : MODE == MLSTM ? CT * 24 + KP * 4 : (CT + 1 + 3) * 4;
     static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 16 + 64 + EXTRA; }
 };
 
 template <int MODE, int KP, typename VT>
-__global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
+__global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT) == 4 ? 2 : 3) chunk_out_kernel(const ChunkArgs a) {
     constexpr int LD = KP + 8, FLD = KP + 4, VPL = sizeof(VT) == 4 ? 3 : 1;
     constexpr int QPL = MODE == MLSTM ? 1 : 3, KPL = MODE == MLSTM ? 1 : 3, KS = KP / 16;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -514,7 +533,6 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
         float* ws = reinterpret_cast<float*>(extra);                                  // [CT][FLD] decays
         float* pre = ws + CT * FLD;                                                   // [CT][FLD] product of the block's decays before the token
         float* blk = pre + CT * FLD;                                                  // [4][KP] product over a block
-        float* diag = blk + 4 * KP;                                                   // [4][16][17] scores inside a block
         for (int e = tid; e < 4 * KP; e += 128) {
             const int J = e / KP, ch = e % KP;
             const bool in = ch < a.D;
@@ -539,8 +557,9 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
             }
         }
         __syncthreads();
-        // inside the block: lanes own channels, running products from every key on; 16 sums over the lanes at a time
-        float* dg = diag + warp * 16 * 17;
+        // inside the block: lanes own channels, running products from every key on; 16 sums over the lanes at a time.  The scores of key j
+        // take the place of the block's row j of decays (columns 0 .. 15), which nothing reads from step j on
+        float* dg = ws + warp * 16 * FLD;
         for (int ch0 = 0; ch0 < KP; ch0 += 64) {
             float r[16][2], ub[2];
             bool in[2];
@@ -572,7 +591,7 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
                 int first = 0;
                 RunReduce<16, 16>::run(sum, lane, first);
                 if ((lane & 1) == 0) {
-                    float* o = dg + first * 17 + j;
+                    float* o = dg + j * FLD + first;
                     *o = ch0 == 0 ? sum[0] : *o + sum[0];
                 }
             }
@@ -610,7 +629,7 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
                         const int r = g + (b & 2 ? 8 : 0), col = i * 8 + 2 * t + (b & 1);
-                        P[2 * J + i][b] = col <= r ? dg[r * 17 + col] : 0.f;
+                        P[2 * J + i][b] = col <= r ? dg[col * FLD + r] : 0.f;
                     }
         row_in[0] = row_in[1] = 1.f;
     } else {
@@ -621,7 +640,7 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const ChunkArgs a) {
         double* Fs = Ms + CT;
         float* nb = reinterpret_cast<float*>(Fs + CT);
         if constexpr (MODE == RET) {
-            if (tid <= CT) pw[tid] = (float)pow((double)a.decay[h], (double)tid);
+            if (tid <= CT) pw[tid] = (float)power((double)a.decay[h], tid);
             __syncthreads();
         } else {
             double F, x, X;
@@ -775,7 +794,7 @@ int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
     a.slot_lo = first; a.slots = slots;
     const dim3 grid(slots, a.H);
     const dim3 carry(ceil_div(a.Dv * a.Dpad + (MODE == MLSTM ? a.Dpad : 0), 4 * CARRY), a.H, a.num_seqs);
-    TTIE_LAUNCH((chunk_sum_kernel<MODE, KP, VT>), grid, 128, sum_smem, st, a);
+    TTIE_LAUNCH((chunk_sum_kernel<MODE, KP, VT>), grid, (SumSmem<MODE, KP>::NT), sum_smem, st, a);
     TTIE_LAUNCH((chunk_carry_kernel<MODE>), carry, CARRY, 0, st, a);
     TTIE_LAUNCH((chunk_out_kernel<MODE, KP, VT>), grid, 128, out_smem, st, a);
     TTIE_CHECK_LAUNCH("matrix_chunks");
