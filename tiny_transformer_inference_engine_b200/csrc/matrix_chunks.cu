@@ -33,12 +33,12 @@
 // partial chunk and needs nothing of the host but the number of tokens and requests.
 //
 // One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 28 + 9 + 65 against the walk's 514; 16 of 64 x 128
-// (mlstm) 13 + 9 + 46 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 30 + 18 + 79 against 473.  What bounds the out kernel is
+// (mlstm) 13 + 9 + 46 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 34 + 20 + 79 against 473.  What bounds the out kernel is
 // latency: 12 warps per SM (168 registers, the planes in shared memory), issue slots 27 % used, the tensor pipe 37 / 15 / 12 %.  The wkv
 // kernels were 39 and 87 with half the threads in the sum (a run of 32 tokens' decays per thread is one serial chain of loads and
 // multiplications in 64 bits) and two blocks of out per SM instead of three.
 // Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
-// 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 4.6e-8 (4.4e-8).
+// 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 3.9e-8 (4.4e-8).
 #include "common.cuh"
 #include "run_reduce.cuh"
 #include <math.h>
@@ -147,6 +147,31 @@ __device__ __forceinline__ void mma_planes(float (&c0)[4], float (&c1)[4], const
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) { c0[i] += h0[i]; c1[i] += h1[i]; }
+}
+// The same for one plane of A and three of B, closer still: the leading products eight at a time, and what rounding the running sum
+// leaves kept beside it (two-sum), with the small planes; acc + left is the result.  The wkv chunk sums take it, whose walk rounds once a
+// token: the state's error against 64 bits 4.6e-8 -> 3.9e-8 (the walk's 4.4e-8) for 4 us of 30.
+__device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b));
+}
+__device__ __forceinline__ void mma_planes_kept(float (&acc)[4], float (&left)[4], const uint32_t (&a)[4], const uint32_t (&b)[3][4], int side) {
+    float l[4] = {0.f, 0.f, 0.f, 0.f};
+    mma(l, a, b[2][2 * side], b[2][2 * side + 1]);
+    mma(l, a, b[1][2 * side], b[1][2 * side + 1]);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float h[4] = {0.f, 0.f, 0.f, 0.f};
+        mma8(h, a[2 * half], a[2 * half + 1], b[0][2 * side + half]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float t = acc[i] + h[i], u = t - acc[i];
+            left[i] += (acc[i] - (t - u)) + (h[i] - u);
+            acc[i] = t;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) left[i] += l[i];
 }
 template <bool TRANS>
 __device__ __forceinline__ void ldsm(uint32_t (&r)[4], const uint16_t* p) {
@@ -354,6 +379,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
         float acc[2 * NP][4];
 #pragma unroll
         for (int i = 0; i < 2 * NP; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+        float left[MODE == WKV ? 2 * NP : 1][4] = {};
 #pragma unroll
         for (int k0 = 0; k0 < CT; k0 += 16) {
             uint32_t av[VPL][4];
@@ -364,8 +390,19 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
                 uint32_t b[3][4];
 #pragma unroll
                 for (int l = 0; l < 3; ++l) ldsm<true>(b[l], at_rows(kd + l * CT * LD, LD, (part * NP + np) * 16, k0, lane));
-                mma_planes<VPL, 3>(acc[2 * np], acc[2 * np + 1], av, b);
+                if constexpr (MODE == WKV) {
+                    mma_planes_kept(acc[2 * np], left[2 * np], av[0], b, 0);
+                    mma_planes_kept(acc[2 * np + 1], left[2 * np + 1], av[0], b, 1);
+                } else {
+                    mma_planes<VPL, 3>(acc[2 * np], acc[2 * np + 1], av, b);
+                }
             }
+        }
+        if constexpr (MODE == WKV) {
+#pragma unroll
+            for (int i = 0; i < 2 * NP; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) if (fabsf(acc[i][j]) < INFINITY) acc[i][j] += left[i][j];      // (behind an overflow it holds inf - inf)
         }
         float* dst = a.part + (unit * a.Dv + col0 + warp * 16) * a.Dpad;
 #pragma unroll
