@@ -402,7 +402,7 @@ class OpRecorder:
              "scale_add_layernorm", "cast_rows", "latent_store", "latent_query", "gate_heads", "batched_linear", "causal_conv",
              "rglru_scan", "glu", "linear_glu", "grouped_glu", "moe_route", "moe_plan", "grouped_linear", "moe_combine",
              "qkv_conv_rope_store", "conv_tail_update", "gate_head_rows", "token_shift_mix", "wkv_scan", "mlstm_scan", "head_norm_gate",
-             "activation", "linear_act", "wkv_decay", "mlstm_gates", "rotate_heads", "retention_scan", "stream_conv", "proj_row_rms",
+             "activation", "linear_act", "wkv_decay", "mlstm_gates", "mlstm_chunks", "rotate_heads", "retention_scan", "stream_conv", "proj_row_rms",
              "rmsnorm_cols", "grouped_act", "sandwich_norm", "joint_qkv_store", "paged_attention_joint", "selective_scan", "activation_rows", "linear_narrow",
              "residual_sum", "token_gate", "moe_plan_table")
 
@@ -448,7 +448,7 @@ def op_cost(name, args, kw, out, kv_lens, window):
     """(bytes that must move, flops) of one recorded call, from its shapes."""
     import torch
     flops = 0
-    if name in ("wkv_scan", "mlstm_scan"):
+    if name in ("wkv_scan", "mlstm_scan", "mlstm_chunks"):
         # the step's rows in and out, each request's state row read and written once; the recurrence's arithmetic is 32-bit on
         # the ordinary cores: three (wkv) or four (mlstm) multiply-adds per state element and token, returned as a second count
         if name == "wkv_scan":
