@@ -859,6 +859,24 @@ def test_gemm_tcgen05_pair_with_swiglu(ops, M, F, K, bias):
     assert ops.tc_error() == 0
 
 
+@pytest.mark.parametrize("gate,values", [("silu", (-87.375, -87.5, -88.0, -88.5, -20.0, 3.0)), ("gelu_tanh", (-10.015625, -10.03125, -10.046875, -5.0, 3.0, -10.0))])
+def test_gemm_tcgen05_pair_gate_far_below_zero(ops, gate, values):
+    """A gate whose 1 + e^-z lies above 2^126 still divides: the result is small, not zero, and a large up value brings it back.  One
+    rounding to bfloat16 is 2^-9; the fast exponential at 88 is off by 2 + 1.17 * 88 units of 2^-23, below 2^-16."""
+    F, K = len(values), 64
+    x, w = torch.zeros(3, K), torch.zeros(2 * F, K)
+    x[:, :2] = 1.0
+    for f, v in enumerate(values):                                    # a gate in two exact pieces
+        w[f, 0] = float(torch.tensor(v).bfloat16())
+        w[f, 1] = v - w[f, 0]
+    w[F:, 0] = 2.0 ** 100
+    out = ops.linear_swiglu_tc_pair(x.bfloat16().to(DEV), w.bfloat16().to(DEV), None, F, gate).double().cpu()
+    g = torch.tensor(values, dtype=torch.float64)
+    z = g if gate == "silu" else 1.5957691216057308 * (g + 0.044715 * g ** 3)
+    assert torch.allclose(out, (g / (1 + torch.exp(-z)) * 2.0 ** 100).expand(3, F), rtol=2.0 ** -8, atol=0.0)
+    assert ops.tc_error() == 0
+
+
 # ------------------------------------------------------------------------------------------ tcgen05 attention
 TC_SHAPES = [(32, 1, 128, 64), (32, 1, 128, 16), (8, 2, 64, 8), (3, 1, 64, 128), (71, 1, 64, 64), (4, 2, 128, 32), (5, 5, 64, 256)]
 

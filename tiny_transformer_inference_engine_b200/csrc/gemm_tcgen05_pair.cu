@@ -281,18 +281,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                             u[j] = __float_as_uint(__uint_as_float(u[j]) + __bfloat162float(p.bias[p.up_offset + col]));
                         }
                     }
-                    // (the result is rounded to bfloat16: the fast exponential and division, about 2^-21, do not show; a full division
-                    // here is a call per value that made a tile's epilogue longer than its products)
+                    // (a full division: the fast one gives 0 for a divisor above 2^126, a gate below about -87)
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        float g = __uint_as_float(v[j]), up = __uint_as_float(u[j]), z;
+                        float g = __uint_as_float(v[j]), up = __uint_as_float(u[j]);
                         if (GROUPED) {
                             g = fminf(g, limit); up = fminf(fmaxf(up, -limit), limit) + p.shift;
-                            z = p.alpha * g;
+                            v[j] = __float_as_uint(__fdividef(g, 1.f + __expf(-p.alpha * g)) * up);
                         } else {
-                            z = p.gelu ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
+                            const float z = p.gelu ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
+                            v[j] = __float_as_uint(g / (1.f + __expf(-z)) * up);
                         }
-                        v[j] = __float_as_uint(__fdividef(g, 1.f + __expf(-z)) * up);
                     }
                 } else {
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
