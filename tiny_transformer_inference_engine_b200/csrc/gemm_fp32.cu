@@ -126,7 +126,9 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
         for (int c = 0; c < 4; ++c)
             if (gn + c < N) C[(size_t)gm * ldc + gn + c] = v[c] + (bias ? bias[gn + c] : 0.f);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // (no CTA leaves while its tile is read)
+    // no CTA leaves while its tile is read.  (Not the .aligned form, which every lane of a warp has to reach together: at the tiles' edges lanes
+    // come out of the loop at different times)
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 int launch_tiles(const float* A, const float* W, const float* bias, float* C, int B, int M, int N, int K, int lda, int ldw, int ldc,
