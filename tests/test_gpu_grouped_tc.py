@@ -58,3 +58,65 @@ def test_plain(ops, counts, identity, top, N, K):
         exp = rows[off[e]:off[e + 1]].double().cpu() @ w[e].double().cpu().T
         assert torch.allclose(got[off[e]:off[e + 1]].double().cpu(), exp, rtol=2.0 ** -8, atol=1e-5 * K ** 0.5)
     assert ops.tc_error() == 0
+
+
+@pytest.mark.parametrize("rows", [3, 300])
+@pytest.mark.parametrize("consts", [(1.702, 7.0, 1.0), (1.0, 0.0, 0.0)])
+def test_gated_on_what_is_not_finite(ops, rows, consts):
+    """Gates and up values that are not finite, through the public call in every form it has: NaN without clamps stays NaN, with clamps it is what
+    the clamp makes of it; infinities likewise.  The gates' columns (+inf, -inf, NaN, 1) against the up columns of the same."""
+    odd = torch.tensor([float("inf"), float("-inf"), float("nan"), 1.0])
+    x, w = torch.zeros(rows, 64), torch.zeros(2, 2 * 16, 64)
+    x[:, 0], x[:, 1] = 1.0, 0.0
+    w[:, :16, 0], w[:, 16:, 0] = odd.repeat_interleave(4), odd.repeat(4)
+    w[:, :, 1:] = 0.0
+    ids = torch.arange(rows, dtype=torch.int32) % 2
+    plan = ops.moe_plan(ids.view(-1, 1).to(DEV), 2)
+    alpha, limit, shift = consts
+    g, u = odd.repeat_interleave(4), odd.repeat(4)
+    if limit:                                                         # (fminf and fmaxf return the number of a number and NaN)
+        g, u = torch.fmin(g, torch.tensor(limit)), torch.fmin(torch.fmax(u, torch.tensor(-limit)), torch.tensor(limit))
+    exp = (g / (1 + torch.exp(-alpha * g)) * (u + shift)).bfloat16()
+    xs, ws = x.bfloat16().to(DEV), w.bfloat16().to(DEV)
+    forms = {"own": ops._grouped_tc(xs, ws, plan, 1, 16, *consts), "call": ops.grouped_glu(xs, ws, plan, 1, 16, *consts),
+             "kernel": ops.glu(torch.cat([odd.repeat_interleave(4), odd.repeat(4)])[None].bfloat16().to(DEV), 16, *consts)}
+    for name, got in forms.items():
+        assert torch.allclose(got.float().cpu(), exp.float().expand(len(got), 16), rtol=2.0 ** -7, equal_nan=True), name
+    assert ops.tc_error() == 0
+
+
+@pytest.mark.parametrize("alpha", [1.0, 1.702])
+def test_gated_gate_far_below_zero(ops, alpha):
+    """A gate whose 1 + e^(-alpha g) lies above 2^126 still divides: small, not zero (one rounding to bfloat16; the rest is 2^-21 and below)."""
+    z = torch.tensor([-87.4, -88.0, -88.5, -60.0, -3.0, 2.0, -0.125, -30.0], dtype=torch.float64)
+    parts, rest = [], z / alpha
+    for _ in range(3):                                                # a gate in three bfloat16 pieces
+        parts.append(rest.bfloat16()); rest = rest - parts[-1].double()
+    x, w = torch.zeros(300, 64), torch.zeros(2, 16, 64)
+    x[:, :3] = 1.0
+    for i, p in enumerate(parts):
+        w[:, :8, i] = p.float()
+    w[:, 8:, 0] = 2.0 ** 100
+    plan = ops.moe_plan((torch.arange(300, dtype=torch.int32) % 2).view(-1, 1).to(DEV), 2)
+    got = ops._grouped_tc(x.bfloat16().to(DEV), w.bfloat16().to(DEV), plan, 1, 8, alpha, 0.0, 0.0).double().cpu()
+    g = sum(p.double() for p in parts)
+    assert torch.allclose(got, (g / (1 + torch.exp(-alpha * g)) * 2.0 ** 100).expand(300, 8), rtol=2.0 ** -8, atol=0.0)
+    assert ops.tc_error() == 0
+
+
+def test_gated_unit_in_32_bits(ops):
+    """The unit on gates and up values that are known exactly (one product each): all but a few results are the correctly rounded ones.  Errors of
+    some four units of 2^-24 turn a rounding to 2^-9 one time in four thousand; the fast exponential's twenty would one time in seven hundred."""
+    F = 8192
+    g = torch.Generator().manual_seed(3)
+    x, w = torch.zeros(260, 64), torch.zeros(1, 2 * F, 64)
+    x[:, 0] = 1.0
+    w[0, :F, 0] = (torch.rand(F, generator=g) * 50 - 40)
+    w[0, F:, 0] = torch.randn(F, generator=g)
+    w = w.bfloat16()
+    plan = ops.moe_plan(torch.zeros(260, 1, dtype=torch.int32, device=DEV), 1)
+    got = ops._grouped_tc(x.bfloat16().to(DEV), w.to(DEV), plan, 1, F, 1.702, 0.0, 1.0).cpu()
+    gate, up = w[0, :F, 0].double(), w[0, F:, 0].double()
+    exp = (gate / (1 + torch.exp(-float(torch.tensor(1.702)) * gate)) * (up + 1)).bfloat16()
+    assert torch.equal(got, got[:1].expand_as(got))
+    assert (got[0] != exp).sum().item() <= 6
