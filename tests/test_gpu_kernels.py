@@ -672,6 +672,23 @@ def test_swiglu_product_for_few_rows_is_chosen_by_measurement(ops):
     assert ops.product_timings[("swiglu", 1024, 8192, "few")]["unfused"] < ops.product_timings[("swiglu", 1024, 8192, "few")]["fused"]
 
 
+@pytest.mark.parametrize("order", [(1024, 1100), (1100, 1024)])
+def test_gate_up_form_of_a_portion_does_not_depend_on_the_sizes_met_before(order):
+    """The form that the rule names, bit for bit, whichever of two portions comes first."""
+    from tiny_transformer_inference_engine_b200.ops import CudaOps
+    ops = CudaOps(DEV)
+    F, K = 11008, 2048
+    g = torch.Generator().manual_seed(2)
+    w = (torch.randn(2 * F, K, generator=g) * 0.02).bfloat16().to(DEV)
+    for M in order:
+        x = torch.randn(M, K, generator=g).bfloat16().to(DEV)
+        parts = torch.empty(M, F, dtype=torch.bfloat16, device=DEV)
+        ops.swiglu(ops.linear(x, w, None), parts)
+        fused = ops.linear_swiglu_tc_pair(x, w, None, F)
+        assert not torch.equal(fused, parts)
+        assert torch.equal(ops.linear_swiglu(x, w, None, F), fused if M == 1024 else parts), M
+
+
 def test_partial_sums_feed_norm_and_rope(ops):
     g = torch.Generator().manual_seed(7)
     S, T, d = 3, 5, 200

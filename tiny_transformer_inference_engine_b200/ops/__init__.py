@@ -192,7 +192,7 @@ class CudaOps:
         self._plans = {}
         self.attn_tc_min_rows = 256             # query rows per request from which the tcgen05 attention kernel is used
         self.skinny_max_rows = 8                # rows up to which the weight-streaming product is the rule (tune_products may hand a shape to the library)
-        self._swiglu_choice = {}                # (F, K, row bucket) -> True where the fused tcgen05 gate/up + SwiGLU kernel measured faster
+        self._swiglu_choice = {}                # (F, K, "few") -> True where the weight-streaming product with SwiGLU in its epilogue measured faster
         self._product_choice = {}               # (N, K, row bucket[, "split"]) -> "skinny" | "library" (tune_products; "split": for callers that take partial sums)
         self._skinny_tuned = {}                 # (N, K, row bucket 8 | 16) -> (K range per CTA, form code) where tune_products found a faster form
         self._grouped_mm = None                 # the library's grouped product: None = not looked up yet, False = this build has none
@@ -514,7 +514,7 @@ class CudaOps:
         act = torch.empty((M, hidden), dtype=x.dtype, device=x.device)
         if self._skinny_ok(x, w_gu) and self._fused_few_rows_wins(x, w_gu, b_gu, hidden):
             return self._linear_swiglu_skinny(x, w_gu, b_gu, hidden, act)
-        if M >= 1024 and x.dtype == torch.bfloat16 and self._skinny_shape_ok(x, w_gu) and self._fused_swiglu_wins(x, w_gu, b_gu, hidden):
+        if x.dtype == torch.bfloat16 and self._fused_swiglu_wins(self.num_sms, M, hidden, K) and self._skinny_shape_ok(x, w_gu):
             return self.linear_swiglu_tc_pair(x, w_gu, b_gu, hidden)
         self.swiglu(self.linear(x, w_gu, b_gu), act)
         return act
@@ -585,34 +585,18 @@ class CudaOps:
             self.product_timings[("swiglu",) + key] = took
         return choice
 
-    def _fused_swiglu_wins(self, x, w_gu, b_gu, hidden) -> bool:
-        """Whether, for portions of this many rows, the gate/up product with SwiGLU in its epilogue (this package's
-        tcgen05 kernel on CTA pairs) is faster than the library's product followed by the activation kernel.  Measured
-        the first time a shape and row bucket (1,024 / 2,048 / 4,096 rows and up) is met outside a graph capture: three
-        launches of each between events.  At the Llama-2-7B and Falcon-7B widths the two are within 3 % of each other
-        at 2,048 rows; below 1,024 rows the pair kernel has too few tiles for the GPU and is not considered."""
-        M, K = x.shape
-        key = (hidden, K, 4096 if M >= 4096 else 2048 if M >= 2048 else 1024)
-        choice = self._swiglu_choice.get(key)
-        if choice is None:
-            if torch.cuda.is_current_stream_capturing():
-                return False
-            launches, took = self.launches, {}
-            act = torch.empty((M, hidden), dtype=x.dtype, device=x.device)
-            for kind, fn in (("library", lambda: self.swiglu(self.linear(x, w_gu, b_gu), act)),
-                             ("pair", lambda: self.linear_swiglu_tc_pair(x, w_gu, b_gu, hidden))):
-                fn()
-                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                a.record()
-                for _ in range(3):
-                    fn()
-                b.record()
-                b.synchronize()
-                took[kind] = a.elapsed_time(b)
-            self.launches = launches
-            choice = self._swiglu_choice[key] = took["pair"] < took["library"]
-            self.product_timings[("swiglu",) + key] = took
-        return choice
+    @staticmethod
+    def _fused_swiglu_wins(num_sms, rows, hidden, K) -> bool:
+        """Whether a portion's gate/up product runs with its unit in the epilogue (this package's tcgen05 kernel on CTA pairs) rather than as
+        the library's product and the activation kernel.  By the sizes alone: the two round differently (the second form rounds gate
+        and up to bfloat16 in between), so a stopwatch would make a model's results depend on the process and on the sizes it met first.
+        The pair kernel wins where rows fill its 256-row tiles and the tiles are 4.5 waves of the pairs or more (us, pair | library, gate/up
+        matrices as hidden x K: 2,048 rows 11,008 x 4,096 257 | 261, 16,384 x 2,048 200 | 225, 8,192 x 2,048 106 | 125; 1,024 rows 133 | 146 and
+        137 | 160; 4,096 rows 558 | 607 and 407 | 469), not with fewer (4,096 x 4,096, 1,280 rows 85 | 77), nor with a ragged last tile (2,000
+        rows 293 | 273 and 267 | 228) unless that is one of many (18,176 x 4,544, 5,000 rows 1,269 | 1,469), nor at small K (8,192 x 1,024,
+        2,048 rows 85 | 76)."""
+        tiles, pairs = -(-rows // 256) * -(-hidden // 128), num_sms // 2
+        return rows >= 1024 and K >= 2048 and (2 * tiles >= 9 * pairs if rows % 256 == 0 else tiles >= 30 * pairs)
 
     def swiglu(self, gate_up, out):
         T, F = out.shape
@@ -1702,7 +1686,7 @@ class CudaOps:
         """The gated unit's activation of x @ [Wg; Wu].T (+ ``bias`` [2 * hidden]) -> [M, hidden].  With SwiGLU's constants this is ``linear_swiglu`` and
         its fused forms; with others, up to 8 rows run the weight-streaming product with the unit in its epilogue (where that
         form measured faster for the shape), more rows the product and the activation kernel; gelu without clamps and shift also has
-        the tcgen05 pair product with the unit in its epilogue (1,024 rows and more, where it measured faster)."""
+        the tcgen05 pair product with the unit in its epilogue (``_fused_swiglu_wins``)."""
         plain = not limit and shift == 0.0
         if act == "silu" and alpha == 1.0 and plain:
             return self.linear_swiglu(x, w_gu, bias, hidden)
@@ -1714,8 +1698,8 @@ class CudaOps:
                         "skinny_gemm_glu")
             self.launches += 1
             return out
-        if (act == "gelu_tanh" and plain and M >= 1024 and x.dtype == torch.bfloat16 and self._skinny_shape_ok(x, w_gu)
-                and self._fused_swiglu_wins(x, w_gu, bias, hidden)):
+        if (act == "gelu_tanh" and plain and x.dtype == torch.bfloat16 and self._fused_swiglu_wins(self.num_sms, M, hidden, K)
+                and self._skinny_shape_ok(x, w_gu)):
             return self.linear_swiglu_tc_pair(x, w_gu, bias, hidden, act)
         return self.glu(self.linear(x, w_gu, bias), hidden, alpha, limit, shift, act)
 
