@@ -183,3 +183,45 @@ def test_what_is_not_finite_stays_behind(ops, kind, what):
         walk, walk_states = sc.run(ops)
         assert torch.equal(torch.isfinite(out), torch.isfinite(walk))
         assert torch.equal(torch.isfinite(states[0]), torch.isfinite(walk_states[0]))
+
+
+def class_of(x):
+    return torch.where(x.isnan(), 3, torch.where(x == float("inf"), 1, torch.where(x == float("-inf"), 2, 0)))
+
+
+@pytest.mark.parametrize("D,Dv", [(64, 64), (48, 136), (128, 128)])
+@pytest.mark.parametrize("what", ["v", "k", "q", "S0"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_what_is_not_finite_comes_out_as_the_walk_has_it(ops, kind, what, D, Dv):
+    """Infinities of either sign and NaN, brought by a token or found in the state row: the same infinities and NaN in every read-out and
+    state element as token by token, and the same values elsewhere."""
+    if kind == "wkv":
+        Dv = D
+    for bad in (float("inf"), float("-inf"), float("nan")):
+        sc = Scan(kind, [150, 40, 9], 2, D, Dv, seed=6)
+        if what == "S0":
+            sc.S0[sc.s_at[0], 1, 3, 5] = bad
+        else:
+            getattr(sc, what)[75, (Dv if what == "v" else D) + 6] = bad
+        ops.scan_chunk_tokens = 1
+        out, states = sc.run(ops)
+        ops.scan_chunk_tokens = 1 << 30
+        walk, walk_states = sc.run(ops)
+        for got, want in zip([out] + states, [walk] + walk_states):
+            assert torch.equal(class_of(got), class_of(want)), (bad, got.shape)
+            fine = want.isfinite()
+            assert torch.allclose(got[fine], want[fine], rtol=1e-2, atol=1e-3)
+        assert not out.isfinite().all()
+
+
+def test_retention_chunks_near_the_largest_number(ops):
+    """Keys that round to an infinite bfloat16 and are finite themselves: no plane form, the same sums."""
+    sc = Scan("retention", [150], 2, 64, 64, seed=8, values=torch.float32)
+    sc.k[75, 64 + 6], sc.k[140, 9] = 3.395e38, -3.39e38
+    sc.v[75], sc.v[140] = 2.0 ** -3, 2.0 ** -4
+    sc.q.mul_(2.0 ** -6)
+    ops.scan_chunk_tokens = 1
+    out, (S,) = sc.run(ops)
+    exp, (e,) = sc.exact()
+    assert out.isfinite().all() and S.isfinite().all()
+    assert rel(out * 2.0 ** -100, exp * 2.0 ** -100) < 1e-6 and rel(S * 2.0 ** -100, e * 2.0 ** -100) < 1e-6

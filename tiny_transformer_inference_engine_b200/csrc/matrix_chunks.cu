@@ -11,7 +11,8 @@
 //   chunk_out     per (chunk, head): o_i = (decay to i) S q_i + sum_(j <= i) (decay from j to i) (q_i . k_j) v_j
 //
 // Everything stays 32-bit as in the walk.  The products run on the tensor cores as bfloat16 instructions on operands split into
-// planes: a 32-bit value is the exact sum of three bfloat16 (8 + 8 + 8 bits), so a product of two of them is the six plane products
+// planes: a 32-bit value is the sum of three bfloat16 (8 + 8 + 8 bits; exact from 2^-110, below which the last bits fall under the smallest
+// bfloat16, up to 3.39e38, above which the first plane is infinite), so a product of two of them is the six plane products
 // that matter at 32 bits, in 32-bit sums; a bfloat16 operand is one plane.  Decays are never divided by: every factor is a product of
 // decays over a span of tokens, or the exponential of a difference that cannot be positive, so nothing overflows however strong a
 // decay is.
@@ -25,9 +26,10 @@
 //               its block's end, whole blocks between them as a vector on the rows; inside a block the 136 scores are summed on the
 //               ordinary cores with running products.
 //
-// A row of keys or values that is not finite reaches only its own and later tokens, as in the walk (masked weights are selected, not
-// multiplied, and the one place where a zero weight would meet a later value - a row's own block of 16 - is summed token
-// by token when a value there is not finite).
+// What is not finite has no planes (an infinity leaves inf - inf in the second) and would meet rows and elements that it does not reach, as a
+// zero weight times an infinity.  It always shows in the results, though: a state element of chunk_carry or a read-out of chunk_out that is not
+// finite is computed again token by token, the former for its own element, the latter for its chunk and head, by the walk's operations from the
+// state before the chunk.  So infinities, NaN and sums that overflow come out as the walk has them.
 //
 // Chunks are numbered over the whole step: request s owns the numbers from qsl[s] / 64 + s on, which leaves room for its last
 // partial chunk and needs nothing of the host but the number of tokens and requests.
@@ -57,6 +59,7 @@ struct ChunkArgs {
     const float* pre; long long ld_pre; float cap;                    // mlstm: gate pre-activations [T, 2H]
     const float* decay;                                               // retention [H]; wkv [T, H*D]
     const float* u;                                                   // wkv [H*D]
+    bool v_f32;                                                       // v is float32
     float* S; float* nrm; float* mx; int state_rows;                  // state rows (mlstm: normaliser and running maximum too)
     const void* x; long long ld_x; int d; float* prev; int prev_rows; // wkv: the mixer's input and the rows that keep its last token
     const int* qsl; const int* slot_ids; int num_seqs;
@@ -237,16 +240,123 @@ __device__ __forceinline__ void stage_rows(uint16_t* dst, const E* src, long lon
     }
 }
 
-// rows t0 .. t0 + n - 1, columns col0 .. col0 + 63 of a head's values; `bad`: per 16 tokens, whether a value is not finite
+// rows t0 .. t0 + n - 1, columns col0 .. col0 + 63 of a head's values
 template <typename VT, int VPL, int NT = 128>
-__device__ __forceinline__ void stage_values(uint16_t* v_s, const VT* vp, long long ld, int n, int col0, int Dv, int* bad) {
-    stage_rows<VPL, VT_COLS, VLD, NT>(v_s, vp + col0, ld, [&](int j, int c) { return j < n && col0 + c < Dv; }, [&](int j, const float (&x)[8]) {
-        if (bad == nullptr) return;
-        bool fine = true;
+__device__ __forceinline__ void stage_values(uint16_t* v_s, const VT* vp, long long ld, int n, int col0, int Dv) {
+    stage_rows<VPL, VT_COLS, VLD, NT>(v_s, vp + col0, ld, [&](int j, int c) { return j < n && col0 + c < Dv; }, [](int, float (&)[8]) {});
+}
+
+// log input gate and log forget gate of a token
+__device__ __forceinline__ float2 log_gates(const ChunkArgs& a, int token, int h) {
+    const float* g = a.pre + (size_t)token * a.ld_pre;
+    const float z = a.cap * tanhf(g[a.H + h] / a.cap);
+    return make_float2(a.cap * tanhf(g[h] / a.cap), fminf(z, 0.f) - log1pf(expf(-fabsf(z))));
+}
+
+// ---- the walk's operations, for what is not finite
+__device__ __forceinline__ bool finite4(float x, float y, float z, float w) { return (x - x) + (y - y) + ((z - z) + (w - w)) == 0.f; }
+
+// four state elements (dv, ch .. ch + 3) of a head over the chunk's tokens; normaliser: its elements ch .. ch + 3.  mlstm: m is the running maximum
+// before the chunk, m_end the one that the result is scaled to
+template <int MODE>
+__device__ __forceinline__ float4 walk_state(const ChunkArgs& a, int t0, int n, int h, int dv, int ch, bool normaliser, float4 S4, float m, float m_end) {
+    float S[4] = {S4.x, S4.y, S4.z, S4.w};
+    const float decay = MODE == RET ? a.decay[h] : 0.f;
+#pragma unroll 1
+    for (int t = t0; t < t0 + n; ++t) {
+        const size_t at = (size_t)t * a.ld_v + h * a.Dv + dv;
+        float v = 1.f, fa = decay, ib = 1.f;
+        if (!normaliser) v = a.v_f32 ? reinterpret_cast<const float*>(a.v)[at] : to_f32(reinterpret_cast<const __nv_bfloat16*>(a.v)[at]);
+        if constexpr (MODE == MLSTM) {
+            const float2 g = log_gates(a, t, h);
+            const float next = fmaxf(g.y + m, g.x);
+            fa = expf(g.y + m - next); ib = expf(g.x - next);
+            m = next;
+        }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) fine = fine && isfinite(x[i]);
-        if (!fine) bad[j >> 4] = 1;
-    });
+        for (int i = 0; i < 4; ++i) {
+            const bool in = ch + i < a.D;                                             // (padded channels have keys and decays of zero)
+            const size_t kat = (size_t)t * a.ld_qk + h * a.D + ch + i;
+            const float k = !in ? 0.f : MODE == RET ? reinterpret_cast<const float*>(a.k)[kat] : to_f32(reinterpret_cast<const __nv_bfloat16*>(a.k)[kat]);
+            if constexpr (MODE == WKV) fa = in ? a.decay[(size_t)t * a.H * a.D + h * a.D + ch + i] : 0.f;
+            const float bk = ib * k;
+            S[i] = fmaf(fa, S[i], normaliser ? bk : bk * v);
+        }
+    }
+    if constexpr (MODE == MLSTM) {
+        const float f = expf(m - m_end);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[i] *= f;
+    }
+    return make_float4(S[0], S[1], S[2], S[3]);
+}
+
+// the read-outs of a chunk and head, 128 threads: a thread per value column, eight key channels of its state at a time over all tokens.  `sm`: 7 * CT
+// floats of shared memory that nothing else uses any more
+template <int MODE, typename VT>
+__device__ __forceinline__ void walk_out(const ChunkArgs& a, size_t unit, int t0, int n, int h, float* sm) {
+    using QT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
+    const QT* qp = reinterpret_cast<const QT*>(a.q) + (size_t)t0 * a.ld_qk + h * a.D;
+    const QT* kp = reinterpret_cast<const QT*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
+    const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
+    const size_t ld_o = (size_t)a.H * a.Dv;
+    float* op = a.out + (size_t)t0 * ld_o + h * a.Dv;
+    const int tid = threadIdx.x;
+    float* gate = sm;                                                                 // mlstm: [CT][3] state decay, input weight, e^-m
+    float* den = sm + 3 * CT;                                                         // mlstm: [4][CT] the warps' shares of n . q
+    if constexpr (MODE == MLSTM) {
+        if (tid == 0) {
+            float m = a.mm[unit].x;
+#pragma unroll 1
+            for (int t = 0; t < n; ++t) {
+                const float2 g = log_gates(a, t0 + t, h);
+                const float next = fmaxf(g.y + m, g.x);
+                gate[3 * t] = expf(g.y + m - next); gate[3 * t + 1] = expf(g.x - next); gate[3 * t + 2] = expf(-next);
+                m = next;
+            }
+        }
+        __syncthreads();
+        float nv = tid < a.Dpad ? a.aux[unit * a.Dpad + tid] : 0.f;
+#pragma unroll 1
+        for (int t = 0; t < n; ++t) {
+            const float k = tid < a.D ? to_f32(kp[(size_t)t * a.ld_qk + tid]) : 0.f, q = tid < a.D ? to_f32(qp[(size_t)t * a.ld_qk + tid]) * a.qscale : 0.f;
+            nv = fmaf(gate[3 * t], nv, gate[3 * t + 1] * k);
+            const float p = warp_sum(tid < a.Dpad ? nv * q : 0.f);
+            if ((tid & 31) == 0) den[(tid >> 5) * CT + t] = p;
+        }
+        __syncthreads();
+    }
+    for (int dv = tid; dv < a.Dv; dv += 128) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < a.Dpad; c0 += 8) {
+            const bool in = c0 < a.D;                                                 // (both are multiples of 8)
+            float S[8];
+            load8(a.part + (unit * a.Dv + dv) * a.Dpad + c0, true, S);
+#pragma unroll 1
+            for (int t = 0; t < n; ++t) {
+                float k[8], q[8], acc = 0.f;
+                load8(kp + (size_t)t * a.ld_qk + c0, in, k);
+                load8(qp + (size_t)t * a.ld_qk + c0, in, q);
+                const float v = to_f32(vp[(size_t)t * a.ld_v + dv]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if constexpr (MODE == WKV) {
+                        const float kv = k[i] * v;
+                        acc = fmaf(q[i], fmaf(in ? a.u[h * a.D + c0 + i] : 0.f, kv, S[i]), acc);
+                        S[i] = fmaf(in ? a.decay[(size_t)(t0 + t) * a.H * a.D + h * a.D + c0 + i] : 0.f, S[i], kv);
+                    } else {
+                        S[i] = MODE == RET ? fmaf(a.decay[h], S[i], k[i] * v) : fmaf(gate[3 * t], S[i], gate[3 * t + 1] * k[i] * v);
+                        acc = fmaf(S[i], MODE == MLSTM ? q[i] * a.qscale : q[i], acc);
+                    }
+                }
+                float* o = op + (size_t)t * ld_o + dv;
+                if (c0 > 0) acc += *o;
+                if (MODE == MLSTM && c0 + 8 >= a.Dpad)
+                    acc /= fmaxf(fabsf((den[t] + den[CT + t]) + (den[2 * CT + t] + den[3 * CT + t])), gate[3 * t + 2]) + 1e-6f;
+                *o = acc;
+            }
+        }
+    }
 }
 
 // ---- the matrix memory's gates over a chunk: threads 0 .. 63 (two warps), thread = token.  F: inclusive sum of the log forget gates,
@@ -256,10 +366,9 @@ __device__ __forceinline__ void chunk_gates(const ChunkArgs& a, int t0, int n, i
     double f = 0.0, ig = -INFINITY;
     x = X = 0.0;
     if (j < n) {
-        const float* g = a.pre + (size_t)(t0 + j) * a.ld_pre;
-        ig = (double)(a.cap * tanhf(g[h] / a.cap));
-        const float z = a.cap * tanhf(g[a.H + h] / a.cap);
-        f = (double)(fminf(z, 0.f) - log1pf(expf(-fabsf(z))));
+        const float2 g = log_gates(a, t0 + j, h);
+        ig = (double)g.x;
+        f = (double)g.y;
     }
     F = f;
     if (j < CT) {
@@ -321,7 +430,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
             w[i] = in && j < n ? wp[(size_t)j * a.H * a.D] : 1.f;
             kv[i] = in && j < n ? kp[(size_t)j * a.ld_qk] : __float2bfloat16(0.f);
         }
-        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
+        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv);
         double all = 1.0;
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) all *= (double)w[i];
@@ -343,7 +452,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
             suf *= (double)w[i];
         }
     } else {
-        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv, nullptr);
+        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv);
         if constexpr (MODE == RET) {
             if (tid < CT) wt[tid] = tid < n ? (float)power((double)a.decay[h], n - 1 - tid) : 0.f;
         } else {
@@ -372,7 +481,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
     for (int col0 = 0; col0 < a.Dv; col0 += VT_COLS) {
         if (col0 > 0) {
             __syncthreads();
-            stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, col0, a.Dv, nullptr);
+            stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, col0, a.Dv);
             __syncthreads();
         }
         constexpr int NP = KP / 16 / PARTS;                                           // 16-channel tiles of this warp
@@ -475,6 +584,8 @@ __global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
             if (c0 + i >= c_hi) continue;
             const size_t off = (size_t)(c0 + i - c_lo);
             *reinterpret_cast<float4*>(pp + off * step) = S;
+            const float4 before = S;
+            const double m_before = m;
             float4 f, x = p[b][i];
             if constexpr (MODE == RET) {
                 const float d = powers[c0 + i == c_hi - 1 ? 1 : 0];
@@ -492,6 +603,10 @@ __global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
                 m = next;
             }
             S.x = fmaf(f.x, S.x, x.x); S.y = fmaf(f.y, S.y, x.y); S.z = fmaf(f.z, S.z, x.z); S.w = fmaf(f.w, S.w, x.w);
+            if (!finite4(S.x, S.y, S.z, S.w)) {
+                const int el = in_state ? e : e - state;
+                S = walk_state<MODE>(a, q0 + (c0 + i) * CT, min(CT, len - (c0 + i) * CT), h, in_state ? el / a.Dpad : 0, el % a.Dpad, !in_state, before, (float)m_before, (float)m);
+            }
         }
     };
     fetch(0, c_lo);
@@ -508,7 +623,7 @@ __global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
 template <int MODE, int KP> struct OutSmem {
     static constexpr int LD = KP + 8, FLD = KP + 4;
     static constexpr int EXTRA = MODE == WKV ? (2 * CT * FLD + 4 * KP) * 4 : MODE == MLSTM ? CT * 24 + KP * 4 : (CT + 1 + 3) * 4;
-    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 16 + 64 + EXTRA; }
+    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + EXTRA; }
 };
 
 template <int MODE, int KP, typename VT>
@@ -518,8 +633,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* pl = reinterpret_cast<uint16_t*>(smem_raw);                             // [3][CT][LD]: keys, then 64 columns of the state
     uint16_t* v_s = pl + 3 * CT * LD;                                                 // [VPL][CT][VLD]
-    int* bad = reinterpret_cast<int*>(v_s + VPL * CT * VLD);                          // [4]
-    double* half = reinterpret_cast<double*>(bad + 4);                                // [8]
+    double* half = reinterpret_cast<double*>(v_s + VPL * CT * VLD);                   // [8]
     unsigned char* extra = reinterpret_cast<unsigned char*>(half + 8);
     TTIE_PDL_ENTRY();
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -531,9 +645,8 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
     const QT* kp = reinterpret_cast<const QT*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
     const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
     const int r0 = warp * 16 + g, r1 = r0 + 8;                                        // this lane's rows (tokens of the chunk)
-    if (tid < 4) bad[tid] = 0;
-    __syncthreads();
-    stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv, bad);
+    bool odd = false;                                                                 // something of this lane's is not finite
+    stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv);
 
     // a lane's part of a 16 x 16 piece of the query rows: rows r0 / r1, channels c0 + 2t, + 1 and those + 8
     auto load_q = [&](int c0, float (&f)[8]) {
@@ -738,6 +851,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
             for (int b = 0; b < 2; ++b) {
                 den[b] += __shfl_xor_sync(0xffffffffu, den[b], 1);
                 den[b] += __shfl_xor_sync(0xffffffffu, den[b], 2);
+                odd = odd || ((b ? r1 : r0) < n && !isfinite(den[b]));
                 den[b] = fmaxf(fabsf(den[b] * a.qscale), floor_[b]) + 1e-6f;
             }
         }
@@ -745,11 +859,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 
     for (int col0 = 0; col0 < a.Dv; col0 += VT_COLS) {
         __syncthreads();                                                              // the keys (or the last columns) have been read by everyone
-        if (col0 > 0) {
-            if (tid < 4) bad[tid] = 0;
-            __syncthreads();
-            stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv, bad);
-        }
+        if (col0 > 0) stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv);
         const float* sp = a.part + (unit * a.Dv + col0) * a.Dpad;
         stage_rows<3, KP, LD>(pl, sp, a.Dpad, [&](int j, int ch) { return col0 + j < a.Dv && ch < a.Dpad; }, [](int, float (&)[8]) {});
         __syncthreads();
@@ -776,25 +886,6 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 #pragma unroll
         for (int J = 0; J < 4; ++J) {
             if (J > warp) continue;
-            if (J == warp && bad[J]) {                                                // a value of the rows' own block is not finite: token by token
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float p0 = __shfl_sync(0xffffffffu, P[2 * J + (j >> 3)][j & 1], (lane & 28) + ((j & 7) >> 1));
-                    const float p1 = __shfl_sync(0xffffffffu, P[2 * J + (j >> 3)][2 + (j & 1)], (lane & 28) + ((j & 7) >> 1));
-                    if (J * 16 + j >= n) continue;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-#pragma unroll
-                        for (int b = 0; b < 2; ++b) {
-                            const int col = col0 + i * 8 + 2 * t + b;
-                            if (col >= a.Dv) continue;
-                            const float x = to_f32(vp[(size_t)(J * 16 + j) * a.ld_v + col]);
-                            if (j <= g) acc[i][b] = fmaf(p0, x, acc[i][b]);
-                            if (j <= g + 8) acc[i][2 + b] = fmaf(p1, x, acc[i][2 + b]);
-                        }
-                }
-                continue;
-            }
             uint32_t p[3][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) split3(P[2 * J + (i >> 1)][(i & 1) * 2], P[2 * J + (i >> 1)][(i & 1) * 2 + 1], p[0][i], p[1][i], p[2][i]);
@@ -818,8 +909,10 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
             }
             if (r0 < n) *reinterpret_cast<float2*>(op + (size_t)r0 * ld_o + col) = make_float2(y[0], y[1]);
             if (r1 < n) *reinterpret_cast<float2*>(op + (size_t)r1 * ld_o + col) = make_float2(y[2], y[3]);
+            odd = odd || (r0 < n && !finite4(y[0], y[1], 0.f, 0.f)) || (r1 < n && !finite4(y[2], y[3], 0.f, 0.f));
         }
     }
+    if (__syncthreads_or(odd)) walk_out<MODE, VT>(a, unit, t0, n, h, reinterpret_cast<float*>(pl));
 }
 
 template <int MODE, int KP, typename VT>
@@ -856,6 +949,7 @@ extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long l
     if (slots < 1 || H > 65535 || num_seqs > 65535) TTIE_FAIL("matrix_chunks: %d chunks a pass, %d heads, %d requests", slots, H, num_seqs);
     ChunkArgs a = {};
     a.q = q; a.k = k; a.ld_qk = ld_qk; a.v = v; a.ld_v = ld_v; a.pre = pre; a.ld_pre = ld_pre; a.cap = cap; a.decay = decay; a.u = u;
+    a.v_f32 = v_dtype == kF32;
     a.S = S; a.nrm = nrm; a.mx = mx; a.state_rows = state_rows; a.x = x; a.ld_x = ld_x; a.d = d; a.prev = prev; a.prev_rows = prev_rows;
     a.qsl = qsl; a.slot_ids = slot_ids; a.num_seqs = num_seqs; a.out = out; a.H = H; a.D = D; a.Dv = Dv; a.Dpad = Dpad; a.qscale = qscale;
     a.part = part; a.aux = aux; a.span = (double2*)span; a.mm = (float2*)mm;
