@@ -225,3 +225,22 @@ def test_retention_chunks_near_the_largest_number(ops):
     exp, (e,) = sc.exact()
     assert out.isfinite().all() and S.isfinite().all()
     assert rel(out * 2.0 ** -100, exp * 2.0 ** -100) < 1e-6 and rel(S * 2.0 ** -100, e * 2.0 ** -100) < 1e-6
+
+
+@pytest.mark.parametrize("lens", [[1000], [40], [129, 5, 127]])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lo,hi", [(0.0, 3.0), (-8.0, 5.0), (-6.0, 0.5), (-8.0, -6.0)])
+def test_wkv_state_is_no_further_off_than_the_walks(ops, lens, D, lo, hi):
+    """Decays exp(-exp(x)), x between lo and hi: from ones that leave the last token alone to ones that forget little.  The walk rounds once a
+    token and ends with a rounding that nothing can spare; the chunks' state may not be further from 64 bits (a tenth for chance)."""
+    sc = Scan("wkv", lens, 4, D, D, seed=7)
+    g = torch.Generator(device=DEV)
+    g.manual_seed(8)
+    sc.w = torch.exp(-torch.exp(torch.rand(sc.w.shape, generator=g, device=DEV) * (hi - lo) + lo))
+    ops.scan_chunk_tokens = 1
+    out, states = sc.run(ops)
+    exp, exp_states = sc.exact()
+    ops.scan_chunk_tokens = 1 << 30
+    walk, walk_states = sc.run(ops)
+    assert rel(states[0], exp_states[0]) < 1.1 * rel(walk_states[0], exp_states[0])
+    assert rel(out, exp) < 1.1 * rel(walk, exp)

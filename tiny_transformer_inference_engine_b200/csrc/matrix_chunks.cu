@@ -40,7 +40,7 @@
 // kernels were 39 and 87 with half the threads in the sum (a run of 32 tokens' decays per thread is one serial chain of loads and
 // multiplications in 64 bits) and two blocks of out per SM instead of three.
 // Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
-// 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 3.9e-8 (4.4e-8).
+// 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 3.4e-8 (4.5e-8).
 #include "common.cuh"
 #include "run_reduce.cuh"
 #include <math.h>
@@ -153,7 +153,7 @@ __device__ __forceinline__ void mma_planes(float (&c0)[4], float (&c1)[4], const
 }
 // The same for one plane of A and three of B, closer still: the leading products eight at a time, and what rounding the running sum
 // leaves kept beside it (two-sum), with the small planes; acc + left is the result.  The wkv chunk sums take it, whose walk rounds once a
-// token: the state's error against 64 bits 4.6e-8 -> 3.9e-8 (the walk's 4.4e-8) for 4 us of 30.
+// token: the state's error against 64 bits 4.6e-8 -> 3.9e-8 (the walk's 4.5e-8) for 4 us of 30, before the last tokens were summed apart.
 __device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b));
@@ -392,26 +392,38 @@ __device__ __forceinline__ void chunk_gates(const ChunkArgs& a, int t0, int n, i
 }
 
 // ------------------------------------------------------------------------------------------- chunk_sum
+// wkv: the chunk's last tokens are added in 64 bits on the ordinary cores, behind the tensor cores' sum of the others.  Under strong decays
+// they are the state, and what the tensor cores cut from products of very different sizes showed there: decays of e^-1 to e^-20 a token
+// 3.9e-8 without this, 2.0e-8 with it and walked; e^-0.0003 to e^-150 3.5e-8, 2.2e-8, walked 3.2e-8.  4 us of the mixer's 240 (2,048 tokens).
+constexpr int TAIL = 8;
 template <int MODE, int KP> struct SumSmem {
     static constexpr int LD = KP + 8;
     static constexpr int NT = MODE == WKV ? 256 : 128;               // wkv: a thread per channel and run of tokens, so more of them
-    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + (MODE == WKV ? NT * 8 : CT * 4); }
+    static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + (MODE == WKV ? (NT + TAIL * (KP + VT_COLS)) * 8 : CT * 4); }
 };
 
 template <int MODE, int KP, typename VT>
-__global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const ChunkArgs a) {
+__global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64 ? 3 : 0) chunk_sum_kernel(const ChunkArgs a) {
     constexpr int NT = SumSmem<MODE, KP>::NT, PARTS = NT / 128, LD = KP + 8, VPL = sizeof(VT) == 4 ? 3 : 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* kd = reinterpret_cast<uint16_t*>(smem_raw);                             // [3][CT][LD]: decayed keys
     uint16_t* v_s = kd + 3 * CT * LD;                                                 // [VPL][CT][VLD]
     double* half = reinterpret_cast<double*>(v_s + VPL * CT * VLD);                   // [8]
     float* wt = reinterpret_cast<float*>(half + 8);                                   // [CT]: a token's weight at the chunk's end
+    double* k_tail = half + 8 + NT;                                                   // wkv: [TAIL][KP] decayed keys of the last tokens (oldest first)
+    double* v_tail = k_tail + TAIL * KP;                                              // wkv: [TAIL][VT_COLS] their values
     TTIE_PDL_ENTRY();
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 3, part = tid >> 7;      // (part: which share of the key channels)
     int s, c, t0, n;
     if (!find_chunk(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
     const size_t unit = (size_t)blockIdx.x * a.H + h;
     const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
+    auto stage_tail = [&](int col0) {
+        for (int e = tid; e < TAIL * VT_COLS; e += NT) {
+            const int j = n - TAIL + e / VT_COLS, col = col0 + e % VT_COLS;
+            v_tail[e] = j >= 0 && col < a.Dv ? (double)to_f32(vp[(size_t)j * a.ld_v + col]) : 0.0;
+        }
+    };
 
     if constexpr (MODE == WKV) {
         // a thread per channel and run of LEN tokens: the decays of the run, its product, then keys times the decays behind them (products
@@ -431,6 +443,8 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
             kv[i] = in && j < n ? kp[(size_t)j * a.ld_qk] : __float2bfloat16(0.f);
         }
         stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv);
+        stage_tail(0);
+        for (int e = tid; e < (TAIL - n) * KP; e += NT) k_tail[e] = 0.0;              // (fewer tokens than that)
         double all = 1.0;
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) all *= (double)w[i];
@@ -448,7 +462,10 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) {
             const int j = run * LEN + i;
-            split3((double)to_f32(kv[i]) * suf, kd[j * LD + ch], kd[CT * LD + j * LD + ch], kd[2 * CT * LD + j * LD + ch]);
+            const double x = (double)to_f32(kv[i]) * suf;
+            const bool last = j >= n - TAIL && j < n;
+            if (last) k_tail[(j - (n - TAIL)) * KP + ch] = x;
+            split3(last ? 0.0 : x, kd[j * LD + ch], kd[CT * LD + j * LD + ch], kd[2 * CT * LD + j * LD + ch]);
             suf *= (double)w[i];
         }
     } else {
@@ -482,6 +499,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
         if (col0 > 0) {
             __syncthreads();
             stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, col0, a.Dv);
+            if constexpr (MODE == WKV) stage_tail(col0);
             __syncthreads();
         }
         constexpr int NP = KP / 16 / PARTS;                                           // 16-channel tiles of this warp
@@ -509,9 +527,22 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT) chunk_sum_kernel(const 
         }
         if constexpr (MODE == WKV) {
 #pragma unroll
-            for (int i = 0; i < 2 * NP; ++i)
+            for (int i = 0; i < 2 * NP; ++i) {
+                double sum[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) if (fabsf(acc[i][j]) < INFINITY) acc[i][j] += left[i][j];      // (behind an overflow it holds inf - inf)
+                for (int j = 0; j < 4; ++j) sum[j] = (double)acc[i][j] + (double)left[i][j];
+                const double* kt = k_tail + (part * NP * 2 + i) * 8 + 2 * t;
+                const double* vt = v_tail + warp * 16 + g;
+#pragma unroll
+                for (int r = 0; r < TAIL; ++r) {
+                    const double2 k = *reinterpret_cast<const double2*>(kt + r * KP);
+                    const double v0 = vt[r * VT_COLS], v1 = vt[r * VT_COLS + 8];
+                    sum[0] = fma(v0, k.x, sum[0]); sum[1] = fma(v0, k.y, sum[1]);
+                    sum[2] = fma(v1, k.x, sum[2]); sum[3] = fma(v1, k.y, sum[3]);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = (float)sum[j];
+            }
         }
         float* dst = a.part + (unit * a.Dv + col0 + warp * 16) * a.Dpad;
 #pragma unroll
