@@ -1,5 +1,6 @@
-"""Which form of the gate/up product a prompt portion takes: by its sizes alone."""
+"""Which form a product or a scan takes: by the sizes of the step alone."""
 import pytest
+import torch
 
 from tiny_transformer_inference_engine_b200.ops import CudaOps
 
@@ -12,3 +13,44 @@ from tiny_transformer_inference_engine_b200.ops import CudaOps
 ])
 def test_gate_up_form_by_sizes(rows, hidden, K, fused):
     assert CudaOps._fused_swiglu_wins(148, rows, hidden, K) is fused
+
+
+RETENTION, MLSTM, WKV = 0, 1, 2
+
+
+def in_chunks(mode, lens, width, known=True, dtype=torch.bfloat16, dim=None, stride=0, at=0):
+    """The decision for a step of requests that bring these many tokens, at the layer sizes of a width."""
+    heads, k, v = {RETENTION: (width // 128, 128, 128), MLSTM: (width // 128, 64, 128), WKV: (width // 64, 64, 64)}[mode]
+    k = dim or k
+    T = sum(lens)
+    qk_type = torch.float32 if mode == RETENTION else dtype
+    rows = lambda n, t: torch.empty_strided((T, n), (n + stride, 1), dtype=t)
+    q, vals = rows(heads * k + at, qk_type)[:, at:], rows(heads * v, dtype)
+    ops = CudaOps.__new__(CudaOps)
+    return ops._in_chunks(mode, T, len(lens), max(lens) if known else None, heads, k, v, q, q, vals)
+
+
+# (what a step brings, kind, width) and whether chunks were measured ahead by enough to pay for their call
+@pytest.mark.parametrize("mode,lens,width,chunks", [
+    (RETENTION, [128], 2048, False), (RETENTION, [512], 2048, True), (RETENTION, [192], 512, False), (RETENTION, [2048], 1024, True),
+    (MLSTM, [128], 2048, False), (MLSTM, [256], 2048, True), (WKV, [160], 2048, False), (WKV, [512], 2048, True),
+    (RETENTION, [16] * 8, 2048, False), (RETENTION, [32] * 8, 512, False), (MLSTM, [32] * 8, 2048, False), (WKV, [64] * 8, 1024, False),      # short prompts
+    (RETENTION, [64] * 8, 2048, True), (MLSTM, [128] * 8, 2048, True), (RETENTION, [128] * 24, 1024, True),                # many: work, not length
+    (RETENTION, [1] * 23 + [192], 2048, False), (WKV, [1] * 23 + [256], 2048, False), (MLSTM, [1] * 7 + [512], 2048, True), (RETENTION, [1] * 23 + [256], 4096, False),
+    (RETENTION, [1] * 256, 2048, False), (WKV, [1] * 64, 4096, False), (MLSTM, [1], 512, False),                          # decoded tokens
+])
+def test_scans_in_chunks_by_cost(mode, lens, width, chunks):
+    assert in_chunks(mode, lens, width) is chunks
+
+
+def test_scans_in_chunks_without_the_longest_request():
+    """A caller that does not say what the longest request brings: the step's tokens less one for every other request."""
+    assert in_chunks(WKV, [512], 2048, known=False) and in_chunks(WKV, [1] * 7 + [512], 2048, known=False)
+    assert in_chunks(WKV, [64] * 8, 1024, known=False) and not in_chunks(WKV, [64] * 8, 1024)
+
+
+@pytest.mark.parametrize("mode", [RETENTION, MLSTM, WKV])
+def test_scans_in_chunks_only_for_rows_and_heads_that_fit(mode):
+    assert in_chunks(mode, [1024], 2048)
+    assert not in_chunks(mode, [1024], 2048, dim=136) and not in_chunks(mode, [1024], 2048, dim=20) and not in_chunks(mode, [1024], 2048, dim=4)
+    assert not in_chunks(mode, [1024], 2048, stride=2) and not in_chunks(mode, [1024], 2048, at=2)

@@ -1314,16 +1314,16 @@ class CudaOps:
         self.launches += 1
         return out
 
-    def wkv_scan(self, r, k, v, decay, u, state, x, prev, query_start_loc, slot_ids, num_seqs, num_heads, dim):
+    def wkv_scan(self, r, k, v, decay, u, state, x, prev, query_start_loc, slot_ids, num_seqs, num_heads, dim, max_q_len=None):
         """The time mix's recurrence over the step's tokens from the state rows ``state`` [slots + 1, H, dim, padded dim]
         (advanced in place): o_t = (S + diag(u) k v^T)^T r, then S <- diag(w) S + k v^T.  r, k, v [T, H*dim] views with one row
         stride; ``decay`` (w) float32 [T, H*dim] contiguous.  Also stores each request's last row of ``x`` into ``prev``.
-        Returns o float32 [T, H*dim]."""
+        ``max_q_len``: the most tokens a request brings, if known (``_in_chunks``).  Returns o float32 [T, H*dim]."""
         T = r.shape[0]
         out = torch.empty((T, num_heads * dim), dtype=torch.float32, device=r.device)
         if not (r.stride(0) == k.stride(0) == v.stride(0)):
             raise KernelError("wkv_scan: r, k and v must share a row stride")
-        if r.dtype == torch.bfloat16 and self._in_chunks(T, num_seqs, dim, dim, r, k, v):
+        if r.dtype == torch.bfloat16 and self._in_chunks(2, T, num_seqs, max_q_len, num_heads, dim, dim, r, k, v):
             self._matrix_chunks(2, r, k, v, None, 0.0, decay, u, state, None, None, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, dim, 1.0)
             return out
         self._check(self.lib.ttie_wkv_scan(_ptr(r), _ptr(k), _ptr(v), r.stride(0), _ptr(decay), _ptr(u),
@@ -1362,9 +1362,10 @@ class CudaOps:
         self.launches += 1
         return out
 
-    def mlstm_in_chunks(self, q, k, v, num_seqs, dim, v_dim):
+    def mlstm_in_chunks(self, q, k, v, num_seqs, dim, v_dim, max_q_len=None):
         """Whether ``mlstm_chunks`` takes this step (in place of ``mlstm_gates`` and ``mlstm_scan``)."""
-        return q.dtype == torch.bfloat16 and q.stride(0) == k.stride(0) == v.stride(0) and self._in_chunks(q.shape[0], num_seqs, dim, v_dim, q, k, v)
+        return (q.dtype == torch.bfloat16 and self._in_chunks(1, q.shape[0], num_seqs, max_q_len, q.shape[1] // dim, dim, v_dim, q, k, v)
+                and q.stride(0) == k.stride(0) == v.stride(0))
 
     def mlstm_chunks(self, q, k, v, pre, S, n, m, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, cap, q_scale):
         """The matrix memory over a step with a prompt portion, in chunks of 64 tokens: ``mlstm_gates`` and ``mlstm_scan`` in one.  ``pre``:
@@ -1373,21 +1374,42 @@ class CudaOps:
         self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale)
         return out
 
-    scan_chunk_tokens = 160                 # tokens that one request of a step may bring from which the matrix-state scans run in chunks,
-    scan_chunk_more = 12                    # and how many more for every other request;
+    scan_chunk_tokens = None                # None: by cost (``_in_chunks``); a number: chunks where a request may bring this many tokens
+    scan_chunk_more = 0                     # and this many more for every other request
     scan_chunk_bytes = 128 << 20            # bytes of the states between chunks that are held at a time (about the L2: a longer step runs in passes)
+    # us of a scan in chunks by kind (retention, mlstm, wkv): the launches, a request, a state element of a request, a token and state element
+    scan_chunk_cost = ((31.0, 0.3, 8.5e-6, 1.6e-7), (24.0, 0.3, 7.5e-6, 1.6e-7), (28.0, 0.3, 1.45e-5, 3.6e-7))
+    scan_walk_cost = (4.0, 0.19, 8.2e-7)    # of a walk: the launch, a token of the longest request, a token and state element of the whole step
+    scan_chunk_gain = 10.0                  # us by which chunks have to be ahead: about what the call with its three launches costs the host more
 
-    def _in_chunks(self, num_tokens, num_seqs, dim, v_dim, q, k, v) -> bool:
+    def _in_chunks(self, mode, num_tokens, num_seqs, longest, num_heads, dim, v_dim, q, k, v) -> bool:
         """Whether a step's matrix-state recurrence runs in chunks of 64 tokens on tensor cores (``csrc/matrix_chunks.cu``) rather than
-        token by token: a request may bring enough tokens (the step's tokens less one for every other request: the
-        host knows no more, and the number holds for a captured graph), and the head sizes and rows are what 16-byte loads and
-        16-channel products take.  Measured at width 2,048: the walk takes 0.17 to 0.23 us a token of the longest request and 0.3 to 0.9 us a
-        request, chunks 32 to 36 us (mlstm 25) and 1.4 to 2.9 us for every further request, so they meet at 160 tokens (mlstm 120) of a
-        lone request and some 10 tokens later for each further one (one request of 128 tokens: retention 41.8 us in chunks, 30.5
-        walked; beside 7 decoding requests 58.6 and 40.5; of 2,048 tokens 100 and 514)."""
-        others = int(num_seqs) - 1
-        return (num_tokens - others >= self.scan_chunk_tokens + self.scan_chunk_more * others and 8 <= dim <= 128 and dim % 8 == 0 and v_dim % 8 == 0
-                and all(t.stride(1) == 1 and t.stride(0) * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
+        token by token, for the head sizes and rows that 16-byte loads and 16-channel products take.  ``longest``: the most tokens that a request brings
+        (StepContext.max_q_len, which also holds for a captured graph); None: the step's tokens less one for every other request.
+
+        A walk takes its time from the longest request's chain of tokens or from the whole step's work on the state elements,
+        whichever is longer; chunks have three launches, a state to load and store per request and less work per token.  The
+        figures above give both within a fifth over widths of 512 to 4,096, 1 to 24 requests and 16 to 1,024 tokens.  Walk | chunks,
+        us, width 2,048: one request of 128 tokens retention 32 | 40, mlstm 31 | 30, wkv 26 | 34, of 512 tokens 116 | 49, 107 | 34,
+        93 | 41; eight of 16 tokens 30 | 54, 22 | 36, 17 | 41, of 64 tokens 97 | 60, 68 | 41, 55 | 44; 256 tokens beside 23 decoding
+        requests 88 | 85, 81 | 52, 63 | 87."""
+        if not 8 <= dim <= 128 or dim % 8 or v_dim % 8:
+            return False
+        others = num_seqs - 1
+        if longest is None:
+            longest = num_tokens - others
+        if self.scan_chunk_tokens is None:
+            state, (start, token, work), (base, request, element, each) = num_heads * dim * v_dim, self.scan_walk_cost, self.scan_chunk_cost[mode]
+            walk = start + max(token * longest, work * num_tokens * state)
+            if walk < self.scan_chunk_gain + base + num_seqs * (request + element * state) + each * num_tokens * state:
+                return False
+        elif longest < self.scan_chunk_tokens + self.scan_chunk_more * others:
+            return False
+        for t in (q, k, v):
+            row, step = t.stride()
+            if step != 1 or row * t.element_size() % 16 or t.data_ptr() % 16:
+                return False
+        return True
 
     def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale):
         T, pad, dev = q.shape[0], S.shape[-1], q.device
@@ -1416,12 +1438,13 @@ class CudaOps:
         self.launches += 1
         return out
 
-    def retention_scan(self, q, k, v, decay, S, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim):
+    def retention_scan(self, q, k, v, decay, S, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, max_q_len=None):
         """Retention's recurrence over the step's tokens from the state rows S [slots + 1, H, v_dim, padded dim] (advanced in
         place): S <- decay_h S + k v^T, o = S^T q.  q, k float32 [T, H*dim] views with one row stride; v [T, H*v_dim] in the
-        compute dtype, a view with a row stride; ``decay`` float32 [H].  Returns o float32 [T, H*v_dim].
+        compute dtype, a view with a row stride; ``decay`` float32 [H].  ``max_q_len``: the most tokens a request brings, if known.
+        Returns o float32 [T, H*v_dim].
 
-        A step that may hold a prompt portion runs in chunks of 64 tokens (``_in_chunks``).  Head sizes that those do not take are walked
+        A step with a prompt portion runs in chunks of 64 tokens (``_in_chunks``).  Head sizes that those do not take are walked
         token by token, and a long prompt (the step's tokens less one for every other request: the host knows no more, and
         the number holds for a captured graph) in ``parts`` (``retention_parts``) by two launches: the decay is a
         constant, so every part's own sum needs no other part and the parts' first states follow from those sums."""
@@ -1429,7 +1452,7 @@ class CudaOps:
         out = torch.empty((T, num_heads * v_dim), dtype=torch.float32, device=q.device)
         if q.stride(0) != k.stride(0) or q.dtype != torch.float32 or k.dtype != torch.float32:
             raise KernelError("retention_scan: q and k must be float32 and share a row stride")
-        if self._in_chunks(T, num_seqs, dim, v_dim, q, k, v):
+        if self._in_chunks(0, T, num_seqs, max_q_len, num_heads, dim, v_dim, q, k, v):
             self._matrix_chunks(0, q, k, v, None, 0.0, decay, None, S, None, None, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, 1.0)
             return out
         parts = self.retention_parts(T, int(num_seqs), S[0].numel())

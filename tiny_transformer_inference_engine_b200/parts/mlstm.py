@@ -74,7 +74,7 @@ class MLSTM(Mixer):
         proj = ops.linear(x, self.w_in, None)                                                  # [T, q | k | v | g]
         gates = ops.linear(x, self.w_gates, self.b_gates, out_dtype=torch.float32)             # [T, 2H] float32
         q, k, v, g = proj[:, :H * D], proj[:, H * D:2 * H * D], proj[:, 2 * H * D:2 * H * D + H * Dv], proj[:, 2 * H * D + H * Dv:]
-        if hasattr(ops, "mlstm_chunks") and ops.mlstm_in_chunks(q, k, v, ctx.num_seqs, D, Dv):
+        if hasattr(ops, "mlstm_chunks") and ops.mlstm_in_chunks(q, k, v, ctx.num_seqs, D, Dv, ctx.max_q_len):
             o = ops.mlstm_chunks(q, k, v, gates, S.state, nrm.state, mx.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, Dv,
                                  self.gate_cap, D ** -0.5)
         else:
