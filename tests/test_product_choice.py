@@ -33,7 +33,7 @@ def in_chunks(mode, lens, width, known=True, dtype=torch.bfloat16, dim=None, str
 # (what a step brings, kind, width) and whether chunks were measured ahead by enough to pay for their call
 @pytest.mark.parametrize("mode,lens,width,chunks", [
     (RETENTION, [128], 2048, False), (RETENTION, [512], 2048, True), (RETENTION, [192], 512, False), (RETENTION, [2048], 1024, True),
-    (MLSTM, [128], 2048, False), (MLSTM, [256], 2048, True), (WKV, [160], 2048, False), (WKV, [512], 2048, True),
+    (MLSTM, [128], 2048, False), (MLSTM, [256], 2048, False), (MLSTM, [400], 2048, True), (WKV, [160], 2048, False), (WKV, [512], 2048, True), (WKV, [300], 1024, False), (WKV, [500], 1024, True), (RETENTION, [300], 1024, True),
     (RETENTION, [16] * 8, 2048, False), (RETENTION, [32] * 8, 512, False), (MLSTM, [32] * 8, 2048, False), (WKV, [64] * 8, 1024, False),      # short prompts
     (RETENTION, [64] * 8, 2048, True), (MLSTM, [128] * 8, 2048, True), (RETENTION, [128] * 24, 1024, True),                # many: work, not length
     (RETENTION, [1] * 23 + [192], 2048, False), (WKV, [1] * 23 + [256], 2048, False), (MLSTM, [1] * 7 + [512], 2048, True), (RETENTION, [1] * 23 + [256], 4096, False),
@@ -46,7 +46,7 @@ def test_scans_in_chunks_by_cost(mode, lens, width, chunks):
 def test_scans_in_chunks_without_the_longest_request():
     """A caller that does not say what the longest request brings: the step's tokens less one for every other request."""
     assert in_chunks(WKV, [512], 2048, known=False) and in_chunks(WKV, [1] * 7 + [512], 2048, known=False)
-    assert in_chunks(WKV, [64] * 8, 1024, known=False) and not in_chunks(WKV, [64] * 8, 1024)
+    assert in_chunks(WKV, [120] * 8, 1024, known=False) and not in_chunks(WKV, [120] * 8, 1024)
 
 
 @pytest.mark.parametrize("mode", [RETENTION, MLSTM, WKV])

@@ -950,8 +950,13 @@ template <int MODE, int KP, typename VT>
 int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
     constexpr int VPL = sizeof(VT) == 4 ? 3 : 1;
     const size_t sum_smem = SumSmem<MODE, KP>::bytes(VPL), out_smem = OutSmem<MODE, KP>::bytes(VPL);
-    cudaFuncSetAttribute(chunk_sum_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
-    cudaFuncSetAttribute(chunk_out_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+    static bool allowed[64] = {false};
+    int dev = 64;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64 || !allowed[dev]) {
+        cudaFuncSetAttribute(chunk_sum_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
+        cudaFuncSetAttribute(chunk_out_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+        if (dev < 64) allowed[dev] = true;
+    }
     a.slot_lo = first; a.slots = slots;
     const dim3 grid(slots, a.H);
     const dim3 carry(ceil_div(a.Dv * a.Dpad + (MODE == MLSTM ? a.Dpad : 0), 4 * CARRY), a.H, a.num_seqs);

@@ -1379,8 +1379,9 @@ class CudaOps:
     scan_chunk_bytes = 128 << 20            # bytes of the states between chunks that are held at a time (about the L2: a longer step runs in passes)
     # us of a scan in chunks by kind (retention, mlstm, wkv): the launches, a request, a state element of a request, a token and state element
     scan_chunk_cost = ((31.0, 0.3, 8.5e-6, 1.6e-7), (24.0, 0.3, 7.5e-6, 1.6e-7), (28.0, 0.3, 1.45e-5, 3.6e-7))
-    scan_walk_cost = (4.0, 0.19, 8.2e-7)    # of a walk: the launch, a token of the longest request, a token and state element of the whole step
-    scan_chunk_gain = 10.0                  # us by which chunks have to be ahead: about what the call with its three launches costs the host more
+    scan_walk_cost = ((4.0, 0.21, 8.2e-7), (4.0, 0.19, 8.2e-7), (4.0, 0.18, 8.2e-7))   # of a walk: the launch, a token of the longest request, a token and state element of the step
+    # of the layer's eager pass around it: host us with a walk, what chunks' call adds; us of its other kernels, a token and squared width of them
+    scan_pass_cost = ((90.0, 10.0, 35.0, 6e-9), (110.0, 2.0, 35.0, 6e-9), (126.0, 14.0, 60.0, 6e-9))
 
     def _in_chunks(self, mode, num_tokens, num_seqs, longest, num_heads, dim, v_dim, q, k, v) -> bool:
         """Whether a step's matrix-state recurrence runs in chunks of 64 tokens on tensor cores (``csrc/matrix_chunks.cu``) rather than
@@ -1389,7 +1390,9 @@ class CudaOps:
 
         A walk takes its time from the longest request's chain of tokens or from the whole step's work on the state elements,
         whichever is longer; chunks have three launches, a state to load and store per request and less work per token.  The
-        figures above give both within a fifth over widths of 512 to 4,096, 1 to 24 requests and 16 to 1,024 tokens.  Walk | chunks,
+        figures above give both within a fifth over widths of 512 to 4,096, 1 to 24 requests and 16 to 1,024 tokens.  And an eager pass of the layer
+        takes the longer of its kernels' and its host's time, of which chunks need more: they pay where the pass is shorter with them
+        (the whole mixer of 300 tokens at width 1,024, walk | chunks: retention 105 | 99, mlstm 108 | 111, wkv 126 | 141).  The scan alone, walk | chunks,
         us, width 2,048: one request of 128 tokens retention 32 | 40, mlstm 31 | 30, wkv 26 | 34, of 512 tokens 116 | 49, 107 | 34,
         93 | 41; eight of 16 tokens 30 | 54, 22 | 36, 17 | 41, of 64 tokens 97 | 60, 68 | 41, 55 | 44; 256 tokens beside 23 decoding
         requests 88 | 85, 81 | 52, 63 | 87."""
@@ -1399,9 +1402,11 @@ class CudaOps:
         if longest is None:
             longest = num_tokens - others
         if self.scan_chunk_tokens is None:
-            state, (start, token, work), (base, request, element, each) = num_heads * dim * v_dim, self.scan_walk_cost, self.scan_chunk_cost[mode]
-            walk = start + max(token * longest, work * num_tokens * state)
-            if walk < self.scan_chunk_gain + base + num_seqs * (request + element * state) + each * num_tokens * state:
+            state, (start, token, work), (base, request, element, each) = num_heads * dim * v_dim, self.scan_walk_cost[mode], self.scan_chunk_cost[mode]
+            host, more, rest, product = self.scan_pass_cost[mode]
+            rest += product * num_tokens * (num_heads * v_dim) ** 2
+            walk = start + max(token * longest, work * num_tokens * state) + rest
+            if walk <= host or walk <= max(host + more, base + num_seqs * (request + element * state) + each * num_tokens * state + rest):
                 return False
         elif longest < self.scan_chunk_tokens + self.scan_chunk_more * others:
             return False
@@ -1412,19 +1417,21 @@ class CudaOps:
         return True
 
     def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale):
-        T, pad, dev = q.shape[0], S.shape[-1], q.device
-        total = T // 64 + int(num_seqs)                                # chunk numbers of the step
-        slots = max(1, min(total, self.scan_chunk_bytes // (num_heads * v_dim * pad * 4)))
-        part = torch.empty((slots, num_heads, v_dim, pad), dtype=torch.float32, device=dev)
-        aux = torch.empty((slots, num_heads, mode, pad), dtype=torch.float32, device=dev) if mode else None
-        span = torch.empty((slots, num_heads, 2), dtype=torch.float64, device=dev) if mode == 1 else None
-        mm = torch.empty((slots, num_heads, 2), dtype=torch.float32, device=dev) if mode == 1 else None
+        T, pad = q.shape[0], S.shape[-1]
+        total = T // 64 + num_seqs                                     # chunk numbers of the step
+        states = num_heads * v_dim * pad                               # floats of a chunk number: its states, their sums or decays, mlstm: spans and maxima
+        slots = max(1, min(total, self.scan_chunk_bytes // (states * 4)))
+        sums = num_heads * mode * pad
+        space = torch.empty(slots * (states + sums + (6 * num_heads if mode == 1 else 0)), dtype=torch.float32, device=q.device)
+        part = space.data_ptr()
+        aux = part + 4 * slots * states
+        span = aux + 4 * slots * sums
         self._check(self.lib.ttie_matrix_chunks(
             mode, _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), self._dt(v), _ptr(pre), 0 if pre is None else pre.stride(0), float(cap),
             _ptr(decay), _ptr(u), _ptr(S), _ptr(n), _ptr(m), S.shape[0], _ptr(x), 0 if x is None else x.stride(0), 0 if x is None else x.shape[1],
             _ptr(prev), 0 if prev is None else prev.shape[0], _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), T, _ptr(out), num_heads, dim,
-            v_dim, pad, float(q_scale), _ptr(part), _ptr(aux), _ptr(span), _ptr(mm), slots, self._stream(q)), "matrix_chunks")
-        self.launches += 3 * math.ceil(total / slots)
+            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, self._stream(q)), "matrix_chunks")
+        self.launches += 3 * -(-total // slots)
 
     def rotate_heads(self, src, heads, dim, cs_table, rot, style, scale_from=None, scale=1.0):
         """float32 [T, heads * dim]: the ``heads`` head rows of ``dim`` values at the start of every row of ``src`` (a view with a
