@@ -58,6 +58,17 @@ class Scan:
             self.w = torch.exp(-torch.exp(torch.rand(T, H * D, generator=g, device=DEV) * (13.0 if strong else 6.5) - (8.0 if strong else 6.0)))
             self.u, self.x, self.prev0 = rn(H * D) * 0.5, rn(T, 40).bfloat16(), rn(R, 40)
 
+    def forced(self, ops, chunks):
+        """run() in chunks or token by token, and sure of it."""
+        ops.scan_chunk_tokens = 1 if chunks else 1 << 30
+        mode = ["retention", "mlstm", "wkv"].index(self.kind)
+        assert ops._in_chunks(mode, sum(self.lens), len(self.lens), None, self.H, self.D, self.Dv, self.q, self.k, self.v) is chunks
+        before = ops.launches
+        result = self.run(ops)
+        self.launched = ops.launches - before
+        assert self.launched >= 3 if chunks else self.launched <= 2
+        return result
+
     def run(self, ops):
         H, D, Dv, N = self.H, self.D, self.Dv, len(self.lens)
         S = self.S0.clone()
@@ -127,8 +138,7 @@ def test_chunks_against_64_bits(ops, kind, lens, H, D, Dv, strong):
     if kind == "wkv":
         Dv = D
     sc = Scan(kind, lens, H, D, Dv, seed=len(lens) + D, strong=strong)
-    ops.scan_chunk_tokens = 1
-    out, states = sc.run(ops)
+    out, states = sc.forced(ops, True)
     exp, exp_states = sc.exact()
     bound = 2e-5 if kind == "mlstm" else 1e-6
     rows = lambda x: x.double().view(-1, H, Dv)[~sc.near]
@@ -136,9 +146,10 @@ def test_chunks_against_64_bits(ops, kind, lens, H, D, Dv, strong):
     assert rel(rows(out), rows(exp)) < bound
     for s, e in zip(states, exp_states):
         assert rel(s, e) < 1e-6
-    ops.scan_chunk_tokens = 1 << 30
-    walk, walk_states = sc.run(ops)
+    walk, walk_states = sc.forced(ops, False)
     assert rel(rows(walk), rows(exp)) < bound
+    for s, e in zip(walk_states, exp_states):                         # (mlstm's walk has its weights from 32-bit sums of 32 log gates of up to 15, off by 480 * 2^-25 = 1.4e-5)
+        assert rel(s, e) < (bound if kind == "mlstm" else 1e-6)
     if kind == "wkv":
         assert torch.equal(states[1], walk_states[1])                 # the request's last input
     print(kind, lens, D, Dv, strong, "out %.3g %.3g" % (rel(rows(out), rows(exp)), rel(rows(walk), rows(exp))),
@@ -147,8 +158,7 @@ def test_chunks_against_64_bits(ops, kind, lens, H, D, Dv, strong):
 
 def test_retention_chunks_with_32_bit_values(ops):
     sc = Scan("retention", [200, 70], 2, 128, 128, seed=9, values=torch.float32)
-    ops.scan_chunk_tokens = 1
-    out, (S,) = sc.run(ops)
+    out, (S,) = sc.forced(ops, True)
     exp, (e,) = sc.exact()
     assert rel(out, exp) < 1e-6 and rel(S, e) < 1e-6
 
@@ -157,10 +167,10 @@ def test_retention_chunks_with_32_bit_values(ops):
 def test_chunks_in_passes(ops, kind):
     """A step whose states between chunks do not fit the workspace runs in passes that carry the state rows on: the same bits."""
     sc = Scan(kind, [500, 3, 260], 2, 64, 64, seed=4)
-    ops.scan_chunk_tokens = 1
-    out, states = sc.run(ops)
+    out, states = sc.forced(ops, True)
     ops.scan_chunk_bytes = 3 * 2 * 64 * 64 * 4
-    out2, states2 = sc.run(ops)
+    out2, states2 = sc.forced(ops, True)
+    assert sc.launched > 3                                            # more than one pass
     assert torch.equal(out, out2) and all(torch.equal(a, b) for a, b in zip(states, states2))
 
 
@@ -173,14 +183,12 @@ def test_what_is_not_finite_stays_behind(ops, kind, what):
     for bad in (float("inf"), float("nan")):
         sc, clean = Scan(kind, lens, 2, 64, 64, seed=5), Scan(kind, lens, 2, 64, 64, seed=5)
         getattr(sc, what)[at, 70] = bad
-        ops.scan_chunk_tokens = 1
-        out, states = sc.run(ops)
+        out, states = sc.forced(ops, True)
         ref, _ = clean.run(ops)
-        # (the 16 rows around a value that is not finite are summed token by token: other roundings)
+        # (the read-outs of a chunk in which something is not finite are computed token by token: other roundings)
         assert torch.allclose(out[:at], ref[:at], rtol=1e-5, atol=1e-5) and torch.equal(out[150:], ref[150:])
         assert not torch.isfinite(out[at + 1:150, 64:]).all()
-        ops.scan_chunk_tokens = 1 << 30
-        walk, walk_states = sc.run(ops)
+        walk, walk_states = sc.forced(ops, False)
         assert torch.equal(torch.isfinite(out), torch.isfinite(walk))
         assert torch.equal(torch.isfinite(states[0]), torch.isfinite(walk_states[0]))
 
@@ -203,10 +211,8 @@ def test_what_is_not_finite_comes_out_as_the_walk_has_it(ops, kind, what, D, Dv)
             sc.S0[sc.s_at[0], 1, 3, 5] = bad
         else:
             getattr(sc, what)[75, (Dv if what == "v" else D) + 6] = bad
-        ops.scan_chunk_tokens = 1
-        out, states = sc.run(ops)
-        ops.scan_chunk_tokens = 1 << 30
-        walk, walk_states = sc.run(ops)
+        out, states = sc.forced(ops, True)
+        walk, walk_states = sc.forced(ops, False)
         for got, want in zip([out] + states, [walk] + walk_states):
             assert torch.equal(class_of(got), class_of(want)), (bad, got.shape)
             fine = want.isfinite()
@@ -220,8 +226,7 @@ def test_retention_chunks_near_the_largest_number(ops):
     sc.k[75, 64 + 6], sc.k[140, 9] = 3.395e38, -3.39e38
     sc.v[75], sc.v[140] = 2.0 ** -3, 2.0 ** -4
     sc.q.mul_(2.0 ** -6)
-    ops.scan_chunk_tokens = 1
-    out, (S,) = sc.run(ops)
+    out, (S,) = sc.forced(ops, True)
     exp, (e,) = sc.exact()
     assert out.isfinite().all() and S.isfinite().all()
     assert rel(out * 2.0 ** -100, exp * 2.0 ** -100) < 1e-6 and rel(S * 2.0 ** -100, e * 2.0 ** -100) < 1e-6
@@ -237,10 +242,8 @@ def test_wkv_state_is_no_further_off_than_the_walks(ops, lens, D, lo, hi):
     g = torch.Generator(device=DEV)
     g.manual_seed(8)
     sc.w = torch.exp(-torch.exp(torch.rand(sc.w.shape, generator=g, device=DEV) * (hi - lo) + lo))
-    ops.scan_chunk_tokens = 1
-    out, states = sc.run(ops)
+    out, states = sc.forced(ops, True)
     exp, exp_states = sc.exact()
-    ops.scan_chunk_tokens = 1 << 30
-    walk, walk_states = sc.run(ops)
+    walk, walk_states = sc.forced(ops, False)
     assert rel(states[0], exp_states[0]) < 1.1 * rel(walk_states[0], exp_states[0])
     assert rel(out, exp) < 1.1 * rel(walk, exp)

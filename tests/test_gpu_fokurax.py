@@ -488,12 +488,22 @@ def test_table_experts_alone(ops, dtype, T, experts, top):
         assert rel(y, pf.table_experts(x.double(), w, "", f, toks)) < (2e-5 if dtype == "float32" else 2e-2)
 
 
-@pytest.mark.parametrize("few", [0, 1, 2])
+@pytest.mark.parametrize("few", [0, "library", 1, 2])
 @pytest.mark.parametrize("T,experts,top,width,ff", [(1, 3, 1, 8, 8), (9, 4, 2, 56, 24), (40, 3, 3, 200, 72), (33, 2, 1, 1032, 136), (70, 20, 5, 128, 40)])
 def test_grouped_products_in_every_form(ops, monkeypatch, few, T, experts, top, width, ff):
-    """The library's, and weights streamed once for eight or sixteen rows at a time: gated and plain, either output, tiles of a single row
-    and of more than sixteen, widths that leave warps without a share of the sum, an activation behind a row's weight."""
-    monkeypatch.setattr(ops, "_grouped_few", lambda x, plan: few)
+    """The tcgen05 product, the library's, and weights streamed once for eight or sixteen rows at a time: gated and plain, either output, tiles
+    of a single row and of more than sixteen, widths that leave warps without a share of the sum, an activation behind a row's weight."""
+    ran = {"own": 0, "library": 0}
+    own, library = ops._grouped_tc, ops._library_grouped
+    def counted(name, fn):
+        def call(*args):
+            out = fn(*args)
+            ran[name] += out is not None
+            return out
+        return call
+    monkeypatch.setattr(ops, "_grouped_few", lambda x, plan: few if few in (1, 2) else 0)
+    monkeypatch.setattr(ops, "_grouped_tc", counted("own", own) if few == 0 else lambda *a: None)
+    monkeypatch.setattr(ops, "_library_grouped", counted("library", library))
     g = torch.Generator().manual_seed(T)
     r = lambda *s: (torch.randn(s, generator=g) / s[-1] ** 0.5).to(torch.bfloat16)
     w_gu, w_down, x = r(experts, 2 * ff, width), r(experts, width, ff), torch.randn(T, width, generator=g).to(torch.bfloat16)
@@ -511,6 +521,7 @@ def test_grouped_products_in_every_form(ops, monkeypatch, few, T, experts, top, 
     scale = torch.rand(T, top, generator=g)
     up = ops.grouped_act(x.to(DEV), w_gu.to(DEV), plan, top, "relu2", row_scale=scale.to(DEV))
     assert rel(up, torch.relu(gu * scale.reshape(-1)[pair][:, None].double()) ** 2) < 2e-2
+    assert ran == {"own": 4 if few == 0 else 0, "library": 4 if few == "library" else 0}      # (gated, plain twice, with the activation)
 
 
 @pytest.mark.parametrize("T", [1, 63, 700])

@@ -120,3 +120,30 @@ def test_gated_unit_in_32_bits(ops):
     exp = (gate / (1 + torch.exp(-float(torch.tensor(1.702)) * gate)) * (up + 1)).bfloat16()
     assert torch.equal(got, got[:1].expand_as(got))
     assert (got[0] != exp).sum().item() <= 6
+
+
+@pytest.mark.parametrize("side", ["own", "library"])
+@pytest.mark.parametrize("counts,identity,top,N,K", CASES[1:])
+def test_both_sides_of_the_rule_through_the_public_calls(ops, monkeypatch, side, counts, identity, top, N, K):
+    """``grouped_linear`` and ``grouped_act`` on the product that the rows-per-expert rule names, over the same plan: experts without rows,
+    and experts without a matrix, whose pairs stand behind all others."""
+    g = torch.Generator().manual_seed(len(counts) + K)
+    plan = plan_of(ops, counts, identity, top, g)
+    E, P = len(counts) - identity, sum(counts)
+    monkeypatch.setattr(ops, "_grouped_few", lambda x, plan: 0)
+    monkeypatch.setattr(ops, "grouped_tc_plain_rows", 1 << 20 if side == "own" else 0)
+    ran, call = [], ops._library_grouped
+    monkeypatch.setattr(ops, "_library_grouped", lambda *a: ran.append(call(*a)) or ran[-1])
+    x = torch.randn(P // top, K, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16().to(DEV)
+    scale = torch.rand(P // top, top, generator=g)
+    rows, up = ops.grouped_linear(x, w, plan, top), ops.grouped_act(x, w, plan, top, "relu2", row_scale=scale.to(DEV))
+    assert len(ran) == (0 if side == "own" else 2) and all(r is not None for r in ran)
+    pos, off = plan["pair_of_pos"].long().cpu(), plan["offsets"].cpu()
+    for e in range(E):
+        at = pos[off[e]:off[e + 1]]
+        exp = x.double().cpu()[at // top] @ w[e].double().cpu().T
+        assert torch.allclose(rows[off[e]:off[e + 1]].double().cpu(), exp, rtol=2.0 ** -8, atol=1e-5 * K ** 0.5)
+        # (the square doubles the rounding of the product, which stands in bfloat16 ahead of it)
+        exp = torch.relu(exp * scale.reshape(-1)[at][:, None].double()) ** 2
+        assert torch.allclose(up[off[e]:off[e + 1]].double().cpu(), exp, rtol=2.0 ** -6, atol=1e-4 * K ** 0.5)

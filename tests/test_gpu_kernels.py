@@ -673,10 +673,8 @@ def test_swiglu_product_for_few_rows_is_chosen_by_measurement(ops):
 
 
 @pytest.mark.parametrize("order", [(1024, 1100), (1100, 1024)])
-def test_gate_up_form_of_a_portion_does_not_depend_on_the_sizes_met_before(order):
+def test_gate_up_form_of_a_portion_does_not_depend_on_the_sizes_met_before(ops, order):
     """The form that the rule names, bit for bit, whichever of two portions comes first."""
-    from tiny_transformer_inference_engine_b200.ops import CudaOps
-    ops = CudaOps(DEV)
     F, K = 11008, 2048
     g = torch.Generator().manual_seed(2)
     w = (torch.randn(2 * F, K, generator=g) * 0.02).bfloat16().to(DEV)

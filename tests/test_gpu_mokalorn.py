@@ -402,11 +402,12 @@ def test_retention_alone(ops, dtype, heads, dim, vdim, decay, rot):
     (1, 160, 24, (0.95,)),
     (2, 48, 8, (0.5, 0.98)),                                            # padded to 64 channels
 ])
-def test_retention_long_prompts_in_parts(ops, dtype, heads, dim, vdim, decay):
-    """Prompts long enough that a step walks them in parts (two launches): a long request beside a short one and beside one
+def test_retention_long_prompts_in_parts(ops, monkeypatch, dtype, heads, dim, vdim, decay):
+    """(Walked whatever the head size; the chunks that most of these would take have tests of their own.)  Prompts long enough that a step walks them in parts (two launches): a long request beside a short one and beside one
     of a single token, whole and cut so that later steps are short again; heads that forget nothing, little, fast and
     everything; a state that the step finds filled (the second and third cut)."""
     L = retention_layer(heads, dim, vdim, decay, {"base": 200.0, "dims": 8})
+    monkeypatch.setattr(ops, "scan_chunk_tokens", 1 << 30)
     part, w = part_with_weights("mixer", _mixer(L, "a", 40, 1e-5), dtype, ops, 14, scale=0.3)
     g = torch.Generator().manual_seed(15)
     lens = (1500, 90, 1)
