@@ -102,3 +102,36 @@ def test_selective_scan_forms(ops, lens, I, N, wide):
         want = torch.cat([tail0[slot].double(), xin[qsl[r]:qsl[r + 1]].double()])[-3:]
         assert torch.equal(tail[slot].double(), want)
     assert torch.equal(S[R], S0[R])
+
+
+@pytest.mark.parametrize("lens,I,N", [([1] * 23 + [700], 264, 16), ([1, 64, 65, 1, 500], 130, 8), ([3] * 40 + [130], 40, 4), ([128] * 5, 72, 13)])
+def test_selective_scan_of_a_mixed_step_in_parts(ops, monkeypatch, lens, I, N):
+    """Decoding requests beside a portion that is walked in parts, with a thread per channel, when the longest request is known: the form with
+    a thread per four states gives the same (one rounding to bfloat16 apart; states to 2e-5, whose decays come from the hardware's exponential)."""
+    T, R, pad = sum(lens), len(lens), ops.selective_state_pad(N)
+    u, z, low = randn(21, T, I).bfloat16(), randn(22, T, I).bfloat16(), randn(23, T, 2 * N).bfloat16()
+    dt, bias, D, xin = randn(24, T, I), randn(25, I) - 4, randn(26, I), randn(27, T, I).bfloat16()
+    A = torch.zeros(I, pad, device=DEV)
+    A[:, :N] = -torch.exp(randn(28, I, N))
+    S0, tail0 = torch.zeros(R + 1, I, pad, device=DEV), randn(30, R + 1, 3, I)
+    S0[..., :N] = randn(29, R + 1, I, N)
+    qsl = [0]
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(ops, "selective_wide_full", 0.0)
+    got = []
+    for work in (0, 1 << 60):
+        monkeypatch.setattr(ops, "selective_wide_work", work)
+        wide = ops.selective_wide(torch.bfloat16, T, R, I, N, max(lens))
+        assert wide is (work == 0)
+        if wide:
+            monkeypatch.setattr(ops, "selective_wide_full", 1e9)      # (parts, however few warps there are)
+            assert ops.selective_parts(T, R, I, N, True, max(lens)) > 1
+        S, tail = S0.clone(), tail0.clone()
+        monkeypatch.setattr(ops, "selective_wide", lambda *a: wide)
+        got.append((ops.selective_scan(u, dt, bias, A, D, low, 0, N, z, S, xin, tail, 4, t(qsl), t(list(range(R))[::-1]), R, N, max_q_len=max(lens)), S, tail))
+        monkeypatch.delattr(ops, "selective_wide")
+    (y, S, tail), (y2, S2, tail2) = got
+    assert torch.allclose(y.double(), y2.double(), rtol=2.0 ** -7, atol=2e-3 * float(y2.abs().max()))
+    assert ((S - S2).norm() / S2.norm()).item() < 2e-5 and torch.equal(tail, tail2)

@@ -54,3 +54,30 @@ def test_scans_in_chunks_only_for_rows_and_heads_that_fit(mode):
     assert in_chunks(mode, [1024], 2048)
     assert not in_chunks(mode, [1024], 2048, dim=136) and not in_chunks(mode, [1024], 2048, dim=20) and not in_chunks(mode, [1024], 2048, dim=4)
     assert not in_chunks(mode, [1024], 2048, stride=2) and not in_chunks(mode, [1024], 2048, at=2)
+
+
+def selective(lens, channels, states, known=True, dtype=torch.bfloat16):
+    """(a thread per channel?, parts) of a selective scan on 148 SMs."""
+    ops = CudaOps.__new__(CudaOps)
+    ops.num_sms = 148
+    step = (sum(lens), len(lens), channels, states)
+    wide = ops.selective_wide(dtype, *step, max(lens) if known else None)
+    return wide, ops.selective_parts(*step, wide, max(lens) if known else None)
+
+
+# (as measured: the form ahead, with the parts that were)
+@pytest.mark.parametrize("lens,channels,states,form", [
+    ([2048], 4096, 16, (True, 32)), ([1024], 4096, 16, (True, 16)), ([512], 8192, 16, (True, 8)), ([512] * 4, 4096, 16, (True, 8)),
+    ([512], 4096, 16, (False, 8)), ([100], 8192, 16, (False, 1)),
+    ([1] * 23 + [2000], 8192, 16, (True, 5)), ([1] * 7 + [1000], 8192, 16, (True, 15)), ([1] * 23 + [2000], 4096, 8, (True, 18)),
+    ([1] * 200 + [2000], 8192, 16, (False, 1)),                       # the parts' sums of so many requests would not fit
+    ([128] * 16, 4096, 16, (True, 1)), ([256] * 8, 4096, 16, (True, 1)), ([128] * 16, 8192, 8, (True, 1)),
+    ([8] * 150, 8192, 4, (False, 1)), ([64] * 32, 4096, 4, (True, 1)), ([2048], 4096, 32, (False, 8)),
+])
+def test_selective_scan_forms(lens, channels, states, form):
+    assert selective(lens, channels, states) == form
+    assert not selective(lens, channels, states, dtype=torch.float32)[0]
+
+
+def test_selective_scan_form_without_the_longest_request():
+    assert selective([2048], 4096, 16, known=False) == (True, 32) and selective([1] * 7 + [2000], 8192, 16, known=False) == (True, 2)

@@ -1176,18 +1176,41 @@ class CudaOps:
 
     selective_wide_work = 4 << 20           # tokens x channels of a step from which a thread owns a channel with all its states;
     selective_wide_warps = 28               # the warps per SM that parts are made for then,
-    selective_wide_parts = 32               # and the most parts
+    selective_wide_parts = 32               # the most parts,
+    selective_wide_full = 6.5               # the warps per SM that walk all the time, from which parts buy nothing and below which the form is not taken,
+    selective_scratch_bytes = 64 << 20      # and the most that the parts' sums may take
 
-    def selective_wide(self, dtype, num_tokens: int, num_seqs: int, channels: int, states: int) -> bool:
+    def selective_wide(self, dtype, num_tokens: int, num_seqs: int, channels: int, states: int, longest=None) -> bool:
         """Whether a thread owns a channel (16-bit operands, up to 16 states) rather than four states of one: fewer instructions and a
         quarter of the threads, so it needs a step large enough to fill the GPU all the same.  16 states, us of a thread per
         channel | per four states: 4,096 channels 512 tokens 42 | 40, 1,024 tokens 68 | 73, 2,048 tokens 117 | 141, four requests of
-        512 107 | 134; 2,048 channels 2,048 tokens 73 | 74; 8,192 channels 256 tokens 41 | 39, 512 65 | 70, 2,048 204 | 273."""
-        return dtype == torch.bfloat16 and states <= 16 and (num_tokens - (num_seqs - 1)) * channels >= self.selective_wide_work
+        512 107 | 134; 2,048 channels 2,048 tokens 73 | 74; 8,192 channels 256 tokens 41 | 39, 512 65 | 70, 2,048 204 | 273.
+        ``longest``: the most tokens that a request brings, if known.  Beside 23 decoding requests a portion of 2,000 tokens is all there is to
+        fill the GPU (8,192 channels 701 in one part, 447 per four states, 260 in eight parts).  Up to four states both forms have a
+        thread per channel, and requests of a few tokens do not pay for the runs' staging (150 of 8 tokens 95 | 83)."""
+        if dtype != torch.bfloat16 or states > 16:
+            return False
+        if longest is None:
+            return (num_tokens - (num_seqs - 1)) * channels >= self.selective_wide_work
+        if num_tokens * channels < self.selective_wide_work:
+            return False
+        if states <= 4 and longest < 32:
+            return False
+        walking = -(-channels // 32) * max(1.0, num_tokens / longest)
+        return states <= 4 or walking * self.selective_parts(num_tokens, num_seqs, channels, states, True, longest) >= self.selective_wide_full * self.num_sms
 
-    def selective_parts(self, num_tokens: int, num_seqs: int, channels: int, states: int, wide: bool = False) -> int:
+    def selective_parts(self, num_tokens: int, num_seqs: int, channels: int, states: int, wide: bool = False, longest=None) -> int:
         """Into how many parts a request's tokens are walked: every part but the last is walked twice, which pays while the
-        channels alone give the SMs too few warps to hide a token's latency."""
+        channels alone give the SMs too few warps to hide a token's latency.  With a thread per channel (``wide``) and ``longest`` known the
+        warps counted are those of the tokens, as so many requests of that length (a request of one token leaves at once); from 6.5 warps
+        per SM on one part is best (4,096 channels, 16 states, 16 requests of 128 tokens 69 us in one part, 90 in two; 8 of 256 94 and 113, 101 in
+        four; 8,192 channels, 2 of 512 145 in one, 107 in eight)."""
+        if wide and longest is not None:
+            walking = -(-channels // 32) * max(1.0, num_tokens / longest)
+            if walking >= self.selective_wide_full * self.num_sms:
+                return 1
+            room = self.selective_scratch_bytes // (4 * num_seqs * channels * (self.selective_state_pad(states) + 1))
+            return max(1, min(self.selective_wide_parts, longest // self.selective_part_tokens, int(self.selective_wide_warps * self.num_sms / walking), room))
         longest = num_tokens - (num_seqs - 1)                          # the most tokens one request of the step can bring
         lanes = 1 if wide else self.selective_state_pad(states) // 4
         warps = num_seqs * -(-channels * lanes // 32)
@@ -1202,16 +1225,17 @@ class CudaOps:
             pad *= 2
         return pad
 
-    def selective_scan(self, u, dt, dt_bias, A, D, bc, col_b, col_c, z, state, xin, tail, taps, query_start_loc, slot_ids, num_seqs, states):
+    def selective_scan(self, u, dt, dt_bias, A, D, bc, col_b, col_c, z, state, xin, tail, taps, query_start_loc, slot_ids, num_seqs, states,
+                       max_q_len=None):
         """The diagonal recurrence over the step's tokens from the state rows ``state`` [slots + 1, channels, padded states] (advanced
         in place), with read-out, skip (``D``) and gate: returns (S C + D u) * silu(z) [T, channels] in the compute dtype.  ``u``,
         ``z``: views [T, channels]; ``dt`` float32 [T, channels] before bias and softplus; ``A`` float32 [channels, padded states];
         ``bc``: rows that hold B at column ``col_b`` and C at ``col_c``.  Also moves the last ``taps - 1`` rows of ``xin`` (the
-        convolution's inputs) into the state rows ``tail`` (None with one tap)."""
+        convolution's inputs) into the state rows ``tail`` (None with one tap).  ``max_q_len``: the most tokens a request brings, if known."""
         T, I = u.shape
         out = torch.empty((T, I), dtype=u.dtype, device=u.device)
-        wide = self.selective_wide(u.dtype, T, int(num_seqs), I, int(states))
-        parts = self.selective_parts(T, int(num_seqs), I, int(states), wide)
+        wide = self.selective_wide(u.dtype, T, int(num_seqs), I, int(states), max_q_len)
+        parts = self.selective_parts(T, int(num_seqs), I, int(states), wide, max_q_len)
         scratch = torch.empty(int(num_seqs) * parts * I * (A.shape[1] + 1), dtype=torch.float32, device=u.device) if parts > 1 else None
         self._check(self.lib.ttie_selective_scan(
             _ptr(u), u.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(A), _ptr(D), _ptr(bc), bc.stride(0), int(col_b), int(col_c), _ptr(z),

@@ -101,5 +101,5 @@ class SelectiveScan(Mixer):
         low = ops.linear_narrow(u, self.w_x)                                                  # [T, d | B | C]
         dt = ops.linear(low[:, :self.w_dt.shape[1]], self.w_dt, None, out_dtype=torch.float32)  # [T, inner] float32
         y = ops.selective_scan(u, dt, self.dt_b, self.A, self.D, low, self.col_b, self.col_c, proj[:, I:], S, proj, tail, self.taps,
-                               ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, self.state)
+                               ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, self.state, max_q_len=ctx.max_q_len)
         return ops.linear(y, self.w_out, None, partial_ok=True)
