@@ -1,7 +1,7 @@
 // True 32-bit matrix product for the float32 path: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]).
 // Plain FFMA with float32 accumulation - no tensor cores, no TF32 - so that the float32
 // path shows faults that reduced precision would hide.  Any M, N, K.
-// Two kernels: a 64 x 128 tile for prompt portions, and for up to 16 rows (decode steps) a form that streams the weight
+// Two kernels: tiles of 64 x 128 or 64 x 64 for prompt portions, and for up to 16 rows (decode steps) a form that streams the weight
 // matrix once: a warp owns four weight rows at a time, its lanes walk K in 16-byte steps, and the activations - a few
 // rows that every warp reads - come through the cache.
 #include "common.cuh"
@@ -14,12 +14,12 @@ namespace {
 // a transposition in between, and a load's four values along K are two pairs for the packed multiply-add.  Accumulators are
 // pairs too (even and odd K), added at the end.  Rows are 20 floats apart: the eight rows that a warp reads at once fall into
 // different banks.  Too few tiles for the GPU: a cluster of CTAs shares a tile, each walks a range of K, and the partial tiles
-// are added through distributed shared memory in the order of the ranges.
+// are added through distributed shared memory in the order of the ranges.  Two widths: 64 columns (8 x 4 outputs) where a 128-wide tile would be
+// half empty or, with few tiles and a K too short to cut, the whole time is one tile's: us, 64 columns | 128, 300 rows of K 64 to N 2,048 SMALL_A,
+// 40 rows of K 128 to N 128 SMALL_B, 32 products of [2,048, 128] with [64, 128] SMALL_C.
 // 300 rows times [2304, 2048], [2048, 2048], [16384, 2048] and [2048, 8192] (36 GFLOP): 1,121 us, 32 TFLOP/s; 2,393 us as a 64 x 64
 // tile of 4 x 4 outputs staged through registers.
-constexpr int BM = 64, BN = 128, BK = 16, PITCH = BK + 4, STAGES = 3, MAX_RANGES = 8;
-constexpr int STAGE_FLOATS = (BM + BN) * PITCH;
-constexpr int TILE_SMEM = STAGES * STAGE_FLOATS * 4;                  // 46,080 bytes; holds a partial tile (32,768) at the end
+constexpr int BM = 64, BK = 16, PITCH = BK + 4, STAGES = 3, MAX_RANGES = 8;
 
 __device__ __forceinline__ void fma_pair(float2& d, float2 a, float2 b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<unsigned long long&>(d))
@@ -40,23 +40,26 @@ __device__ __forceinline__ void stage_operand(float* dst, const float* src, int 
     }
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(128, 2)
+// TN: columns per thread (8 rows); a tile has 16 TN columns
+template <bool VEC, int TN>
+__global__ void __launch_bounds__(128, TN == 8 ? 2 : 3)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                 float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
                 long long batch_a, long long batch_w, long long batch_c, int ranges, int range_len) {
-    __shared__ __align__(16) float smem[STAGES * STAGE_FLOATS];
+    constexpr int BN = 16 * TN, STAGE_FLOATS = (BM + BN) * PITCH;
+    static_assert(STAGES * STAGE_FLOATS >= BM * BN, "the stages hold a partial tile at the end");
+    __shared__ __align__(16) float smem[STAGES * STAGE_FLOATS];           // 46,080 bytes (TN 8), 30,720
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = blockIdx.x % ranges;                                                 // clusters are consecutive CTAs along x
     A += blockIdx.z * batch_a; W += blockIdx.z * batch_w; C += blockIdx.z * batch_c;      // (a batch of products: grid z)
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x / ranges * BN;
     const int k_lo = rank * range_len, k_hi = min(K, k_lo + range_len);
-    const int tm = (warp >> 1) * 32 + (lane >> 3), tn = (warp & 1) * 64 + (lane & 7);     // the thread's rows tm + 4 i, columns tn + 8 j
-    float2 acc[8][8];
+    const int tm = (warp >> 1) * 32 + (lane >> 3), tn = (warp & 1) * 8 * TN + (lane & 7);     // the thread's rows tm + 4 i, columns tn + 8 j
+    float2 acc[8][TN];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+        for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
     const int steps = (k_hi - k_lo + BK - 1) / BK;
     auto stage = [&](int it) {
         if (it < steps) {
@@ -80,7 +83,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 #pragma unroll
             for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(as + 4 * i * PITCH + k);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < TN; ++j) {
                 const float4 w = *reinterpret_cast<const float4*>(ws + 8 * j * PITCH + k);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -95,7 +98,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
         for (int i = 0; i < 8; ++i) {
             const int gm = m0 + tm + 4 * i;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < TN; ++j) {
                 const int gn = n0 + tn + 8 * j;
                 if (gm < M && gn < N) C[(size_t)gm * ldc + gn] = acc[i][j].x + acc[i][j].y + (bias ? bias[gn] : 0.f);
             }
@@ -107,7 +110,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) smem[(tm + 4 * i) * BN + tn + 8 * j] = acc[i][j].x + acc[i][j].y;
+        for (int j = 0; j < TN; ++j) smem[(tm + 4 * i) * BN + tn + 8 * j] = acc[i][j].x + acc[i][j].y;
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     const uint32_t mine = (uint32_t)__cvta_generic_to_shared(smem);
     for (int e = rank * 128 + tid; e < BM * BN / 4; e += ranges * 128) {
@@ -133,7 +136,10 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 
 int launch_tiles(const float* A, const float* W, const float* bias, float* C, int B, int M, int N, int K, int lda, int ldw, int ldc,
                  long long batch_a, long long batch_w, long long batch_c, cudaStream_t s) {
-    const long long tiles = (long long)B * ceil_div(M, BM) * ceil_div(N, BN), slots = 2LL * num_sms();
+    const long long wide_tiles = (long long)B * ceil_div(M, BM) * ceil_div(N, 128), slots = 2LL * num_sms();
+    const bool narrow = N <= 64 || (K <= 128 && wide_tiles <= num_sms());
+    const int BN = narrow ? 64 : 128;
+    const long long tiles = (long long)B * ceil_div(M, BM) * ceil_div(N, BN);
     // K ranges per tile: the fewest waves of two CTAs per SM times a wave's length, a range's fixed cost taken as 64 values of K
     // (filling the stages) and 48 more for adding the partial tiles.  [300, 2048] x [2304, 2048]: 90 tiles alone leave half
     // of the SMs' places empty.
@@ -155,8 +161,9 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ranges; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = ranges > 1 ? 1 : 0;
-    const cudaError_t e = vec ? cudaLaunchKernelEx(&cfg, gemm_f32_kernel<true>, A, W, bias, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, ranges, range_len)
-                              : cudaLaunchKernelEx(&cfg, gemm_f32_kernel<false>, A, W, bias, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, ranges, range_len);
+    auto launch = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, A, W, bias, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, ranges, range_len); };
+    const cudaError_t e = narrow ? (vec ? launch(gemm_f32_kernel<true, 4>) : launch(gemm_f32_kernel<false, 4>))
+                                 : (vec ? launch(gemm_f32_kernel<true, 8>) : launch(gemm_f32_kernel<false, 8>));
     if (e != cudaSuccess) TTIE_FAIL("gemm_f32: launch failed: %s", cudaGetErrorString(e));
     return 0;
 }
