@@ -1030,7 +1030,7 @@ def test_score_softcap_in_every_attention_kernel(ops, dtype, plan, seqs, spike):
 @pytest.mark.parametrize("B,M,N,K,off", [(1, 64, 128, 16, 0), (1, 65, 129, 20, 0), (1, 63, 127, 4100, 0), (1, 300, 2304, 2048, 0), (1, 40, 3, 8192, 0),
                                          (1, 34, 260, 1021, 0), (1, 129, 130, 516, 3), (3, 70, 40, 260, 0), (5, 33, 257, 1283, 1),
                                          (1, 33, 131, 4096, 0), (1, 65, 5, 4096, 0), (2, 63, 197, 2052, 0),    # (last columns that part of a warp adds up)
-                                         (1, 40, 64, 64, 0), (1, 33, 65, 128, 0), (7, 65, 63, 36, 0), (1, 200, 2048, 64, 2), (33, 129, 64, 128, 0), (1, 300, 1, 2048, 0)])   # (64 columns)
+                                         (1, 40, 64, 64, 0), (1, 33, 65, 128, 0), (7, 65, 63, 36, 0), (1, 200, 2048, 64, 2), (33, 129, 64, 128, 0), (1, 300, 1, 2048, 0), (1, 65, 256, 240, 0)])   # (64 columns)
 def test_gemm_f32_tile_ranges(ops, B, M, N, K, off):
     """The tile form at the edges of its tiles, with one K range and with several that a cluster adds up, in 16-byte and in
     single copies, alone and in a batch.  A sum of K products of unit-variance values in 32 bits, in any order, is off by less than

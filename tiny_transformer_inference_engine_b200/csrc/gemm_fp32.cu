@@ -15,8 +15,8 @@ namespace {
 // pairs too (even and odd K), added at the end.  Rows are 20 floats apart: the eight rows that a warp reads at once fall into
 // different banks.  Too few tiles for the GPU: a cluster of CTAs shares a tile, each walks a range of K, and the partial tiles
 // are added through distributed shared memory in the order of the ranges.  Two widths: 64 columns (8 x 4 outputs) where a 128-wide tile would be
-// half empty or, with few tiles and a K too short to cut, the whole time is one tile's: us, 64 columns | 128, 300 rows of K 64 to N 2,048 SMALL_A,
-// 40 rows of K 128 to N 128 SMALL_B, 32 products of [2,048, 128] with [64, 128] SMALL_C.
+// half empty or, with few tiles and a K too short to cut, the whole time is one tile's: us, 64 columns | 128, 300 rows of K 64 to N 2,048 7.0 | 7.6,
+// of K 128 to N 128 8.0 | 12.1, of K 2,048 to N 64 15.3 | 22.5, 32 products of [2,048, 128] with [64, 128] 33 | 59.
 // 300 rows times [2304, 2048], [2048, 2048], [16384, 2048] and [2048, 8192] (36 GFLOP): 1,121 us, 32 TFLOP/s; 2,393 us as a 64 x 64
 // tile of 4 x 4 outputs staged through registers.
 constexpr int BM = 64, BK = 16, PITCH = BK + 4, STAGES = 3, MAX_RANGES = 8;
@@ -137,7 +137,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 int launch_tiles(const float* A, const float* W, const float* bias, float* C, int B, int M, int N, int K, int lda, int ldw, int ldc,
                  long long batch_a, long long batch_w, long long batch_c, cudaStream_t s) {
     const long long wide_tiles = (long long)B * ceil_div(M, BM) * ceil_div(N, 128), slots = 2LL * num_sms();
-    const bool narrow = N <= 64 || (K <= 128 && wide_tiles <= num_sms());
+    const bool narrow = N <= 64 || (K <= 240 && wide_tiles <= num_sms());
     const int BN = narrow ? 64 : 128;
     const long long tiles = (long long)B * ceil_div(M, BM) * ceil_div(N, BN);
     // K ranges per tile: the fewest waves of two CTAs per SM times a wave's length, a range's fixed cost taken as 64 values of K
