@@ -524,7 +524,7 @@ def test_grouped_products_in_every_form(ops, monkeypatch, few, T, experts, top, 
     assert ran == {"own": 4 if few == 0 else 0, "library": 4 if few == "library" else 0}      # (gated, plain twice, with the activation)
 
 
-@pytest.mark.parametrize("T", [1, 63, 700])
+@pytest.mark.parametrize("T", [1, 63, 90, 300, 341, 342, 700, 1365, 1366, 6000])
 def test_plans_from_tables(ops, T):
     """Three layers' plans in one launch: every pair stands once among its expert's rows; the row tiles cover each expert's rows once."""
     vocab, top, E = 50, 3, 11

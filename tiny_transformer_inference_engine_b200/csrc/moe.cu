@@ -680,9 +680,12 @@ static int launch_plan(const Choices& ch, int layers, long long out_stride, int 
     if (P <= 0) return 0;
     if (E > MAX_EXPERTS) TTIE_FAIL("moe_plan: %d experts (limit %d)", E, MAX_EXPERTS);
     if (tile_experts < 0 || tile_experts > E) TTIE_FAIL("moe_plan: %d of %d experts own matrices", tile_experts, E);
-    // (a decode step's few pairs: a small block, whose barriers are short)
-    if (P <= 256) TTIE_LAUNCH(moe_plan_kernel<1>, layers, 256, 0, s, ch, P, E, tile_experts, BM, max_tiles, offsets, pos_of_pair, pair_of_pos, tiles, meta, out_stride);
-    else TTIE_LAUNCH(moe_plan_kernel<16>, layers, 1024, 0, s, ch, P, E, tile_experts, BM, max_tiles, offsets, pos_of_pair, pair_of_pos, tiles, meta, out_stride);
+    // (a decode step's few pairs: a small block, whose barriers are short; and no more turns of the unrolled loops than there are pairs)
+    const int threads = P <= 256 ? 256 : P <= 512 ? 512 : 1024;
+    auto launch = [&](auto kernel) {
+        TTIE_LAUNCH(kernel, layers, threads, 0, s, ch, P, E, tile_experts, BM, max_tiles, offsets, pos_of_pair, pair_of_pos, tiles, meta, out_stride);
+    };
+    if (P <= 1024) launch(moe_plan_kernel<1>); else if (P <= 4096) launch(moe_plan_kernel<4>); else launch(moe_plan_kernel<16>);
     TTIE_CHECK_LAUNCH("moe_plan");
     return 0;
 }
