@@ -680,7 +680,8 @@ static int launch_plan(const Choices& ch, int layers, long long out_stride, int 
     if (P <= 0) return 0;
     if (E > MAX_EXPERTS) TTIE_FAIL("moe_plan: %d experts (limit %d)", E, MAX_EXPERTS);
     if (tile_experts < 0 || tile_experts > E) TTIE_FAIL("moe_plan: %d of %d experts own matrices", tile_experts, E);
-    // (a decode step's few pairs: a small block, whose barriers are short; and no more turns of the unrolled loops than there are pairs)
+    // (a decode step's few pairs: a small block, whose barriers are short; and no more turns of the unrolled loops than there are pairs: 300 pairs
+    // of 4 experts 2.3 us, 3.8 unrolled for 16,384, 2,048 of 4 3.2 and 4.6)
     const int threads = P <= 256 ? 256 : P <= 512 ? 512 : 1024;
     auto launch = [&](auto kernel) {
         TTIE_LAUNCH(kernel, layers, threads, 0, s, ch, P, E, tile_experts, BM, max_tiles, offsets, pos_of_pair, pair_of_pos, tiles, meta, out_stride);
