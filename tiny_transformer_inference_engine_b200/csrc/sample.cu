@@ -431,7 +431,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     unsigned cut_key = 0;
     // (without top-p the radix select takes four passes, not twelve, and lists above 256 tokens have two lanes a token instead of four: 8 rows of
     // 4,096 tokens, top-k 65, some 300 listed: 21.8 us by pairs, 18.6 by radix; with top-p 21.8 and 26.1)
-    const bool pairs = listed && n_cur <= (top_p < 1.0f ? SMALL_LIST : 256);
+    const bool pairs = listed && (n_cur <= 256 || (n_cur <= SMALL_LIST && top_p < 1.0f));
     if (pairs) {
         int sh = 0;
         while (sh < 5 && (n_cur << (sh + 1)) <= THREADS) ++sh;
