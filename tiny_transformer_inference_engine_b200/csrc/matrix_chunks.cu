@@ -34,11 +34,11 @@
 // Chunks are numbered over the whole step: request s owns the numbers from qsl[s] / 64 + s on, which leaves room for its last
 // partial chunk and needs nothing of the host but the number of tokens and requests.
 //
-// One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 28 + 9 + 65 against the walk's 514; 16 of 64 x 128
-// (mlstm) 13 + 9 + 46 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 34 + 20 + 79 against 473.  What bounds the out kernel is
-// latency: 12 warps per SM (168 registers, the planes in shared memory), issue slots 27 % used, the tensor pipe 37 / 15 / 12 %.  The wkv
-// kernels were 39 and 87 with half the threads in the sum (a run of 32 tokens' decays per thread is one serial chain of loads and
-// multiplications in 64 bits) and two blocks of out per SM instead of three.
+// One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 30 + 12 + 69 against the walk's 514; 16 of 64 x 128
+// (mlstm) 16 + 13 + 47 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 41 + 12 + 85 against 473.  What bounds the out kernel is
+// latency: 12 warps per SM fit (168 registers, the planes in shared memory), issue slots 30 % used, the tensor pipe 34 / 16 / 13 %.  With half
+// the threads in wkv's sum (a run of 32 tokens' decays per thread is one serial chain of loads and multiplications in 64 bits) and two blocks
+// of its out per SM instead of three its mixer took 257 us, 240 with them.
 // Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
 // 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 3.4e-8 (4.5e-8).
 #include "common.cuh"
