@@ -1040,3 +1040,53 @@ def test_gemm_f32_tile_ranges(ops, B, M, N, K, off):
     exp = torch.einsum("bmk,bnk->bmn", x.double(), w.double())
     got = ops.batched_linear(x, w) if B > 1 else ops.linear(x[0], w[0], torch.ones(N, device=DEV))[None] - 1.0
     assert (got.double() - exp).abs().max().item() < 4 * K ** 0.5 * K ** 0.5 * 2.0 ** -24 + 2e-6
+
+
+# one range of K and several, one token tile and several, halves of 128 rows that are missing or ragged, K that ends inside a block of 64
+@pytest.mark.parametrize("M,N,K", [(33, 512, 3072), (17, 1024, 1024), (32, 1100, 1028), (160, 2305, 1024), (161, 513, 4100), (97, 640, 4096), (320, 12400, 132),
+                                   (40, 16500, 2048), (300, 2304, 2048), (96, 514, 16384)])
+def test_gemm_f32_on_tensor_cores(ops, M, N, K):
+    """A float32 product as three bfloat16 a value, whole and as partial sums.  What is left out of a product is below 2^-24 of it and
+    each sum is rounded or cut off: at most K roundings of the running magnitude, as for multiply-adds; typically far less."""
+    g = torch.Generator().manual_seed(41)
+    x, w, b = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    assert ops._f32_planes_ok(x, w)
+    exp = x.double() @ w.double().T
+    whole = ops.linear(x, w, b)
+    part = ops.linear(x, w, None, partial_ok=True)
+    assert whole.shape == (M, N) and part.shape[-2:] == (M, N) and part.dtype == torch.float32
+    for got in (whole.double() - b.double(), part.double().sum(0) if part.dim() == 3 else part.double()):
+        assert (got - exp).abs().max().item() < 4 * K * 2.0 ** -24 + 2e-6
+        assert rel(got.cpu(), exp.cpu()) < 3e-7                # (multiply-adds leave 2e-7 to 5e-7 here)
+    wide = torch.randn(M, K + 4, generator=g).to(DEV)          # a strided input, and one that is not on 16 bytes
+    assert ops._f32_planes_ok(wide[:, :K], w) and not ops._f32_planes_ok(wide[:, 1:K + 1], w)
+    assert rel(ops.linear(wide[:, :K], w, None).cpu(), (wide[:, :K].double() @ w.double().T).cpu()) < 3e-7
+    assert ops.lib.ttie_tc_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 2304, 2048), (40, 16400, 260), (33, 520, 4096)])
+def test_gemm_f32_on_tensor_cores_extreme_values(ops, M, N, K):
+    """Infinities, NaN, values that round to an infinity as a bfloat16, and rows so small that their lower planes are not bfloat16
+    numbers: what 32-bit multiply-adds give."""
+    g = torch.Generator().manual_seed(43)
+    x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    x[3, 7], x[5, K - 1], x[8, 1], x[8, 2], w[9, 3], w[12, 5] = float("inf"), float("nan"), 3.4e38, -3.4e38, float("-inf"), 3.3999e38
+    x[7] *= 1e-36
+    w[11] *= 1e-34
+    w[N - 1] *= 1e-37
+    x[12], w[100], x[13] = 0, 0, x[13] * 2e-38
+    x, w = x.to(DEV), w.to(DEV)
+    assert ops._f32_planes_ok(x, w)
+    exp, scale = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    plain = torch.empty(M, N, device=DEV)
+    assert ops.lib.ttie_gemm_f32(x.data_ptr(), w.data_ptr(), None, plain.data_ptr(), M, N, K, K, K, N, ops._stream(x)) == 0
+    part = ops.linear(x, w, None, partial_ok=True)
+    for got in (ops.linear(x, w, None), part.sum(0) if part.dim() == 3 else part):
+        # (an intermediate sum may overflow in one order and not in another: only rows and columns far from the limit are compared there)
+        clear = torch.ones(M, N, dtype=torch.bool, device=DEV)
+        clear[8], clear[:, 12] = False, False
+        assert torch.equal(torch.isnan(got)[clear], torch.isnan(plain)[clear])
+        assert torch.equal(torch.isinf(got)[clear], torch.isinf(plain)[clear])
+        ok = torch.isfinite(plain) & clear & (scale > 1e-36)
+        assert ((got.double() - exp).abs()[ok] <= K * 2.0 ** -24 * scale[ok]).all()
+        assert (got[12] == 0).logical_or(torch.isnan(plain[12])).all()

@@ -81,3 +81,15 @@ def test_selective_scan_forms(lens, channels, states, form):
 
 def test_selective_scan_form_without_the_longest_request():
     assert selective([2048], 4096, 16, known=False) == (True, 32) and selective([1] * 7 + [2000], 8192, 16, known=False) == (True, 2)
+
+
+def test_float32_products_on_tensor_cores_by_shape_and_alignment():
+    """The rule that sends a float32 product to the three-plane kernel: sizes, strides and addresses that its copies can take."""
+    ok = CudaOps._f32_planes_ok
+    w = torch.zeros(1024, 2048)
+    x = torch.zeros(64, 2048)
+    assert ok(x, w) and ok(x[:33], w) and ok(x[:17], w) and not ok(x[:16], w)
+    assert not ok(x[:, 1:], w[:, 1:]) and not ok(x[:, :2046], w[:, :2046])              # rows off 16 bytes; K % 4
+    assert ok(x[:, 4:], w[:, 4:]) and not ok(torch.zeros(64, 2049)[:, :2048], w)        # a stride that is not a multiple of 4
+    assert not ok(x, w[:511]) and not ok(x[:, :512], w[:, :512]) and ok(torch.zeros(33, 128), torch.zeros(12288, 128))
+    assert not ok(x[:32, :1020], torch.zeros(4096, 1020)) and ok(x[:32, :1024], w[:, :1024])

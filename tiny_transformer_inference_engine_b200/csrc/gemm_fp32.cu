@@ -1,6 +1,6 @@
 // True 32-bit matrix product for the float32 path: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]).
-// Plain FFMA with float32 accumulation - no tensor cores, no TF32 - so that the float32
-// path shows faults that reduced precision would hide.  Any M, N, K.
+// Plain FFMA with float32 accumulation.  Any M, N, K; larger products of aligned operands run on the tensor cores with three
+// bfloat16 a value and a smaller error (gemm_fp32_tc.cu; the rule is the caller's, ops/__init__.py).
 // Two kernels: tiles of 64 x 128 or 64 x 64 for prompt portions, and for up to 16 rows (decode steps) a form that streams the weight
 // matrix once: a warp owns four weight rows at a time, its lanes walk K in 16-byte steps, and the activations - a few
 // rows that every warp reads - come through the cache.

@@ -254,19 +254,23 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2-D map over a row-major [rows][K] bfloat16 matrix with row stride ld; box = 64 (K) x box_rows.
-int make_map(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
+// 2-D map over a row-major [rows][cols] matrix of bfloat16 or float32 with row stride ld; 128-byte swizzle, so a box is at most 128 bytes wide.
+int make_map_of(CUtensorMap* map, bool f32, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) TTIE_FAIL("gemm_tc: cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
+    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) TTIE_FAIL("gemm_tc: cuTensorMapEncodeTiled failed with code %d", (int)r);
     return 0;
+}
+// The products' operands: bfloat16, box = 64 (K) x box_rows.
+int make_map(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
+    return make_map_of(map, false, base, rows, K, ld, BK, box_rows);
 }
 
 template <int BN, int STAGES, typename OutT>
@@ -306,6 +310,9 @@ int gemm_tc_error_words(int** word, int** mirror) {
 }
 int gemm_tc_make_map(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
     return make_map(map, base, rows, K, ld, box_rows);
+}
+int gemm_tc_make_map_of(CUtensorMap* map, int f32, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows) {
+    return make_map_of(map, f32 != 0, base, rows, cols, ld, box_cols, box_rows);
 }
 }  // namespace ttie
 

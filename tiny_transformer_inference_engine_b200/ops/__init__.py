@@ -7,8 +7,9 @@ Every call launches on torch's current stream of the tensors' device and returns
 
 Matrix products of the bfloat16 path go to the library product (cuBLAS through
 ``torch.mm``), as the reference's ``nn.Linear`` layers do (models/mqa.py:123-126,
-models/mlp.py:20-22); the float32 path uses this package's own FFMA kernel so that no
-reduced-precision matrix mode can slip in.
+models/mlp.py:20-22); the float32 path uses this package's own kernels (multiply-adds, or three
+bfloat16 a value on the tensor cores, which is closer to 64 bits) so that no reduced-precision
+matrix mode can slip in.
 """
 from __future__ import annotations
 
@@ -43,6 +44,8 @@ _SIGNATURES = {
     "ttie_rope_store": [_c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_void, _c_int, _c_void,
                         _c_void, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_f32": [_c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
+    "ttie_gemm_f32_tc": [_c_void, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
+    "ttie_gemm_f32_tc_parts": [_c_int, _c_int, _c_int],
     "ttie_paged_attention": [_c_void, _c_ll, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void, _c_void, _c_void,
                              _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_int, _c_int,
                              _c_void, _c_int, _c_void],
@@ -413,6 +416,21 @@ class CudaOps:
                 best, best_eff = ks, eff
         return best
 
+    @staticmethod
+    def _f32_planes_ok(x, w):
+        """Whether a float32 product runs on the tensor cores, each value as three bfloat16 (csrc/gemm_fp32_tc.cu): rows that its
+        copies can take (16 bytes), and enough work for its fixed cost of 8 to 12 us.  Measured on the other side, us here | multiply-adds:
+        [1024, 1024] 64 rows 13.9 | 13.5, 320 rows 20.6 | 37.7; [512, 512] 320 rows 16.5 | 13.9; [2048, 512] 128 rows 16.1 | 14.2;
+        [512, 2048] 33 rows 15.8 | 22.1; [2048, 2048] 33 rows 17 | 35.  17 to 32 rows (there the weights are streamed twice, and sums
+        over short K are closer to 64 bits): [256, 1024] 11.8 | 16.6, [8192, 2048] 24 | 63, [50257, 512] has a short K and stays."""
+        M, K = x.shape
+        N = w.shape[0]
+        if K % 4 or x.stride(0) % 4 or w.stride(0) % 4 or (x.data_ptr() | w.data_ptr()) & 15:
+            return False
+        if M <= 32:
+            return M > 16 and K >= 1024 and N * K >= 1 << 20
+        return N >= 512 and K >= 128 and N * K >= 3 << 19
+
     def linear(self, x, w, bias, out_dtype=None, partial_ok=False):
         """y = x @ w.T (+ bias); x [M, K], w [N, K] -> [M, N].  With ``partial_ok`` the result may
         instead be float32 partial sums [S, M, N] of a K-split product, which ``add_rmsnorm``,
@@ -420,6 +438,14 @@ class CudaOps:
         M, K = x.shape
         N = w.shape[0]
         if x.dtype == torch.float32:
+            if self._f32_planes_ok(x, w):
+                parts = self.lib.ttie_gemm_f32_tc_parts(M, N, K) if partial_ok and bias is None else 1
+                out = torch.empty((parts, M, N) if parts > 1 else (M, N), dtype=torch.float32, device=x.device)
+                planes = torch.empty(3 * M * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
+                self._check(self.lib.ttie_gemm_f32_tc(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(planes), M, N, K, x.stride(0),
+                                                      w.stride(0), N, parts, self._stream(x)), "gemm_f32_tc")
+                self.launches += 2
+                return out
             out = torch.empty((M, N), dtype=torch.float32, device=x.device)
             self._check(self.lib.ttie_gemm_f32(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), M, N, K, x.stride(0),
                                                w.stride(0), N, self._stream(x)), "gemm_f32")
