@@ -247,3 +247,44 @@ def test_wkv_state_is_no_further_off_than_the_walks(ops, lens, D, lo, hi):
     walk, walk_states = sc.forced(ops, False)
     assert rel(states[0], exp_states[0]) < 1.1 * rel(walk_states[0], exp_states[0])
     assert rel(out, exp) < 1.1 * rel(walk, exp)
+
+
+# whole and partial chunks of 128, requests of one token, heads of one piece of 8 channels up to a full tile, padded keys
+@pytest.mark.parametrize("strong", [False, True])
+@pytest.mark.parametrize("lens,H,D,Dv", [([128], 2, 128, 128), ([129, 127], 3, 64, 128), ([1, 255, 2], 2, 40, 104), ([300], 2, 8, 8), ([64, 1, 130], 1, 96, 64), ([1000], 2, 128, 120)])
+@pytest.mark.parametrize("kind", ["retention", "mlstm"])
+def test_chunks_of_128_tokens_against_64_bits(ops, monkeypatch, kind, lens, H, D, Dv, strong):
+    """The tcgen05 form against 64 bits and against the chunks of 64 tokens; bounds as above, and no further from 64 bits than the
+    walk (the matrix memory under strong gates, where single rows that nearly cancel decide, apart)."""
+    sc = Scan(kind, lens, H, D, Dv, seed=len(lens) + D, strong=strong)
+    exp, exp_states = sc.exact()
+    rows = lambda x: x.double().view(-1, H, Dv)[~sc.near]
+    results = {}
+    for tokens in (64, 128):
+        monkeypatch.setattr(type(ops), "_chunk_tokens", staticmethod(lambda *a: tokens))
+        results[tokens] = sc.forced(ops, True)
+    walk, walk_states = sc.forced(ops, False)
+    bound = 2e-5 if kind == "mlstm" else 1e-6
+    for out, states in results.values():
+        assert rel(rows(out), rows(exp)) < bound
+        for s, e in zip(states, exp_states):
+            assert rel(s, e) < 1e-6
+    out, states = results[128]
+    if kind == "retention":
+        assert rel(out, exp) < 1.2 * max(rel(walk, exp), rel(results[64][0], exp))
+    # (the matrix state: the normaliser's and the maximum's few numbers are a rounding off or not)
+    assert rel(states[0], exp_states[0]) < 1.2 * max(rel(walk_states[0], exp_states[0]), rel(results[64][1][0], exp_states[0]))
+    assert ops.lib.ttie_tc_error() == 0
+
+
+@pytest.mark.parametrize("tokens", [64, 128])
+@pytest.mark.parametrize("kind", ["retention", "mlstm"])
+def test_chunks_in_passes_carry_on(ops, monkeypatch, kind, tokens):
+    """Room for two chunks' states: a step of 700 tokens runs in passes, with the state between them."""
+    monkeypatch.setattr(type(ops), "_chunk_tokens", staticmethod(lambda *a: tokens))
+    sc = Scan(kind, [500, 200], 2, 64, 128, seed=4)
+    once, states = sc.forced(ops, True)
+    ops.scan_chunk_bytes = 2 * 2 * 64 * 128 * 4
+    passes, pass_states = sc.forced(ops, True)
+    assert sc.launched > 3
+    assert rel(passes, once.double()) < 1e-5 and all(rel(a, b.double()) < 1e-6 for a, b in zip(pass_states, states))

@@ -93,3 +93,11 @@ def test_float32_products_on_tensor_cores_by_shape_and_alignment():
     assert ok(x[:, 4:], w[:, 4:]) and not ok(torch.zeros(64, 2049)[:, :2048], w)        # a stride that is not a multiple of 4
     assert not ok(x, w[:511]) and not ok(x[:, :512], w[:, :512]) and ok(torch.zeros(33, 128), torch.zeros(12288, 128))
     assert not ok(x[:32, :1020], torch.zeros(4096, 1020)) and ok(x[:32, :1024], w[:, :1024])
+
+
+@pytest.mark.parametrize("mode,lens,key,value,dtype,tokens", [
+    (RETENTION, [2048], 128, 128, torch.bfloat16, 128), (MLSTM, [128], 64, 128, torch.bfloat16, 128), (RETENTION, [100] * 4, 128, 128, torch.bfloat16, 128),
+    (RETENTION, [2048], 64, 64, torch.bfloat16, 64), (RETENTION, [2048], 128, 136, torch.bfloat16, 64), (RETENTION, [2048], 128, 128, torch.float32, 64),
+    (WKV, [2048], 128, 128, torch.bfloat16, 64), (RETENTION, [1] * 23 + [256], 128, 128, torch.bfloat16, 64), (MLSTM, [1] * 31 + [2000], 64, 128, torch.bfloat16, 128)])
+def test_tokens_of_a_chunk(mode, lens, key, value, dtype, tokens):
+    assert CudaOps._chunk_tokens(mode, dtype, sum(lens), len(lens), key, value) == tokens

@@ -30,7 +30,7 @@
 // a sum that is not finite, and a row of A, or of W within the range of K, whose largest value is below 2^-95 is marked with a NaN,
 // since its lower planes reach into numbers that bfloat16 does not have (2^-126 and less).
 // Every mbarrier wait is bounded by a clock deadline; one that runs out records a code and the roles leave their loops.
-#include "common.cuh"
+#include "planes.cuh"
 #include <cuda.h>
 #include <atomic>
 using namespace ttie;
@@ -117,25 +117,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
-// 2 P values into their three planes, pairs of bfloat16 (the first value in the lower half): the nearest bfloat16 (ties away from zero), the
-// rest's leading 8 bits, what is left (at most 7 bits, so nothing is lost).  Integer and add instructions, a step for all
-// values at a time: a chain of conversions, pair by pair, was measured at 2,000 clocks for a thread's 64 values.
-template <int P>
-__device__ __forceinline__ void split_values(float (&x)[2 * P], uint32_t (&p0)[P], uint32_t (&p1)[P], uint32_t (&p2)[P]) {
-    uint32_t t[2 * P];
-#pragma unroll
-    for (int i = 0; i < 2 * P; ++i) t[i] = __float_as_uint(x[i]) + 0x8000u;
-#pragma unroll
-    for (int i = 0; i < P; ++i) p0[i] = __byte_perm(t[2 * i], t[2 * i + 1], 0x7632);
-#pragma unroll
-    for (int i = 0; i < 2 * P; ++i) x[i] -= __uint_as_float(t[i] & 0xffff0000u);       // exact; a NaN or an infinity leaves a NaN here
-#pragma unroll
-    for (int i = 0; i < P; ++i) p1[i] = __byte_perm(__float_as_uint(x[2 * i]), __float_as_uint(x[2 * i + 1]), 0x7632);
-#pragma unroll
-    for (int i = 0; i < 2 * P; ++i) x[i] -= __uint_as_float(__float_as_uint(x[i]) & 0xffff0000u);
-#pragma unroll
-    for (int i = 0; i < P; ++i) p2[i] = __byte_perm(__float_as_uint(x[2 * i]), __float_as_uint(x[2 * i + 1]), 0x7632);
-}
 // From the OR of a row's first planes: whether its largest value is below 2^-95 (its exponent's upper three bits are 0) and not 0
 __device__ __forceinline__ bool is_tiny(uint32_t m) {
     m = (m | m >> 16) & 0x7fffu;

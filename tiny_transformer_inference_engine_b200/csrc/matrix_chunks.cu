@@ -1,5 +1,5 @@
 // The matrix-state recurrences of matrix_memory.cu (retention, the xLSTM matrix memory, the RWKV-style time mix) over prompts, in
-// chunks of 64 tokens instead of token by token.
+// chunks of 64 tokens instead of token by token (chunks of 128 with products on tcgen05: matrix_chunks_tc.cu; both share matrix_chunks.cuh).
 //
 // A token-by-token walk has no parallelism but the state's elements and waits for its own chain: one prompt of 2,048 tokens and 16
 // heads of 128 x 128 took 514 us at 3 TFLOP/s.  Over a chunk the same sums are four small matrix products, and only the state
@@ -41,66 +41,14 @@
 // of its out per SM instead of three its mixer took 257 us, 240 with them.
 // Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
 // 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 3.4e-8 (4.5e-8).
-#include "common.cuh"
+#include "matrix_chunks.cuh"
 #include "run_reduce.cuh"
-#include <math.h>
-#include <type_traits>
 using namespace ttie;
+using namespace ttie::chunks;
 
 namespace {
 constexpr int CT = 64;                       // tokens per chunk
 constexpr int VT_COLS = 64, VLD = VT_COLS + 8;  // value columns per pass; row pitch of the staged values
-constexpr int CARRY = 128;                   // threads of a carry block
-enum Mode { RET = 0, MLSTM = 1, WKV = 2 };
-
-struct ChunkArgs {
-    const void* q; const void* k; long long ld_qk;                    // [T, H*D]; float32 (retention) or bfloat16
-    const void* v; long long ld_v;                                    // [T, H*Dv], bfloat16 or (retention) float32
-    const float* pre; long long ld_pre; float cap;                    // mlstm: gate pre-activations [T, 2H]
-    const float* decay;                                               // retention [H]; wkv [T, H*D]
-    const float* u;                                                   // wkv [H*D]
-    bool v_f32;                                                       // v is float32
-    float* S; float* nrm; float* mx; int state_rows;                  // state rows (mlstm: normaliser and running maximum too)
-    const void* x; long long ld_x; int d; float* prev; int prev_rows; // wkv: the mixer's input and the rows that keep its last token
-    const int* qsl; const int* slot_ids; int num_seqs;
-    float* out;                                                       // [T, H*Dv]
-    int H, D, Dv, Dpad; float qscale;
-    int slot_lo, slots;                                               // the chunk numbers of this pass
-    float* part;                                                      // [slots, H, Dv, Dpad]
-    float* aux;                                                       // mlstm: [slots, H, Dpad] normaliser sums; wkv: [slots, H, 2, Dpad] chunk decays and what rounding them left
-    double2* span;                                                    // mlstm: [slots, H] (F at the end, max of x)
-    float2* mm;                                                       // mlstm: [slots, H] the running maximum before and behind the chunk
-};
-
-__device__ __forceinline__ int state_row(int slot, int num_rows) { return slot < 0 ? num_rows - 1 : slot; }
-
-// chunk number -> request, chunk of the request, first token (of the step's rows) and number of tokens; false: the number is not in use
-__device__ __forceinline__ bool find_chunk(const int* qsl, int num_seqs, int number, int& s, int& c, int& t0, int& n) {
-    int lo = 0, hi = num_seqs - 1;
-    while (lo < hi) {                                                 // the last request whose first number is <= number
-        const int mid = (lo + hi + 1) >> 1;
-        if ((qsl[mid] >> 6) + mid <= number) lo = mid; else hi = mid - 1;
-    }
-    s = lo;
-    c = number - (qsl[s] >> 6) - s;
-    const int len = qsl[s + 1] - qsl[s];
-    t0 = qsl[s] + c * CT;
-    n = min(CT, len - c * CT);
-    return c >= 0 && n > 0;
-}
-
-// x^n for 0 <= n <= 64 in 64 bits by squaring (0^0 = 1: a head that keeps nothing still sees the token itself): seven roundings at most, a
-// tenth of the time of the general function
-__device__ __forceinline__ double power(double x, int n) {
-    double r = 1.0;
-#pragma unroll
-    for (int b = 0; b < 7; ++b) {
-        if (n >> b & 1) r *= x;
-        x *= x;
-    }
-    return r;
-}
-
 // ---- planes
 // a pair of values as three pairs of bfloat16 whose sum it is
 __device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
@@ -118,7 +66,6 @@ __device__ __forceinline__ void split3(double x, uint16_t& p0, uint16_t& p1, uin
     const __nv_bfloat16 b = __float2bfloat16_rn(r);
     p0 = __bfloat16_as_ushort(a); p1 = __bfloat16_as_ushort(b); p2 = __bfloat16_as_ushort(__float2bfloat16_rn((r - __bfloat162float(b)) + lo));
 }
-__device__ __forceinline__ float2 unpack(uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); }
 
 __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -195,18 +142,6 @@ __device__ __forceinline__ const uint16_t* at_rows_a(const uint16_t* base, int l
     return base + (k0 + (lane & 7) + (lane >> 4) * 8) * ld + m0 + ((lane >> 3) & 1) * 8;
 }
 
-// eight consecutive values of a row as floats (zeros where `in` is false)
-__device__ __forceinline__ void load8(const float* p, bool in, float (&o)[8]) {
-    const float4 a = in ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 b = in ? *reinterpret_cast<const float4*>(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-}
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, bool in, float (&o)[8]) {
-    const uint4 a = in ? *reinterpret_cast<const uint4*>(p) : make_uint4(0u, 0u, 0u, 0u);
-    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { const float2 f = unpack(w[i]); o[2 * i] = f.x; o[2 * i + 1] = f.y; }
-}
 // eight values into PL planes at element offset `at`, planes `step` elements apart (PL 1: the values are bfloat16 already)
 template <int PL>
 __device__ __forceinline__ void store_planes(uint16_t* base, int step, int at, const float (&x)[8]) {
@@ -246,151 +181,6 @@ __device__ __forceinline__ void stage_values(uint16_t* v_s, const VT* vp, long l
     stage_rows<VPL, VT_COLS, VLD, NT>(v_s, vp + col0, ld, [&](int j, int c) { return j < n && col0 + c < Dv; }, [](int, float (&)[8]) {});
 }
 
-// log input gate and log forget gate of a token
-__device__ __forceinline__ float2 log_gates(const ChunkArgs& a, int token, int h) {
-    const float* g = a.pre + (size_t)token * a.ld_pre;
-    const float z = a.cap * tanhf(g[a.H + h] / a.cap);
-    return make_float2(a.cap * tanhf(g[h] / a.cap), fminf(z, 0.f) - log1pf(expf(-fabsf(z))));
-}
-
-// ---- the walk's operations, for what is not finite
-__device__ __forceinline__ bool finite4(float x, float y, float z, float w) { return (x - x) + (y - y) + ((z - z) + (w - w)) == 0.f; }
-
-// four state elements (dv, ch .. ch + 3) of a head over the chunk's tokens; normaliser: its elements ch .. ch + 3.  mlstm: m is the running maximum
-// before the chunk, m_end the one that the result is scaled to
-template <int MODE>
-__device__ __forceinline__ float4 walk_state(const ChunkArgs& a, int t0, int n, int h, int dv, int ch, bool normaliser, float4 S4, float m, float m_end) {
-    float S[4] = {S4.x, S4.y, S4.z, S4.w};
-    const float decay = MODE == RET ? a.decay[h] : 0.f;
-#pragma unroll 1
-    for (int t = t0; t < t0 + n; ++t) {
-        const size_t at = (size_t)t * a.ld_v + h * a.Dv + dv;
-        float v = 1.f, fa = decay, ib = 1.f;
-        if (!normaliser) v = a.v_f32 ? reinterpret_cast<const float*>(a.v)[at] : to_f32(reinterpret_cast<const __nv_bfloat16*>(a.v)[at]);
-        if constexpr (MODE == MLSTM) {
-            const float2 g = log_gates(a, t, h);
-            const float next = fmaxf(g.y + m, g.x);
-            fa = expf(g.y + m - next); ib = expf(g.x - next);
-            m = next;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const bool in = ch + i < a.D;                                             // (padded channels have keys and decays of zero)
-            const size_t kat = (size_t)t * a.ld_qk + h * a.D + ch + i;
-            const float k = !in ? 0.f : MODE == RET ? reinterpret_cast<const float*>(a.k)[kat] : to_f32(reinterpret_cast<const __nv_bfloat16*>(a.k)[kat]);
-            if constexpr (MODE == WKV) fa = in ? a.decay[(size_t)t * a.H * a.D + h * a.D + ch + i] : 0.f;
-            const float bk = ib * k;
-            S[i] = fmaf(fa, S[i], normaliser ? bk : bk * v);
-        }
-    }
-    if constexpr (MODE == MLSTM) {
-        const float f = expf(m - m_end);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) S[i] *= f;
-    }
-    return make_float4(S[0], S[1], S[2], S[3]);
-}
-
-// the read-outs of a chunk and head, 128 threads: a thread per value column, eight key channels of its state at a time over all tokens.  `sm`: 7 * CT
-// floats of shared memory that nothing else uses any more
-template <int MODE, typename VT>
-__device__ __forceinline__ void walk_out(const ChunkArgs& a, size_t unit, int t0, int n, int h, float* sm) {
-    using QT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
-    const QT* qp = reinterpret_cast<const QT*>(a.q) + (size_t)t0 * a.ld_qk + h * a.D;
-    const QT* kp = reinterpret_cast<const QT*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
-    const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
-    const size_t ld_o = (size_t)a.H * a.Dv;
-    float* op = a.out + (size_t)t0 * ld_o + h * a.Dv;
-    const int tid = threadIdx.x;
-    float* gate = sm;                                                                 // mlstm: [CT][3] state decay, input weight, e^-m
-    float* den = sm + 3 * CT;                                                         // mlstm: [4][CT] the warps' shares of n . q
-    if constexpr (MODE == MLSTM) {
-        if (tid == 0) {
-            float m = a.mm[unit].x;
-#pragma unroll 1
-            for (int t = 0; t < n; ++t) {
-                const float2 g = log_gates(a, t0 + t, h);
-                const float next = fmaxf(g.y + m, g.x);
-                gate[3 * t] = expf(g.y + m - next); gate[3 * t + 1] = expf(g.x - next); gate[3 * t + 2] = expf(-next);
-                m = next;
-            }
-        }
-        __syncthreads();
-        float nv = tid < a.Dpad ? a.aux[unit * a.Dpad + tid] : 0.f;
-#pragma unroll 1
-        for (int t = 0; t < n; ++t) {
-            const float k = tid < a.D ? to_f32(kp[(size_t)t * a.ld_qk + tid]) : 0.f, q = tid < a.D ? to_f32(qp[(size_t)t * a.ld_qk + tid]) * a.qscale : 0.f;
-            nv = fmaf(gate[3 * t], nv, gate[3 * t + 1] * k);
-            const float p = warp_sum(tid < a.Dpad ? nv * q : 0.f);
-            if ((tid & 31) == 0) den[(tid >> 5) * CT + t] = p;
-        }
-        __syncthreads();
-    }
-    for (int dv = tid; dv < a.Dv; dv += 128) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < a.Dpad; c0 += 8) {
-            const bool in = c0 < a.D;                                                 // (both are multiples of 8)
-            float S[8];
-            load8(a.part + (unit * a.Dv + dv) * a.Dpad + c0, true, S);
-#pragma unroll 1
-            for (int t = 0; t < n; ++t) {
-                float k[8], q[8], acc = 0.f;
-                load8(kp + (size_t)t * a.ld_qk + c0, in, k);
-                load8(qp + (size_t)t * a.ld_qk + c0, in, q);
-                const float v = to_f32(vp[(size_t)t * a.ld_v + dv]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if constexpr (MODE == WKV) {
-                        const float kv = k[i] * v;
-                        acc = fmaf(q[i], fmaf(in ? a.u[h * a.D + c0 + i] : 0.f, kv, S[i]), acc);
-                        S[i] = fmaf(in ? a.decay[(size_t)(t0 + t) * a.H * a.D + h * a.D + c0 + i] : 0.f, S[i], kv);
-                    } else {
-                        S[i] = MODE == RET ? fmaf(a.decay[h], S[i], k[i] * v) : fmaf(gate[3 * t], S[i], gate[3 * t + 1] * k[i] * v);
-                        acc = fmaf(S[i], MODE == MLSTM ? q[i] * a.qscale : q[i], acc);
-                    }
-                }
-                float* o = op + (size_t)t * ld_o + dv;
-                if (c0 > 0) acc += *o;
-                if (MODE == MLSTM && c0 + 8 >= a.Dpad)
-                    acc /= fmaxf(fabsf((den[t] + den[CT + t]) + (den[2 * CT + t] + den[3 * CT + t])), gate[3 * t + 2]) + 1e-6f;
-                *o = acc;
-            }
-        }
-    }
-}
-
-// ---- the matrix memory's gates over a chunk: threads 0 .. 63 (two warps), thread = token.  F: inclusive sum of the log forget gates,
-// x = i - F, X: inclusive maximum of x.  Tokens behind the chunk's n-th: F stays, x = -inf.  `half` holds four doubles in shared memory.
-__device__ __forceinline__ void chunk_gates(const ChunkArgs& a, int t0, int n, int h, double* half, double& F, double& x, double& X) {
-    const int j = threadIdx.x, lane = j & 31;
-    double f = 0.0, ig = -INFINITY;
-    x = X = 0.0;
-    if (j < n) {
-        const float2 g = log_gates(a, t0 + j, h);
-        ig = (double)g.x;
-        f = (double)g.y;
-    }
-    F = f;
-    if (j < CT) {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const double y = __shfl_up_sync(0xffffffffu, F, o); if (lane >= o) F += y; }
-        if (j == 31) half[0] = F;
-    }
-    __syncthreads();
-    if (j < CT) {
-        if (j >= 32) F += half[0];
-        x = ig - F;
-        X = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const double y = __shfl_up_sync(0xffffffffu, X, o); if (lane >= o) X = fmax(X, y); }
-        if (j == 31) half[1] = X;
-    }
-    __syncthreads();
-    if (j >= 32 && j < CT) X = fmax(X, half[1]);
-    if (j == CT - 1) { half[2] = F; half[3] = X; }
-    __syncthreads();
-}
-
 // ------------------------------------------------------------------------------------------- chunk_sum
 // wkv: the chunk's last tokens are added in 64 bits on the ordinary cores, behind the tensor cores' sum of the others.  Under strong decays
 // they are the state, and what the tensor cores cut from products of very different sizes showed there: decays of e^-1 to e^-20 a token
@@ -415,7 +205,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
     TTIE_PDL_ENTRY();
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 3, part = tid >> 7;      // (part: which share of the key channels)
     int s, c, t0, n;
-    if (!find_chunk(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
+    if (!find_chunk<CT>(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
     const size_t unit = (size_t)blockIdx.x * a.H + h;
     const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
     auto stage_tail = [&](int col0) {
@@ -474,9 +264,9 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
             if (tid < CT) wt[tid] = tid < n ? (float)power((double)a.decay[h], n - 1 - tid) : 0.f;
         } else {
             double F, x, X;
-            chunk_gates(a, t0, n, h, half, F, x, X);
-            if (tid < CT) wt[tid] = expf((float)(x - half[3]));
-            if (tid == 0) a.span[unit] = make_double2(half[2], half[3]);
+            chunk_gates<CT>(a, t0, n, h, half, F, x, X);
+            if (tid < CT) wt[tid] = expf((float)(x - half[5]));
+            if (tid == 0) a.span[unit] = make_double2(half[4], half[5]);
         }
         __syncthreads();
         using KT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
@@ -556,100 +346,6 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
     }
 }
 
-// ------------------------------------------------------------------------------------------- chunk_carry
-// A thread per four elements of a (request, head)'s state; the request's chunks of this pass one after the other, the next chunks'
-// sums on their way meanwhile.  mlstm: the elements behind the state are the normaliser's.
-template <int MODE>
-__global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
-    __shared__ float powers[2];
-    TTIE_PDL_ENTRY();
-    const int h = blockIdx.y, s = blockIdx.z;
-    const int q0 = a.qsl[s], len = a.qsl[s + 1] - q0;
-    const int base = (q0 >> 6) + s;
-    const int c_lo = max(0, a.slot_lo - base), c_hi = min((len + CT - 1) / CT, a.slot_lo + a.slots - base);
-    if (c_lo >= c_hi) return;
-    if (MODE == RET) {
-        const int last = len - (c_hi - 1) * CT;
-        if (threadIdx.x < 2) powers[threadIdx.x] = (float)power((double)a.decay[h], threadIdx.x == 0 ? CT : min(CT, last));
-        __syncthreads();
-    }
-    const size_t row = state_row(a.slot_ids[s], a.state_rows);
-    if (MODE == WKV && h == 0 && blockIdx.x == 0 && c_hi == (len + CT - 1) / CT) {     // the request's last input is the next step's previous token
-        const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(a.x) + (size_t)(q0 + len - 1) * a.ld_x;
-        float* p = a.prev + (size_t)state_row(a.slot_ids[s], a.prev_rows) * a.d;
-        for (int i = threadIdx.x; i < a.d; i += blockDim.x) p[i] = to_f32(x[i]);
-    }
-    const int state = a.Dv * a.Dpad;
-    const int e = (blockIdx.x * CARRY + threadIdx.x) * 4;
-    if (e >= state + (MODE == MLSTM ? a.Dpad : 0)) return;
-    const bool in_state = e < state;                                                  // (only mlstm has elements behind it)
-    float* sp = in_state ? a.S + (row * a.H + h) * state + e : a.nrm + (row * a.H + h) * a.Dpad + (e - state);
-    float* pp = in_state ? a.part + e : a.aux + (e - state);
-    const size_t step = (size_t)a.H * (in_state ? state : a.Dpad);
-    const size_t unit = (size_t)(base + c_lo - a.slot_lo) * a.H + h;                  // of chunk c_lo
-    pp += (in_state ? state : a.Dpad) * unit;
-    float4 S = *reinterpret_cast<const float4*>(sp);
-    // the running maximum as the request's state row has it; every CTA reads the row here, so the new one is written by chunk_out
-    double m = MODE == MLSTM ? (double)a.mx[row * a.H + h] : 0.0;
-    // two batches of chunks in registers: the next one's sums are on their way while this one is worked off
-    constexpr int AHEAD = MODE == RET ? 8 : 4;
-    float4 p[2][AHEAD], w[2][MODE == WKV ? AHEAD : 1], wl[2][MODE == WKV ? AHEAD : 1];
-    double2 sc[2][MODE == MLSTM ? AHEAD : 1];
-    auto fetch = [&](int b, int c0) {
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i) {
-            if (c0 + i >= c_hi) continue;
-            const size_t off = (size_t)(c0 + i - c_lo);
-            p[b][i] = *reinterpret_cast<const float4*>(pp + off * step);
-            if constexpr (MODE == WKV) {
-                const float* f = a.aux + 2 * (unit + off * a.H) * a.Dpad + e % a.Dpad;
-                w[b][i] = *reinterpret_cast<const float4*>(f);
-                wl[b][i] = *reinterpret_cast<const float4*>(f + a.Dpad);
-            }
-            if constexpr (MODE == MLSTM) sc[b][i] = a.span[unit + off * a.H];
-        }
-    };
-    auto work = [&](int b, int c0) {
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i) {
-            if (c0 + i >= c_hi) continue;
-            const size_t off = (size_t)(c0 + i - c_lo);
-            *reinterpret_cast<float4*>(pp + off * step) = S;
-            const float4 before = S;
-            const double m_before = m;
-            float4 f, x = p[b][i];
-            if constexpr (MODE == RET) {
-                const float d = powers[c0 + i == c_hi - 1 ? 1 : 0];
-                f = make_float4(d, d, d, d);
-            } else if constexpr (MODE == WKV) {
-                f = w[b][i];
-                const float4 l = wl[b][i];
-                x = make_float4(fmaf(l.x, S.x, x.x), fmaf(l.y, S.y, x.y), fmaf(l.z, S.z, x.z), fmaf(l.w, S.w, x.w));
-            } else {
-                const double next = (double)(float)(sc[b][i].x + fmax(m, sc[b][i].y));      // as the state row will hold it
-                const float d = expf((float)(sc[b][i].x + m - next)), own = expf((float)(sc[b][i].x + sc[b][i].y - next));
-                f = make_float4(d, d, d, d);
-                x = make_float4(x.x * own, x.y * own, x.z * own, x.w * own);
-                if (e == 0) a.mm[unit + off * a.H] = make_float2((float)m, (float)next);
-                m = next;
-            }
-            S.x = fmaf(f.x, S.x, x.x); S.y = fmaf(f.y, S.y, x.y); S.z = fmaf(f.z, S.z, x.z); S.w = fmaf(f.w, S.w, x.w);
-            if (!finite4(S.x, S.y, S.z, S.w)) {
-                const int el = in_state ? e : e - state;
-                S = walk_state<MODE>(a, q0 + (c0 + i) * CT, min(CT, len - (c0 + i) * CT), h, in_state ? el / a.Dpad : 0, el % a.Dpad, !in_state, before, (float)m_before, (float)m);
-            }
-        }
-    };
-    fetch(0, c_lo);
-    for (int c0 = c_lo; c0 < c_hi; c0 += 2 * AHEAD) {
-        fetch(1, c0 + AHEAD);
-        work(0, c0);
-        fetch(0, c0 + 2 * AHEAD);
-        work(1, c0 + AHEAD);
-    }
-    *reinterpret_cast<float4*>(sp) = S;
-}
-
 // ------------------------------------------------------------------------------------------- chunk_out
 template <int MODE, int KP> struct OutSmem {
     static constexpr int LD = KP + 8, FLD = KP + 4;
@@ -669,7 +365,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
     TTIE_PDL_ENTRY();
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     int s, c, t0, n;
-    if (!find_chunk(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
+    if (!find_chunk<CT>(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
     const size_t unit = (size_t)blockIdx.x * a.H + h;
     using QT = typename std::conditional<MODE == RET, float, __nv_bfloat16>::type;
     const QT* qp = reinterpret_cast<const QT*>(a.q) + (size_t)t0 * a.ld_qk + h * a.D;
@@ -825,7 +521,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
             __syncthreads();
         } else {
             double F, x, X;
-            chunk_gates(a, t0, n, h, half, F, x, X);
+            chunk_gates<CT>(a, t0, n, h, half, F, x, X);
             const float2 mm = a.mm[unit];
             const double m = (double)mm.x;
             if (tid < CT) { xs[tid] = x; Ms[tid] = fmax(m, X); Fs[tid] = F; }
@@ -943,7 +639,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
             odd = odd || (r0 < n && !finite4(y[0], y[1], 0.f, 0.f)) || (r1 < n && !finite4(y[2], y[3], 0.f, 0.f));
         }
     }
-    if (__syncthreads_or(odd)) walk_out<MODE, VT>(a, unit, t0, n, h, reinterpret_cast<float*>(pl));
+    if (__syncthreads_or(odd)) walk_out<MODE, CT, VT>(a, unit, t0, n, h, reinterpret_cast<float*>(pl));
 }
 
 template <int MODE, int KP, typename VT>
@@ -961,7 +657,7 @@ int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
     const dim3 grid(slots, a.H);
     const dim3 carry(ceil_div(a.Dv * a.Dpad + (MODE == MLSTM ? a.Dpad : 0), 4 * CARRY), a.H, a.num_seqs);
     TTIE_LAUNCH((chunk_sum_kernel<MODE, KP, VT>), grid, (SumSmem<MODE, KP>::NT), sum_smem, st, a);
-    TTIE_LAUNCH((chunk_carry_kernel<MODE>), carry, CARRY, 0, st, a);
+    TTIE_LAUNCH((chunk_carry_kernel<MODE, CT>), carry, CARRY, 0, st, a);
     TTIE_LAUNCH((chunk_out_kernel<MODE, KP, VT>), grid, 128, out_smem, st, a);
     TTIE_CHECK_LAUNCH("matrix_chunks");
     return 0;
@@ -970,13 +666,14 @@ int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
 
 // mode: 0 retention (q, k float32; v either type), 1 mlstm, 2 wkv (q, k, v bfloat16).  T: rows of the step.  D and Dv multiples of
 // 8, D at most 128, rows that start on 16 bytes.  part / aux / span / mm hold `slots` chunk numbers' worth; a step of more chunk
-// numbers (T / 64 + requests) is done in passes.
+// numbers (T / chunk + requests) is done in passes.  chunk: tokens of one, 64 or (modes 0 and 1, bfloat16 values of at most 128 columns) 128.
 extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, int v_dtype,
                                   const float* pre, long long ld_pre, float cap, const float* decay, const float* u, float* S, float* nrm,
                                   float* mx, int state_rows, const void* x, long long ld_x, int d, float* prev, int prev_rows, const int* qsl,
                                   const int* slot_ids, int num_seqs, int T, float* out, int H, int D, int Dv, int Dpad, float qscale,
-                                  float* part, float* aux, void* span, void* mm, int slots, void* stream) {
+                                  float* part, float* aux, void* span, void* mm, int slots, int chunk, void* stream) {
     if (num_seqs <= 0 || T <= 0) return 0;
+    if (chunk != CT && (chunk != 128 || mode == WKV || v_dtype != kBF16 || Dv > 128)) TTIE_FAIL("matrix_chunks: chunks of %d tokens, mode %d, %d value channels", chunk, mode, Dv);
     if (mode < 0 || mode > 2 || (v_dtype != kBF16 && !(v_dtype == kF32 && mode == RET))) TTIE_FAIL("matrix_chunks: mode %d with values of type %d", mode, v_dtype);
     const int ce = mode == RET ? 4 : 8, ve = v_dtype == kF32 ? 4 : 8;                 // values per 16 bytes
     if (D < 8 || D > 128 || D % 8 || Dv < 8 || Dv % 8 || Dpad < D || Dpad > 128 || Dpad % 8 || ld_qk % ce || ld_v % ve || (mode == WKV && D != Dv)
@@ -989,8 +686,9 @@ extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long l
     a.S = S; a.nrm = nrm; a.mx = mx; a.state_rows = state_rows; a.x = x; a.ld_x = ld_x; a.d = d; a.prev = prev; a.prev_rows = prev_rows;
     a.qsl = qsl; a.slot_ids = slot_ids; a.num_seqs = num_seqs; a.out = out; a.H = H; a.D = D; a.Dv = Dv; a.Dpad = Dpad; a.qscale = qscale;
     a.part = part; a.aux = aux; a.span = (double2*)span; a.mm = (float2*)mm;
-    const int total = T / CT + num_seqs;
     cudaStream_t st = (cudaStream_t)stream;
+    if (chunk == 128) return matrix_chunks_tc(mode, a, T, slots, st);
+    const int total = T / CT + num_seqs;
     for (int first = 0; first < total; first += slots) {
         const int cnt = total - first < slots ? total - first : slots;
         int rc;

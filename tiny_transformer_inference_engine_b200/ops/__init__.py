@@ -141,7 +141,7 @@ _SIGNATURES = {
                             _c_int, _c_int, _c_int, _c_void, _c_int, _c_void],
     "ttie_matrix_chunks": [_c_int, _c_void, _c_void, _c_ll, _c_void, _c_ll, _c_int, _c_void, _c_ll, _c_float, _c_void, _c_void, _c_void, _c_void,
                            _c_void, _c_int, _c_void, _c_ll, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_int, _c_void, _c_int, _c_int,
-                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_void],
+                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void],
     "ttie_head_norm_gate": [_c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void, _c_int, _c_void],
     "ttie_activation": [_c_void, _c_void, _c_ll, _c_int, _c_float, _c_float, _c_int, _c_int, _c_void],
     "ttie_matrix_state_pad": [_c_int],
@@ -1429,12 +1429,13 @@ class CudaOps:
     scan_chunk_bytes = 128 << 20            # bytes of the states between chunks that are held at a time (about the L2: a longer step runs in passes)
     # us of a scan in chunks by kind (retention, mlstm, wkv): the launches, a request, a state element of a request, a token and state element
     scan_chunk_cost = ((31.0, 0.3, 8.5e-6, 1.6e-7), (24.0, 0.3, 7.5e-6, 1.6e-7), (28.0, 0.3, 1.45e-5, 3.6e-7))
+    scan_chunk128_cost = ((24.0, 0.3, 6.9e-6, 4.4e-8), (24.0, 0.3, 5.0e-6, 8.4e-8))      # the same in chunks of 128 tokens (retention, mlstm)
     scan_walk_cost = ((4.0, 0.21, 8.2e-7), (4.0, 0.19, 8.2e-7), (4.0, 0.18, 8.2e-7))   # of a walk: the launch, a token of the longest request, a token and state element of the step
     # of the layer's eager pass around it: host us with a walk, what chunks' call adds; us of its other kernels, a token and squared width of them
     scan_pass_cost = ((90.0, 10.0, 35.0, 6e-9), (110.0, 2.0, 35.0, 6e-9), (126.0, 14.0, 60.0, 6e-9))
 
     def _in_chunks(self, mode, num_tokens, num_seqs, longest, num_heads, dim, v_dim, q, k, v) -> bool:
-        """Whether a step's matrix-state recurrence runs in chunks of 64 tokens on tensor cores (``csrc/matrix_chunks.cu``) rather than
+        """Whether a step's matrix-state recurrence runs in chunks of 64 or 128 tokens on tensor cores (``_chunk_tokens``) rather than
         token by token, for the head sizes and rows that 16-byte loads and 16-channel products take.  ``longest``: the most tokens that a request brings
         (StepContext.max_q_len, which also holds for a captured graph); None: the step's tokens less one for every other request.
 
@@ -1443,16 +1444,18 @@ class CudaOps:
         figures above give both within a fifth over widths of 512 to 4,096, 1 to 24 requests and 16 to 1,024 tokens.  And an eager pass of the layer
         takes the longer of its kernels' and its host's time, of which chunks need more: they pay where the pass is shorter with them
         (the whole mixer of 300 tokens at width 1,024, walk | chunks: retention 105 | 99, mlstm 108 | 111, wkv 126 | 141).  The scan alone, walk | chunks,
-        us, width 2,048: one request of 128 tokens retention 32 | 40, mlstm 31 | 30, wkv 26 | 34, of 512 tokens 116 | 49, 107 | 34,
-        93 | 41; eight of 16 tokens 30 | 54, 22 | 36, 17 | 41, of 64 tokens 97 | 60, 68 | 41, 55 | 44; 256 tokens beside 23 decoding
-        requests 88 | 85, 81 | 52, 63 | 87."""
+us, width 2,048: one request of 128 tokens retention 32 | 25, mlstm 33 | 25, wkv 26 | 34, of 512 tokens 116 | 28, 107 | 28,
+        93 | 41; eight of 16 tokens 32 | 35, 25 | 30, 17 | 41, of 64 tokens 99 | 38, 71 | 32, 55 | 44; 256 tokens beside 23 decoding
+        requests 92 | 95, 85 | 64, 63 | 87."""
         if not 8 <= dim <= 128 or dim % 8 or v_dim % 8:
             return False
         others = num_seqs - 1
         if longest is None:
             longest = num_tokens - others
         if self.scan_chunk_tokens is None:
-            state, (start, token, work), (base, request, element, each) = num_heads * dim * v_dim, self.scan_walk_cost[mode], self.scan_chunk_cost[mode]
+            state, (start, token, work) = num_heads * dim * v_dim, self.scan_walk_cost[mode]
+            large = self._chunk_tokens(mode, v.dtype, num_tokens, num_seqs, dim, v_dim) == 128
+            base, request, element, each = (self.scan_chunk128_cost if large else self.scan_chunk_cost)[mode]
             host, more, rest, product = self.scan_pass_cost[mode]
             rest += product * num_tokens * (num_heads * v_dim) ** 2
             walk = start + max(token * longest, work * num_tokens * state) + rest
@@ -1466,9 +1469,19 @@ class CudaOps:
                 return False
         return True
 
+    @staticmethod
+    def _chunk_tokens(mode, v_dtype, num_tokens, num_seqs, key_pad, v_dim) -> int:
+        """Tokens of a chunk: 128 with products on tcgen05 (csrc/matrix_chunks_tc.cu: retention and the matrix memory, bfloat16 values of at most 128
+        columns), else 64 (csrc/matrix_chunks.cu).  us, 64 | 128: 16 heads of 128 x 128 one request of 2,048 tokens 99 | 49, of 128 41 | 25,
+        16 of 128 129 | 83; 16 of 64 x 128 67 | 46, 32 | 25, 74 | 61; 8 of 64 x 64 one of 300 tokens 16 | 18 (one tile of 128 rows a chunk is
+        too much for so little).  Every request has a chunk of its own, so decoded tokens beside a short portion are better
+        off with small ones: 23 and 256 tokens 95 | 102 (mlstm 64 | 75), 7 and 512 63 | 55 (49 | 47), 31 and 2,000 208 | 185 (139 | 139)."""
+        return 128 if mode < 2 and v_dtype == torch.bfloat16 and v_dim <= 128 and max(key_pad, v_dim) > 64 and num_tokens >= 24 * num_seqs else 64
+
     def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale):
         T, pad = q.shape[0], S.shape[-1]
-        total = T // 64 + num_seqs                                     # chunk numbers of the step
+        tokens = self._chunk_tokens(mode, v.dtype, T, num_seqs, pad, v_dim)
+        total = T // tokens + num_seqs                                 # chunk numbers of the step
         states = num_heads * v_dim * pad                               # floats of a chunk number: its states, their sums or decays, mlstm: spans and maxima
         slots = max(1, min(total, self.scan_chunk_bytes // (states * 4)))
         sums = num_heads * mode * pad
@@ -1480,7 +1493,7 @@ class CudaOps:
             mode, _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), self._dt(v), _ptr(pre), 0 if pre is None else pre.stride(0), float(cap),
             _ptr(decay), _ptr(u), _ptr(S), _ptr(n), _ptr(m), S.shape[0], _ptr(x), 0 if x is None else x.stride(0), 0 if x is None else x.shape[1],
             _ptr(prev), 0 if prev is None else prev.shape[0], _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), T, _ptr(out), num_heads, dim,
-            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, self._stream(q)), "matrix_chunks")
+            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, tokens, self._stream(q)), "matrix_chunks")
         self.launches += 3 * -(-total // slots)
 
     def rotate_heads(self, src, heads, dim, cs_table, rot, style, scale_from=None, scale=1.0):
