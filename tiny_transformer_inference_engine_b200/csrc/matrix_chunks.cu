@@ -667,13 +667,15 @@ int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
 // mode: 0 retention (q, k float32; v either type), 1 mlstm, 2 wkv (q, k, v bfloat16).  T: rows of the step.  D and Dv multiples of
 // 8, D at most 128, rows that start on 16 bytes.  part / aux / span / mm hold `slots` chunk numbers' worth; a step of more chunk
 // numbers (T / chunk + requests) is done in passes.  chunk: tokens of one, 64 or (modes 0 and 1, bfloat16 values of at most 128 columns) 128.
+// pre_bias (chunks of 128): bfloat16 [2H] on mlstm's gate pre-activations.
 extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, int v_dtype,
                                   const float* pre, long long ld_pre, float cap, const float* decay, const float* u, float* S, float* nrm,
                                   float* mx, int state_rows, const void* x, long long ld_x, int d, float* prev, int prev_rows, const int* qsl,
                                   const int* slot_ids, int num_seqs, int T, float* out, int H, int D, int Dv, int Dpad, float qscale,
-                                  float* part, float* aux, void* span, void* mm, int slots, int chunk, void* stream) {
+                                  float* part, float* aux, void* span, void* mm, int slots, int chunk, const void* pre_bias, void* stream) {
     if (num_seqs <= 0 || T <= 0) return 0;
     if (chunk != CT && (chunk != 128 || mode == WKV || v_dtype != kBF16 || Dv > 128)) TTIE_FAIL("matrix_chunks: chunks of %d tokens, mode %d, %d value channels", chunk, mode, Dv);
+    if (pre_bias && (chunk != 128 || mode != MLSTM)) TTIE_FAIL("matrix_chunks: a gate bias goes with mlstm in chunks of 128 tokens");
     if (mode < 0 || mode > 2 || (v_dtype != kBF16 && !(v_dtype == kF32 && mode == RET))) TTIE_FAIL("matrix_chunks: mode %d with values of type %d", mode, v_dtype);
     const int ce = mode == RET ? 4 : 8, ve = v_dtype == kF32 ? 4 : 8;                 // values per 16 bytes
     if (D < 8 || D > 128 || D % 8 || Dv < 8 || Dv % 8 || Dpad < D || Dpad > 128 || Dpad % 8 || ld_qk % ce || ld_v % ve || (mode == WKV && D != Dv)
@@ -686,6 +688,7 @@ extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long l
     a.S = S; a.nrm = nrm; a.mx = mx; a.state_rows = state_rows; a.x = x; a.ld_x = ld_x; a.d = d; a.prev = prev; a.prev_rows = prev_rows;
     a.qsl = qsl; a.slot_ids = slot_ids; a.num_seqs = num_seqs; a.out = out; a.H = H; a.D = D; a.Dv = Dv; a.Dpad = Dpad; a.qscale = qscale;
     a.part = part; a.aux = aux; a.span = (double2*)span; a.mm = (float2*)mm;
+    a.pre_bias = (const __nv_bfloat16*)pre_bias;
     cudaStream_t st = (cudaStream_t)stream;
     if (chunk == 128) return matrix_chunks_tc(mode, a, T, slots, st);
     const int total = T / CT + num_seqs;

@@ -27,6 +27,7 @@ struct ChunkArgs {
     float* aux;                                                       // mlstm: [slots, H, Dpad] normaliser sums; wkv: [slots, H, 2, Dpad] chunk decays and what rounding them left
     double2* span;                                                    // mlstm: [slots, H] (F at the end, max of x)
     float2* mm;                                                       // mlstm: [slots, H] the running maximum before and behind the chunk
+    const __nv_bfloat16* pre_bias;                                    // mlstm in chunks of 128 tokens: [2H] on the gates' pre-activations, or null
 };
 
 __device__ __forceinline__ int state_row(int slot, int num_rows) { return slot < 0 ? num_rows - 1 : slot; }
@@ -74,10 +75,13 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, bool in, float (&o
     for (int i = 0; i < 4; ++i) { const float2 f = unpack(w[i]); o[2 * i] = f.x; o[2 * i + 1] = f.y; }
 }
 // log input gate and log forget gate of a token
+template <int CT>
 __device__ __forceinline__ float2 log_gates(const ChunkArgs& a, int token, int h) {
     const float* g = a.pre + (size_t)token * a.ld_pre;
-    const float z = a.cap * tanhf(g[a.H + h] / a.cap);
-    return make_float2(a.cap * tanhf(g[h] / a.cap), fminf(z, 0.f) - log1pf(expf(-fabsf(z))));
+    float i = g[h], f = g[a.H + h];
+    if (CT == 128 && a.pre_bias) { i += __bfloat162float(a.pre_bias[h]); f += __bfloat162float(a.pre_bias[a.H + h]); }
+    const float z = a.cap * tanhf(f / a.cap);
+    return make_float2(a.cap * tanhf(i / a.cap), fminf(z, 0.f) - log1pf(expf(-fabsf(z))));
 }
 
 // ---- the walk's operations, for what is not finite
@@ -85,7 +89,7 @@ __device__ __forceinline__ bool finite4(float x, float y, float z, float w) { re
 
 // four state elements (dv, ch .. ch + 3) of a head over the chunk's tokens; normaliser: its elements ch .. ch + 3.  mlstm: m is the running maximum
 // before the chunk, m_end the one that the result is scaled to
-template <int MODE>
+template <int MODE, int CT>
 __device__ __forceinline__ float4 walk_state(const ChunkArgs& a, int t0, int n, int h, int dv, int ch, bool normaliser, float4 S4, float m, float m_end) {
     float S[4] = {S4.x, S4.y, S4.z, S4.w};
     const float decay = MODE == RET ? a.decay[h] : 0.f;
@@ -95,7 +99,7 @@ __device__ __forceinline__ float4 walk_state(const ChunkArgs& a, int t0, int n, 
         float v = 1.f, fa = decay, ib = 1.f;
         if (!normaliser) v = a.v_f32 ? reinterpret_cast<const float*>(a.v)[at] : to_f32(reinterpret_cast<const __nv_bfloat16*>(a.v)[at]);
         if constexpr (MODE == MLSTM) {
-            const float2 g = log_gates(a, t, h);
+            const float2 g = log_gates<CT>(a, t, h);
             const float next = fmaxf(g.y + m, g.x);
             fa = expf(g.y + m - next); ib = expf(g.x - next);
             m = next;
@@ -136,7 +140,7 @@ __device__ __forceinline__ void walk_out(const ChunkArgs& a, size_t unit, int t0
             double m = (double)a.mm[unit].x;                                           // (in 64 bits, as the chunks have it: over 128 tokens it drifts otherwise)
 #pragma unroll 1
             for (int t = 0; t < n; ++t) {
-                const float2 g = log_gates(a, t0 + t, h);
+                const float2 g = log_gates<CT>(a, t0 + t, h);
                 const double next = fmax((double)g.y + m, (double)g.x);
                 gate[3 * t] = expf((float)((double)g.y + m - next)); gate[3 * t + 1] = expf((float)((double)g.x - next)); gate[3 * t + 2] = expf((float)-next);
                 m = next;
@@ -196,7 +200,7 @@ __device__ __forceinline__ void chunk_gates(const ChunkArgs& a, int t0, int n, i
     double f = 0.0, ig = -INFINITY;
     x = X = 0.0;
     if (j < n) {
-        const float2 g = log_gates(a, t0 + j, h);
+        const float2 g = log_gates<CT>(a, t0 + j, h);
         ig = (double)g.x;
         f = (double)g.y;
     }
@@ -301,7 +305,7 @@ __global__ void __launch_bounds__(CARRY) chunk_carry_kernel(const ChunkArgs a) {
             S.x = fmaf(f.x, S.x, x.x); S.y = fmaf(f.y, S.y, x.y); S.z = fmaf(f.z, S.z, x.z); S.w = fmaf(f.w, S.w, x.w);
             if (!finite4(S.x, S.y, S.z, S.w)) {
                 const int el = in_state ? e : e - state;
-                S = walk_state<MODE>(a, q0 + (c0 + i) * CT, min(CT, len - (c0 + i) * CT), h, in_state ? el / a.Dpad : 0, el % a.Dpad, !in_state, before, (float)m_before, (float)m);
+                S = walk_state<MODE, CT>(a, q0 + (c0 + i) * CT, min(CT, len - (c0 + i) * CT), h, in_state ? el / a.Dpad : 0, el % a.Dpad, !in_state, before, (float)m_before, (float)m);
             }
         }
     };

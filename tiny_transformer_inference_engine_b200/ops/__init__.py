@@ -141,7 +141,7 @@ _SIGNATURES = {
                             _c_int, _c_int, _c_int, _c_void, _c_int, _c_void],
     "ttie_matrix_chunks": [_c_int, _c_void, _c_void, _c_ll, _c_void, _c_ll, _c_int, _c_void, _c_ll, _c_float, _c_void, _c_void, _c_void, _c_void,
                            _c_void, _c_int, _c_void, _c_ll, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_int, _c_void, _c_int, _c_int,
-                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void],
+                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void, _c_void],
     "ttie_head_norm_gate": [_c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void, _c_int, _c_void],
     "ttie_activation": [_c_void, _c_void, _c_ll, _c_int, _c_float, _c_float, _c_int, _c_int, _c_void],
     "ttie_matrix_state_pad": [_c_int],
@@ -1417,12 +1417,17 @@ class CudaOps:
         return (q.dtype == torch.bfloat16 and self._in_chunks(1, q.shape[0], num_seqs, max_q_len, q.shape[1] // dim, dim, v_dim, q, k, v)
                 and q.stride(0) == k.stride(0) == v.stride(0))
 
-    def mlstm_chunks(self, q, k, v, pre, S, n, m, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, cap, q_scale):
-        """The matrix memory over a step with a prompt portion, in chunks of 64 tokens: ``mlstm_gates`` and ``mlstm_scan`` in one.  ``pre``:
-        the gates' pre-activations float32 [T, 2H]; the state rows S, n and m are advanced in place.  Returns o float32 [T, H*v_dim]."""
+    def mlstm_chunks(self, q, k, v, pre, S, n, m, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, cap, q_scale, pre_bias=None):
+        """The matrix memory over a step with a prompt portion, in chunks of tokens: ``mlstm_gates`` and ``mlstm_scan`` in one.  ``pre``:
+        the gates' pre-activations float32 [T, 2H]; the state rows S, n and m are advanced in place.  ``pre_bias`` (bfloat16 [2H], where
+        ``mlstm_adds_bias``): added to ``pre``.  Returns o float32 [T, H*v_dim]."""
         out = torch.empty((q.shape[0], num_heads * v_dim), dtype=torch.float32, device=q.device)
-        self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale)
+        self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale, pre_bias)
         return out
+
+    def mlstm_adds_bias(self, v, num_seqs, pad, v_dim) -> bool:
+        """Whether ``mlstm_chunks`` takes the gates' bias (a sum apart costs two small kernels, 5 us of a layer's 127)."""
+        return self._chunk_tokens(1, v.dtype, v.shape[0], num_seqs, pad, v_dim) == 128
 
     scan_chunk_tokens = None                # None: by cost (``_in_chunks``); a number: chunks where a request may bring this many tokens
     scan_chunk_more = 0                     # and this many more for every other request
@@ -1478,7 +1483,7 @@ us, width 2,048: one request of 128 tokens retention 32 | 25, mlstm 33 | 25, wkv
         off with small ones: 23 and 256 tokens 95 | 102 (mlstm 64 | 75), 7 and 512 63 | 55 (49 | 47), 31 and 2,000 208 | 185 (139 | 139)."""
         return 128 if mode < 2 and v_dtype == torch.bfloat16 and v_dim <= 128 and max(key_pad, v_dim) > 64 and num_tokens >= 24 * num_seqs else 64
 
-    def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale):
+    def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale, pre_bias=None):
         T, pad = q.shape[0], S.shape[-1]
         tokens = self._chunk_tokens(mode, v.dtype, T, num_seqs, pad, v_dim)
         total = T // tokens + num_seqs                                 # chunk numbers of the step
@@ -1493,7 +1498,7 @@ us, width 2,048: one request of 128 tokens retention 32 | 25, mlstm 33 | 25, wkv
             mode, _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), self._dt(v), _ptr(pre), 0 if pre is None else pre.stride(0), float(cap),
             _ptr(decay), _ptr(u), _ptr(S), _ptr(n), _ptr(m), S.shape[0], _ptr(x), 0 if x is None else x.stride(0), 0 if x is None else x.shape[1],
             _ptr(prev), 0 if prev is None else prev.shape[0], _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), T, _ptr(out), num_heads, dim,
-            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, tokens, self._stream(q)), "matrix_chunks")
+            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, tokens, _ptr(pre_bias), self._stream(q)), "matrix_chunks")
         self.launches += 3 * -(-total // slots)
 
     def rotate_heads(self, src, heads, dim, cs_table, rot, style, scale_from=None, scale=1.0):

@@ -72,11 +72,13 @@ class MLSTM(Mixer):
         ops, H, D, Dv = self.ops, self.num_heads, self.dim, self.vdim
         S, nrm, mx = cache
         proj = ops.linear(x, self.w_in, None)                                                  # [T, q | k | v | g]
-        gates = ops.linear(x, self.w_gates, self.b_gates, out_dtype=torch.float32)             # [T, 2H] float32
         q, k, v, g = proj[:, :H * D], proj[:, H * D:2 * H * D], proj[:, 2 * H * D:2 * H * D + H * Dv], proj[:, 2 * H * D + H * Dv:]
-        if hasattr(ops, "mlstm_chunks") and ops.mlstm_in_chunks(q, k, v, ctx.num_seqs, D, Dv, ctx.max_q_len):
+        in_chunks = hasattr(ops, "mlstm_chunks") and ops.mlstm_in_chunks(q, k, v, ctx.num_seqs, D, Dv, ctx.max_q_len)
+        bias = self.b_gates if in_chunks and ops.mlstm_adds_bias(v, ctx.num_seqs, S.state.shape[-1], Dv) else None
+        gates = ops.linear(x, self.w_gates, self.b_gates if bias is None else None, out_dtype=torch.float32)             # [T, 2H] float32
+        if in_chunks:
             o = ops.mlstm_chunks(q, k, v, gates, S.state, nrm.state, mx.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, Dv,
-                                 self.gate_cap, D ** -0.5)
+                                 self.gate_cap, D ** -0.5, pre_bias=bias)
         else:
             weights, n_before = ops.mlstm_gates(gates, mx.state, nrm.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, self.gate_cap)
             o = ops.mlstm_scan(q, k, v, weights, S.state, nrm.state, n_before, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs,
