@@ -1090,3 +1090,57 @@ def test_gemm_f32_on_tensor_cores_extreme_values(ops, M, N, K):
         ok = torch.isfinite(plain) & clear & (scale > 1e-36)
         assert ((got.double() - exp).abs()[ok] <= K * 2.0 ** -24 * scale[ok]).all()
         assert (got[12] == 0).logical_or(torch.isnan(plain[12])).all()
+
+
+# 1 and 8 rows, 9 and 16; rows of W that end inside a set of 16, 32 or 64; K that ends inside a stage of 512, 256 or 128; fewer units than run at once, and more
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(4096, 512), (4090, 1088), (16410, 192), (700, 4160), (33, 32768), (9999, 576)])
+def test_skinny_gemm_through_shared_memory(ops, M, N, K):
+    """The weight-streaming product whose weights come by TMA: every epilogue, one, two and four sets of rows, K whole and cut, against 64 bits.
+    A warp's sum takes K / 64 instructions, each of which cuts the running sum by up to 2^-23 of it, half of that on average."""
+    tol32 = 1e-6 + K / 64 * 2.0 ** -24
+    g = torch.Generator().manual_seed(47)
+    x, w, b = (torch.randn(M, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV), torch.randn(N, generator=g).bfloat16().to(DEV))
+    exp, stream = x.double() @ w.double().T, torch.cuda.current_stream().cuda_stream
+    call = lambda out, bias, n, kslice, epi, up, form: ops.lib.ttie_skinny_gemm_tuned(
+        x.data_ptr(), K, w.data_ptr(), K, None if bias is None else bias.data_ptr(), out.data_ptr(), n, M, n, K, kslice, epi, up, form, stream)
+    whole = -(-K // 128) * 128
+    for form in (0, 16, 32):
+        for kslice in {whole, 256, -(-whole // 384) * 128}:
+            part = torch.full((-(-K // kslice), M, N), float("nan"), device=DEV)
+            assert call(part, None, N, kslice, 1, 0, form) == 0
+            assert rel(part.double().sum(0).cpu(), exp.cpu()) < tol32
+        for epi, dtype, tol in ((0, torch.bfloat16, 4e-3), (3, torch.float32, tol32), (4, torch.bfloat16, 4e-3)):
+            out = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
+            assert call(out, b, N, whole, epi, 0, form) == 0
+            ref = exp + b.double()
+            assert rel(out.double().cpu(), (ref.clamp(min=0) ** 2 if epi == 4 else ref).cpu()) < tol
+    F = N // 2
+    act = torch.full((M, F), float("nan"), dtype=torch.bfloat16, device=DEV)
+    assert call(act, None, F, whole, 2, F, 0) == 0
+    gate, up = exp[:, :F], exp[:, F:2 * F]
+    assert rel(act.double().cpu(), (gate * torch.sigmoid(gate) * up).cpu()) < 4e-3
+    assert ops.lib.ttie_tc_error() == 0
+
+
+def test_skinny_gemm_through_shared_memory_in_a_chain(ops):
+    """Products behind one another and behind a norm, each let in before the one ahead is done: activations are only read once they are there."""
+    g = torch.Generator().manual_seed(48)
+    D, F, eps = 2048, 4096, 1e-6
+    wu, wd = [torch.randn(n, k, generator=g).mul(k ** -0.5).bfloat16().to(DEV) for n, k in ((2 * F, D), (D, F))]
+    nw = torch.ones(D, device=DEV)
+    resid = torch.randn(8, D, generator=g).to(DEV)
+    stream, ref = resid.clone(), resid.double()
+    h = torch.empty(8, D, dtype=torch.bfloat16, device=DEV)
+    delta = None
+    for _ in range(12):
+        ops.add_rmsnorm(stream, delta, nw, eps, h)
+        delta = ops.linear(ops.linear_swiglu(h, wu, None, F), wd, None, partial_ok=True)
+    delta = delta.sum(0) if delta.dim() == 3 else delta
+    for _ in range(12):
+        n = (ref * torch.rsqrt((ref * ref).mean(-1, keepdim=True) + eps)).bfloat16().double()
+        gu = n @ wu.double().T
+        ref_delta = (gu[:, :F] * torch.sigmoid(gu[:, :F]) * gu[:, F:]).bfloat16().double() @ wd.double().T
+        last, ref = ref, ref + ref_delta
+    assert rel((stream.double() + delta.double()).cpu(), ref.cpu()) < 1e-2
+    assert ops.lib.ttie_tc_error() == 0

@@ -273,7 +273,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ ws_o, const float* _
 template <typename T, int NS>
 __global__ void __launch_bounds__(128)
 attn_merge_small_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, T* __restrict__ out, int num_splits, int D) {
-    TTIE_PDL_ENTRY();
+    TTIE_PDL_ENTRY_EARLY();
     const size_t row = blockIdx.x;
     const int d = blockIdx.y * blockDim.x + threadIdx.x;
     if (d >= D) return;

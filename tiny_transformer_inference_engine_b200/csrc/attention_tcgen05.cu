@@ -283,6 +283,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         pdl_wait();                                                // this warp asks for the pages the predecessor has just written
+        pdl_launch_dependents();                                   // (the merge, and the product behind it, whose weights travel meanwhile)
     } else {
         // queries of the tile -> shared memory in the K-major swizzled operand layout (they are the predecessor's output)
         pdl_wait();

@@ -25,6 +25,10 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A small kernel in front of a product that streams weights lets it in before its own wait: the product fills its rings while this
+// kernel and the end of the one before run.  Only for kernels whose successors read nothing but weights ahead of their wait: what such a
+// successor may count on by then is a kernel further back.
+#define TTIE_PDL_ENTRY_EARLY() do { ::ttie::pdl_launch_dependents(); ::ttie::pdl_wait(); } while (0)
 // first statement of a kernel: wait for the predecessor's results, then let the successor be scheduled
 #define TTIE_PDL_ENTRY() do { ::ttie::pdl_wait(); ::ttie::pdl_launch_dependents(); } while (0)
 
@@ -122,17 +126,17 @@ bool pdl_enabled();
 // asks (and clears) whether the next kernel is to be launched as an ordinary one although pdl_enabled(): the first kernel of a stream
 // behind a wait for another stream's event
 bool pdl_skip_once();
-// cluster: CTAs per thread-block cluster along x, y, z (the grid must be a multiple); dim3(1) for none.
-template <typename... KArgs, typename... Args>
+// cluster: CTAs per thread-block cluster along x, y, z (the grid must be a multiple); dim3(1) for none.  ALWAYS: a cluster launch takes the
+// attribute too (else it does not: as a programmatic dependent it was measured to start late).
+template <bool ALWAYS = false, typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, dim3 cluster,
                                  Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    // (a cluster launch does not take the attribute: as a programmatic dependent it was measured to start late)
     const bool clustered = cluster.x * cluster.y * cluster.z > 1;
-    if (!pdl_skip_once() && pdl_enabled() && !clustered) {
+    if (!pdl_skip_once() && pdl_enabled() && (ALWAYS || !clustered)) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -146,9 +150,11 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 #define TTIE_LAUNCH(kernel, grid, block, smem, stream, ...) \
-    ::ttie::launch_kernel(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, dim3(1), __VA_ARGS__)
+    ::ttie::launch_kernel<false>(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, dim3(1), __VA_ARGS__)
 #define TTIE_LAUNCH_CLUSTER(kernel, grid, block, smem, stream, cluster, ...) \
-    ::ttie::launch_kernel(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, dim3(cluster), __VA_ARGS__)
+    ::ttie::launch_kernel<false>(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, dim3(cluster), __VA_ARGS__)
+#define TTIE_LAUNCH_CLUSTER_PDL(kernel, grid, block, smem, stream, cluster, ...) \
+    ::ttie::launch_kernel<true>(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, dim3(cluster), __VA_ARGS__)
 
 
 }  // namespace ttie

@@ -197,7 +197,7 @@ add_rmsnorm_cluster_kernel(float* __restrict__ resid, const T* __restrict__ delt
         const int ch = c_begin + threadIdx.x + c * NT;
         if (ch < c_end) w[c] = Vec4<W>::load(weight + ch * 4);
     }
-    TTIE_PDL_ENTRY();
+    TTIE_PDL_ENTRY_EARLY();
     const size_t src = (size_t)(rows ? rows[r] : r) * d;
     float4 v[MAXC];
     float ss = 0.f;
@@ -257,8 +257,8 @@ static int launch_rmsnorm(float* resid, const void* delta, const float* dpart, i
                          && (part_stride % 4 == 0);
     if (d % 4 == 0 && d <= 8192 && d >= 1024 && aligned && R <= 96 && (w_dtype == kF32 || w_dtype == kBF16)) {
         constexpr int C = 4;                                        // (d / 4) chunks over 4 CTAs of 256 threads, 2 chunks each at most
-        if (w_dtype == kF32) TTIE_LAUNCH_CLUSTER((add_rmsnorm_cluster_kernel<T, float, 256, 2, C>), R * C, 256, 0, s, C, resid, (const T*)delta, dpart, S, part_stride, rows, (const float*)weight, (T*)out, d, eps);
-        else TTIE_LAUNCH_CLUSTER((add_rmsnorm_cluster_kernel<T, __nv_bfloat16, 256, 2, C>), R * C, 256, 0, s, C, resid, (const T*)delta, dpart, S, part_stride, rows, (const __nv_bfloat16*)weight, (T*)out, d, eps);
+        if (w_dtype == kF32) TTIE_LAUNCH_CLUSTER_PDL((add_rmsnorm_cluster_kernel<T, float, 256, 2, C>), R * C, 256, 0, s, C, resid, (const T*)delta, dpart, S, part_stride, rows, (const float*)weight, (T*)out, d, eps);
+        else TTIE_LAUNCH_CLUSTER_PDL((add_rmsnorm_cluster_kernel<T, __nv_bfloat16, 256, 2, C>), R * C, 256, 0, s, C, resid, (const T*)delta, dpart, S, part_stride, rows, (const __nv_bfloat16*)weight, (T*)out, d, eps);
         TTIE_CHECK_LAUNCH("rmsnorm (cluster)");
         return 0;
     }

@@ -16,7 +16,14 @@
 // silu(g)*u (models/mlp.py:24-32; silu in 32-bit as kernels/fused_swiglu/kernel.py:20-25);
 // (3) float32 out (logits).
 #include "common.cuh"
+#include <cuda.h>
 using namespace ttie;
+
+namespace ttie {
+// the product kernels' error word and its mirror, and the builder of maps over blocks of 64 columns (gemm_tcgen05.cu)
+int gemm_tc_error_words(int** word, int** mirror);
+int gemm_tc_make_block_map(CUtensorMap* map, const void* base, long long rows, long long blocks, long long ld, int box_rows, int box_blocks);
+}  // namespace ttie
 
 namespace {
 struct SkinnyParams {
@@ -43,6 +50,55 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// thread (lane, c) of 128 finishes accumulator element c of `lane`: the four warps' K ranges in a fixed order, then the epilogue
+template <int MT, int EPI, int NSET>
+__device__ __forceinline__ void finish_tile(const SkinnyParams& p, const float (&red)[4][NSET][MT][32][4], int n0, int split, int c, int lane) {
+    const int r = lane >> 2, q = lane & 3;
+    float up1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < MT; ++j) {
+        const int m = 8 * j + 2 * q + (c & 1);
+        float v[NSET];
+#pragma unroll
+        for (int s = 0; s < NSET; ++s)
+            v[s] = ((red[0][s][j][lane][c] + red[1][s][j][lane][c]) + red[2][s][j][lane][c]) + red[3][s][j][lane][c];
+        if (m >= p.M) continue;
+        if (EPI == 2) {
+            // (two sets: gate rows and up rows; one: gate rows, and eight further on their up rows, which the threads of elements 0 and 1 finish)
+            const int row = n0 + r + (NSET == 2 ? 8 * (c >> 1) : 0);
+            if (row >= p.N || (NSET == 1 && c > 1)) continue;
+            if (NSET == 1) {
+                const int c2 = c + 2 < 4 ? c + 2 : c;
+                up1 = ((red[0][0][j][lane][c2] + red[1][0][j][lane][c2]) + red[2][0][j][lane][c2]) + red[3][0][j][lane][c2];
+            }
+            float g = v[0] + (p.bias ? __bfloat162float(p.bias[row]) : 0.f);
+            float u = (NSET == 1 ? up1 : v[NSET - 1]) + (p.bias ? __bfloat162float(p.bias[row + p.up_offset]) : 0.f);
+            if (p.glu_limit > 0.f) { g = fminf(g, p.glu_limit); u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit); }
+            reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + row] =
+                __float2bfloat16_rn(gate_act(p.glu_act, p.glu_alpha, g) * (u + p.glu_shift));
+            continue;
+        }
+#pragma unroll
+        for (int s = 0; s < NSET; ++s) {
+            const int row = n0 + 16 * s + r + 8 * (c >> 1);
+            if (row >= p.N) continue;
+            if (EPI == 0) {
+                const float b = p.bias ? __bfloat162float(p.bias[row]) : 0.f;
+                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + row] = __float2bfloat16_rn(v[s] + b);
+            } else if (EPI == 4) {                                   // the square of relu, for feed-forwards of two matrices
+                const float b = p.bias ? __bfloat162float(p.bias[row]) : 0.f;
+                const float a = fmaxf(v[s] + b, 0.f);
+                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + row] = __float2bfloat16_rn(a * a);
+            } else if (EPI == 1) {
+                reinterpret_cast<float*>(p.out)[((long long)split * p.M + m) * p.ldo + row] = v[s];
+            } else {
+                const float b = p.bias ? __bfloat162float(p.bias[row]) : 0.f;
+                reinterpret_cast<float*>(p.out)[(long long)m * p.ldo + row] = v[s] + b;
+            }
+        }
+    }
 }
 
 // SETS: sets of 16 weight rows per CTA for the plain epilogues.  Every set is multiplied with the same activation
@@ -142,44 +198,237 @@ skinny_gemm_kernel(const SkinnyParams p) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) red[warp][s][j][lane][c] = acc[s][j][c];
     __syncthreads();
-    const int c = warp;                                         // thread (lane, c) finishes accumulator element c of `lane`
-#pragma unroll
-    for (int j = 0; j < MT; ++j) {
-        const int m = 8 * j + 2 * q + (c & 1);
-        float v[NSET];
-#pragma unroll
-        for (int s = 0; s < NSET; ++s)
-            v[s] = ((red[0][s][j][lane][c] + red[1][s][j][lane][c]) + red[2][s][j][lane][c]) + red[3][s][j][lane][c];
-        if (m >= p.M) continue;
-        if (EPI == 2) {
-            const int row = n0 + r + 8 * (c >> 1);
-            if (row >= p.N) continue;
-            float g = v[0] + (p.bias ? __bfloat162float(p.bias[row]) : 0.f);
-            float u = v[NSET - 1] + (p.bias ? __bfloat162float(p.bias[row + p.up_offset]) : 0.f);
-            if (p.glu_limit > 0.f) { g = fminf(g, p.glu_limit); u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit); }
-            reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + row] =
-                __float2bfloat16_rn(gate_act(p.glu_act, p.glu_alpha, g) * (u + p.glu_shift));
-            continue;
-        }
-#pragma unroll
-        for (int s = 0; s < NSET; ++s) {
-            const int row = n0 + 16 * s + r + 8 * (c >> 1);
-            if (row >= p.N) continue;
-            if (EPI == 0) {
-                const float b = p.bias ? __bfloat162float(p.bias[row]) : 0.f;
-                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + row] = __float2bfloat16_rn(v[s] + b);
-            } else if (EPI == 4) {                                   // the square of relu, for feed-forwards of two matrices
-                const float b = p.bias ? __bfloat162float(p.bias[row]) : 0.f;
-                const float a = fmaxf(v[s] + b, 0.f);
-                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + row] = __float2bfloat16_rn(a * a);
-            } else if (EPI == 1) {
-                reinterpret_cast<float*>(p.out)[((long long)split * p.M + m) * p.ldo + row] = v[s];
-            } else {
-                const float b = p.bias ? __bfloat162float(p.bias[row]) : 0.f;
-                reinterpret_cast<float*>(p.out)[(long long)m * p.ldo + row] = v[s] + b;
-            }
+    finish_tile<MT, EPI, NSET>(p, red, n0, split, warp, lane);
+}
+
+// ---- up to 16 rows: the weights through shared memory, by TMA.
+// What bounds such a product is HBM, and what decides how close it comes is how many bytes are on their way and that the stream does not stop
+// between two tiles: copies alone, without the products, reach 6.2 TB/s with 128 KB in flight per SM and 7.0 with 192 KB, whatever the order of the
+// rows (180 MB; 33 MB 5.5 and 6.1).  So a CTA stays (two per SM), walks over units (16 rows of W, or 32 or 64: 2 or 4 sets; a
+// range of K), and one thread keeps a ring of stages filled (16 KB of W: 512 values of K of 16 rows, 256 of 32, 128 of 64; and the activations'
+// values, of which more sets need fewer copies) across the units' borders; the weights of the first stages are asked for before the wait for
+// the kernel before, whose results they do not depend on.  Four warps split a stage's K among themselves, take their operand fragments from
+// shared memory as the other form takes them from global memory (the swizzle spreads eight rows' 16 bytes over all banks), and add up
+// their ranges at the end of a unit.  Activations through the cache instead of the ring were slower (8 rows: 36 against 31 us).
+constexpr long long WAIT_CYCLES = 2000000000LL;             // about one second
+constexpr int BULK_STAGES_MOST = 8;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+struct BulkParams {
+    SkinnyParams g;
+    int tiles, units, stages, stage_bytes, dynamic;
+    int *err, *mirror;
+};
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code, const BulkParams& p) {
+    if (mbar_try(bar, parity)) return true;
+    const long long deadline = clock64() + WAIT_CYCLES;
+    while (!mbar_try(bar, parity)) {
+        if (clock64() > deadline) {
+            atomicCAS(p.err, 0, code);
+            if (p.mirror) { *reinterpret_cast<volatile int*>(p.mirror) = code; __threadfence_system(); }
+            return false;
         }
     }
+    return true;
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row, int block) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"(row), "r"(block) : "memory");
+}
+
+// the gated unit with SETS 1: a set's first eight rows are gate rows, the others their up rows (half as long a unit, twice the activations' copies)
+__host__ __device__ constexpr int row_sets(int epi, int sets) { return epi == 2 && sets > 2 ? 2 : sets; }
+__host__ __device__ constexpr int unit_columns(int epi, int sets) { return epi == 2 ? (sets == 1 ? 8 : 16) : 16 * sets; }
+template <int NSET> struct BulkShape {
+    static constexpr int KS = 512 / NSET, BLOCKS = KS / 64;      // K of a stage
+    static constexpr uint32_t SET = BLOCKS * 16 * 128, WEIGHTS = NSET * SET;           // bytes of 16 rows, of a stage's weights (16 KB)
+};
+
+template <int MT, int EPI, int SETS>
+__global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const BulkParams bp) {
+    constexpr int NSET = row_sets(EPI, SETS);
+    constexpr bool PAIRED = EPI == 2 && NSET == 1;
+    using Sh = BulkShape<NSET>;
+    constexpr int KS = Sh::KS, KW = KS / 4;                      // KW: K of a warp
+    const SkinnyParams& p = bp.g;
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) unsigned long long bars[2 * BULK_STAGES_MOST + 1];
+    __shared__ __align__(16) uint4 next_unit;                    // the answer to the question for another unit
+    __shared__ int stage_unit[BULK_STAGES_MOST], stage_k[BULK_STAGES_MOST], stage_more[BULK_STAGES_MOST];      // what a stage holds; whether a unit follows its last one
+    __shared__ float red[2][4][NSET][MT][32][4];                 // (in turn: the next unit's sums need not wait for this one's to be read)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, q = lane & 3;
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * BULK_STAGES_MOST, asked = empty0 + 8 * BULK_STAGES_MOST, ring0 = smem_u32(ring);
+    if (tid == 0) {
+        for (int s = 0; s < bp.stages; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(empty0 + 8 * s) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(asked) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    auto range_of = [&](int unit, int& n0, int& split, int& k_begin, int& k_end) {
+        split = unit / bp.tiles;
+        n0 = (unit - split * bp.tiles) * unit_columns(EPI, NSET);
+        k_begin = split * p.kslice;
+        k_end = min(p.K, k_begin + p.kslice);
+    };
+    if (warp == 4) {
+        if (lane != 0) return;
+        const uint32_t bytes = Sh::WEIGHTS + (uint32_t)(Sh::BLOCKS * p.M * 128);
+        int s = 0, round = 0, ahead = 0, turn = 0;               // ahead: stages whose activations are still to come; turn: questions answered
+        bool ok = true, waited = false;
+        auto acts = [&](int k0, int st) { tma_load_3d(ring0 + (uint32_t)st * bp.stage_bytes + Sh::WEIGHTS, &tmX, full0 + 8 * st, 0, k0 / 64); };
+        auto settle = [&]() {                                    // the kernel before is done: the activations of the stages filled so far
+            pdl_wait();
+            pdl_launch_dependents();
+            waited = true;
+            for (int i = 0; i < ahead; ++i) acts(stage_k[i], i);
+        };
+        auto free_stage = [&]() {
+            if (!waited && ahead == bp.stages) settle();
+            if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, 61, bp);
+            return ok;
+        };
+        // a CTA that has not started yet gives its unit to one that has room for it
+        auto ask = [&]() {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(asked) : "memory");
+            asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_unit)), "r"(asked) : "memory");
+        };
+        auto answer = [&]() -> int {                             // its number, or -1: all have started
+            if (!mbar_wait(asked, turn++ & 1, 63, bp)) { ok = false; return -1; }
+            uint32_t given, x;
+            asm volatile("{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tld.shared.b128 h, [%2];\n\t"
+                         "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+                         "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+                         : "=r"(given), "=r"(x) : "r"(smem_u32(&next_unit)) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");                  // (read before the next answer is written)
+            return given ? (int)x : -1;
+        };
+        int unit = blockIdx.x;
+        while (ok && unit >= 0) {
+            if (bp.dynamic) ask();
+            int n0, split, k_begin, k_end, next = -1;
+            range_of(unit, n0, split, k_begin, k_end);
+            for (int k0 = k_begin; k0 < k_end; k0 += KS) {
+                if (!waited && ahead == bp.stages) settle();
+                if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, 61, bp);
+                if (ok && bp.dynamic && k0 + KS >= k_end) next = answer();
+                if (!ok) break;
+                const uint32_t bar = full0 + 8 * s, dst = ring0 + (uint32_t)s * bp.stage_bytes;
+                stage_unit[s] = unit;
+                stage_k[s] = k0;
+                stage_more[s] = next >= 0;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+#pragma unroll
+                for (int i = 0; i < (PAIRED ? 2 : NSET); ++i)    // (rows and blocks past the end are zeros; blocks of the next range are not used)
+                    tma_load_3d(dst + i * (PAIRED ? Sh::SET / 2 : Sh::SET), &tmW, bar, n0 + (EPI == 2 ? i * p.up_offset : i * 16), k0 / 64);
+                if (waited) acts(k0, s);
+                else ++ahead;
+                if (++s == bp.stages) { s = 0; ++round; }
+            }
+            unit = next;
+        }
+        if (!waited) settle();
+        if (!ok)                                                 // (nothing may land in a CTA that has left; each wait is bounded)
+            for (int i = 0; i < bp.stages; ++i) if (round > 0 || i < s) mbar_wait(full0 + 8 * i, (i < s ? round : round - 1) & 1, 61, bp);
+        return;
+    }
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    int s = 0, round = 0;
+    auto arrived = [&]() { return (bool)__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, round & 1, 62, bp)); };
+    auto next_stage = [&]() { if (++s == bp.stages) { s = 0; ++round; } };
+    bool more = true;
+    for (int turn = 0; more; turn ^= 1) {
+        bool ok = arrived();
+        if (!ok) break;
+        int n0, split, k_begin, k_end;
+        range_of(stage_unit[s], n0, split, k_begin, k_end);
+        float acc[NSET][MT][4];
+#pragma unroll
+        for (int i = 0; i < NSET; ++i)
+#pragma unroll
+            for (int j = 0; j < MT; ++j) { acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f; }
+        for (int k0 = k_begin; k0 < k_end; k0 += KS) {
+            if (k0 > k_begin) { ok = arrived(); if (!ok) break; }
+            const unsigned char* base = ring + (size_t)s * bp.stage_bytes;
+            more = stage_more[s];
+#pragma unroll
+            for (int u = 0; u < KW / 32; ++u) {
+                const int k = warp * KW + 32 * u, block = k >> 6, chunk = ((k >> 3) & 7) + q, at = (chunk ^ r) << 4;       // (row & 7 is r for all of this lane's rows)
+                const bool in = k0 + k < k_end;                  // (ranges are multiples of 64)
+                uint4 wv[NSET][2], xv[MT];
+#pragma unroll
+                for (int i = 0; i < NSET; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        wv[i][h] = in ? *reinterpret_cast<const uint4*>(base + (PAIRED ? h * (Sh::SET / 2) + (block * 8 + r) * 128 : i * Sh::SET + (block * 16 + h * 8 + r) * 128) + at) : zero;
+#pragma unroll
+                for (int j = 0; j < MT; ++j) {
+                    const int line = block * p.M + 8 * j + r;    // (as many lines a block as there are rows)
+                    xv[j] = in && 8 * j + r < p.M ? *reinterpret_cast<const uint4*>(base + Sh::WEIGHTS + line * 128 + ((chunk ^ (line & 7)) << 4)) : zero;
+                }
+#pragma unroll
+                for (int i = 0; i < NSET; ++i)
+#pragma unroll
+                    for (int j = 0; j < MT; ++j) {
+                        mma_bf16(acc[i][j], wv[i][0].x, wv[i][1].x, wv[i][0].y, wv[i][1].y, xv[j].x, xv[j].y);
+                        mma_bf16(acc[i][j], wv[i][0].z, wv[i][1].z, wv[i][0].w, wv[i][1].w, xv[j].z, xv[j].w);
+                    }
+            }
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty0 + 8 * s) : "memory");
+            next_stage();
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < NSET; ++i)
+#pragma unroll
+            for (int j = 0; j < MT; ++j)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) red[turn][warp][i][j][lane][c] = acc[i][j][c];
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        finish_tile<MT, EPI, NSET>(p, red[turn], n0, split, warp, lane);
+    }
+}
+
+template <int MT, int EPI, int SETS>
+int launch_bulk(const SkinnyParams& p, int splits, cudaStream_t s) {
+    constexpr int NSET = row_sets(EPI, SETS);
+    using Sh = BulkShape<NSET>;
+    constexpr int ROOM = 228 * 512 - 1024 - 320 - 2 * 4 * NSET * MT * 512 - 1024;              // what two CTAs per SM leave for a ring
+    BulkParams b;
+    b.g = p;
+    b.tiles = ceil_div(p.N, unit_columns(EPI, NSET));
+    b.units = b.tiles * splits;
+    b.stage_bytes = ((int)Sh::WEIGHTS + Sh::BLOCKS * p.M * 128 + 1023) / 1024 * 1024;
+    b.stages = ROOM / b.stage_bytes < BULK_STAGES_MOST ? ROOM / b.stage_bytes : BULK_STAGES_MOST;
+    CUtensorMap mw, mx;
+    if (gemm_tc_make_block_map(&mw, p.w, EPI == 2 ? (long long)p.up_offset + p.N : p.N, p.K / 64, p.ldw, EPI == 2 && NSET == 1 ? 8 : 16, Sh::BLOCKS)) return -1;
+    if (gemm_tc_make_block_map(&mx, p.x, p.M, p.K / 64, p.ldx, p.M, Sh::BLOCKS)) return -1;
+    if (gemm_tc_error_words(&b.err, &b.mirror)) TTIE_FAIL("skinny_gemm: the error word's address is not to be had");
+    auto kernel = skinny_bulk_kernel<MT, EPI, SETS>;
+    static bool allowed[64] = {false};
+    int dev = 64;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64 || !allowed[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROOM + 1024);
+        if (e != cudaSuccess) TTIE_FAIL("skinny_gemm: %d bytes of shared memory refused: %s", ROOM + 1024, cudaGetErrorString(e));
+        if (dev < 64) allowed[dev] = true;
+    }
+    // A CTA per unit; where they are more than fit at once, a running one takes over the units of those that have not started.  (Equal shares
+    // decided beforehand end at different times - 29 to 43 us for [32000, 4096] -, since the SMs do not get equal shares of the memory's rate.)
+    b.dynamic = b.units > 2 * num_sms();
+    TTIE_LAUNCH(kernel, b.units, 160, b.stages * b.stage_bytes + 1024, s, mw, mx, b);
+    TTIE_CHECK_LAUNCH("skinny_gemm (bulk)");
+    return 0;
 }
 
 template <int MT, int EPI, int U, int SETS>
@@ -192,10 +441,23 @@ int launch(const SkinnyParams& p, int splits, cudaStream_t s) {
 
 template <int EPI>
 int dispatch(const SkinnyParams& p, int splits, int unroll, cudaStream_t s) {
-    // unroll: low four bits 0 (chosen here), 2 or 4; + 16 asks for two row sets per CTA (plain epilogues)
-    const bool two = EPI != 2 && (unroll & 16);
+    // unroll: low four bits 0 (chosen here), 2 or 4; + 16 asks for two row sets per CTA, + 32 for four (plain epilogues)
+    const int unroll0 = unroll;
+    const bool two = EPI != 2 && (unroll & 48);
     unroll &= 15;
     const int mt = ceil_div(p.M, 8);
+    // Through shared memory from 1 Mi weights on ([1024, 1024] 1.8 us either way, [512, 2048] 2.5 | 3.3).  us, this form | the other, 1 row and 8:
+    // [4352, 4096] 6.7 | 7.5, 7.2 | 7.6; [4096, 4096] 6.4 | 6.7, 7.0 | 7.0; gate and up of [22016, 4096] 27.0 | 31.2, 27.5 | 31.6; [4096, 11008]
+    // 13.9 | 15.5, 15.0 | 16.2; [32000, 4096] 37.8 | 44.1, 38.8 | 45.4; [256000, 2048] 146 | 145, 147 | 145 (copies alone: 5.5 us for 33 MB,
+    // 25.9 for 180, 37.0 for 262).  The gated unit in sets of 8 + 8 rows where these are long enough a unit: [22016, 4096] 27.0 against 29.6 in 16 +
+    // 16, [32768, 2048] 20.7 against 19.9.
+    const long long weights = (long long)p.N * (EPI == 2 ? 2 : 1) * p.K;
+    // (A gated unit of fewer units than SMs stays with the other form: its caller has a product cut over K, with the activation behind it, for that.)
+    if (mt <= 2 && p.K % 64 == 0 && weights >= (1LL << 20) && (EPI != 2 || p.N >= 8 * num_sms())) {
+        const int sets = EPI == 2 ? (p.K >= 4096 ? 1 : 2) : unroll0 & 32 ? 4 : unroll0 & 16 ? 2 : 1;
+        if (mt == 1) return sets == 4 ? launch_bulk<1, EPI, 4>(p, splits, s) : sets == 2 ? launch_bulk<1, EPI, 2>(p, splits, s) : launch_bulk<1, EPI, 1>(p, splits, s);
+        return sets == 4 ? launch_bulk<2, EPI, 4>(p, splits, s) : sets == 2 ? launch_bulk<2, EPI, 2>(p, splits, s) : launch_bulk<2, EPI, 1>(p, splits, s);
+    }
     // a product that is not split over CTAs streams best with deep unrolling, a split one with more CTAs per SM
     const bool deep = EPI != 2 && (unroll ? unroll >= 4 : splits == 1);
     if (two) {
@@ -236,7 +498,7 @@ extern "C" int ttie_skinny_gemm_glu(const void* x, long long ldx, const void* w,
     return rc;
 }
 // unroll: 0 = chosen from kslice; 2 or 4 = 32-key blocks per register buffer (rows <= 8 only); + 16 = two sets of 16
-// weight rows per CTA (plain epilogues; halves the 32-key blocks per buffer).
+// weight rows per CTA, + 32 = four (plain epilogues; halves the 32-key blocks per buffer).
 extern "C" int ttie_skinny_gemm_tuned(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* out,
                                       long long ldo, int M, int N, int K, int kslice, int epilogue, int up_offset, int unroll,
                                       void* stream) {

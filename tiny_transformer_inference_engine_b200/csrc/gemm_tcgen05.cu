@@ -268,6 +268,20 @@ int make_map_of(CUtensorMap* map, bool f32, const void* base, long long rows, lo
     if (r != CUDA_SUCCESS) TTIE_FAIL("gemm_tc: cuTensorMapEncodeTiled failed with code %d", (int)r);
     return 0;
 }
+// 3-D map over a row-major [rows][64 * blocks] bfloat16 matrix with row stride ld, as [blocks][rows][64]: a box is box_blocks blocks of 64 columns of
+// box_rows rows, each block's rows together in shared memory (128-byte swizzle).
+int make_block_map(CUtensorMap* map, const void* base, long long rows, long long blocks, long long ld, int box_rows, int box_blocks) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) TTIE_FAIL("gemm_tc: cuTensorMapEncodeTiled is not available from the driver");
+    cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)blocks};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, 128};
+    cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)box_blocks};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) TTIE_FAIL("gemm_tc: cuTensorMapEncodeTiled failed with code %d", (int)r);
+    return 0;
+}
 // The products' operands: bfloat16, box = 64 (K) x box_rows.
 int make_map(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
     return make_map_of(map, false, base, rows, K, ld, BK, box_rows);
@@ -310,6 +324,9 @@ int gemm_tc_error_words(int** word, int** mirror) {
 }
 int gemm_tc_make_map(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
     return make_map(map, base, rows, K, ld, box_rows);
+}
+int gemm_tc_make_block_map(CUtensorMap* map, const void* base, long long rows, long long blocks, long long ld, int box_rows, int box_blocks) {
+    return make_block_map(map, base, rows, blocks, ld, box_rows, box_blocks);
 }
 int gemm_tc_make_map_of(CUtensorMap* map, int f32, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows) {
     return make_map_of(map, f32 != 0, base, rows, cols, ld, box_cols, box_rows);

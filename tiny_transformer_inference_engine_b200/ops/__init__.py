@@ -343,8 +343,8 @@ class CudaOps:
         [2048, 16384] it leaves half of the memory bandwidth unused), and the faster one is remembered.  Up to 8 rows the
         weight-streaming product is the rule and is ahead on most shapes, by up to 3x on narrow deep ones; a shape goes to
         the library where that is more than 5 % faster (measured: [10240, 8192] and [8192, 28672] by 9-10 %).  At 8 and
-        16 rows the weight-streaming product's own form is measured too - K cut into 1 to 16 ranges over CTAs, one or two
-        sets of 16 weight rows per CTA - and a form that beats the rule of thumb (``_kslice``) by 3 % is kept: [4352, 4096]
+        16 rows the weight-streaming product's own form is measured too - K cut into 1 to 16 ranges over CTAs, one, two or
+        four sets of 16 weight rows per CTA - and a form that beats the rule of thumb (``_kslice``) by 3 % is kept: [4352, 4096]
         at 8 rows takes 7.8 us in 6 ranges with two row sets against 9.1 in 8 ranges with one, [4544, 18176] 28.5 us in 6
         ranges against 38.3 uncut.  Small matrices (under 4 Mi elements) are left alone."""
         groups, launches = {}, self.launches
@@ -374,9 +374,9 @@ class CudaOps:
                 took = {"library": measure("library"), "skinny_uncut": measure("skinny", partial_ok=False), "skinny": measure("skinny")}
                 form = None
                 if M <= 16:
-                    # up to 16 rows the weight-streaming product's own form is measured as well: one or two sets of 16 weight
+                    # up to 16 rows the weight-streaming product's own form is measured as well: one, two or four sets of 16 weight
                     # rows per CTA, K cut into 1 to 16 ranges
-                    for code in (0, 16):
+                    for code in (0, 16, 32):
                         for S in (1, 2, 3, 4, 6, 8, 12, 16):
                             kslice = math.ceil(math.ceil(K / S) / 128) * 128
                             if kslice < 256 or math.ceil(K / kslice) != S:
@@ -387,7 +387,7 @@ class CudaOps:
                 self._skinny_tuned.pop((N, K, M), None)
                 if form is not None:
                     self._skinny_tuned[(N, K, M)] = form
-                    took["skinny_form"] = {"k_ranges": math.ceil(K / form[0]), "row_sets": 2 if form[1] & 16 else 1}
+                    took["skinny_form"] = {"k_ranges": math.ceil(K / form[0]), "row_sets": 4 if form[1] & 32 else 2 if form[1] & 16 else 1}
                 # callers that take partial sums of a cut K range, and callers that want the whole sum
                 self._product_choice[(N, K, M, "split")] = decide(took["skinny"], took["library"])
                 self._product_choice[(N, K, M)] = decide(took["skinny_uncut"], took["library"])
