@@ -275,6 +275,36 @@ def test_split_keys_merge(ops, dtype, kernel, unit, splits):
     assert rel(out, exp) < TOL[dtype]
 
 
+@pytest.mark.parametrize("Hq,Hkv,D,page", [(4, 4, 4, 16), (4, 1, 36, 8), (3, 1, 64, 64), (2, 2, 68, 3), (16, 1, 128, 64)])
+@pytest.mark.parametrize("opts", [{}, {"window": 50}, {"window": 40, "keep_first": 9}, {"chunk": 96}, {"softcap": 3.0},
+                                  {"weights": "sigmoid", "bias": True}])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_float32_tiles_agree_with_the_general_form(ops, Hq, Hkv, D, page, opts, splits):
+    """Portions of 64 query rows and more take tiles of 64 rows x 64 keys; an output that does not start on 16 bytes keeps to the
+    general kernel.  Both compute in 32 bits with expf: they differ by the order of sums of up to 400 terms and D products."""
+    opts = dict(opts)
+    g = torch.Generator().manual_seed(D)
+    seqs = [(65, 65), (400, 63), (64, 64), (17, 17), (130, 1), (257, 129)]            # (keys, new tokens): edges of tiles, tails of up to 16 keys
+    T, N, mk = sum(n for _, n in seqs), len(seqs), 400
+    width = -(-mk // page)
+    table = (torch.randperm(N * width, generator=g).int() + 1).view(N, width).to(DEV)
+    kp, vp = (torch.randn(N * width + 1, Hkv, page, D, generator=g).to(DEV) for _ in range(2))
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, generator=g).to(DEV)
+    bias = torch.randn(Hq, generator=g).to(DEV) if opts.pop("bias", False) else None
+    qsl = torch.tensor([0] + list(torch.tensor([n for _, n in seqs]).cumsum(0)), dtype=torch.int32, device=DEV)
+    lens = torch.tensor([L for L, _ in seqs], dtype=torch.int32, device=DEV)
+    plan = ("simt", 1, 0) if splits == 1 else ("simt", splits, 192)
+    outs = []
+    for shift in (0, 1):
+        buf = torch.full((T * Hq * D + 4,), float("nan"), device=DEV)
+        out = buf[shift:shift + T * Hq * D].view(T, Hq * D)
+        ops.paged_attention(qkv, Hq, Hkv, D, kp, vp, table, page, qsl, lens, N, 129, mk, D ** -0.5, opts.get("window", 0), out, plan=plan,
+                            head_bias=bias, **{k: v for k, v in opts.items() if k != "window"})
+        outs.append(out.double().cpu())
+    assert torch.isfinite(outs[0]).all()
+    assert (outs[0] - outs[1]).abs().max() <= 2 * (400 + D) ** 0.5 * 2.0 ** -23 * outs[1].abs().max()
+
+
 @pytest.mark.parametrize("dtype,kernel", [("float32", "simt"), ("bfloat16", "simt"), ("bfloat16", "mma")])
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_window(ops, dtype, kernel, window):

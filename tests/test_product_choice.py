@@ -101,3 +101,20 @@ def test_float32_products_on_tensor_cores_by_shape_and_alignment():
     (WKV, [2048], 128, 128, torch.bfloat16, 64), (RETENTION, [1] * 23 + [256], 128, 128, torch.bfloat16, 64), (MLSTM, [1] * 31 + [2000], 64, 128, torch.bfloat16, 128)])
 def test_tokens_of_a_chunk(mode, lens, key, value, dtype, tokens):
     assert CudaOps._chunk_tokens(mode, dtype, sum(lens), len(lens), key, value) == tokens
+
+
+@pytest.mark.parametrize("heads,rows,group,dim,new,keys", [(1, 64, 16, 128, 4, 4), (1, 4800, 16, 128, 300, 300), (8, 300, 1, 64, 300, 300), (1, 2048, 16, 128, 128, 4096),
+                                                           (4, 80, 16, 128, 5, 1000), (16, 64, 16, 128, 4, 4096), (1, 32768, 16, 128, 2048, 2048),
+                                                           (6, 64, 1, 36, 64, 100000)])
+def test_float32_pieces_cover_the_keys(heads, rows, group, dim, new, keys):
+    """Pieces of whole tiles that cover every key, the last one not empty; many row tiles are left uncut."""
+    ops = CudaOps.__new__(CudaOps)
+    ops.num_sms = 148
+    kernel, n, length = ops._f32_tile_pieces(heads, rows, group, dim, new, keys)
+    assert kernel == "simt" and n >= 1
+    if n > 1:
+        assert length % 64 == 0 and (n - 1) * length < keys <= n * length
+    if keys <= 64 or rows >= 32768:
+        assert n == 1
+    if keys >= 32 * new:                                                             # few rows behind many keys
+        assert n >= 8

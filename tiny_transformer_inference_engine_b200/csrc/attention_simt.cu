@@ -2,7 +2,8 @@
 // any number of heads and kv heads, head sizes that are multiples of 4 up to 512, any page
 // size, optional window, float32 or bfloat16 storage with float32 arithmetic throughout
 // (scores, running maximum and sum, output accumulators; expf, not a fast approximation).
-// It is the attention of the float32 path and the fallback of the bfloat16 path.
+// It is the attention of the float32 path (prompt portions with head sizes up to 128 take paged_attn_f32_tile_kernel) and the
+// fallback of the bfloat16 path.
 //
 // Mask and scale as kernels/pagedattn/pagedattn.cu:196-207,256 of the reference: a request
 // with kv_len keys and q_len new tokens has ctx = kv_len - q_len; query row r sits at position
@@ -25,6 +26,7 @@
 // key row may be long (16 kv heads of 64: 1,024), so scores are accumulated over pieces of JC of its columns.
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 using namespace ttie;
 
 namespace {
@@ -302,9 +304,9 @@ attn_merge_small_kernel(const float* __restrict__ ws_o, const float* __restrict_
 // The same for up to 8 splits with four columns per thread and the rows packed into blocks of 256 threads: a prompt
 // portion whose key range was cut brings thousands of rows, and one small block per row (16,384 rows x 2 splits: 24 us)
 // spends its time on block launches, not on the 21 MB it moves.  The arithmetic per element is that of the kernel above.
-template <int NS>
+template <typename T, int NS>
 __global__ void __launch_bounds__(256)
-attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, __nv_bfloat16* __restrict__ out,
+attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, T* __restrict__ out,
                       long long rows, int num_splits, int D) {
     TTIE_PDL_ENTRY();
     const int per_row = D / 4;
@@ -337,41 +339,258 @@ attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ 
         den = fmaf(e, v[s].y, den);
     }
     const bool any = den > 0.f;
-    __nv_bfloat162 lo = __floats2bfloat162_rn(any ? acc.x / den : 0.f, any ? acc.y / den : 0.f);
-    __nv_bfloat162 hi = __floats2bfloat162_rn(any ? acc.z / den : 0.f, any ? acc.w / den : 0.f);
-    uint2 packed;
-    packed.x = *reinterpret_cast<unsigned*>(&lo);
-    packed.y = *reinterpret_cast<unsigned*>(&hi);
-    *reinterpret_cast<uint2*>(out + row * D + d) = packed;
+    const float4 y = any ? make_float4(acc.x / den, acc.y / den, acc.z / den, acc.w / den) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(out + row * D + d) = y;
+    } else {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+        *reinterpret_cast<uint2*>(out + row * D + d) = make_uint2(*reinterpret_cast<unsigned*>(&lo), *reinterpret_cast<unsigned*>(&hi));
+    }
 }
 
+template <typename T>
+int attn_merge(const float* ws_o, const float* ws_ml, T* out, long long rows, int num_splits, int D, cudaStream_t s) {
+    const dim3 grid((unsigned)rows, ceil_div(D, 128));
+    const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(ws_o) | reinterpret_cast<uintptr_t>(ws_ml)) & 15) == 0
+                     && (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(T) - 1)) == 0;
+    if (vec && num_splits <= 8) {
+        const unsigned blocks = (unsigned)((rows * (D / 4) + 255) / 256);
+        if (num_splits <= 2) { TTIE_LAUNCH((attn_merge_vec_kernel<T, 2>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
+        else if (num_splits <= 4) { TTIE_LAUNCH((attn_merge_vec_kernel<T, 4>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
+        else { TTIE_LAUNCH((attn_merge_vec_kernel<T, 8>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
+    } else if (num_splits <= 4) {
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 4>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+    } else if (num_splits <= 8) {
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 8>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+    } else if (num_splits <= 16) {
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 16>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+    } else if (num_splits <= 32) {
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 32>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+    } else {
+        TTIE_LAUNCH(attn_merge_kernel<T>, (unsigned)rows, MERGE_GROUPS * (D >= 128 ? 128 : 64), (num_splits + MERGE_GROUPS * D) * sizeof(float), s,
+                    ws_o, ws_ml, out, num_splits, D);
+    }
+    TTIE_CHECK_LAUNCH("attention merge");
+    return 0;
+}
+
+// ---- float32 prompt portions (64 query rows of a kv head and more), head sizes up to 128.  The kernel above reads shared memory once for every
+// two multiply-adds.  Here a CTA of 256 threads owns 64 query rows and walks tiles of 64 keys: a thread computes 4 rows x 4 keys of the
+// scores (8 loads of 16 bytes for 64 multiply-adds) and 4 rows x 8 (4) columns of the output (12 (8) loads for 128 (64)); the 16 threads of
+// a row are half a warp, so a row's weights pass through shared memory without a block barrier.  Bound by the loads from shared
+// memory: a tile step of head size 128 takes an SM 10.3 us with two CTAs side by side (113 KB each) and 11.2 with one; 4.3 us of it
+// are multiply-adds.  Before and now, 16 heads on one kv head of 128: 300 tokens 85 -> 32 us, 600: 183 -> 70, 2,048: 1,372 -> 583, 128
+// behind 4,096 keys: 330 -> 144; 8 heads of 64, 300 tokens: 31 -> 17.  Measured and left out: 8 rows a thread with half the threads
+// (660 us at 2,048 tokens: too few warps), tiles by cp.async beside the computation (630), one CTA an SM at all sizes (671).
+constexpr int FT_ROWS = 64, FT_KEYS = 64, FT_R = 4, FT_THREADS = FT_ROWS / FT_R * 16;
+template <int DP> constexpr size_t tile_smem() { return sizeof(float) * ((size_t)FT_ROWS * DP + (size_t)FT_KEYS * (DP + 4) + (size_t)FT_KEYS * DP + FT_ROWS * FT_KEYS); }
+
+template <int DP>
+__global__ void __launch_bounds__(FT_THREADS, 2) paged_attn_f32_tile_kernel(const AttnParams p) {
+    constexpr int KP = DP + 4, D4 = DP / 4, NC = DP / 64;            // pitch of the keys; 16-byte pieces of a row; column groups of a thread
+    extern __shared__ __align__(16) float smem[];
+    float* Qs = smem;                       // [FT_ROWS][DP]
+    float* Ks = Qs + FT_ROWS * DP;          // [FT_KEYS][KP]
+    float* Vs = Ks + FT_KEYS * KP;          // [FT_KEYS][DP]
+    float* Ps = Vs + FT_KEYS * DP;          // [FT_ROWS][FT_KEYS]
+    const int D = p.D, G = p.Hq / p.Hkv, tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    int tile = blockIdx.x;
+    const int split = blockIdx.y;
+    const int rt = p.row_tiles - 1 - tile % p.row_tiles; tile /= p.row_tiles;     // (long tiles first)
+    const int kvh = tile % p.Hkv, seq = tile / p.Hkv;
+    TTIE_PDL_ENTRY();
+    const int q0 = p.qsl[seq], q_len = p.qsl[seq + 1] - q0, kv_len = p.seq_lens[seq];
+    const int nrows = q_len * G, row0 = rt * FT_ROWS;
+    if (row0 >= nrows) return;
+    const int ctx = kv_len - q_len;
+    const int tok_lo = row0 / G, tok_hi = (min(nrows, row0 + FT_ROWS) - 1) / G;
+    const KeySpan span = visible_span(ctx + tok_lo, ctx + tok_hi + 1, p.window, p.chunk, p.keep, FT_KEYS);
+    int v_lo, v_hi;                                                  // this CTA's piece, as indices into the span
+    span_piece(span, kv_len, p.window > 0 || p.chunk > 0, split, p.num_splits, p.split_len, FT_KEYS, v_lo, v_hi);
+    const float* qp = reinterpret_cast<const float*>(p.q);
+    const float* kp = reinterpret_cast<const float*>(p.k_pages);
+    const float* vp = reinterpret_cast<const float*>(p.v_pages);
+    const int* table = p.block_table + (size_t)seq * p.table_width;
+
+    float m[FT_R], l[FT_R], o[FT_R][4 * NC];
+    int pos[FT_R];
+#pragma unroll
+    for (int i = 0; i < FT_R; ++i) {
+        const int row = row0 + ty * FT_R + i, tok = row < nrows ? row / G : 0;
+        pos[i] = row < nrows ? ctx + tok : -1;                       // (no key is visible to a row that is not there)
+        m[i] = -INFINITY; l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4 * NC; ++c) o[i][c] = 0.f;
+    }
+    if (v_lo < v_hi)
+        for (int e = tid; e < FT_ROWS * D4; e += FT_THREADS) {
+            const int r = e / D4, d = e % D4 * 4, row = row0 + r;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < nrows && d < D) {
+                const int tok = row / G;
+                v = load4(qp + (size_t)(q0 + tok) * p.q_stride + (size_t)(kvh * G + row - tok * G) * D + d);
+            }
+            *reinterpret_cast<float4*>(Qs + r * DP + d) = v;
+        }
+    for (int vt = v_lo; vt < v_hi; vt += FT_KEYS) {
+        __syncthreads();
+        // a thread's pieces are the same columns of keys STEP apart; eight loads are on their way together
+        constexpr int STEP = FT_THREADS / D4, BATCH = FT_KEYS / STEP < 8 ? FT_KEYS / STEP : 8;
+        const int d = tid % D4 * 4, nk = min(FT_KEYS, v_hi - vt);
+#pragma unroll
+        for (int j0 = tid / D4; j0 < FT_KEYS; j0 += BATCH * STEP) {
+            size_t src[BATCH];
+            bool in[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int j = j0 + i * STEP, key = span.key(vt + j);
+                in[i] = j < nk && d < D;
+                const int pg = key / p.page_size;
+                const int page = in[i] && pg < p.table_width ? table[pg] : 0;    // (a table that is too short: the scratch page, not a wild read)
+                src[i] = (((size_t)page * p.Hkv + kvh) * p.page_size + (key - pg * p.page_size)) * D + d;
+            }
+            float4 x[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) x[i] = in[i] ? load4(kp + src[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) *reinterpret_cast<float4*>(Ks + (j0 + i * STEP) * KP + d) = x[i];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) x[i] = in[i] ? load4(vp + src[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) *reinterpret_cast<float4*>(Vs + (j0 + i * STEP) * DP + d) = x[i];
+        }
+        __syncthreads();
+
+        float s[FT_R][4];
+#pragma unroll
+        for (int i = 0; i < FT_R; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+        auto scores = [&](auto groups) {                             // (a tail of up to 16 keys: the first group of every thread's four)
+            constexpr int J = decltype(groups)::value;
+#pragma unroll 2
+            for (int c = 0; c < DP; c += 4) {
+                float4 q[FT_R], k[J];
+#pragma unroll
+                for (int j = 0; j < J; ++j) k[j] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * KP + c);
+#pragma unroll
+                for (int i = 0; i < FT_R; ++i) q[i] = *reinterpret_cast<const float4*>(Qs + (ty * FT_R + i) * DP + c);
+#pragma unroll
+                for (int i = 0; i < FT_R; ++i)
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+                        s[i][j] = fmaf(q[i].w, k[j].w, fmaf(q[i].z, k[j].z, fmaf(q[i].y, k[j].y, fmaf(q[i].x, k[j].x, s[i][j]))));
+            }
+        };
+        if (nk > 16) scores(std::integral_constant<int, 4>{});
+        else scores(std::integral_constant<int, 1>{});
+#pragma unroll
+        for (int i = 0; i < FT_R; ++i) {
+            const int lo = first_visible_key(pos[i], p.window, p.chunk);
+            float top = -INFINITY;
+            bool vis[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int v = vt + tx + 16 * j, key = span.key(v);
+                vis[j] = v < v_hi && key <= pos[i] && (key >= lo || key < p.keep);
+                s[i][j] *= p.scale;
+                if (p.softcap > 0.f) s[i][j] = p.softcap * tanhf(s[i][j] / p.softcap);
+                if (vis[j]) top = fmaxf(top, s[i][j]);
+            }
+            float sum = 0.f;
+            if (p.sigmoid) {
+                const float hb = p.head_bias && pos[i] >= 0 ? p.head_bias[kvh * G + (row0 + ty * FT_R + i) % G] : 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = vis[j] ? 1.0f / (1.0f + expf(-(s[i][j] + hb))) : 0.f;
+            } else {
+#pragma unroll
+                for (int k = 1; k < 16; k <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, k));
+                const float m_new = fmaxf(m[i], top);
+                const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { s[i][j] = vis[j] ? expf(s[i][j] - m_new) : 0.f; sum += s[i][j]; }
+#pragma unroll
+                for (int k = 1; k < 16; k <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+                l[i] = l[i] * alpha + sum;
+                m[i] = m_new;
+#pragma unroll
+                for (int c = 0; c < 4 * NC; ++c) o[i][c] *= alpha;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) Ps[(ty * FT_R + i) * FT_KEYS + tx + 16 * j] = s[i][j];
+        }
+        __syncwarp();                                                // (a row's weights come from and go to one half of this warp)
+#pragma unroll 2
+        for (int j = 0; j < nk; j += 4) {                            // (past the last key: weights of zero, values of zero)
+            float4 w[FT_R];
+#pragma unroll
+            for (int i = 0; i < FT_R; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (ty * FT_R + i) * FT_KEYS + j);
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float4 v = *reinterpret_cast<const float4*>(Vs + (j + jj) * DP + tx * 4 + 64 * c);
+#pragma unroll
+                    for (int i = 0; i < FT_R; ++i) {
+                        const float a = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
+                        o[i][4 * c] = fmaf(a, v.x, o[i][4 * c]); o[i][4 * c + 1] = fmaf(a, v.y, o[i][4 * c + 1]);
+                        o[i][4 * c + 2] = fmaf(a, v.z, o[i][4 * c + 2]); o[i][4 * c + 3] = fmaf(a, v.w, o[i][4 * c + 3]);
+                    }
+                }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < FT_R; ++i) {
+        const int row = row0 + ty * FT_R + i;
+        if (row >= nrows) continue;
+        const int tok = row / G;
+        const size_t grow = (size_t)(q0 + tok) * p.Hq + kvh * G + (row - tok * G);
+        const bool whole = p.num_splits == 1;
+        float* dst = whole ? reinterpret_cast<float*>(p.out) + grow * D : p.ws_o + (grow * p.num_splits + split) * D;
+        const float inv = !whole || p.sigmoid ? 1.f : l[i] > 0.f ? 1.f / l[i] : 0.f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int col = tx * 4 + 64 * c;
+            if (col < D) *reinterpret_cast<float4*>(dst + col) = make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+        }
+        if (!whole && tx == 0) {
+            float* ml = p.ws_ml + (grow * p.num_splits + split) * 2;
+            ml[0] = p.sigmoid ? 0.f : m[i]; ml[1] = p.sigmoid ? 1.0f / (float)p.num_splits : l[i];
+        }
+    }
+}
+
+// CTAs of the grid that find a key to look at, at least (the pieces of the key range behind a row tile's own tokens hold none), up to `limit`
+long long ctas_with_work(const AttnParams& p, int max_q_len, long long limit) {
+    const long long seqs = (long long)p.num_seqs * p.Hkv;
+    if (p.num_splits <= 1 || p.split_len <= 0 || p.window > 0 || p.chunk > 0) return seqs * p.row_tiles * p.num_splits;
+    const int G = p.Hq / p.Hkv;
+    const long long ctx = max((long long)(p.num_splits - 1) * p.split_len + 1 - max_q_len, 0LL);      // (at least: the last piece is not empty)
+    long long n = 0;
+    for (int rt = 0; rt < p.row_tiles && n * seqs <= limit; ++rt)
+        n += min((long long)p.num_splits, (ctx + (min((rt + 1) * FT_ROWS, max_q_len * G) - 1) / G) / p.split_len + 1);
+    return n * seqs;
+}
+
+template <int DP>
+int launch_f32_tile(AttnParams p, int T_tokens, int max_q_len, cudaStream_t s) {
+    p.row_tiles = ceil_div(max_q_len * (p.Hq / p.Hkv), FT_ROWS);
+    // where every SM can have at most one CTA with work, the launch asks for more than half of an SM's shared memory: left to
+    // itself the hardware pairs CTAs on one SM while others stand empty (300 tokens of 16 heads of 128 in three pieces: 48 us, 32 spread)
+    constexpr size_t SPREAD = 115 * 1024;
+    const bool spread = ctas_with_work(p, max_q_len, num_sms()) <= num_sms();
+    cudaFuncSetAttribute(paged_attn_f32_tile_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SPREAD);
+    TTIE_LAUNCH(paged_attn_f32_tile_kernel<DP>, dim3(p.num_seqs * p.Hkv * p.row_tiles, p.num_splits), FT_THREADS,
+                spread ? SPREAD : tile_smem<DP>(), s, p);
+    TTIE_CHECK_LAUNCH("paged_attention (float32 tiles)");
+    return p.num_splits > 1 ? attn_merge(p.ws_o, p.ws_ml, (float*)p.out, (long long)T_tokens * p.Hq, p.num_splits, p.D, s) : 0;
+}
 }  // namespace
 
 namespace ttie {
 int attn_merge_bf16(const float* ws_o, const float* ws_ml, void* out, int rows, int num_splits, int D, cudaStream_t s) {
-    const dim3 grid(rows, ceil_div(D, 128));
-    const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(ws_o) | reinterpret_cast<uintptr_t>(ws_ml)) & 15) == 0
-                     && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
-    if (vec && num_splits <= 8) {
-        const long long threads = (long long)rows * (D / 4);
-        const unsigned blocks = (unsigned)((threads + 255) / 256);
-        if (num_splits <= 2) { TTIE_LAUNCH(attn_merge_vec_kernel<2>, blocks, 256, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, (long long)rows, num_splits, D); }
-        else if (num_splits <= 4) { TTIE_LAUNCH(attn_merge_vec_kernel<4>, blocks, 256, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, (long long)rows, num_splits, D); }
-        else { TTIE_LAUNCH(attn_merge_vec_kernel<8>, blocks, 256, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, (long long)rows, num_splits, D); }
-    } else if (num_splits <= 4) {
-        TTIE_LAUNCH((attn_merge_small_kernel<__nv_bfloat16, 4>), grid, 128, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, num_splits, D);
-    } else if (num_splits <= 8) {
-        TTIE_LAUNCH((attn_merge_small_kernel<__nv_bfloat16, 8>), grid, 128, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, num_splits, D);
-    } else if (num_splits <= 16) {
-        TTIE_LAUNCH((attn_merge_small_kernel<__nv_bfloat16, 16>), grid, 128, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, num_splits, D);
-    } else if (num_splits <= 32) {
-        TTIE_LAUNCH((attn_merge_small_kernel<__nv_bfloat16, 32>), grid, 128, 0, s, ws_o, ws_ml, (__nv_bfloat16*)out, num_splits, D);
-    } else {
-        TTIE_LAUNCH(attn_merge_kernel<__nv_bfloat16>, rows, MERGE_GROUPS * (D >= 128 ? 128 : 64), (num_splits + MERGE_GROUPS * D) * sizeof(float), s,
-                    ws_o, ws_ml, (__nv_bfloat16*)out, num_splits, D);
-    }
-    TTIE_CHECK_LAUNCH("attention merge");
-    return 0;
+    return attn_merge(ws_o, ws_ml, (__nv_bfloat16*)out, rows, num_splits, D, s);
 }
 }  // namespace ttie
 
@@ -384,12 +603,7 @@ int launch(const AttnParams& p, int T_tokens, cudaStream_t s) {
     dim3 grid(p.num_seqs * p.Hkv * p.row_tiles, p.num_splits);
     k<<<grid, WARPS * 32, smem, s>>>(p);
     TTIE_CHECK_LAUNCH("paged_attention");
-    if (p.num_splits > 1) {
-        attn_merge_kernel<T><<<T_tokens * p.Hq, MERGE_GROUPS * (p.D >= 128 ? 128 : 64), (p.num_splits + MERGE_GROUPS * p.D) * sizeof(float), s>>>(
-            p.ws_o, p.ws_ml, (T*)p.out, p.num_splits, p.D);
-        TTIE_CHECK_LAUNCH("attention merge");
-    }
-    return 0;
+    return p.num_splits > 1 ? attn_merge(p.ws_o, p.ws_ml, (T*)p.out, (long long)T_tokens * p.Hq, p.num_splits, p.D, s) : 0;
 }
 
 template <typename T>
@@ -690,6 +904,9 @@ extern "C" int ttie_paged_attention_weights(const void* q, long long q_stride, c
     if ((long long)p.num_seqs * p.Hkv * p.row_tiles > 2147483647LL) TTIE_FAIL("paged_attention: grid too large");
     if (num_splits > 65535) TTIE_FAIL("paged_attention: too many splits (%d)", num_splits);
     cudaStream_t s = (cudaStream_t)stream;
+    // (rows of queries on 16 bytes, and outputs)
+    if (dtype == kF32 && D <= 128 && max_q_len * G >= FT_ROWS && q_stride % 4 == 0 && !(((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out | (uintptr_t)scratch) & 15))
+        return D <= 64 ? launch_f32_tile<64>(p, T, max_q_len, s) : launch_f32_tile<128>(p, T, max_q_len, s);
     if (dtype == kF32) return dispatch<float>(p, T, s);
     if (dtype == kBF16) return dispatch<__nv_bfloat16>(p, T, s);
     TTIE_FAIL("paged_attention: unknown dtype %d", dtype);

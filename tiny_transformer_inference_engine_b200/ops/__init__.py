@@ -723,6 +723,8 @@ class CudaOps:
         else:
             kernel, tile_rows, unit, min_len = "simt", 32, 32, 32      # (one 32-key tile per CTA where the GPU has room: 10.6 us
                                                                       # against 21 for 200 keys in two pieces of 128)
+        if dtype == torch.float32 and head_dim <= 128 and rows >= 64:
+            return self._f32_tile_pieces(num_seqs * num_kv_heads, rows, G, head_dim, max_q_len, max_kv_len)
         base = num_seqs * num_kv_heads * math.ceil(rows / tile_rows)
         if kernel == "mma" and rows <= 64:      # (one row tile per request and kv head: decoded tokens and the like)
             return self._mma_split_plan(base, head_dim, max_q_len, num_heads, num_kv_heads, max_kv_len)
@@ -733,6 +735,38 @@ class CudaOps:
         split_len = math.ceil(math.ceil(max_kv_len / want) / unit) * unit
         num_splits = math.ceil(max_kv_len / split_len)
         return (kernel, num_splits, split_len) if num_splits > 1 else (kernel, 1, 0)
+
+    def _f32_tile_pieces(self, heads, rows, group, head_dim, max_q_len, max_kv_len):
+        """Pieces of the key range for the float32 tiles of 64 rows and 64 keys, by a cost model fitted to measurements (one to 16
+        requests of 4 to 2,048 tokens behind up to 4,096 keys, head sizes 64 and 128): a tile step takes an SM 11.2 us at head
+        size 128 and 7.3 at 64 with one CTA, 1.84 of that for two CTAs' steps side by side; a piece behind a row tile's own tokens
+        is empty; a cut range costs 3 us and its partial results' way through memory at 2 TB/s.  (16 heads on one kv head of 128:
+        300 tokens 32 us in three pieces, 62 uncut; 600 tokens 70 in four, 148 uncut; 128 tokens behind 4,096 keys 144 in ten,
+        194 in four; 2,048 tokens 583 uncut, 614 in four.)"""
+        step = 3.4 + 0.061 * (64 if head_dim <= 64 else 128)
+        tiles, ctx = math.ceil(rows / 64), max(0, max_kv_len - max_q_len)
+        ends = [ctx + -(-min(rows, (t + 1) * 64) // group) for t in range(tiles)]          # (keys that a row tile sees)
+        work = sum(-(-e // 64) for e in ends) * heads / self.num_sms * 0.92 * step
+        best, best_cost, last = ("simt", 1, 0), None, 0
+        for want in range(1, min(64, math.ceil(max_kv_len / 64)) + 1):
+            split_len = math.ceil(math.ceil(max_kv_len / want) / 64) * 64
+            n = math.ceil(max_kv_len / split_len)
+            if n == last:
+                continue
+            last = n
+            ctas = heads * sum(-(-e // split_len) for e in ends)
+            alone = split_len / 64 * step
+            if ctas <= self.num_sms:
+                cost = alone
+            elif ctas <= 2.2 * self.num_sms or n == 1:                 # (two a SM; the last pieces are the short ones)
+                cost = max(1.84 * alone, work)
+            else:
+                cost = work + 0.5 * alone
+            if n > 1:
+                cost += 3.0 + heads * rows * (n * (4 * head_dim + 8) + 4 * head_dim) / 2e6
+            if best_cost is None or cost < 0.97 * best_cost:
+                best, best_cost = (("simt", n, split_len) if n > 1 else ("simt", 1, 0)), cost
+        return best
 
     def _portion_pieces(self, all_rows, head_dim, max_kv_len, kernels, may_cut):
         """The cheapest of ``kernels`` (name, CTAs per piece, us per key) and cuts of the key range for prompt portions whose
