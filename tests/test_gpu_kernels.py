@@ -1174,3 +1174,27 @@ def test_skinny_gemm_through_shared_memory_in_a_chain(ops):
         last, ref = ref, ref + ref_delta
     assert rel((stream.double() + delta.double()).cpu(), ref.cpu()) < 1e-2
     assert ops.lib.ttie_tc_error() == 0
+
+
+@pytest.mark.parametrize("N,K", [(4096, 512), (1024, 16384), (32000, 1024)])
+def test_skinny_gemm_ends_when_one_warp_gives_up(ops, N, K):
+    """A multiplying warp whose wait runs out takes the whole CTA with it: the launch ends (the copying thread's limit is about a second), leaves
+    its code, and the next launch is right.  Units that fit the ring, units that do not, units that are handed on."""
+    g = torch.Generator().manual_seed(49)
+    x, w = torch.randn(8, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV)
+    assert ops.lib.ttie_tc_error() == 0
+    call = lambda out: ops.lib.ttie_skinny_gemm_tuned(x.data_ptr(), K, w.data_ptr(), K, None, out.data_ptr(), N, 8, N, K, -(-K // 128) * 128, 3, 0, 0,
+                                                      torch.cuda.current_stream().cuda_stream)
+    out = torch.empty(8, N, device=DEV)
+    for warp in (0, 3):
+        ops.lib.ttie_skinny_quitter(warp)
+        try:
+            assert call(out) == 0
+        finally:
+            ops.lib.ttie_skinny_quitter(-1)
+        torch.cuda.synchronize()
+        assert ops._tc_words[0] != 0 and ops.lib.ttie_tc_error() in (61, 62)
+        ops._tc_words[:] = 0
+        assert call(out) == 0
+        assert rel(out.double().cpu(), (x.double() @ w.double().T).cpu()) < 1e-6 + K / 64 * 2.0 ** -24
+        assert ops.lib.ttie_tc_error() == 0 and not ops._tc_words.any()

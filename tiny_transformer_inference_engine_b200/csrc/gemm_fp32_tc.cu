@@ -320,10 +320,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                         tma_load_2d(dst + HALF * 128, &tmW, BAR(WFULL + s), (kb0 + kb) * KB + 32, n0 + h * HALF);
                         if (++s == p.w_stages) { s = 0; ++round; }
                     }
-                if (!ok)                                         // (nothing may land in a CTA that has left; each wait is bounded)
-                    for (int i = 0; i < p.w_stages; ++i) {
-                        if (round > 0 || i < s) mbar_wait(BAR(WFULL + i), (i < s ? round : round - 1) & 1, 44, p);
-                    }
+                // nothing may land in a CTA that has left, and the other roles may have given up (each wait is bounded)
+                for (int i = 0; i < p.w_stages; ++i)
+                    if (round > 0 || i < s) mbar_wait(BAR(WFULL + i), (i < s ? round : round - 1) & 1, 44, p);
             }
         } else if (warp == ISSUE + 2) {
             if (lane == 0) {
@@ -337,8 +336,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                     for (int i = 0; i < 3; ++i)
                         tma_load_2d(x_ring + (uint32_t)s * x_stage + (uint32_t)i * plane, &tmX, BAR(XFULL + s), (kb0 + kb) * KB, i * p.M + m0);
                 }
-                if (kb < nkb)
-                    for (int i = kb - 2 < 0 ? 0 : kb - 2; i < kb; ++i) mbar_wait(BAR(XFULL + (i & 1)), (i >> 1) & 1, 45, p);
+                for (int i = kb - 2 < 0 ? 0 : kb - 2; i < kb; ++i) mbar_wait(BAR(XFULL + (i & 1)), (i >> 1) & 1, 45, p);
             }
         } else if (((warp - ISSUE) >> 1) < halves) {
             if (lane == 0) {
@@ -346,7 +344,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 // D float32, A and B bfloat16, both K-major, M 128, N the rows of A here up to a multiple of 16
                 const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((toks + 15) / 16 * 2) << 17) | ((uint32_t)(HALF >> 4) << 24);
                 const uint32_t d = tmem_base + D_COL + (uint32_t)(h * TOK_MOST), a = tmem_base + P_COL + (uint32_t)h * P_COLS;
-                for (int kb = 0; kb < nkb; ++kb) {
+                int kb = 0;
+                for (; kb < nkb; ++kb) {
                     const int s = kb & 1;
                     if (!mbar_wait(BAR(XFULL + s), (kb >> 1) & 1, 46, p)) break;
                     if (!mbar_wait(BAR(DEMPTY + h), (kb & 1) ^ 1, 48, p) || !mbar_wait(BAR(AFULL + h), kb & 1, 47, p)) break;
@@ -363,6 +362,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                     umma_commit(BAR(XEMPTY + s));
                     umma_commit(BAR(DFULL + h));
                 }
+                if (kb > 0) mbar_wait(BAR(DFULL + h), (kb - 1) & 1, 48, p);      // (its products are done before the CTA frees their tensor memory)
             }
         }
         __syncwarp();

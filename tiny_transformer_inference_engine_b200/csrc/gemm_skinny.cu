@@ -224,18 +224,27 @@ struct BulkParams {
     SkinnyParams g;
     int tiles, units, stages, stage_bytes, dynamic;
     int *err, *mirror;
+    int quitter;                                             // a multiplying warp whose waits run out at once (tests of giving up), or -1
 };
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code, const BulkParams& p) {
-    if (mbar_try(bar, parity)) return true;
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code, const BulkParams& p, bool quits = false) {
+    if (!quits && mbar_try(bar, parity)) return true;
     const long long deadline = clock64() + WAIT_CYCLES;
-    while (!mbar_try(bar, parity)) {
-        if (clock64() > deadline) {
+    while (quits || !mbar_try(bar, parity)) {
+        if (quits || clock64() > deadline) {
             atomicCAS(p.err, 0, code);
             if (p.mirror) { *reinterpret_cast<volatile int*>(p.mirror) = code; __threadfence_system(); }
             return false;
         }
     }
     return true;
+}
+// Barrier of the 128 multiplying threads, each of which comes here once a unit whether its waits ran out or not: a warp that went away alone
+// would leave the others waiting without a limit.  Tells all of them whether one of them gave up.
+__device__ __forceinline__ bool any_of_128(bool bad) {
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(any) : "r"((uint32_t)bad) : "memory");
+    return any != 0;
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row, int block) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -285,7 +294,7 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
         if (lane != 0) return;
         const uint32_t bytes = Sh::WEIGHTS + (uint32_t)(Sh::BLOCKS * p.M * 128);
         int s = 0, round = 0, ahead = 0, turn = 0;               // ahead: stages whose activations are still to come; turn: questions answered
-        bool ok = true, waited = false;
+        bool ok = true, waited = false, open = false;               // open: a question without its answer
         auto acts = [&](int k0, int st) { tma_load_3d(ring0 + (uint32_t)st * bp.stage_bytes + Sh::WEIGHTS, &tmX, full0 + 8 * st, 0, k0 / 64); };
         auto settle = [&]() {                                    // the kernel before is done: the activations of the stages filled so far
             pdl_wait();
@@ -293,17 +302,14 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
             waited = true;
             for (int i = 0; i < ahead; ++i) acts(stage_k[i], i);
         };
-        auto free_stage = [&]() {
-            if (!waited && ahead == bp.stages) settle();
-            if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, 61, bp);
-            return ok;
-        };
         // a CTA that has not started yet gives its unit to one that has room for it
         auto ask = [&]() {
+            open = true;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(asked) : "memory");
             asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_unit)), "r"(asked) : "memory");
         };
         auto answer = [&]() -> int {                             // its number, or -1: all have started
+            open = false;
             if (!mbar_wait(asked, turn++ & 1, 63, bp)) { ok = false; return -1; }
             uint32_t given, x;
             asm volatile("{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tld.shared.b128 h, [%2];\n\t"
@@ -338,27 +344,29 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
             unit = next;
         }
         if (!waited) settle();
-        if (!ok)                                                 // (nothing may land in a CTA that has left; each wait is bounded)
-            for (int i = 0; i < bp.stages; ++i) if (round > 0 || i < s) mbar_wait(full0 + 8 * i, (i < s ? round : round - 1) & 1, 61, bp);
+        // nothing may land in a CTA that has left, and the multiplying warps may have given up (each wait is bounded)
+        for (int i = 0; i < bp.stages; ++i) if (round > 0 || i < s) mbar_wait(full0 + 8 * i, (i < s ? round : round - 1) & 1, 61, bp);
+        if (open) mbar_wait(asked, turn & 1, 63, bp);
         return;
     }
+    pdl_wait();                                                  // (so that a wait's limit does not count the time of the kernel before)
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     int s = 0, round = 0;
-    auto arrived = [&]() { return (bool)__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, round & 1, 62, bp)); };
+    auto arrived = [&]() { return (bool)__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, round & 1, 62, bp, warp == bp.quitter)); };
     auto next_stage = [&]() { if (++s == bp.stages) { s = 0; ++round; } };
     bool more = true;
     for (int turn = 0; more; turn ^= 1) {
         bool ok = arrived();
-        if (!ok) break;
         int n0, split, k_begin, k_end;
-        range_of(stage_unit[s], n0, split, k_begin, k_end);
+        range_of(ok ? stage_unit[s] : 0, n0, split, k_begin, k_end);
         float acc[NSET][MT][4];
 #pragma unroll
         for (int i = 0; i < NSET; ++i)
 #pragma unroll
             for (int j = 0; j < MT; ++j) { acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f; }
         for (int k0 = k_begin; k0 < k_end; k0 += KS) {
-            if (k0 > k_begin) { ok = arrived(); if (!ok) break; }
+            if (k0 > k_begin) ok = arrived();
+            if (!ok) break;
             const unsigned char* base = ring + (size_t)s * bp.stage_bytes;
             more = stage_more[s];
 #pragma unroll
@@ -388,17 +396,18 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty0 + 8 * s) : "memory");
             next_stage();
         }
-        if (!ok) break;
 #pragma unroll
         for (int i = 0; i < NSET; ++i)
 #pragma unroll
             for (int j = 0; j < MT; ++j)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) red[turn][warp][i][j][lane][c] = acc[i][j][c];
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (any_of_128(!ok)) break;
         finish_tile<MT, EPI, NSET>(p, red[turn], n0, split, warp, lane);
     }
 }
+
+thread_local int g_quitter = -1;
 
 template <int MT, int EPI, int SETS>
 int launch_bulk(const SkinnyParams& p, int splits, cudaStream_t s) {
@@ -407,6 +416,7 @@ int launch_bulk(const SkinnyParams& p, int splits, cudaStream_t s) {
     constexpr int ROOM = 228 * 512 - 1024 - 320 - 2 * 4 * NSET * MT * 512 - 1024;              // what two CTAs per SM leave for a ring
     BulkParams b;
     b.g = p;
+    b.quitter = g_quitter;
     b.tiles = ceil_div(p.N, unit_columns(EPI, NSET));
     b.units = b.tiles * splits;
     b.stage_bytes = ((int)Sh::WEIGHTS + Sh::BLOCKS * p.M * 128 + 1023) / 1024 * 1024;
@@ -485,6 +495,8 @@ extern "C" int ttie_skinny_gemm(const void* x, long long ldx, const void* w, lon
                                 long long ldo, int M, int N, int K, int kslice, int epilogue, int up_offset, void* stream) {
     return ttie_skinny_gemm_tuned(x, ldx, w, ldw, bias, out, ldo, M, N, K, kslice, epilogue, up_offset, 0, stream);
 }
+// for tests: multiplying warp `warp` (0 to 3; -1: none) of this thread's launches gives up at its first wait; an error code and no hang is what follows
+extern "C" void ttie_skinny_quitter(int warp) { g_quitter = warp; }
 static thread_local float g_glu[3] = {1.f, 0.f, 0.f};
 static thread_local int g_glu_act = 0;
 // the gated-unit epilogue (2) with constants other than SwiGLU's: alpha, limit (<= 0: none), shift, act (1: gelu's tanh form on the gate);
