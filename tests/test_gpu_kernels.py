@@ -1198,3 +1198,33 @@ def test_skinny_gemm_ends_when_one_warp_gives_up(ops, N, K):
         assert call(out) == 0
         assert rel(out.double().cpu(), (x.double() @ w.double().T).cpu()) < 1e-6 + K / 64 * 2.0 ** -24
         assert ops.lib.ttie_tc_error() == 0 and not ops._tc_words.any()
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 2304, 2048), (40, 16400, 260), (33, 520, 4096)])
+def test_gemm_f32_on_tensor_cores_whole_exponent_range(ops, M, N, K):
+    """Every finite value counts with all of its bits, whatever stands beside it in its row: rows of subnormal numbers alone, small values beside
+    large ones that meet a zero, sums that are subnormal themselves.  Bound: K roundings of the magnitudes that are added, as for 32-bit
+    multiply-adds, and of 2^-149."""
+    g = torch.Generator().manual_seed(50)
+    x, w = torch.randn(M, K, generator=g, dtype=torch.float64), torch.randn(N, K, generator=g, dtype=torch.float64)
+    x[1], x[2], x[3], x[4], x[5] = x[1] * 1e-41, x[2] * 3e-45, x[3] * 1e-38, x[4] * 1e-36, x[5] * 1e-20
+    x[4, 0], x[6, ::2] = 1.0, x[6, ::2] * 1e-33                       # (one large value, which meets a zero in some columns; every other value small)
+    x[7] = torch.where(torch.arange(K) % 3 == 0, 2.0 ** 100, 2.0 ** -140) * x[7]
+    w[0], w[1], w[2], w[3] = w[0] * 1e30, w[1] * 1e-41, w[2] * 1e33, w[3] * 1e-20
+    w[:, 0] = 0
+    w[4], w[5, ::2] = w[4] * 1e-44, w[5, ::2] * 2.0 ** -120
+    w[6] = torch.where(torch.arange(K) % 3 == 0, 0.0, 2.0 ** 120) * w[6]
+    x, w = x.float().to(DEV), w.float().to(DEV)
+    assert ops._f32_planes_ok(x, w)
+    exp, scale = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    clear = scale < 1e38
+    bound = K * 2.0 ** -24 * scale + K * 2.0 ** -149
+    plain = torch.empty(M, N, device=DEV)
+    assert ops.lib.ttie_gemm_f32(x.data_ptr(), w.data_ptr(), None, plain.data_ptr(), M, N, K, K, K, N, ops._stream(x)) == 0
+    part = ops.linear(x, w, None, partial_ok=True)
+    for got in (plain, ops.linear(x, w, None), part.double().sum(0) if part.dim() == 3 else part):
+        assert ((got.double() - exp).abs()[clear] <= bound[clear]).all()
+    # closer than that: a random walk of the K / 64 additions of 64 terms' sums, at most 64 of them, where sums are no subnormal numbers
+    ok = clear & (scale > 1e-30)
+    assert ((ops.linear(x, w, None).double() - exp).abs()[ok] <= 2.0 ** -21 * scale[ok]).all()
+    assert ops.lib.ttie_tc_error() == 0

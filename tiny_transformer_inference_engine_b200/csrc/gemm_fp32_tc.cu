@@ -2,8 +2,10 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias), all float32, for more than a few rows.
 //
 // A float32 value is the exact sum of three bfloat16 values (24 significant bits in pieces of 8): a = a0 + a1 + a2 with a0 the nearest bfloat16,
-// a1 the rest's leading bits, a2 what is left.  Of the nine products of two such sums six are taken - a0 b0, a0 b1, a1 b0, a1 b1,
-// a0 b2, a2 b0; the other three together are below 2^-24 of |a b|, of either sign.  bfloat16 products are exact in the tensor core's 32-bit
+// a1 the rest's leading bits, a2 what is left.  Both operands are taken times 2^24, and the sums times 2^-48: so every value but 0 has its
+// leading bits in a0 and all of its last ones in a2, subnormal values too (2^-149 becomes 2^-125, and bfloat16 goes down to
+// 2^-133).  Of the nine products of two such sums six are taken - a0 b0, a0 b1, a1 b0, a1 b1, a0 b2, a2 b0; the other three together are below
+// 2^-24 of |a b|, of either sign.  bfloat16 products are exact in the tensor core's 32-bit
 // sums, whose additions are cut off, not rounded: so a sum in tensor memory spans 64 values of K only, its large products (a0 b0) come
 // last, and these sums are added up in registers by ordinary rounded additions.  Error against 64 bits (2-norm over 2-norm, normal
 // values; the multiply-add kernel of gemm_fp32.cu in brackets): 300 rows of K 2,048 1.0e-7 (3.3e-7), of K 8,192 1.3e-7 (4.4e-7), 33 rows of K 64
@@ -26,9 +28,8 @@
 // Tensor memory: two halves' sums of 160 columns, planes of two units of 96: 512.  K ranges are CTAs of a cluster, whose
 // partial tiles are added through distributed shared memory in the order of the ranges: the result does not depend on timing.
 //
-// What three bfloat16 cannot hold is found and computed again by 32-bit multiply-adds: an infinity, NaN or a value that rounds to an infinity leaves
-// a sum that is not finite, and a row of A, or of W within the range of K, whose largest value is below 2^-95 is marked with a NaN,
-// since its lower planes reach into numbers that bfloat16 does not have (2^-126 and less).
+// What that does not hold is found and computed again by 32-bit multiply-adds: an infinity, a NaN, a value from 2^104 on or a sum from 2^80 on leaves
+// a sum that is not finite.
 // Every mbarrier wait is bounded by a clock deadline; one that runs out records a code and the roles leave their loops.
 #include "planes.cuh"
 #include <cuda.h>
@@ -45,6 +46,7 @@ constexpr int HALF = 128, KB = 64, TOK_MOST = 160, MAX_RANGES = 8, MAX_PARTIAL =
 constexpr uint32_t W_BYTES = HALF * KB * 4, D_COL = 0, P_COL = 2 * TOK_MOST, P_COLS = 3 * KB / 2, TMEM_COLS = 512;
 constexpr uint32_t SMEM_MOST = 226 * 1024;
 constexpr int W_STAGES_MOST = 6;
+constexpr float UP = 16777216.f, DOWN = 3.5527136788005009e-15f;          // 2^24 on the operands, 2^-48 on the sums
 constexpr long long WAIT_CYCLES = 2000000000LL;                 // about one second
 
 enum { WFULL = 0, WEMPTY = W_STAGES_MOST, XFULL = 2 * W_STAGES_MOST, XEMPTY = XFULL + 2, AFULL = XEMPTY + 2, AEMPTY = AFULL + 2, DFULL = AEMPTY + 2,
@@ -117,40 +119,22 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
-// From the OR of a row's first planes: whether its largest value is below 2^-95 (its exponent's upper three bits are 0) and not 0
-__device__ __forceinline__ bool is_tiny(uint32_t m) {
-    m = (m | m >> 16) & 0x7fffu;
-    return m != 0 && (m & 0x7000u) == 0;
-}
-
 // Rows of A -> planes [3, M, pitch].  One block per row: memory-bound, 4 bytes read and 6 written a value (300 rows of 2,048: 2.4 us).
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, int lda, __nv_bfloat16* __restrict__ planes, int M, int K, int pitch) {
-    __shared__ uint32_t block_bits[8];
     TTIE_PDL_ENTRY();
     const int row = blockIdx.x;
     const float* src = A + (size_t)row * lda;
     uint32_t* dst[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) dst[i] = reinterpret_cast<uint32_t*>(planes + ((size_t)i * M + row) * pitch);
-    uint32_t m = 0;
     for (int k = threadIdx.x * 4; k < K; k += 1024) {            // (K is a multiple of 4)
         const float4 v = *reinterpret_cast<const float4*>(src + k);
-        float x[4] = {v.x, v.y, v.z, v.w};
+        float x[4] = {v.x * UP, v.y * UP, v.z * UP, v.w * UP};
         uint32_t q[3][2];
         split_values<2>(x, q[0], q[1], q[2]);
-        m |= q[0][0] | q[0][1];
 #pragma unroll
         for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(dst[i] + k / 2) = make_uint2(q[i][0], q[i][1]);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
-    if ((threadIdx.x & 31) == 0) block_bits[threadIdx.x >> 5] = m;
-    __syncthreads();                                             // (also: the planes' words are written before some are overwritten)
-    m = 0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) m |= block_bits[w];
-    if (is_tiny(m))                                              // every range's sums of the row become NaN and are computed from A itself
-        for (int k = threadIdx.x * KB; k < K; k += 256 * KB) dst[0][k / 2] = 0x7fff7fffu;
 }
 
 // One output by 32-bit multiply-adds (where the planes do not hold the values)
@@ -175,7 +159,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) unsigned long long bars[NBARS];
     __shared__ uint32_t tmem_slot;
-    __shared__ unsigned char row_tiny[2 * HALF];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x % p.ranges, tile = blockIdx.x / p.ranges;               // clusters are consecutive CTAs
     const int m0 = tile % p.tok_tiles * p.width, n0 = tile / p.tok_tiles * (2 * HALF);
@@ -235,7 +218,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");         // every product is done: the stages take the partial tile, [row of A][row of W]
-        const bool tiny = row_tiny[row];
         if (direct) {                                           // straight from the registers: neighbouring lanes are neighbouring columns
             const int n = n0 + row;
             if (n < p.N) {
@@ -243,11 +225,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 float* dst = C + (size_t)m0 * p.ldc + n;
 #pragma unroll
                 for (int i = 0; i < TOK; ++i) {
-                    if (i < toks) *dst = acc[i] + b;
+                    if (i < toks) *dst = fmaf(acc[i], DOWN, b);
                     dst += p.ldc;
                     bad |= i < toks && !(fabsf(acc[i]) <= 3.4028234e38f);
                 }
-                bad |= tiny;
             }
         } else {
             float* part = reinterpret_cast<float*>(smem) + row;
@@ -255,7 +236,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             for (int c = 0; c < TOK / 16; ++c)
                 if (c * 16 < toks) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) part[(c * 16 + j) * (2 * HALF)] = tiny ? __int_as_float(0x7fffffff) : acc[c * 16 + j];
+                    for (int j = 0; j < 16; ++j) part[(c * 16 + j) * (2 * HALF)] = acc[c * 16 + j];
                 }
         }
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SPLIT == 1 ? 128 : 96) : "memory");
@@ -265,7 +246,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             // SPLIT 2: four warps for each half, else four for both in turn
             const int quarter = warp & 3, r = quarter * 32 + lane, own = SPLIT == 2 ? (warp - 8) >> 2 : 0;
             const uint32_t a = tmem_base + ((uint32_t)(quarter * 32) << 16) + P_COL;
-            uint32_t bits[2] = {0, 0};                            // OR of the rows' first planes
             int s = 0, round = 0;
             bool ok = true;
             auto next_stage = [&]() { if (++s == p.w_stages) { s = 0; ++round; } };
@@ -289,9 +269,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                             const uint32_t src = stage + (uint32_t)(g >> 1) * (HALF * 128) + (uint32_t)((((g & 1) * 4 + c) ^ (r & 7)) << 4);
                             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[4 * c]), "=f"(x[4 * c + 1]), "=f"(x[4 * c + 2]), "=f"(x[4 * c + 3]) : "r"(src));
                         }
-                        split_values<8>(x, q0, q1, q2);
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) bits[i] |= q0[c];
+                        for (int c = 0; c < 16; ++c) x[c] *= UP;
+                        split_values<8>(x, q0, q1, q2);
                         const uint32_t dst = a + (uint32_t)h * P_COLS + (uint32_t)g * 8;
                         tmem_st8(dst, q0);
                         tmem_st8(dst + KB / 2, q1);
@@ -305,8 +285,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                     if (SPLIT == 2 && halves == 2) next_stage();   // (the other half's)
                 }
             }
-            if (SPLIT == 2) row_tiny[own * HALF + r] = is_tiny(bits[0]);
-            else { row_tiny[r] = is_tiny(bits[0]); row_tiny[HALF + r] = is_tiny(bits[1]); }
         } else if (warp == ISSUE) {
             if (lane == 0) {
                 int s = 0, round = 0;
@@ -377,7 +355,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 if (n >= p.N) continue;
                 float* dst = C + (size_t)m * p.ldc + n;
                 const int k0 = kb0 * KB;
-                if (row_tiny[r] || !(fabsf(*dst) <= 3.4028234e38f))
+                if (!(fabsf(*dst) <= 3.4028234e38f))
                     *dst = plain_dot(p.A + (size_t)m * p.lda + k0, p.W + (size_t)n * p.ldw + k0, min(p.K - k0, nkb * KB)) + (p.bias ? p.bias[n] : 0.f);
             }
     } else {
@@ -413,8 +391,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
                     if (n + c < p.N) {
-                        if (!(fabsf(v[c]) <= 3.4028234e38f)) v[c] = plain_dot(p.A + (size_t)m * p.lda, p.W + (size_t)(n + c) * p.ldw, p.K);
-                        if (p.bias) v[c] += p.bias[n + c];
+                        const float b = p.bias ? p.bias[n + c] : 0.f;
+                        v[c] = fabsf(v[c]) <= 3.4028234e38f ? fmaf(v[c], DOWN, b) : plain_dot(p.A + (size_t)m * p.lda, p.W + (size_t)(n + c) * p.ldw, p.K) + b;
                     }
                 float* dst = p.C + (size_t)m * p.ldc + n;
                 if (vec && n + 3 < p.N) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
