@@ -1228,3 +1228,31 @@ def test_gemm_f32_on_tensor_cores_whole_exponent_range(ops, M, N, K):
     ok = clear & (scale > 1e-30)
     assert ((ops.linear(x, w, None).double() - exp).abs()[ok] <= 2.0 ** -21 * scale[ok]).all()
     assert ops.lib.ttie_tc_error() == 0
+
+
+def test_gemm_f32_on_tensor_cores_from_several_threads(ops):
+    """Row counts whose launches ask for different amounts of shared memory, from four threads with a stream each: none is refused."""
+    import threading
+    g = torch.Generator().manual_seed(51)
+    w = torch.randn(1024, 1536, generator=g).to(DEV)
+    failed = []
+
+    def work(M):
+        x = torch.randn(M, 1536, generator=torch.Generator().manual_seed(M)).to(DEV)
+        stream = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(stream):
+                first = ops.linear(x, w, None)
+                for _ in range(400):
+                    last = ops.linear(x, w, None)
+                stream.synchronize()
+            assert torch.equal(first, last)
+        except Exception as e:                                            # (an assertion in a thread would be lost)
+            failed.append((M, e))
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(M,)) for M in (128, 160, 112, 144)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed

@@ -406,6 +406,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
     if (warp == ISSUE + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
 }
+// The most shared memory that a launch may ask for, set once per device: it is the function's, not the launch's, so setting what one launch needs would
+// refuse another thread's that needs more
+template <int TOK, int SPLIT>
+cudaError_t allow_most() {
+    static std::atomic<bool> done[64];
+    int dev = 64;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev < 64 && done[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<TOK, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
+    if (e == cudaSuccess && dev < 64) done[dev].store(true, std::memory_order_relaxed);
+    return e;
+}
 // Clusters of r CTAs, one CTA per SM, that run at the same time on this device (asked once per device and size)
 int clusters_at_once(int r) {
     static std::atomic<int> known[64][MAX_RANGES + 1];
@@ -415,7 +426,7 @@ int clusters_at_once(int r) {
     int n = known[dev][r].load(std::memory_order_relaxed);
     if (n > 0) return n;
     const int smem = (int)SMEM_MOST;
-    cudaFuncSetAttribute(gemm_f32_tc_kernel<160, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_most<160, 1>();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(r * 64); cfg.blockDim = dim3(512); cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
@@ -482,8 +493,8 @@ extern "C" int ttie_gemm_f32_tc(const float* A, const float* W, const float* bia
     if (p.w_stages > W_STAGES_MOST) p.w_stages = W_STAGES_MOST;
     const size_t smem = (size_t)p.w_stages * W_BYTES + x_ring + 1024;
     auto kernel = narrow ? gemm_f32_tc_kernel<96, 2> : gemm_f32_tc_kernel<160, 1>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) TTIE_FAIL("gemm_f32_tc: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+    cudaError_t e = narrow ? allow_most<96, 2>() : allow_most<160, 1>();
+    if (e != cudaSuccess) TTIE_FAIL("gemm_f32_tc: %u bytes of shared memory refused: %s", SMEM_MOST, cudaGetErrorString(e));
     CUtensorMap mw, mx;
     if (gemm_tc_make_map_of(&mw, 1, W, N, K, ldw, 32, HALF)) return -1;
     if (gemm_tc_make_map_of(&mx, 0, planes, 3LL * M, K, pitch, KB, p.width)) return -1;
