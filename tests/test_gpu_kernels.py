@@ -1122,11 +1122,11 @@ def test_gemm_f32_on_tensor_cores_extreme_values(ops, M, N, K):
         assert (got[12] == 0).logical_or(torch.isnan(plain[12])).all()
 
 
-# 1 and 8 rows, 9 and 16; rows of W that end inside a set of 16, 32 or 64; K that ends inside a stage of 512, 256 or 128; fewer units than run at once, and more
+# 1 and 8 rows, 9 and 16; rows of W that end inside a set of 16 or 32; K that ends inside a stage of 512 or 256; fewer units than run at once, and more
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(4096, 512), (4090, 1088), (16410, 192), (700, 4160), (33, 32768), (9999, 576)])
 def test_skinny_gemm_through_shared_memory(ops, M, N, K):
-    """The weight-streaming product whose weights come by TMA: every epilogue, one, two and four sets of rows, K whole and cut, against 64 bits.
+    """The weight-streaming product whose weights come by TMA: every epilogue, one and two sets of rows, K whole and cut, against 64 bits.
     A warp's sum takes K / 64 instructions, each of which cuts the running sum by up to 2^-23 of it, half of that on average."""
     tol32 = 1e-6 + K / 64 * 2.0 ** -24
     g = torch.Generator().manual_seed(47)
@@ -1135,7 +1135,7 @@ def test_skinny_gemm_through_shared_memory(ops, M, N, K):
     call = lambda out, bias, n, kslice, epi, up, form: ops.lib.ttie_skinny_gemm_tuned(
         x.data_ptr(), K, w.data_ptr(), K, None if bias is None else bias.data_ptr(), out.data_ptr(), n, M, n, K, kslice, epi, up, form, stream)
     whole = -(-K // 128) * 128
-    for form in (0, 16, 32):
+    for form in (0, 16):
         for kslice in {whole, 256, -(-whole // 384) * 128}:
             part = torch.full((-(-K // kslice), M, N), float("nan"), device=DEV)
             assert call(part, None, N, kslice, 1, 0, form) == 0
@@ -1256,3 +1256,40 @@ def test_gemm_f32_on_tensor_cores_from_several_threads(ops):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("M", [1, 8, 13])
+@pytest.mark.parametrize("N,K", [(4352, 4096), (4096, 11008), (9999, 576), (4090, 1088)])
+def test_skinny_gemm_sums_do_not_depend_on_the_row_sets(ops, M, N, K):
+    """One set of 16 weight rows a unit or two: the same sums to the last bit, whole and in ranges of K; and the same again in a second call,
+    wherever the units ran."""
+    g = torch.Generator().manual_seed(52)
+    x, w = torch.randn(M, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV)
+    whole = -(-K // 128) * 128
+    for kslice in (whole, -(-whole // 384) * 128):
+        outs = []
+        for form in (0, 16, 0, 16):
+            out = torch.full((-(-K // kslice), M, N), float("nan"), device=DEV)
+            assert ops.lib.ttie_skinny_gemm_tuned(x.data_ptr(), K, w.data_ptr(), K, None, out.data_ptr(), N, M, N, K, kslice, 1, 0, form,
+                                                  torch.cuda.current_stream().cuda_stream) == 0
+            outs.append(out)
+        assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
+def test_decode_product_is_the_same_after_its_shape_was_measured(ops):
+    """``tune_products`` decides between this package's product and the library's only: the order of this one's sums comes from the sizes."""
+    g = torch.Generator().manual_seed(53)
+    ws = [(torch.randn(4352, 2048, generator=g) * 0.02).bfloat16().to(DEV) for _ in range(2)]
+    keep = dict(ops._product_choice), dict(ops._skinny_tuned)
+    try:
+        ops._product_choice.clear()
+        x = torch.randn(16, 2048, generator=g).bfloat16().to(DEV)
+        before = {M: ops.linear(x[:M], ws[0], None, partial_ok=True) for M in (1, 8)}
+        ops.tune_products(ws)
+        for key in list(ops._product_choice):
+            ops._product_choice[key] = "skinny"
+        for M in (1, 8):
+            assert torch.equal(ops.linear(x[:M], ws[0], None, partial_ok=True), before[M])
+    finally:
+        ops._product_choice.clear(); ops._product_choice.update(keep[0])
+        ops._skinny_tuned.clear(); ops._skinny_tuned.update(keep[1])

@@ -204,9 +204,9 @@ skinny_gemm_kernel(const SkinnyParams p) {
 // ---- up to 16 rows: the weights through shared memory, by TMA.
 // What bounds such a product is HBM, and what decides how close it comes is how many bytes are on their way and that the stream does not stop
 // between two tiles: copies alone, without the products, reach 6.2 TB/s with 128 KB in flight per SM and 7.0 with 192 KB, whatever the order of the
-// rows (180 MB; 33 MB 5.5 and 6.1).  So a CTA stays (two per SM), walks over units (16 rows of W, or 32 or 64: 2 or 4 sets; a
-// range of K), and one thread keeps a ring of stages filled (16 KB of W: 512 values of K of 16 rows, 256 of 32, 128 of 64; and the activations'
-// values, of which more sets need fewer copies) across the units' borders; the weights of the first stages are asked for before the wait for
+// rows (180 MB; 33 MB 5.5 and 6.1).  So a CTA stays (two per SM), walks over units (16 rows of W, or 32: two sets; a
+// range of K), and one thread keeps a ring of stages filled (16 KB of W: 512 values of K of 16 rows, 256 of 32; and the activations'
+// values, of which two sets need half the copies) across the units' borders; the weights of the first stages are asked for before the wait for
 // the kernel before, whose results they do not depend on.  Four warps split a stage's K among themselves, take their operand fragments from
 // shared memory as the other form takes them from global memory (the swizzle spreads eight rows' 16 bytes over all banks), and add up
 // their ranges at the end of a unit.  Activations through the cache instead of the ring were slower (8 rows: 36 against 31 us).
@@ -252,7 +252,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 }
 
 // the gated unit with SETS 1: a set's first eight rows are gate rows, the others their up rows (half as long a unit, twice the activations' copies)
-__host__ __device__ constexpr int row_sets(int epi, int sets) { return epi == 2 && sets > 2 ? 2 : sets; }
 __host__ __device__ constexpr int unit_columns(int epi, int sets) { return epi == 2 ? (sets == 1 ? 8 : 16) : 16 * sets; }
 template <int NSET> struct BulkShape {
     static constexpr int KS = 512 / NSET, BLOCKS = KS / 64;      // K of a stage
@@ -261,10 +260,10 @@ template <int NSET> struct BulkShape {
 
 template <int MT, int EPI, int SETS>
 __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const BulkParams bp) {
-    constexpr int NSET = row_sets(EPI, SETS);
+    constexpr int NSET = SETS;
     constexpr bool PAIRED = EPI == 2 && NSET == 1;
     using Sh = BulkShape<NSET>;
-    constexpr int KS = Sh::KS, KW = KS / 4;                      // KW: K of a warp
+    constexpr int KS = Sh::KS, KW = KS / 4;                      // KW: K of a warp, in every fourth piece of 32: the same pieces with any number of sets
     const SkinnyParams& p = bp.g;
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -371,7 +370,7 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
             more = stage_more[s];
 #pragma unroll
             for (int u = 0; u < KW / 32; ++u) {
-                const int k = warp * KW + 32 * u, block = k >> 6, chunk = ((k >> 3) & 7) + q, at = (chunk ^ r) << 4;       // (row & 7 is r for all of this lane's rows)
+                const int k = 32 * (warp + 4 * u), block = k >> 6, chunk = ((k >> 3) & 7) + q, at = (chunk ^ r) << 4;       // (row & 7 is r for all of this lane's rows)
                 const bool in = k0 + k < k_end;                  // (ranges are multiples of 64)
                 uint4 wv[NSET][2], xv[MT];
 #pragma unroll
@@ -411,7 +410,7 @@ thread_local int g_quitter = -1;
 
 template <int MT, int EPI, int SETS>
 int launch_bulk(const SkinnyParams& p, int splits, cudaStream_t s) {
-    constexpr int NSET = row_sets(EPI, SETS);
+    constexpr int NSET = SETS;
     using Sh = BulkShape<NSET>;
     constexpr int ROOM = 228 * 512 - 1024 - 320 - 2 * 4 * NSET * MT * 512 - 1024;              // what two CTAs per SM leave for a ring
     BulkParams b;
@@ -451,9 +450,8 @@ int launch(const SkinnyParams& p, int splits, cudaStream_t s) {
 
 template <int EPI>
 int dispatch(const SkinnyParams& p, int splits, int unroll, cudaStream_t s) {
-    // unroll: low four bits 0 (chosen here), 2 or 4; + 16 asks for two row sets per CTA, + 32 for four (plain epilogues)
-    const int unroll0 = unroll;
-    const bool two = EPI != 2 && (unroll & 48);
+    // unroll: low four bits 0 (chosen here), 2 or 4; + 16 asks for two row sets per CTA (plain epilogues)
+    const bool two = EPI != 2 && (unroll & 16);
     unroll &= 15;
     const int mt = ceil_div(p.M, 8);
     // Through shared memory from 1 Mi weights on ([1024, 1024] 1.8 us either way, [512, 2048] 2.5 | 3.3).  us, this form | the other, 1 row and 8:
@@ -464,9 +462,9 @@ int dispatch(const SkinnyParams& p, int splits, int unroll, cudaStream_t s) {
     const long long weights = (long long)p.N * (EPI == 2 ? 2 : 1) * p.K;
     // (A gated unit of fewer units than SMs stays with the other form: its caller has a product cut over K, with the activation behind it, for that.)
     if (mt <= 2 && p.K % 64 == 0 && weights >= (1LL << 20) && (EPI != 2 || p.N >= 8 * num_sms())) {
-        const int sets = EPI == 2 ? (p.K >= 4096 ? 1 : 2) : unroll0 & 32 ? 4 : unroll0 & 16 ? 2 : 1;
-        if (mt == 1) return sets == 4 ? launch_bulk<1, EPI, 4>(p, splits, s) : sets == 2 ? launch_bulk<1, EPI, 2>(p, splits, s) : launch_bulk<1, EPI, 1>(p, splits, s);
-        return sets == 4 ? launch_bulk<2, EPI, 4>(p, splits, s) : sets == 2 ? launch_bulk<2, EPI, 2>(p, splits, s) : launch_bulk<2, EPI, 1>(p, splits, s);
+        const bool wide = EPI == 2 ? p.K < 4096 : two;
+        if (mt == 1) return wide ? launch_bulk<1, EPI, 2>(p, splits, s) : launch_bulk<1, EPI, 1>(p, splits, s);
+        return wide ? launch_bulk<2, EPI, 2>(p, splits, s) : launch_bulk<2, EPI, 1>(p, splits, s);
     }
     // a product that is not split over CTAs streams best with deep unrolling, a split one with more CTAs per SM
     const bool deep = EPI != 2 && (unroll ? unroll >= 4 : splits == 1);
@@ -510,7 +508,7 @@ extern "C" int ttie_skinny_gemm_glu(const void* x, long long ldx, const void* w,
     return rc;
 }
 // unroll: 0 = chosen from kslice; 2 or 4 = 32-key blocks per register buffer (rows <= 8 only); + 16 = two sets of 16
-// weight rows per CTA, + 32 = four (plain epilogues; halves the 32-key blocks per buffer).
+// weight rows per CTA (plain epilogues; halves the 32-key blocks per buffer).
 extern "C" int ttie_skinny_gemm_tuned(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* out,
                                       long long ldo, int M, int N, int K, int kslice, int epilogue, int up_offset, int unroll,
                                       void* stream) {

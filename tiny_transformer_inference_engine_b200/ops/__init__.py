@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import math
 import os
 from typing import Optional
@@ -160,6 +161,30 @@ def _row_bucket(M: int) -> int:
 
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
+
+
+@functools.lru_cache(maxsize=4096)
+def _ring_form(N, K, num_sms, may_split):
+    """(K range of a CTA, form code) of the weight-streaming product through shared memory for a matrix of 4 Mi elements or more: one
+    or two sets of 16 weight rows a unit, K in 1 to 8 ranges of 768 or more where the caller takes partial sums.  By sizes and not
+    by a stopwatch: the ranges decide the order of the sums, so a choice between forms a few percent apart, made anew in every process,
+    would give other last bits from one to the next (the row sets do not).  The cost: a unit's bytes (its weights, the copies of the activations, a
+    start) times the waves of units on two CTAs an SM, the last one with the fill to the power of 0.4, since fewer CTAs get
+    more of the memory's rate each.  Fitted to 50 shapes of [1024, 4096] to [256000, 2048] at 1, 8 and 16 rows: on average 2.6 % above the
+    fastest of 18 to 27 forms, a tenth at one in twenty; at the Llama sizes, us at 1 row and 8: [4352, 4096] 7.3, 7.8 in two ranges of two sets (8.0,
+    8.5 uncut with one), [4096, 4096] 6.9, 7.7 (7.7, 8.2), [4096, 11008] 15.6, 16.3 (16.2, 16.7), [32000, 4096] uncut with one set 38.8, 39.4."""
+    best, best_cost = None, None
+    for sets in (1, 2):
+        for S in (1, 2, 3, 4, 5, 6, 8) if may_split else (1,):
+            kslice = math.ceil(math.ceil(K / S) / 128) * 128
+            if S > 1 and (K < 768 * S or math.ceil(K / kslice) != S):
+                continue
+            waves = math.ceil(N / (16 * sets)) * S / (2 * num_sms)
+            cost = (kslice * (16 * sets + 8) + 4000) * (math.floor(waves) + (waves % 1) ** 0.4)
+            if best_cost is None or cost < best_cost:
+                best, best_cost = (kslice, 16 * (sets - 1)), cost
+    return best
+
 
 
 class CudaOps:
@@ -343,10 +368,9 @@ class CudaOps:
         [2048, 16384] it leaves half of the memory bandwidth unused), and the faster one is remembered.  Up to 8 rows the
         weight-streaming product is the rule and is ahead on most shapes, by up to 3x on narrow deep ones; a shape goes to
         the library where that is more than 5 % faster (measured: [10240, 8192] and [8192, 28672] by 9-10 %).  At 8 and
-        16 rows the weight-streaming product's own form is measured too - K cut into 1 to 16 ranges over CTAs, one, two or
-        four sets of 16 weight rows per CTA - and a form that beats the rule of thumb (``_kslice``) by 3 % is kept: [4352, 4096]
-        at 8 rows takes 7.8 us in 6 ranges with two row sets against 9.1 in 8 ranges with one, [4544, 18176] 28.5 us in 6
-        ranges against 38.3 uncut.  Small matrices (under 4 Mi elements) are left alone."""
+        16 rows the weight-streaming product's own form is measured too where its weights do not come through shared memory (K no
+        multiple of 64; else ``_ring_form``) - K cut into 1 to 16 ranges over CTAs, one or two sets of 16 weight rows per CTA - and a form that
+        beats the rule of thumb (``_kslice``) by 3 % is kept.  Small matrices (under 4 Mi elements) are left alone."""
         groups, launches = {}, self.launches
         for w in weights:
             if w.dtype == torch.bfloat16 and w.dim() == 2 and w.stride(1) == 1 and w.shape[0] * w.shape[1] >= (4 << 20):
@@ -373,10 +397,10 @@ class CudaOps:
 
                 took = {"library": measure("library"), "skinny_uncut": measure("skinny", partial_ok=False), "skinny": measure("skinny")}
                 form = None
-                if M <= 16:
-                    # up to 16 rows the weight-streaming product's own form is measured as well: one, two or four sets of 16 weight
+                if M <= 16 and K % 64:
+                    # up to 16 rows the weight-streaming product's own form is measured as well: one or two sets of 16 weight
                     # rows per CTA, K cut into 1 to 16 ranges
-                    for code in (0, 16, 32):
+                    for code in (0, 16):
                         for S in (1, 2, 3, 4, 6, 8, 12, 16):
                             kslice = math.ceil(math.ceil(K / S) / 128) * 128
                             if kslice < 256 or math.ceil(K / kslice) != S:
@@ -387,7 +411,7 @@ class CudaOps:
                 self._skinny_tuned.pop((N, K, M), None)
                 if form is not None:
                     self._skinny_tuned[(N, K, M)] = form
-                    took["skinny_form"] = {"k_ranges": math.ceil(K / form[0]), "row_sets": 4 if form[1] & 32 else 2 if form[1] & 16 else 1}
+                    took["skinny_form"] = {"k_ranges": math.ceil(K / form[0]), "row_sets": 2 if form[1] & 16 else 1}
                 # callers that take partial sums of a cut K range, and callers that want the whole sum
                 self._product_choice[(N, K, M, "split")] = decide(took["skinny"], took["library"])
                 self._product_choice[(N, K, M)] = decide(took["skinny_uncut"], took["library"])
@@ -453,8 +477,11 @@ class CudaOps:
             return out
         may_split = partial_ok and bias is None and out_dtype is None
         if self._skinny_ok(x, w, may_split):
-            tuned = self._skinny_tuned.get((N, K, 8 if M <= 8 else 16)) if (may_split and M <= 16) else None
-            kslice, form = tuned if tuned is not None else (self._kslice(N, K, may_split), 0)
+            if M <= 16 and K % 64 == 0 and N * K >= 4 << 20:
+                kslice, form = _ring_form(N, K, self.num_sms, may_split)
+            else:
+                tuned = self._skinny_tuned.get((N, K, 8 if M <= 8 else 16)) if (may_split and M <= 16) else None
+                kslice, form = tuned if tuned is not None else (self._kslice(N, K, may_split), 0)
             S = math.ceil(K / kslice)
             if S > 1:
                 out, epi = torch.empty((S, M, N), dtype=torch.float32, device=x.device), 1
