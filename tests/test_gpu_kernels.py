@@ -1293,3 +1293,27 @@ def test_decode_product_is_the_same_after_its_shape_was_measured(ops):
     finally:
         ops._product_choice.clear(); ops._product_choice.update(keep[0])
         ops._skinny_tuned.clear(); ops._skinny_tuned.update(keep[1])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("n", [6, 100])
+@pytest.mark.parametrize("D", [64, 36])
+@pytest.mark.parametrize("splits", [1, 2, 4, 6, 15, 30, 60])
+def test_nan_key_reaches_the_rows_that_see_it_through_the_merge(ops, dtype, n, D, splits):
+    """A NaN among the keys makes every row that sees it NaN, with the key range whole or in pieces: no merge turns it into a zero."""
+    g = torch.Generator().manual_seed(55)
+    kv_len, H, page, dt = 3840, 2, 16, getattr(torch, dtype)
+    width = kv_len // page
+    table = (torch.randperm(width, generator=g).int() + 1).view(1, width).to(DEV)
+    kp, vp = (torch.randn(width + 1, H, page, D, generator=g).to(dt).to(DEV) for _ in range(2))
+    qkv = torch.randn(n, 3 * H * D, generator=g).to(dt).to(DEV)
+    qsl, lens = torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.tensor([kv_len], dtype=torch.int32, device=DEV)
+    for token in (0, 1400, kv_len - 3):
+        keys = kp.clone()
+        keys[int(table[0, token // page]), 0, token % page, 5] = float("nan")
+        out = torch.zeros(n, H * D, dtype=dt, device=DEV)
+        ops.paged_attention(qkv, H, H, D, keys, vp, table, page, qsl, lens, 1, n, kv_len, D ** -0.5, 0, out,
+                            plan=("simt", splits, kv_len // splits if splits > 1 else 0))
+        sees = torch.arange(n, device=DEV) + kv_len - n >= token
+        assert torch.isnan(out.view(n, H, D)[sees, 0]).all()
+        assert torch.isfinite(out.view(n, H, D)[:, 1]).all() and torch.isfinite(out.view(n, H, D)[~sees, 0]).all()

@@ -272,7 +272,9 @@ __global__ void attn_merge_kernel(const float* __restrict__ ws_o, const float* _
 
 // Up to NS <= 32 splits: every thread asks for all (max, sum) pairs of its row and for its column of every split's
 // partial output at once, so the whole merge costs one memory latency; weights are computed redundantly per thread.
-template <typename T, int NS>
+// NANS: a piece whose sum is a NaN makes the row NaN (as in the merge above and in a row that was not cut); else it counts as empty
+template <bool NANS> __device__ __forceinline__ bool has_sum(float l) { return NANS ? !(l <= 0.f) : l > 0.f; }
+template <typename T, int NS, bool NANS>
 __global__ void __launch_bounds__(128)
 attn_merge_small_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, T* __restrict__ out, int num_splits, int D) {
     TTIE_PDL_ENTRY_EARLY();
@@ -290,21 +292,22 @@ attn_merge_small_kernel(const float* __restrict__ ws_o, const float* __restrict_
     }
     float M = -INFINITY;
 #pragma unroll
-    for (int s = 0; s < NS; ++s) if (v[s].y > 0.f) M = fmaxf(M, v[s].x);
+    for (int s = 0; s < NS; ++s) if (has_sum<NANS>(v[s].y)) M = fmaxf(M, v[s].x);
     float acc = 0.f, den = 0.f;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {                               // fixed order
-        const float e = v[s].y > 0.f ? expf(v[s].x - M) : 0.f;
-        acc = fmaf(e, v[s].y > 0.f ? x[s] : 0.f, acc);
+        const bool live = has_sum<NANS>(v[s].y);
+        const float e = live ? expf(v[s].x - M) : 0.f;
+        acc = fmaf(e, live ? x[s] : 0.f, acc);
         den = fmaf(e, v[s].y, den);
     }
-    out[row * D + d] = from_f32<T>(den > 0.f ? acc / den : 0.f);
+    out[row * D + d] = from_f32<T>(has_sum<NANS>(den) ? acc / den : 0.f);
 }
 
 // The same for up to 8 splits with four columns per thread and the rows packed into blocks of 256 threads: a prompt
 // portion whose key range was cut brings thousands of rows, and one small block per row (16,384 rows x 2 splits: 24 us)
 // spends its time on block launches, not on the 21 MB it moves.  The arithmetic per element is that of the kernel above.
-template <typename T, int NS>
+template <typename T, int NS, bool NANS>
 __global__ void __launch_bounds__(256)
 attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, T* __restrict__ out,
                       long long rows, int num_splits, int D) {
@@ -325,12 +328,12 @@ attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ 
     }
     float M = -INFINITY;
 #pragma unroll
-    for (int s = 0; s < NS; ++s) if (v[s].y > 0.f) M = fmaxf(M, v[s].x);
+    for (int s = 0; s < NS; ++s) if (has_sum<NANS>(v[s].y)) M = fmaxf(M, v[s].x);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float den = 0.f;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {                               // fixed order
-        const bool live = v[s].y > 0.f;
+        const bool live = has_sum<NANS>(v[s].y);
         const float e = live ? expf(v[s].x - M) : 0.f;
         acc.x = fmaf(e, live ? x[s].x : 0.f, acc.x);
         acc.y = fmaf(e, live ? x[s].y : 0.f, acc.y);
@@ -338,7 +341,7 @@ attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ 
         acc.w = fmaf(e, live ? x[s].w : 0.f, acc.w);
         den = fmaf(e, v[s].y, den);
     }
-    const bool any = den > 0.f;
+    const bool any = has_sum<NANS>(den);
     const float4 y = any ? make_float4(acc.x / den, acc.y / den, acc.z / den, acc.w / den) : make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (sizeof(T) == 4) {
         *reinterpret_cast<float4*>(out + row * D + d) = y;
@@ -348,24 +351,24 @@ attn_merge_vec_kernel(const float* __restrict__ ws_o, const float* __restrict__ 
     }
 }
 
-template <typename T>
+template <typename T, bool NANS>
 int attn_merge(const float* ws_o, const float* ws_ml, T* out, long long rows, int num_splits, int D, cudaStream_t s) {
     const dim3 grid((unsigned)rows, ceil_div(D, 128));
     const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(ws_o) | reinterpret_cast<uintptr_t>(ws_ml)) & 15) == 0
                      && (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(T) - 1)) == 0;
     if (vec && num_splits <= 8) {
         const unsigned blocks = (unsigned)((rows * (D / 4) + 255) / 256);
-        if (num_splits <= 2) { TTIE_LAUNCH((attn_merge_vec_kernel<T, 2>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
-        else if (num_splits <= 4) { TTIE_LAUNCH((attn_merge_vec_kernel<T, 4>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
-        else { TTIE_LAUNCH((attn_merge_vec_kernel<T, 8>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
+        if (num_splits <= 2) { TTIE_LAUNCH((attn_merge_vec_kernel<T, 2, NANS>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
+        else if (num_splits <= 4) { TTIE_LAUNCH((attn_merge_vec_kernel<T, 4, NANS>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
+        else { TTIE_LAUNCH((attn_merge_vec_kernel<T, 8, NANS>), blocks, 256, 0, s, ws_o, ws_ml, out, rows, num_splits, D); }
     } else if (num_splits <= 4) {
-        TTIE_LAUNCH((attn_merge_small_kernel<T, 4>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 4, NANS>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
     } else if (num_splits <= 8) {
-        TTIE_LAUNCH((attn_merge_small_kernel<T, 8>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 8, NANS>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
     } else if (num_splits <= 16) {
-        TTIE_LAUNCH((attn_merge_small_kernel<T, 16>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 16, NANS>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
     } else if (num_splits <= 32) {
-        TTIE_LAUNCH((attn_merge_small_kernel<T, 32>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
+        TTIE_LAUNCH((attn_merge_small_kernel<T, 32, NANS>), grid, 128, 0, s, ws_o, ws_ml, out, num_splits, D);
     } else {
         TTIE_LAUNCH(attn_merge_kernel<T>, (unsigned)rows, MERGE_GROUPS * (D >= 128 ? 128 : 64), (num_splits + MERGE_GROUPS * D) * sizeof(float), s,
                     ws_o, ws_ml, out, num_splits, D);
@@ -584,13 +587,13 @@ int launch_f32_tile(AttnParams p, int T_tokens, int max_q_len, cudaStream_t s) {
     TTIE_LAUNCH(paged_attn_f32_tile_kernel<DP>, dim3(p.num_seqs * p.Hkv * p.row_tiles, p.num_splits), FT_THREADS,
                 spread ? SPREAD : tile_smem<DP>(), s, p);
     TTIE_CHECK_LAUNCH("paged_attention (float32 tiles)");
-    return p.num_splits > 1 ? attn_merge(p.ws_o, p.ws_ml, (float*)p.out, (long long)T_tokens * p.Hq, p.num_splits, p.D, s) : 0;
+    return p.num_splits > 1 ? attn_merge<float, true>(p.ws_o, p.ws_ml, (float*)p.out, (long long)T_tokens * p.Hq, p.num_splits, p.D, s) : 0;
 }
 }  // namespace
 
 namespace ttie {
 int attn_merge_bf16(const float* ws_o, const float* ws_ml, void* out, int rows, int num_splits, int D, cudaStream_t s) {
-    return attn_merge(ws_o, ws_ml, (__nv_bfloat16*)out, rows, num_splits, D, s);
+    return attn_merge<__nv_bfloat16, false>(ws_o, ws_ml, (__nv_bfloat16*)out, rows, num_splits, D, s);
 }
 }  // namespace ttie
 
@@ -603,7 +606,7 @@ int launch(const AttnParams& p, int T_tokens, cudaStream_t s) {
     dim3 grid(p.num_seqs * p.Hkv * p.row_tiles, p.num_splits);
     k<<<grid, WARPS * 32, smem, s>>>(p);
     TTIE_CHECK_LAUNCH("paged_attention");
-    return p.num_splits > 1 ? attn_merge(p.ws_o, p.ws_ml, (T*)p.out, (long long)T_tokens * p.Hq, p.num_splits, p.D, s) : 0;
+    return p.num_splits > 1 ? attn_merge<T, true>(p.ws_o, p.ws_ml, (T*)p.out, (long long)T_tokens * p.Hq, p.num_splits, p.D, s) : 0;
 }
 
 template <typename T>
