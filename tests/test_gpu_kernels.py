@@ -1317,3 +1317,36 @@ def test_nan_key_reaches_the_rows_that_see_it_through_the_merge(ops, dtype, n, D
         sees = torch.arange(n, device=DEV) + kv_len - n >= token
         assert torch.isnan(out.view(n, H, D)[sees, 0]).all()
         assert torch.isfinite(out.view(n, H, D)[:, 1]).all() and torch.isfinite(out.view(n, H, D)[~sees, 0]).all()
+
+
+@pytest.mark.parametrize("Hq,Hkv,D", [(4, 4, 64), (4, 1, 128), (3, 1, 36)])
+@pytest.mark.parametrize("opts", [{}, {"window": 40}, {"weights": "sigmoid"}])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_float32_tiles_rows_do_not_meet_values_they_must_not_see(ops, Hq, Hkv, D, opts, splits):
+    """An infinite or NaN key or value reaches the rows that see its token and no others: those are the same to the last bit as without it."""
+    g = torch.Generator().manual_seed(54)
+    n, page, window = 300, 16, opts.get("window", 0)
+    width = -(-n // page)
+    table = (torch.randperm(width, generator=g).int() + 1).view(1, width).to(DEV)
+    kp, vp = (torch.randn(width + 1, Hkv, page, D, generator=g).to(DEV) for _ in range(2))
+    qkv = torch.randn(n, (Hq + 2 * Hkv) * D, generator=g).to(DEV)
+    qsl, lens = torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.tensor([n], dtype=torch.int32, device=DEV)
+    plan = ("simt", 1, 0) if splits == 1 else ("simt", splits, 128)
+
+    def run():
+        out = torch.full((n, Hq * D), float("nan"), device=DEV)
+        ops.paged_attention(qkv, Hq, Hkv, D, kp, vp, table, page, qsl, lens, 1, n, n, D ** -0.5, window, out, plan=plan,
+                            **{k: v for k, v in opts.items() if k != "window"})
+        return out
+    clean = run()
+    for pages, value in ((vp, float("inf")), (vp, float("nan")), (kp, float("nan"))):
+        for token in (70, 129, 255):
+            at = (int(table[0, token // page]), 0, token % page, 3)
+            kept = pages[at].clone()
+            pages[at] = value
+            got = run()
+            pages[at] = kept
+            sees = torch.zeros(n, dtype=torch.bool, device=DEV)
+            sees[token:token + window if window else n] = True
+            assert torch.equal(got[~sees], clean[~sees]), (value, token)
+            assert not torch.isfinite(got[sees].view(-1, Hq, D)[:, :Hq // Hkv]).all(-1).any(), (value, token)

@@ -382,8 +382,8 @@ int attn_merge(const float* ws_o, const float* ws_ml, T* out, long long rows, in
 // scores (8 loads of 16 bytes for 64 multiply-adds) and 4 rows x 8 (4) columns of the output (12 (8) loads for 128 (64)); the 16 threads of
 // a row are half a warp, so a row's weights pass through shared memory without a block barrier.  Bound by the loads from shared
 // memory: a tile step of head size 128 takes an SM 10.3 us with two CTAs side by side (113 KB each) and 11.2 with one; 4.3 us of it
-// are multiply-adds.  Before and now, 16 heads on one kv head of 128: 300 tokens 85 -> 32 us, 600: 183 -> 70, 2,048: 1,372 -> 583, 128
-// behind 4,096 keys: 330 -> 144; 8 heads of 64, 300 tokens: 31 -> 17.  Measured and left out: 8 rows a thread with half the threads
+// are multiply-adds.  Before and now, 16 heads on one kv head of 128: 300 tokens 85 -> 32 us, 600: 183 -> 68, 2,048: 1,372 -> 571, 128
+// behind 4,096 keys: 330 -> 144; 8 heads of 64, 300 tokens: 31 -> 17.  (At head size 128 the 128 registers of two CTAs an SM leave 20 bytes a thread spilled.)  Measured and left out: 8 rows a thread with half the threads
 // (660 us at 2,048 tokens: too few warps), tiles by cp.async beside the computation (630), one CTA an SM at all sizes (671).
 constexpr int FT_ROWS = 64, FT_KEYS = 64, FT_R = 4, FT_THREADS = FT_ROWS / FT_R * 16;
 template <int DP> constexpr size_t tile_smem() { return sizeof(float) * ((size_t)FT_ROWS * DP + (size_t)FT_KEYS * (DP + 4) + (size_t)FT_KEYS * DP + FT_ROWS * FT_KEYS); }
@@ -440,6 +440,7 @@ __global__ void __launch_bounds__(FT_THREADS, 2) paged_attn_f32_tile_kernel(cons
         // a thread's pieces are the same columns of keys STEP apart; eight loads are on their way together
         constexpr int STEP = FT_THREADS / D4, BATCH = FT_KEYS / STEP < 8 ? FT_KEYS / STEP : 8;
         const int d = tid % D4 * 4, nk = min(FT_KEYS, v_hi - vt);
+        float odd = 0.f;
 #pragma unroll
         for (int j0 = tid / D4; j0 < FT_KEYS; j0 += BATCH * STEP) {
             size_t src[BATCH];
@@ -460,9 +461,12 @@ __global__ void __launch_bounds__(FT_THREADS, 2) paged_attn_f32_tile_kernel(cons
 #pragma unroll
             for (int i = 0; i < BATCH; ++i) x[i] = in[i] ? load4(vp + src[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < BATCH; ++i) *reinterpret_cast<float4*>(Vs + (j0 + i * STEP) * DP + d) = x[i];
+            for (int i = 0; i < BATCH; ++i) {
+                *reinterpret_cast<float4*>(Vs + (j0 + i * STEP) * DP + d) = x[i];
+                odd = fmaf(x[i].x, 0.f, fmaf(x[i].y, 0.f, fmaf(x[i].z, 0.f, fmaf(x[i].w, 0.f, odd))));
+            }
         }
-        __syncthreads();
+        const bool careful = __syncthreads_or(!(odd == 0.f));        // (a value of the tile is not finite)
 
         float s[FT_R][4];
 #pragma unroll
@@ -504,14 +508,14 @@ __global__ void __launch_bounds__(FT_THREADS, 2) paged_attn_f32_tile_kernel(cons
             if (p.sigmoid) {
                 const float hb = p.head_bias && pos[i] >= 0 ? p.head_bias[kvh * G + (row0 + ty * FT_R + i) % G] : 0.f;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = vis[j] ? 1.0f / (1.0f + expf(-(s[i][j] + hb))) : 0.f;
+                for (int j = 0; j < 4; ++j) s[i][j] = vis[j] ? 1.0f / (1.0f + expf(-(s[i][j] + hb))) : -0.f;
             } else {
 #pragma unroll
                 for (int k = 1; k < 16; k <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, k));
                 const float m_new = fmaxf(m[i], top);
                 const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { s[i][j] = vis[j] ? expf(s[i][j] - m_new) : 0.f; sum += s[i][j]; }
+                for (int j = 0; j < 4; ++j) { s[i][j] = vis[j] ? expf(s[i][j] - m_new) : -0.f; sum += s[i][j]; }
 #pragma unroll
                 for (int k = 1; k < 16; k <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
                 l[i] = l[i] * alpha + sum;
@@ -523,24 +527,31 @@ __global__ void __launch_bounds__(FT_THREADS, 2) paged_attn_f32_tile_kernel(cons
             for (int j = 0; j < 4; ++j) Ps[(ty * FT_R + i) * FT_KEYS + tx + 16 * j] = s[i][j];
         }
         __syncwarp();                                                // (a row's weights come from and go to one half of this warp)
+        // (a key that a row must not see has the weight -0, which a visible one never has: it is left out where a value may not be finite, since
+        // 0 times that is a NaN)
+        auto weigh = [&](auto care) {
 #pragma unroll 2
-        for (int j = 0; j < nk; j += 4) {                            // (past the last key: weights of zero, values of zero)
-            float4 w[FT_R];
+            for (int j = 0; j < nk; j += 4) {                        // (past the last key: weights of zero, values of zero)
+                float4 w[FT_R];
 #pragma unroll
-            for (int i = 0; i < FT_R; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (ty * FT_R + i) * FT_KEYS + j);
+                for (int i = 0; i < FT_R; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (ty * FT_R + i) * FT_KEYS + j);
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
+                for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const float4 v = *reinterpret_cast<const float4*>(Vs + (j + jj) * DP + tx * 4 + 64 * c);
+                    for (int c = 0; c < NC; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(Vs + (j + jj) * DP + tx * 4 + 64 * c);
 #pragma unroll
-                    for (int i = 0; i < FT_R; ++i) {
-                        const float a = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
-                        o[i][4 * c] = fmaf(a, v.x, o[i][4 * c]); o[i][4 * c + 1] = fmaf(a, v.y, o[i][4 * c + 1]);
-                        o[i][4 * c + 2] = fmaf(a, v.z, o[i][4 * c + 2]); o[i][4 * c + 3] = fmaf(a, v.w, o[i][4 * c + 3]);
+                        for (int i = 0; i < FT_R; ++i) {
+                            const float a = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
+                            if (decltype(care)::value && __float_as_uint(a) == 0x80000000u) continue;
+                            o[i][4 * c] = fmaf(a, v.x, o[i][4 * c]); o[i][4 * c + 1] = fmaf(a, v.y, o[i][4 * c + 1]);
+                            o[i][4 * c + 2] = fmaf(a, v.z, o[i][4 * c + 2]); o[i][4 * c + 3] = fmaf(a, v.w, o[i][4 * c + 3]);
+                        }
                     }
-                }
-        }
+            }
+        };
+        if (careful) weigh(std::true_type{});
+        else weigh(std::false_type{});
         __syncwarp();
     }
 #pragma unroll
