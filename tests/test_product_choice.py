@@ -133,3 +133,11 @@ def test_form_of_a_decode_product_comes_from_its_sizes(N, K):
     assert _ring_form(N, K, 148, True)[0] == kslice
     if N <= 4352 and K >= 4096:
         assert S >= 2
+
+
+@pytest.mark.parametrize("mode,lens,heads,tokens", [
+    (RETENTION, [2048], 16, 128), (MLSTM, [2048] * 4, 64, 128), (RETENTION, [128] * 16, 16, 128),            # full chunks, however many
+    (RETENTION, [1] * 31 + [2000], 16, 64), (MLSTM, [1] * 15 + [512], 32, 64), (MLSTM, [64] * 32, 16, 64),   # short chunks, more of them and heads than run at once
+    (RETENTION, [1] * 7 + [512], 16, 128), (MLSTM, [1] * 15 + [512], 8, 128), (RETENTION, [64] * 8, 16, 128)])   # ... and fewer
+def test_tokens_of_a_chunk_by_what_runs_at_once(mode, lens, heads, tokens):
+    assert CudaOps._chunk_tokens(mode, torch.bfloat16, sum(lens), len(lens), 128, 128, heads, 148) == tokens

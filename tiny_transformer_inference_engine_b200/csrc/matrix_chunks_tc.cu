@@ -1,22 +1,23 @@
 // The chunked matrix-state recurrences of matrix_chunks.cu (retention, the xLSTM matrix memory) with their products on the 5th-generation tensor
 // cores, in chunks of 128 tokens: bfloat16 values of at most 128 columns and at most 128 key channels.
 //
-// The arithmetic is that of matrix_chunks.cu: 32-bit operands as three bfloat16, six plane products for a product of two of them.  What differs is
-// where the sums lie: a CTA of 512 threads owns a (chunk, head), an instruction multiplies 128 rows by up to 128 columns from
-// shared memory (the weights of the scores: from tensor memory, where the threads that computed them leave them), and its sums are in tensor
-// memory, a thread per row and half of the columns.  The tensor cores cut bits off where an addition rounds: so every sum there spans 64 terms (32 in
-// the chunks' own sums) with the large plane products last, and the spans are added by ordinary additions.
+// The arithmetic is that of matrix_chunks.cu: 32-bit operands as three bfloat16, six plane products for a product of two of them, differences of the
+// gates' sums in 64 bits (as two floats).  What differs is where the sums lie: a CTA of 512 threads owns a (chunk, head), an instruction multiplies
+// 128 rows by up to 128 columns from shared memory, and its sums are in tensor memory, a thread per row and quarter of the columns.  They come
+// out in rounds (below): 16 terms of the leading planes at a time.
 //
-//   chunk_sum_tc   D[value column][channel] = V^T K', both operands as they lie (token by row); four spans of 32 tokens
-//   chunk_out_tc   S = Q K^T, then O = Q (state)^T while the threads weigh the scores, then the weights times V; spans of 64 channels and tokens
+//   chunk_sum_tc   D[value column][channel] = V^T K', both operands as they lie (token by row); what rounding the rounds' sum leaves is kept
+//   chunk_out_tc   S = Q K^T, then O = Q (state)^T while the threads weigh the scores, then the weights, in the place of queries and state, times V
 //
-// One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 14 + 6 + 30 (27 + 9 + 64 in chunks of 64), 16 of 64 x 128 12 + 6 + 25
-// (13 + 11 + 40).  A CTA of the out kernel takes some 21,000 clocks, one after the other (one fits an SM: six planes of 32 KB): 6,000 for the rows
-// of q and k, as fast as the L2 gives them to all SMs, 3,400 + 3,300 + 1,600 for the products, whose two operands come
-// from shared memory at its bandwidth (73 clocks a product, 64 at the tensor cores' rate), 2,000 for splitting the state and the weights, 2,500 for the
-// stores; 256 of them on 148 SMs are two rounds.  With 256 threads, a half row each, it took 31,000 (conversions and divisions wait for issue slots).
-// Error against 64 bits (1,000 tokens, chunks of 64 and the walk behind it): read-out 0.97e-7 (1.0e-7, 2.4e-7), state 5.3e-8 (5.2e-8, 1.7e-7); read-out
-// without CUT64 1.5e-7.
+// One prompt of 2,048 tokens, us of the scan (in chunks of 64): 16 heads of 128 x 128 retention 59 (95), mlstm 65 (100), 16 of 64 x 128 40 (54)
+// and 48 (65).  One CTA of the out kernel fits an SM (six planes of 32 KB), its phases run one after the other, and 256 of them on 148 SMs are
+// two turns.  With sums of 64 terms (32 in chunk_sum_tc) in one place the four took 51, 58, 34 and 43, but then the tensor cores cut off 6.7e-8 (2.3e-8)
+// of each sum.  Chunk_out_tc spills 40 bytes a thread (mlstm, 128 channels) for its rows' weights and read-outs.  Tried and slower: rounds left out
+// for tokens that are not there (the thread that issues the products then computes their addresses: 69 us for the 59), no sums for keys that
+// no row of a warp sees (63: 300 bytes spilled).
+// Error against 64 bits (mean of six inputs, 700 tokens, normal values; chunks of 64 and the walk behind it): retention of 128 x 128 read-out 8.8e-8
+// (9.3e-8, 14.8e-8), state 4.0e-8 (4.4e-8, 8.7e-8); mlstm of 64 x 128 7.1e-7 (7.8e-7, 14.9e-7), 1.80e-7 (1.80e-7, 5.3e-7).  Values of one sign: 5.4e-8
+// (5.0e-8, 4.1e-8), 4.2e-8 (4.1e-8, 11.8e-8).
 //
 // Every mbarrier wait is bounded by a clock deadline; one that runs out records a code and the CTA goes on to its end.
 #include "matrix_chunks.cuh"
@@ -29,9 +30,7 @@ namespace ttie { int gemm_tc_error_words(int** word, int** mirror); }
 namespace {
 constexpr int CT = 128, NT = 512, DVP = 128, GROUPS = NT / 128;   // tokens of a chunk, threads, value columns (zeros behind Dv), threads of a row
 constexpr int OWN = 128 / GROUPS;                                // columns of a thread
-// What cutting instead of rounding leaves: a sum of 64 terms of one sign-independent size comes out 6.7e-8 of itself too small on average, one of 32
-// 2.3e-8 (measured against 64 bits), the same for every sum, so it is put back.
-constexpr float CUT64 = 6.7e-8f, CUT32 = 2.3e-8f;
+constexpr int SLOTS = 4;                                         // sums of a round in tensor memory
 constexpr long long WAIT_CYCLES = 2000000000LL;                 // about one second
 constexpr uint32_t BLOCK = CT * 128;                             // 128 rows of 64 bfloat16, 128-byte swizzle
 
@@ -39,6 +38,12 @@ constexpr uint32_t BLOCK = CT * 128;                             // 128 rows of 
 __device__ __forceinline__ float2 two_floats(double x) {
     const float hi = (float)x;
     return make_float2(hi, isinf(hi) ? 0.f : (float)(x - (double)hi));
+}
+// e^d for d in 64 bits: what rounding d to 32 bits leaves counts too
+__device__ __forceinline__ float exp_of(double d) {
+    const float2 f = two_floats(d);
+    const float e = expf(f.x);
+    return fmaf(e, f.y, e);
 }
 struct ErrorWords { int* word; int* mirror; };
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -79,11 +84,6 @@ __device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
                  ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 db, {%2, %3};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-                 ::"r"(d), "r"(a), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(accumulate) : "memory");
-}
 // D float32, A and B bfloat16; M 128, N columns; which operands have K down the rows
 __host__ __device__ constexpr uint32_t idesc_of(int n, bool a_cols, bool b_cols) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (a_cols ? 1u << 15 : 0u) | (b_cols ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -100,30 +100,50 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {     // (the va
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
                    "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
 }
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-// sixteen columns of SPANS sums, `step` columns apart, added, with what their cut additions lost on average
-template <int SPANS>
-__device__ __forceinline__ void tmem_sum16(uint32_t taddr, int step, float (&o)[16]) {
-    uint32_t v[SPANS][16];
-#pragma unroll
-    for (int s = 0; s < SPANS; ++s) tmem_ld16(taddr + s * step, v[s]);
-#pragma unroll
-    for (int s = 0; s < SPANS; ++s) tmem_ld_wait(v[s]);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        if constexpr (SPANS == 1) {
-            const float t = __uint_as_float(v[0][i]);
-            o[i] = fmaf(t, CUT64, t);
-        } else {                                                     // (with what the last addition rounds off: the correction is about half a unit)
-            float x = __uint_as_float(v[0][i]), y = __uint_as_float(v[1][i]);
-            if constexpr (SPANS == 4) { x += y; y = __uint_as_float(v[2][i]) + __uint_as_float(v[3][i]); }
-            const float t = x + y, u = t - x;
-            o[i] = t + fmaf(t, SPANS == 4 ? CUT32 : CUT64, (x - (t - u)) + (y - u));
-        }
+// A product of two operands of which one has, or both have, three planes, in rounds.  The tensor cores cut bits off where an addition rounds, so the
+// leading planes' products - 16 bits each, 16 of them all but exact together - are summed 16 terms at a time, each 16 from zero in a
+// slot of their own, and the small planes' products (at most 2^-8 of those) all in the last slot.  The slots are added in
+// registers by ordinary additions.  A round is up to three 16 terms (four without small planes) and a share of the small products, which
+// keep the tensor cores busy while the threads add.
+template <int TERMS, bool SMALL> struct Rounds {
+    static constexpr int PER = SMALL ? SLOTS - 1 : SLOTS, N = (TERMS + PER - 1) / PER, BARS = N + (SMALL ? 1 : 0);
+};
+// large(d, i): terms 16 i .. 16 i + 15 of the leading planes into columns d; small(d, i): the i-th of n_small small products, which adds to d unless i is 0
+template <int TERMS, bool SMALL, typename Large, typename Small>
+__device__ __forceinline__ void issue_round(int r, uint32_t d, int step, uint32_t bar, int n_small, Large large, Small small) {
+    using R = Rounds<TERMS, SMALL>;
+    for (int i = 0; i < R::PER; ++i)
+        if (r * R::PER + i < TERMS) large(d + i * step, r * R::PER + i);
+    umma_commit(bar + 8 * r);
+    if constexpr (SMALL) {
+        for (int i = n_small * r / R::N; i < n_small * (r + 1) / R::N; ++i) small(d + (SLOTS - 1) * step, i);
+        if (r == R::N - 1) umma_commit(bar + 8 * R::N);
     }
+}
+// 16 columns of this thread's row, added
+__device__ __forceinline__ void add_slot(uint32_t d, float (&acc)[16]) {
+    uint32_t v[16];
+    tmem_ld16(d, v);
+    tmem_ld_wait(v);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc[c] += __uint_as_float(v[c]);
+}
+// this thread's row of a round: 16 columns from `d` on of each slot, added to one another and then to acc (fewer roundings of the large sum)
+template <int TERMS, bool SMALL>
+__device__ __forceinline__ void add_round(int r, uint32_t d, int step, float (&acc)[16]) {
+    using R = Rounds<TERMS, SMALL>;
+    const int n = min(R::PER, TERMS - r * R::PER);
+    uint32_t v[16];
+    tmem_ld16(d, v);
+    tmem_ld_wait(v);
+    float t[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) t[c] = __uint_as_float(v[c]);
+#pragma unroll
+    for (int i = 1; i < R::PER; ++i)
+        if (i < n) add_slot(d + i * step, t);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc[c] += t[c];
 }
 // byte offset of eight values (columns c .. c + 7) of row j in an operand's plane
 __device__ __forceinline__ uint32_t piece_at(int j, int c) { return (uint32_t)(c >> 6) * BLOCK + (uint32_t)j * 128 + (uint32_t)((((c >> 3) & 7) ^ (j & 7)) << 4); }
@@ -207,7 +227,7 @@ __device__ __forceinline__ void tc_free(uint32_t tmem, uint32_t cols) {
 
 // ------------------------------------------------------------------------------------------- chunk_sum
 template <int KP> struct SumTc {
-    static constexpr uint32_t PLANE = KP / 64 * BLOCK, COLS = 4 * KP;
+    static constexpr uint32_t PLANE = KP / 64 * BLOCK, COLS = SLOTS * KP;
     static constexpr size_t bytes = 3 * PLANE + DVP / 64 * BLOCK + 1024;
 };
 
@@ -217,7 +237,8 @@ __global__ void __launch_bounds__(NT, KP == 64 ? 2 : 1) chunk_sum_tc_kernel(cons
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* kd = align1024(smem_dyn);                         // [3] planes of decayed keys
     unsigned char* v_s = kd + 3 * PLANE;
-    __shared__ __align__(8) unsigned long long bars[1];
+    using R = Rounds<CT / 16, true>;
+    __shared__ __align__(8) unsigned long long bars[R::BARS];
     __shared__ uint32_t slot;
     __shared__ double ends[2 * CT / 32 + 2];
     __shared__ float wt[CT], norm_part[NT];
@@ -232,7 +253,7 @@ __global__ void __launch_bounds__(NT, KP == 64 ? 2 : 1) chunk_sum_tc_kernel(cons
     } else {
         double F, x, X;
         chunk_gates<CT>(a, t0, n, h, ends, F, x, X);
-        if (tid < CT) wt[tid] = expf((float)(x - ends[2 * CT / 32 + 1]));
+        if (tid < CT) wt[tid] = exp_of(x - ends[2 * CT / 32 + 1]);
         if (tid == 0) a.span[unit] = make_double2(ends[2 * CT / 32], ends[2 * CT / 32 + 1]);
     }
     __syncthreads();
@@ -243,20 +264,15 @@ __global__ void __launch_bounds__(NT, KP == 64 ? 2 : 1) chunk_sum_tc_kernel(cons
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = j < n ? x[i] * w : 0.f;
     });
-    tc_setup<1>(bars, &slot, COLS);
-    const uint32_t tmem = slot, bar = smem_u32(bars);
-    if (tid == 0) {
+    tc_setup<R::BARS>(bars, &slot, COLS);
+    const uint32_t tmem = slot, bar = smem_u32(bars), va = smem_u32(v_s), ka = smem_u32(kd);
+    auto issue = [&](int r) {
         constexpr uint32_t idesc = idesc_of(KP, true, true);
-        const uint32_t va = smem_u32(v_s), ka = smem_u32(kd);
-#pragma unroll
-        for (int sp = 0; sp < 4; ++sp)
-#pragma unroll
-            for (int l = 2; l >= 0; --l)
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks)
-                    umma_ss(tmem + sp * KP, desc_cols(va, sp * 2 + ks), desc_cols(ka + l * PLANE, sp * 2 + ks), idesc, l != 2 || ks != 0);
-        umma_commit(bar);
-    }
+        issue_round<CT / 16, true>(r, tmem, KP, bar, 2 * (CT / 16),
+            [&](uint32_t d, int i) { umma_ss(d, desc_cols(va, i), desc_cols(ka, i), idesc, 0); },
+            [&](uint32_t d, int i) { umma_ss(d, desc_cols(va, i & 7), desc_cols(ka + (i < 8 ? 2 : 1) * PLANE, i & 7), idesc, i > 0); });
+    };
+    if (tid == 0) issue(0);
     __syncwarp();
     if constexpr (MODE == MLSTM) {                                   // the normaliser's sum: the same without the values
         constexpr int PARTS = NT / KP;
@@ -276,19 +292,48 @@ __global__ void __launch_bounds__(NT, KP == 64 ? 2 : 1) chunk_sum_tc_kernel(cons
             a.aux[unit * a.Dpad + tid] = t;
         }
     }
-    mbar_wait(bar, 51, err);
+    constexpr int OWN_K = KP / GROUPS;                               // columns of a thread
+    const int row = quarter * 32 + lane;
+    const uint32_t mine = tmem + ((uint32_t)(quarter * 32) << 16) + group * OWN_K;
+    float o[OWN_K / 16][16], left[OWN_K / 16][16];                   // left: what rounding the sums leaves
+#pragma unroll
+    for (int g = 0; g < OWN_K / 16; ++g)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[g][i] = left[g][i] = 0.f;
+#pragma unroll
+    for (int r = 0; r < R::N; ++r) {
+        mbar_wait(bar + 8 * r, 51, err);
+#pragma unroll
+        for (int g = 0; g < OWN_K / 16; ++g) {
+            float v[16] = {};
+            add_round<CT / 16, true>(r, mine + g * 16, KP, v);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                const float t = o[g][c] + v[c], u = t - o[g][c];
+                if (r > 0) left[g][c] += (o[g][c] - (t - u)) + (v[c] - u);
+                o[g][c] = t;
+            }
+        }
+        if (r + 1 < R::N) {
+            sync_tc();
+            if (tid == 0) issue(r + 1);
+            __syncwarp();
+        }
+    }
+    mbar_wait(bar + 8 * R::N, 51, err);
+#pragma unroll
+    for (int g = 0; g < OWN_K / 16; ++g) {
+        add_slot(mine + (SLOTS - 1) * KP + g * 16, left[g]);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) o[g][c] += left[g][c];
+    }
     __syncthreads();                                                 // (the keys have been read, by the normaliser too: the sums take their place on their way out)
     constexpr int LD = KP + 4;
     float* tile = reinterpret_cast<float*>(kd);
-    const int row = quarter * 32 + lane;
 #pragma unroll
-    for (int g = 0; g < KP / 16 / GROUPS; ++g) {
-        const int col = group * (KP / GROUPS) + g * 16;
-        float o[16];
-        tmem_sum16<4>(tmem + ((uint32_t)(quarter * 32) << 16) + col, KP, o);
+    for (int g = 0; g < OWN_K / 16; ++g)
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(tile + row * LD + col + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-    }
+        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(tile + row * LD + group * OWN_K + g * 16 + i) = make_float4(o[g][i], o[g][i + 1], o[g][i + 2], o[g][i + 3]);
     tc_free(tmem, COLS);
     copy_tile<LD>(a.part + unit * a.Dv * a.Dpad, a.Dpad, tile, a.Dv, a.Dpad);
 }
@@ -297,20 +342,26 @@ __global__ void __launch_bounds__(NT, KP == 64 ? 2 : 1) chunk_sum_tc_kernel(cons
 template <int MODE, int KP> struct OutTc {
     static constexpr int QPL = MODE == MLSTM ? 1 : 3;
     static constexpr uint32_t PLANE = KP / 64 * BLOCK, COLS = 512;
-    static constexpr size_t bytes = (QPL + 3) * PLANE + DVP / 64 * BLOCK + 1024;
-    static_assert((QPL + 3) * PLANE + DVP / 64 * BLOCK >= CT * (DVP + 4) * 4, "the operands' place takes the output tile");
+    static constexpr uint32_t W_PLANE = CT / 64 * BLOCK;             // of the weights, which take the place of the queries and the state
+    static constexpr uint32_t OPERANDS = (QPL + 3) * PLANE > 3 * W_PLANE ? (QPL + 3) * PLANE : 3 * W_PLANE;
+    static constexpr size_t bytes = OPERANDS + DVP / 64 * BLOCK + 1024;
+    static_assert(OPERANDS >= CT * (DVP + 4) * 4, "the operands' place takes the output tile");
+    // rounds of the scores, of the read-out of the state, of weights times values
+    using Scores = Rounds<KP / 16, QPL == 3>;
+    using State = Rounds<KP / 16, true>;
+    using Values = Rounds<CT / 16, true>;
 };
 
 template <int MODE, int KP>
 __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, const ErrorWords err) {
-    constexpr int QPL = OutTc<MODE, KP>::QPL, SPANS = KP / 64;
-    constexpr uint32_t PLANE = OutTc<MODE, KP>::PLANE, COLS = OutTc<MODE, KP>::COLS;
-    constexpr uint32_t S_COL = 0, P_COL = 0, O_COL = 256;            // scores, then (over them) three planes of weights; read-outs
+    using Tc = OutTc<MODE, KP>;
+    constexpr int QPL = Tc::QPL, TERMS = KP / 16;
+    constexpr uint32_t PLANE = Tc::PLANE, W_PLANE = Tc::W_PLANE, COLS = Tc::COLS, SLOT = 128;
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* q_s = align1024(smem_dyn);                        // [QPL] planes of the queries
     unsigned char* k_s = q_s + QPL * PLANE;                          // [QPL] planes of the keys, then [3] of the state
-    unsigned char* v_s = k_s + 3 * PLANE;
-    __shared__ __align__(8) unsigned long long bars[3];
+    unsigned char* v_s = q_s + Tc::OPERANDS;
+    __shared__ __align__(8) unsigned long long bars[Tc::Scores::BARS + Tc::State::BARS + Tc::Values::BARS];
     __shared__ uint32_t slot;
     __shared__ double ends[2 * CT / 32 + 2], Ms[MODE == MLSTM ? CT : 1];
     __shared__ __align__(16) float2 xs[MODE == MLSTM ? CT : 1];      // mlstm: x of a token, the sum of two floats
@@ -337,38 +388,43 @@ __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, 
         chunk_gates<CT>(a, t0, n, h, ends, F, x, X);
         const float2 mm = a.mm[unit];
         const double m = (double)mm.x;
-        if (tid < CT) { xs[tid] = two_floats(x); Ms[tid] = fmax(m, X); den_s[0][tid] = expf((float)-(F + fmax(m, X))); }
+        if (tid < CT) { xs[tid] = tid < n ? two_floats(x) : make_float2(-3e38f, 0.f); Ms[tid] = fmax(m, X); den_s[0][tid] = exp_of(-(F + fmax(m, X))); }
         if (tid < KP) nb[tid] = tid < a.Dpad ? a.aux[unit * a.Dpad + tid] : 0.f;
         // (a chunk is the request's last of this pass if the next chunk is not there or not in the pass)
         if (tid == 0 && ((c + 1) * CT >= a.qsl[s + 1] - a.qsl[s] || (int)blockIdx.x + 1 == a.slots))
             a.mx[(size_t)state_row(a.slot_ids[s], a.state_rows) * a.H + h] = mm.y;
         __syncthreads();
-        row_in = expf((float)(m - Ms[row]));
+        row_in = exp_of(m - Ms[row]);
         floor_ = den_s[0][row];
     }
     stage_plain<DVP>(v_s, reinterpret_cast<const __nv_bfloat16*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv, a.ld_v, n, a.Dv);
-    tc_setup<3>(bars, &slot, COLS);
+    tc_setup<Tc::Scores::BARS + Tc::State::BARS + Tc::Values::BARS>(bars, &slot, COLS);
     if constexpr (MODE == RET) row_in = pw[row + 1];
-    const uint32_t tmem = slot, bar = smem_u32(bars), mine = tmem + ((uint32_t)(quarter * 32) << 16);
+    const uint32_t tmem = slot, mine = tmem + ((uint32_t)(quarter * 32) << 16) + group * OWN;
+    const uint32_t bar_s = smem_u32(bars), bar_o = bar_s + 8 * Tc::Scores::BARS, bar_v = bar_o + 8 * Tc::State::BARS;
     const uint32_t qa = smem_u32(q_s), ka = smem_u32(k_s), va = smem_u32(v_s);
-    // products of QPL planes of one operand and BPL of the other that matter at 32 bits, the smallest first, over a span of 64 channels
-    auto products = [&](uint32_t d, uint32_t b_base, int bpl, int sp) {
-        bool first = true;
-        for (int sum = QPL == 3 || bpl == 3 ? 2 : 0; sum >= 0; --sum)
-            for (int i = 0; i < QPL; ++i) {
-                const int j = sum - i;
-                if (j < 0 || j >= bpl) continue;
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    umma_ss(d, desc_rows(qa + i * PLANE, sp * 4 + ks), desc_rows(b_base + j * PLANE, sp * 4 + ks), idesc_of(128, false, false), !(first && ks == 0));
-                }
-                first = false;
-            }
+    // queries times BPL planes of keys or state: the products of planes that matter at 32 bits, the smallest first
+    auto issue_rows = [&](auto planes, int r, uint32_t bar) {
+        constexpr int BPL = decltype(planes)::value;
+        constexpr bool SMALL = QPL + BPL > 2;
+        constexpr uint32_t idesc = idesc_of(128, false, false);
+        issue_round<TERMS, SMALL>(r, tmem, SLOT, bar, (QPL == 3 && BPL == 3 ? 5 : 2) * TERMS,
+            [&](uint32_t d, int i) { umma_ss(d, desc_rows(qa, i), desc_rows(ka, i), idesc, 0); },
+            [&](uint32_t d, int i) {
+                const int pair = i / TERMS, ks = i % TERMS;
+                const int bp = QPL == 1 ? 2 - pair : pair == 0 ? 2 : pair == 1 || pair == 3 ? 1 : 0;                      // 2 1 0 1 0 of the second operand beside
+                const int qp = QPL == 1 ? 0 : pair == 0 || pair == 3 ? 0 : pair == 1 || pair == 4 ? 1 : 2;                // 0 1 2 0 1 of the queries
+                umma_ss(d, desc_rows(qa + qp * PLANE, ks), desc_rows(ka + bp * PLANE, ks), idesc, i > 0);
+            });
     };
-    if (tid == 0) {
-        for (int sp = 0; sp < SPANS; ++sp) products(tmem + S_COL + sp * 128, ka, QPL, sp);
-        umma_commit(bar);
-    }
+    using KeyPlanes = std::integral_constant<int, QPL>;
+    using StatePlanes = std::integral_constant<int, 3>;
+    float w[OWN / 16][16], o[OWN / 16][16];                          // scores, then weights, of this row and a quarter of the keys; read-outs of a quarter of the columns
+#pragma unroll
+    for (int g = 0; g < OWN / 16; ++g)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) w[g][i] = o[g][i] = 0.f;
+    if (tid == 0) issue_rows(KeyPlanes{}, 0, bar_s);
     __syncwarp();
     // the state before the chunk travels meanwhile: 128 value columns of KP channels
     constexpr int PIECES = KP / 8, ITERS = DVP * PIECES / NT;
@@ -389,7 +445,22 @@ __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, 
         }
         den *= row_in;
     }
-    mbar_wait(bar, 52, err);                                         // the scores are there, the keys have been read
+#pragma unroll
+    for (int r = 0; r < Tc::Scores::N; ++r) {
+        mbar_wait(bar_s + 8 * r, 52, err);
+#pragma unroll
+        for (int g = 0; g < OWN / 16; ++g) add_round<TERMS, (QPL > 1)>(r, mine + g * 16, SLOT, w[g]);
+        if (r + 1 < Tc::Scores::N) {
+            sync_tc();
+            if (tid == 0) issue_rows(KeyPlanes{}, r + 1, bar_s);
+            __syncwarp();
+        }
+    }
+    if constexpr (QPL > 1) {
+        mbar_wait(bar_s + 8 * Tc::Scores::N, 52, err);
+#pragma unroll
+        for (int g = 0; g < OWN / 16; ++g) add_slot(mine + (SLOTS - 1) * SLOT + g * 16, w[g]);
+    }
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
         const int e = i * NT + tid;
@@ -397,85 +468,96 @@ __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, 
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     sync_tc();
-    if (tid == 0) {
-        for (int sp = 0; sp < SPANS; ++sp) products(tmem + O_COL + sp * 128, ka, 3, sp);
-        umma_commit(bar + 8);
-    }
+    if (tid == 0) issue_rows(StatePlanes{}, 0, bar_o);
     __syncwarp();
-    // the scores of this row and a quarter of the keys: weighed, masked, and back as planes
-    float w[OWN];
+    // the scores weighed and masked
     const float2 M = two_floats(MODE == MLSTM ? Ms[row] : 0.0);
 #pragma unroll
     for (int g = 0; g < OWN / 16; ++g) {
-        float o[16];
-        tmem_sum16<SPANS>(mine + S_COL + group * OWN + g * 16, 128, o);
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int j = group * OWN + g * 16 + i;
             float f;
-            if constexpr (MODE == RET) f = pw[max(row - j, 0)];
-            else f = expf((xs[j].x - M.x) + (xs[j].y - M.y));
-            const float x = j <= row ? o[i] * f : 0.f;
-            if constexpr (MODE == MLSTM) den += x;
-            w[g * 16 + i] = x;
+            if constexpr (MODE == RET) {
+                f = pw[max(row - j, 0)];
+            } else {                                                 // e^(x - M): the difference, and what rounding it to 32 bits leaves
+                const float2 x = xs[j];
+                const float d = x.x - M.x, u = d - x.x, e = expf(d);
+                f = fmaf(e, ((x.x - (d - u)) - (M.x + u)) + (x.y - M.y), e);
+            }
+            const float y = j <= row ? w[g][i] * f : 0.f;
+            if constexpr (MODE == MLSTM) sum[i & 3] += y;
+            w[g][i] = y;
         }
+        if constexpr (MODE == MLSTM) den += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
     if constexpr (MODE == MLSTM) den_s[group][row] = den;            // (its first row held e^-m, which every thread has read)
-    sync_tc();                                                       // all scores have been read: the planes go over them
+#pragma unroll
+    for (int r = 0; r < Tc::State::N; ++r) {
+        mbar_wait(bar_o + 8 * r, 53, err);
+#pragma unroll
+        for (int g = 0; g < OWN / 16; ++g) add_round<TERMS, true>(r, mine + g * 16, SLOT, o[g]);
+        sync_tc();
+        if (r + 1 < Tc::State::N) {
+            if (tid == 0) issue_rows(StatePlanes{}, r + 1, bar_o);
+            __syncwarp();
+        }
+    }
     if constexpr (MODE == MLSTM) den = (den_s[0][row] + den_s[1][row]) + (den_s[2][row] + den_s[3][row]);
+    mbar_wait(bar_o + 8 * Tc::State::N, 53, err);                    // what the state before the chunk gives; queries and state have been read
 #pragma unroll
     for (int g = 0; g < OWN / 16; ++g) {
-        float x[16];
-        uint32_t p0[8], p1[8], p2[8];
+        add_slot(mine + (SLOTS - 1) * SLOT + g * 16, o[g]);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = w[g * 16 + i];
-        split_values<8>(x, p0, p1, p2);
-        const uint32_t at = mine + P_COL + group * (OWN / 2) + g * 8;
-        tmem_st8(at, p0);
-        tmem_st8(at + 64, p1);
-        tmem_st8(at + 128, p2);
+        for (int i = 0; i < 16; ++i) o[g][i] *= row_in;
+#pragma unroll
+        for (int c = 0; c < 16; c += 8) {
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = w[g][c + i];
+            store_piece<3>(q_s, W_PLANE, piece_at(row, group * OWN + g * 16 + c), x);
+        }
     }
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    mbar_wait(bar + 8, 53, err);                                     // what the state before the chunk gives
-    float o[OWN];
-#pragma unroll
-    for (int g = 0; g < OWN / 16; ++g) {
-        float x[16];
-        tmem_sum16<SPANS>(mine + O_COL + group * OWN + g * 16, 128, x);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) o[g * 16 + i] = x[i] * row_in;
-    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     sync_tc();
-    if (tid == 0) {                                                  // weights times values, spans of 64 tokens, the small planes first
-        for (int sp = 0; sp < 2; ++sp)
-            for (int l = 2; l >= 0; --l)
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks)
-                    umma_ts(tmem + O_COL + sp * 128, tmem + P_COL + l * 64 + sp * 32 + ks * 8, desc_cols(va, sp * 4 + ks), idesc_of(DVP, false, true), !(l == 2 && ks == 0));
-        umma_commit(bar + 16);
-    }
+    auto issue_values = [&](int r) {                                 // weights times values, the small planes of the weights apart
+        constexpr uint32_t idesc = idesc_of(DVP, false, true);
+        issue_round<CT / 16, true>(r, tmem, SLOT, bar_v, 2 * (CT / 16),
+            [&](uint32_t d, int i) { umma_ss(d, desc_rows(qa, i), desc_cols(va, i), idesc, 0); },
+            [&](uint32_t d, int i) { umma_ss(d, desc_rows(qa + (i < 8 ? 2 : 1) * W_PLANE, i & 7), desc_cols(va, i & 7), idesc, i > 0); });
+    };
+    if (tid == 0) issue_values(0);
     __syncwarp();
     float scale = 1.f, odd = 0.f;                                    // odd: not 0 if something of this thread's is not finite
     if constexpr (MODE == MLSTM) {
         odd = den * 0.f;
         scale = a.qscale / (fmaxf(fabsf(den * a.qscale), floor_) + 1e-6f);
     }
-    mbar_wait(bar + 16, 54, err);                                    // (all products are done: the output tile takes the operands' place)
+#pragma unroll
+    for (int r = 0; r < Tc::Values::N; ++r) {
+        mbar_wait(bar_v + 8 * r, 54, err);
+#pragma unroll
+        for (int g = 0; g < OWN / 16; ++g) add_round<CT / 16, true>(r, mine + g * 16, SLOT, o[g]);
+        if (r + 1 < Tc::Values::N) {
+            sync_tc();
+            if (tid == 0) issue_values(r + 1);
+            __syncwarp();
+        }
+    }
+    mbar_wait(bar_v + 8 * Tc::Values::N, 54, err);                   // (all products are done: the output tile takes the operands' place)
     constexpr int LD = DVP + 4;
     float* tile = reinterpret_cast<float*>(q_s);
 #pragma unroll
     for (int g = 0; g < OWN / 16; ++g) {
-        const int col = group * OWN + g * 16;
-        float x[16];
-        tmem_sum16<2>(mine + O_COL + col, 128, x);
+        add_slot(mine + (SLOTS - 1) * SLOT + g * 16, o[g]);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            x[i] += o[g * 16 + i];
-            if constexpr (MODE == MLSTM) x[i] *= scale;
-            odd = fmaf(x[i], 0.f, odd);
+            if constexpr (MODE == MLSTM) o[g][i] *= scale;
+            odd = fmaf(o[g][i], 0.f, odd);
         }
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(tile + row * LD + col + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(tile + row * LD + group * OWN + g * 16 + i) = make_float4(o[g][i], o[g][i + 1], o[g][i + 2], o[g][i + 3]);
     }
     tc_free(tmem, COLS);
     const size_t ld_o = (size_t)a.H * a.Dv;

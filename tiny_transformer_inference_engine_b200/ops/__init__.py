@@ -189,6 +189,7 @@ def _ring_form(N, K, num_sms, may_split):
 
 class CudaOps:
     name = "cuda-sm100a"
+    num_sms = 148                           # a B200's; what the device says, once there is one
 
     def __init__(self, device):
         if not torch.cuda.is_available():
@@ -1488,14 +1489,14 @@ class CudaOps:
 
     def mlstm_adds_bias(self, v, num_seqs, pad, v_dim) -> bool:
         """Whether ``mlstm_chunks`` takes the gates' bias (a sum apart costs two small kernels, 5 us of a layer's 127)."""
-        return self._chunk_tokens(1, v.dtype, v.shape[0], num_seqs, pad, v_dim) == 128
+        return self._chunk_tokens(1, v.dtype, v.shape[0], num_seqs, pad, v_dim, v.shape[1] // v_dim, self.num_sms) == 128
 
     scan_chunk_tokens = None                # None: by cost (``_in_chunks``); a number: chunks where a request may bring this many tokens
     scan_chunk_more = 0                     # and this many more for every other request
     scan_chunk_bytes = 128 << 20            # bytes of the states between chunks that are held at a time (about the L2: a longer step runs in passes)
     # us of a scan in chunks by kind (retention, mlstm, wkv): the launches, a request, a state element of a request, a token and state element
     scan_chunk_cost = ((31.0, 0.3, 8.5e-6, 1.6e-7), (24.0, 0.3, 7.5e-6, 1.6e-7), (28.0, 0.3, 1.45e-5, 3.6e-7))
-    scan_chunk128_cost = ((24.0, 0.3, 6.9e-6, 4.4e-8), (24.0, 0.3, 5.0e-6, 8.4e-8))      # the same in chunks of 128 tokens (retention, mlstm)
+    scan_chunk128_cost = ((28.0, 0.3, 6.2e-6, 5.2e-8), (24.0, 0.3, 5.0e-6, 8.4e-8))      # the same in chunks of 128 tokens (retention, mlstm)
     scan_walk_cost = ((4.0, 0.21, 8.2e-7), (4.0, 0.19, 8.2e-7), (4.0, 0.18, 8.2e-7))   # of a walk: the launch, a token of the longest request, a token and state element of the step
     # of the layer's eager pass around it: host us with a walk, what chunks' call adds; us of its other kernels, a token and squared width of them
     scan_pass_cost = ((90.0, 10.0, 35.0, 6e-9), (110.0, 2.0, 35.0, 6e-9), (126.0, 14.0, 60.0, 6e-9))
@@ -1510,9 +1511,9 @@ class CudaOps:
         figures above give both within a fifth over widths of 512 to 4,096, 1 to 24 requests and 16 to 1,024 tokens.  And an eager pass of the layer
         takes the longer of its kernels' and its host's time, of which chunks need more: they pay where the pass is shorter with them
         (the whole mixer of 300 tokens at width 1,024, walk | chunks: retention 105 | 99, mlstm 108 | 111, wkv 126 | 141).  The scan alone, walk | chunks,
-us, width 2,048: one request of 128 tokens retention 32 | 25, mlstm 33 | 25, wkv 26 | 34, of 512 tokens 116 | 28, 107 | 28,
-        93 | 41; eight of 16 tokens 32 | 35, 25 | 30, 17 | 41, of 64 tokens 99 | 38, 71 | 32, 55 | 44; 256 tokens beside 23 decoding
-        requests 92 | 95, 85 | 64, 63 | 87."""
+        us, width 2,048: one request of 128 tokens retention 31 | 30, mlstm 30 | 26, wkv 26 | 34, of 512 tokens 116 | 32, 107 | 27,
+        93 | 41; eight of 16 tokens 29 | 57, 21 | 44, 17 | 41, of 64 tokens 96 | 41, 68 | 32, 55 | 44; 256 tokens beside 23 decoding
+        requests 87 | 87, 81 | 59, 63 | 87."""
         if not 8 <= dim <= 128 or dim % 8 or v_dim % 8:
             return False
         others = num_seqs - 1
@@ -1520,7 +1521,7 @@ us, width 2,048: one request of 128 tokens retention 32 | 25, mlstm 33 | 25, wkv
             longest = num_tokens - others
         if self.scan_chunk_tokens is None:
             state, (start, token, work) = num_heads * dim * v_dim, self.scan_walk_cost[mode]
-            large = self._chunk_tokens(mode, v.dtype, num_tokens, num_seqs, dim, v_dim) == 128
+            large = self._chunk_tokens(mode, v.dtype, num_tokens, num_seqs, dim, v_dim, num_heads, self.num_sms) == 128
             base, request, element, each = (self.scan_chunk128_cost if large else self.scan_chunk_cost)[mode]
             host, more, rest, product = self.scan_pass_cost[mode]
             rest += product * num_tokens * (num_heads * v_dim) ** 2
@@ -1536,17 +1537,21 @@ us, width 2,048: one request of 128 tokens retention 32 | 25, mlstm 33 | 25, wkv
         return True
 
     @staticmethod
-    def _chunk_tokens(mode, v_dtype, num_tokens, num_seqs, key_pad, v_dim) -> int:
+    def _chunk_tokens(mode, v_dtype, num_tokens, num_seqs, key_pad, v_dim, num_heads=1, num_sms=148) -> int:
         """Tokens of a chunk: 128 with products on tcgen05 (csrc/matrix_chunks_tc.cu: retention and the matrix memory, bfloat16 values of at most 128
-        columns), else 64 (csrc/matrix_chunks.cu).  us, 64 | 128: 16 heads of 128 x 128 one request of 2,048 tokens 99 | 49, of 128 41 | 25,
-        16 of 128 129 | 83; 16 of 64 x 128 67 | 46, 32 | 25, 74 | 61; 8 of 64 x 64 one of 300 tokens 16 | 18 (one tile of 128 rows a chunk is
-        too much for so little).  Every request has a chunk of its own, so decoded tokens beside a short portion are better
-        off with small ones: 23 and 256 tokens 95 | 102 (mlstm 64 | 75), 7 and 512 63 | 55 (49 | 47), 31 and 2,000 208 | 185 (139 | 139)."""
-        return 128 if mode < 2 and v_dtype == torch.bfloat16 and v_dim <= 128 and max(key_pad, v_dim) > 64 and num_tokens >= 24 * num_seqs else 64
+        columns), else 64 (csrc/matrix_chunks.cu).  us, 64 | 128: 16 heads of 128 x 128 one request of 2,048 tokens 95 | 59, of 128 43 | 30,
+        16 of 128 122 | 87; 16 of 64 x 128 54 | 40, 25 | 22, 64 | 56; 8 of 64 x 64 one of 300 tokens 16 | 22 (one tile of 128 rows a chunk is
+        too much for so little).  Every request has a chunk of its own, and a short one costs what a full one does: decoded tokens beside a
+        portion are better off with small chunks, where more chunks and heads than run at once make that time - 31 beside 2,000 tokens 198 | 212
+        (mlstm 128 | 143), 15 beside 512 with 32 heads 150 | 176 (97 | 118), 23 beside 256 87 | 108 (59 | 78) -, while with fewer the shorter chain of
+        large ones counts: 7 beside 512 65 | 61 (49 | 48), 15 beside 512 with 8 heads 64 | 61 (47 | 47), eight of 64 tokens 64 | 41 (41 | 32)."""
+        if not (mode < 2 and v_dtype == torch.bfloat16 and v_dim <= 128 and max(key_pad, v_dim) > 64 and num_tokens >= 24 * num_seqs):
+            return 64
+        return 128 if num_tokens >= 100 * num_seqs or (num_tokens // 128 + num_seqs) * num_heads <= 1.5 * num_sms else 64
 
     def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale, pre_bias=None):
         T, pad = q.shape[0], S.shape[-1]
-        tokens = self._chunk_tokens(mode, v.dtype, T, num_seqs, pad, v_dim)
+        tokens = self._chunk_tokens(mode, v.dtype, T, num_seqs, pad, v_dim, num_heads, self.num_sms)
         total = T // tokens + num_seqs                                 # chunk numbers of the step
         states = num_heads * v_dim * pad                               # floats of a chunk number: its states, their sums or decays, mlstm: spans and maxima
         slots = max(1, min(total, self.scan_chunk_bytes // (states * 4)))
