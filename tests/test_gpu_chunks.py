@@ -321,3 +321,68 @@ def test_chunks_of_128_tokens_are_no_further_off_than_chunks_of_64(ops, monkeypa
             err[tokens][0] += rel(rows(out), rows(exp))
             err[tokens][1] += rel(states[0], exp_states[0])
     assert err[128][0] < 1.04 * err[64][0] and err[128][1] < 1.04 * err[64][1], err
+
+
+@pytest.mark.parametrize("odd", [False, True])
+def test_gate_bias_added_in_the_chunks(ops, monkeypatch, odd):
+    """The matrix memory with the gates' bias read in its kernels against the same bias added to the pre-activations before: the same 32-bit sums, so
+    the same to the last bit; also where a chunk and the states behind it are not finite and are walked.  And against 64 bits."""
+    monkeypatch.setattr(type(ops), "_chunk_tokens", staticmethod(lambda *a: 128))
+    H, D, Dv = 3, 64, 128
+    sc = Scan("mlstm", [300, 7, 130], H, D, Dv, seed=9)
+    bias = torch.cat([torch.linspace(-1.3, 2.1, H), torch.linspace(3.0, -0.7, H)]).bfloat16().to(DEV)      # input gates, forget gates
+    if odd:
+        sc.v[150, 5], sc.v[310, 200] = float("inf"), float("nan")
+    ops.scan_chunk_tokens = 1
+    added = sc.pre + bias.float()
+    results = []
+    for pre, b in ((sc.pre, bias), (added, None)):
+        S, n, m = sc.S0.clone(), sc.n0.clone(), sc.m0.clone()
+        out = ops.mlstm_chunks(sc.q, sc.k, sc.v, pre, S, n, m, sc.qsl, sc.slots, 3, H, D, Dv, 15.0, D ** -0.5, pre_bias=b)
+        results.append((out, S, n, m))
+    for a, b in zip(*results):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
+    assert torch.isfinite(results[0][0]).all() != odd
+    if not odd:
+        sc.pre = added
+        exp, exp_states = sc.exact()
+        rows = lambda x: x.double().view(-1, H, Dv)[~sc.near]
+        assert rel(rows(results[0][0]), rows(exp)) < 2e-6
+        for s, e in zip(results[0][1:], exp_states):
+            assert rel(s, e) < 1e-6
+
+
+def test_gate_bias_is_refused_by_chunks_of_64(ops, monkeypatch):
+    from tiny_transformer_inference_engine_b200.ops import KernelError
+    monkeypatch.setattr(type(ops), "_chunk_tokens", staticmethod(lambda *a: 64))
+    ops.scan_chunk_tokens = 1
+    sc = Scan("mlstm", [200], 2, 64, 128)
+    with pytest.raises(KernelError, match="gate bias"):
+        ops.mlstm_chunks(sc.q, sc.k, sc.v, sc.pre, sc.S0, sc.n0, sc.m0, sc.qsl, sc.slots, 1, 2, 64, 128, 15.0, 0.125, pre_bias=torch.zeros(4, dtype=torch.bfloat16, device=DEV))
+
+
+@pytest.mark.parametrize("lens", [[256], [1, 300, 200]])
+def test_mlstm_layer_hands_its_gate_bias_to_the_chunks(ops, monkeypatch, lens):
+    """The layer over a prompt in chunks of 128 tokens: it leaves the bias to the chunks, and gives what it gives with the bias in the product."""
+    from test_gpu_mizupel import part_with_weights, ctx_for, rel_norm, pm
+    from tiny_transformer_inference_engine_b200.parts.base import FixedStateView, PartSpec
+    heads, dim, vdim, d = 2, 64, 128, 64
+    spec = PartSpec("mlstm", "", {"d_model": d, "num_heads": heads, "dim": dim, "vdim": vdim, "gate_cap": 15.0, "eps": 1e-5})
+    part, w = part_with_weights("mixer", spec, "bfloat16", ops, 5, scale=0.2, scales={"i": 0.5, "f": 0.5, "i.b": 1.0, "f.b": 2.0})
+    assert len(set(part.b_gates.tolist())) == 2 * heads
+    x = torch.randn(sum(lens), d, generator=torch.Generator().manual_seed(3)).bfloat16()
+    ops.scan_chunk_tokens = 1
+    took, results = [], []
+    adds = type(ops).mlstm_adds_bias
+    for answer in (adds, lambda *a: False):
+        monkeypatch.setattr(type(ops), "mlstm_adds_bias", lambda *a, f=answer: took.append(f(*a)) or took[-1])
+        states = [torch.zeros(len(lens) + 1, *need.shape, device=DEV) for need in part.cache_needs()]
+        y = part.forward(x.to(DEV), ctx_for(ops, torch.bfloat16, [(0, n) for n in lens], None, slots=list(range(len(lens)))), [FixedStateView(s) for s in states])
+        results.append([y.sum(0) if y.dim() == 3 else y] + states)
+    assert took == [True, False]
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    at = 0
+    for n in lens:
+        exp = pm.mlstm(x[at:at + n].double(), w, "", {"heads": heads, "dim": dim, "vdim": vdim, "gate_cap": 15.0}, 1e-5)
+        assert rel_norm(results[0][0][at:at + n], exp) < 3e-2
+        at += n
