@@ -1,8 +1,10 @@
 """Which form a product or a scan takes: by the sizes of the step alone."""
+import random
+
 import pytest
 import torch
 
-from tiny_transformer_inference_engine_b200.ops import CudaOps, _ring_form
+from tiny_transformer_inference_engine_b200.ops import CudaOps, _floor_sum, _ring_form
 
 
 @pytest.mark.parametrize("rows,hidden,K,fused", [
@@ -141,3 +143,54 @@ def test_form_of_a_decode_product_comes_from_its_sizes(N, K):
     (RETENTION, [1] * 7 + [512], 16, 128), (MLSTM, [1] * 15 + [512], 8, 128), (RETENTION, [64] * 8, 16, 128)])   # ... and fewer
 def test_tokens_of_a_chunk_by_what_runs_at_once(mode, lens, heads, tokens):
     assert CudaOps._chunk_tokens(mode, torch.bfloat16, sum(lens), len(lens), 128, 128, heads, 148) == tokens
+
+
+def _pieces_tile_by_tile(num_sms, heads, rows, group, head_dim, max_q_len, max_kv_len):
+    """The cost model of the float32 pieces, every candidate and every tile."""
+    step, tiles, ctx = 3.4 + 0.061 * (64 if head_dim <= 64 else 128), -(-rows // 64), max(0, max_kv_len - max_q_len)
+    ends = [ctx + -(-min(rows, (t + 1) * 64) // group) for t in range(tiles)]
+    work = sum(-(-e // 64) for e in ends) * heads / num_sms * 0.92 * step
+    best, best_cost, last = ("simt", 1, 0), None, 0
+    for want in range(1, min(64, -(-max_kv_len // 64)) + 1):
+        length = -(-(-(-max_kv_len // want)) // 64) * 64
+        n = -(-max_kv_len // length)
+        if n == last:
+            continue
+        last = n
+        ctas, alone = heads * sum(-(-e // length) for e in ends), length / 64 * step
+        cost = alone if ctas <= num_sms else max(1.84 * alone, work) if ctas <= 2.2 * num_sms or n == 1 else work + 0.5 * alone
+        if n > 1:
+            cost += 3.0 + heads * rows * (n * (4 * head_dim + 8) + 4 * head_dim) / 2e6
+        if best_cost is None or cost < 0.97 * best_cost:
+            best, best_cost = (("simt", n, length) if n > 1 else ("simt", 1, 0)), cost
+    return best
+
+
+def test_float32_pieces_in_closed_form():
+    """The plan is the one of the model tile by tile, for all kinds of portions, and is not paid for tile by tile."""
+    rng = random.Random(5)
+    ops = CudaOps.__new__(CudaOps)
+    for _ in range(600):
+        group, kv_heads, seqs = rng.choice([1, 2, 3, 7, 8, 16, 32, 71]), rng.choice([1, 1, 2, 4, 8]), rng.choice([1, 1, 2, 5, 16])
+        new = int(2 ** rng.uniform(0, 11))
+        keys = new + rng.choice([0, 0, int(2 ** rng.uniform(0, 13))])
+        if new * group < 64:
+            continue
+        case = (seqs * kv_heads, new * group, group, rng.choice([36, 64, 128]), new, keys)
+        assert ops._f32_tile_pieces(*case) == _pieces_tile_by_tile(148, *case), case
+
+
+def test_float32_pieces_stop_where_no_candidate_can_be_better(monkeypatch):
+    from tiny_transformer_inference_engine_b200 import ops as module
+    calls = []
+    monkeypatch.setattr(module, "_floor_sum", lambda *a: calls.append(a) or _floor_sum(*a))
+    ops = CudaOps.__new__(CudaOps)
+    for heads, group, new in ((1, 71, 2048), (1, 32, 2048), (8, 4, 2048), (32, 1, 2048)):
+        calls.clear()
+        assert ops._f32_tile_pieces(heads, new * group, group, 128, new, new) == ("simt", 1, 0)
+        assert len(calls) == 2
+
+
+@pytest.mark.parametrize("n,m,a,b", [(0, 5, 3, 2), (1, 1, 0, 0), (7, 3, 5, 4), (500, 64 * 71, 64, 4543), (33, 10, 10, 0), (12, 7, 0, 20), (1000, 997, 996, 5)])
+def test_floor_sum(n, m, a, b):
+    assert _floor_sum(n, m, a, b) == sum((a * i + b) // m for i in range(n))

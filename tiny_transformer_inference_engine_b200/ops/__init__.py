@@ -163,6 +163,20 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+def _floor_sum(n, m, a, b):
+    """Sum of floor((a i + b) / m) over i = 0 .. n - 1 (n, a, b >= 0, m > 0), by the Euclidean algorithm on a and m."""
+    total = 0
+    while n > 0:
+        total += a // m * (n * (n - 1) // 2) + b // m * n
+        a, b = a % m, b % m
+        top = a * n + b
+        if top < m:
+            break
+        n, b = divmod(top, m)
+        m, a = a, m
+    return total
+
+
 @functools.lru_cache(maxsize=4096)
 def _ring_form(N, K, num_sms, may_split):
     """(K range of a CTA, form code) of the weight-streaming product through shared memory for a matrix of 4 Mi elements or more: one
@@ -769,12 +783,19 @@ class CudaOps:
         requests of 4 to 2,048 tokens behind up to 4,096 keys, head sizes 64 and 128): a tile step takes an SM 11.2 us at head
         size 128 and 7.3 at 64 with one CTA, 1.84 of that for two CTAs' steps side by side; a piece behind a row tile's own tokens
         is empty; a cut range costs 3 us and its partial results' way through memory at 2 TB/s.  (16 heads on one kv head of 128:
-        300 tokens 32 us in three pieces, 62 uncut; 600 tokens 70 in four, 148 uncut; 128 tokens behind 4,096 keys 144 in ten,
-        194 in four; 2,048 tokens 583 uncut, 614 in four.)"""
+        300 tokens 32 us in three pieces, 62 uncut; 600 tokens 68 in four, 148 uncut; 128 tokens behind 4,096 keys 144 in ten,
+        194 in four; 2,048 tokens 571 uncut, 614 in four.)
+
+        A portion's length is part of the plan's key, so every portion of a long prompt pays for this: tiles are summed in closed form, and
+        candidates end where none can be better (2,048 tokens of 32 heads on one: 1.2 ms tile by tile, 3 us now)."""
         step = 3.4 + 0.061 * (64 if head_dim <= 64 else 128)
         tiles, ctx = math.ceil(rows / 64), max(0, max_kv_len - max_q_len)
-        ends = [ctx + -(-min(rows, (t + 1) * 64) // group) for t in range(tiles)]          # (keys that a row tile sees)
-        work = sum(-(-e // 64) for e in ends) * heads / self.num_sms * 0.92 * step
+
+        def pieces(length):                                    # of `length` keys, over the row tiles: tile t sees ctx + ceil(min(rows, 64 (t + 1)) / group) keys
+            m = group * length
+            return _floor_sum(tiles - 1, m, 64, ctx * group + 64 + m - 1) + -(-(ctx * group + rows) // m)
+
+        work = pieces(64) * heads / self.num_sms * 0.92 * step
         best, best_cost, last = ("simt", 1, 0), None, 0
         for want in range(1, min(64, math.ceil(max_kv_len / 64)) + 1):
             split_len = math.ceil(math.ceil(max_kv_len / want) / 64) * 64
@@ -782,8 +803,10 @@ class CudaOps:
             if n == last:
                 continue
             last = n
-            ctas = heads * sum(-(-e // split_len) for e in ends)
-            alone = split_len / 64 * step
+            alone, merge = split_len / 64 * step, 3.0 + heads * rows * (n * (4 * head_dim + 8) + 4 * head_dim) / 2e6
+            if n > 1 and merge >= 0.97 * best_cost:            # (nor any more pieces)
+                break
+            ctas = heads * pieces(split_len)
             if ctas <= self.num_sms:
                 cost = alone
             elif ctas <= 2.2 * self.num_sms or n == 1:                 # (two a SM; the last pieces are the short ones)
@@ -791,7 +814,9 @@ class CudaOps:
             else:
                 cost = work + 0.5 * alone
             if n > 1:
-                cost += 3.0 + heads * rows * (n * (4 * head_dim + 8) + 4 * head_dim) / 2e6
+                cost += merge
+            elif cost == work and ctas > self.num_sms:
+                break                                          # several waves: pieces have the same work, and their merge on top
             if best_cost is None or cost < 0.97 * best_cost:
                 best, best_cost = (("simt", n, split_len) if n > 1 else ("simt", 1, 0)), cost
         return best
