@@ -1350,3 +1350,38 @@ def test_float32_tiles_rows_do_not_meet_values_they_must_not_see(ops, Hq, Hkv, D
             sees[token:token + window if window else n] = True
             assert torch.equal(got[~sees], clean[~sees]), (value, token)
             assert not torch.isfinite(got[sees].view(-1, Hq, D)[:, :Hq // Hkv]).all(-1).any(), (value, token)
+
+
+@pytest.mark.parametrize("kv_len,splits", [(3000, 24), (3000, 12), (1000, 4)])
+def test_decode_chain_is_the_same_with_and_without_waits_between_kernels(ops, kv_len, splits):
+    """Attention over a cut key range, its merge, a product in partial sums, the norm that adds them, a gated product, and again: every kernel may start before
+    the one ahead is done, and each must wait for what it reads.  The host waits after every call in the second run; the results are the same bits."""
+    g = torch.Generator().manual_seed(56)
+    B, H, D, page, F, d = 4, 16, 64, 64, 4096, 1024
+    width = -(-kv_len // page)
+    table = (torch.randperm(B * width, generator=g).int() + 1).view(B, width).to(DEV)
+    kp, vp = (torch.randn(B * width + 1, 1, page, D, generator=g).bfloat16().to(DEV) for _ in range(2))
+    mats = lambda n, k: (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16().to(DEV)
+    w_q, w_o, w_gu, w_down, norm = mats((H + 2) * D, d), mats(d, H * D), mats(2 * F, d), mats(d, F), torch.ones(d, device=DEV)
+    qsl, lens = torch.arange(B + 1, dtype=torch.int32, device=DEV), torch.full((B,), kv_len, dtype=torch.int32, device=DEV)
+    plan = ("tc", splits, -(-kv_len // splits // 128) * 128) if splits * 128 <= kv_len else ("tc", 1, 0)
+    plan = (plan[0], -(-kv_len // plan[2]), plan[2]) if plan[2] else plan
+    start = torch.randn(B, d, generator=g).to(DEV)
+
+    def run(wait):
+        done = torch.cuda.synchronize if wait else (lambda: None)
+        resid, delta, x = start.clone(), None, torch.empty(B, d, dtype=torch.bfloat16, device=DEV)
+        for _ in range(12):
+            ops.add_rmsnorm(resid, delta, norm, 1e-6, x); done()
+            q = ops.linear(x, w_q, None); done()
+            out = torch.empty(B, H * D, dtype=torch.bfloat16, device=DEV)
+            ops.paged_attention(q, H, 1, D, kp, vp, table, page, qsl, lens, B, 1, kv_len, D ** -0.5, 0, out, plan=plan); done()
+            delta = ops.linear(out, w_o, None, partial_ok=True); done()
+            ops.add_rmsnorm(resid, delta, norm, 1e-6, x); done()
+            delta = ops.linear(ops.linear_swiglu(x, w_gu, None, F), w_down, None, partial_ok=True); done()
+        return resid + (delta.sum(0) if delta.dim() == 3 else delta)
+    first, again = run(True), run(False)
+    assert torch.isfinite(first).all() and torch.equal(first, again)
+    for _ in range(5):
+        assert torch.equal(run(False), first)
+    assert ops.tc_error() == 0

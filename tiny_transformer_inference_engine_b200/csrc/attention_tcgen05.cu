@@ -283,7 +283,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         pdl_wait();                                                // this warp asks for the pages the predecessor has just written
-        pdl_launch_dependents();                                   // (the merge, and the product behind it, whose weights travel meanwhile)
     } else {
         // queries of the tile -> shared memory in the K-major swizzled operand layout (they are the predecessor's output)
         pdl_wait();
@@ -304,10 +303,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_slot;
-    // (No griddepcontrol.launch_dependents here: with it the merge kernel's CTAs sit beside this kernel's from its start, and
-    // a decode step of 8 requests at 4,096 tokens was measured at 3.00 ms instead of 2.74.  Asking for the successor only
-    // when a CTA starts its last tile costs as well: 2.95 ms instead of 2.69, the kernel alone 10.4 instead of 9.0 us at
-    // 2,048 keys.  The successor is scheduled as this grid's CTAs exit.)
+    // (No griddepcontrol.launch_dependents here: the merge kernel's CTAs would sit beside this kernel's from its start, and the product's behind them.
+    // With it a decode step of 32 layers was measured at 2.632 ms instead of 2.635 for 8 requests at 4,096 tokens, 2.416 instead of 2.397 for one
+    // at 600; before the product's weights came through shared memory at 3.00 instead of 2.74.  Asking for the successor
+    // only when a CTA starts its last tile cost then as well: 2.95 ms instead of 2.69, the kernel alone 10.4 instead of 9.0 us at 2,048 keys.  The
+    // successor is scheduled as this grid's CTAs exit.)
 
     if (warp == 0 && AHEAD) {
         // Prompt portions.  The whole warp walks the tiles: lane b looks up the page of box b (a

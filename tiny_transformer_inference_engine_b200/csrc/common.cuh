@@ -28,6 +28,9 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // A small kernel in front of a product that streams weights lets it in before its own wait: the product fills its rings while this
 // kernel and the end of the one before run.  Only for kernels whose successors read nothing but weights ahead of their wait: what such a
 // successor may count on by then is a kernel further back.
+// (The decode norm and the small merge of attention pieces: a step of 32 layers at Llama-7B sizes 2.711 -> 2.632 ms for 8 requests at 4,096
+// tokens, 2.481 -> 2.416 for one at 600.  While products loaded their weights into registers the same was slower: they have little to ask for
+// ahead of their wait, and their CTAs took the SMs' room.)
 #define TTIE_PDL_ENTRY_EARLY() do { ::ttie::pdl_launch_dependents(); ::ttie::pdl_wait(); } while (0)
 // first statement of a kernel: wait for the predecessor's results, then let the successor be scheduled
 #define TTIE_PDL_ENTRY() do { ::ttie::pdl_wait(); ::ttie::pdl_launch_dependents(); } while (0)
@@ -119,8 +122,9 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 int num_sms();
 
 // Programmatic dependent launch: a kernel launched this way may be scheduled while its predecessor in
-// the stream drains; it must call pdl_wait() before it touches anything the predecessor wrote (the
-// kernels here call it first thing, so only launch latency and CTA scheduling overlap).  Works inside
+// the stream drains; it must call pdl_wait() before it touches anything the predecessor wrote (most
+// kernels here call it first thing, so only launch latency and CTA scheduling overlap; the weight-streaming products ask for weights, and
+// others set up barriers and tensor memory, ahead of it).  Works inside
 // captured graphs.  ttie_set_pdl(0) turns it off.
 bool pdl_enabled();
 // asks (and clears) whether the next kernel is to be launched as an ordinary one although pdl_enabled(): the first kernel of a stream
