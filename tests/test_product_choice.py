@@ -194,3 +194,11 @@ def test_float32_pieces_stop_where_no_candidate_can_be_better(monkeypatch):
 @pytest.mark.parametrize("n,m,a,b", [(0, 5, 3, 2), (1, 1, 0, 0), (7, 3, 5, 4), (500, 64 * 71, 64, 4543), (33, 10, 10, 0), (12, 7, 0, 20), (1000, 997, 996, 5)])
 def test_floor_sum(n, m, a, b):
     assert _floor_sum(n, m, a, b) == sum((a * i + b) // m for i in range(n))
+
+
+@pytest.mark.parametrize("M,N,K,planes", [
+    (320, 1024, 1024, True), (200, 1024, 1024, True), (33, 512, 2048, True), (1200, 1024, 256, True), (600, 4096, 128, True), (33, 1536, 1024, True),
+    (48, 1024, 1024, False), (320, 512, 512, False), (96, 2048, 256, False), (200, 2048, 128, False), (64, 1024, 1024, False), (1200, 256, 1024, False)])
+def test_float32_products_on_tensor_cores_by_their_work(M, N, K, planes):
+    """Both sides of each line of the rule: the weights, the three sizes' product, a long K."""
+    assert CudaOps._f32_planes_ok(torch.zeros(M, K), torch.zeros(N, K)) is planes

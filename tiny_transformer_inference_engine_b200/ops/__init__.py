@@ -458,17 +458,22 @@ class CudaOps:
     @staticmethod
     def _f32_planes_ok(x, w):
         """Whether a float32 product runs on the tensor cores, each value as three bfloat16 (csrc/gemm_fp32_tc.cu): rows that its
-        copies can take (16 bytes), and enough work for its fixed cost of 8 to 12 us.  Measured on the other side, us here | multiply-adds:
-        [1024, 1024] 64 rows 13.9 | 13.5, 320 rows 20.6 | 37.7; [512, 512] 320 rows 16.5 | 13.9; [2048, 512] 128 rows 16.1 | 14.2;
-        [512, 2048] 33 rows 15.8 | 22.1; [2048, 2048] 33 rows 17 | 35.  17 to 32 rows (there the weights are streamed twice, and sums
-        over short K are closer to 64 bits): [256, 1024] 11.8 | 16.6, [8192, 2048] 24 | 63, [50257, 512] has a short K and stays."""
+        copies can take (16 bytes), and enough work for its fixed cost of 8 to 12 us - by the weights, which stream once whatever the rows are, by
+        the products of all three sizes, or by a K that is a long chain for multiply-adds.  Measured on both sides of each line, us here |
+        multiply-adds, rows by [N, K]: 33 by [1536, 1024] 12 | 13, 48 by [1024, 1024] 12 | 14 (left there), 200 by [1024, 1024] 17 | 21, 320 by it 20 | 39;
+        96 by [512, 1536] 17 | 18, 33 by [512, 2048] 15 | 22, 320 by [512, 1024] 20 | 20; 1,200 by [1024, 256] 18 | 33, 96 by [2048, 256] 12 | 15 (left there);
+        600 by [4096, 128] 17 | 27, 200 by [2048, 128] 14 | 8.  Of 531 shapes of more rows and N from 512 on what is taken is 4.8 % above the faster
+        one on average (18 % by the weights alone), and this one, where taken, never more than 9 %.  17 to 32 rows (there the weights are streamed twice, and sums over short K are closer to 64 bits):
+        [256, 1024] 11.8 | 16.6, [8192, 2048] 24 | 63, [50257, 512] has a short K and stays."""
         M, K = x.shape
         N = w.shape[0]
         if K % 4 or x.stride(0) % 4 or w.stride(0) % 4 or (x.data_ptr() | w.data_ptr()) & 15:
             return False
         if M <= 32:
             return M > 16 and K >= 1024 and N * K >= 1 << 20
-        return N >= 512 and K >= 128 and N * K >= 3 << 19
+        if N < 512 or K < 128:
+            return False
+        return N * K >= 3 << 19 or K >= 1536 or M * N * K >= (1 << 27 if K >= 256 else 1 << 28)
 
     def linear(self, x, w, bias, out_dtype=None, partial_ok=False):
         """y = x @ w.T (+ bias); x [M, K], w [N, K] -> [M, N].  With ``partial_ok`` the result may
