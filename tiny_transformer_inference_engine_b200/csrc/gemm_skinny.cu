@@ -457,12 +457,14 @@ int dispatch(const SkinnyParams& p, int splits, int unroll, cudaStream_t s) {
     // Through shared memory from 1 Mi weights on ([1024, 1024] 1.8 us either way, [512, 2048] 2.5 | 3.3).  us, this form | the other, 1 row and 8:
     // [4352, 4096] 6.7 | 7.5, 7.2 | 7.6; [4096, 4096] 6.4 | 6.7, 7.0 | 7.0; gate and up of [22016, 4096] 27.0 | 31.2, 27.5 | 31.6; [4096, 11008]
     // 13.9 | 15.5, 15.0 | 16.2; [32000, 4096] 37.8 | 44.1, 38.8 | 45.4; [256000, 2048] 146 | 145, 147 | 145 (copies alone: 5.5 us for 33 MB,
-    // 25.9 for 180, 37.0 for 262).  The gated unit in sets of 8 + 8 rows where these are long enough a unit: [22016, 4096] 27.0 against 29.6 in 16 +
-    // 16, [32768, 2048] 20.7 against 19.9.
+    // 25.9 for 180, 37.0 for 262).  The gated unit in sets of 8 + 8 rows where these are long enough a unit.  8 + 8 | 16 + 16 at 1 row and 8: [16384, 1024]
+    // 9.4 | 8.4, 9.4 | 9.2; [16384, 2048] 12.8 | 11.7, 13.1 | 12.5; [32768, 2048] 21.0 | 21.1, 22.4 | 22.0; [13824, 2560] 12.9 | 12.8, 13.7 | 14.5;
+    // [16384, 3072] 16.2 | 16.9, 17.9 | 18.2; [19456, 3584] 23.4 | 25.9, 24.6 | 26.8; [22016, 4096] 27.9 | 31.0, 28.8 | 31.9; [36352, 4544] 47.9 | 48.7,
+    // 49.4 | 49.9; [57344, 8192] 131.5 | 137.0, 135.4 | 137.4.  The sums are the same to the last bit either way.
     const long long weights = (long long)p.N * (EPI == 2 ? 2 : 1) * p.K;
     // (A gated unit of fewer units than SMs stays with the other form: its caller has a product cut over K, with the activation behind it, for that.)
     if (mt <= 2 && p.K % 64 == 0 && weights >= (1LL << 20) && (EPI != 2 || p.N >= 8 * num_sms())) {
-        const bool wide = EPI == 2 ? p.K < 4096 : two;
+        const bool wide = EPI == 2 ? p.K < 2560 : two;
         if (mt == 1) return wide ? launch_bulk<1, EPI, 2>(p, splits, s) : launch_bulk<1, EPI, 1>(p, splits, s);
         return wide ? launch_bulk<2, EPI, 2>(p, splits, s) : launch_bulk<2, EPI, 1>(p, splits, s);
     }

@@ -184,9 +184,13 @@ def _ring_form(N, K, num_sms, may_split):
     by a stopwatch: the ranges decide the order of the sums, so a choice between forms a few percent apart, made anew in every process,
     would give other last bits from one to the next (the row sets do not).  The cost: a unit's bytes (its weights, the copies of the activations, a
     start) times the waves of units on two CTAs an SM, the last one with the fill to the power of 0.4, since fewer CTAs get
-    more of the memory's rate each.  Fitted to 50 shapes of [1024, 4096] to [256000, 2048] at 1, 8 and 16 rows: on average 2.6 % above the
-    fastest of 18 to 27 forms, a tenth at one in twenty; at the Llama sizes, us at 1 row and 8: [4352, 4096] 7.3, 7.8 in two ranges of two sets (8.0,
-    8.5 uncut with one), [4096, 4096] 6.9, 7.7 (7.7, 8.2), [4096, 11008] 15.6, 16.3 (16.2, 16.7), [32000, 4096] uncut with one set 38.8, 39.4."""
+    more of the memory's rate each.  From 2.5 waves of tiles of one set on (2 where K stays whole) these as they are: they are handed on as CTAs come free, so that no last wave
+    is left ([32000, 4096] 38.8 us, two sets 39.5; [12288, 4096] 16.1 and 18.8).  Fitted to 50 shapes of [1024, 4096] to [256000, 2048] at 1, 8
+    and 16 rows: on average 2.3 % above the fastest of 18 to 27 forms (uncut 0.7 % above the faster of two), a tenth at one in twenty, 29 % at worst; at the
+    Llama sizes, us at 1 row and 8: [4352, 4096] 7.3, 7.8 in two ranges of two sets (8.0, 8.5 uncut with one), [4096, 4096] 6.9, 7.7 (7.7, 8.2),
+    [4096, 11008] 15.6, 16.3 (16.2, 16.7)."""
+    if math.ceil(N / 16) >= (5 if may_split else 4) * num_sms:
+        return math.ceil(K / 128) * 128, 0
     best, best_cost = None, None
     for sets in (1, 2):
         for S in (1, 2, 3, 4, 5, 6, 8) if may_split else (1,):
@@ -198,7 +202,6 @@ def _ring_form(N, K, num_sms, may_split):
             if best_cost is None or cost < best_cost:
                 best, best_cost = (kslice, 16 * (sets - 1)), cost
     return best
-
 
 
 class CudaOps:
