@@ -569,7 +569,8 @@ class CudaOps:
 
     def tc_error(self) -> int:
         """Error word of the tcgen05 kernels (0 = none; otherwise the code of the first bounded wait that
-        ran out: product 1-4, attention 101-110); synchronises the device."""
+        ran out: products 1-4 and so on by kernel, float32 product 41-48, chunks of 128 tokens 51-54, decode product 61-63,
+        attention 101-110); synchronises the device."""
         g = int(self.lib.ttie_tc_error())
         a = int(self.lib.ttie_attn_tc_error())
         return g or (100 + a if a else 0)
