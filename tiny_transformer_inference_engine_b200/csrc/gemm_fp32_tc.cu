@@ -32,14 +32,10 @@
 // a sum that is not finite.
 // Every mbarrier wait is bounded by a clock deadline; one that runs out records a code and the roles leave their loops.
 #include "planes.cuh"
-#include <cuda.h>
+#include "tc_ptx.cuh"
 #include <atomic>
 using namespace ttie;
-
-namespace ttie {
-int gemm_tc_error_words(int** word, int** mirror);               // the product kernels' error word and its mirror (gemm_tcgen05.cu)
-int gemm_tc_make_map_of(CUtensorMap* map, int f32, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows);
-}  // namespace ttie
+using namespace ttie::tc;
 
 namespace {
 constexpr int HALF = 128, KB = 64, TOK_MOST = 160, MAX_RANGES = 8, MAX_PARTIAL = 16;
@@ -47,7 +43,6 @@ constexpr uint32_t W_BYTES = HALF * KB * 4, D_COL = 0, P_COL = 2 * TOK_MOST, P_C
 constexpr uint32_t SMEM_MOST = 226 * 1024;
 constexpr int W_STAGES_MOST = 6;
 constexpr float UP = 16777216.f, DOWN = 3.5527136788005009e-15f;          // 2^24 on the operands, 2^-48 on the sums
-constexpr long long WAIT_CYCLES = 2000000000LL;                 // about one second
 
 enum { WFULL = 0, WEMPTY = W_STAGES_MOST, XFULL = 2 * W_STAGES_MOST, XEMPTY = XFULL + 2, AFULL = XEMPTY + 2, AEMPTY = AFULL + 2, DFULL = AEMPTY + 2,
        DEMPTY = DFULL + 2, NBARS = DEMPTY + 2 };
@@ -58,35 +53,9 @@ struct F32Params {
     int M, N, K, lda, ldw, ldc;
     long long part_stride;                                       // > 0: the ranges' sums leave one by one, C + rank * part_stride (no cluster)
     int width, tok_tiles, ranges, num_kb, w_stages;
-    int *err, *mirror;
+    ErrorWords err;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code, const F32Params& p) {
-    if (mbar_try(bar, parity)) return true;
-    const long long deadline = clock64() + WAIT_CYCLES;
-    while (!mbar_try(bar, parity)) {
-        if (clock64() > deadline) {
-            atomicCAS(p.err, 0, code);
-            if (p.mirror) { *reinterpret_cast<volatile int*>(p.mirror) = code; __threadfence_system(); }
-            return false;
-        }
-    }
-    return true;
-}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y) : "memory");
@@ -98,27 +67,6 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
                  ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"((1024u >> 4) | (1u << 14) | (2u << 29)), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-// the loads before have arrived (the values pass through, so that nothing that uses them moves ahead of this)
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-
 // Rows of A -> planes [3, M, pitch].  One block per row: memory-bound, 4 bytes read and 6 written a value (300 rows of 2,048: 2.4 us).
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, int lda, __nv_bfloat16* __restrict__ planes, int M, int K, int pitch) {
     TTIE_PDL_ENTRY();
@@ -199,7 +147,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
         if (h < halves) {
             for (int kb = 0; kb < nkb; ++kb) {
-                bool ok = mbar_wait(BAR(DFULL + h), kb & 1, 41, p);
+                bool ok = mbar_wait(BAR(DFULL + h), kb & 1, 41, p.err);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -255,7 +203,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 for (int i = 0; i < 3 - SPLIT; ++i) {
                     const int h = SPLIT == 2 ? own : i;
                     if (h >= halves || !ok) break;
-                    ok = mbar_wait(BAR(WFULL + s), round & 1, 42, p) && mbar_wait(BAR(AEMPTY + h), (kb & 1) ^ 1, 43, p);
+                    ok = mbar_wait(BAR(WFULL + s), round & 1, 42, p.err) && mbar_wait(BAR(AEMPTY + h), (kb & 1) ^ 1, 43, p.err);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -291,7 +239,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 bool ok = true;
                 for (int kb = 0; kb < nkb && ok; ++kb)
                     for (int h = 0; h < halves; ++h) {
-                        if (!mbar_wait(BAR(WEMPTY + s), (round & 1) ^ 1, 44, p)) { ok = false; break; }
+                        if (!mbar_wait(BAR(WEMPTY + s), (round & 1) ^ 1, 44, p.err)) { ok = false; break; }
                         mbar_expect_tx(BAR(WFULL + s), W_BYTES);
                         const uint32_t dst = w_ring + (uint32_t)s * W_BYTES;
                         tma_load_2d(dst, &tmW, BAR(WFULL + s), (kb0 + kb) * KB, n0 + h * HALF);
@@ -300,7 +248,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                     }
                 // nothing may land in a CTA that has left, and the other roles may have given up (each wait is bounded)
                 for (int i = 0; i < p.w_stages; ++i)
-                    if (round > 0 || i < s) mbar_wait(BAR(WFULL + i), (i < s ? round : round - 1) & 1, 44, p);
+                    if (round > 0 || i < s) mbar_wait(BAR(WFULL + i), (i < s ? round : round - 1) & 1, 44, p.err);
             }
         } else if (warp == ISSUE + 2) {
             if (lane == 0) {
@@ -309,12 +257,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 int kb = 0;
                 for (; kb < nkb; ++kb) {
                     const int s = kb & 1;
-                    if (!mbar_wait(BAR(XEMPTY + s), ((kb >> 1) & 1) ^ 1, 45, p)) break;
+                    if (!mbar_wait(BAR(XEMPTY + s), ((kb >> 1) & 1) ^ 1, 45, p.err)) break;
                     mbar_expect_tx(BAR(XFULL + s), x_stage);
                     for (int i = 0; i < 3; ++i)
                         tma_load_2d(x_ring + (uint32_t)s * x_stage + (uint32_t)i * plane, &tmX, BAR(XFULL + s), (kb0 + kb) * KB, i * p.M + m0);
                 }
-                for (int i = kb - 2 < 0 ? 0 : kb - 2; i < kb; ++i) mbar_wait(BAR(XFULL + (i & 1)), (i >> 1) & 1, 45, p);
+                for (int i = kb - 2 < 0 ? 0 : kb - 2; i < kb; ++i) mbar_wait(BAR(XFULL + (i & 1)), (i >> 1) & 1, 45, p.err);
             }
         } else if (((warp - ISSUE) >> 1) < halves) {
             if (lane == 0) {
@@ -325,8 +273,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 int kb = 0;
                 for (; kb < nkb; ++kb) {
                     const int s = kb & 1;
-                    if (!mbar_wait(BAR(XFULL + s), (kb >> 1) & 1, 46, p)) break;
-                    if (!mbar_wait(BAR(DEMPTY + h), (kb & 1) ^ 1, 48, p) || !mbar_wait(BAR(AFULL + h), kb & 1, 47, p)) break;
+                    if (!mbar_wait(BAR(XFULL + s), (kb >> 1) & 1, 46, p.err)) break;
+                    if (!mbar_wait(BAR(DEMPTY + h), (kb & 1) ^ 1, 48, p.err) || !mbar_wait(BAR(AFULL + h), kb & 1, 47, p.err)) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t b = (((x_ring + (uint32_t)s * x_stage) & 0x3FFFFu) >> 4) | (1u << 16);
 #pragma unroll
@@ -340,7 +288,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                     umma_commit(BAR(XEMPTY + s));
                     umma_commit(BAR(DFULL + h));
                 }
-                if (kb > 0) mbar_wait(BAR(DFULL + h), (kb - 1) & 1, 48, p);      // (its products are done before the CTA frees their tensor memory)
+                if (kb > 0) mbar_wait(BAR(DFULL + h), (kb - 1) & 1, 48, p.err);      // (its products are done before the CTA frees their tensor memory)
             }
         }
         __syncwarp();
@@ -498,7 +446,7 @@ extern "C" int ttie_gemm_f32_tc(const float* A, const float* W, const float* bia
     CUtensorMap mw, mx;
     if (gemm_tc_make_map_of(&mw, 1, W, N, K, ldw, 32, HALF)) return -1;
     if (gemm_tc_make_map_of(&mx, 0, planes, 3LL * M, K, pitch, KB, p.width)) return -1;
-    if (gemm_tc_error_words(&p.err, &p.mirror)) TTIE_FAIL("gemm_f32_tc: the error word's address is not to be had");
+    if (gemm_tc_error_words(&p.err.word, &p.err.mirror)) TTIE_FAIL("gemm_f32_tc: the error word's address is not to be had");
     cudaStream_t s = (cudaStream_t)stream;
     TTIE_LAUNCH(split_rows_kernel, M, 256, 0, s, A, lda, (__nv_bfloat16*)planes, M, K, pitch);
     TTIE_CHECK_LAUNCH("gemm_f32_tc (planes)");

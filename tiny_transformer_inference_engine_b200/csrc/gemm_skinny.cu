@@ -15,15 +15,9 @@
 // depend on timing; (2) SwiGLU: the CTA streams gate rows n and up rows n+F together and writes
 // silu(g)*u (models/mlp.py:24-32; silu in 32-bit as kernels/fused_swiglu/kernel.py:20-25);
 // (3) float32 out (logits).
-#include "common.cuh"
-#include <cuda.h>
+#include "tc_ptx.cuh"
 using namespace ttie;
-
-namespace ttie {
-// the product kernels' error word and its mirror, and the builder of maps over blocks of 64 columns (gemm_tcgen05.cu)
-int gemm_tc_error_words(int** word, int** mirror);
-int gemm_tc_make_block_map(CUtensorMap* map, const void* base, long long rows, long long blocks, long long ld, int box_rows, int box_blocks);
-}  // namespace ttie
+using namespace ttie::tc;
 
 namespace {
 struct SkinnyParams {
@@ -210,34 +204,14 @@ skinny_gemm_kernel(const SkinnyParams p) {
 // the kernel before, whose results they do not depend on.  Four warps split a stage's K among themselves, take their operand fragments from
 // shared memory as the other form takes them from global memory (the swizzle spreads eight rows' 16 bytes over all banks), and add up
 // their ranges at the end of a unit.  Activations through the cache instead of the ring were slower (8 rows: 36 against 31 us).
-constexpr long long WAIT_CYCLES = 2000000000LL;             // about one second
 constexpr int BULK_STAGES_MOST = 8;
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
 struct BulkParams {
     SkinnyParams g;
     int tiles, units, stages, stage_bytes, dynamic;
-    int *err, *mirror;
+    ErrorWords err;
     int quitter;                                             // a multiplying warp whose waits run out at once (tests of giving up), or -1
 };
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code, const BulkParams& p, bool quits = false) {
-    if (!quits && mbar_try(bar, parity)) return true;
-    const long long deadline = clock64() + WAIT_CYCLES;
-    while (quits || !mbar_try(bar, parity)) {
-        if (quits || clock64() > deadline) {
-            atomicCAS(p.err, 0, code);
-            if (p.mirror) { *reinterpret_cast<volatile int*>(p.mirror) = code; __threadfence_system(); }
-            return false;
-        }
-    }
-    return true;
-}
 // Barrier of the 128 multiplying threads, each of which comes here once a unit whether its waits ran out or not: a warp that went away alone
 // would leave the others waiting without a limit.  Tells all of them whether one of them gave up.
 __device__ __forceinline__ bool any_of_128(bool bad) {
@@ -275,10 +249,10 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * BULK_STAGES_MOST, asked = empty0 + 8 * BULK_STAGES_MOST, ring0 = smem_u32(ring);
     if (tid == 0) {
         for (int s = 0; s < bp.stages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(empty0 + 8 * s) : "memory");
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 4);
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(asked) : "memory");
+        mbar_init(asked, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -304,12 +278,12 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
         // a CTA that has not started yet gives its unit to one that has room for it
         auto ask = [&]() {
             open = true;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(asked) : "memory");
+            mbar_expect_tx(asked, 16);
             asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(&next_unit)), "r"(asked) : "memory");
         };
         auto answer = [&]() -> int {                             // its number, or -1: all have started
             open = false;
-            if (!mbar_wait(asked, turn++ & 1, 63, bp)) { ok = false; return -1; }
+            if (!mbar_wait(asked, turn++ & 1, 63, bp.err)) { ok = false; return -1; }
             uint32_t given, x;
             asm volatile("{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tld.shared.b128 h, [%2];\n\t"
                          "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
@@ -325,14 +299,14 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
             range_of(unit, n0, split, k_begin, k_end);
             for (int k0 = k_begin; k0 < k_end; k0 += KS) {
                 if (!waited && ahead == bp.stages) settle();
-                if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, 61, bp);
+                if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, 61, bp.err);
                 if (ok && bp.dynamic && k0 + KS >= k_end) next = answer();
                 if (!ok) break;
                 const uint32_t bar = full0 + 8 * s, dst = ring0 + (uint32_t)s * bp.stage_bytes;
                 stage_unit[s] = unit;
                 stage_k[s] = k0;
                 stage_more[s] = next >= 0;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+                mbar_expect_tx(bar, bytes);
 #pragma unroll
                 for (int i = 0; i < (PAIRED ? 2 : NSET); ++i)    // (rows and blocks past the end are zeros; blocks of the next range are not used)
                     tma_load_3d(dst + i * (PAIRED ? Sh::SET / 2 : Sh::SET), &tmW, bar, n0 + (EPI == 2 ? i * p.up_offset : i * 16), k0 / 64);
@@ -344,14 +318,14 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
         }
         if (!waited) settle();
         // nothing may land in a CTA that has left, and the multiplying warps may have given up (each wait is bounded)
-        for (int i = 0; i < bp.stages; ++i) if (round > 0 || i < s) mbar_wait(full0 + 8 * i, (i < s ? round : round - 1) & 1, 61, bp);
-        if (open) mbar_wait(asked, turn & 1, 63, bp);
+        for (int i = 0; i < bp.stages; ++i) if (round > 0 || i < s) mbar_wait(full0 + 8 * i, (i < s ? round : round - 1) & 1, 61, bp.err);
+        if (open) mbar_wait(asked, turn & 1, 63, bp.err);
         return;
     }
     pdl_wait();                                                  // (so that a wait's limit does not count the time of the kernel before)
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     int s = 0, round = 0;
-    auto arrived = [&]() { return (bool)__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, round & 1, 62, bp, warp == bp.quitter)); };
+    auto arrived = [&]() { return (bool)__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, round & 1, 62, bp.err, warp == bp.quitter)); };
     auto next_stage = [&]() { if (++s == bp.stages) { s = 0; ++round; } };
     bool more = true;
     for (int turn = 0; more; turn ^= 1) {
@@ -392,7 +366,7 @@ __global__ void __launch_bounds__(160, 2) skinny_bulk_kernel(const __grid_consta
                     }
             }
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty0 + 8 * s) : "memory");
+            if (lane == 0) mbar_arrive(empty0 + 8 * s);
             next_stage();
         }
 #pragma unroll
@@ -423,7 +397,7 @@ int launch_bulk(const SkinnyParams& p, int splits, cudaStream_t s) {
     CUtensorMap mw, mx;
     if (gemm_tc_make_block_map(&mw, p.w, EPI == 2 ? (long long)p.up_offset + p.N : p.N, p.K / 64, p.ldw, EPI == 2 && NSET == 1 ? 8 : 16, Sh::BLOCKS)) return -1;
     if (gemm_tc_make_block_map(&mx, p.x, p.M, p.K / 64, p.ldx, p.M, Sh::BLOCKS)) return -1;
-    if (gemm_tc_error_words(&b.err, &b.mirror)) TTIE_FAIL("skinny_gemm: the error word's address is not to be had");
+    if (gemm_tc_error_words(&b.err.word, &b.err.mirror)) TTIE_FAIL("skinny_gemm: the error word's address is not to be had");
     auto kernel = skinny_bulk_kernel<MT, EPI, SETS>;
     static bool allowed[64] = {false};
     int dev = 64;

@@ -22,16 +22,15 @@
 // Every mbarrier wait is bounded by a clock deadline; one that runs out records a code and the CTA goes on to its end.
 #include "matrix_chunks.cuh"
 #include "planes.cuh"
+#include "tc_ptx.cuh"
 using namespace ttie;
 using namespace ttie::chunks;
-
-namespace ttie { int gemm_tc_error_words(int** word, int** mirror); }
+using namespace ttie::tc;
 
 namespace {
 constexpr int CT = 128, NT = 512, DVP = 128, GROUPS = NT / 128;   // tokens of a chunk, threads, value columns (zeros behind Dv), threads of a row
 constexpr int OWN = 128 / GROUPS;                                // columns of a thread
 constexpr int SLOTS = 4;                                         // sums of a round in tensor memory
-constexpr long long WAIT_CYCLES = 2000000000LL;                 // about one second
 constexpr uint32_t BLOCK = CT * 128;                             // 128 rows of 64 bfloat16, 128-byte swizzle
 
 // a value in 64 bits as the sum of two floats (an infinity: and zero)
@@ -45,34 +44,15 @@ __device__ __forceinline__ float exp_of(double d) {
     const float e = expf(f.x);
     return fmaf(e, f.y, e);
 }
-struct ErrorWords { int* word; int* mirror; };
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool mbar_try(uint32_t bar) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
-    return ok != 0;
-}
-// each barrier here completes once
+// each barrier here completes once; a wait that runs out leaves its code, and the thread goes on
 __device__ __forceinline__ void mbar_wait(uint32_t bar, int code, const ErrorWords& e) {
-    if (!mbar_try(bar)) {
-        const long long deadline = clock64() + WAIT_CYCLES;
-        while (!mbar_try(bar)) {
-            if (clock64() > deadline) {
-                atomicCAS(e.word, 0, code);
-                if (e.mirror) { *reinterpret_cast<volatile int*>(e.mirror) = code; __threadfence_system(); }
-                break;
-            }
-        }
-    }
+    tc::mbar_wait(bar, 0, code, e);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 __device__ __forceinline__ void sync_tc() {                      // a block barrier that also orders tensor memory accesses
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 // Lower words of shared-memory operand descriptors.  K along the row: 64-value blocks, a step of 16 is 32 bytes.  K down the rows: a step
 // of 16 is 2048 bytes, neighbouring 64-column blocks are BLOCK bytes apart.  Upper word: 8-row groups 1024 bytes apart, 128-byte swizzle.
@@ -87,18 +67,6 @@ __device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo
 // D float32, A and B bfloat16; M 128, N columns; which operands have K down the rows
 __host__ __device__ constexpr uint32_t idesc_of(int n, bool a_cols, bool b_cols) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (a_cols ? 1u << 15 : 0u) | (b_cols ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {     // (the values pass through, so that nothing that uses them moves ahead of this)
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
 }
 // A product of two operands of which one has, or both have, three planes, in rounds.  The tensor cores cut bits off where an addition rounds, so the
 // leading planes' products - 16 bits each, 16 of them all but exact together - are summed 16 terms at a time, each 16 from zero in a
@@ -210,7 +178,7 @@ __device__ __forceinline__ void copy_tile(float* dst, long long ld, const float*
 template <int NBARS>
 __device__ __forceinline__ void tc_setup(unsigned long long* bars, uint32_t* slot, uint32_t cols) {      // barriers and tensor memory; ends in a block barrier
     if (threadIdx.x == 32) {
-        for (int i = 0; i < NBARS; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + i)) : "memory");
+        for (int i = 0; i < NBARS; ++i) mbar_init(smem_u32(bars + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < 32) {
