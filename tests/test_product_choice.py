@@ -124,15 +124,16 @@ def test_float32_pieces_cover_the_keys(heads, rows, group, dim, new, keys):
 
 @pytest.mark.parametrize("N,K", [(4352, 4096), (4096, 4096), (4096, 11008), (32000, 4096), (1024, 4096), (256000, 2048), (5120, 1024), (2304, 64 * 31), (8192, 28672)])
 def test_form_of_a_decode_product_comes_from_its_sizes(N, K):
-    """K ranges and row sets of the weight-streaming product: ranges that cover K, the last one not empty, 768 or more; whole where the caller
+    """K ranges and row sets of the weight-streaming product: ranges that cover K, the last one not empty, 512 or more; whole where the caller
     wants whole sums; the same answer every time."""
-    kslice, code = _ring_form(N, K, 148, True)
-    S = -(-K // kslice)
-    assert kslice % 128 == 0 and code in (0, 16) and (S == 1 or K >= 768 * S) and S <= 8 and (S - 1) * kslice < K
-    whole, code = _ring_form(N, K, 148, False)
-    assert whole == -(-K // 128) * 128 and code in (0, 16)
-    _ring_form.cache_clear()
-    assert _ring_form(N, K, 148, True)[0] == kslice
+    for few in (True, False):
+        kslice, code = _ring_form(N, K, 148, True, few)
+        S = -(-K // kslice)
+        assert kslice % 128 == 0 and code in (0, 16) and (S == 1 or K >= 512 * S) and S <= 8 and (S - 1) * kslice < K
+        whole, code = _ring_form(N, K, 148, False, few)
+        assert whole == -(-K // 128) * 128 and code in (0, 16)
+        _ring_form.cache_clear()
+        assert _ring_form(N, K, 148, True, few)[0] == kslice
     if N <= 4352 and K >= 4096:
         assert S >= 2
 

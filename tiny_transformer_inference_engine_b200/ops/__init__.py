@@ -178,27 +178,32 @@ def _floor_sum(n, m, a, b):
 
 
 @functools.lru_cache(maxsize=4096)
-def _ring_form(N, K, num_sms, may_split):
-    """(K range of a CTA, form code) of the weight-streaming product through shared memory for a matrix of 4 Mi elements or more: one
-    or two sets of 16 weight rows a unit, K in 1 to 8 ranges of 768 or more where the caller takes partial sums.  By sizes and not
-    by a stopwatch: the ranges decide the order of the sums, so a choice between forms a few percent apart, made anew in every process,
-    would give other last bits from one to the next (the row sets do not).  The cost: a unit's bytes (its weights, the copies of the activations, a
-    start) times the waves of units on two CTAs an SM, the last one with the fill to the power of 0.4, since fewer CTAs get
-    more of the memory's rate each.  From 2.5 waves of tiles of one set on (2 where K stays whole) these as they are: they are handed on as CTAs come free, so that no last wave
-    is left ([32000, 4096] 38.8 us, two sets 39.5; [12288, 4096] 16.1 and 18.8).  Fitted to 50 shapes of [1024, 4096] to [256000, 2048] at 1, 8
-    and 16 rows: on average 2.3 % above the fastest of 18 to 27 forms (uncut 0.7 % above the faster of two), a tenth at one in twenty, 29 % at worst; at the
-    Llama sizes, us at 1 row and 8: [4352, 4096] 7.3, 7.8 in two ranges of two sets (8.0, 8.5 uncut with one), [4096, 4096] 6.9, 7.7 (7.7, 8.2),
-    [4096, 11008] 15.6, 16.3 (16.2, 16.7)."""
-    if math.ceil(N / 16) >= (5 if may_split else 4) * num_sms:
+def _ring_form(N, K, num_sms, may_split, few=True):
+    """(K range of a CTA, form code) of the weight-streaming product through shared memory: one or two sets of 16 weight rows a unit, K in 1
+    to 8 ranges of 512 or more where the caller takes partial sums.  ``few``: up to 8 rows, else 9 to 16.  By sizes and not by a stopwatch: the
+    ranges decide the order of the sums, so a choice between forms a few percent apart, made anew in every process, would give other
+    last bits from one to the next (the row sets do not).
+
+    The cost: a unit's bytes (its weights, the copies of the activations, a start) times the waves of units on two CTAs an SM, the last one with its
+    fill to the power of 0.35, since fewer CTAs get more of the memory's rate each; a second wave costs nearly a whole one however few
+    its units.  From 2.5 waves of tiles of one set on (2 where K stays whole) these as they are: they are handed on as CTAs come free,
+    so that no last wave is left ([32000, 4096] 38.8 us, two sets 39.5; [12288, 4096] 16.1 and 18.8); with 9 rows and more only up to 3.4 waves
+    ([256000, 2048] at 12 and 16 rows 169 and 174, two sets 154 and 163).  Fitted to 70 shapes of [256, 8192] to [256000, 2048] at 1, 8, 12 and 16
+    rows: on average 3.1 % above the fastest of 12 to 18 forms (uncut 0.3 % above the faster of two), and 6 % faster than the register form in the
+    best of its own, one in twenty more than 3 % slower and none more than 9 %.  At the Llama sizes, us at 1 row and 8: [4352, 4096] 7.3, 7.8 in
+    two ranges of two sets (8.0, 8.5 uncut with one), [4096, 4096] 6.9, 7.7 (7.7, 8.2), [4096, 11008] 15.6, 16.3 (16.2, 16.7)."""
+    tiles = math.ceil(N / 16) / (2 * num_sms)                 # waves of tiles of one set
+    if tiles >= (2.5 if may_split else 2) and (few or tiles < 3.4):
         return math.ceil(K / 128) * 128, 0
     best, best_cost = None, None
     for sets in (1, 2):
         for S in (1, 2, 3, 4, 5, 6, 8) if may_split else (1,):
             kslice = math.ceil(math.ceil(K / S) / 128) * 128
-            if S > 1 and (K < 768 * S or math.ceil(K / kslice) != S):
+            if S > 1 and (K < 512 * S or math.ceil(K / kslice) != S):
                 continue
             waves = math.ceil(N / (16 * sets)) * S / (2 * num_sms)
-            cost = (kslice * (16 * sets + 8) + 4000) * (math.floor(waves) + (waves % 1) ** 0.4)
+            whole, last = int(waves), waves % 1
+            cost = (kslice * (16 * sets + (6 if few else 12)) + 12000) * (whole + (last ** (0.05 if whole == 1 else 0.35) if last else 0))
             if best_cost is None or cost < best_cost:
                 best, best_cost = (kslice, 16 * (sets - 1)), cost
     return best
@@ -500,8 +505,8 @@ class CudaOps:
             return out
         may_split = partial_ok and bias is None and out_dtype is None
         if self._skinny_ok(x, w, may_split):
-            if M <= 16 and K % 64 == 0 and N * K >= 4 << 20:
-                kslice, form = _ring_form(N, K, self.num_sms, may_split)
+            if M <= 16 and K % 64 == 0 and N * K >= 1 << 20:
+                kslice, form = _ring_form(N, K, self.num_sms, may_split, M <= 8)
             else:
                 tuned = self._skinny_tuned.get((N, K, 8 if M <= 8 else 16)) if (may_split and M <= 16) else None
                 kslice, form = tuned if tuned is not None else (self._kslice(N, K, may_split), 0)
