@@ -428,7 +428,7 @@ int dispatch(const SkinnyParams& p, int splits, int unroll, cudaStream_t s) {
     const bool two = EPI != 2 && (unroll & 16);
     unroll &= 15;
     const int mt = ceil_div(p.M, 8);
-    // Through shared memory from 1 Mi weights on ([1024, 1024] 1.8 us either way, [512, 2048] 2.5 | 3.3).  us, this form | the other, 1 row and 8:
+    // Through shared memory from 1 Mi weights on ([1024, 1024] in two ranges 1.9 | 2.0, [512, 2048] in four 1.9 | 2.0, whole 2.7 | 3.9).  us, this form | the other, 1 row and 8:
     // [4352, 4096] 6.7 | 7.5, 7.2 | 7.6; [4096, 4096] 6.4 | 6.7, 7.0 | 7.0; gate and up of [22016, 4096] 27.0 | 31.2, 27.5 | 31.6; [4096, 11008]
     // 13.9 | 15.5, 15.0 | 16.2; [32000, 4096] 37.8 | 44.1, 38.8 | 45.4; [256000, 2048] 146 | 145, 147 | 145 (copies alone: 5.5 us for 33 MB,
     // 25.9 for 180, 37.0 for 262).  The gated unit in sets of 8 + 8 rows where these are long enough a unit.  8 + 8 | 16 + 16 at 1 row and 8: [16384, 1024]
