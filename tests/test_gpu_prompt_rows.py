@@ -135,3 +135,30 @@ def test_selective_scan_of_a_mixed_step_in_parts(ops, monkeypatch, lens, I, N):
     (y, S, tail), (y2, S2, tail2) = got
     assert torch.allclose(y.double(), y2.double(), rtol=2.0 ** -7, atol=2e-3 * float(y2.abs().max()))
     assert ((S - S2).norm() / S2.norm()).item() < 2e-5 and torch.equal(tail, tail2)
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("lens,width,wdtype", [([1027], 1024, torch.float32), ([1, 2, 3, 1, 700, 2, 400], 1032, torch.float32), ([5] * 60, 4096, torch.bfloat16), ([130], 8200, torch.bfloat16)])
+def test_causal_conv_in_runs_of_tokens(ops, lens, width, wdtype, taps):
+    """Runs that start inside a request, cross requests and end short, behind state rows, with and without silu and bias; 32-bit sums of five terms
+    (2^-23 each of the largest) and one rounding to bfloat16."""
+    T, R = sum(lens), len(lens)
+    assert T * width >= 1 << 20
+    x = randn(51, T, width + 8).bfloat16()
+    w, b = randn(52, taps, width).to(wdtype), randn(53, width).to(wdtype)
+    state = randn(54, R + 1, max(1, taps - 1), width)
+    qsl = [0]
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    seq = t([r for r, n in enumerate(lens) for _ in range(n)])
+    rows = torch.cat([torch.cat([state[R - 1 - r, :taps - 1].double(), x[qsl[r]:qsl[r + 1], 8:].double()]).unfold(0, taps, 1) for r in range(R)])
+    terms = rows * w.double().t()
+    for bias, act in ((b, "silu"), (None, None), (None, "silu")):
+        u32, u = ops.causal_conv(x, 8, width, taps, w, bias, state, seq, t(qsl), t(list(range(R))[::-1]), True, first_row=0, act=act, want_f32=act is None)
+        e = terms.sum(-1) + (bias.double() if bias is not None else 0.0)
+        slack = 5 * 2.0 ** -23 * (terms.abs().sum(-1) + (bias.double().abs() if bias is not None else 0.0))
+        if u32 is not None:
+            assert ((u32.double() - e).abs() <= slack).all()
+        y = e * torch.sigmoid(e) if act else e
+        assert ((u.double() - y).abs() <= 2.0 ** -8 * y.abs() + 2 * slack + 1e-6).all()
