@@ -137,6 +137,38 @@ def test_selective_scan_of_a_mixed_step_in_parts(ops, monkeypatch, lens, I, N):
     assert ((S - S2).norm() / S2.norm()).item() < 2e-5 and torch.equal(tail, tail2)
 
 
+@pytest.mark.parametrize("lens,I,N,parts", [([2048], 1024, 16, 7), ([1] * 23 + [520], 136, 16, 4), ([259, 64, 65], 132, 16, 4), ([200, 8, 300], 130, 7, 3),
+                                            ([71, 1, 136], 127, 4, 2), ([64 * 5 + 1], 260, 16, 5)])
+def test_selective_scan_with_a_thread_per_channel_at_its_edges(ops, monkeypatch, lens, I, N, parts):
+    """Rows on 16, 8, 4 and 2 bytes, runs of fewer than eight tokens, channels past the last whole CTA, parts whose last one is short, and the
+    last request placed first, against the form with a thread per four states (bfloat16 outputs one rounding apart; states to 2e-5, whose decays come
+    from the hardware's exponential)."""
+    T, R, pad = sum(lens), len(lens), ops.selective_state_pad(N)
+    u, z, low = randn(41, T, I).bfloat16(), randn(42, T, 2 * I).bfloat16()[:, I:], randn(43, T, 2 * N).bfloat16()
+    dt, bias, D, xin = randn(44, T, I), randn(45, I) - 4, randn(46, I), randn(47, T, I).bfloat16()
+    A = torch.zeros(I, pad, device=DEV)
+    A[:, :N] = -torch.exp(randn(48, I, N))
+    S0, tail0 = torch.zeros(R + 1, I, pad, device=DEV), randn(50, R + 1, 3, I)
+    S0[..., :N] = randn(49, R + 1, I, N)
+    qsl = [0]
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    import tiny_transformer_inference_engine_b200.ops as module
+    got = []
+    for wide in (True, False):
+        with monkeypatch.context() as m:
+            m.setattr(ops, "selective_wide", lambda *a: wide)
+            if wide:
+                m.setattr(ops, "selective_parts", lambda *a: parts)
+                m.setattr(module, "_even_parts", lambda *a: parts)
+            S, tail = S0.clone(), tail0.clone()
+            got.append((ops.selective_scan(u, dt, bias, A, D, low, 0, N, z, S, xin, tail, 4, t(qsl), t(list(range(R))[::-1]), R, N, max_q_len=max(lens)), S, tail))
+    (y, S, tail), (y2, S2, tail2) = got
+    assert torch.allclose(y.double(), y2.double(), rtol=2.0 ** -7, atol=2e-3 * float(y2.abs().max()))
+    assert ((S - S2).norm() / S2.norm()).item() < 2e-5 and torch.equal(tail, tail2) and torch.equal(S[R], S0[R])
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
 @pytest.mark.parametrize("lens,width,wdtype", [([1027], 1024, torch.float32), ([1, 2, 3, 1, 700, 2, 400], 1032, torch.float32), ([5] * 60, 4096, torch.bfloat16), ([130], 8200, torch.bfloat16)])
 def test_causal_conv_in_runs_of_tokens(ops, lens, width, wdtype, taps):

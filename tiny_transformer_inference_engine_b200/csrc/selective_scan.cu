@@ -42,13 +42,15 @@ template <typename T> struct Act {
     static __device__ __forceinline__ float softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
     static __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }
 };
+__device__ __forceinline__ float lg2(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 template <> struct Act<__nv_bfloat16> {
     static __device__ __forceinline__ float softplus(float x) {
-        const float e = __expf(-fabsf(x));
+        const float e = ex2(-1.4426950408889634f * fabsf(x));
         const float small = e * fmaf(e, fmaf(e, 0.33333334f, -0.5f), 1.0f);
-        return fmaxf(x, 0.f) + (e < 0.01f ? small : __logf(1.0f + e));
+        return fmaxf(x, 0.f) + (e < 0.01f ? small : 0.6931471805599453f * lg2(1.0f + e));
     }
-    static __device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+    static __device__ __forceinline__ float silu(float x) { return x * rcp(1.0f + ex2(-1.4426950408889634f * x)); }
 };
 template <typename T> struct Decay {
     static __device__ __forceinline__ float hold(float a) { return a; }
@@ -73,6 +75,7 @@ struct SelArgs {
     void* out;                                                        // [T, I] compute dtype
     int I, N, Np;
     float* scratch; float* scratch_dt; int parts, mode;               // [requests * parts, I, Np], [requests * parts, I]
+    int copies16, pairs;                                              // u, dt and z rows lie on 16 bytes (channels a multiple of 8); pairs of u and z on 4 (an even number)
 };
 
 template <int SL> __device__ __forceinline__ float slices_sum(float v) {
@@ -281,10 +284,13 @@ __global__ void __launch_bounds__(NT) selective_scan_kernel(const SelArgs a) {
 // What a token costs besides its states - loads, softplus, silu, the store - is then paid once per channel instead of being
 // dealt out to the lanes of a channel with shuffles and predicates (that was seven of twelve instructions per state), rows
 // of a warp's 32 channels are 64 and 128 contiguous bytes, and the states' multiplications go in pairs (one instruction for two;
-// the exponentials have no such form).  B and C of a run of tokens lie in shared memory, which every thread reads at
-// the same address.  The next run's values are in registers while this one is computed.  What bounds
-// it is the exponential unit: 16 a token for the states and five for softplus and silu, 73 us for the two walks of 2,048 tokens of
-// 4,096 channels, which take 117 (141 with a thread per four states).
+// the exponentials have no such form).  Step sizes, inputs and gates travel into shared memory by asynchronous copies three runs ahead, B
+// and C of a run lie there widened, read by every thread at the same address; so a thread's registers are its states and the
+// values of several tokens at once: a whole run is straight-line code in which the next tokens' exponentials go ahead of this one's sums (with a branch per
+// token and the next run in registers 117 us, so 101 in as many parts, with the parts of _even_parts 99; two walks of 2,048 tokens of 4,096 channels).
+// What bounds it: without the states' exponentials 72 us, with nothing but loads, sums and loop 65; the exponential unit alone needs 69 (16 a token for the
+// states, four for softplus and silu).  Two channels a thread 139, a quarter of the exponentials as polynomials on the multiply-add pipe 114, more CTAs an SM with fewer
+// registers 105 to 121.
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
@@ -297,96 +303,149 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return d;
 }
 
+// What a CTA's walk keeps in shared memory: STAGES runs of its 128 channels' step sizes (before bias and softplus), inputs and gates, which
+// come from memory three runs ahead, and two runs of B and C, which all CTAs share.
+constexpr int STAGES = 4, WIDE_CTAS = 4;      // runs in shared memory; CTAs of an SM (of 128 registers a thread)
+template <int NS>
+struct __align__(16) WideRuns {
+    float d[STAGES][TB][NT];
+    unsigned short u[STAGES][TB][NT], z[STAGES][TB][NT];
+    float b[2][TB][NS], c[2][TB][NS];
+};
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void copy4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 template <int NS, bool READ>
-__device__ __forceinline__ float wide_walk(const SelArgs& a, int t0, int n, int c, bool cv, const float2 (&A)[NS / 2], float2 (&S)[NS / 2], float (*smem)[2][TB][NS]) {
+__device__ __forceinline__ float wide_walk(const SelArgs& a, int t0, int n, int c, bool cv, const float2 (&A)[NS / 2], float2 (&S)[NS / 2], WideRuns<NS>& w) {
     using T = __nv_bfloat16;
     using Raw = unsigned short;
-    const int cc = cv ? c : 0;
-    const float* dp = a.dt + (size_t)t0 * a.ld_dt + cc;
-    const Raw* up = reinterpret_cast<const Raw*>(a.u) + (size_t)t0 * a.ld_u + cc;
-    const Raw* zp = reinterpret_cast<const Raw*>(a.z) + (size_t)t0 * a.ld_z + cc;
-    const Raw* bc = reinterpret_cast<const Raw*>(a.bc) + (size_t)t0 * a.ld_bc;
-    T* op = reinterpret_cast<T*>(a.out) + (size_t)t0 * a.I + cc;
-    const float bias = a.dt_bias[cc], Dc = a.D[cc];
+    const int tid = threadIdx.x, c0 = c - tid, cc = cv ? c : 0;
+    const float bias = a.dt_bias[cc], Dc = READ ? a.D[cc] : 0.f;
+    T* o = reinterpret_cast<T*>(a.out) + (size_t)t0 * a.I + cc;
     auto wide = [](Raw r) { return __uint_as_float((unsigned)r << 16); };
-    float sum_dt = 0.f, d_next[TB];
-    Raw u_next[TB], z_next[TB];
-    constexpr int PB = (TB * NS + NT - 1) / NT;                      // values of B (and of C) of a run per thread
-    Raw b_next[PB], c_next[PB];
-    auto fetch = [&](int r0, int nb) {
+    // asks for step sizes, inputs and gates of run r (an empty group of copies past the last run)
+    auto fetch = [&](int r) {
+        const int r0 = r * TB, nb = min(TB, n - r0), st = r % STAGES;
+        if (nb > 0) {
+            const float* d = a.dt + (size_t)(t0 + r0) * a.ld_dt + c0;
+            const Raw* u = reinterpret_cast<const Raw*>(a.u) + (size_t)(t0 + r0) * a.ld_u + c0;
+            const Raw* z = reinterpret_cast<const Raw*>(a.z) + (size_t)(t0 + r0) * a.ld_z + c0;
+            if (a.copies16) {
+                const int dk = tid % 32 * 4, uk = tid % 16 * 8;
+                static_assert(NT / 16 == TB, "16 threads a row of inputs");
+                if (c0 + dk < a.I)
 #pragma unroll
-        for (int i = 0; i < PB; ++i) {
-            const int e = i * NT + threadIdx.x, tt = e / NS, k = e % NS;
-            const bool ok = tt < nb && k < a.N;
-            b_next[i] = ok ? bc[(size_t)(r0 + tt) * a.ld_bc + a.col_b + k] : (Raw)0;
-            if (READ) c_next[i] = ok ? bc[(size_t)(r0 + tt) * a.ld_bc + a.col_c + k] : (Raw)0;
-        }
-        const float* d = dp + (size_t)r0 * a.ld_dt;
-        const Raw* u = up + (size_t)r0 * a.ld_u;
-        const Raw* z = zp + (size_t)r0 * a.ld_z;
-#pragma unroll
-        for (int tt = 0; tt < TB; ++tt) {
-            if (tt < nb) {                                            // (the same for every thread)
-                d_next[tt] = *d; u_next[tt] = *u;
-                if (READ) z_next[tt] = *z;
-            }
-            d += a.ld_dt; u += a.ld_u; z += a.ld_z;
-        }
-    };
-    auto settle = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < PB; ++i) {
-            const int e = i * NT + threadIdx.x;
-            if (e < TB * NS) { (&smem[buf][0][0][0])[e] = wide(b_next[i]); if (READ) (&smem[buf][1][0][0])[e] = wide(c_next[i]); }
-        }
-    };
-    fetch(0, min(TB, n));
-    settle(0);
-    __syncthreads();
-    for (int r0 = 0, it = 0; r0 < n; r0 += TB, ++it) {
-        const int nb = min(TB, n - r0), buf = it & 1;
-        float d[TB];
-        Raw u[TB], z[TB];
-#pragma unroll
-        for (int tt = 0; tt < TB; ++tt) { d[tt] = d_next[tt]; u[tt] = u_next[tt]; if (READ) z[tt] = z_next[tt]; }
-        const bool more = r0 + TB < n;
-        if (more) fetch(r0 + TB, min(TB, n - r0 - TB));
-        T* o = op + (size_t)r0 * a.I;
-#pragma unroll
-        for (int tt = 0; tt < TB; ++tt) {
-            if (tt < nb) {
-                const float dt = Act<T>::softplus(d[tt] + bias), uv = wide(u[tt]);
-                const float2 dt2 = make_float2(dt, dt), du2 = make_float2(dt * uv, dt * uv);
-                float2 y2 = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < NS / 2; i += 2) {
-                    const float4 b = *reinterpret_cast<const float4*>(&smem[buf][0][tt][2 * i]);
-                    const float2 e0 = mul2(dt2, A[i]), e1 = mul2(dt2, A[i + 1]);
-                    S[i] = fma2(make_float2(ex2(e0.x), ex2(e0.y)), S[i], mul2(du2, make_float2(b.x, b.y)));
-                    S[i + 1] = fma2(make_float2(ex2(e1.x), ex2(e1.y)), S[i + 1], mul2(du2, make_float2(b.z, b.w)));
-                    if (READ) {
-                        const float4 q = *reinterpret_cast<const float4*>(&smem[buf][1][tt][2 * i]);
-                        y2 = fma2(S[i], make_float2(q.x, q.y), y2);
-                        y2 = fma2(S[i + 1], make_float2(q.z, q.w), y2);
-                    }
+                    for (int tt = tid / 32; tt < TB; tt += NT / 32)
+                        if (tt < nb) copy16(&w.d[st][tt][dk], d + (size_t)tt * a.ld_dt + dk);
+                if (c0 + uk < a.I && tid / 16 < nb) {
+                    copy16(&w.u[st][tid / 16][uk], u + (size_t)(tid / 16) * a.ld_u + uk);
+                    if (READ) copy16(&w.z[st][tid / 16][uk], z + (size_t)(tid / 16) * a.ld_z + uk);
                 }
-                if (READ) {
-                    if (cv) *o = from_f32<T>(fmaf(Dc, uv, y2.x + y2.y) * Act<T>::silu(wide(z[tt])));
-                    o += a.I;
-                } else sum_dt += dt;
+            } else {                                                  // rows that do not lie on 16 bytes: two channels a copy, or one
+#pragma unroll
+                for (int tt = 0; tt < TB; ++tt)
+                    if (tt < nb && cv) copy4(&w.d[st][tt][tid], d + (size_t)tt * a.ld_dt + tid);
+                if (a.pairs) {
+                    const int uk = tid % 64 * 2;
+                    if (c0 + uk < a.I)
+#pragma unroll
+                        for (int tt = tid / 64; tt < TB; tt += NT / 64)
+                            if (tt < nb) {
+                                copy4(&w.u[st][tt][uk], u + (size_t)tt * a.ld_u + uk);
+                                if (READ) copy4(&w.z[st][tt][uk], z + (size_t)tt * a.ld_z + uk);
+                            }
+                } else if (cv) {
+                    Raw ur[TB], zr[TB];
+#pragma unroll
+                    for (int tt = 0; tt < TB; ++tt) {
+                        ur[tt] = tt < nb ? u[(size_t)tt * a.ld_u + tid] : (Raw)0;
+                        if (READ) zr[tt] = tt < nb ? z[(size_t)tt * a.ld_z + tid] : (Raw)0;
+                    }
+#pragma unroll
+                    for (int tt = 0; tt < TB; ++tt) { w.u[st][tt][tid] = ur[tt]; if (READ) w.z[st][tt][tid] = zr[tt]; }
+                }
             }
         }
-        if (more) settle(buf ^ 1);                                    // (read two runs ago, with a barrier since)
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // B and C of a run, through a register each (they are widened)
+    constexpr int PB = (TB * NS + NT - 1) / NT;
+    Raw b_next[PB], c_next[PB];
+    auto fetch_bc = [&](int r) {
+        const int r0 = r * TB, nb = min(TB, n - r0);
+        const Raw* bc = reinterpret_cast<const Raw*>(a.bc) + (size_t)(t0 + r0) * a.ld_bc;
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {
+            const int e = i * NT + tid, tt = e / NS, k = e % NS;
+            const bool ok = tt < nb && k < a.N;
+            b_next[i] = ok ? bc[(size_t)tt * a.ld_bc + a.col_b + k] : (Raw)0;
+            if (READ) c_next[i] = ok ? bc[(size_t)tt * a.ld_bc + a.col_c + k] : (Raw)0;
+        }
+    };
+    // makes run r readable for all threads; what was read before may be overwritten behind it
+    auto settle = [&](int r) {
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {
+            const int e = i * NT + tid;
+            if (e < TB * NS) { (&w.b[r & 1][0][0])[e] = wide(b_next[i]); if (READ) (&w.c[r & 1][0][0])[e] = wide(c_next[i]); }
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();
+    };
+    float sum_dt = 0.f;
+    const int nruns = (n + TB - 1) / TB;
+#pragma unroll
+    for (int r = 0; r < STAGES - 1; ++r) fetch(r);
+    fetch_bc(0);
+    for (int r = 0; r < nruns; ++r) {
+        settle(r);
+        fetch(r + STAGES - 1);                                        // (into the run before r, which every thread has read)
+        if (r + 1 < nruns) fetch_bc(r + 1);
+        const int nb = min(TB, n - r * TB), st = r % STAGES, bb = r & 1;
+        auto token = [&](int tt) {
+            const float dt = Act<T>::softplus(w.d[st][tt][tid] + bias), uv = wide(w.u[st][tt][tid]);
+            const float2 dt2 = make_float2(dt, dt), du2 = make_float2(dt * uv, dt * uv);
+            float2 y2 = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < NS / 2; i += 2) {
+                const float4 b = *reinterpret_cast<const float4*>(&w.b[bb][tt][2 * i]);
+                const float2 e0 = mul2(dt2, A[i]), e1 = mul2(dt2, A[i + 1]);
+                S[i] = fma2(make_float2(ex2(e0.x), ex2(e0.y)), S[i], mul2(du2, make_float2(b.x, b.y)));
+                S[i + 1] = fma2(make_float2(ex2(e1.x), ex2(e1.y)), S[i + 1], mul2(du2, make_float2(b.z, b.w)));
+                if (READ) {
+                    const float4 q = *reinterpret_cast<const float4*>(&w.c[bb][tt][2 * i]);
+                    y2 = fma2(S[i], make_float2(q.x, q.y), y2);
+                    y2 = fma2(S[i + 1], make_float2(q.z, q.w), y2);
+                }
+            }
+            if (READ) {
+                if (cv) *o = from_f32<T>(fmaf(Dc, uv, y2.x + y2.y) * Act<T>::silu(wide(w.z[st][tt][tid])));
+                o += a.I;
+            } else sum_dt += dt;
+        };
+        if (nb == TB) {                                               // (without a branch per token: the next token's loads and exponentials go ahead of this one's sums)
+#pragma unroll
+            for (int tt = 0; tt < TB; ++tt) token(tt);
+        } else {
+#pragma unroll 1
+            for (int tt = 0; tt < nb; ++tt) token(tt);
+        }
     }
     return sum_dt;
 }
 
 template <int NS>
-__global__ void __launch_bounds__(NT) selective_wide_kernel(const SelArgs a) {
+__global__ void __launch_bounds__(NT, WIDE_CTAS) selective_wide_kernel(const SelArgs a) {
     pdl_wait();                                                      // (the successor is let in at the end, as in the other form)
-    __shared__ __align__(16) float smem[2][2][TB][NS];               // two buffers of B and C
-    const int s = blockIdx.y / a.parts, p = blockIdx.y - s * a.parts;
+    __shared__ WideRuns<NS> smem;
+    // the last request first: a prompt portion stands behind the decoded tokens of a step, and its CTAs spread over idle SMs only if they are
+    // the first to be placed (8,192 channels, 23 requests of one token and one of 2,000: 405 us in four parts, now 265)
+    const int y = blockIdx.y / a.parts, s = gridDim.y / a.parts - 1 - y, p = blockIdx.y - y * a.parts;
     const int q0 = a.qsl[s], n = a.qsl[s + 1] - q0;
     int L = n, p_last = 0;                                           // tokens of a part, the part of the request's last token
     if (a.parts > 1 && n > 0) {
@@ -429,12 +488,22 @@ __global__ void __launch_bounds__(NT) selective_wide_kernel(const SelArgs a) {
         sum_dt = wide_walk<NS, false>(a, q0 + p * L, min(L, n - p * L), c, cv, A, S, smem);
     } else {
         load(p_last == 0 ? sp : scratch_at(a.parts - 1), S);         // the state row as it was before the step
-        for (int j = 0; j < p; ++j) {                                // then the parts before this one
-            float2 add[NS / 2];
-            load(scratch_at(j), add);
-            const float sdt = a.scratch_dt[((size_t)s * a.parts + j) * a.I + cc];
+        constexpr int AHEAD = 4;                                     // then the parts before this one, the loads of AHEAD of them at once
+        for (int j0 = 0; j0 < p; j0 += AHEAD) {
+            float2 add[AHEAD][NS / 2];
+            float sdt[AHEAD];
 #pragma unroll
-            for (int i = 0; i < NS / 2; ++i) S[i] = fma2(make_float2(ex2(sdt * A[i].x), ex2(sdt * A[i].y)), S[i], add[i]);
+            for (int k = 0; k < AHEAD; ++k) {
+                const int j = min(j0 + k, p - 1);
+                load(scratch_at(j), add[k]);
+                sdt[k] = a.scratch_dt[((size_t)s * a.parts + j) * a.I + cc];
+            }
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                if (j0 + k >= p) break;
+#pragma unroll
+                for (int i = 0; i < NS / 2; ++i) S[i] = fma2(make_float2(ex2(sdt[k] * A[i].x), ex2(sdt[k] * A[i].y)), S[i], add[k][i]);
+            }
         }
         wide_walk<NS, true>(a, q0 + p * L, min(L, n - p * L), c, cv, A, S, smem);
     }
@@ -474,6 +543,8 @@ extern "C" int ttie_selective_scan(const void* u, long long ld_u, const float* d
     a.u = u; a.ld_u = ld_u; a.dt = dt; a.ld_dt = ld_dt; a.dt_bias = dt_bias; a.A = A; a.D = D; a.bc = bc; a.ld_bc = ld_bc; a.col_b = col_b;
     a.col_c = col_c; a.z = z; a.ld_z = ld_z; a.state = state; a.state_rows = state_rows; a.xin = xin; a.ld_x = ld_x; a.tail = tail;
     a.tail_rows = tail_rows; a.taps = taps; a.qsl = qsl; a.slot_ids = slot_ids; a.out = out; a.I = I; a.N = N;
+    a.copies16 = I % 8 == 0 && ld_u % 8 == 0 && ld_z % 8 == 0 && ld_dt % 4 == 0 && (((uintptr_t)u | (uintptr_t)z | (uintptr_t)dt) & 15) == 0;
+    a.pairs = I % 2 == 0 && ld_u % 2 == 0 && ld_z % 2 == 0 && (((uintptr_t)u | (uintptr_t)z) & 3) == 0;
     const int sl = state_slices(N);
     a.Np = KPT * sl; a.parts = parts; a.scratch = scratch;
     a.scratch_dt = scratch ? scratch + (size_t)num_seqs * parts * I * a.Np : nullptr;

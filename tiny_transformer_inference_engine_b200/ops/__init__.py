@@ -209,6 +209,24 @@ def _ring_form(N, K, num_sms, may_split, few=True):
     return best
 
 
+@functools.lru_cache(maxsize=4096)
+def _even_parts(blocks: float, longest: int, most: int, num_sms: int) -> int:
+    """How many parts, up to ``most``, a selective scan with a thread per channel cuts its requests into: those whose CTAs (one per part and
+    128 channels; ``blocks`` CTAs walk ``longest`` tokens in one part) divide well over the SMs.  k CTAs of an SM take 0.30, 0.46, 0.62 and 0.80 us a
+    token of their parts in both walks together, further ones wait for a place; one part is walked once, in 0.55 of that.  Fitted to 44
+    shapes of 1,024 to 8,192 channels: 1.3 % behind the best number of parts on average, 11 % at most; 4,096 channels and 2,048 tokens 97 us in
+    19 parts, 107 in 32; 2,048 channels 60 in 26, 66 in 32."""
+    best, best_cost = 1, None
+    for p in range(1, most + 1):
+        tokens = longest if p == 1 else max(64, -(-longest // (8 * p)) * 8)
+        k = max(1, math.ceil(blocks * longest / (num_sms * tokens)))
+        full, rest = divmod(k, 4)
+        cost = (0.80 * full + (0.0, 0.30, 0.46, 0.62)[rest]) * tokens * (0.55 if p == 1 else 1.0) + 0.1 * p
+        if best_cost is None or cost < best_cost:
+            best, best_cost = p, cost
+    return best
+
+
 class CudaOps:
     name = "cuda-sm100a"
     num_sms = 148                           # a B200's; what the device says, once there is one
@@ -1363,6 +1381,9 @@ class CudaOps:
         out = torch.empty((T, I), dtype=u.dtype, device=u.device)
         wide = self.selective_wide(u.dtype, T, int(num_seqs), I, int(states), max_q_len)
         parts = self.selective_parts(T, int(num_seqs), I, int(states), wide, max_q_len)
+        if wide and parts > 1:
+            longest = int(max_q_len) if max_q_len is not None else T - (int(num_seqs) - 1)
+            parts = _even_parts(-(-I // 128) * T / longest, longest, parts, self.num_sms)
         scratch = torch.empty(int(num_seqs) * parts * I * (A.shape[1] + 1), dtype=torch.float32, device=u.device) if parts > 1 else None
         self._check(self.lib.ttie_selective_scan(
             _ptr(u), u.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(A), _ptr(D), _ptr(bc), bc.stride(0), int(col_b), int(col_c), _ptr(z),
