@@ -81,6 +81,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
                  "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
@@ -646,12 +650,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 //   warp 15      one thread issues the scores  S(j) = Q K(j)^T  of both tiles, as soon as K(j) is there and P(j-2) is used up
 // Register budgets follow the roles (setmaxnreg).  Threads of one role run up to two steps apart, so every barrier
 // that counts thread arrivals exists twice (by step parity).
+//
+// ONE tile per CTA (head size 256, joint rows of 512): warps 4-7 take the odd steps of the tile and warps 0-3 the even ones, and the four score buffers
+// are all the tile's, so scores run up to four steps ahead of the products.  With two buffers a buffer's round - scores, their way to
+// the softmax threads, softmax, its way back, product - takes 3,800 clocks for two steps, whatever the tensor core could do meanwhile (clock
+// stamps of one CTA; handing a barrier over costs 200-450 each time); with four the tensor core is busy 1,310 of 1,540 clocks a step (16 products of
+// 128 x 64 x 16 at 50 clocks, with the queries in shared or in tensor memory alike; 4 of 128 x 256 x 16 at 128).  8 heads of 256: 8,192 tokens 271 -> 227 us,
+// 2,048 tokens 43.5 -> 37.2, the last 512 of 6,144 in four pieces 41.8 -> 37.5, 15 decoding requests behind 6,200 keys 24.3 -> 23.1.
+// What bounds two tiles: the thread that issues the scores, 850 clocks a tile and step (it is blocked until its products are through).
 namespace pp {
 constexpr int BNK = 64;                                          // keys per step
 constexpr int NS = 8;                                            // stages of the key/value ring (head size 256: 4 of them, of twice the size)
 constexpr int NS_MOST = 11;                                      // the longest ring of any form
 enum { PP_FULL = 0, PP_EMPTY = NS_MOST, PP_SF = 2 * NS_MOST, PP_PF = PP_SF + 4, PP_SC = PP_PF + 4, PP_OC = PP_SC + 4, PP_OF = PP_OC + 4,
-       PP_LF = PP_OF + 4, PP_NBARS = PP_LF + 2 };                // SF, PF, SC, OC, OF: [tile][step parity]
+       PP_LF = PP_OF + 4, PP_NBARS = PP_LF + 2 };                // SF, PF, SC, OC, OF: [buffer], [tile][step parity] or, with one tile, [step % 4]
 constexpr int PP_NTHREADS = 512;
 // What 227 KB leave beside NT query tiles: with two tiles of 256-column rows, or one of 512, a key tile travels as two or four
 // entries of the ring (128 columns each), so that five entries of 16 KB fit.  QR: rows of a query tile that are staged - a step of
@@ -698,15 +710,22 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     constexpr uint32_t QBLK = QR * 128, KVBLK = BNK * 128;       // bytes of one 64-column block of a query / key tile
     constexpr uint32_t QT_BYTES = CB * QBLK, KV_BYTES = entry_blocks(D, DO, NT) * KVBLK, K_BYTES = CBK * KVBLK, V_BYTES = CBV * KVBLK;
     constexpr uint32_t TMEM_COLS = 512;
-    constexpr uint32_t S_COL = 0, O_COL = 256;                   // scores of (tile t, buffer b) at t * 128 + b * 64; output of tile t at 256 + t * DO
+    constexpr uint32_t S_COL = 0, O_COL = 256;                   // score buffers of 64 columns; output of tile t at 256 + t * DO
+    // Score buffers, and the barriers that go with them: two per tile of two tiles (by step parity), four of one.  `slot` is the buffer of step j
+    // of tile t, `phase` the parity of its use, and step j + REUSE comes to the same buffer.
+    constexpr int REUSE = NT == 2 ? 2 : 4;
+    auto slot = [](int t, int j) { return REUSE == 2 ? 2 * t + (j & 1) : j & 3; };
+    auto phase = [](int j) -> uint32_t { return REUSE == 2 ? (j >> 1) & 1 : (j >> 2) & 1; };
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     unsigned char* Qs = smem;                                    // [NT tiles]
     unsigned char* ring = Qs + NT * QT_BYTES;                    // [NSD stages]
     __shared__ __align__(8) unsigned long long bars[PP_NBARS];
     __shared__ uint32_t tmem_slot;
-    __shared__ float alpha_s[2][2][BM];                          // [step parity][tile]: factor for a row of O before the step's product is added
-    __shared__ float lsum_s[2][BM], mrun_s[2][BM];               // a row's sum and the maximum it is relative to, at the end
+    __shared__ int rows_s[64];                                   // the page rows of the next tiles
+    __shared__ float alpha_s[4][BM];                             // [slot]: factor for a row of O before the step's product is added
+    __shared__ float mref_s[NT == 2 ? 1 : 4][BM];                // one tile: the maximum in use behind the slot's step
+    __shared__ float lsum_s[2][BM], mrun_s[2][BM];               // a row's sum and the maximum it is relative to, at the end ([tile], or [which four warps] of one tile)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.Hq / p.Hkv;
@@ -779,7 +798,9 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     if (warp < 8) {
         // ---------------------------------------------------------------- softmax of tile t, one thread per row
         asm volatile("setmaxnreg.inc.sync.aligned.u32 192;" ::: "memory");
-        const int t = warp >> 2;
+        // (one tile: its even steps are warps 0-3's, its odd ones warps 4-7's; the maximum in use passes from step to step through shared memory,
+        // each side keeps the sum of its own steps)
+        const int side = warp >> 2, t = NT == 2 ? side : 0;
         if (t < ntq) {
             const int quarter = warp & 3, r = quarter * 32 + lane;
             const int row = row0 + t * BM + r;
@@ -787,16 +808,15 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             const int tok = valid ? row / G : 0;
             const int pos = valid ? ctx + tok : -1;
             const int lo = first_visible_key(pos, p.window, p.chunk);
-            const uint32_t s_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + S_COL + (uint32_t)t * 128;
+            const uint32_t s_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + S_COL;
             const float sl2 = p.scale_log2;
             float m_run = -INFINITY, l_run = 0.f;
             const float hb2 = (p.sigmoid && p.head_bias && valid) ? p.head_bias[kvh * G + (row - tok * G)] * 1.4426950408889634f : 0.f;
             bool ok = true;
-            for (int j = 0; j < nsteps; ++j) {
-                const int b = j & 1;
-                const uint32_t par = (j >> 1) & 1;
+            for (int j = NT == 2 ? 0 : side; j < nsteps; j += NT == 2 ? 1 : 2) {
+                const int b = slot(t, j);
                 const uint32_t s_addr = s_base + (uint32_t)b * BNK;
-                ok = mbar_wait(BAR(PP_SF + 2 * t + b), par, 8);
+                ok = mbar_wait(BAR(PP_SF + b), phase(j), 8);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -827,12 +847,24 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                                        fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]))) * sl2;   // -inf stays -inf (the scale is positive)
                 // The maximum in use moves only when it has grown by more than the threshold (or was -inf): then the
                 // row of O is scaled by alpha before this step's product is added.
-                const float m_cand = fmaxf(m_run, mx);
-                const bool up = !p.sigmoid && (m_cand - m_run) > RESCALE_LOG2;   // false for -inf - -inf (NaN); sigmoid weights: never
-                const float alpha = up ? ex2(m_run - m_cand) : 1.f;
-                m_run = up ? m_cand : m_run;
-                alpha_s[b][t][r] = j > 0 ? alpha : 1.f;                      // nothing to scale before the first product
-                mbar_arrive(BAR(PP_SC + 2 * t + b));
+                float m_prev = m_run;
+                if constexpr (NT == 1) {
+                    if (j > 0) {                                             // the other side's decision of the step before
+                        ok = mbar_wait(BAR(PP_SC + slot(t, j - 1)), phase(j - 1), 11);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        m_prev = mref_s[slot(t, j - 1)][r];
+                    }
+                }
+                const float m_cand = fmaxf(m_prev, mx);
+                const bool up = !p.sigmoid && (m_cand - m_prev) > RESCALE_LOG2;   // false for -inf - -inf (NaN); sigmoid weights: never
+                const float step_alpha = up ? ex2(m_prev - m_cand) : 1.f;
+                const float m_new = up ? m_cand : m_prev;
+                const float alpha = NT == 2 ? step_alpha : m_new == m_run ? 1.f : ex2(m_run - m_new);   // for this side's sum (m_run -inf: 0)
+                m_run = m_new;
+                alpha_s[b][r] = j > 0 ? step_alpha : 1.f;                    // nothing to scale before the first product
+                if constexpr (NT == 1) mref_s[b][r] = m_new;
+                mbar_arrive(BAR(PP_SC + b));
                 const float msub = m_run == -INFINITY ? 0.f : m_run;
                 float ls4[4] = {0.f, 0.f, 0.f, 0.f};
                 const float nmsub = -msub;
@@ -862,13 +894,13 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(BAR(PP_PF + 2 * t + b));                     // P is in tensor memory
+                mbar_arrive(BAR(PP_PF + b));                             // P is in tensor memory
                 l_run = l_run * alpha + ((ls4[0] + ls4[1]) + (ls4[2] + ls4[3]));
             }
             if (ok) {                                                    // (sigmoid weights: the pieces of a cut key range simply add)
-                lsum_s[t][r] = p.sigmoid ? (p.num_splits > 1 ? 1.0f / (float)p.num_splits : 1.f) : l_run;
-                mrun_s[t][r] = p.sigmoid ? 0.f : m_run;
-                mbar_arrive(BAR(PP_LF + t));
+                lsum_s[side][r] = p.sigmoid ? (NT == 1 && side ? 0.f : p.num_splits > 1 ? 1.0f / (float)p.num_splits : 1.f) : l_run;
+                mrun_s[side][r] = p.sigmoid ? 0.f : m_run;
+                mbar_arrive(BAR(PP_LF + side));
             }
         }
     } else if (warp < 12) {
@@ -882,16 +914,15 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         // signal two barriers in turn (by step parity): whoever waits for product j is then at most one phase of
         // that barrier away from it.
         auto product_done = [&](int t, int j) -> bool {         // waits until product j of tile t has landed
-            return __all_sync(0xffffffffu, mbar_wait(BAR(PP_OF + 2 * t + (j & 1)), (j >> 1) & 1, 10));
+            return __all_sync(0xffffffffu, mbar_wait(BAR(PP_OF + slot(t, j)), phase(j), 10));
         };
         for (int j = 0; j < nsteps && ok; ++j) {
-            const int b = j & 1;
-            const uint32_t par = (j >> 1) & 1;
             for (int t = 0; t < ntq; ++t) {
-                ok = mbar_wait(BAR(PP_SC + 2 * t + b), par, 9);
+                const int b = slot(t, j);
+                ok = mbar_wait(BAR(PP_SC + b), phase(j), 9);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const float a = alpha_s[b][t][r];
+                const float a = alpha_s[b][r];
                 if (__any_sync(0xffffffffu, a != 1.f)) {                // never in step 0
                     ok = product_done(t, j - 1);                        // the product of the step before has landed
                     if (!ok) break;
@@ -908,11 +939,11 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(BAR(PP_OC + 2 * t + b));
+                mbar_arrive(BAR(PP_OC + b));
             }
         }
         for (int t = 0; t < ntq && ok; ++t) {
-            ok = mbar_wait(BAR(PP_LF + t), 0, 12);
+            ok = mbar_wait(BAR(PP_LF + t), 0, 12) && (NT == 2 || mbar_wait(BAR(PP_LF + 1), 0, 12));
             ok = __all_sync(0xffffffffu, ok);
             if (ok) ok = product_done(t, nsteps - 1);
             if (!ok) break;
@@ -921,7 +952,12 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             const bool valid = row < nrows;
             const int tok = valid ? row / G : 0, g = valid ? row - tok * G : 0;
             const size_t grow = (size_t)(q0 + tok) * p.Hq + kvh * G + g;
-            const float l_tot = lsum_s[t][r];
+            float l_tot = lsum_s[t][r], m_tot = mrun_s[t][r];
+            if constexpr (NT == 1) {                                 // the sides' sums, relative to the later (larger) maximum: the last step's
+                const float m_even = m_tot, m_odd = nsteps > 1 ? mrun_s[1][r] : m_even;
+                m_tot = (nsteps - 1) & 1 ? m_odd : m_even;
+                l_tot = (m_even == m_tot ? l_tot : l_tot * ex2(m_even - m_tot)) + (m_odd == m_tot ? lsum_s[1][r] : lsum_s[1][r] * ex2(m_odd - m_tot));
+            }
             const bool partial = p.num_splits > 1;
             const float inv = partial ? 1.f : (l_tot > 0.f ? 1.f / l_tot : 0.f);
             const int ow = p.out_width(DO), oc = valid ? p.out_col0(kvh * G + g) : 0;
@@ -953,7 +989,7 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             }
             if (valid && partial) {
                 float* ml = p.ws_ml + (grow * p.num_splits + split) * 2;
-                ml[0] = mrun_s[t][r] * 0.6931471805599453f;          // natural-log units for the merge
+                ml[0] = m_tot * 0.6931471805599453f;                 // natural-log units for the merge
                 ml[1] = l_tot;
             }
         }
@@ -978,6 +1014,46 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             };
             int it = 0;                                         // tiles copied so far
             const int v_x = p.joint ? kvh * DO : 0;             // first value column
+            if (nboxes == 1) {
+                // Pages of 64 keys and more: one thread, one copy per entry (a box of the map is 64 columns x 64 keys x the entry's column
+                // blocks), page rows looked up 32 tiles at a time.  What this warp does per entry is on the critical path of every step: its
+                // instructions come through slowly beside the softmax warps, and with a look-up, a warp vote and four copies per entry it took 1,930
+                // clocks a step, whatever the other roles had to do (with half of the bytes, a quarter of the products or no exponentials the
+                // same).
+                bool go = true;
+                uint32_t st = 0, lap = 1;                       // ring entry, parity to wait for
+                auto put = [&](const CUtensorMap* map, int j, int code, uint32_t bytes, int block) -> bool {
+                    if (!mbar_wait_relaxed(BAR(PP_EMPTY + st), lap, code)) return false;
+                    mbar_expect_tx(BAR(PP_FULL + st), bytes);
+                    tma_load_3d(smem_u32(ring) + st * KV_BYTES, map, BAR(PP_FULL + st), 0, rows_s[j & 63], block);
+                    if (++st == NSD) { st = 0; lap ^= 1; }
+                    return true;
+                };
+                auto put_keys = [&](int j) -> bool {
+                    bool ok = true;
+                    for (int part = 0; part < KE && ok; ++part) ok = put(&tmK, j, 1, K_BYTES, part * CBK);
+                    return ok;
+                };
+                auto look_up = [&](int j) {
+                    if (j >= nsteps) return;
+                    const int key = span.key(v_lo + j * BNK), pg = key / ps;
+                    rows_s[j & 63] = p.page_row(pg < p.table_width ? table[pg] : 0, kvh) + (key - pg * ps);
+                };
+                look_up(lane);
+                for (int j0 = 0; j0 < nsteps && go; j0 += 32) {
+                    __syncwarp();                               // (the entries of tiles j0 - 32 .. have been used)
+                    look_up(j0 + 32 + lane);
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (j0 == 0) go = put_keys(0) && (nsteps <= 1 || put_keys(1));
+                        for (int j = j0; j < min(j0 + 32, nsteps) && go; ++j) {
+                            go = put(&tmV, j, 2, V_BYTES, v_x / 64);
+                            if (go && j + 2 < nsteps) go = put_keys(j + 2);
+                        }
+                    }
+                    go = __shfl_sync(0xffffffffu, go, 0);
+                }
+            } else {
             auto emit_entry = [&](const CUtensorMap* map, int y_lane, int code, bool values, int part) -> bool {
                 const int st = it % NSD;
                 int ok = 1;
@@ -1009,6 +1085,7 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 if (go && j + 2 < nsteps) go = emit(&tmK, y2, 1, false);
                 y0 = y1; y1 = y2; y2 = y3;
             }
+            }
         } else if (lane == 0) {
             // ------------------------------------------------------------ product issuers
             // Measured on this part: after a thread has issued tcgen05.mma, its next instruction that touches memory
@@ -1033,7 +1110,6 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     for (int cb = 0; cb < CB; ++cb) q_lo[t][cb] = desc_lo(smem_u32(Qs + t * QT_BYTES + cb * QBLK), 16);
                 const uint32_t ring_k_lo = desc_lo(smem_u32(ring), 16);
                 for (int j = 0; j < nsteps; ++j) {
-                    const int b = j & 1;
                     int st[KE];
                     uint32_t k_lo[KE];
                     bool ok = true;
@@ -1048,10 +1124,11 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
                     for (int t = 0; t < NT; ++t) {
                         if (t < ntq) {
-                            // the buffer holds P(j-2) until its product with V has finished
-                            if (j >= 2 && !mbar_wait(BAR(PP_OF + 2 * t + b), ((j - 2) >> 1) & 1, 4)) { ok = false; break; }
+                            // the buffer holds P(j - REUSE) until its product with V has finished
+                            const int b = slot(t, j);
+                            if (j >= REUSE && !mbar_wait(BAR(PP_OF + b), phase(j - REUSE), 4)) { ok = false; break; }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t d = tmem_base + S_COL + (uint32_t)t * 128 + (uint32_t)b * BNK;
+                            const uint32_t d = tmem_base + S_COL + (uint32_t)b * BNK;
 #pragma unroll
                             for (int cb = 0; cb < CB; ++cb)
 #pragma unroll
@@ -1060,7 +1137,7 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                                     if (cb | k) umma_ss_lean<true>(d, q_lo[t][cb] + 2 * k, kb, idesc_s);
                                     else umma_ss_lean<false>(d, q_lo[t][cb] + 2 * k, kb, idesc_s);
                                 }
-                            umma_commit(BAR(PP_SF + 2 * t + b));
+                            umma_commit(BAR(PP_SF + b));
 #pragma unroll
                             for (int e = 0; e < KE; ++e) umma_commit(BAR(PP_EMPTY + st[e]));           // one arrival per tile in use
                         }
@@ -1070,14 +1147,14 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             } else if (warp - 13 < ntq) {
                 const int t = warp - 13;
                 const uint32_t ring_v_lo = desc_lo(smem_u32(ring), KVBLK);
-                const uint32_t s_tmem = tmem_base + S_COL + (uint32_t)t * 128, o_tmem = tmem_base + O_COL + (uint32_t)t * DO;
+                const uint32_t s_tmem = tmem_base + S_COL, o_tmem = tmem_base + O_COL + (uint32_t)t * DO;
                 for (int j = 0; j < nsteps; ++j) {
-                    const int b = j & 1, idx = v_index(j), st = idx % NSD;
-                    const uint32_t par = (j >> 1) & 1;
+                    const int b = slot(t, j), idx = v_index(j), st = idx % NSD;
+                    const uint32_t par = phase(j);
                     // the copy is waited for last: with P there its keys were, so the entry's barrier is at most a phase behind
                     // (short rings: on its first lap a wait for the second lap's parity would pass)
-                    if (!mbar_wait(BAR(PP_PF + 2 * t + b), par, 7)) break;
-                    if (!mbar_wait(BAR(PP_OC + 2 * t + b), par, 6)) break;
+                    if (!mbar_wait(BAR(PP_PF + b), par, 7)) break;
+                    if (!mbar_wait(BAR(PP_OC + b), par, 6)) break;
                     if (!mbar_wait(BAR(PP_FULL + st), (idx / NSD) & 1, 5)) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t v_lo = ring_v_lo + (uint32_t)st * (KV_BYTES >> 4);
@@ -1086,7 +1163,7 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     else umma_ts_lean<false>(o_tmem, p_tmem, v_lo, idesc_o);
 #pragma unroll
                     for (int k = 1; k < BNK / 16; ++k) umma_ts_lean<true>(o_tmem, p_tmem + (uint32_t)(k * 8), v_lo + k * 128, idesc_o);   // 16 keys = 2048 bytes on
-                    umma_commit(BAR(PP_OF + 2 * t + b));
+                    umma_commit(BAR(PP_OF + b));
                     umma_commit(BAR(PP_EMPTY + st));
                 }
             }
@@ -1116,29 +1193,30 @@ EncodeTiledFn encode_fn() {
 // pages [num_pages][Hkv][page][D] seen as a matrix [num_pages*Hkv*page][D]; box = 64 columns x box_rows keys.
 // A pool keeps its address for the life of an engine and every layer of every step asks for the same few maps, so the
 // last ones made are kept (per host thread) and an encode is paid once per pool, layer and kernel form.
-int encode_page_map(CUtensorMap* map, const void* base, long long rows, int D, int box_rows);
-int make_page_map(CUtensorMap* map, const void* base, long long rows, int D, int box_rows) {
-    struct Kept { const void* base; long long rows; int D, box_rows; CUtensorMap map; };
+// blocks > 0: seen as [num_pages*Hkv*page][D / 64][64] with boxes of 64 columns x box_rows keys x `blocks` column blocks, which a copy leaves block after block.
+int encode_page_map(CUtensorMap* map, const void* base, long long rows, int D, int box_rows, int blocks);
+int make_page_map(CUtensorMap* map, const void* base, long long rows, int D, int box_rows, int blocks = 0) {
+    struct Kept { const void* base; long long rows; int D, box_rows, blocks; CUtensorMap map; };
     constexpr int KEEP = 256;
     thread_local Kept kept[KEEP];
     thread_local int used = 0, next = 0;
     for (int i = 0; i < used; ++i)
-        if (kept[i].base == base && kept[i].rows == rows && kept[i].D == D && kept[i].box_rows == box_rows) { *map = kept[i].map; return 0; }
-    if (encode_page_map(map, base, rows, D, box_rows)) return -1;
+        if (kept[i].base == base && kept[i].rows == rows && kept[i].D == D && kept[i].box_rows == box_rows && kept[i].blocks == blocks) { *map = kept[i].map; return 0; }
+    if (encode_page_map(map, base, rows, D, box_rows, blocks)) return -1;
     Kept& k = kept[next];
-    k.base = base; k.rows = rows; k.D = D; k.box_rows = box_rows; k.map = *map;
+    k.base = base; k.rows = rows; k.D = D; k.box_rows = box_rows; k.blocks = blocks; k.map = *map;
     next = (next + 1) % KEEP;
     if (used < KEEP) ++used;
     return 0;
 }
-int encode_page_map(CUtensorMap* map, const void* base, long long rows, int D, int box_rows) {
+int encode_page_map(CUtensorMap* map, const void* base, long long rows, int D, int box_rows, int blocks) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) TTIE_FAIL("attention_tc: cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)D * 2};
-    cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    cuuint64_t dims[3] = {blocks ? 64u : (cuuint64_t)D, (cuuint64_t)rows, (cuuint64_t)(D / 64)};
+    cuuint64_t strides[2] = {(cuuint64_t)D * 2, 128};
+    cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, (cuuint32_t)blocks};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, blocks ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) TTIE_FAIL("attention_tc: cuTensorMapEncodeTiled failed with code %d", (int)r);
@@ -1276,8 +1354,11 @@ extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride
     const long long rows = (long long)num_pages * (joint ? 1 : Hkv) * page_size;
     const int tile_keys = two_tiles ? pp::BNK : BN;              // keys per copy tile of the kernel
     const int box_rows = page_size < tile_keys ? page_size : tile_keys;
-    if (make_page_map(&mk, k_pages, rows, D, box_rows)) return -1;
-    if (make_page_map(&mv, v_pages, rows, D, box_rows)) return -1;
+    // the prompt-portion form copies whole ring entries where a page holds a tile's keys
+    const bool whole = two_tiles && page_size >= pp::BNK;
+    const int nt = D > 256 || (D > 128 && !joint) ? 1 : 2;
+    if (make_page_map(&mk, k_pages, rows, D, box_rows, whole ? D / 64 / pp::key_entries(D, nt) : 0)) return -1;
+    if (make_page_map(&mv, v_pages, rows, D, box_rows, whole ? (joint ? joint : D) / 64 : 0)) return -1;
     AttnTcParams p;
     p.q = (const __nv_bfloat16*)q; p.q_stride = q_stride; p.block_table = block_table; p.table_width = table_width;
     p.page_size = page_size; p.qsl = qsl; p.seq_lens = seq_lens; p.out = (__nv_bfloat16*)out;
