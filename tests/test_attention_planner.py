@@ -124,3 +124,23 @@ def test_portions_are_cut_within_one_wave_and_only_behind_a_context():
                         assert n == 1, (kernel, n, split_len)
                     if n > 1:
                         assert tiles * n <= 148, (seqs, q_len, kv_len, heads, head_dim, kernel, n)
+
+
+def test_one_launch_for_decoded_tokens_and_portions():
+    """Head size 256 only, with one row tile for each leading request; the pieces cover the longest key range; a step where the portion's few keys
+    would be cut as often as the decoding requests' many keeps a launch for each."""
+    import types
+
+    import torch
+    from tiny_transformer_inference_engine_b200.ops import CudaOps
+    ops = CudaOps.__new__(CudaOps)
+    ops.num_sms, ops._plans = 148, {}
+    ops.lib = types.SimpleNamespace(ttie_attn_tc_supported=lambda d, page: d in (64, 128, 256) and page % 8 == 0)
+    bf, lead, others = torch.bfloat16, (15, 1, 6200, 15), (1, 512, 6144, 512)
+    kernel, pieces, length = ops.mixed_plan(bf, 8, 1, 256, 64, lead, others)
+    assert kernel == "tcpp" and (pieces - 1) * length < 6200 <= pieces * length and length % 128 == 0
+    assert ops.mixed_plan(bf, 8, 1, 256, 64, (1, 1, 128, 1), (1, 128, 128, 128)) == ("tcpp", 1, 0)
+    assert ops.mixed_plan(bf, 8, 1, 256, 64, lead, (1, 512, 512, 512)) is None
+    for args in ((torch.float32, 8, 1, 256, 64, lead, others), (bf, 32, 1, 128, 64, lead, others), (bf, 8, 1, 256, 60, lead, others),
+                 (bf, 8, 1, 256, 64, (15, 17, 6200, 255), others), (bf, 8, 1, 256, 64, lead, (1, 16, 6144, 16))):
+        assert ops.mixed_plan(*args) is None

@@ -157,6 +157,7 @@ struct AttnTcParams {
     const int* qsl; const int* seq_lens;
     __nv_bfloat16* out;
     int num_seqs, Hq, Hkv;
+    int lead;                                                    // two-tile kernel: so many first requests have one row tile each (decoded tokens before prompt portions)
     float scale_log2; int window, chunk, keep;                   // keep: first tokens of the sequence that stay visible behind a window
     float cap_in, cap_out;                                       // score softcap: raw score s becomes cap_out * tanh(s * cap_in) (cap_in 0: none)
     int row_tiles;
@@ -729,10 +730,13 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.Hq / p.Hkv;
+    // CTAs: the row tiles of the requests behind the first `lead`, long (late) tiles first, then one tile for each of those
     int tile = blockIdx.x;
-    const int rt = p.row_tiles - 1 - tile % p.row_tiles;         // long (late) tiles first
-    tile /= p.row_tiles;
-    const int kvh = tile % p.Hkv, seq = tile / p.Hkv;
+    const int longs = (p.num_seqs - p.lead) * p.Hkv * p.row_tiles;
+    const bool led = tile >= longs;
+    const int rt = led ? 0 : p.row_tiles - 1 - tile % p.row_tiles;
+    tile = led ? tile - longs : tile / p.row_tiles;
+    const int kvh = tile % p.Hkv, seq = tile / p.Hkv + (led ? 0 : p.lead);
     const int q0 = p.qsl[seq], q_len = p.qsl[seq + 1] - q0, kv_len = p.seq_lens[seq];
     const int nrows = q_len * G, row0 = rt * (NT * BM);
     if (row0 >= nrows) return;                                   // uniform over the CTA, before anything is allocated
@@ -1256,7 +1260,7 @@ int launch_pp(const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& 
         if (e != cudaSuccess) TTIE_FAIL("attention_tc: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
         allowed[dev] = true;
     }
-    TTIE_LAUNCH(k, dim3(p.num_seqs * p.Hkv * p.row_tiles, p.num_splits), pp::PP_NTHREADS, smem, s, mk, mv, p);
+    TTIE_LAUNCH(k, dim3(((p.num_seqs - p.lead) * p.row_tiles + p.lead) * p.Hkv, p.num_splits), pp::PP_NTHREADS, smem, s, mk, mv, p);
     TTIE_CHECK_LAUNCH("attention_tc (two query tiles)");
     return 0;
 }
@@ -1315,11 +1319,12 @@ extern "C" int ttie_attn_tc_joint_supported(int W, int dv, int page_size) {
 // Joint rows (one cache head holds the rows of all kv heads side by side; D is that row's width).  dv > 0 (a multiple of 32): with
 // Hkv 1, head h's output is the columns (h / per) * dv .. of its row only; out is [T, Hq, dv].  joint = 64 or 128 (two_tiles only):
 // Hkv row groups, one per kv head, whose values are the columns kvh * joint .. + joint; out is [T, Hq, joint].
+// lead (two_tiles only): the first requests that bring no more rows than a row tile has; they get one row tile each.
 extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                                int num_pages, const int* block_table, int table_width, int page_size, const int* qsl,
                                                const int* seq_lens, void* out, int T, int num_seqs, int Hq, int Hkv, int D,
                                                int max_q_len, float scale, float softcap, int window, int chunk, int keep, int num_splits, int split_len,
-                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, void* stream);
+                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, int lead, void* stream);
 
 extern "C" int ttie_paged_attention_tc(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                        int num_pages, const int* block_table, int table_width, int page_size, const int* qsl,
@@ -1328,14 +1333,14 @@ extern "C" int ttie_paged_attention_tc(const void* q, long long q_stride, const 
                                        int two_tiles, void* stream) {
     return ttie_paged_attention_tc_weights(q, q_stride, k_pages, v_pages, num_pages, block_table, table_width, page_size, qsl, seq_lens, out, T,
                                            num_seqs, Hq, Hkv, D, max_q_len, scale, softcap, window, chunk, 0, num_splits, split_len, scratch,
-                                           two_tiles, 0, nullptr, 0, 1, 0, stream);
+                                           two_tiles, 0, nullptr, 0, 1, 0, 0, stream);
 }
 
 extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                                int num_pages, const int* block_table, int table_width, int page_size, const int* qsl,
                                                const int* seq_lens, void* out, int T, int num_seqs, int Hq, int Hkv, int D,
                                                int max_q_len, float scale, float softcap, int window, int chunk, int keep, int num_splits, int split_len,
-                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, void* stream) {
+                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, int lead, void* stream) {
     if (T <= 0 || num_seqs <= 0) return 0;
     if (weights != 0 && weights != 1) TTIE_FAIL("attention_tc: unknown kind of weights %d", weights);
     if (!joint && !ttie_attn_tc_supported(D, page_size)) TTIE_FAIL("attention_tc: head size %d with pages of %d keys is not supported", D, page_size);
@@ -1347,6 +1352,7 @@ extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride
     if (num_splits > 1 && (split_len <= 0 || split_len % BN || !scratch))
         TTIE_FAIL("attention_tc: splits need scratch and a split length that is a multiple of %d", BN);
     if (num_splits > 65535) TTIE_FAIL("attention_tc: too many splits (%d)", num_splits);
+    if (lead < 0 || lead > num_seqs || (lead && !two_tiles)) TTIE_FAIL("attention_tc: %d leading requests of %d", lead, num_seqs);
     CUtensorMap mk, mv;
     if (dv > 0 && (dv % 32 || per <= 0 || (long long)ceil_div(Hq, per) * dv > D)) TTIE_FAIL("attention_tc: %d value columns per %d heads in rows of %d", dv, per, D);
     if (joint && (!two_tiles || !ttie_attn_tc_joint_supported(D, joint, page_size) || (long long)Hkv * joint > D))
@@ -1362,7 +1368,7 @@ extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride
     AttnTcParams p;
     p.q = (const __nv_bfloat16*)q; p.q_stride = q_stride; p.block_table = block_table; p.table_width = table_width;
     p.page_size = page_size; p.qsl = qsl; p.seq_lens = seq_lens; p.out = (__nv_bfloat16*)out;
-    p.num_seqs = num_seqs; p.Hq = Hq; p.Hkv = Hkv; p.scale_log2 = scale * 1.4426950408889634f; p.window = window; p.chunk = chunk;
+    p.num_seqs = num_seqs; p.lead = lead; p.Hq = Hq; p.Hkv = Hkv; p.scale_log2 = scale * 1.4426950408889634f; p.window = window; p.chunk = chunk;
     p.keep = window > 0 ? keep : 0;
     p.cap_in = softcap > 0.f ? scale / softcap : 0.f; p.cap_out = softcap > 0.f ? softcap / scale : 0.f;
     p.row_tiles = ceil_div(max_q_len * (Hq / Hkv), two_tiles && (D <= 128 || (joint && D <= 256)) ? 2 * BM : BM);

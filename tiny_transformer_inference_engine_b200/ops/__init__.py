@@ -67,7 +67,7 @@ _SIGNATURES = {
                                 _c_void],
     "ttie_paged_attention_tc_weights": [_c_void, _c_ll, _c_void, _c_void, _c_int, _c_void, _c_int, _c_int, _c_void, _c_void, _c_void,
                                         _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_int,
-                                        _c_int, _c_void, _c_int, _c_int, _c_int, _c_void],
+                                        _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_tc": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_tc_pair": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_grouped_gemm_tc": [_c_void, _c_ll, _c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_float,
@@ -909,6 +909,45 @@ class CudaOps:
                 best, best_cost = (("mma", n, split_len) if n > 1 else ("mma", 1, 0)), cost
         return best
 
+    def mixed_plan(self, dtype, num_heads, num_kv_heads, head_dim, page_size, lead, others):
+        """Whether a step of ``lead`` requests (decoded tokens) before ``others`` (prompt portions) takes one attention launch for both, where
+        both kinds run the same kernel (head size 256): the plan, or None.  ``lead`` and ``others``: (requests, most tokens of one, most keys that its
+        rows walk, tokens).  One launch fills the SMs once instead of twice and saves the host a launch and a merge, but every request is
+        cut into the same number of pieces.  Both ways are rated by one model: waves of a CTA per SM at 5 us + 14.5 ns per key of a piece, and for cut
+        ranges 2 us and the partial results' way through memory at 3 TB/s.  Of 21 steps (8 heads of 256; 1 to 100 decoding requests behind 128 to
+        8,000 keys, portions of 80 to 1,000 tokens) 19 were faster in one launch, by a quarter on average (15 requests behind 6,200 keys and 512
+        tokens behind 5,632: 67.1 -> 51.3 us in three pieces; 8 behind 349 and 222 behind 2,954: 40.2 -> 26.8); the model takes 18 of them, none
+        that was slower (15 behind 6,200 and 512 alone 42.4 | 45.5), in pieces 5 % behind the best on average."""
+        key = ("mixed", dtype, num_heads, num_kv_heads, head_dim, page_size, lead, others)
+        plan = self._plans.get(key, False)
+        if plan is False:
+            if len(self._plans) >= 4096:
+                self._plans.clear()
+            plan = self._plans[key] = self._mixed_plan(*key[1:])
+        return plan
+
+    def _mixed_plan(self, dtype, num_heads, num_kv_heads, head_dim, page_size, lead, others):
+        G = num_heads // num_kv_heads
+        if (dtype != torch.bfloat16 or head_dim != 256 or lead[1] * G > 128 or others[1] * G <= 128
+                or not self.lib.ttie_attn_tc_supported(head_dim, page_size)):
+            return None
+        tiles = (lead[0] * num_kv_heads, others[0] * num_kv_heads * math.ceil(others[1] * G / 128))
+
+        def cost(ctas, keys, pieces, tokens):
+            piece = math.ceil(math.ceil(keys / pieces) / 128) * 128 if pieces > 1 else keys
+            return (math.ceil(pieces * ctas / self.num_sms) * (5.0 + 0.0145 * piece)
+                    + (2.0 + tokens * num_heads * pieces * (head_dim + 2) * 8 / 3e6 if pieces > 1 else 0.0))
+        apart = sum(cost(t, c[2], self._tc_wide_plan(c[0], num_kv_heads, c[1] * G, c[2], c[1])[1], c[3]) for t, c in zip(tiles, (lead, others)))
+        best, keys = None, max(lead[2], others[2])
+        for pieces in range(1, min(16, math.ceil(keys / 128)) + 1):
+            piece = math.ceil(math.ceil(keys / pieces) / 128) * 128
+            if pieces > 1 and math.ceil(keys / piece) != pieces:
+                continue                                             # (the same cut as a smaller count)
+            c = cost(sum(tiles), keys, pieces, lead[3] + others[3])
+            if best is None or c < best[0]:
+                best = (c, ("tcpp", pieces, piece if pieces > 1 else 0))
+        return best[1] if best[0] <= apart else None
+
     def _tc_wide_plan(self, num_seqs, num_kv_heads, rows, max_kv_len, max_q_len):
         """Head size 256: every step takes the prompt-portion tcgen05 kernel with one 128-row tile per CTA.  Steps of few
         rows (decoded tokens) have their key range cut by the cost model of the one-tile decode kernel, at 20 ns per key
@@ -1000,7 +1039,7 @@ class CudaOps:
 
     def paged_attention(self, qkv, num_heads, num_kv_heads, head_dim, k_pages, v_pages, block_table, page_size,
                         query_start_loc, seq_lens, num_seqs, max_q_len, max_kv_len, scale, window, out,
-                        plan=None, softcap=0.0, chunk=0, weights="softmax", head_bias=None, keep_first=0, value_cols=None):
+                        plan=None, softcap=0.0, chunk=0, weights="softmax", head_bias=None, keep_first=0, value_cols=None, lead=0):
         """Causal attention of the step's query rows over the paged keys and values.  ``window`` > 0: a row at position p
         sees keys p - window + 1 .. p, and with ``keep_first`` > 0 also the sequence's first ``keep_first`` keys.  ``chunk`` > 0 (instead of a window): a row at position p sees the keys of its own
         chunk of ``chunk`` positions up to p, chunks counted from position 0 of the sequence.  ``softcap`` > 0: a score s
@@ -1008,7 +1047,8 @@ class CudaOps:
         weighs sigmoid(score + head_bias[head]) (``head_bias`` float32 [num_heads] or None) and nothing is normalised over the
         keys; every kernel but the thread-block-cluster decode form computes them.  ``value_cols`` (n, heads): of a value row
         only a piece is a head's own, the columns h // heads * n .. + n, and ``out`` is [T, num_heads * n] (tensor-core kernels: n
-        a multiple of 8, of 32 with tcgen05)."""
+        a multiple of 8, of 32 with tcgen05).  ``lead`` (kernel "tcpp"): so many first requests bring no more rows than a row tile
+        has and get one tile each, whatever the others bring (``mixed_plan``)."""
         if weights not in ("softmax", "sigmoid"):
             raise KernelError(f"paged_attention: unknown kind of weights {weights!r}")
         sig = weights == "sigmoid"
@@ -1017,6 +1057,8 @@ class CudaOps:
         T = qkv.shape[0]
         if max_kv_len > block_table.shape[1] * page_size:
             raise KernelError(f"paged_attention: a block table of {block_table.shape[1]} pages of {page_size} keys cannot cover {max_kv_len} keys")
+        if lead and (plan is None or plan[0] != "tcpp"):
+            raise KernelError("paged_attention: leading requests go with the two-tile tcgen05 kernel")
         kernel, num_splits, split_len = plan if plan is not None else self.attention_plan(
             qkv.dtype, num_seqs, num_heads, num_kv_heads, head_dim, max_q_len, self.visible_keys(max_q_len, max_kv_len, window, chunk, keep_first),
             page_size, sig)
@@ -1033,7 +1075,7 @@ class CudaOps:
                 _ptr(qkv), qkv.stride(0), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
                 block_table.shape[1], page_size, _ptr(query_start_loc), _ptr(seq_lens), _ptr(out), T, num_seqs, num_heads,
                 num_kv_heads, head_dim, max_q_len, float(scale), float(softcap or 0.0), int(window), int(chunk), int(keep_first), num_splits, split_len, _ptr(scratch),
-                1 if kernel == "tcpp" else 0, 1 if sig else 0, _ptr(head_bias), dv, per, 0, self._stream(qkv)), "paged_attention_tc")
+                1 if kernel == "tcpp" else 0, 1 if sig else 0, _ptr(head_bias), dv, per, 0, lead, self._stream(qkv)), "paged_attention_tc")
             self.launches += 2 if num_splits > 1 else 1
             return
         form = {"mma": 0, "mma_c2": 2, "mma_c4": 4}.get(kernel)
@@ -1149,7 +1191,7 @@ class CudaOps:
             self._check(self.lib.ttie_paged_attention_tc_weights(
                 _ptr(q), q.stride(0), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.shape[1], page_size,
                 _ptr(query_start_loc), _ptr(seq_lens), _ptr(out), T, num_seqs, num_heads, kv_heads, width, max_q_len, float(scale), 0.0,
-                int(window), int(chunk), int(keep_first), num_splits, split_len, _ptr(scratch), 1, 0, None, 0, 1, v_dim, self._stream(q)),
+                int(window), int(chunk), int(keep_first), num_splits, split_len, _ptr(scratch), 1, 0, None, 0, 1, v_dim, 0, self._stream(q)),
                 "paged_attention_tc (joint rows)")
             self.launches += 2 if num_splits > 1 else 1
             return

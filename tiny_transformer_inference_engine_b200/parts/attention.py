@@ -332,8 +332,21 @@ class PagedAttention(Mixer):
             out = ops.gate_head_rows(out, proj[:, C:] if self.gated else None, Hq, Dv, Dp, per_value=self.gate_per_value)
         return ops.linear(out, self.w_out, None, partial_ok=True)
 
+    def _mixed_plan(self, dtype, D, ctx, cache, classes):
+        """The plan of one attention launch for a step of two classes that lie one behind the other, or None."""
+        plan = getattr(self.ops, "mixed_plan", None)
+        if plan is None or len(classes) != 2:
+            return None
+        a, b = classes
+        if a.seq_lo or a.tok_lo or (a.seq_hi, a.tok_hi) != (b.seq_lo, b.tok_lo) or b.seq_hi != ctx.num_seqs:
+            return None
+        step = [(c.seq_hi - c.seq_lo, c.max_q_len, self.ops.visible_keys(c.max_q_len, c.max_kv_len, self.window or 0, self.chunk or 0, self.keep_first),
+                 c.tok_hi - c.tok_lo) for c in classes]
+        return plan(dtype, self.num_heads, self.num_kv_heads, D, cache.page_size, *step)
+
     def _attend(self, q, D, ctx, cache, out):
-        """One attention launch per class of requests (decoded tokens; prompt portions), each planned as if it were alone."""
+        """One attention launch per class of requests (decoded tokens; prompt portions), each planned as if it were alone, or one for both
+        where the kernel is the same and that is faster."""
         ops, Hq, Hkv = self.ops, self.num_heads, self.num_kv_heads
         extra = {} if self.weights == "softmax" else {"weights": self.weights, "head_bias": self.head_bias}
         if self.keep_first:
@@ -344,6 +357,12 @@ class PagedAttention(Mixer):
             ops.paged_attention(q, Hq, Hkv, D, cache.k_pages, cache.v_pages, cache.block_table, cache.page_size,
                                 c.query_start_loc, ctx.seq_lens, ctx.num_seqs, c.max_q_len, c.max_kv_len,
                                 self.scale, self.window or 0, out, softcap=self.softcap or 0.0, chunk=self.chunk or 0, **extra)
+            return
+        plan = self._mixed_plan(q.dtype, D, ctx, cache, classes)
+        if plan is not None:
+            ops.paged_attention(q, Hq, Hkv, D, cache.k_pages, cache.v_pages, cache.block_table, cache.page_size, ctx.query_start_loc,
+                                ctx.seq_lens, ctx.num_seqs, classes[1].max_q_len, max(c.max_kv_len for c in classes), self.scale, self.window or 0, out,
+                                plan=plan, softcap=self.softcap or 0.0, chunk=self.chunk or 0, lead=classes[0].seq_hi, **extra)
             return
         for ci, c in enumerate(classes):
             views = self._class_views(ctx, cache, ci, c)
