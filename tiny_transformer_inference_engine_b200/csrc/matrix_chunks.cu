@@ -35,14 +35,15 @@
 // partial chunk and needs nothing of the host but the number of tokens and requests.
 //
 // One prompt of 2,048 tokens, us of sum + carry + out: 16 heads of 128 x 128 (retention) 30 + 12 + 69 against the walk's 514; 16 of 64 x 128
-// (mlstm) 16 + 13 + 47 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 41 + 12 + 85 against 473.  What bounds the out kernel is
-// latency: 12 warps per SM fit (168 registers, the planes in shared memory), issue slots 30 % used, the tensor pipe 34 / 16 / 13 %.  With half
-// the threads in wkv's sum (a run of 32 tokens' decays per thread is one serial chain of loads and multiplications in 64 bits) and two blocks
-// of its out per SM instead of three its mixer took 257 us, 240 with them.
+// (mlstm) 16 + 13 + 47 against 413, and 15 for its gates; 32 of 64 x 64 (wkv) 31 + 10 + 48 against 473.  What bounds the out kernels is
+// latency: 12 or 16 warps per SM fit (the planes in shared memory), issue slots 30 % used, the tensor pipe 34 / 16 / 13 %.
+// wkv took 41 + 12 + 85 (116 us in a row, now 89; 16 heads of 128 301, now 237): its CTAs' clocks went to products of decays in 64 bits with their conversions
+// and to loads one run after the other (13,700 of 46,600), and to scores whose 16 sums at a time went through shuffles (16,600).  Now
+// products are pairs of 32-bit numbers, everything a chunk needs is asked for at once by asynchronous copies, a score is a lane's own sum, and the table
+// of decays is the table of the rows' products afterwards, so that four CTAs fit an SM (102 us with three).
 // Error against 64 bits (2-norm; 1,000 tokens, the walk's behind it): read-out 1.0e-7 (2.3e-7), 6.4e-7 (1.1e-6), 8.4e-8 (8.6e-8); state
 // 6.1e-8 (2.0e-7), 1.6e-7 (3.6e-7), 3.4e-8 (4.5e-8).
 #include "matrix_chunks.cuh"
-#include "run_reduce.cuh"
 using namespace ttie;
 using namespace ttie::chunks;
 
@@ -58,13 +59,29 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t&
     p1 = pack(rx, ry);
     p2 = pack(rx - __uint_as_float(p1 << 16), ry - __uint_as_float(p1 & 0xffff0000u));
 }
-// one value known in 64 bits (its third plane keeps what rounding it to 32 would cut)
-__device__ __forceinline__ void split3(double x, uint16_t& p0, uint16_t& p1, uint16_t& p2) {
-    const float hi = (float)x, lo = (float)(x - (double)hi);
-    const __nv_bfloat16 a = __float2bfloat16_rn(hi);
-    const float r = hi - __bfloat162float(a);
+// A product of many decays as a pair of 32-bit numbers whose sum it is, some 46 bits: each multiplication keeps what it rounds (a fused
+// multiply-add gives it exactly) and carries it along.  A chain of them has the latency of 32-bit multiplications; in 64 bits, with the
+// conversions to and fro, the decays of a chunk took a third of a wkv read-out's time.
+struct Pair {
+    float hi, lo;
+    __device__ __forceinline__ void operator*=(float w) {
+        const float p = hi * w;
+        lo = fmaf(lo, w, fmaf(hi, w, -p));
+        hi = p;
+    }
+    __device__ __forceinline__ void operator*=(const Pair& b) {
+        const float p = hi * b.hi;
+        lo = fmaf(lo, b.hi, fmaf(hi, b.lo, fmaf(hi, b.hi, -p)));
+        hi = p;
+    }
+    __device__ __forceinline__ float value() const { return hi + lo; }
+};
+// planes of such a product (its third plane keeps what rounding it to 32 bits would cut)
+__device__ __forceinline__ void split3(const Pair& x, uint16_t& p0, uint16_t& p1, uint16_t& p2) {
+    const __nv_bfloat16 a = __float2bfloat16_rn(x.hi);
+    const float r = x.hi - __bfloat162float(a);
     const __nv_bfloat16 b = __float2bfloat16_rn(r);
-    p0 = __bfloat16_as_ushort(a); p1 = __bfloat16_as_ushort(b); p2 = __bfloat16_as_ushort(__float2bfloat16_rn((r - __bfloat162float(b)) + lo));
+    p0 = __bfloat16_as_ushort(a); p1 = __bfloat16_as_ushort(b); p2 = __bfloat16_as_ushort(__float2bfloat16_rn((r - __bfloat162float(b)) + x.lo));
 }
 
 __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -122,6 +139,30 @@ __device__ __forceinline__ void mma_planes_kept(float (&acc)[4], float (&left)[4
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) left[i] += l[i];
+}
+// A key times the decays behind it.  Decays that have all but vanished (a pair has no more than 32-bit range) beside a key that could still
+// matter make it NaN: such states and chunks are walked.
+__device__ __forceinline__ Pair decayed_key(Pair f, float k) {
+    const bool lost = fabsf(k) >= 0x1p40f && fabsf(f.hi) < 0x1p-100f;
+    f *= k;
+    if (lost) f.hi = __int_as_float(0x7fc00000);
+    return f;
+}
+// two 32-bit operations in one instruction
+#define F32X2(name, op, ...) \
+    asm(op : "=l"(reinterpret_cast<unsigned long long&>(name)) : __VA_ARGS__)
+#define F32X2_IN(x) "l"(reinterpret_cast<const unsigned long long&>(x))
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { float2 d; F32X2(d, "mul.rn.f32x2 %0, %1, %2;", F32X2_IN(a), F32X2_IN(b)); return d; }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { float2 d; F32X2(d, "add.rn.f32x2 %0, %1, %2;", F32X2_IN(a), F32X2_IN(b)); return d; }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    F32X2(d, "fma.rn.f32x2 %0, %1, %2, %3;", F32X2_IN(a), F32X2_IN(b), F32X2_IN(c));
+    return d;
+}
+#undef F32X2
+#undef F32X2_IN
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 template <bool TRANS>
 __device__ __forceinline__ void ldsm(uint32_t (&r)[4], const uint16_t* p) {
@@ -208,55 +249,78 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
     if (!find_chunk<CT>(a.qsl, a.num_seqs, a.slot_lo + blockIdx.x, s, c, t0, n)) return;
     const size_t unit = (size_t)blockIdx.x * a.H + h;
     const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
-    auto stage_tail = [&](int col0) {
+    auto stage_tail = [&]() {
         for (int e = tid; e < TAIL * VT_COLS; e += NT) {
-            const int j = n - TAIL + e / VT_COLS, col = col0 + e % VT_COLS;
-            v_tail[e] = j >= 0 && col < a.Dv ? (double)to_f32(vp[(size_t)j * a.ld_v + col]) : 0.0;
+            const int j = n - TAIL + e / VT_COLS;                                     // (the staged values; columns past the last are zeros)
+            v_tail[e] = j >= 0 ? (double)__uint_as_float((uint32_t)v_s[j * VLD + e % VT_COLS] << 16) : 0.0;
         }
     };
 
     if constexpr (MODE == WKV) {
         // a thread per channel and run of LEN tokens: the decays of the run, its product, then keys times the decays behind them (products
-        // of up to 64 decays in 64 bits: in 32 they leave more than the walk's one rounding per token)
+        // of up to 64 decays as pairs: in 32 bits they leave more than the walk's one rounding per token)
         constexpr int LEN = CT * KP / NT, RUNS = CT / LEN;
-        double* tot = half;                                                           // [RUNS][KP]: product over a run (over wt, which is not used here)
+        Pair* tot = reinterpret_cast<Pair*>(half);                                    // [RUNS][KP]: product over a run (over wt, which is not used here)
         const int ch = tid % KP, run = tid / KP;
         const bool in = ch < a.D;
-        const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D + ch;
-        const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D + ch;
+        const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D;
+        const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k) + (size_t)t0 * a.ld_qk + h * a.D;
+        // decays, keys and values are all asked for at once, 16 bytes a copy; decays and keys wait where the planes will lie
+        float* w_raw = reinterpret_cast<float*>(kd);
+        uint16_t* k_raw = kd + 2 * CT * LD;
+        const bool wide = ((uintptr_t)a.decay & 15) == 0;
+        for (int e = tid; e < CT * (KP / 4); e += NT) {
+            const int j = e / (KP / 4), c4 = e % (KP / 4) * 4;
+            float* dst = w_raw + j * KP + c4;
+            const float* src = wp + (size_t)j * a.H * a.D + c4;
+            if (j >= n || c4 >= a.D) *reinterpret_cast<float4*>(dst) = make_float4(1.f, 1.f, 1.f, 1.f);
+            else if (wide) copy16(dst, src);
+            else *reinterpret_cast<float4*>(dst) = make_float4(src[0], src[1], src[2], src[3]);
+        }
+        for (int e = tid; e < CT * (KP / 8); e += NT) {
+            const int j = e / (KP / 8), c8 = e % (KP / 8) * 8;
+            if (j < n && c8 < a.D) copy16(k_raw + j * LD + c8, kp + (size_t)j * a.ld_qk + c8);
+            else *reinterpret_cast<uint4*>(k_raw + j * LD + c8) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (int e = tid; e < CT * (VT_COLS / 8); e += NT) {
+            const int j = e / (VT_COLS / 8), c8 = e % (VT_COLS / 8) * 8;
+            if (j < n && c8 < a.Dv) copy16(v_s + j * VLD + c8, vp + (size_t)j * a.ld_v + c8);
+            else *reinterpret_cast<uint4*>(v_s + j * VLD + c8) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (int e = tid; e < (TAIL - n) * KP; e += NT) k_tail[e] = 0.0;              // (fewer tokens than that)
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
         float w[LEN];
-        __nv_bfloat16 kv[LEN];
+        uint16_t kv[LEN];
 #pragma unroll
         for (int i = 0; i < LEN; ++i) {
-            const int j = run * LEN + i;
-            w[i] = in && j < n ? wp[(size_t)j * a.H * a.D] : 1.f;
-            kv[i] = in && j < n ? kp[(size_t)j * a.ld_qk] : __float2bfloat16(0.f);
+            w[i] = w_raw[(run * LEN + i) * KP + ch];
+            kv[i] = k_raw[(run * LEN + i) * LD + ch];
         }
-        stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv);
-        stage_tail(0);
-        for (int e = tid; e < (TAIL - n) * KP; e += NT) k_tail[e] = 0.0;              // (fewer tokens than that)
-        double all = 1.0;
+        stage_tail();
+        Pair all = {1.f, 0.f};
 #pragma unroll
-        for (int i = LEN - 1; i >= 0; --i) all *= (double)w[i];
+        for (int i = LEN - 1; i >= 0; --i) all *= w[i];
         tot[run * KP + ch] = all;
         __syncthreads();
-        double suf = 1.0;
+        Pair suf = {1.f, 0.f};
 #pragma unroll
         for (int i = RUNS - 1; i > 0; --i)
             if (i > run) suf *= tot[i * KP + ch];
         if (run == 0 && ch < a.Dpad) {
-            const double f = in ? all * suf : 1.0;
-            a.aux[2 * unit * a.Dpad + ch] = (float)f;
-            a.aux[(2 * unit + 1) * a.Dpad + ch] = (float)(f - (double)(float)f);
+            all *= suf;
+            const float f = in ? all.value() : 1.f;
+            a.aux[2 * unit * a.Dpad + ch] = f;
+            a.aux[(2 * unit + 1) * a.Dpad + ch] = in ? (all.hi - f) + all.lo : 0.f;
         }
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) {
             const int j = run * LEN + i;
-            const double x = (double)to_f32(kv[i]) * suf;
+            Pair x = decayed_key(suf, __uint_as_float((uint32_t)kv[i] << 16));
             const bool last = j >= n - TAIL && j < n;
-            if (last) k_tail[(j - (n - TAIL)) * KP + ch] = x;
-            split3(last ? 0.0 : x, kd[j * LD + ch], kd[CT * LD + j * LD + ch], kd[2 * CT * LD + j * LD + ch]);
-            suf *= (double)w[i];
+            if (last) { k_tail[(j - (n - TAIL)) * KP + ch] = (double)x.hi + (double)x.lo; x = {0.f, 0.f}; }
+            split3(x, kd[j * LD + ch], kd[CT * LD + j * LD + ch], kd[2 * CT * LD + j * LD + ch]);
+            suf *= w[i];
         }
     } else {
         stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, 0, a.Dv);
@@ -289,7 +353,7 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
         if (col0 > 0) {
             __syncthreads();
             stage_values<VT, VPL, NT>(v_s, vp, a.ld_v, n, col0, a.Dv);
-            if constexpr (MODE == WKV) stage_tail(col0);
+            if constexpr (MODE == WKV) { __syncthreads(); stage_tail(); }
             __syncthreads();
         }
         constexpr int NP = KP / 16 / PARTS;                                           // 16-channel tiles of this warp
@@ -349,12 +413,13 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
 // ------------------------------------------------------------------------------------------- chunk_out
 template <int MODE, int KP> struct OutSmem {
     static constexpr int LD = KP + 8, FLD = KP + 4;
-    static constexpr int EXTRA = MODE == WKV ? (2 * CT * FLD + 4 * KP) * 4 : MODE == MLSTM ? CT * 24 + KP * 4 : (CT + 1 + 3) * 4;
+    static constexpr bool SHARED = MODE == WKV && KP == 64;          // wkv: one table takes first the decays, then the rows' products of them
+    static constexpr int EXTRA = MODE == WKV ? ((SHARED ? 1 : 2) * CT * FLD + 4 * KP) * 4 : MODE == MLSTM ? CT * 24 + KP * 4 : (CT + 1 + 3) * 4;
     static size_t bytes(int vpl) { return (size_t)(3 * CT * LD + vpl * CT * VLD) * 2 + 64 + EXTRA; }
 };
 
-template <int MODE, int KP, typename VT>
-__global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT) == 4 ? 2 : 3) chunk_out_kernel(const ChunkArgs a) {
+template <int MODE, int KP, typename VT, int CTAS = MODE == WKV && KP == 128 ? 1 : sizeof(VT) == 4 ? 2 : 3>
+__global__ void __launch_bounds__(128, CTAS) chunk_out_kernel(const ChunkArgs a) {
     constexpr int LD = KP + 8, FLD = KP + 4, VPL = sizeof(VT) == 4 ? 3 : 1;
     constexpr int QPL = MODE == MLSTM ? 1 : 3, KPL = MODE == MLSTM ? 1 : 3, KS = KP / 16;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -373,7 +438,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
     const VT* vp = reinterpret_cast<const VT*>(a.v) + (size_t)t0 * a.ld_v + h * a.Dv;
     const int r0 = warp * 16 + g, r1 = r0 + 8;                                        // this lane's rows (tokens of the chunk)
     bool odd = false;                                                                 // something of this lane's is not finite
-    stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv);
+    if (MODE != WKV) stage_values<VT, VPL>(v_s, vp, a.ld_v, n, 0, a.Dv);
 
     // a lane's part of a 16 x 16 piece of the query rows: rows r0 / r1, channels c0 + 2t, + 1 and those + 8
     auto load_q = [&](int c0, float (&f)[8]) {
@@ -408,72 +473,149 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 
     if constexpr (MODE == WKV) {
         float* ws = reinterpret_cast<float*>(extra);                                  // [CT][FLD] decays
-        float* pre = ws + CT * FLD;                                                   // [CT][FLD] product of the block's decays before the token
+        constexpr bool SHARED = OutSmem<MODE, KP>::SHARED;
+        float* pre = SHARED ? ws : ws + CT * FLD;                                     // [CT][FLD] product of the block's decays before the token
         float* blk = pre + CT * FLD;                                                  // [4][KP] product over a block
-        for (int e = tid; e < 4 * KP; e += 128) {
-            const int J = e / KP, ch = e % KP;
-            const bool in = ch < a.D;
-            const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D + ch;
-            float w[16], k[16];
+        // decays, keys and query rows are all asked for at once, 16 bytes a copy; the keys wait where their last plane will lie, the query rows (64
+        // channels of them) where the values will
+        uint16_t* k_raw = pl + 2 * CT * LD;
+        const float* wp = a.decay + (size_t)t0 * a.H * a.D + h * a.D;
+        const bool wide = ((uintptr_t)a.decay & 15) == 0;
+        for (int e = tid; e < CT * (KP / 4); e += 128) {
+            const int j = e / (KP / 4), ch = e % (KP / 4) * 4;
+            float* dst = ws + j * FLD + ch;
+            const float* src = wp + (size_t)j * a.H * a.D + ch;
+            if (j >= n || ch >= a.D) *reinterpret_cast<float4*>(dst) = make_float4(1.f, 1.f, 1.f, 1.f);
+            else if (wide) copy16(dst, src);
+            else *reinterpret_cast<float4*>(dst) = make_float4(src[0], src[1], src[2], src[3]);
+        }
+        for (int e = tid; e < CT * (KP / 8); e += 128) {
+            const int j = e / (KP / 8), ch = e % (KP / 8) * 8;
+            const bool in = j < n && ch < a.D;
+            uint16_t* dst = k_raw + j * LD + ch;
+            if (in) copy16(dst, kp + (size_t)j * a.ld_qk + ch);
+            else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+            if (ch >= 64) continue;
+            if (in) copy16(v_s + j * VLD + ch, qp + (size_t)j * a.ld_qk + ch);
+            else *reinterpret_cast<uint4*>(v_s + j * VLD + ch) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        constexpr int ITEMS = 4 * KP / 128;                                           // (block, channel) pairs of a thread
+        uint16_t k[ITEMS][16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int j = J * 16 + i;
-                w[i] = in && j < n ? wp[(size_t)j * a.H * a.D] : 1.f;
-                k[i] = in && j < n ? to_f32(kp[(size_t)j * a.ld_qk + ch]) : 0.f;
+        for (int it = 0; it < ITEMS; ++it) {
+            const int e = it * 128 + tid, J = e / KP, ch = e % KP;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) k[it][i] = k_raw[(J * 16 + i) * LD + ch];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < ITEMS; ++it) {
+            const int e = it * 128 + tid, J = e / KP, ch = e % KP;
+            const float* w = ws + J * 16 * FLD + ch;
+            Pair f = {1.f, 0.f};                                                      // (as in chunk_sum)
+            if (!SHARED) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) { pre[(J * 16 + i) * FLD + ch] = f.value(); f *= w[i * FLD]; }
+                blk[J * KP + ch] = f.value();
+                f = {1.f, 0.f};
             }
-            double f = 1.0;                                                           // (in 64 bits, as in chunk_sum)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) { ws[(J * 16 + i) * FLD + ch] = w[i]; pre[(J * 16 + i) * FLD + ch] = (float)f; f *= (double)w[i]; }
-            blk[J * KP + ch] = (float)f;
-            f = 1.0;
 #pragma unroll
             for (int i = 15; i >= 0; --i) {
                 const int at = (J * 16 + i) * LD + ch;
-                split3((double)k[i] * f, pl[at], pl[CT * LD + at], pl[2 * CT * LD + at]);
-                f *= (double)w[i];
+                split3(decayed_key(f, __uint_as_float((uint32_t)k[it][i] << 16)), pl[at], pl[CT * LD + at], pl[2 * CT * LD + at]);
+                f *= w[i * FLD];
             }
         }
+        auto row_products = [&]() {                                                   // of decays before a token within its block, and over whole blocks
+#pragma unroll
+            for (int it = 0; it < ITEMS; ++it) {
+                const int e = it * 128 + tid, J = e / KP, ch = e % KP;
+                Pair f = {1.f, 0.f};
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int at = (J * 16 + i) * FLD + ch;
+                    const float w = ws[at];
+                    pre[at] = f.value();
+                    f *= w;
+                }
+                blk[J * KP + ch] = f.value();
+            }
+        };
         __syncthreads();
-        // inside the block: lanes own channels, running products from every key on; 16 sums over the lanes at a time.  The scores of key j
-        // take the place of the block's row j of decays (columns 0 .. 15), which nothing reads from step j on
-        float* dg = ws + warp * 16 * FLD;
+        // inside the block: a lane owns a key j and 32 channels, the rows come one after the other; the key's running product moves on with each
+        // row behind it.  The 32 terms of a score are added as pairs, then in a tree (as when lanes owned channels and 16 sums at a time
+        // went through shuffles; those were two thirds of the scores' instructions, 16,600 clocks of a CTA's 46,600).  The scores of key j take
+        // the place of query row j, which nothing reads from row j + 1 on (more than 64 channels: of the row of decays).
+        const float* dw = ws + warp * 16 * FLD;
+        uint16_t* rows = v_s + warp * 16 * VLD;
+        constexpr int GLD = SHARED ? VLD / 2 : FLD;
+        float* dg = SHARED ? reinterpret_cast<float*>(rows) : ws + warp * 16 * FLD;
+        const int jl = lane & 15, side = (lane >> 4) * 32;
         for (int ch0 = 0; ch0 < KP; ch0 += 64) {
-            float r[16][2], ub[2];
-            bool in[2];
+            if (ch0 > 0) {
+                __syncwarp();                                                         // (the last channels' rows have been read)
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                in[m] = ch0 + lane + 32 * m < a.D;
-                ub[m] = in[m] ? a.u[h * a.D + ch0 + lane + 32 * m] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-#pragma unroll
-                for (int m = 0; m < 2; ++m)
-                    r[i][m] = in[m] && warp * 16 + i < n ? to_f32(qp[(size_t)(warp * 16 + i) * a.ld_qk + ch0 + lane + 32 * m]) : 0.f;
-            const float* w = ws + warp * 16 * FLD + ch0 + lane;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                float p[2], sum[16];
-#pragma unroll
-                for (int m = 0; m < 2; ++m)
-                    p[m] = in[m] && warp * 16 + j < n ? to_f32(kp[(size_t)(warp * 16 + j) * a.ld_qk + ch0 + lane + 32 * m]) : 0.f;
-#pragma unroll
-                for (int i = 0; i < j; ++i) sum[i] = 0.f;
-                sum[j] = fmaf(r[j][1], ub[1] * p[1], r[j][0] * (ub[0] * p[0]));
-#pragma unroll
-                for (int i = j + 1; i < 16; ++i) {
-                    sum[i] = fmaf(r[i][1], p[1], r[i][0] * p[0]);
-                    p[0] *= w[i * FLD]; p[1] *= w[i * FLD + 32];
-                }
-                int first = 0;
-                RunReduce<16, 16>::run(sum, lane, first);
-                if ((lane & 1) == 0) {
-                    float* o = dg + j * FLD + first;
-                    *o = ch0 == 0 ? sum[0] : *o + sum[0];
+                for (int e = lane; e < 16 * 8; e += 32) {
+                    const int i = e >> 3, c = (e & 7) * 8;
+                    const bool in = warp * 16 + i < n && ch0 + c < a.D;
+                    *reinterpret_cast<uint4*>(rows + i * VLD + c) =
+                        in ? *reinterpret_cast<const uint4*>(qp + (size_t)(warp * 16 + i) * a.ld_qk + ch0 + c) : make_uint4(0u, 0u, 0u, 0u);
                 }
             }
+            float2 p[16];                                                             // the key's channels side + 2 m, + 1, times the decays up to the row
+#pragma unroll
+            for (int m = 0; m < 16; m += 4) {
+                const int c = ch0 + side + 2 * m;
+                const bool in = warp * 16 + jl < n && c < a.D;
+                const uint4 x = in ? *reinterpret_cast<const uint4*>(kp + (size_t)(warp * 16 + jl) * a.ld_qk + c) : make_uint4(0u, 0u, 0u, 0u);
+                p[m] = unpack(x.x); p[m + 1] = unpack(x.y); p[m + 2] = unpack(x.z); p[m + 3] = unpack(x.w);
+            }
+            __syncwarp();
+            // sum over this lane's channels of row i (its pieces at `row`) times `x`, as a tree
+            auto dot = [&](const uint16_t* row, auto x) {
+                float2 t[8];
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const uint2 r = *reinterpret_cast<const uint2*>(row + side + 4 * m);
+                    t[m] = fma2(unpack(r.y), x(2 * m + 1), mul2(unpack(r.x), x(2 * m)));
+                }
+#pragma unroll
+                for (int d = 1; d < 8; d *= 2)
+#pragma unroll
+                    for (int m = 0; m < 8; m += 2 * d) t[m] = add2(t[m], t[m + d]);
+                const float sum = t[0].x + t[0].y;
+                return sum + __shfl_xor_sync(0xffffffffu, sum, 16);
+            };
+            const float* up = a.u + h * a.D + ch0 + side;
+            const float own = dot(rows + jl * VLD, [&](int m) {
+                const bool in = ch0 + side + 2 * m < a.D;                             // (a multiple of 8)
+                return mul2(p[m], in ? make_float2(up[2 * m], up[2 * m + 1]) : make_float2(0.f, 0.f));
+            });
+#pragma unroll 1
+            for (int i = 1; i < 16; ++i) {
+                const float sum = dot(rows + i * VLD, [&](int m) { return p[m]; });
+                if (i > jl) {
+                    const float4* w = reinterpret_cast<const float4*>(dw + i * FLD + ch0 + side);
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        const float4 x = w[m];
+                        p[2 * m] = mul2(p[2 * m], make_float2(x.x, x.y));
+                        p[2 * m + 1] = mul2(p[2 * m + 1], make_float2(x.z, x.w));
+                    }
+                }
+                __syncwarp();
+                if (i > jl && lane < 16) { float* o = dg + jl * GLD + i; *o = ch0 == 0 ? sum : *o + sum; }
+            }
+            __syncwarp();
+            if (lane < 16) { float* o = dg + jl * GLD + jl; *o = ch0 == 0 ? own : *o + own; }
         }
-        __syncwarp();
+        if (SHARED) {
+            __syncthreads();                                                          // (every warp's decays have been read)
+            row_products();
+            __syncthreads();
+        } else __syncwarp();
         // between blocks: rows times the decays from their block's start, then times whole blocks going back
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
@@ -506,8 +648,18 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
                         const int r = g + (b & 2 ? 8 : 0), col = i * 8 + 2 * t + (b & 1);
-                        P[2 * J + i][b] = col <= r ? dg[col * FLD + r] : 0.f;
+                        P[2 * J + i][b] = col <= r ? dg[col * GLD + r] : 0.f;
                     }
+        if (SHARED) {                                                                 // the rows wait in their own places of the table
+            __syncwarp();
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const int r = (i >> 1) & 1 ? r1 : r0, ch = ks * 16 + 2 * t + (i & 4 ? 8 : 0);
+                    *reinterpret_cast<float2*>(pre + r * FLD + ch) = make_float2(rq[ks][i], rq[ks][i + 1]);
+                }
+        }
         row_in[0] = row_in[1] = 1.f;
     } else {
         stage_rows<KPL, KP, LD>(pl, kp, a.ld_qk, [&](int j, int ch) { return j < n && ch < a.D; }, [](int, float (&)[8]) {});
@@ -586,7 +738,7 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 
     for (int col0 = 0; col0 < a.Dv; col0 += VT_COLS) {
         __syncthreads();                                                              // the keys (or the last columns) have been read by everyone
-        if (col0 > 0) stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv);
+        if (col0 > 0 || MODE == WKV) stage_values<VT, VPL>(v_s, vp, a.ld_v, n, col0, a.Dv);
         const float* sp = a.part + (unit * a.Dv + col0) * a.Dpad;
         stage_rows<3, KP, LD>(pl, sp, a.Dpad, [&](int j, int ch) { return col0 + j < a.Dv && ch < a.Dpad; }, [](int, float (&)[8]) {});
         __syncthreads();
@@ -596,7 +748,17 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
             uint32_t q[QPL][4];
-            if constexpr (MODE == WKV) planes_of(rq[ks], q);
+            if constexpr (MODE == WKV && OutSmem<MODE, KP>::SHARED) {
+                const float* pre = reinterpret_cast<const float*>(extra);
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const int r = (i >> 1) & 1 ? r1 : r0, ch = ks * 16 + 2 * t + (i & 4 ? 8 : 0);
+                    const float2 x = *reinterpret_cast<const float2*>(pre + r * FLD + ch);
+                    f[i] = x.x; f[i + 1] = x.y;
+                }
+                planes_of(f, q);
+            } else if constexpr (MODE == WKV) planes_of(rq[ks], q);
             else { float f[8]; load_q(ks * 16, f); planes_of(f, q); }
 #pragma unroll
             for (int np = 0; np < 4; ++np) {
@@ -645,12 +807,14 @@ __global__ void __launch_bounds__(128, MODE == WKV && KP == 128 ? 1 : sizeof(VT)
 template <int MODE, int KP, typename VT>
 int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
     constexpr int VPL = sizeof(VT) == 4 ? 3 : 1;
+    constexpr bool MANY = OutSmem<MODE, KP>::SHARED;
     const size_t sum_smem = SumSmem<MODE, KP>::bytes(VPL), out_smem = OutSmem<MODE, KP>::bytes(VPL);
     static bool allowed[64] = {false};
     int dev = 64;
     if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64 || !allowed[dev]) {
         cudaFuncSetAttribute(chunk_sum_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
         cudaFuncSetAttribute(chunk_out_kernel<MODE, KP, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+        if constexpr (MANY) cudaFuncSetAttribute(chunk_out_kernel<MODE, KP, VT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
         if (dev < 64) allowed[dev] = true;
     }
     a.slot_lo = first; a.slots = slots;
@@ -658,6 +822,14 @@ int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
     const dim3 carry(ceil_div(a.Dv * a.Dpad + (MODE == MLSTM ? a.Dpad : 0), 4 * CARRY), a.H, a.num_seqs);
     TTIE_LAUNCH((chunk_sum_kernel<MODE, KP, VT>), grid, (SumSmem<MODE, KP>::NT), sum_smem, st, a);
     TTIE_LAUNCH((chunk_carry_kernel<MODE, CT>), carry, CARRY, 0, st, a);
+    // wkv, heads of up to 64: four CTAs an SM with 128 registers where three with 168 do not hold the grid at once
+    if constexpr (MANY) {
+        if ((long long)slots * a.H > 3LL * num_sms()) {
+            TTIE_LAUNCH((chunk_out_kernel<MODE, KP, VT, 4>), grid, 128, out_smem, st, a);
+            TTIE_CHECK_LAUNCH("matrix_chunks");
+            return 0;
+        }
+    }
     TTIE_LAUNCH((chunk_out_kernel<MODE, KP, VT>), grid, 128, out_smem, st, a);
     TTIE_CHECK_LAUNCH("matrix_chunks");
     return 0;
