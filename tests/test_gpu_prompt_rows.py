@@ -194,3 +194,16 @@ def test_causal_conv_in_runs_of_tokens(ops, lens, width, wdtype, taps):
             assert ((u32.double() - e).abs() <= slack).all()
         y = e * torch.sigmoid(e) if act else e
         assert ((u.double() - y).abs() <= 2.0 ** -8 * y.abs() + 2 * slack + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,d,off", [(1, 8, 0), (3, 12, 0), (5, 1032, 0), (2, 4104, 8), (4, 100, 0), (3, 64, 1), (70, 516, 4)])
+def test_embed_forms(ops, T, d, off, dtype):
+    """Rows that fill their last piece and not, tables on 16 bytes and off them, ids past either end: one 32-bit multiplication, exactly."""
+    V = 50
+    table = randn(61, V * d + off).to(dtype)[off:].view(V, d)
+    ids = torch.randint(0, V, (T,), dtype=torch.int32, device=DEV)
+    ids[0], ids[-1] = -3, V + 7
+    out = torch.empty(T, d, device=DEV)
+    ops.embed(ids, table, out, scale=1.7)
+    assert torch.equal(out, table[ids.clamp(0, V - 1).long()].float() * 1.7)

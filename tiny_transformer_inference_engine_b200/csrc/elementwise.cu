@@ -64,14 +64,46 @@ __global__ void embed_kernel(const int* __restrict__ ids, const T* __restrict__ 
     for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = to_f32<T>(row[i]) * scale;
 }
 
+// ... 16 bytes of a row per thread (rows and arrays on 16 bytes): a token's row is asked for at once instead of in 16 dependent turns of 2 bytes a
+// thread.  Alone, table out of cache: 1 token of 4,096 columns 3.7 -> 1.4 us, 2,048 tokens 17.1 -> 10.6 (50 MB), in 32 bits 18.6 -> 17.6; as the first kernel of a decode step,
+// where it stands behind the copy of the token ids, 11.2 -> 1.9.
+template <typename T>
+__global__ void __launch_bounds__(128) embed_vec_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out,
+                                                        int T_, int d, int vocab, float scale) {
+    constexpr int V = 16 / sizeof(T);
+    TTIE_PDL_ENTRY();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * V;               // grid: (columns, tokens)
+    if (c >= d) return;
+    for (int t = blockIdx.y; t < T_; t += gridDim.y) {
+        const int id = min(max(ids[t], 0), vocab - 1);
+        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(table + (size_t)id * d + c));
+        float v[V];
+        if constexpr (V == 8) {
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+        } else {
+            v[0] = __uint_as_float(raw.x); v[1] = __uint_as_float(raw.y); v[2] = __uint_as_float(raw.z); v[3] = __uint_as_float(raw.w);
+        }
+        float4* o = reinterpret_cast<float4*>(out + (size_t)t * d + c);
+#pragma unroll
+        for (int i = 0; i < V; i += 4) o[i / 4] = make_float4(v[i] * scale, v[i + 1] * scale, v[i + 2] * scale, v[i + 3] * scale);
+    }
+}
+
 // out[t, :] = table[ids[t], :] * scale, 32-bit
 extern "C" int ttie_embed(const int* ids, const void* table, float* out, int T, int d, int vocab, float scale, int dtype, void* stream) {
     if (T <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = d >= 1024 ? 256 : 128;
-    if (dtype == kF32) TTIE_LAUNCH(embed_kernel<float>, T, threads, 0, s, ids, (const float*)table, out, d, vocab, scale);
-    else if (dtype == kBF16) TTIE_LAUNCH(embed_kernel<__nv_bfloat16>, T, threads, 0, s, ids, (const __nv_bfloat16*)table, out, d, vocab, scale);
-    else TTIE_FAIL("embed: unknown dtype %d", dtype);
+    const int v = dtype == kF32 ? 4 : 8;                              // values of 16 bytes
+    const bool wide = d % v == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0;
+    const dim3 grid(ceil_div(d, 128 * v), T < 65535 ? T : 65535);
+    if (dtype != kF32 && dtype != kBF16) TTIE_FAIL("embed: unknown dtype %d", dtype);
+    if (wide && dtype == kF32) TTIE_LAUNCH(embed_vec_kernel<float>, grid, 128, 0, s, ids, (const float*)table, out, T, d, vocab, scale);
+    else if (wide) TTIE_LAUNCH(embed_vec_kernel<__nv_bfloat16>, grid, 128, 0, s, ids, (const __nv_bfloat16*)table, out, T, d, vocab, scale);
+    else if (dtype == kF32) TTIE_LAUNCH(embed_kernel<float>, T, threads, 0, s, ids, (const float*)table, out, d, vocab, scale);
+    else TTIE_LAUNCH(embed_kernel<__nv_bfloat16>, T, threads, 0, s, ids, (const __nv_bfloat16*)table, out, d, vocab, scale);
     TTIE_CHECK_LAUNCH("embed");
     return 0;
 }
