@@ -161,9 +161,6 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 #undef F32X2
 #undef F32X2_IN
-__device__ __forceinline__ void copy16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 template <bool TRANS>
 __device__ __forceinline__ void ldsm(uint32_t (&r)[4], const uint16_t* p) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
@@ -422,6 +419,7 @@ template <int MODE, int KP, typename VT, int CTAS = MODE == WKV && KP == 128 ? 1
 __global__ void __launch_bounds__(128, CTAS) chunk_out_kernel(const ChunkArgs a) {
     constexpr int LD = KP + 8, FLD = KP + 4, VPL = sizeof(VT) == 4 ? 3 : 1;
     constexpr int QPL = MODE == MLSTM ? 1 : 3, KPL = MODE == MLSTM ? 1 : 3, KS = KP / 16;
+    constexpr bool GATES = OutSmem<MODE, KP>::SHARED;                // (the gate's rows take the place of the table, one tile of columns)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* pl = reinterpret_cast<uint16_t*>(smem_raw);                             // [3][CT][LD]: keys, then 64 columns of the state
     uint16_t* v_s = pl + 3 * CT * LD;                                                 // [VPL][CT][VLD]
@@ -768,6 +766,15 @@ __global__ void __launch_bounds__(128, CTAS) chunk_out_kernel(const ChunkArgs a)
                 mma_planes<QPL, 3>(acc[2 * np], acc[2 * np + 1], q, b);
             }
         }
+        if (GATES && a.y) {                                                           // the warp's rows of the table have been read: the gate's, while the values are multiplied
+            __syncwarp();
+            const __nv_bfloat16* gp = a.gate + (size_t)t0 * a.ld_gate + h * a.Dv;
+#pragma unroll
+            for (int e = lane; e < 16 * VT_COLS / 8; e += 32) {
+                const int r = warp * 16 + e / 8, piece = e % 8;
+                if (r < n && piece * 8 < a.Dv) copy16(reinterpret_cast<float*>(extra) + r * FLD + piece * 4, gp + (size_t)r * a.ld_gate + piece * 8);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             acc[i][0] *= row_in[0]; acc[i][1] *= row_in[0]; acc[i][2] *= row_in[1]; acc[i][3] *= row_in[1];
@@ -788,6 +795,41 @@ __global__ void __launch_bounds__(128, CTAS) chunk_out_kernel(const ChunkArgs a)
         }
         const size_t ld_o = (size_t)a.H * a.Dv;
         float* op = a.out + (size_t)t0 * ld_o + h * a.Dv + col0;
+        // Gated where the gate's row lies, then out in whole rows.  With the products over, a row's 64 values are in four lanes: no tile is needed.
+        // 101 -> 97 us of a scan of 2,048 tokens and 32 heads (the pass apart: 8).
+        if (GATES && a.y) {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s0 = fmaf(acc[i][0], acc[i][0], fmaf(acc[i][1], acc[i][1], s0));
+                s1 = fmaf(acc[i][2], acc[i][2], fmaf(acc[i][3], acc[i][3], s1));
+                odd = odd || (r0 < n && !finite4(acc[i][0], acc[i][1], 0.f, 0.f)) || (r1 < n && !finite4(acc[i][2], acc[i][3], 0.f, 0.f));
+            }
+#pragma unroll
+            for (int k = 1; k < 4; k <<= 1) { s0 += __shfl_xor_sync(0xffffffffu, s0, k); s1 += __shfl_xor_sync(0xffffffffu, s1, k); }
+            s0 = inverse_rms(a, s0); s1 = inverse_rms(a, s1);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            uint32_t* gate = reinterpret_cast<uint32_t*>(extra);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int col = i * 8 + 2 * t;
+                if (col >= a.Dv) continue;
+                const float2 w = a.norm_w ? *reinterpret_cast<const float2*>(a.norm_w + h * a.Dv + col) : make_float2(1.f, 1.f);
+                uint32_t* g0 = gate + r0 * FLD + i * 4 + t;
+                uint32_t* g1 = gate + r1 * FLD + i * 4 + t;
+                *g0 = gated_pair(a, acc[i][0] * s0, acc[i][1] * s0, w, *g0);
+                *g1 = gated_pair(a, acc[i][2] * s1, acc[i][3] * s1, w, *g1);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int e = lane; e < 16 * VT_COLS / 8; e += 32) {
+                const int r = warp * 16 + e / 8, piece = e % 8;
+                if (r < n && piece * 8 < a.Dv)
+                    *reinterpret_cast<uint4*>(a.y + (size_t)(t0 + r) * ld_o + h * a.Dv + piece * 8) = *reinterpret_cast<const uint4*>(gate + r * FLD + piece * 4);
+            }
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int col = i * 8 + 2 * t;
@@ -801,7 +843,10 @@ __global__ void __launch_bounds__(128, CTAS) chunk_out_kernel(const ChunkArgs a)
             odd = odd || (r0 < n && !finite4(y[0], y[1], 0.f, 0.f)) || (r1 < n && !finite4(y[2], y[3], 0.f, 0.f));
         }
     }
-    if (__syncthreads_or(odd)) walk_out<MODE, CT, VT>(a, unit, t0, n, h, reinterpret_cast<float*>(pl));
+    if (__syncthreads_or(odd)) {
+        walk_out<MODE, CT, VT>(a, unit, t0, n, h, reinterpret_cast<float*>(pl));
+        if (GATES && a.y) gate_walked(a, t0, n, h);
+    }
 }
 
 template <int MODE, int KP, typename VT>
@@ -839,12 +884,14 @@ int launch_chunks(ChunkArgs a, int first, int slots, cudaStream_t st) {
 // mode: 0 retention (q, k float32; v either type), 1 mlstm, 2 wkv (q, k, v bfloat16).  T: rows of the step.  D and Dv multiples of
 // 8, D at most 128, rows that start on 16 bytes.  part / aux / span / mm hold `slots` chunk numbers' worth; a step of more chunk
 // numbers (T / chunk + requests) is done in passes.  chunk: tokens of one, 64 or (modes 0 and 1, bfloat16 values of at most 128 columns) 128.
-// pre_bias (chunks of 128): bfloat16 [2H] on mlstm's gate pre-activations.
+// pre_bias (chunks of 128): bfloat16 [2H] on mlstm's gate pre-activations.  y (or null; chunks of 128, or mode 2 with at most 64 channels):
+// bfloat16 [T, H*Dv], the read-outs normalised over a head, times norm_w [H*Dv] (or null) and act(gate) (0 silu, 1 sigmoid); `out` is scratch then.
 extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long long ld_qk, const void* v, long long ld_v, int v_dtype,
                                   const float* pre, long long ld_pre, float cap, const float* decay, const float* u, float* S, float* nrm,
                                   float* mx, int state_rows, const void* x, long long ld_x, int d, float* prev, int prev_rows, const int* qsl,
                                   const int* slot_ids, int num_seqs, int T, float* out, int H, int D, int Dv, int Dpad, float qscale,
-                                  float* part, float* aux, void* span, void* mm, int slots, int chunk, const void* pre_bias, void* stream) {
+                                  float* part, float* aux, void* span, void* mm, int slots, int chunk, const void* pre_bias, void* y,
+                                  const void* gate, long long ld_gate, const float* norm_w, float eps, int act, void* stream) {
     if (num_seqs <= 0 || T <= 0) return 0;
     if (chunk != CT && (chunk != 128 || mode == WKV || v_dtype != kBF16 || Dv > 128)) TTIE_FAIL("matrix_chunks: chunks of %d tokens, mode %d, %d value channels", chunk, mode, Dv);
     if (pre_bias && (chunk != 128 || mode != MLSTM)) TTIE_FAIL("matrix_chunks: a gate bias goes with mlstm in chunks of 128 tokens");
@@ -854,7 +901,10 @@ extern "C" int ttie_matrix_chunks(int mode, const void* q, const void* k, long l
         || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)S | (uintptr_t)nrm | (uintptr_t)part | (uintptr_t)aux) & 15))
         TTIE_FAIL("matrix_chunks: heads of %d key channels (padded %d) and %d value channels, strides %lld and %lld: multiples of 8, at most 128 key channels, rows on 16 bytes", D, Dpad, Dv, ld_qk, ld_v);
     if (slots < 1 || H > 65535 || num_seqs > 65535) TTIE_FAIL("matrix_chunks: %d chunks a pass, %d heads, %d requests", slots, H, num_seqs);
+    if (y && (!(chunk == 128 || (mode == WKV && Dpad <= 64)) || !gate || ld_gate % 8 || (((uintptr_t)gate | (uintptr_t)y) & 15) || ((uintptr_t)norm_w & 7)))
+        TTIE_FAIL("matrix_chunks: a gate with mode %d in chunks of %d, its rows %lld apart", mode, chunk, ld_gate);
     ChunkArgs a = {};
+    a.y = (__nv_bfloat16*)y; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate; a.norm_w = norm_w; a.eps = eps; a.act = act;
     a.q = q; a.k = k; a.ld_qk = ld_qk; a.v = v; a.ld_v = ld_v; a.pre = pre; a.ld_pre = ld_pre; a.cap = cap; a.decay = decay; a.u = u;
     a.v_f32 = v_dtype == kF32;
     a.S = S; a.nrm = nrm; a.mx = mx; a.state_rows = state_rows; a.x = x; a.ld_x = ld_x; a.d = d; a.prev = prev; a.prev_rows = prev_rows;

@@ -28,6 +28,8 @@ struct ChunkArgs {
     double2* span;                                                    // mlstm: [slots, H] (F at the end, max of x)
     float2* mm;                                                       // mlstm: [slots, H] the running maximum before and behind the chunk
     const __nv_bfloat16* pre_bias;                                    // mlstm in chunks of 128 tokens: [2H] on the gates' pre-activations, or null
+    // the read-outs normalised over a head and gated (head_norm_gate of matrix_memory.cu), where y is not null: `out` then only holds what is walked
+    __nv_bfloat16* y; const __nv_bfloat16* gate; long long ld_gate; const float* norm_w; float eps; int act;
 };
 
 __device__ __forceinline__ int state_row(int slot, int num_rows) { return slot < 0 ? num_rows - 1 : slot; }
@@ -62,6 +64,9 @@ __device__ __forceinline__ double power(double x, int n) {
 
 __device__ __forceinline__ float2 unpack(uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); }
 
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 // eight consecutive values of a row as floats (zeros where `in` is false)
 __device__ __forceinline__ void load8(const float* p, bool in, float (&o)[8]) {
     const float4 a = in ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -187,6 +192,34 @@ __device__ __forceinline__ void walk_out(const ChunkArgs& a, size_t unit, int t0
                 *o = acc;
             }
         }
+    }
+}
+
+// ---- normalised and gated read-outs: o * weight / rms(o over the head) * act(gate), 32-bit until the result is rounded to bfloat16 (2^-9; the
+// approximations of e^x, 1 / x and 1 / sqrt(x) are good to 2^-21)
+__device__ __forceinline__ float inverse_rms(const ChunkArgs& a, float squares) { return rsqrtf(squares / (float)a.Dv + a.eps); }
+__device__ __forceinline__ float gate_of(const ChunkArgs& a, float g) {
+    const float s = __fdividef(1.0f, 1.0f + __expf(-g));
+    return a.act == 0 ? g * s : s;
+}
+__device__ __forceinline__ uint32_t gated_pair(const ChunkArgs& a, float x, float y, float2 w, uint32_t gate) {
+    const float2 g = unpack(gate);
+    const __nv_bfloat162 p = __floats2bfloat162_rn(x * w.x * gate_of(a, g.x), y * w.y * gate_of(a, g.y));
+    return *reinterpret_cast<const uint32_t*>(&p);
+}
+// the chunk's rows behind the walk, which leaves its read-outs in `out`; the whole block calls
+__device__ __forceinline__ void gate_walked(const ChunkArgs& a, int t0, int n, int h) {
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int r = threadIdx.x >> 5; r < n; r += blockDim.x >> 5) {
+        const size_t at = ((size_t)(t0 + r) * a.H + h) * a.Dv;
+        const __nv_bfloat16* gate = a.gate + (size_t)(t0 + r) * a.ld_gate + h * a.Dv;
+        float ss = 0.f;
+        for (int c = lane; c < a.Dv; c += 32) ss = fmaf(a.out[at + c], a.out[at + c], ss);
+        const float inv = inverse_rms(a, warp_sum(ss));
+        for (int c = lane; c < a.Dv; c += 32)
+            a.y[at + c] = __float2bfloat16(a.out[at + c] * inv * (a.norm_w ? a.norm_w[h * a.Dv + c] : 1.f) * gate_of(a, __bfloat162float(gate[c])));
     }
 }
 

@@ -7,7 +7,11 @@
 // out in rounds (below): 16 terms of the leading planes at a time.
 //
 //   chunk_sum_tc   D[value column][channel] = V^T K', both operands as they lie (token by row); what rounding the rounds' sum leaves is kept
-//   chunk_out_tc   S = Q K^T, then O = Q (state)^T while the threads weigh the scores, then the weights, in the place of queries and state, times V
+//   chunk_out_tc   S = Q K^T, then O = Q (state)^T while the threads weigh the scores, then the weights, in the place of queries and state, times V;
+//                  with a gate the read-outs are normalised over the head and gated before they leave: the gate's rows come into the place of the
+//                  state while the weights are multiplied, and leave as the results.  The whole mixer 149.4 -> 145.6 us (retention), 120.9 -> 114.9
+//                  (mlstm of 64 x 128) at 2,048 tokens: the pass over the read-outs took 9 us, of which 3 to 6 more stay in this kernel.  From the
+//                  sums' tile in shared memory, a warp a row, with divisions rounded to 32 bits they took 8 to 14.
 //
 // One prompt of 2,048 tokens, us of the scan (in chunks of 64): 16 heads of 128 x 128 retention 59 (95), mlstm 65 (100), 16 of 64 x 128 40 (54)
 // and 48 (65).  One CTA of the out kernel fits an SM (six planes of 32 KB), its phases run one after the other, and 256 of them on 148 SMs are
@@ -311,9 +315,12 @@ template <int MODE, int KP> struct OutTc {
     static constexpr int QPL = MODE == MLSTM ? 1 : 3;
     static constexpr uint32_t PLANE = KP / 64 * BLOCK, COLS = 512;
     static constexpr uint32_t W_PLANE = CT / 64 * BLOCK;             // of the weights, which take the place of the queries and the state
-    static constexpr uint32_t OPERANDS = (QPL + 3) * PLANE > 3 * W_PLANE ? (QPL + 3) * PLANE : 3 * W_PLANE;
+    // behind the weights, in place of the state: the gate's rows, the rows' sums of squares and the norm's weights
+    static constexpr uint32_t GATE_LD = DVP * 2 + 16, GATE = (CT * GATE_LD + (GROUPS * CT + DVP) * 4 + 1023) / 1024 * 1024;
+    static constexpr uint32_t OPERANDS = (QPL + 3) * PLANE > 3 * W_PLANE + GATE ? (QPL + 3) * PLANE : 3 * W_PLANE + GATE;
     static constexpr size_t bytes = OPERANDS + DVP / 64 * BLOCK + 1024;
     static_assert(OPERANDS >= CT * (DVP + 4) * 4, "the operands' place takes the output tile");
+    static_assert(OPERANDS % 1024 == 0, "the values' swizzle starts on 1024 bytes");
     // rounds of the scores, of the read-out of the state, of weights times values
     using Scores = Rounds<KP / 16, QPL == 3>;
     using State = Rounds<KP / 16, true>;
@@ -474,6 +481,18 @@ __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, 
     }
     if constexpr (MODE == MLSTM) den = (den_s[0][row] + den_s[1][row]) + (den_s[2][row] + den_s[3][row]);
     mbar_wait(bar_o + 8 * Tc::State::N, 53, err);                    // what the state before the chunk gives; queries and state have been read
+    unsigned char* gate_s = q_s + 3 * W_PLANE;                       // [CT] rows of GATE_LD bytes
+    float* squares = reinterpret_cast<float*>(gate_s + CT * Tc::GATE_LD);                            // [GROUPS][CT]
+    float* norm_w = squares + GROUPS * CT;                           // [DVP]
+    if (a.y) {
+        const __nv_bfloat16* gp = a.gate + (size_t)t0 * a.ld_gate + h * a.Dv;
+#pragma unroll
+        for (int e = tid; e < CT * DVP / 8; e += NT) {
+            const int r = e / (DVP / 8), col = e % (DVP / 8) * 8;
+            if (r < n && col < a.Dv) copy16(gate_s + r * Tc::GATE_LD + col * 2, gp + (size_t)r * a.ld_gate + col);
+        }
+        if (tid < DVP) norm_w[tid] = a.norm_w && tid < a.Dv ? a.norm_w[h * a.Dv + tid] : 1.f;
+    }
 #pragma unroll
     for (int g = 0; g < OWN / 16; ++g) {
         add_slot(mine + (SLOTS - 1) * SLOT + g * 16, o[g]);
@@ -516,6 +535,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, 
     mbar_wait(bar_v + 8 * Tc::Values::N, 54, err);                   // (all products are done: the output tile takes the operands' place)
     constexpr int LD = DVP + 4;
     float* tile = reinterpret_cast<float*>(q_s);
+    float ss = 0.f;
 #pragma unroll
     for (int g = 0; g < OWN / 16; ++g) {
         add_slot(mine + (SLOTS - 1) * SLOT + g * 16, o[g]);
@@ -523,14 +543,42 @@ __global__ void __launch_bounds__(NT, 1) chunk_out_tc_kernel(const ChunkArgs a, 
         for (int i = 0; i < 16; ++i) {
             if constexpr (MODE == MLSTM) o[g][i] *= scale;
             odd = fmaf(o[g][i], 0.f, odd);
+            ss = fmaf(o[g][i], o[g][i], ss);
         }
+        if (a.y) continue;
 #pragma unroll
         for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(tile + row * LD + group * OWN + g * 16 + i) = make_float4(o[g][i], o[g][i + 1], o[g][i + 2], o[g][i + 3]);
     }
+    if (a.y) {
+        squares[group * CT + row] = ss;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
     tc_free(tmem, COLS);
     const size_t ld_o = (size_t)a.H * a.Dv;
-    copy_tile<LD>(a.out + (size_t)t0 * ld_o + h * a.Dv, ld_o, tile, n, a.Dv);
-    if (__syncthreads_or(row < n && !(odd == 0.f))) walk_out<MODE, CT, __nv_bfloat16>(a, unit, t0, n, h, tile);
+    if (a.y) {                                                       // gated where the gate's row lies, then out in whole rows
+        const float inv = inverse_rms(a, (squares[row] + squares[CT + row]) + (squares[2 * CT + row] + squares[3 * CT + row]));
+        uint4* gr = reinterpret_cast<uint4*>(gate_s + row * Tc::GATE_LD + group * OWN * 2);
+        const float2* w2 = reinterpret_cast<const float2*>(norm_w + group * OWN);
+#pragma unroll
+        for (int c = 0; c < OWN / 8; ++c) {
+            const uint4 g4 = gr[c];
+            const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
+            uint32_t y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] = gated_pair(a, o[c / 2][(c & 1) * 8 + 2 * i] * inv, o[c / 2][(c & 1) * 8 + 2 * i + 1] * inv, w2[c * 4 + i], g[i]);
+            gr[c] = make_uint4(y[0], y[1], y[2], y[3]);
+        }
+        __syncthreads();
+        const int col = tid % (DVP / 8) * 8;
+        if (col < a.Dv)
+#pragma unroll 4
+            for (int r = tid / (DVP / 8); r < n; r += NT / (DVP / 8))
+                *reinterpret_cast<uint4*>(a.y + (size_t)(t0 + r) * ld_o + h * a.Dv + col) = *reinterpret_cast<const uint4*>(gate_s + r * Tc::GATE_LD + col * 2);
+    } else copy_tile<LD>(a.out + (size_t)t0 * ld_o + h * a.Dv, ld_o, tile, n, a.Dv);
+    if (__syncthreads_or(row < n && !(odd == 0.f))) {
+        walk_out<MODE, CT, __nv_bfloat16>(a, unit, t0, n, h, tile);
+        if (a.y) gate_walked(a, t0, n, h);
+    }
 }
 
 template <int MODE, int KP>

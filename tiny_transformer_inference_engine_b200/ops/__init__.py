@@ -142,7 +142,8 @@ _SIGNATURES = {
                             _c_int, _c_int, _c_int, _c_void, _c_int, _c_void],
     "ttie_matrix_chunks": [_c_int, _c_void, _c_void, _c_ll, _c_void, _c_ll, _c_int, _c_void, _c_ll, _c_float, _c_void, _c_void, _c_void, _c_void,
                            _c_void, _c_int, _c_void, _c_ll, _c_int, _c_void, _c_int, _c_void, _c_void, _c_int, _c_int, _c_void, _c_int, _c_int,
-                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void, _c_void],
+                           _c_int, _c_int, _c_float, _c_void, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void, _c_void, _c_void, _c_ll, _c_void,
+                           _c_float, _c_int, _c_void],
     "ttie_head_norm_gate": [_c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void, _c_int, _c_void],
     "ttie_activation": [_c_void, _c_void, _c_ll, _c_int, _c_float, _c_float, _c_int, _c_int, _c_void],
     "ttie_matrix_state_pad": [_c_int],
@@ -1528,24 +1529,25 @@ class CudaOps:
         self.launches += 1
         return out
 
-    def wkv_scan(self, r, k, v, decay, u, state, x, prev, query_start_loc, slot_ids, num_seqs, num_heads, dim, max_q_len=None):
+    def wkv_scan(self, r, k, v, decay, u, state, x, prev, query_start_loc, slot_ids, num_seqs, num_heads, dim, max_q_len=None, gated=None):
         """The time mix's recurrence over the step's tokens from the state rows ``state`` [slots + 1, H, dim, padded dim]
         (advanced in place): o_t = (S + diag(u) k v^T)^T r, then S <- diag(w) S + k v^T.  r, k, v [T, H*dim] views with one row
         stride; ``decay`` (w) float32 [T, H*dim] contiguous.  Also stores each request's last row of ``x`` into ``prev``.
-        ``max_q_len``: the most tokens a request brings, if known (``_in_chunks``).  Returns o float32 [T, H*dim]."""
+        ``max_q_len``: the most tokens a request brings, if known (``_in_chunks``).  Returns o float32 [T, H*dim], or with ``gated`` (gate, weight, eps,
+        act) ``head_norm_gate`` of it."""
         T = r.shape[0]
         out = torch.empty((T, num_heads * dim), dtype=torch.float32, device=r.device)
         if not (r.stride(0) == k.stride(0) == v.stride(0)):
             raise KernelError("wkv_scan: r, k and v must share a row stride")
         if r.dtype == torch.bfloat16 and self._in_chunks(2, T, num_seqs, max_q_len, num_heads, dim, dim, r, k, v):
-            self._matrix_chunks(2, r, k, v, None, 0.0, decay, u, state, None, None, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, dim, 1.0)
-            return out
+            return self._matrix_chunks(2, r, k, v, None, 0.0, decay, u, state, None, None, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim,
+                                       dim, 1.0, gated=gated)
         self._check(self.lib.ttie_wkv_scan(_ptr(r), _ptr(k), _ptr(v), r.stride(0), _ptr(decay), _ptr(u),
                                            _ptr(state), state.shape[0], _ptr(x), x.stride(0), x.shape[1], _ptr(prev), prev.shape[0],
                                            _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), _ptr(out), num_heads, dim,
                                            self._dt(r), self._stream(r)), "wkv_scan")
         self.launches += 1
-        return out
+        return self._gated(out, gated, num_heads, dim)
 
     def mlstm_gates(self, pre, m, n, query_start_loc, slot_ids, num_seqs, num_heads, cap):
         """Per token and head (state decay, input weight, exp(-running maximum)) from the gate pre-activations ``pre`` float32
@@ -1561,11 +1563,11 @@ class CudaOps:
         self.launches += 1
         return out, snap
 
-    def mlstm_scan(self, q, k, v, gates, S, n, n_before, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, q_scale):
+    def mlstm_scan(self, q, k, v, gates, S, n, n_before, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, q_scale, gated=None):
         """The matrix memory's recurrence over the step's tokens from the state rows S [slots + 1, H, v_dim, padded dim] (advanced
         in place) and from ``n_before``, the copy of the normaliser state that ``mlstm_gates`` made (the new one is written
         into ``n`` [slots + 1, H, padded dim]).  q, k [T, H*dim], v [T, H*v_dim]: views with one row stride; ``gates`` from
-        ``mlstm_gates``.  Returns o float32 [T, H*v_dim]."""
+        ``mlstm_gates``.  Returns o float32 [T, H*v_dim], or with ``gated`` (gate, weight, eps, act) ``head_norm_gate`` of it."""
         T = q.shape[0]
         out = torch.empty((T, num_heads * v_dim), dtype=torch.float32, device=q.device)
         if not (q.stride(0) == k.stride(0) == v.stride(0)):
@@ -1574,20 +1576,20 @@ class CudaOps:
                                              S.shape[0], _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), _ptr(out), num_heads,
                                              dim, v_dim, float(q_scale), self._dt(q), self._stream(q)), "mlstm_scan")
         self.launches += 1
-        return out
+        return self._gated(out, gated, num_heads, v_dim)
 
     def mlstm_in_chunks(self, q, k, v, num_seqs, dim, v_dim, max_q_len=None):
         """Whether ``mlstm_chunks`` takes this step (in place of ``mlstm_gates`` and ``mlstm_scan``)."""
         return (q.dtype == torch.bfloat16 and self._in_chunks(1, q.shape[0], num_seqs, max_q_len, q.shape[1] // dim, dim, v_dim, q, k, v)
                 and q.stride(0) == k.stride(0) == v.stride(0))
 
-    def mlstm_chunks(self, q, k, v, pre, S, n, m, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, cap, q_scale, pre_bias=None):
+    def mlstm_chunks(self, q, k, v, pre, S, n, m, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, cap, q_scale, pre_bias=None, gated=None):
         """The matrix memory over a step with a prompt portion, in chunks of tokens: ``mlstm_gates`` and ``mlstm_scan`` in one.  ``pre``:
         the gates' pre-activations float32 [T, 2H]; the state rows S, n and m are advanced in place.  ``pre_bias`` (bfloat16 [2H], where
-        ``mlstm_adds_bias``): added to ``pre``.  Returns o float32 [T, H*v_dim]."""
+        ``mlstm_adds_bias``): added to ``pre``.  Returns o float32 [T, H*v_dim], or with ``gated`` (gate, weight, eps, act) ``head_norm_gate`` of it."""
         out = torch.empty((q.shape[0], num_heads * v_dim), dtype=torch.float32, device=q.device)
-        self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale, pre_bias)
-        return out
+        return self._matrix_chunks(1, q, k, v, pre, cap, None, None, S, n, m, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim,
+                                   q_scale, pre_bias, gated)
 
     def mlstm_adds_bias(self, v, num_seqs, pad, v_dim) -> bool:
         """Whether ``mlstm_chunks`` takes the gates' bias (a sum apart costs two small kernels, 5 us of a layer's 127)."""
@@ -1651,7 +1653,8 @@ class CudaOps:
             return 64
         return 128 if num_tokens >= 100 * num_seqs or (num_tokens // 128 + num_seqs) * num_heads <= 1.5 * num_sms else 64
 
-    def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale, pre_bias=None):
+    def _matrix_chunks(self, mode, q, k, v, pre, cap, decay, u, S, n, m, x, prev, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, q_scale, pre_bias=None,
+                       gated=None):
         T, pad = q.shape[0], S.shape[-1]
         tokens = self._chunk_tokens(mode, v.dtype, T, num_seqs, pad, v_dim, num_heads, self.num_sms)
         total = T // tokens + num_seqs                                 # chunk numbers of the step
@@ -1662,12 +1665,36 @@ class CudaOps:
         part = space.data_ptr()
         aux = part + 4 * slots * states
         span = aux + 4 * slots * sums
+        y = gate = weight = None
+        eps = act = 0
+        if self._gates_in_chunks(gated, mode, tokens, pad):
+            gate, weight, eps, act = gated
+            y, act = torch.empty((T, num_heads * v_dim), dtype=gate.dtype, device=q.device), self._GATES[act]
         self._check(self.lib.ttie_matrix_chunks(
             mode, _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), self._dt(v), _ptr(pre), 0 if pre is None else pre.stride(0), float(cap),
             _ptr(decay), _ptr(u), _ptr(S), _ptr(n), _ptr(m), S.shape[0], _ptr(x), 0 if x is None else x.stride(0), 0 if x is None else x.shape[1],
             _ptr(prev), 0 if prev is None else prev.shape[0], _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), T, _ptr(out), num_heads, dim,
-            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, tokens, _ptr(pre_bias), self._stream(q)), "matrix_chunks")
+            v_dim, pad, float(q_scale), part, aux, span, span + 16 * slots * num_heads, slots, tokens, _ptr(pre_bias), _ptr(y), _ptr(gate),
+            0 if gate is None else gate.stride(0), _ptr(weight), float(eps), act, self._stream(q)), "matrix_chunks")
         self.launches += 3 * -(-total // slots)
+        return y if y is not None else self._gated(out, gated, num_heads, v_dim)
+
+    _GATES = {"silu": 0, "sigmoid": 1}
+
+    @staticmethod
+    def _gates_in_chunks(gated, mode, tokens, pad) -> bool:
+        """Whether the chunks' last kernel norms and gates the read-outs itself: where a block has all columns of a head (chunks of 128 tokens;
+        wkv's of 64 for heads of up to 64) and the gate's rows take loads of 16 bytes.  us of the scan with a pass over the read-outs
+        apart | without, one request of 2,048 tokens (of 300): retention of 16 heads of 128 x 128 74 | 65 (32 | 30), mlstm of 64 x 128 56 | 49
+        (28 | 26), wkv of 32 heads of 64 101 | 97 (40 | 38), and a launch less: 8 us of the host's time."""
+        if gated is None or not (tokens == 128 or (mode == 2 and pad <= 64)):
+            return False
+        gate, weight = gated[0], gated[1]
+        return (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0
+                and (weight is None or weight.data_ptr() % 8 == 0))
+
+    def _gated(self, o, gated, num_heads, v_dim):
+        return o if gated is None else self.head_norm_gate(o, gated[0], gated[1], num_heads, v_dim, gated[2], gated[3])
 
     def rotate_heads(self, src, heads, dim, cs_table, rot, style, scale_from=None, scale=1.0):
         """float32 [T, heads * dim]: the ``heads`` head rows of ``dim`` values at the start of every row of ``src`` (a view with a
@@ -1681,11 +1708,11 @@ class CudaOps:
         self.launches += 1
         return out
 
-    def retention_scan(self, q, k, v, decay, S, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, max_q_len=None):
+    def retention_scan(self, q, k, v, decay, S, query_start_loc, slot_ids, num_seqs, num_heads, dim, v_dim, max_q_len=None, gated=None):
         """Retention's recurrence over the step's tokens from the state rows S [slots + 1, H, v_dim, padded dim] (advanced in
         place): S <- decay_h S + k v^T, o = S^T q.  q, k float32 [T, H*dim] views with one row stride; v [T, H*v_dim] in the
         compute dtype, a view with a row stride; ``decay`` float32 [H].  ``max_q_len``: the most tokens a request brings, if known.
-        Returns o float32 [T, H*v_dim].
+        Returns o float32 [T, H*v_dim], or with ``gated`` (gate, weight, eps, act) ``head_norm_gate`` of it.
 
         A step with a prompt portion runs in chunks of 64 tokens (``_in_chunks``).  Head sizes that those do not take are walked
         token by token, and a long prompt (the step's tokens less one for every other request: the host knows no more, and
@@ -1696,15 +1723,15 @@ class CudaOps:
         if q.stride(0) != k.stride(0) or q.dtype != torch.float32 or k.dtype != torch.float32:
             raise KernelError("retention_scan: q and k must be float32 and share a row stride")
         if self._in_chunks(0, T, num_seqs, max_q_len, num_heads, dim, v_dim, q, k, v):
-            self._matrix_chunks(0, q, k, v, None, 0.0, decay, None, S, None, None, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim, v_dim, 1.0)
-            return out
+            return self._matrix_chunks(0, q, k, v, None, 0.0, decay, None, S, None, None, None, None, query_start_loc, slot_ids, num_seqs, out, num_heads, dim,
+                                       v_dim, 1.0, gated=gated)
         parts = self.retention_parts(T, int(num_seqs), S[0].numel())
         scratch = torch.empty((int(num_seqs) * parts,) + tuple(S.shape[1:]), dtype=torch.float32, device=q.device) if parts > 1 else None
         self._check(self.lib.ttie_retention_scan(_ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(decay), _ptr(S), S.shape[0],
                                                  _ptr(query_start_loc), _ptr(slot_ids), int(num_seqs), _ptr(out), num_heads, dim, v_dim,
                                                  parts, _ptr(scratch), self._dt(v), self._stream(q)), "retention_scan")
         self.launches += 2 if parts > 1 else 1
-        return out
+        return self._gated(out, gated, num_heads, v_dim)
 
     retention_part_tokens = 256             # a long prompt is walked in parts of about this many tokens,
     retention_max_parts = 16                # at most this many a request,
@@ -1727,7 +1754,7 @@ class CudaOps:
         T = o.shape[0]
         out = torch.empty((T, num_heads * v_dim), dtype=gate.dtype, device=o.device)
         self._check(self.lib.ttie_head_norm_gate(_ptr(o), _ptr(gate), gate.stride(0), _ptr(weight), T, num_heads, v_dim, float(eps),
-                                                 {"silu": 0, "sigmoid": 1}[act], _ptr(out), self._dt(gate), self._stream(o)),
+                                                 self._GATES[act], _ptr(out), self._dt(gate), self._stream(o)),
                     "head_norm_gate")
         self.launches += 1
         return out

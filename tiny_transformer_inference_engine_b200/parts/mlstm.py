@@ -76,12 +76,12 @@ class MLSTM(Mixer):
         in_chunks = hasattr(ops, "mlstm_chunks") and ops.mlstm_in_chunks(q, k, v, ctx.num_seqs, D, Dv, ctx.max_q_len)
         bias = self.b_gates if in_chunks and ops.mlstm_adds_bias(v, ctx.num_seqs, S.state.shape[-1], Dv) else None
         gates = ops.linear(x, self.w_gates, self.b_gates if bias is None else None, out_dtype=torch.float32)             # [T, 2H] float32
+        gated = g, self.norm_w, self.eps, "sigmoid"
         if in_chunks:
-            o = ops.mlstm_chunks(q, k, v, gates, S.state, nrm.state, mx.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, Dv,
-                                 self.gate_cap, D ** -0.5, pre_bias=bias)
+            y = ops.mlstm_chunks(q, k, v, gates, S.state, nrm.state, mx.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, Dv,
+                                 self.gate_cap, D ** -0.5, pre_bias=bias, gated=gated)
         else:
             weights, n_before = ops.mlstm_gates(gates, mx.state, nrm.state, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, self.gate_cap)
-            o = ops.mlstm_scan(q, k, v, weights, S.state, nrm.state, n_before, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs,
-                               H, D, Dv, D ** -0.5)
-        y = ops.head_norm_gate(o, g, self.norm_w, H, Dv, self.eps, "sigmoid")
+            y = ops.mlstm_scan(q, k, v, weights, S.state, nrm.state, n_before, ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs,
+                               H, D, Dv, D ** -0.5, gated=gated)
         return ops.linear(y, self.w_out, None, partial_ok=True)

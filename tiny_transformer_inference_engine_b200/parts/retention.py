@@ -103,8 +103,9 @@ class Retention(Mixer):
             rot = self.rot_dim if inv_freq is not None else 0
             cs = self.position.step_table(ctx) if rot else None
             qk = ops.rotate_heads(proj, 2 * H, D, cs, rot, style, scale_from=H, scale=self.key_scale)   # float32 [T, q | k]
-        o = ops.retention_scan(qk[:, :H * D], qk[:, H * D:2 * H * D], v, self.decay_t, S.state, ctx.query_start_loc, ctx.slot_ids,
-                               ctx.num_seqs, H, D, Dv, max_q_len=ctx.max_q_len)
-        heads, width = (1, H * Dv) if self.norm_over == "all" else (H, Dv)
-        y = ops.head_norm_gate(o, g, self.norm_w, heads, width, self.eps, self.gate_act)
+        gated = g, self.norm_w, self.eps, self.gate_act
+        y = ops.retention_scan(qk[:, :H * D], qk[:, H * D:2 * H * D], v, self.decay_t, S.state, ctx.query_start_loc, ctx.slot_ids,
+                               ctx.num_seqs, H, D, Dv, max_q_len=ctx.max_q_len, gated=None if self.norm_over == "all" else gated)
+        if self.norm_over == "all":
+            y = ops.head_norm_gate(y, g, self.norm_w, 1, H * Dv, self.eps, self.gate_act)
         return ops.linear(y, self.w_out, None, partial_ok=True)

@@ -90,7 +90,6 @@ class WKV(Mixer):
         rkvg = ops.batched_linear(mixes[:4], self.w_rkvg)                                                         # [4, T, H*dim]
         lora = ops.activation(ops.linear(mixes[4], self.w1, None, out_dtype=torch.float32), "tanh", out_dtype=x.dtype)
         wlog = ops.linear(lora, self.w2, None, out_dtype=torch.float32)                                           # [T, H*dim] float32
-        o = ops.wkv_scan(rkvg[0], rkvg[1], rkvg[2], ops.wkv_decay(wlog, self.w0), self.u, S.state, x, prev.state,
-                         ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, max_q_len=ctx.max_q_len)
-        y = ops.head_norm_gate(o, rkvg[3], self.norm_w, H, D, self.eps, "silu")
+        y = ops.wkv_scan(rkvg[0], rkvg[1], rkvg[2], ops.wkv_decay(wlog, self.w0), self.u, S.state, x, prev.state,
+                         ctx.query_start_loc, ctx.slot_ids, ctx.num_seqs, H, D, max_q_len=ctx.max_q_len, gated=(rkvg[3], self.norm_w, self.eps, "silu"))
         return ops.linear(y, self.w_out, None, partial_ok=True)
