@@ -110,6 +110,8 @@ _SIGNATURES = {
     "ttie_token_gate": [_c_void, _c_void, _c_int, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_int, _c_void],
     "ttie_moe_route": [_c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void, _c_void, _c_void, _c_void],
     "ttie_moe_plan_table": [_c_void, _c_int, _c_ll, _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_void, _c_void, _c_void, _c_void],
+    "ttie_moe_route_plan": [_c_void, _c_ll, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void, _c_void, _c_void, _c_int, _c_int, _c_void,
+                            _c_void, _c_void, _c_void, _c_void, _c_void],
     "ttie_moe_plan": [_c_void, _c_int, _c_int, _c_int, _c_int, _c_void, _c_void, _c_void, _c_void, _c_void, _c_void],
     "ttie_grouped_gemm": [_c_void, _c_ll, _c_void, _c_int, _c_void, _c_ll, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_int, _c_int, _c_int,
                           _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_float, _c_void],
@@ -1878,17 +1880,39 @@ class CudaOps:
         the row-tile table and its size bound.  The last ``identity`` of the ``num_experts`` own no matrices: their pairs are
         sorted behind the others and get no row tiles."""
         P = idx.numel()
-        tile = int(self.lib.ttie_moe_tile_rows())
-        max_tiles = P // tile + num_experts
-        buf = torch.empty(2 * P + num_experts + 1 + 4 * max_tiles + 4, dtype=torch.int32, device=idx.device)
-        plan = {"pos_of_pair": buf[:P], "pair_of_pos": buf[P:2 * P], "offsets": buf[2 * P:2 * P + num_experts + 1],
-                "tiles": buf[2 * P + num_experts + 1:2 * P + num_experts + 1 + 4 * max_tiles], "meta": buf[-4:], "max_tiles": max_tiles,
-                "pairs": P, "idx": idx, "real_experts": num_experts - int(identity)}
-        self._check(self.lib.ttie_moe_plan(_ptr(idx), P, num_experts, num_experts - int(identity), max_tiles, _ptr(plan["offsets"]), _ptr(plan["pos_of_pair"]),
-                                           _ptr(plan["pair_of_pos"]), _ptr(plan["tiles"]), _ptr(plan["meta"]), self._stream(idx)),
-                    "moe_plan")
+        plan = self._plan_of(idx, P, num_experts, identity)
+        self._check(self.lib.ttie_moe_plan(_ptr(idx), P, num_experts, num_experts - int(identity), plan["max_tiles"], _ptr(plan["offsets"]),
+                                           _ptr(plan["pos_of_pair"]), _ptr(plan["pair_of_pos"]), _ptr(plan["tiles"]), _ptr(plan["meta"]),
+                                           self._stream(idx)), "moe_plan")
         self.launches += 1
         return plan
+
+    def _plan_of(self, idx, P, num_experts, identity):
+        """A plan's tensors, not yet filled."""
+        max_tiles = P // int(self.lib.ttie_moe_tile_rows()) + num_experts
+        tiles = (2 * P + num_experts + 1 + 3) & ~3                      # (a tile's four numbers are written at once)
+        buf = torch.empty(tiles + 4 * max_tiles + 4, dtype=torch.int32, device=idx.device)
+        return {"pos_of_pair": buf[:P], "pair_of_pos": buf[P:2 * P], "offsets": buf[2 * P:2 * P + num_experts + 1],
+                "tiles": buf[tiles:tiles + 4 * max_tiles], "meta": buf[-4:], "max_tiles": max_tiles,
+                "pairs": P, "idx": idx, "real_experts": num_experts - int(identity)}
+
+    route_plan_tokens = 32                  # tokens up to which routing and plan are one launch (one CTA, a warp a token)
+
+    def moe_route_plan(self, logits, groups, keep, group_top, top, scale, renorm=False, score="sigmoid", correction=None, identity=0):
+        """(expert ids, weights, plan): ``moe_route`` and the ``moe_plan`` of its choices, for few tokens in one launch."""
+        T, E = logits.shape
+        if not (1 <= T <= self.route_plan_tokens and 1 <= top <= E <= 32 and groups == keep == 1 and group_top in (1, 2)):
+            idx, wts = self.moe_route(logits, groups, keep, group_top, top, scale, renorm, score=score, correction=correction)
+            return idx, wts, self.moe_plan(idx, E, identity=identity)
+        idx = torch.empty((T, top), dtype=torch.int32, device=logits.device)
+        wts = torch.empty((T, top), dtype=torch.float32, device=logits.device)
+        plan = self._plan_of(idx, T * top, E, identity)
+        self._check(self.lib.ttie_moe_route_plan(_ptr(logits), logits.stride(0), T, E, top, float(scale), 1 if renorm else 0,
+                                                 {"sigmoid": 0, "softmax": 1}[score], _ptr(correction), _ptr(idx), _ptr(wts), plan["real_experts"],
+                                                 plan["max_tiles"], _ptr(plan["offsets"]), _ptr(plan["pos_of_pair"]), _ptr(plan["pair_of_pos"]),
+                                                 _ptr(plan["tiles"]), _ptr(plan["meta"]), self._stream(logits)), "moe_route_plan")
+        self.launches += 1
+        return idx, wts, plan
 
     def moe_plan_table(self, tables, token_ids, num_experts):
         """``moe_plan`` for experts that tables name: row ``token_ids[t]`` of layer l's table (``tables`` int32 [layers, vocab, top])

@@ -166,9 +166,8 @@ class GroupedMoE(FeedForward):
             return self._table_forward(x, ctx)
         all_logits = ops.linear(x, self.w_router, None, out_dtype=torch.float32)
         logits = all_logits[:, :self.routed]
-        idx, wts = ops.moe_route(logits, self.groups, self.keep, self.group_top, self.top, self.scale, self.renorm,
-                                 score=self.score, correction=self.correction)
-        plan = ops.moe_plan(idx, self.routed, identity=self.identity)
+        _, wts, plan = ops.moe_route_plan(logits, self.groups, self.keep, self.group_top, self.top, self.scale, self.renorm,
+                                          score=self.score, correction=self.correction, identity=self.identity)
         if self.experts and self.expert_kind == "mlp":
             act = ops.grouped_act(x, self.w_gu, plan, self.top, self.act, row_scale=wts if self.weight_on_input else None)
             y = ops.grouped_linear(act, self.w_down, plan, out_dtype=torch.float32)
