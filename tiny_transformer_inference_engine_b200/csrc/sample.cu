@@ -31,6 +31,16 @@ __device__ __forceinline__ unsigned ordered_key(float x) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+__device__ __forceinline__ float value_of_key(unsigned key) { return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key); }
+
+// the warp's largest value (no NaN among them) and the lowest index that holds it
+__device__ __forceinline__ void warp_best(float& best, int& best_i) {
+    const unsigned key = ordered_key(best + 0.f);                    // (minus zero and zero are equal)
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    best_i = (int)__reduce_min_sync(0xffffffffu, key == top ? (unsigned)best_i : 0x7fffffffu);
+    best = value_of_key(top);
+}
+
 __device__ __forceinline__ u64 mass_of(float y, float ymax) {
     return (u64)(expf(y - ymax) * 1099511627776.0f);                 // 2^40
 }
@@ -147,6 +157,96 @@ __device__ __forceinline__ void all_gather(T* buf, int n, T v, unsigned rank) {
     }
 }
 
+// The rest of the way of a short list by comparing all pairs (neighbouring lanes share a token), with a barrier between one decision and the next.  The
+// tokens and the mass above a token decide both cuts: a token is among the k largest iff fewer than k are larger, and stays under
+// top-p iff the mass of the larger ones (which stay if it does) is at most top_p of the mass of the k largest.  The mass down to the
+// last token that stays is the mass of all that do, and a scan of the masses that stay places the draw.  Equal keys have equal
+// masses.  Sums of integers: the order is nothing.
+struct Draw { unsigned seed_lo, seed_hi, draws; int top_k; float top_p; int best_i; };
+__device__ __forceinline__ void draw_from_list(const unsigned* l_key, const u64* l_mass, const int* tok, int total, const Draw d, const u64* z_row, int* out, int* st,
+                                            float* probs, int V) {
+    __shared__ unsigned s_prefix, s_draw;
+    __shared__ u64 s_acc, s_total, s_warp[THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) { s_prefix = 0xffffffffu; s_acc = s_total = 0; }
+    __syncthreads();                                                  // (the list is there as well)
+    int sh = 0;
+    while (sh < 4 && (total << (sh + 1)) <= (total > 64 ? THREADS : THREADS / 2)) ++sh;
+    const int i = tid >> sh, part = tid & ((1 << sh) - 1);
+    const bool busy = (tid & ~31) >> sh < total;                      // (whole warps)
+    const unsigned key = i < total ? l_key[i] : 0u;
+    const u64 mass = i < total ? l_mass[i] : 0;
+    int counts = 0;                                                   // of the equal tokens (high half), and with the larger ones
+    u64 down_to = 0;                                                  // mass of the larger and the equal ones
+    if (busy) {
+        if (i < total) {
+#pragma unroll 4
+            for (int j = part; j < total; j += 1 << sh) {
+                const unsigned other = l_key[j];
+                const u64 m = l_mass[j];
+                if (other >= key) { ++counts; down_to += m; }
+                if (other == key) counts += 1 << 16;
+            }
+        }
+        for (int o = 1; o < (1 << sh); o <<= 1) {
+            counts += __shfl_xor_sync(0xffffffffu, counts, o);
+            down_to += __shfl_xor_sync(0xffffffffu, down_to, o);
+        }
+    }
+    const int upto = counts & 0xffff, above = upto - (counts >> 16);
+    const u64 more = down_to - (u64)(unsigned)(counts >> 16) * mass;  // mass of the larger ones
+    const int k = d.top_k > 0 && d.top_k < V ? d.top_k : 0x7fffffff;
+    bool stays = i < total && above < k, last = upto >= k || upto == total;       // last: no smaller token stays
+    if (warp == THREADS / 32 - 1) {                                   // (the warp that has least to do)
+        unsigned rnd[4];
+        philox4x32_10(d.draws, 0u, 0u, 0u, d.seed_lo, d.seed_hi, rnd);
+        if (lane == 0) s_draw = rnd[0];
+    }
+    if (d.top_p < 1.0f) {
+        u64 z;
+        if (z_row) z = *z_row;                                        // (top-p alone: of the whole row)
+        else {
+            if (stays && last) s_acc = down_to;                       // (several write the same value)
+            __syncthreads();
+            z = s_acc;
+        }
+        const u64 limit = (u64)((double)d.top_p * (double)z);
+        stays = stays && more <= limit;
+        last = last || down_to > limit;
+    }
+    if (stays && last) { s_prefix = key; s_total = down_to; }
+    if (tid == 0) { *out = d.best_i; st[2] = (int)(d.draws + 1); }    // (what is not finite may have no mass at all)
+    __syncthreads();
+    const unsigned cut_key = s_prefix;
+    const u64 all = s_total;
+    const double u = (double)(s_draw >> 8) * (1.0 / 16777216.0);
+    u64 target = (u64)(u * (double)all);
+    if (target >= all) target = all ? all - 1 : 0;
+    const bool kept = part == 0 && i < total && key >= cut_key;
+    u64 incl = kept ? mass : 0, below = 0;
+    if (busy) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+    }
+    __syncthreads();
+    if (busy) {
+        below = lane < warp ? s_warp[lane] : 0;                       // (all of them are busy)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+        below += incl - (kept ? mass : 0);
+    }
+    if (kept && target >= below && target < below + mass) *out = tok[i];
+    if (probs) {                                                      // this CTA is the only one left: the whole row is its to write
+        for (int t = tid; t < V; t += THREADS) probs[t] = 0.f;
+        __syncthreads();
+        if (kept) probs[tok[i]] = (float)((double)mass * (all ? 1.0 / (double)all : 0.0));
+    }
+}
+
 // One row of logits is shared by C CTAs: CTA `rank` owns tokens [v0, v1) and keeps them (divided by the temperature)
 // in its shared memory after the first pass, so the later passes do not go back to global memory; a slice too long
 // for that (staged == 0) is read from global memory every time.  Maxima, histograms and sums of the slices are
@@ -154,13 +254,17 @@ __device__ __forceinline__ void all_gather(T* buf, int n, T v, unsigned rank) {
 //
 // With a top-k of a few hundred at most the row is left after two walks.  Every warp knows the largest value among its
 // own tokens from the first walk, and the exchange that finds the row's maximum brings all of them to every CTA: the k-th largest
-// of the row's 32 C such values is a bound that at least k tokens of the row reach, so nothing below it can be among the
-// k largest (8 CTAs, k 32: some 40 tokens are left; 8 rows of 32,000 tokens take 15.3 us, 29.1 when every CTA took the k-th largest of
-// its own threads' maxima by a radix select, which left 300).  Where k is more than a quarter of the warps, a CTA's bound is that radix select.
-// The tokens at or above the bound are gathered in token order, handed to the first CTA of the cluster, and that CTA alone does the exact top-k
+// of them (of groups of them, where that leaves twice k or more) is a bound that at least k tokens of the row reach, so nothing below it can be among
+// the k largest (8 CTAs, k 32: 64 groups, some 44 tokens are left).  Where k is more than a quarter of the warps, a CTA's bound is the k-th largest
+// of its own threads' maxima, by a radix select (300 tokens left).
+// The tokens at or above the bound go to the first CTA of the cluster, in token order, in the same exchange that tells every CTA how many there are
+// (a CTA with more than 512 / C of them: in one of its own), and that CTA alone does the exact top-k
 // cut, top-p and the draw on the list (`list_cap` entries fit the shared memory that held its slice).  A list of up to SMALL_LIST
-// tokens needs no radix select for that: every token counts the tokens and the mass above it, which decides both cuts at once.  If the list would
+// tokens needs no radix select for that (draw_from_list).  If the list would
 // overflow (thousands of equal values at the bound), every CTA goes on with its whole slice instead.
+// What bounds all this is latency.  8 rows of 32,000 tokens, k 32, top-p 0.9: clocks to the row's maximum 6,300 -> 4,700, the bound 5,600 -> 1,600 (of
+// 256 keys, each compared with all), the list and its way 5,000 -> 4,500 (two exchanges), cuts and draw 8,600 -> 3,900 (12 barriers, sums by
+// shuffles and atomics); the launch 13.7 -> 8.3 us, k 1 12.8 -> 7.6, 32 rows 18.5 -> 15.6, 256,000 tokens 20.2 -> 14.1.
 // Top-p without a top-k leaves the row the same way when the distribution is peaked: the (at most 1,024) tokens that hold
 // 1 / 1,024 of the row's mass or more each are listed, and if together they hold more than top_p of the mass the cut lies
 // among them.  A flat row (the listed tokens hold too little) is walked whole as before.
@@ -173,17 +277,21 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     __shared__ int s_idx[32];
     __shared__ u64 s_u64[32];
     __shared__ u64 s_hist[256];
-    __shared__ u64 x_hist[2][C * 256];                               // exchange buffers, by exchange parity
+    __shared__ __align__(16) u64 x_hist[2][C * 256];                 // exchange buffers, by exchange parity
     __shared__ u64 x_u64[2][C];
     __shared__ u64 x_best[C * (THREADS / 32)];                        // every warp's maximum: place (high word) and value
     __shared__ int x_cnt[C];
     __shared__ float c_y[KEEP_CAP];                                   // this slice's tokens for the short list: value ...
     __shared__ int c_i[KEEP_CAP];                                     // ... and place in the slice
     __shared__ int s_scan[THREADS / 32];
-    // a short list's masses and keys: they lie where the slices' histograms are exchanged while there is no list
+    // a short list's masses and keys, and what the cluster's CTAs hand in for it: they lie where the slices' histograms are exchanged while there is no list
+    static_assert(SMALL_LIST % 2 == 0, "the keys are read 16 bytes at a time");
     static_assert(SMALL_LIST * 12 <= 2 * 256 * 8 && 8 * (THREADS / 32) <= SMALL_LIST, "one CTA's exchange buffers hold a short list");
     u64* l_mass = &x_hist[0][0];
     unsigned* l_key = reinterpret_cast<unsigned*>(l_mass + SMALL_LIST);
+    constexpr int HAND_IN = 512 / C;                                  // tokens (id, value) that a CTA may hand in right away
+    __shared__ u64 one_hand_in[C == 1 ? 512 : 1];
+    u64* handed = C == 1 ? one_hand_in : &x_hist[0][512];
     __shared__ unsigned s_prefix;
     __shared__ u64 s_acc;
     __shared__ int s_found;
@@ -194,6 +302,9 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     const int r = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int v0 = min(V, (int)rank * slice), n = min(V, v0 + slice) - v0;     // this CTA's tokens: v0 .. v0 + n - 1
     const float* row = logits + (size_t)r * V + v0;
+    const bool wide = staged && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+    float4 first = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);        // (on its way while the request's state is looked up)
+    if (wide && tid * 4 < n) first = *reinterpret_cast<const float4*>(row + tid * 4);
     const int slot = slot_ids[r];
     if (slot < 0) {                                                   // a padding row of a fixed-size batch: no request, no draw
         if (tid == 0 && rank == 0) out[r] = 0;
@@ -211,9 +322,9 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
 
     // 1. maximum and the lowest index that holds it (and the slice into shared memory)
     float best = -INFINITY; int best_i = 0x7fffffff;
-    if (staged && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+    if (wide) {
         for (int i = tid * 4; i < n; i += THREADS * 4) {
-            const float4 x = *reinterpret_cast<const float4*>(row + i);
+            const float4 x = i == tid * 4 ? first : *reinterpret_cast<const float4*>(row + i);
             *reinterpret_cast<float4*>(s_row + i) = x;
             const float xs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -228,12 +339,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
         }
     }
     const float my_best = best;                                       // the largest among this thread's tokens (-inf: it has none)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-        if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
-    }
+    warp_best(best, best_i);
     if (lane == 0) { s_val[warp] = best; s_idx[warp] = best_i == 0x7fffffff ? 0x7fffffff : best_i + v0; }
     __syncthreads();
     // every warp's maximum to every CTA in one exchange; the row's is the largest of them (lower tokens win ties)
@@ -248,12 +354,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
         const int oi = (int)(x >> 32);
         if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-        if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
-    }
+    warp_best(best, best_i);
     if (best_i == 0x7fffffff) best_i = 0;                            // a row of NaNs: report token 0
     if (greedy) {
         if (tid == 0 && rank == 0) { out[r] = best_i; st[2] = (int)(draws + 1); }
@@ -302,24 +403,34 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     unsigned low_key = 0;                                             // the list takes every token at or above this key
     u64 z_row = 0, limit_row = 0;                                     // top-p alone: the row's whole mass and top_p of it
     bool have_z = false;
-    constexpr int GROUPS = C * (THREADS / 32), PER_GROUP = THREADS / GROUPS;
+    constexpr int GROUPS = C * (THREADS / 32);
     if (staged && list_cap > 0 && top_k > 0 && top_k < V && 4 * top_k <= GROUPS) {
-        // (a) the bound: the top_k-th largest of the row's warps' maxima, PER_GROUP neighbouring lanes counting for each
-        const int g = tid / PER_GROUP;
-        if (tid < GROUPS) l_key[tid] = ordered_key(__uint_as_float((unsigned)x_best[tid]) / temperature);
+        // (a) the bound: the top_k-th largest of the maxima of G groups of the row's warps, twice top_k of them or more; four neighbouring lanes count
+        // for each
+        // (slices of fewer tokens leave warps without any, and their bounds with nothing to choose from)
+        const int G = slice <= THREADS * 4 - 128 ? GROUPS : GROUPS > 64 && top_k <= 32 ? 64 : GROUPS > 128 ? 128 : GROUPS;
+        if (tid < G) {
+            float x = -INFINITY;
+            for (int j = tid; j < GROUPS; j += G) x = fmaxf(x, __uint_as_float((unsigned)x_best[j]));
+            l_key[tid] = ordered_key((x == 0.f ? -0.f : x) / temperature);       // (the maximum of both zeros is the larger key, which may not be there)
+        }
         __syncthreads();
-        const unsigned key = l_key[g];
-        int above = 0, same = 0;
-        for (int j = tid % PER_GROUP; j < GROUPS; j += PER_GROUP) {
-            const unsigned other = l_key[j];
-            above += other > key; same += other == key;
-        }
+        const int g = tid >> 2;
+        if ((tid & ~31) < 4 * G) {                // (whole warps)
+            const unsigned key = l_key[min(g, G - 1)];
+            int above = 0, same = 0;
+            for (int j = tid & 3; j < G / 4; j += 4) {
+                const uint4 o = reinterpret_cast<const uint4*>(l_key)[j];
+                above += (int)(o.x > key) + (int)(o.y > key) + ((int)(o.z > key) + (int)(o.w > key));
+                same += (int)(o.x == key) + (int)(o.y == key) + ((int)(o.z == key) + (int)(o.w == key));
+            }
 #pragma unroll
-        for (int o = 1; o < PER_GROUP; o <<= 1) {
-            above += __shfl_xor_sync(0xffffffffu, above, o);
-            same += __shfl_xor_sync(0xffffffffu, same, o);
+            for (int o = 1; o < 4; o <<= 1) {
+                above += __shfl_xor_sync(0xffffffffu, above, o);
+                same += __shfl_xor_sync(0xffffffffu, same, o);
+            }
+            if (g < G && above < top_k && above + same >= top_k) s_prefix = key;      // (several write the same value)
         }
-        if (above < top_k && above + same >= top_k) s_prefix = key;   // (several write the same value)
         __syncthreads();
         low_key = s_prefix; try_list = true;
     } else if (staged && list_cap > 0 && top_k > 0 && top_k < V && top_k <= LIST_TOP_K) {
@@ -353,8 +464,9 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
         try_list = true; by_mass = true;
     }
     if (try_list) {
-        // (b) the tokens at or above the bound, in token order: a thread counts them in its run of consecutive tokens (an
-        // odd run length: different banks), a scan over the block gives each run its place
+        // (b) the tokens at or above the bound, in token order: a thread counts them in its run of consecutive tokens (an odd run length: different banks), the
+        // sums over the threads and warps before it give each run its place; then they go to the first CTA (if it has room for all of this
+        // CTA's) and into this CTA's own arrays (for a list that takes longer)
         const int run = ((n + THREADS - 1) / THREADS) | 1;
         const int a = min(n, tid * run), b = min(n, a + run);
         int cnt = 0;
@@ -371,38 +483,32 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
         }
         if (lane == 31) s_scan[warp] = incl;
         __syncthreads();
-        if (warp == 0) {
-            int w = s_scan[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += up;
-            }
-            s_scan[lane] = w;
-        }
-        __syncthreads();
-        int at = incl - cnt + (warp ? s_scan[warp - 1] : 0);
-        const int kept = s_scan[THREADS / 32 - 1];
-        if (kept <= KEEP_CAP) {
+        const int others = s_scan[lane];
+        const int kept = __reduce_add_sync(0xffffffffu, others);
+        int at = __reduce_add_sync(0xffffffffu, lane < warp ? others : 0) + incl - cnt;
+        if (cnt && kept <= KEEP_CAP) {
             for (int i = a; i < b; ++i) {
                 const float y = s_row[i];
-                if (ordered_key(y) >= low_key) { c_y[at] = y; c_i[at] = i; ++at; }
+                if (ordered_key(y) < low_key) continue;
+                c_y[at] = y; c_i[at] = i;
+                if (kept <= HAND_IN) {
+                    const u64 entry = (u64)(unsigned)(v0 + i) << 32 | __float_as_uint(y);
+                    if (C > 1) put_remote(handed + (int)rank * HAND_IN + at, 0u, entry);
+                    else handed[at] = entry;
+                }
+                ++at;
             }
         }
         // (c) how many each CTA brings (this exchange also tells that every CTA is done reading its slice)
         int before = 0, total = 0;
-        bool fits = true;
-        if (C > 1) {
-            all_gather<C, int>(x_cnt, 1, kept, rank);
+        bool fits = true, at_hand = true;
+        all_gather<C, int>(x_cnt, 1, kept, rank);
 #pragma unroll
-            for (int k = 0; k < C; ++k) {
-                fits = fits && x_cnt[k] <= KEEP_CAP;
-                if (k < (int)rank) before += x_cnt[k];
-                total += x_cnt[k];
-            }
-        } else {
-            __syncthreads();
-            fits = kept <= KEEP_CAP; total = kept;
+        for (int k = 0; k < C; ++k) {
+            fits = fits && x_cnt[k] <= KEEP_CAP;
+            at_hand = at_hand && x_cnt[k] <= HAND_IN;
+            if (k < (int)rank) before += x_cnt[k];
+            total += x_cnt[k];
         }
         fits = fits && total <= list_cap;
         if (by_mass) {                                                // the list must reach past the cut
@@ -410,61 +516,51 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
             fits = sum_u64(lm, nullptr) > limit_row && fits;
         }
         if (fits) {
-            // (d) into the first CTA's list, slice after slice; the others are done
-            for (int j = tid; j < kept; j += THREADS) {
-                if (C > 1) { put_remote(u_y + before + j, 0u, c_y[j]); put_remote(u_tok + before + j, 0u, v0 + c_i[j]); }
-                else { u_y[j] = c_y[j]; u_tok[j] = v0 + c_i[j]; }
-            }
-            if (C > 1) {
-                cluster_sync_all();
+            // (d) into the first CTA's list, slice after slice; the others are done.  (without top-p the radix select takes four passes, not twelve, and
+            // lists above 256 tokens have two lanes a token instead of four: 8 rows of 4,096 tokens, top-k 65, some 300 listed: 21.8 us by pairs,
+            // 18.6 by radix; with top-p 21.8 and 26.1)
+            const bool pairs = total <= 256 || (total <= SMALL_LIST && top_p < 1.0f);
+            if (pairs && at_hand) {
                 if (rank != 0) return;
+                const int k = tid / HAND_IN, j = tid % HAND_IN;
+                if (k < C && j < x_cnt[k]) {
+                    int to = j;
+                    for (int c = 0; c < k; ++c) to += x_cnt[c];
+                    const u64 entry = handed[tid];
+                    const float y = __uint_as_float((unsigned)entry);
+                    l_key[to] = ordered_key(y); l_mass[to] = mass_of(y, ymax); u_tok[to] = (int)(entry >> 32);
+                }
             } else {
-                __syncthreads();
+                for (int j = tid; j < kept; j += THREADS) {
+                    if (C > 1) { put_remote(u_y + before + j, 0u, c_y[j]); put_remote(u_tok + before + j, 0u, v0 + c_i[j]); }
+                    else { u_y[j] = c_y[j]; u_tok[j] = v0 + c_i[j]; }
+                }
+                if (C > 1) {
+                    cluster_sync_all();
+                    if (rank != 0) return;
+                } else {
+                    __syncthreads();
+                }
+                if (pairs)
+                    for (int i = tid; i < total; i += THREADS) { const float y = u_y[i]; l_key[i] = ordered_key(y); l_mass[i] = mass_of(y, ymax); }
+            }
+            if (pairs) {
+                if (tid == 0) s_acc = z_row;
+                draw_from_list(l_key, l_mass, u_tok, total, {seed_lo, seed_hi, draws, top_k, top_p, best_i}, have_z ? &s_acc : nullptr, out + r, st,
+                               probs_out ? probs_out + (size_t)r * V : nullptr, V);
+                return;
             }
             listed = true; solo = true; n_cur = total;
         }
     }
-
-    // A short list: the tokens and the mass above every token by comparing all pairs (neighbouring lanes share a token), which
-    // decides both cuts - a token is among the k largest iff fewer than k are larger, and stays under top-p iff the mass of the
-    // larger ones (which stay if it does) is at most top_p of the mass of the k largest.  Sums of integers: the order is nothing.
     unsigned cut_key = 0;
-    // (without top-p the radix select takes four passes, not twelve, and lists above 256 tokens have two lanes a token instead of four: 8 rows of
-    // 4,096 tokens, top-k 65, some 300 listed: 21.8 us by pairs, 18.6 by radix; with top-p 21.8 and 26.1)
-    const bool pairs = listed && (n_cur <= 256 || (n_cur <= SMALL_LIST && top_p < 1.0f));
-    if (pairs) {
-        int sh = 0;
-        while (sh < 5 && (n_cur << (sh + 1)) <= THREADS) ++sh;
-        for (int i = tid; i < n_cur; i += THREADS) { const float y = u_y[i]; l_key[i] = ordered_key(y); l_mass[i] = mass_of(y, ymax); }
-        if (tid == 0) s_prefix = 0xffffffffu;
-        __syncthreads();
-        const int i = tid >> sh, part = tid & ((1 << sh) - 1);
-        const unsigned key = i < n_cur ? l_key[i] : 0xffffffffu;
-        int above = 0;
-        u64 mass_above = 0;
-        if (i < n_cur)
-            for (int j = part; j < n_cur; j += 1 << sh)
-                if (l_key[j] > key) { ++above; mass_above += l_mass[j]; }
-        for (int o = 1; o < (1 << sh); o <<= 1) {
-            above += __shfl_xor_sync(0xffffffffu, above, o);
-            mass_above += __shfl_xor_sync(0xffffffffu, mass_above, o);
-        }
-        bool stays = i < n_cur && !(top_k > 0 && top_k < V && above >= top_k);
-        if (top_p < 1.0f) {
-            const u64 z = have_z ? z_row : block_sum_u64(stays && part == 0 ? l_mass[i] : 0, s_u64);
-            stays = stays && mass_above <= (u64)((double)top_p * (double)z);
-        }
-        if (stays && part == 0) atomicMin(&s_prefix, key);
-        __syncthreads();
-        cut_key = s_prefix;
-    }
 
     // The passes below visit every token of the slice several times.  A slice of up to 8 tokens per thread is kept in
     // registers as (key, probability mass) - the mass is computed once, not once per pass - ; a longer one is read from
     // shared (or global) memory and its masses recomputed on each visit.
     constexpr int EPT = 8;
     const int iters = (n_cur + THREADS - 1) / THREADS;             // visits per thread (the same for all: whole warps go round together)
-    const bool cached = !pairs && iters <= EPT && (top_k > 0 || top_p < 1.0f);
+    const bool cached = iters <= EPT && (top_k > 0 || top_p < 1.0f);
     unsigned ck[EPT];
     u64 cm[EPT];
 #pragma unroll
@@ -489,7 +585,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     };
 
     // 2. top-k threshold: the k-th largest key, by radix select over 4 digits of 8 bits
-    if (!pairs && top_k > 0 && top_k < V) {
+    if (top_k > 0 && top_k < V) {
         unsigned prefix = 0; u64 remaining = (u64)top_k;
         for (int shift = 24; shift >= 0; shift -= 8) {
             for (int b = tid; b < 256; b += THREADS) s_hist[b] = 0;
@@ -513,7 +609,7 @@ sample_kernel(const float* __restrict__ logits, int V, int slice, const int* __r
     }
 
     // 3. top-p threshold: the smallest key whose strictly-larger keys hold mass <= top_p * total
-    if (!pairs && top_p < 1.0f) {
+    if (top_p < 1.0f) {
         u64 z = z_row;                                                // (known already if the short list was tried for top-p alone)
         if (!have_z) {
             for_all(true, [&](bool there, unsigned key, u64 mass) { if (there && key >= cut_key) z += mass; });
