@@ -912,6 +912,8 @@ class CudaOps:
                 best, best_cost = (("mma", n, split_len) if n > 1 else ("mma", 1, 0)), cost
         return best
 
+    mixed_head_dim = 256                    # the head size at which decoded tokens and prompt portions run the same kernel
+
     def mixed_plan(self, dtype, num_heads, num_kv_heads, head_dim, page_size, lead, others):
         """Whether a step of ``lead`` requests (decoded tokens) before ``others`` (prompt portions) takes one attention launch for both, where
         both kinds run the same kernel (head size 256): the plan, or None.  ``lead`` and ``others``: (requests, most tokens of one, most keys that its
@@ -931,7 +933,7 @@ class CudaOps:
 
     def _mixed_plan(self, dtype, num_heads, num_kv_heads, head_dim, page_size, lead, others):
         G = num_heads // num_kv_heads
-        if (dtype != torch.bfloat16 or head_dim != 256 or lead[1] * G > 128 or others[1] * G <= 128
+        if (dtype != torch.bfloat16 or head_dim != self.mixed_head_dim or lead[1] * G > 128 or others[1] * G <= 128
                 or not self.lib.ttie_attn_tc_supported(head_dim, page_size)):
             return None
         tiles = (lead[0] * num_kv_heads, others[0] * num_kv_heads * math.ceil(others[1] * G / 128))
@@ -954,9 +956,9 @@ class CudaOps:
     def _tc_wide_plan(self, num_seqs, num_kv_heads, rows, max_kv_len, max_q_len):
         """Head size 256: every step takes the prompt-portion tcgen05 kernel with one 128-row tile per CTA.  Steps of few
         rows (decoded tokens) have their key range cut by the cost model of the one-tile decode kernel, at 20 ns per key
-        (8 heads on one kv head, 2 requests at 1,024 keys: 9.3 us in 8 pieces of 128 against 11.5 in 4; 96 requests at
-        8,192 keys: 132 us in 3 pieces against 153 uncut).  Portions whose row tiles fill less than half of the GPU are cut
-        by the portions' cost model at 21 ns per key (512 tokens behind 2,048 keys: 25.5 us in 4 pieces against 33.0 in 2)."""
+        (8 heads on one kv head, 2 requests at 1,024 keys: 9.5 us in 8 pieces of 128 against 11.2 in 4; 96 requests at
+        8,192 keys: 129 us in 3 pieces against 142 uncut).  Portions whose row tiles fill less than half of the GPU are cut
+        by the portions' cost model at 21 ns per key (512 tokens behind 2,048 keys: 25.3 us in 4 pieces against 32.6 in 2)."""
         base = num_seqs * num_kv_heads * math.ceil(rows / 128)
         if rows <= 128:
             return self._one_per_sm_pieces("tcpp", base, max_kv_len, 0.020, waves_min_keys=640)
@@ -1373,8 +1375,8 @@ class CudaOps:
     def selective_wide(self, dtype, num_tokens: int, num_seqs: int, channels: int, states: int, longest=None) -> bool:
         """Whether a thread owns a channel (16-bit operands, up to 16 states) rather than four states of one: fewer instructions and a
         quarter of the threads, so it needs a step large enough to fill the GPU all the same.  16 states, us of a thread per
-        channel | per four states: 4,096 channels 512 tokens 42 | 40, 1,024 tokens 68 | 73, 2,048 tokens 117 | 141, four requests of
-        512 107 | 134; 2,048 channels 2,048 tokens 73 | 74; 8,192 channels 256 tokens 41 | 39, 512 65 | 70, 2,048 204 | 273.
+        channel | per four states: 4,096 channels 512 tokens 37 | 39, 1,024 tokens 57 | 70, 2,048 tokens 98 | 141, four requests of
+        512 114 | 131; 2,048 channels 2,048 tokens 61 | 72; 8,192 channels 256 tokens 36 | 37, 512 56 | 68, 2,048 184 | 270.
         ``longest``: the most tokens that a request brings, if known.  Beside 23 decoding requests a portion of 2,000 tokens is all there is to
         fill the GPU (8,192 channels 701 in one part, 447 per four states, 260 in eight parts).  Up to four states both forms have a
         thread per channel, and requests of a few tokens do not pay for the runs' staging (150 of 8 tokens 95 | 83)."""

@@ -334,15 +334,14 @@ class PagedAttention(Mixer):
 
     def _mixed_plan(self, dtype, D, ctx, cache, classes):
         """The plan of one attention launch for a step of two classes that lie one behind the other, or None."""
-        plan = getattr(self.ops, "mixed_plan", None)
-        if plan is None or len(classes) != 2:
+        if len(classes) != 2 or D != getattr(self.ops, "mixed_head_dim", None):        # (asked at every layer: before anything that takes time)
             return None
         a, b = classes
         if a.seq_lo or a.tok_lo or (a.seq_hi, a.tok_hi) != (b.seq_lo, b.tok_lo) or b.seq_hi != ctx.num_seqs:
             return None
         step = [(c.seq_hi - c.seq_lo, c.max_q_len, self.ops.visible_keys(c.max_q_len, c.max_kv_len, self.window or 0, self.chunk or 0, self.keep_first),
                  c.tok_hi - c.tok_lo) for c in classes]
-        return plan(dtype, self.num_heads, self.num_kv_heads, D, cache.page_size, *step)
+        return self.ops.mixed_plan(dtype, self.num_heads, self.num_kv_heads, D, cache.page_size, *step)
 
     def _attend(self, q, D, ctx, cache, out):
         """One attention launch per class of requests (decoded tokens; prompt portions), each planned as if it were alone, or one for both
