@@ -1395,7 +1395,7 @@ class CudaOps:
         """Into how many parts a request's tokens are walked: every part but the last is walked twice, which pays while the
         channels alone give the SMs too few warps to hide a token's latency.  With a thread per channel (``wide``) and ``longest`` known the
         warps counted are those of the tokens, as so many requests of that length (a request of one token leaves at once); from 6.5 warps
-        per SM on one part is best (4,096 channels, 16 states, 16 requests of 128 tokens 69 us in one part, 90 in two; 8 of 256 94 and 113, 101 in
+        per SM on one part is best (with the runs as a loop; 4,096 channels, 16 states, 16 requests of 128 tokens 69 us in one part, 90 in two; 8 of 256 94 and 113, 101 in
         four; 8,192 channels, 2 of 512 145 in one, 107 in eight)."""
         if wide and longest is not None:
             walking = -(-channels // 32) * max(1.0, num_tokens / longest)
