@@ -2,7 +2,8 @@
 
 `csrc/attention_tcgen05.cu` (`attn_tc_pp_kernel`, NT = 1): four score buffers, the even steps' softmax in one warpgroup and the odd
 steps' in another, the maximum in use handed from step to step through shared memory, sums kept per side.  As in the model of the two-tile form every access
-is checked for the step that it is meant for; waits are by parity, so a waiter may be at most one phase away.  `BUFFERS` of them are modelled.
+is checked for the step that it is meant for; waits are by parity, so a waiter may be at most one phase away.  Nothing orders the copies' completion: they
+may take any time, and value copies another than key copies (`delay`).
 """
 import random
 
@@ -10,8 +11,11 @@ import pytest
 from test_tc_attention_protocol import Barrier, Deadlock
 
 
-def simulate(nsteps, seed, NS=4, KE=1, buffers=4, threads=2, chained=True):
+def simulate(nsteps, seed, NS=4, KE=1, buffers=4, threads=2, chained=True, product_first=True, delay=None):
+    """`delay(rnd, kind, j)`: how long the copy of a piece of tile j takes ("K" or "V").  `product_first`: the score thread waits for the product that
+    used its buffer before it waits for the tile's keys, as the kernel does."""
     rnd = random.Random(seed)
+    delay = delay or (lambda rnd, kind, j: rnd.randint(1, 6))
     W = threads
     bars = {("FULL", i): Barrier(1) for i in range(NS)}
     bars.update({("EMPTY", i): Barrier(1) for i in range(NS)})
@@ -38,18 +42,24 @@ def simulate(nsteps, seed, NS=4, KE=1, buffers=4, threads=2, chained=True):
             order += [("V", j)] + ([("K", j + 2)] * KE if j + 2 < nsteps else [])
         for it, tile in enumerate(order):
             yield from wait(("EMPTY", it % NS), ((it // NS) & 1) ^ 1)
-            copies.append([rnd.randint(1, 6), it % NS, tile])
+            copies.append([delay(rnd, *tile), it % NS, tile])
 
     def score_issuer():
+        def buffer_free(j):
+            if j >= buffers:
+                yield from wait(("OF", slot(j)), phase(j - buffers))
+                assert done["landed"] >= j - buffers, ("scores over probabilities still in use", j)
+
         for j in range(nsteps):
+            if product_first:
+                yield from buffer_free(j)
             entries = [k_index(j) + e for e in range(KE)]
             for idx in entries:
                 yield from wait(("FULL", idx % NS), (idx // NS) & 1)
             sts = [idx % NS for idx in entries]
             assert all(ring[st] == ("K", j) for st in sts), ("scores from the wrong tile", j)
-            if j >= buffers:
-                yield from wait(("OF", slot(j)), phase(j - buffers))
-                assert done["landed"] >= j - buffers, ("scores over probabilities still in use", j)
+            if not product_first:
+                yield from buffer_free(j)
             queues[1] += [("S", j, sts), ("commit", ("SF", slot(j)))] + [("commit", ("EMPTY", st)) for st in sts]
 
     def pv_issuer():
@@ -133,6 +143,32 @@ def simulate(nsteps, seed, NS=4, KE=1, buffers=4, threads=2, chained=True):
 def test_one_tile_protocol_holds_under_random_schedules(nsteps, stages, key_entries, buffers):
     for seed in range(60):
         simulate(nsteps, seed, NS=stages, KE=key_entries, buffers=buffers)
+
+
+DELAYS = {
+    "any time": lambda rnd, kind, j: rnd.choice((1, 6, 60, 600)),
+    "slow values": lambda rnd, kind, j: 400 if kind == "V" else rnd.randint(1, 6),
+    "slow keys": lambda rnd, kind, j: 400 if kind == "K" else rnd.randint(1, 6),
+    "a late value tile": lambda rnd, kind, j: 3000 if (kind, j) == ("V", 1) else rnd.randint(1, 6),
+    "a late key tile": lambda rnd, kind, j: 3000 if (kind, j) == ("K", 2) else rnd.randint(1, 6),
+    "values of the first tile late": lambda rnd, kind, j: 3000 if (kind, j) == ("V", 0) else rnd.randint(1, 6),
+}
+
+
+@pytest.mark.parametrize("delay", sorted(DELAYS))
+@pytest.mark.parametrize("stages,key_entries", [(4, 1), (5, 4), (11, 4)])
+@pytest.mark.parametrize("nsteps", [2, 4, 5, 6, 9, 14])
+def test_one_tile_protocol_holds_whatever_the_copies_take(nsteps, stages, key_entries, delay):
+    for seed in range(10):
+        simulate(nsteps, seed, NS=stages, KE=key_entries, delay=DELAYS[delay])
+
+
+def test_keys_must_not_be_waited_for_before_the_product():
+    """Eleven entries: the first piece of K(j) takes the entry of V(j - 4).  Only product j - 4 tells that those values had come; polled before it, the
+    entry's barrier may still be in their phase, and a wait for the other parity passes."""
+    with pytest.raises(AssertionError, match="wrong tile"):
+        for seed in range(60):
+            simulate(9, seed, NS=11, KE=4, product_first=False, delay=DELAYS["slow values"])
 
 
 def test_the_maximum_must_wait_for_the_step_before():

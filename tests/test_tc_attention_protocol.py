@@ -36,10 +36,11 @@ class Deadlock(Exception):
     pass
 
 
-def simulate(nsteps, ntq, seed, product_barriers_per_tile=2, softmax_threads=2, correction_threads=2, NS=NS, KE=1):
-    """One CTA walking `nsteps` key steps with `ntq` query tiles.  Raises AssertionError when a role touches data of
+def simulate(nsteps, ntq, seed, product_barriers_per_tile=2, softmax_threads=2, correction_threads=2, NS=NS, KE=1, delay=None):
+    """One CTA walking `nsteps` key steps with `ntq` query tiles; `delay(rnd, kind, j)`: how long a copy of tile j ("K" or "V") takes.  Raises AssertionError when a role touches data of
     the wrong step and Deadlock when nothing can move."""
     rnd = random.Random(seed)
+    delay = delay or (lambda rnd, kind, j: rnd.randint(1, 6))
     W, C, PB = softmax_threads, correction_threads, product_barriers_per_tile
     bars = {}
     for i in range(NS):
@@ -80,7 +81,7 @@ def simulate(nsteps, ntq, seed, product_barriers_per_tile=2, softmax_threads=2, 
         for it, tile in enumerate(order):
             st = it % NS
             yield from wait(("EMPTY", st), ((it // NS) & 1) ^ 1)
-            copies.append([rnd.randint(1, 6), st, tile])
+            copies.append([delay(rnd, *tile), st, tile])
 
     def score_issuer():
         for j in range(nsteps):
@@ -200,6 +201,25 @@ def test_protocol_holds_with_other_rings(nsteps, stages, key_entries):
     for ntq in (1, 2):
         for seed in range(60):
             simulate(nsteps, ntq, seed, NS=stages, KE=key_entries)
+
+
+DELAYS = {
+    "any time": lambda rnd, kind, j: rnd.choice((1, 6, 60, 600)),
+    "slow values": lambda rnd, kind, j: 400 if kind == "V" else rnd.randint(1, 6),
+    "slow keys": lambda rnd, kind, j: 400 if kind == "K" else rnd.randint(1, 6),
+    "a late value tile": lambda rnd, kind, j: 3000 if (kind, j) == ("V", 1) else rnd.randint(1, 6),
+    "a late key tile": lambda rnd, kind, j: 3000 if (kind, j) == ("K", 2) else rnd.randint(1, 6),
+    "values of the first tile late": lambda rnd, kind, j: 3000 if (kind, j) == ("V", 0) else rnd.randint(1, 6),
+}
+
+
+@pytest.mark.parametrize("delay", sorted(DELAYS))
+@pytest.mark.parametrize("stages,key_entries", [(8, 1), (5, 2)])
+@pytest.mark.parametrize("nsteps", [2, 5, 8, 13])
+def test_protocol_holds_whatever_the_copies_take(nsteps, stages, key_entries, delay):
+    for ntq in (1, 2):
+        for seed in range(10):
+            simulate(nsteps, ntq, seed, NS=stages, KE=key_entries, delay=DELAYS[delay])
 
 
 def test_one_product_barrier_per_tile_is_not_enough():

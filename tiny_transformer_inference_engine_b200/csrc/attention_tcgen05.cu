@@ -1113,10 +1113,16 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
                     for (int cb = 0; cb < CB; ++cb) q_lo[t][cb] = desc_lo(smem_u32(Qs + t * QT_BYTES + cb * QBLK), 16);
                 const uint32_t ring_k_lo = desc_lo(smem_u32(ring), 16);
+                // The buffer of step j holds P(j - REUSE) until its product with V has finished.  With one tile that wait stands before the keys'
+                // waits, not only before the product: of eleven entries the first of K(j) is that of V(j - 4), whose barrier is known to be
+                // out of V(j - 4)'s phase only when product j - 4 has landed (copies may complete in any order); polled before, a wait for
+                // the other parity would pass.  All other entries of K(j) are those of keys that this thread has waited for, or (two tiles,
+                // five entries) of V(j - 3), whose product it waited for a step ago.
+                auto buffer_free = [&](int t, int j) -> bool { return j < REUSE || mbar_wait(BAR(PP_OF + slot(t, j)), phase(j - REUSE), 4); };
                 for (int j = 0; j < nsteps; ++j) {
                     int st[KE];
                     uint32_t k_lo[KE];
-                    bool ok = true;
+                    bool ok = NT == 2 || buffer_free(0, j);
 #pragma unroll
                     for (int e = 0; e < KE; ++e) {
                         const int idx = k_index(j) + e;
@@ -1128,9 +1134,8 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
                     for (int t = 0; t < NT; ++t) {
                         if (t < ntq) {
-                            // the buffer holds P(j - REUSE) until its product with V has finished
                             const int b = slot(t, j);
-                            if (j >= REUSE && !mbar_wait(BAR(PP_OF + b), phase(j - REUSE), 4)) { ok = false; break; }
+                            if (NT == 2 && !buffer_free(t, j)) { ok = false; break; }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             const uint32_t d = tmem_base + S_COL + (uint32_t)b * BNK;
 #pragma unroll
