@@ -4,7 +4,7 @@ import random
 import pytest
 import torch
 
-from tiny_transformer_inference_engine_b200.ops import CudaOps, _floor_sum, _ring_form
+from tiny_transformer_inference_engine_b200.ops import CudaOps, _even_parts, _floor_sum, _ring_form
 
 
 @pytest.mark.parametrize("rows,hidden,K,fused", [
@@ -79,6 +79,19 @@ def selective(lens, channels, states, known=True, dtype=torch.bfloat16):
 def test_selective_scan_forms(lens, channels, states, form):
     assert selective(lens, channels, states) == form
     assert not selective(lens, channels, states, dtype=torch.float32)[0]
+
+
+# (what a step brings, channels) and the parts of the wide form: as measured, us of the choice | of other counts
+@pytest.mark.parametrize("lens,channels,parts", [
+    ([2048], 4096, 19), ([2048], 2048, 26), ([4096], 2048, 27), ([1024], 4096, 13), ([512], 8192, 7),                      # one long request: even waves
+    ([512] * 4, 4096, 8), ([512] * 2, 8192, 8), ([512] * 8, 2048, 8), ([512] * 16, 1024, 8), ([1024] * 4, 4096, 8),        # 97 | 114 in one part, 179 | 225
+    ([500] * 3, 5120, 7), ([512] * 2, 4096, 8), ([700, 300], 8192, 10), ([512, 1, 1, 512, 512, 1, 512], 4096, 8),          # 87 | 112, 59 | 68 in seven, 95 | 106 in six
+    ([512] * 3, 4096, 6), ([2048] * 3, 2048, 12), ([2048] * 2, 2048, 19), ([400] * 6, 4096, 1), ([128] * 16, 4096, 1), ([256] * 8, 4096, 1), ([200] * 12, 4096, 1),      # 75 | 81, 145 | 164, 99 | 110, 101 | 110; 60 | 80 in two
+])
+def test_parts_of_a_selective_scan_with_a_thread_per_channel(lens, channels, parts):
+    wide, most = selective(lens, channels, 16)
+    T, longest = sum(lens), max(lens)
+    assert wide and _even_parts(-(-channels // 128) * T / longest, longest, most, 148, T > 1.2 * longest) == parts
 
 
 def test_selective_scan_form_without_the_longest_request():

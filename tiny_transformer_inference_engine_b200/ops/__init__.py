@@ -213,21 +213,24 @@ def _ring_form(N, K, num_sms, may_split, few=True):
 
 
 @functools.lru_cache(maxsize=4096)
-def _even_parts(blocks: float, longest: int, most: int, num_sms: int) -> int:
+def _even_parts(blocks: float, longest: int, most: int, num_sms: int, several: bool = False) -> int:
     """How many parts, up to ``most``, a selective scan with a thread per channel cuts its requests into: those whose CTAs (one per part and
     128 channels; ``blocks`` CTAs walk ``longest`` tokens in one part) divide well over the SMs.  k CTAs of an SM take 0.30, 0.46, 0.62 and 0.80 us a
-    token of their parts in both walks together, further ones wait for a place; one part is walked once, in 0.55 of that.  Fitted to 44
-    shapes of 1,024 to 8,192 channels: 1.3 % behind the best number of parts on average, 11 % at most; 4,096 channels and 2,048 tokens 97 us in
-    19 parts, 107 in 32; 2,048 channels 60 in 26, 66 in 32."""
-    best, best_cost = 1, None
+    token of their parts in both walks together, further ones wait for a place.  One part is walked once, and its CTAs do not come as full SMs: k of
+    them (a fraction) take 0.15 + 0.09 k us a token, one alone 0.192 (128 CTAs 0.22, on some SMs two of them; 512 tokens of them 114 us in one part, 97 in
+    eight).  ``several``: the step has more than one long request.  Parts of up to 1,024 tokens then end at different times and the model is right to a
+    tenth only: fewer of them than ``most`` are taken for a gain of a tenth (4,096 channels, two of 512 tokens 68 us in seven, 59 in eight).  Over 58 shapes of 1,024 to 8,192 channels, 1 to 16 requests of 200 to 4,096 tokens, equal, unequal and beside
+    decoded tokens: 1.7 % behind the best of these numbers on average, 15 % at most (15 decoded tokens beside one request of 2,000, 4,096 channels:
+    130 us in 13 parts, 114 in 15); 4,096 channels and 2,048 tokens 99 us in 19 parts, 108 in 32; 2,048 channels 60 in 26, 66 in 32."""
+    best, best_cost, cost = 1, None, 0.0
     for p in range(1, most + 1):
         tokens = longest if p == 1 else max(64, -(-longest // (8 * p)) * 8)
-        k = max(1, math.ceil(blocks * longest / (num_sms * tokens)))
-        full, rest = divmod(k, 4)
-        cost = (0.80 * full + (0.0, 0.30, 0.46, 0.62)[rest]) * tokens * (0.55 if p == 1 else 1.0) + 0.1 * p
+        per_sm = blocks * longest / (num_sms * tokens)
+        full, rest = divmod(max(1, math.ceil(per_sm)), 4)
+        cost = tokens * (max(0.192, 0.15 + 0.09 * per_sm) if p == 1 else 0.80 * full + (0.0, 0.30, 0.46, 0.62)[rest]) + (0.0 if p == 1 else 0.1 * p)
         if best_cost is None or cost < best_cost:
             best, best_cost = p, cost
-    return best
+    return most if several and longest <= 1024 and best > 1 and best_cost > 0.9 * cost else best
 
 
 class CudaOps:
@@ -1375,8 +1378,8 @@ class CudaOps:
     def selective_wide(self, dtype, num_tokens: int, num_seqs: int, channels: int, states: int, longest=None) -> bool:
         """Whether a thread owns a channel (16-bit operands, up to 16 states) rather than four states of one: fewer instructions and a
         quarter of the threads, so it needs a step large enough to fill the GPU all the same.  16 states, us of a thread per
-        channel | per four states: 4,096 channels 512 tokens 37 | 39, 1,024 tokens 57 | 70, 2,048 tokens 98 | 141, four requests of
-        512 114 | 131; 2,048 channels 2,048 tokens 61 | 72; 8,192 channels 256 tokens 36 | 37, 512 56 | 68, 2,048 184 | 270.
+        channel | per four states: 4,096 channels 512 tokens 37 | 39, 1,024 tokens 57 | 70, 2,048 tokens 99 | 140, four requests of
+        512 97 | 133; 2,048 channels 2,048 tokens 61 | 72; 8,192 channels 256 tokens 36 | 37, 512 56 | 68, 2,048 184 | 270.
         ``longest``: the most tokens that a request brings, if known.  Beside 23 decoding requests a portion of 2,000 tokens is all there is to
         fill the GPU (8,192 channels 701 in one part, 447 per four states, 260 in eight parts).  Up to four states both forms have a
         thread per channel, and requests of a few tokens do not pay for the runs' staging (150 of 8 tokens 95 | 83)."""
@@ -1395,8 +1398,8 @@ class CudaOps:
         """Into how many parts a request's tokens are walked: every part but the last is walked twice, which pays while the
         channels alone give the SMs too few warps to hide a token's latency.  With a thread per channel (``wide``) and ``longest`` known the
         warps counted are those of the tokens, as so many requests of that length (a request of one token leaves at once); from 6.5 warps
-        per SM on one part is best (with the runs as a loop; 4,096 channels, 16 states, 16 requests of 128 tokens 69 us in one part, 90 in two; 8 of 256 94 and 113, 101 in
-        four; 8,192 channels, 2 of 512 145 in one, 107 in eight)."""
+        per SM on one part is best (4,096 channels, 16 states, 16 requests of 128 tokens 60 us in one part, 80 in two; 8 of 256 78 and 104, 91 in
+        four; with fewer warps not: 8,192 channels, 2 of 512 114 in one, 97 in eight).  With a thread per channel the number is the most that ``_even_parts`` chooses from."""
         if wide and longest is not None:
             walking = -(-channels // 32) * max(1.0, num_tokens / longest)
             if walking >= self.selective_wide_full * self.num_sms:
@@ -1430,7 +1433,7 @@ class CudaOps:
         parts = self.selective_parts(T, int(num_seqs), I, int(states), wide, max_q_len)
         if wide and parts > 1:
             longest = int(max_q_len) if max_q_len is not None else T - (int(num_seqs) - 1)
-            parts = _even_parts(-(-I // 128) * T / longest, longest, parts, self.num_sms)
+            parts = _even_parts(-(-I // 128) * T / longest, longest, parts, self.num_sms, T > 1.2 * longest)
         scratch = torch.empty(int(num_seqs) * parts * I * (A.shape[1] + 1), dtype=torch.float32, device=u.device) if parts > 1 else None
         self._check(self.lib.ttie_selective_scan(
             _ptr(u), u.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(A), _ptr(D), _ptr(bc), bc.stride(0), int(col_b), int(col_c), _ptr(z),
