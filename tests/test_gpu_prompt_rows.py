@@ -196,6 +196,27 @@ def test_causal_conv_in_runs_of_tokens(ops, lens, width, wdtype, taps):
         assert ((u.double() - y).abs() <= 2.0 ** -8 * y.abs() + 2 * slack + 1e-6).all()
 
 
+def test_causal_conv_silu_of_large_sums(ops):
+    """One tap: the sum is one rounded product, and silu of it is rounded correctly but where the exact value lies within the function's 32-bit
+    error of a tie (2^-21.2 at most, about a quarter of it on average, beside ties 2^-8 to 2^-7 apart: 2^-15 of them, 2^-13 are the limit; with
+    the exponent's rounding left in, 2^-19.5 on average at -80 to -64, 2^-12).  Beyond -87 it is 0 to 2^-119; what is not finite as in the general form."""
+    T, W = 1024, 1024
+    x = randn(61, T, W)
+    x[:, ::2] = x[:, ::2].abs().clamp(max=1.0) * -16 - 64
+    special = torch.tensor([float("inf"), -float("inf"), float("nan"), -88.5, -104.0, -3e38, 3e38, 88.5, -0.0], device=DEV)
+    x[5, :9], x[1023, :9] = special, special
+    x, w = x.bfloat16(), 1 + 0.1 * randn(62, 1, W)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    conv = lambda x, T: ops.causal_conv(x, 0, W, 1, w, None, torch.zeros(1, 1, W, device=DEV), t([0] * T), t([0, T]), t([0]), True,
+                                        first_row=0, act="silu", want_f32=False)[1]
+    got, x32 = conv(x, T), x.float() * w
+    exact = x32.double() * torch.sigmoid(x32.double())
+    assert (got != exact.bfloat16())[(x32 > -87) & (x32 <= -64)].double().mean() <= 2.0 ** -13
+    assert (got.double() - exact)[x.isfinite()].abs().le(2.0 ** -8 * exact.abs()[x.isfinite()] + 2.0 ** -119).all()
+    general = conv(x[1020:].contiguous(), 4)
+    assert torch.equal(got[1020:].isnan(), general.isnan()) and torch.equal(got[1020:].isinf(), general.isinf())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T,d,off", [(1, 8, 0), (3, 12, 0), (5, 1032, 0), (2, 4104, 8), (4, 100, 0), (3, 64, 1), (70, 516, 4)])
 def test_embed_forms(ops, T, d, off, dtype):

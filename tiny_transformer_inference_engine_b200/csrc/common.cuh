@@ -107,6 +107,17 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // merges split-KV partial results (attention_simt.cu)
 int attn_merge_bf16(const float* ws_o, const float* ws_ml, void* out, int rows, int num_splits, int D, cudaStream_t s);
 
+// 1 / (1 + e^-x) by the hardware's 2^x and reciprocal: over all 32-bit x relative error 2^-21.5 (of x times it; 2^-21.9 with expf and division) down
+// to -87, where it ends.  -x log2(e) rounded is off by more the larger x is; what the rounding left out of the exponent comes back as a factor 1 + r.
+__device__ __forceinline__ float sigmoid_close(float x) {
+    float a, e, q;
+    asm("{.reg .f32 m; min.NaN.f32 m, %1, 0f43000000; max.NaN.f32 %0, m, 0fC2B00000;}" : "=f"(a) : "f"(x));        // to 128 and -88
+    const float t = a * -1.4426950408889634f, r = fmaf(t, -0.6931471805599453f, -a);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(1.0f + fmaf(e, r, e)));
+    return q;
+}
+
 // The activation of a gated unit's gate, 32-bit.  0: g * sigmoid(alpha * g) (alpha 1: silu); 1: the tanh form of gelu,
 // 0.5 g (1 + tanh(u)) = g / (1 + exp(-2u)) with u = sqrt(2 / pi) (g + 0.044715 g^3).
 __device__ __forceinline__ float gelu_tanh(float g) {

@@ -118,9 +118,9 @@ causal_conv_vec8_kernel(const __nv_bfloat16* __restrict__ in, long long ld, int 
 // The same for prompt portions: a thread takes eight channels of CONV_RUN consecutive tokens.  The weights stay in registers and an input row
 // is loaded and widened once, not once per tap; all rows of the run are asked for before the first sum.  A run that crosses the start
 // of a request's tokens (or needs inputs from before the step) goes row by row through the state rows.  The sums are those of the other form,
-// term by term; silu of an output that is only wanted in bfloat16 takes the hardware's exponential and reciprocal (error against
-// 64 bits the same to nine digits).  What bounds it: the instructions of silu and of widening.  Four taps, silu, bfloat16 out: 2,048 tokens of
-// 4,096 channels 19.4 -> 10.7 us (17.8 with silu in full), 2,048 channels 11.1 -> 6.6; 32-bit and bfloat16 out without silu 20.0 -> 13.5.
+// term by term; silu of an output that is only wanted in bfloat16 is sigmoid_close's, as good as the other form's to a few units in the last of its 32 bits.
+// What bounds it: the instructions of silu and of widening.  Four taps, silu, bfloat16 out: 2,048 tokens of
+// 4,096 channels 19.5 -> 11.1 us (17.8 with the library's function), 2,048 channels 11.3 -> 6.8; 32-bit and bfloat16 out without silu 20.3 -> 13.6.
 // Runs of 2 and 8: 13.0 and 9.8, but 300 requests of 7 tokens 18.8 in runs of 4, and 1 Mi values 4.2 | 6.4 in runs of 4 | 8.
 constexpr int CONV_RUN = 4;
 template <typename W, int TAPS>
@@ -148,7 +148,7 @@ causal_conv_run_kernel(const __nv_bfloat16* __restrict__ in, long long ld, int c
     auto finish = [&](int t, float (&acc)[8]) {
         if (silu) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i] = u32 ? acc[i] * sigmoidf_(acc[i]) : __fdividef(acc[i], 1.0f + __expf(-acc[i]));
+            for (int i = 0; i < 8; ++i) acc[i] *= u32 ? sigmoidf_(acc[i]) : sigmoid_close(acc[i]);
         }
         if (u32) {
             float* o = u32 + (size_t)t * width + c;
@@ -457,8 +457,9 @@ extern "C" int ttie_causal_conv(const void* in, long long ld, int col0, int T, i
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == kBF16 && width % 8 == 0 && ld % 8 == 0 && col0 % 8 == 0 && row_stride % 4 == 0 && tail_off % 4 == 0 && ((((uintptr_t)in) | ((uintptr_t)state) | ((uintptr_t)u32) | ((uintptr_t)u_c) | ((uintptr_t)cw) | ((uintptr_t)cb)) & 15) == 0) {
         const dim3 g8(ceil_div(width / 8, 128), T < 65535 ? T : 65535);
-        // prompt portions: four tokens a thread, from 1 Mi values on (below it such runs leave SMs idle: 512 Ki values 3.3 us a token per thread,
-        // 3.8 in runs; 1 Mi 5.1 and 4.2)
+        // four tokens a thread, from 1 Mi values on (below it such runs leave SMs idle: 512 Ki values 3.3 us a token per thread, 3.8 in runs; 1 Mi
+        // 5.2 and 4.3).  Requests of few tokens too, all of whose runs go row by row: 4,096 channels, one of 256 tokens 5.2 | 4.3, 256 of one token 5.8 | 4.6,
+        // 300 of 7 21.1 | 19.4; behind another kernel 300 of one token 5.8 | 5.3, 60 of 5 5.5 | 5.8, 91 of 7 9.2 | 8.3
         if (taps <= 4 && (long long)T * width >= 1 << 20) {
             const int runs = ceil_div(T, CONV_RUN);
             const dim3 g(ceil_div(width, 8 * 128), runs < 65535 ? runs : 65535);
