@@ -60,6 +60,32 @@ def test_gated_read_outs(ops, kind, lens, H, D, Dv):  # noqa: F811
             assert all(torch.equal(torch.nan_to_num(a), torch.nan_to_num(b)) for a, b in zip(states, states2))
 
 
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_gates_far_from_zero(ops, kind, act):  # noqa: F811
+    """Gates at which e^-x takes the largest exponents.  The results are correctly rounded but where the exact value lies within their 32-bit error of a
+    tie: 2^-21.2 of the gate at most, about a quarter of it on average, some 2^-23 of the norm, beside ties 2^-8 to 2^-7 apart, so 2^-14 of them differ
+    and 2^-13 are the limit (with the exponent's rounding left in, 2^-19.5 on average at these gates, 2^-12).  Beyond -87 a gate is 0 to 2^-126."""
+    H, D = (16, 64) if kind == "wkv" else (8, 64)
+    Dv, T = (64, 1000) if kind == "wkv" else (128, 1000)
+    sc = Scan(kind, [T], H, D, Dv, seed=8)
+    o, _ = sc.forced(ops, True)
+    g = torch.Generator(device=DEV)
+    g.manual_seed(9)
+    gate = (torch.rand(T, H * Dv, generator=g, device=DEV) * -16 - 64).bfloat16()
+    y, _ = sc.run(Gating(ops, (gate, None, 0.0, act)))
+    x = o.double().view(T, H, Dv)
+    x = (x / (x * x).mean(-1, keepdim=True).sqrt()).flatten(1)
+    of = lambda gate: torch.sigmoid(gate.double()) * (gate.double() if act == "silu" else 1.0)
+    assert (y != (x * of(gate)).bfloat16()).double().mean() <= 2.0 ** -13
+    special = [float("inf"), -float("inf"), float("nan"), -87.0, -88.0, -89.0, -104.0, -3e38, 3e38, 88.0, 200.0, -0.0]
+    gate[:] = torch.tensor((special * (H * Dv))[:H * Dv], device=DEV).bfloat16()
+    y, _ = sc.run(Gating(ops, (gate, None, 0.0, act)))
+    ref = ops.head_norm_gate(o, gate, None, H, Dv, 0.0, act)
+    assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf()) and y.isinf().any() == (act == "silu")
+    assert ((y.float() - ref.float()).abs() <= 2.0 ** -7 * ref.float().abs() + 1e-33)[ref.isfinite()].all()
+
+
 @pytest.mark.parametrize("kind", KINDS)
 def test_gated_in_passes_and_walked(ops, kind):  # noqa: F811
     """A step in passes: the same bits.  A walk: the pass over the read-outs, also for gates of 32 bits."""

@@ -195,11 +195,11 @@ __device__ __forceinline__ void walk_out(const ChunkArgs& a, size_t unit, int t0
     }
 }
 
-// ---- normalised and gated read-outs: o * weight / rms(o over the head) * act(gate), 32-bit until the result is rounded to bfloat16 (2^-9; the
-// approximations of e^x, 1 / x and 1 / sqrt(x) are good to 2^-21)
+// ---- normalised and gated read-outs: o * weight / rms(o over the head) * act(gate), 32-bit until the result is rounded to bfloat16 (2^-9; gates are
+// good to 2^-21 down to -87 and end there, 1 / rms to two units in the last place)
 __device__ __forceinline__ float inverse_rms(const ChunkArgs& a, float squares) { return rsqrtf(squares / (float)a.Dv + a.eps); }
 __device__ __forceinline__ float gate_of(const ChunkArgs& a, float g) {
-    const float s = __fdividef(1.0f, 1.0f + __expf(-g));
+    const float s = sigmoid_close(g);
     return a.act == 0 ? g * s : s;
 }
 __device__ __forceinline__ uint32_t gated_pair(const ChunkArgs& a, float x, float y, float2 w, uint32_t gate) {
