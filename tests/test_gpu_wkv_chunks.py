@@ -37,3 +37,31 @@ def test_wkv_keys_that_outlast_their_decays(ops):  # noqa: F811
     out, (S, _) = sc.forced(ops, True)
     walk, (W, _) = sc.forced(ops, False)
     assert W.abs().max() > 0 and torch.allclose(S, W, rtol=1e-6) and torch.allclose(out, walk, rtol=1e-5, atol=1e-5 * float(walk.abs().max()))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("key", [2.0 ** 9, -(2.0 ** 11), 2.0 ** 39])
+@pytest.mark.parametrize("tokens", [30, 34, 37, 40, 64])
+def test_wkv_large_keys_behind_small_decays(ops, tokens, key, D):  # noqa: F811
+    """Products of decays from 2^-99 to 2^-300 beside a key: the state to 32 bits (2e-6), or to 2^-131 of the values where the planes of a key end at 2^-133."""
+    sc = Scan("wkv", [tokens], 2, D, D, seed=2)
+    sc.k.zero_()
+    sc.k[0] = key
+    sc.w.uniform_(0.03, 0.1, generator=torch.Generator(device=DEV).manual_seed(5))
+    sc.S0.zero_()
+    out, (S, _) = sc.forced(ops, True)
+    exp, (E,) = sc.exact()
+    assert ((S.double() - E).abs() <= 2e-6 * E.abs() + 2.0 ** -131 * float(sc.v.float().abs().max())).all()
+    assert rel(out, exp) < 1e-6
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_wkv_large_states_behind_small_decays(ops, D):  # noqa: F811
+    """The state's factor over a chunk, 2^-114 beside states of 2^60."""
+    sc = Scan("wkv", [30], 2, D, D, seed=2)
+    sc.k.zero_()
+    sc.w.uniform_(0.06, 0.08, generator=torch.Generator(device=DEV).manual_seed(5))
+    sc.S0 *= 2.0 ** 60
+    _, (S, _) = sc.forced(ops, True)
+    _, (E,) = sc.exact()
+    assert float(E.abs().max()) > 2.0 ** -70 and rel(S, E) < 2e-7

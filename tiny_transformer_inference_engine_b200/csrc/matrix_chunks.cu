@@ -74,6 +74,7 @@ struct Pair {
         lo = fmaf(lo, b.hi, fmaf(hi, b.lo, fmaf(hi, b.hi, -p)));
         hi = p;
     }
+    __device__ __forceinline__ Pair times(float power_of_two) const { return {hi * power_of_two, lo * power_of_two}; }
     __device__ __forceinline__ float value() const { return hi + lo; }
 };
 // planes of such a product (its third plane keeps what rounding it to 32 bits would cut)
@@ -140,10 +141,10 @@ __device__ __forceinline__ void mma_planes_kept(float (&acc)[4], float (&left)[4
 #pragma unroll
     for (int i = 0; i < 4; ++i) left[i] += l[i];
 }
-// A key times the decays behind it.  Decays that have all but vanished (a pair has no more than 32-bit range) beside a key that could still
-// matter make it NaN: such states and chunks are walked.
+// A key times the decays behind it.  Below 2^-102 a pair keeps what lies above 2^-149 and no more: beside keys under 2^10 the up to 64 roundings there
+// stay below 2^-133, where the planes end as well.  Larger keys beside such decays make it NaN: such states and chunks are walked.
 __device__ __forceinline__ Pair decayed_key(Pair f, float k) {
-    const bool lost = fabsf(k) >= 0x1p40f && fabsf(f.hi) < 0x1p-100f;
+    const bool lost = fabsf(k) >= 0x1p10f && fabsf(f.hi) < 0x1p-100f;
     f *= k;
     if (lost) f.hi = __int_as_float(0x7fc00000);
     return f;
@@ -295,21 +296,25 @@ __global__ void __launch_bounds__(SumSmem<MODE, KP>::NT, MODE == WKV && KP == 64
             kv[i] = k_raw[(run * LEN + i) * LD + ch];
         }
         stage_tail();
-        Pair all = {1.f, 0.f};
+        // (over runs and the chunk the products are held times 2^64: the state's factor, a pair of 32-bit numbers in memory too, keeps all that these hold)
+        Pair all = {0x1p64f, 0.f};
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) all *= w[i];
-        tot[run * KP + ch] = all;
+        tot[run * KP + ch] = all.times(0x1p-32f);
         __syncthreads();
-        Pair suf = {1.f, 0.f};
+        Pair suf = {0x1p64f, 0.f};
 #pragma unroll
         for (int i = RUNS - 1; i > 0; --i)
-            if (i > run) suf *= tot[i * KP + ch];
+            if (i > run) { suf = suf.times(0x1p-32f); suf *= tot[i * KP + ch]; }
         if (run == 0 && ch < a.Dpad) {
+            suf = suf.times(0x1p-32f);
+            all = all.times(0x1p-32f);
             all *= suf;
-            const float f = in ? all.value() : 1.f;
-            a.aux[2 * unit * a.Dpad + ch] = f;
-            a.aux[(2 * unit + 1) * a.Dpad + ch] = in ? (all.hi - f) + all.lo : 0.f;
-        }
+            const float f = all.value();
+            a.aux[2 * unit * a.Dpad + ch] = in ? f * 0x1p-64f : 1.f;
+            a.aux[(2 * unit + 1) * a.Dpad + ch] = in ? ((all.hi - f) + all.lo) * 0x1p-64f : 0.f;
+            suf = suf.times(0x1p-32f);
+        } else suf = suf.times(0x1p-64f);
 #pragma unroll
         for (int i = LEN - 1; i >= 0; --i) {
             const int j = run * LEN + i;
