@@ -49,14 +49,17 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ void record_error(int code) {
+    atomicCAS(&g_attn_tc_error, 0, code);
+    if (g_attn_tc_error_mirror) { *reinterpret_cast<volatile int*>(g_attn_tc_error_mirror) = code; __threadfence_system(); }
+}
 // limit: clocks after which the wait gives up (about a second by default)
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code, long long limit = WAIT_CYCLES) {
     if (mbar_try(bar, parity)) return true;
     const long long deadline = clock64() + limit;
     while (!mbar_try(bar, parity)) {
         if (clock64() > deadline) {
-            atomicCAS(&g_attn_tc_error, 0, code);
-            if (g_attn_tc_error_mirror) { *reinterpret_cast<volatile int*>(g_attn_tc_error_mirror) = code; __threadfence_system(); }
+            record_error(code);
             return false;
         }
     }
@@ -70,8 +73,7 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity,
     while (!mbar_try(bar, parity)) {
         __nanosleep(64);
         if (clock64() > deadline) {
-            atomicCAS(&g_attn_tc_error, 0, code);
-            if (g_attn_tc_error_mirror) { *reinterpret_cast<volatile int*>(g_attn_tc_error_mirror) = code; __threadfence_system(); }
+            record_error(code);
             return false;
         }
     }
@@ -157,7 +159,7 @@ struct AttnTcParams {
     const int* qsl; const int* seq_lens;
     __nv_bfloat16* out;
     int num_seqs, Hq, Hkv;
-    int lead;                                                    // two-tile kernel: so many first requests have one row tile each (decoded tokens before prompt portions)
+    int lead;                                                    // head size 256: so many first requests have one row tile each (decoded tokens before prompt portions)
     float scale_log2; int window, chunk, keep;                   // keep: first tokens of the sequence that stay visible behind a window
     float cap_in, cap_out;                                       // score softcap: raw score s becomes cap_out * tanh(s * cap_in) (cap_in 0: none)
     int row_tiles;
@@ -740,6 +742,7 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     const int q0 = p.qsl[seq], q_len = p.qsl[seq + 1] - q0, kv_len = p.seq_lens[seq];
     const int nrows = q_len * G, row0 = rt * (NT * BM);
     if (row0 >= nrows) return;                                   // uniform over the CTA, before anything is allocated
+    if (led && nrows > NT * BM && threadIdx.x == 0) record_error(13);       // (the caller's word does not hold: the rows behind the tile are nobody's)
     const int ctx = kv_len - q_len;
     const int rows_here = min(NT * BM, nrows - row0);
     const int tok_lo = row0 / G, tok_hi = (row0 + rows_here - 1) / G;
@@ -1324,12 +1327,13 @@ extern "C" int ttie_attn_tc_joint_supported(int W, int dv, int page_size) {
 // Joint rows (one cache head holds the rows of all kv heads side by side; D is that row's width).  dv > 0 (a multiple of 32): with
 // Hkv 1, head h's output is the columns (h / per) * dv .. of its row only; out is [T, Hq, dv].  joint = 64 or 128 (two_tiles only):
 // Hkv row groups, one per kv head, whose values are the columns kvh * joint .. + joint; out is [T, Hq, joint].
-// lead (two_tiles only): the first requests that bring no more rows than a row tile has; they get one row tile each.
+// lead (two_tiles, head size 256): the first requests, which bring at most lead_q_len tokens (0: not said) and no more rows than a row tile has; they get
+// one row tile each.  One that brings more leaves error 13.
 extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                                int num_pages, const int* block_table, int table_width, int page_size, const int* qsl,
                                                const int* seq_lens, void* out, int T, int num_seqs, int Hq, int Hkv, int D,
                                                int max_q_len, float scale, float softcap, int window, int chunk, int keep, int num_splits, int split_len,
-                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, int lead, void* stream);
+                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, int lead, int lead_q_len, void* stream);
 
 extern "C" int ttie_paged_attention_tc(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                        int num_pages, const int* block_table, int table_width, int page_size, const int* qsl,
@@ -1338,14 +1342,14 @@ extern "C" int ttie_paged_attention_tc(const void* q, long long q_stride, const 
                                        int two_tiles, void* stream) {
     return ttie_paged_attention_tc_weights(q, q_stride, k_pages, v_pages, num_pages, block_table, table_width, page_size, qsl, seq_lens, out, T,
                                            num_seqs, Hq, Hkv, D, max_q_len, scale, softcap, window, chunk, 0, num_splits, split_len, scratch,
-                                           two_tiles, 0, nullptr, 0, 1, 0, 0, stream);
+                                           two_tiles, 0, nullptr, 0, 1, 0, 0, 0, stream);
 }
 
 extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride, const void* k_pages, const void* v_pages,
                                                int num_pages, const int* block_table, int table_width, int page_size, const int* qsl,
                                                const int* seq_lens, void* out, int T, int num_seqs, int Hq, int Hkv, int D,
                                                int max_q_len, float scale, float softcap, int window, int chunk, int keep, int num_splits, int split_len,
-                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, int lead, void* stream) {
+                                               float* scratch, int two_tiles, int weights, const float* head_bias, int dv, int per, int joint, int lead, int lead_q_len, void* stream) {
     if (T <= 0 || num_seqs <= 0) return 0;
     if (weights != 0 && weights != 1) TTIE_FAIL("attention_tc: unknown kind of weights %d", weights);
     if (!joint && !ttie_attn_tc_supported(D, page_size)) TTIE_FAIL("attention_tc: head size %d with pages of %d keys is not supported", D, page_size);
@@ -1357,7 +1361,9 @@ extern "C" int ttie_paged_attention_tc_weights(const void* q, long long q_stride
     if (num_splits > 1 && (split_len <= 0 || split_len % BN || !scratch))
         TTIE_FAIL("attention_tc: splits need scratch and a split length that is a multiple of %d", BN);
     if (num_splits > 65535) TTIE_FAIL("attention_tc: too many splits (%d)", num_splits);
-    if (lead < 0 || lead > num_seqs || (lead && !two_tiles)) TTIE_FAIL("attention_tc: %d leading requests of %d", lead, num_seqs);
+    if (lead < 0 || lead > num_seqs || (lead && (!two_tiles || joint || D != 256 || (long long)lead_q_len * (Hq / Hkv) > BM)))
+        TTIE_FAIL("attention_tc: %d leading requests of %d, head size %d, up to %d tokens of %d heads each: head size 256 and one row tile of %d", lead, num_seqs,
+                  D, lead_q_len, Hq / Hkv, BM);
     CUtensorMap mk, mv;
     if (dv > 0 && (dv % 32 || per <= 0 || (long long)ceil_div(Hq, per) * dv > D)) TTIE_FAIL("attention_tc: %d value columns per %d heads in rows of %d", dv, per, D);
     if (joint && (!two_tiles || !ttie_attn_tc_joint_supported(D, joint, page_size) || (long long)Hkv * joint > D))

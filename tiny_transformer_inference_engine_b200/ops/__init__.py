@@ -67,7 +67,7 @@ _SIGNATURES = {
                                 _c_void],
     "ttie_paged_attention_tc_weights": [_c_void, _c_ll, _c_void, _c_void, _c_int, _c_void, _c_int, _c_int, _c_void, _c_void, _c_void,
                                         _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void, _c_int,
-                                        _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_void],
+                                        _c_int, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_tc": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_gemm_tc_pair": [_c_void, _c_ll, _c_void, _c_ll, _c_void, _c_void, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void],
     "ttie_grouped_gemm_tc": [_c_void, _c_ll, _c_void, _c_void, _c_ll, _c_void, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_float,
@@ -599,7 +599,7 @@ class CudaOps:
     def tc_error(self) -> int:
         """Error word of the tcgen05 kernels (0 = none; otherwise the code of the first bounded wait that
         ran out: products 1-4 and so on by kernel, float32 product 41-48, chunks of 128 tokens 51-54, decode product 61-63,
-        attention 101-110); synchronises the device."""
+        attention 101-112; 113: a leading request of an attention launch brought more rows than a row tile has); synchronises the device."""
         g = int(self.lib.ttie_tc_error())
         a = int(self.lib.ttie_attn_tc_error())
         return g or (100 + a if a else 0)
@@ -612,7 +612,8 @@ class CudaOps:
         if self._tc_words[0] or self._tc_words[1]:
             self._tc_words[:] = 0
             code = self.tc_error() or -1
-            raise KernelError(f"a tcgen05 kernel gave up waiting on a barrier (code {code}); its output is invalid")
+            what = "attention's leading request brought more rows than a row tile" if code == 113 else "a tcgen05 kernel gave up waiting on a barrier"
+            raise KernelError(f"{what} (code {code}); its output is invalid")
 
     def linear_swiglu(self, x, w_gu, b_gu, hidden):
         """silu(x @ Wg.T) * (x @ Wu.T) with w_gu = [Wg; Wu] ([2*hidden, K]) -> [M, hidden]."""
@@ -1047,7 +1048,7 @@ class CudaOps:
 
     def paged_attention(self, qkv, num_heads, num_kv_heads, head_dim, k_pages, v_pages, block_table, page_size,
                         query_start_loc, seq_lens, num_seqs, max_q_len, max_kv_len, scale, window, out,
-                        plan=None, softcap=0.0, chunk=0, weights="softmax", head_bias=None, keep_first=0, value_cols=None, lead=0):
+                        plan=None, softcap=0.0, chunk=0, weights="softmax", head_bias=None, keep_first=0, value_cols=None, lead=0, lead_q_len=0):
         """Causal attention of the step's query rows over the paged keys and values.  ``window`` > 0: a row at position p
         sees keys p - window + 1 .. p, and with ``keep_first`` > 0 also the sequence's first ``keep_first`` keys.  ``chunk`` > 0 (instead of a window): a row at position p sees the keys of its own
         chunk of ``chunk`` positions up to p, chunks counted from position 0 of the sequence.  ``softcap`` > 0: a score s
@@ -1055,8 +1056,9 @@ class CudaOps:
         weighs sigmoid(score + head_bias[head]) (``head_bias`` float32 [num_heads] or None) and nothing is normalised over the
         keys; every kernel but the thread-block-cluster decode form computes them.  ``value_cols`` (n, heads): of a value row
         only a piece is a head's own, the columns h // heads * n .. + n, and ``out`` is [T, num_heads * n] (tensor-core kernels: n
-        a multiple of 8, of 32 with tcgen05).  ``lead`` (kernel "tcpp"): so many first requests bring no more rows than a row tile
-        has and get one tile each, whatever the others bring (``mixed_plan``)."""
+        a multiple of 8, of 32 with tcgen05).  ``lead`` (kernel "tcpp", head size 256): so many first requests bring no more rows than a row tile
+        has and get one tile each, whatever the others bring (``mixed_plan``); ``lead_q_len``: the most tokens that one of them brings, if known.  One
+        that does bring more is an error of the step (``check_tc``)."""
         if weights not in ("softmax", "sigmoid"):
             raise KernelError(f"paged_attention: unknown kind of weights {weights!r}")
         sig = weights == "sigmoid"
@@ -1065,8 +1067,10 @@ class CudaOps:
         T = qkv.shape[0]
         if max_kv_len > block_table.shape[1] * page_size:
             raise KernelError(f"paged_attention: a block table of {block_table.shape[1]} pages of {page_size} keys cannot cover {max_kv_len} keys")
-        if lead and (plan is None or plan[0] != "tcpp"):
-            raise KernelError("paged_attention: leading requests go with the two-tile tcgen05 kernel")
+        if lead and (plan is None or plan[0] != "tcpp" or head_dim != self.mixed_head_dim):
+            raise KernelError("paged_attention: leading requests go with the prompt-portion tcgen05 kernel at head size 256")
+        if lead and lead_q_len * (num_heads // num_kv_heads) > 128:
+            raise KernelError(f"paged_attention: {lead_q_len} tokens of {num_heads // num_kv_heads} heads are more rows than a row tile, leading requests have one")
         kernel, num_splits, split_len = plan if plan is not None else self.attention_plan(
             qkv.dtype, num_seqs, num_heads, num_kv_heads, head_dim, max_q_len, self.visible_keys(max_q_len, max_kv_len, window, chunk, keep_first),
             page_size, sig)
@@ -1083,7 +1087,7 @@ class CudaOps:
                 _ptr(qkv), qkv.stride(0), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
                 block_table.shape[1], page_size, _ptr(query_start_loc), _ptr(seq_lens), _ptr(out), T, num_seqs, num_heads,
                 num_kv_heads, head_dim, max_q_len, float(scale), float(softcap or 0.0), int(window), int(chunk), int(keep_first), num_splits, split_len, _ptr(scratch),
-                1 if kernel == "tcpp" else 0, 1 if sig else 0, _ptr(head_bias), dv, per, 0, lead, self._stream(qkv)), "paged_attention_tc")
+                1 if kernel == "tcpp" else 0, 1 if sig else 0, _ptr(head_bias), dv, per, 0, lead, lead_q_len, self._stream(qkv)), "paged_attention_tc")
             self.launches += 2 if num_splits > 1 else 1
             return
         form = {"mma": 0, "mma_c2": 2, "mma_c4": 4}.get(kernel)
@@ -1199,7 +1203,7 @@ class CudaOps:
             self._check(self.lib.ttie_paged_attention_tc_weights(
                 _ptr(q), q.stride(0), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table), block_table.shape[1], page_size,
                 _ptr(query_start_loc), _ptr(seq_lens), _ptr(out), T, num_seqs, num_heads, kv_heads, width, max_q_len, float(scale), 0.0,
-                int(window), int(chunk), int(keep_first), num_splits, split_len, _ptr(scratch), 1, 0, None, 0, 1, v_dim, 0, self._stream(q)),
+                int(window), int(chunk), int(keep_first), num_splits, split_len, _ptr(scratch), 1, 0, None, 0, 1, v_dim, 0, 0, self._stream(q)),
                 "paged_attention_tc (joint rows)")
             self.launches += 2 if num_splits > 1 else 1
             return

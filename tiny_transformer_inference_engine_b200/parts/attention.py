@@ -361,7 +361,8 @@ class PagedAttention(Mixer):
         if plan is not None:
             ops.paged_attention(q, Hq, Hkv, D, cache.k_pages, cache.v_pages, cache.block_table, cache.page_size, ctx.query_start_loc,
                                 ctx.seq_lens, ctx.num_seqs, classes[1].max_q_len, max(c.max_kv_len for c in classes), self.scale, self.window or 0, out,
-                                plan=plan, softcap=self.softcap or 0.0, chunk=self.chunk or 0, lead=classes[0].seq_hi, **extra)
+                                plan=plan, softcap=self.softcap or 0.0, chunk=self.chunk or 0, lead=classes[0].seq_hi,
+                                lead_q_len=classes[0].max_q_len, **extra)
             return
         for ci, c in enumerate(classes):
             views = self._class_views(ctx, cache, ci, c)
