@@ -650,12 +650,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 //   warp 12      TMA producer: key and value tiles through one ring, in the order the products need them
 //                (K0 K1 V0 K2 V1 K3 ...)
 //   warps 13-14  one thread each issues  O += P(j) V(j)  of one tile
-//   warp 15      one thread issues the scores  S(j) = Q K(j)^T  of both tiles, as soon as K(j) is there and P(j-2) is used up
+//   warp 15      one thread issues the scores  S(j) = Q K(j)^T  of both tiles, as soon as K(j) is there and P(j-2) is used up (one tile: P(j-4))
 // Register budgets follow the roles (setmaxnreg).  Threads of one role run up to two steps apart, so every barrier
 // that counts thread arrivals exists twice (by step parity).
 //
-// ONE tile per CTA (head size 256, joint rows of 512): warps 4-7 take the odd steps of the tile and warps 0-3 the even ones, and the four score buffers
-// are all the tile's, so scores run up to four steps ahead of the products.  With two buffers a buffer's round - scores, their way to
+// ONE tile per CTA (head size 256, joint rows of 512): warps 4-7 take the odd steps of the tile and warps 0-3 the even ones, warp 14 has nothing to
+// do, and the four score buffers (barriers by step % 4) are all the tile's, so scores run up to four steps ahead of the products.  With two buffers a buffer's round - scores, their way to
 // the softmax threads, softmax, its way back, product - takes 3,800 clocks for two steps, whatever the tensor core could do meanwhile (clock
 // stamps of one CTA; handing a barrier over costs 200-450 each time); with four the tensor core is busy 1,310 of 1,540 clocks a step (16 products of
 // 128 x 64 x 16 at 50 clocks, with the queries in shared or in tensor memory alike; 4 of 128 x 256 x 16 at 128).  8 heads of 256: 8,192 tokens 271 -> 227 us,
@@ -701,8 +701,8 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
 }
 
 // D: key size; DO: value columns (D, or fewer: the value columns of one kv head of a joint row).  NT: query tiles per CTA.  Tensor
-// memory holds 2 x 2 x 64 score columns and NT x DO output columns: two tiles up to 128 output columns, one tile (its scores
-// at columns 0..127, its output at 256..511) at 256, and one at 512 key columns, where shared memory holds one query tile.
+// memory holds 256 score columns (two buffers of 64 for each of two tiles, four for one) and behind them NT x DO output columns: two tiles up to
+// 128 output columns, one tile at 256, and one at 512 key columns, where shared memory holds one query tile.
 template <int D, int DO, int NT, int QR = BM>
 __global__ void __launch_bounds__(pp::PP_NTHREADS, 1)
 attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnTcParams p) {
@@ -1100,7 +1100,7 @@ attn_tc_pp_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             // does not complete until those products have finished, 160-260 clocks after the tensor core is done with
             // them.  One issuing thread therefore leaves the tensor core idle for that long between batches.  Three
             // threads issue here, each blocked only behind its own batch: warp 15 the scores of both tiles, warps 13
-            // and 14 the P V products of one tile each.  Between threads nothing is ordered by issue: S(j+2) goes over
+            // and 14 the P V products of one tile each.  Between threads nothing is ordered by issue: S(j + REUSE) goes over
             // P(j) only after the barrier of O += P(j) V(j) has completed.
             // A product of 48-64 clocks leaves its thread a dozen instructions: the descriptors' upper words are
             // constants, the lower words are one addition away from values kept in registers.

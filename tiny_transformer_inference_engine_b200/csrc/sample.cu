@@ -262,9 +262,9 @@ __device__ __forceinline__ void draw_from_list(const unsigned* l_key, const u64*
 // cut, top-p and the draw on the list (`list_cap` entries fit the shared memory that held its slice).  A list of up to SMALL_LIST
 // tokens needs no radix select for that (draw_from_list).  If the list would
 // overflow (thousands of equal values at the bound), every CTA goes on with its whole slice instead.
-// What bounds all this is latency.  8 rows of 32,000 tokens, k 32, top-p 0.9: clocks to the row's maximum 6,300 -> 5,300, the bound 5,600 -> 1,600 (of
-// 256 keys, each compared with all), the list and its way 5,000 -> 4,300 (two exchanges), cuts and draw 8,600 -> 3,200 (12 barriers, sums by
-// shuffles and atomics); the launch 13.7 -> 8.2 us, k 1 13.0 -> 7.6, 32 rows 13.1 -> 9.1, 8 rows of 256,000 tokens 20.1 -> 14.6.
+// What bounds all this is latency.  8 rows of 32,000 tokens, k 32, top-p 0.9: clocks to the row's maximum 6,300 -> 5,400, the bound 5,600 -> 1,300 (of
+// 256 keys, each compared with all), the list and its way 5,000 -> 4,100 (two exchanges), cuts and draw 8,600 -> 3,400 (12 barriers, sums by
+// shuffles and atomics); the launch 13.8 -> 8.3 us, k 1 13.1 -> 7.8, 32 rows 13.2 -> 9.0, 8 rows of 256,000 tokens 20.1 -> 14.6.
 // Top-p without a top-k leaves the row the same way when the distribution is peaked: the (at most 1,024) tokens that hold
 // 1 / 1,024 of the row's mass or more each are listed, and if together they hold more than top_p of the mass the cut lies
 // among them.  A flat row (the listed tokens hold too little) is walked whole as before.

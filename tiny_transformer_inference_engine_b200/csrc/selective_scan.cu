@@ -37,7 +37,8 @@ __device__ __forceinline__ int slot_row_(int slot, int num_rows) { return slot <
 // bfloat16 operands around it).
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // softplus and silu: the library's accurate functions in a 32-bit run; else the hardware's exponential, logarithm and reciprocal
-// (relative error about 1e-6 as well: log(1 + e) of a small e, where 1 + e has lost its digits, by the series e - e^2/2 + e^3/3).
+// (relative error about 1e-6 as well: log(1 + e) of a small e, where 1 + e has lost its digits, by the series e - e^2/2 + e^3/3; a step size below
+// 2^-126 counts as none: with such ones kept the scan takes 1 % longer).
 template <typename T> struct Act {
     static __device__ __forceinline__ float softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
     static __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }

@@ -1622,13 +1622,15 @@ class CudaOps:
         (StepContext.max_q_len, which also holds for a captured graph); None: the step's tokens less one for every other request.
 
         A walk takes its time from the longest request's chain of tokens or from the whole step's work on the state elements,
-        whichever is longer; chunks have three launches, a state to load and store per request and less work per token.  The
-        figures above give both within a fifth over widths of 512 to 4,096, 1 to 24 requests and 16 to 1,024 tokens.  And an eager pass of the layer
-        takes the longer of its kernels' and its host's time, of which chunks need more: they pay where the pass is shorter with them
-        (the whole mixer of 300 tokens at width 1,024, walk | chunks: retention 105 | 99, mlstm 108 | 111, wkv 126 | 141).  The scan alone, walk | chunks,
-        us, width 2,048: one request of 128 tokens retention 31 | 30, mlstm 30 | 26, wkv 26 | 34, of 512 tokens 116 | 32, 107 | 27,
-        93 | 41; eight of 16 tokens 29 | 57, 21 | 44, 17 | 41, of 64 tokens 96 | 41, 68 | 32, 55 | 44; 256 tokens beside 23 decoding
-        requests 87 | 87, 81 | 59, 63 | 87."""
+        whichever is longer; chunks have three launches, a state to load and store per request and less work per token.  And an eager pass of the layer
+        takes the longer of its kernels' and its host's time: chunks pay where the pass is shorter with them (the whole mixer of 300 tokens at
+        width 1,024, walk | chunks: retention 95 | 92, mlstm 106 | 90, wkv 120 | 133).  The scan alone with norm and gate, walk | chunks,
+        us, width 2,048: one request of 128 tokens retention 37 | 32, mlstm 32 | 27, wkv 35 | 37, of 512 tokens 134 | 33, 109 | 28,
+        123 | 44; eight of 16 tokens 31 | 60, 23 | 47, 20 | 46, of 64 tokens 99 | 42, 71 | 33, 58 | 53; 256 tokens beside 23 decoding
+        requests 89 | 90, 83 | 62, 66 | 96.  The figures above are older than chunks that norm and gate their read-outs and than wkv's
+        present kernels: a layer comes out a fifth (walk) to a half (chunks) too long with them, and mlstm's chunks of 128 tokens now need 16 us less of the host
+        than a walk, not 2 more.  Over 123 steps of each kind (widths of 512 to 4,096, 1 to 32 requests, 64 to 2,048 tokens) the choice is 0.3 %
+        (retention), 7 % (mlstm; 39 % for 450 tokens of three requests at width 2,048, walked) and 0.5 % (wkv) behind the better one on average."""
         if not 8 <= dim <= 128 or dim % 8 or v_dim % 8:
             return False
         others = num_seqs - 1
